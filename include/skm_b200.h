@@ -243,12 +243,13 @@ skm_status skm_comm_wrap(void* nccl_comm, int rank, int world, skm_comm** out);
 void skm_comm_destroy(skm_comm* comm);
 skm_status skm_set_shard_comm(skm_handle* h, uint64_t n_global, uint64_t row_offset, skm_comm* comm);
 
-/* Workspace cache (off by default).  When on, device buffers of 32 MB and more that a handle releases (the rotated
- * copy of the training rows, sort and list workspaces) are kept by the library and reused by later calls that need
- * about the same size on the same GPU, so that repeated Train calls of one shape do not pay cudaMalloc / cudaFree of
- * tens of gigabytes (both synchronise the device) every time.  The memory stays with the library until
- * skm_release_cached_memory, skm_set_workspace_cache(0) or the end of the process; an allocation that fails drops the
- * cache and retries.  No counterpart in the reference. */
+/* Workspace cache.  Device buffers that a call or a handle releases (the rotated copy of the training rows, sort and
+ * list workspaces) are kept by the library and reused by later calls that need about the same size on the same GPU, so
+ * that repeated calls do not pay cudaMalloc / cudaFree (both synchronise the device) every time.  By default what is
+ * kept stays within a sixteenth of the GPU's memory.  skm_set_workspace_cache(1) lifts that bound (repeated Train calls
+ * over tens of gigabytes), skm_set_workspace_cache(0) keeps nothing from then on; skm_get_workspace_cache tells whether
+ * the bound is lifted.  The memory goes back to the driver with skm_release_cached_memory, skm_set_workspace_cache(0)
+ * or the end of the process; an allocation that fails releases it and retries.  No counterpart in the reference. */
 void skm_set_workspace_cache(int enabled);
 int skm_get_workspace_cache(void);
 void skm_release_cached_memory(void);

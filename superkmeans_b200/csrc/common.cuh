@@ -4,6 +4,8 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 #include <stdexcept>
@@ -29,18 +31,38 @@ void note_kernel_launch();
 unsigned long long device_alloc_count();
 void note_device_alloc();
 
-// Device memory of DeviceBuffer.  With the workspace cache switched on (off by default), blocks of 32 MB and more are
-// kept when released and handed out again to later requests of about the same size on the same device, so that
-// repeated Train calls of one shape do not pay cudaMalloc / cudaFree (both synchronise the device, and both take
-// tens of milliseconds at tens of gigabytes) every time.  The price: the memory stays with this library until
-// release_cached_memory() or the end of the process.
-void* device_alloc(size_t bytes);
-void device_free(void* p, size_t bytes);
+// Device memory of DeviceBuffer, pinned host memory of PinnedBuffer, and the engines' streams.  What is released is parked
+// for the next request (memory.cu says within which bounds); set_workspace_cache(true) lifts the bound, so that repeated
+// Train calls over tens of gigabytes do not pay cudaMalloc / cudaFree either, and set_workspace_cache(false) parks nothing.
+struct MemoryBlock {
+    void* p = nullptr;
+    size_t bytes = 0;   // true size: what was asked for, rounded up
+    int device = 0;     // GPU that was current when it was allocated
+};
+MemoryBlock device_alloc(size_t bytes);
+void device_free(const MemoryBlock& m);
+MemoryBlock pinned_alloc(size_t bytes);
+void pinned_free(const MemoryBlock& m);
+// A non-blocking stream of the current device; release_stream waits for the work on it.
+cudaStream_t acquire_stream();
+void release_stream(cudaStream_t s, int device);
+// While one is alive, what its thread allocates and releases is used by work on `stream`.
+class WorkStream {
+  public:
+    explicit WorkStream(cudaStream_t stream);
+    ~WorkStream();
+    WorkStream(const WorkStream&) = delete;
+    WorkStream& operator=(const WorkStream&) = delete;
+
+  private:
+    bool was_on_;
+    cudaStream_t previous_;
+};
 void set_workspace_cache(bool on);
 bool workspace_cache_enabled();
 void release_cached_memory();
 size_t cached_memory_bytes();
-// wall-clock milliseconds this thread has spent inside cudaMalloc / cudaFree through device_alloc / device_free
+// wall-clock milliseconds this thread has spent inside device_alloc / device_free
 double alloc_free_ms();
 // After every kernel launch: count it and surface launch-configuration errors.
 #define SKM_LAUNCH_CHECK()                                                                         \

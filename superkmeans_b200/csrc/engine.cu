@@ -31,6 +31,13 @@ struct DeviceGuard {
     }
 };
 
+// Every entry point: the engine's GPU is current, and memory it takes or gives up is used on its stream.
+struct Entry {
+    DeviceGuard guard;
+    WorkStream work;
+    Entry(int device, cudaStream_t stream) : guard(device), work(stream) {}
+};
+
 __global__ void u64_to_f64_kernel(const unsigned long long* in, double* out) { *out = static_cast<double>(*in); }
 
 __global__ void widen_u32_kernel(const uint32_t* __restrict__ in, uint64_t* __restrict__ out, size_t n) {
@@ -158,8 +165,9 @@ Engine::Engine(const skm_config& cfg, size_t n_clusters, size_t d, bool hierarch
     device_ = resolve_device(device);
     if (device_ >= count) throw std::invalid_argument("device ordinal out of range");
     DeviceGuard guard(device_);
-    SKM_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
-    SKM_CUDA(cudaStreamCreateWithFlags(&copy_stream_, cudaStreamNonBlocking));
+    stream_ = acquire_stream();
+    copy_stream_ = acquire_stream();
+    WorkStream work(stream_);
     ratios_host_ = make_ratios(d, epsilon0_);
     SKM_CUDA(cudaMemcpy(ratios_dev_.ensure(d + 1), ratios_host_.data(), sizeof(float) * (d + 1), cudaMemcpyHostToDevice));
     scalars_dev_.ensure(8);
@@ -173,9 +181,13 @@ Engine::Engine(const skm_config& cfg, size_t n_clusters, size_t d, bool hierarch
 }
 
 Engine::~Engine() {
-    cudaSetDevice(device_);
-    if (stream_) cudaStreamDestroy(stream_);
-    if (copy_stream_) cudaStreamDestroy(copy_stream_);
+    // the streams are waited for: the buffers released after this are idle
+    int prev = device_;
+    cudaGetDevice(&prev);
+    if (prev != device_) cudaSetDevice(device_);
+    release_stream(stream_, device_);
+    release_stream(copy_stream_, device_);
+    if (prev != device_) cudaSetDevice(prev);
 }
 
 const std::vector<skm_iter_stats>& Engine::stats(int phase) const {
@@ -201,14 +213,14 @@ void Engine::ensure_rotation() {
 }
 
 void Engine::set_rotation(const float* m_host) {
-    DeviceGuard guard(device_);
+    Entry entry(device_, stream_);
     rotation_host_.assign(m_host, m_host + d_ * d_);
     rotation_ready_ = false;
     ensure_rotation();
 }
 
 void Engine::get_rotation(float* m_out) {
-    DeviceGuard guard(device_);
+    Entry entry(device_, stream_);
     ensure_rotation();
     std::memcpy(m_out, rotation_host_.data(), sizeof(float) * d_ * d_);
 }
@@ -279,6 +291,9 @@ void Engine::rotate_to_device(const float* src, bool src_on_device, size_t n, fl
         SKM_CUDA(cudaEventCreateWithFlags(&copied[i], cudaEventDisableTiming));
         SKM_CUDA(cudaEventCreateWithFlags(&consumed[i], cudaEventDisableTiming));
     }
+    // the staging buffers may still be in use by earlier work that was enqueued on stream_
+    SKM_CUDA(cudaEventRecord(consumed[0], stream_));
+    SKM_CUDA(cudaStreamWaitEvent(copy_stream_, consumed[0], 0));
     size_t ci = 0, handed = 0;
     for (size_t r0 = 0; r0 < n; r0 += rows, ++ci) {
         const int b = static_cast<int>(ci & 1);
@@ -1118,7 +1133,7 @@ void Engine::run_iteration(bool gemm_only, const IterationInput& in, size_t iter
 // Train
 // -------------------------------------------------------------------------------------------------
 void Engine::train(const float* data, size_t n, bool on_device, const float* queries, size_t n_queries, float* centroids_out) {
-    DeviceGuard guard(device_);
+    Entry entry(device_, stream_);
     ensure_positive(n > 0, "n");
     if (trained_) throw std::runtime_error("The clustering has already been trained");
     const size_t n_global = sharded_() ? shard_n_global_ : n;
@@ -1575,7 +1590,7 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
 // chunks so that host inputs of any size fit.
 // -------------------------------------------------------------------------------------------------
 void Engine::assign(const float* vectors, const float* centroids, size_t n, size_t n_centroids, bool on_device, uint32_t* out) {
-    DeviceGuard guard(device_);
+    Entry entry(device_, stream_);
     if (n == 0) return;
     if (n_centroids == 0) throw std::invalid_argument("Value must be positive: n_centroids");
     DeviceBuffer<float> c_dev_own, cn;
@@ -1612,6 +1627,9 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
         SKM_CUDA(cudaEventCreateWithFlags(&copied[i], cudaEventDisableTiming));
         SKM_CUDA(cudaEventCreateWithFlags(&consumed[i], cudaEventDisableTiming));
     }
+    // the staging buffers may still be in use by earlier work that was enqueued on stream_
+    SKM_CUDA(cudaEventRecord(consumed[0], stream_));
+    SKM_CUDA(cudaStreamWaitEvent(copy_stream_, consumed[0], 0));
     size_t ci = 0;
     top2_.ensure(rows);
     y_split_.ensure(2 * n_centroids * d_);
@@ -1641,7 +1659,7 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
 // AssignTrainingPoints (superkmeans.h:397-564)
 // -------------------------------------------------------------------------------------------------
 void Engine::assign_training_points(const float* vectors, const float* centroids, size_t n, size_t n_centroids, bool on_device, uint32_t* out) {
-    DeviceGuard guard(device_);
+    Entry entry(device_, stream_);
     if (!trained_) throw std::runtime_error("AssignTrainingPoints requires SuperKMeans to be trained first");
     if (cfg_.use_blas_only || d_ < kDimensionThresholdForPruning || k_ <= kNClustersThresholdForPruning) {
         if (!cfg_.suppress_warnings) {
@@ -1742,19 +1760,19 @@ void Engine::assign_training_points(const float* vectors, const float* centroids
 }
 
 void Engine::get_assignments(uint32_t* out, size_t n) {
-    DeviceGuard guard(device_);
+    Entry entry(device_, stream_);
     if (n > n_state_rows_ || n > assignments_.capacity()) throw std::invalid_argument("more assignments requested than the engine holds");
     SKM_CUDA(cudaMemcpy(out, assignments_.get(), sizeof(uint32_t) * n, cudaMemcpyDeviceToHost));
 }
 
 void Engine::get_distances(float* out, size_t n) {
-    DeviceGuard guard(device_);
+    Entry entry(device_, stream_);
     if (n > n_state_rows_ || n > distances_.capacity()) throw std::invalid_argument("more distances requested than the engine holds");
     SKM_CUDA(cudaMemcpy(out, distances_.get(), sizeof(float) * n, cudaMemcpyDeviceToHost));
 }
 
 void Engine::get_rotated_centroids(float* out) {
-    DeviceGuard guard(device_);
+    Entry entry(device_, stream_);
     if (!trained_) throw std::runtime_error("the model has not been trained");
     SKM_CUDA(cudaMemcpy(out, c_cur_.get(), sizeof(float) * k_ * d_, cudaMemcpyDeviceToHost));
 }
@@ -1764,12 +1782,12 @@ void Engine::get_rotated_centroids(float* out) {
 // -------------------------------------------------------------------------------------------------
 namespace {
 struct OpContext {
+    int device;
     DeviceGuard guard;
-    cudaStream_t stream = nullptr;
-    explicit OpContext(int device) : guard(resolve_device(device)) { SKM_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking)); }
-    ~OpContext() {
-        if (stream) cudaStreamDestroy(stream);
-    }
+    cudaStream_t stream;
+    WorkStream work;
+    explicit OpContext(int device_) : device(resolve_device(device_)), guard(device), stream(acquire_stream()), work(stream) {}
+    ~OpContext() { release_stream(stream, device); }
     template <class T>
     T* upload(DeviceBuffer<T>& buf, const T* host, size_t count) {
         T* p = buf.ensure(count);

@@ -16,70 +16,43 @@
 
 namespace skmb {
 
-template <class T>
-class DeviceBuffer {
+// A typed array in memory that ALLOC / FREE hand out.
+template <class T, MemoryBlock (*ALLOC)(size_t), void (*FREE)(const MemoryBlock&)>
+class Buffer {
   public:
-    DeviceBuffer() = default;
-    DeviceBuffer(const DeviceBuffer&) = delete;
-    DeviceBuffer& operator=(const DeviceBuffer&) = delete;
-    ~DeviceBuffer() { release(); }
+    Buffer() = default;
+    Buffer(const Buffer&) = delete;
+    Buffer& operator=(const Buffer&) = delete;
+    ~Buffer() { release(); }
     void release() {
-        if (p_) device_free(p_, bytes_);
-        p_ = nullptr;
+        FREE(m_);
+        m_ = MemoryBlock{};
         cap_ = 0;
-        bytes_ = 0;
     }
     // Grows (never shrinks) to at least `count` elements; contents are not preserved on growth.
     T* ensure(size_t count) {
-        if (count > cap_) {
+        if (count > cap_ || !m_.p) {
             release();
-            bytes_ = sizeof(T) * (count ? count : 1);
-            p_ = static_cast<T*>(device_alloc(bytes_));
+            m_ = ALLOC(sizeof(T) * (count ? count : 1));
             cap_ = count;
         }
-        return p_;
+        return get();
     }
-    T* get() const { return p_; }
+    T* get() const { return static_cast<T*>(m_.p); }
     size_t capacity() const { return cap_; }
-    void swap(DeviceBuffer& o) {
-        std::swap(p_, o.p_);
+    void swap(Buffer& o) {
+        std::swap(m_, o.m_);
         std::swap(cap_, o.cap_);
-        std::swap(bytes_, o.bytes_);
     }
 
   private:
-    T* p_ = nullptr;
+    MemoryBlock m_;
     size_t cap_ = 0;
-    size_t bytes_ = 0;
 };
-
 template <class T>
-class PinnedBuffer {
-  public:
-    PinnedBuffer() = default;
-    PinnedBuffer(const PinnedBuffer&) = delete;
-    PinnedBuffer& operator=(const PinnedBuffer&) = delete;
-    ~PinnedBuffer() { release(); }
-    void release() {
-        if (p_) cudaFreeHost(p_);
-        p_ = nullptr;
-        cap_ = 0;
-    }
-    T* ensure(size_t count) {
-        if (count > cap_) {
-            release();
-            note_device_alloc();
-            SKM_CUDA(cudaMallocHost(&p_, sizeof(T) * (count ? count : 1)));
-            cap_ = count;
-        }
-        return p_;
-    }
-    T* get() const { return p_; }
-
-  private:
-    T* p_ = nullptr;
-    size_t cap_ = 0;
-};
+using DeviceBuffer = Buffer<T, device_alloc, device_free>;
+template <class T>
+using PinnedBuffer = Buffer<T, pinned_alloc, pinned_free>;
 
 // Accumulating per-phase device timers (CUDA events on the engine's stream); names follow the
 // sections of the reference's profiler (profiler.h): rotator, norms_calc, search/1st_blas, search,

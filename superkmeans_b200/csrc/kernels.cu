@@ -13,11 +13,6 @@
 
 #include <atomic>
 #include <cfloat>
-#include <cstdlib>
-#include <chrono>
-#include <mutex>
-#include <unordered_map>
-#include <vector>
 
 namespace skmb {
 
@@ -25,130 +20,6 @@ namespace skmb {
 static std::atomic<unsigned long long> g_kernel_launches{0};
 unsigned long long kernel_launch_count() { return g_kernel_launches.load(); }
 void note_kernel_launch() { g_kernel_launches.fetch_add(1, std::memory_order_relaxed); }
-static std::atomic<unsigned long long> g_device_allocs{0};
-unsigned long long device_alloc_count() { return g_device_allocs.load(std::memory_order_relaxed); }
-void note_device_alloc() { g_device_allocs.fetch_add(1, std::memory_order_relaxed); }
-
-// ---- device memory with an optional cache of large blocks (see common.cuh)
-namespace {
-struct CachedBlock {
-    void* p;
-    size_t bytes;
-    int device;
-};
-std::mutex g_cache_mu;
-std::vector<CachedBlock> g_cache;
-std::unordered_map<void*, size_t> g_block_bytes;   // true size of every live block that was allocated through the cache path
-bool g_cache_on = false;
-constexpr size_t kCacheMinBytes = size_t{64} << 10;
-
-// Sizes are rounded up to one of eight steps per power of two, so that requests that differ a little from call to call
-// (buffers sized by a count that the data decide) land on the same block sizes and find each other in the cache.
-size_t cache_bucket(size_t bytes) {
-    size_t p2 = size_t{1} << 16;
-    while (p2 * 2 <= bytes) p2 *= 2;
-    const size_t step = p2 / 8;
-    return (bytes + step - 1) / step * step;
-}
-thread_local double g_alloc_ms = 0.0;
-
-struct AllocClock {
-    std::chrono::steady_clock::time_point t0 = std::chrono::steady_clock::now();
-    ~AllocClock() { g_alloc_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count(); }
-};
-
-void drop_cache_locked() {
-    int cur = 0;
-    cudaGetDevice(&cur);
-    for (auto& b : g_cache) {
-        cudaSetDevice(b.device);
-        cudaFree(b.p);
-    }
-    g_cache.clear();
-    cudaSetDevice(cur);
-}
-} // namespace
-
-void* device_alloc(size_t bytes) {
-    AllocClock clock;
-    int device = 0;
-    SKM_CUDA(cudaGetDevice(&device));
-    const bool cached_path = g_cache_on && bytes >= kCacheMinBytes;
-    if (cached_path) {
-        bytes = cache_bucket(bytes);
-        std::lock_guard<std::mutex> lock(g_cache_mu);
-        size_t best = g_cache.size();
-        for (size_t i = 0; i < g_cache.size(); ++i) {
-            const CachedBlock& b = g_cache[i];
-            if (b.device == device && b.bytes >= bytes && b.bytes <= bytes + bytes / 4 && (best == g_cache.size() || b.bytes < g_cache[best].bytes)) best = i;
-        }
-        if (best != g_cache.size()) {
-            void* p = g_cache[best].p;
-            g_block_bytes[p] = g_cache[best].bytes;
-            g_cache.erase(g_cache.begin() + static_cast<long>(best));
-            return p;
-        }
-    }
-    note_device_alloc();
-    void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, bytes);
-    if (e == cudaErrorMemoryAllocation) {
-        // what the cache holds may be exactly what is missing
-        cudaGetLastError();
-        {
-            std::lock_guard<std::mutex> lock(g_cache_mu);
-            drop_cache_locked();
-        }
-        e = cudaMalloc(&p, bytes);
-    }
-    cuda_check(e, "cudaMalloc", __FILE__, __LINE__);
-    if (cached_path) {
-        std::lock_guard<std::mutex> lock(g_cache_mu);
-        g_block_bytes[p] = bytes;
-    }
-    return p;
-}
-
-void device_free(void* p, size_t bytes) {
-    if (!p) return;
-    AllocClock clock;
-    {
-        std::lock_guard<std::mutex> lock(g_cache_mu);
-        const auto it = g_block_bytes.find(p);
-        if (it != g_block_bytes.end()) {
-            bytes = it->second;   // the block's true (rounded-up) size
-            g_block_bytes.erase(it);
-        }
-    }
-    if (g_cache_on && bytes >= kCacheMinBytes) {
-        int device = 0;
-        if (cudaGetDevice(&device) == cudaSuccess) {
-            std::lock_guard<std::mutex> lock(g_cache_mu);
-            g_cache.push_back(CachedBlock{p, bytes, device});
-            return;
-        }
-    }
-    cudaFree(p);
-}
-
-void set_workspace_cache(bool on) {
-    std::lock_guard<std::mutex> lock(g_cache_mu);
-    g_cache_on = on;
-    if (!on) drop_cache_locked();
-}
-bool workspace_cache_enabled() { return g_cache_on; }
-void release_cached_memory() {
-    std::lock_guard<std::mutex> lock(g_cache_mu);
-    drop_cache_locked();
-}
-size_t cached_memory_bytes() {
-    std::lock_guard<std::mutex> lock(g_cache_mu);
-    size_t total = 0;
-    for (const auto& b : g_cache) total += b.bytes;
-    return total;
-}
-double alloc_free_ms() { return g_alloc_ms; }
-
 // =================================================================================================
 // Row squared norms over the first `upto` columns: one warp per row.
 // =================================================================================================

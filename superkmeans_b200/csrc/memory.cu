@@ -1,0 +1,282 @@
+// Device memory, pinned host memory and streams of this library (see common.cuh).
+//
+// cudaMalloc and cudaFree synchronise the device and cost from 10 microseconds to hundreds of milliseconds each
+// (measured on a B200: 70 pairs per flat Train of 1M x 1024, 0.1 - 0.7 s of its 0.6 - 1.1 s of wall time), so blocks that
+// a call or a handle gives up are parked here and handed to the next request of about their size.
+//
+//   * Bounded: by default the parked blocks of one GPU stay within a sixteenth of its memory and the pinned ones within
+//     256 MB; beyond that the blocks parked longest are returned to the driver.  set_workspace_cache(1) lifts the bound,
+//     set_workspace_cache(0) parks nothing, release_cached_memory() returns everything that is parked, and an
+//     allocation that fails does so before it is tried again.
+//   * Safe between streams and threads: a block released while its thread works on a stream (WorkStream) carries an event
+//     recorded there, and whoever gets the block next makes its own stream wait for that event.  A block released
+//     outside such a scope must be idle (the owners synchronise first).
+#include <chrono>
+#include <mutex>
+#include <vector>
+
+#include "common.cuh"
+
+namespace skmb {
+
+namespace {
+
+std::atomic<unsigned long long> g_device_allocs{0};
+thread_local double g_alloc_ms = 0.0;
+thread_local bool t_on_stream = false;
+thread_local cudaStream_t t_stream = nullptr;
+
+struct AllocClock {
+    std::chrono::steady_clock::time_point t0 = std::chrono::steady_clock::now();
+    ~AllocClock() { g_alloc_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count(); }
+};
+
+struct Parked {
+    void* p;
+    size_t bytes;
+    int device;
+    cudaEvent_t last_use;   // null: idle
+};
+
+constexpr int kMaxDevices = 64;
+constexpr int kHost = -1;                 // "device" of pinned host blocks
+constexpr size_t kPinnedBound = size_t{256} << 20;
+constexpr size_t kMaxIdleStreams = 16;    // per device
+
+enum class CacheMode { bounded, everything, nothing };
+
+std::mutex g_mu;
+std::vector<Parked> g_parked;   // oldest first
+CacheMode g_mode = CacheMode::bounded;
+std::vector<cudaEvent_t> g_events[kMaxDevices];
+std::vector<cudaStream_t> g_streams[kMaxDevices];
+
+// Sizes are rounded up to one of eight steps per power of two, so that requests that differ a little from call to call
+// (buffers sized by a count that the data decide) land on the same block sizes and find each other's blocks.
+size_t bucket(size_t bytes) {
+    size_t p2 = 512;
+    while (p2 * 2 <= bytes) p2 *= 2;
+    const size_t step = p2 / 8;
+    return std::max<size_t>(512, (bytes + step - 1) / step * step);
+}
+
+size_t bound_of(int device) {
+    if (device == kHost) return kPinnedBound;
+    static size_t bounds[kMaxDevices] = {0};   // under g_mu
+    if (bounds[device] == 0) {
+        size_t free_bytes = 0, total = 0;
+        bounds[device] = cudaMemGetInfo(&free_bytes, &total) == cudaSuccess ? total / 16 : size_t{1} << 30;
+    }
+    return bounds[device];
+}
+
+void give_back(const Parked& b) {
+    if (b.last_use) {
+        cudaEventSynchronize(b.last_use);
+        cudaEventDestroy(b.last_use);
+    }
+    if (b.device == kHost) {
+        cudaFreeHost(b.p);
+        return;
+    }
+    int cur = 0;
+    cudaGetDevice(&cur);
+    if (cur != b.device) cudaSetDevice(b.device);
+    cudaFree(b.p);
+    if (cur != b.device) cudaSetDevice(cur);
+}
+
+void give_back_all(const std::vector<Parked>& blocks) {
+    for (const Parked& b : blocks) give_back(b);
+}
+
+std::vector<Parked> take_all_parked() {
+    std::lock_guard<std::mutex> lock(g_mu);
+    std::vector<Parked> out;
+    out.swap(g_parked);
+    return out;
+}
+
+// The smallest parked block of this device (or of the host) that holds `bytes` and is at most a quarter larger.
+bool take_parked(size_t bytes, int device, Parked& out) {
+    std::lock_guard<std::mutex> lock(g_mu);
+    size_t best = g_parked.size();
+    for (size_t i = 0; i < g_parked.size(); ++i) {
+        const Parked& b = g_parked[i];
+        if (b.device == device && b.bytes >= bytes && b.bytes <= bytes + bytes / 4 && (best == g_parked.size() || b.bytes < g_parked[best].bytes)) best = i;
+    }
+    if (best == g_parked.size()) return false;
+    out = g_parked[best];
+    g_parked.erase(g_parked.begin() + static_cast<long>(best));
+    return true;
+}
+
+// Orders the new owner of a block after its last one.
+void settle(const Parked& b, int event_device) {
+    if (!b.last_use) return;
+    if (b.device == kHost || !t_on_stream) cudaEventSynchronize(b.last_use);
+    else SKM_CUDA(cudaStreamWaitEvent(t_stream, b.last_use, 0));
+    std::lock_guard<std::mutex> lock(g_mu);
+    g_events[event_device].push_back(b.last_use);
+}
+
+void park(Parked b, int event_device) {
+    if (t_on_stream) {
+        {
+            std::lock_guard<std::mutex> lock(g_mu);
+            auto& pool = g_events[event_device];
+            if (!pool.empty()) {
+                b.last_use = pool.back();
+                pool.pop_back();
+            }
+        }
+        if (!b.last_use && cudaEventCreateWithFlags(&b.last_use, cudaEventDisableTiming) != cudaSuccess) b.last_use = nullptr;
+        if (!b.last_use || cudaEventRecord(b.last_use, t_stream) != cudaSuccess) {
+            give_back(b);
+            return;
+        }
+    }
+    std::vector<Parked> surplus;
+    {
+        std::lock_guard<std::mutex> lock(g_mu);
+        if (g_mode == CacheMode::nothing) {
+            surplus.push_back(b);
+        } else {
+            g_parked.push_back(b);
+            if (g_mode == CacheMode::bounded) {
+                size_t total = 0;
+                for (const Parked& q : g_parked) total += q.device == b.device ? q.bytes : 0;
+                for (size_t i = 0; i < g_parked.size() && total > bound_of(b.device);) {
+                    if (g_parked[i].device != b.device) {
+                        ++i;
+                        continue;
+                    }
+                    total -= g_parked[i].bytes;
+                    surplus.push_back(g_parked[i]);
+                    g_parked.erase(g_parked.begin() + static_cast<long>(i));
+                }
+            }
+        }
+    }
+    give_back_all(surplus);
+}
+
+} // namespace
+
+unsigned long long device_alloc_count() { return g_device_allocs.load(std::memory_order_relaxed); }
+void note_device_alloc() { g_device_allocs.fetch_add(1, std::memory_order_relaxed); }
+double alloc_free_ms() { return g_alloc_ms; }
+
+WorkStream::WorkStream(cudaStream_t stream) : was_on_(t_on_stream), previous_(t_stream) {
+    t_on_stream = true;
+    t_stream = stream;
+}
+WorkStream::~WorkStream() {
+    t_on_stream = was_on_;
+    t_stream = previous_;
+}
+
+MemoryBlock device_alloc(size_t bytes) {
+    AllocClock clock;
+    MemoryBlock m;
+    SKM_CUDA(cudaGetDevice(&m.device));
+    bytes = bucket(bytes);
+    Parked b;
+    if (take_parked(bytes, m.device, b)) {
+        settle(b, m.device);
+        m.p = b.p;
+        m.bytes = b.bytes;
+        return m;
+    }
+    note_device_alloc();
+    cudaError_t e = cudaMalloc(&m.p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        // what is parked may be exactly what is missing
+        cudaGetLastError();
+        give_back_all(take_all_parked());
+        e = cudaMalloc(&m.p, bytes);
+    }
+    cuda_check(e, "cudaMalloc", __FILE__, __LINE__);
+    m.bytes = bytes;
+    return m;
+}
+
+void device_free(const MemoryBlock& m) {
+    if (!m.p) return;
+    AllocClock clock;
+    park(Parked{m.p, m.bytes, m.device, nullptr}, m.device);
+}
+
+MemoryBlock pinned_alloc(size_t bytes) {
+    MemoryBlock m;
+    SKM_CUDA(cudaGetDevice(&m.device));
+    bytes = bucket(bytes);
+    Parked b;
+    if (take_parked(bytes, kHost, b)) {
+        settle(b, m.device);
+        m.p = b.p;
+        m.bytes = b.bytes;
+        return m;
+    }
+    note_device_alloc();
+    SKM_CUDA(cudaHostAlloc(&m.p, bytes, cudaHostAllocPortable));
+    m.bytes = bytes;
+    return m;
+}
+
+void pinned_free(const MemoryBlock& m) {
+    if (m.p) park(Parked{m.p, m.bytes, kHost, nullptr}, m.device);
+}
+
+cudaStream_t acquire_stream() {
+    int device = 0;
+    SKM_CUDA(cudaGetDevice(&device));
+    {
+        std::lock_guard<std::mutex> lock(g_mu);
+        auto& pool = g_streams[device];
+        if (!pool.empty()) {
+            const cudaStream_t s = pool.back();
+            pool.pop_back();
+            return s;
+        }
+    }
+    cudaStream_t s = nullptr;
+    SKM_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    return s;
+}
+
+void release_stream(cudaStream_t s, int device) {
+    if (!s) return;
+    if (cudaStreamSynchronize(s) == cudaSuccess) {
+        std::lock_guard<std::mutex> lock(g_mu);
+        if (g_streams[device].size() < kMaxIdleStreams) {
+            g_streams[device].push_back(s);
+            return;
+        }
+    }
+    cudaStreamDestroy(s);
+}
+
+void set_workspace_cache(bool on) {
+    {
+        std::lock_guard<std::mutex> lock(g_mu);
+        g_mode = on ? CacheMode::everything : CacheMode::nothing;
+    }
+    if (!on) release_cached_memory();
+}
+
+bool workspace_cache_enabled() {
+    std::lock_guard<std::mutex> lock(g_mu);
+    return g_mode == CacheMode::everything;
+}
+
+void release_cached_memory() { give_back_all(take_all_parked()); }
+
+size_t cached_memory_bytes() {
+    std::lock_guard<std::mutex> lock(g_mu);
+    size_t total = 0;
+    for (const Parked& b : g_parked) total += b.device == kHost ? 0 : b.bytes;
+    return total;
+}
+
+} // namespace skmb

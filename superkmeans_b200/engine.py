@@ -253,7 +253,8 @@ class Comm:
 
 
 def set_workspace_cache(enabled: bool) -> None:
-    """Keep large device buffers between calls (see skm_set_workspace_cache); off by default."""
+    """Keep device buffers between calls without a bound (True) or not at all (False); the default keeps a bounded amount
+    (see skm_set_workspace_cache)."""
     lib.skm_set_workspace_cache(int(enabled))
 
 
