@@ -181,6 +181,7 @@ Engine::Engine(const skm_config& cfg, size_t n_clusters, size_t d, bool hierarch
 }
 
 Engine::~Engine() {
+    if (draws_done_.valid()) draws_done_.wait();
     // the streams are waited for: the buffers released after this are idle
     int prev = device_;
     cudaGetDevice(&prev);
@@ -202,14 +203,47 @@ const std::vector<skm_iter_stats>& Engine::stats(int phase) const {
 // -------------------------------------------------------------------------------------------------
 // Rotation (adsampling.h:76-85, :191-215, :273-298)
 // -------------------------------------------------------------------------------------------------
+void Engine::start_rotation_draws() {
+    if (rotation_ready_ || !rotation_host_.empty() || draws_) return;
+    draws_ = std::make_unique<NormalDraws>(d_ * d_, cfg_.seed);
+    uint32_t* bits = draw_bits_.ensure(draws_->scratch());
+    float* values = draw_values_.ensure(draws_->scratch());
+    draws_done_ = std::async(std::launch::async, [this, bits, values] { return draws_->make(bits, values); });
+}
+
 void Engine::ensure_rotation() {
     if (rotation_ready_) return;
-    if (rotation_host_.empty()) rotation_host_ = make_rotation_matrix(d_, cfg_.seed);
-    SKM_CUDA(cudaMemcpyAsync(m_dev_.ensure(d_ * d_), rotation_host_.data(), sizeof(float) * d_ * d_, cudaMemcpyHostToDevice, stream_));
-    mt_dev_.ensure(d_ * d_);
-    launch_transpose_square(m_dev_.get(), mt_dev_.get(), d_, stream_);
+    float* m = m_dev_.ensure(d_ * d_);
+    bool made = false;
+    if (rotation_host_.empty()) {
+        start_rotation_draws();
+        if (draws_done_.get()) {
+            float* dst = mt_dev_.ensure(d_ * d_);   // (not needed for the transpose yet)
+            const float* draws = dst;
+            for (const auto& piece : draws_->pieces()) {
+                SKM_CUDA(cudaMemcpyAsync(dst, piece.values, sizeof(float) * piece.count, cudaMemcpyHostToDevice, stream_));
+                dst += piece.count;
+            }
+            made = make_rotation_matrix_on_device(draws, d_, m, stream_);
+        }
+        if (!made) rotation_host_ = make_rotation_matrix(d_, cfg_.seed);
+    }
+    if (!made) SKM_CUDA(cudaMemcpyAsync(m, rotation_host_.data(), sizeof(float) * d_ * d_, cudaMemcpyHostToDevice, stream_));
+    launch_transpose_square(m, mt_dev_.ensure(d_ * d_), d_, stream_);
     sync();
     rotation_ready_ = true;
+    if (draws_done_.valid()) draws_done_.wait();
+    draws_.reset();
+    draw_bits_.release();
+    draw_values_.release();
+}
+
+void Engine::ensure_rotation_host() {
+    ensure_rotation();
+    if (!rotation_host_.empty()) return;
+    rotation_host_.resize(d_ * d_);
+    SKM_CUDA(cudaMemcpyAsync(rotation_host_.data(), m_dev_.get(), sizeof(float) * d_ * d_, cudaMemcpyDeviceToHost, stream_));
+    sync();
 }
 
 void Engine::set_rotation(const float* m_host) {
@@ -221,7 +255,7 @@ void Engine::set_rotation(const float* m_host) {
 
 void Engine::get_rotation(float* m_out) {
     Entry entry(device_, stream_);
-    ensure_rotation();
+    ensure_rotation_host();
     std::memcpy(m_out, rotation_host_.data(), sizeof(float) * d_ * d_);
 }
 
@@ -1187,6 +1221,7 @@ void Engine::train_flat(const float* data, size_t n, bool on_device, const float
     }
     n_samples_ = sharded_() ? n : n_samples_global;
     const bool rotate = !cfg_.data_already_rotated;
+    if (rotate || cfg_.unrotate_centroids) start_rotation_draws();
     partial_d_ = initial_partial_d(vertical_d_);
     // The Forgy shuffle runs over all n_samples indices with std::mt19937 (a tenth of a second at 1e7): on a thread of
     // its own, while this one allocates the buffers and starts the rotation.
@@ -1390,6 +1425,7 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
     }
     const size_t n_all = n_samples_;
     const bool rotate = !cfg_.data_already_rotated;
+    if (rotate || cfg_.unrotate_centroids) start_rotation_draws();
     partial_d_ = initial_partial_d(vertical_d_);
     const uint32_t initial_pd = partial_d_;
 
@@ -1715,7 +1751,10 @@ void Engine::assign_training_points(const float* vectors, const float* centroids
             tmp.data_already_rotated = cfg_.data_already_rotated;
             const size_t n_meso = static_cast<size_t>(std::sqrt(n_centroids));
             Engine nested(tmp, n_meso, d_, false, device_);
-            if (!rotation_host_.empty()) nested.set_rotation(rotation_host_.data());
+            if (rotation_ready_) {
+                ensure_rotation_host();
+                nested.set_rotation(rotation_host_.data());
+            }
             std::vector<float> meso_centroids(n_meso * d_);
             nested.train(cent_host.data(), n_centroids, false, nullptr, 0, meso_centroids.data());
             std::vector<uint32_t> meso_assign(n), cent_to_meso(n_centroids);

@@ -7,6 +7,8 @@
 #include <stdexcept>
 #include <string>
 #include <functional>
+#include <future>
+#include <memory>
 #include <vector>
 
 #include "../../include/skm_b200.h"
@@ -144,6 +146,10 @@ void set_prune_split_mode(int mode);
 int prune_split_mode();
 void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, int device, cudaStream_t stream, PhaseTimers* timers = nullptr);
 
+// out (device, d x d) = the matrix make_rotation_matrix computes, from its draws normal_draws(d * d, seed) (device), on `stream`
+// (synchronised once or twice on the way).  False: declined, nothing usable in `out` (rotation_matrix.cu).
+bool make_rotation_matrix_on_device(const float* draws, size_t d, float* out, cudaStream_t stream);
+
 class Engine {
   public:
     Engine(const skm_config& cfg, size_t n_clusters, size_t d, bool hierarchical, int device);
@@ -216,7 +222,9 @@ class Engine {
         float* norms;         // device, full or partial norms of x (rewritten when d' changes)
     };
 
+    void start_rotation_draws();   // the Gaussian draws of a matrix that is still to be made, on a host thread
     void ensure_rotation();
+    void ensure_rotation_host();
     // after_rows(r0, cnt), if given, is called (host side, work enqueued on stream_) whenever rows [r0, r0 + cnt) of dst
     // have been enqueued, in order, in pieces of at least `piece` rows: lets the caller's kernels run between the
     // copies of a host source instead of after them.
@@ -270,7 +278,11 @@ class Engine {
 
     // pruner state
     float epsilon0_;
-    std::vector<float> rotation_host_;  // d x d, empty until needed
+    std::vector<float> rotation_host_;  // d x d, empty until needed (a matrix made on the device is fetched on demand)
+    std::unique_ptr<NormalDraws> draws_;   // of a matrix that is being made
+    std::future<bool> draws_done_;
+    PinnedBuffer<uint32_t> draw_bits_;
+    PinnedBuffer<float> draw_values_;
     bool rotation_ready_ = false;
     DeviceBuffer<float> m_dev_, mt_dev_, ratios_dev_;
     uint32_t vertical_d_ = 0, horizontal_d_ = 0, partial_d_ = 0;
