@@ -75,7 +75,8 @@ constexpr int kTileM = 128;        // points per CTA tile
 constexpr int kTileN = 128;        // centroids per GEMM sub-tile (SIMT path)
 constexpr int kChunk = 1024;       // centroids per pruning chunk (reference VECTOR_CHUNK_SIZE)
 constexpr int kHBlock = 64;        // dimensions per horizontal block (reference H_DIM_SIZE)
-constexpr int kUpdateTile = 1024;  // sorted points per segmented-sum tile
+constexpr int kUpdateTile = 1024;      // sorted points per segmented-sum tile
+constexpr int kUpdateTileSmall = 128;  // ... when there are few points
 
 // ---------------------------------------------------------------------------------------------
 // Launchers (all asynchronous on `stream`; pointers are device pointers unless stated otherwise)
@@ -257,6 +258,7 @@ struct UpdateWorkspace {
     double* block_sums = nullptr;     // reduction partials (>= 1024)
     size_t n_cap = 0, k_cap = 0, d = 0;
 };
+// sizes of digit_table (256 per unit) and tile_partials (2 d per tile) for up to n points
 size_t update_sort_units(size_t n);
 size_t update_tiles(size_t n);
 

@@ -502,22 +502,43 @@ void launch_assign_pruned(const PrunedParams& p, int grid, cudaStream_t stream) 
 // Centroid update: stable LSD radix sort of point ids by assignment, then a segmented row sum in
 // sorted order.  Everything is order-deterministic, so the same input gives bit-identical sums.
 // =================================================================================================
-constexpr int kSortUnit = 2048;  // elements handled by one warp
+// Elements handled by one warp, 32 at a time.  A warp's steps are a chain (each ranks its elements behind those of the
+// steps before), and the digit table has 256 entries per unit: short units while there are fewer than a few warps per SM,
+// long ones above.  At n = 6000 a pass takes 10 us where units of 2048 took 46 us.
+static int sort_unit(size_t n) { return n < (size_t{1} << 17) ? 256 : (n < (size_t{1} << 20) ? 512 : 2048); }
+constexpr int kSortAhead = 8;   // steps whose elements are loaded before the first of them is used
 
-size_t update_sort_units(size_t n) { return (n + kSortUnit - 1) / kSortUnit; }
-size_t update_tiles(size_t n) { return (n + kUpdateTile - 1) / kUpdateTile; }
+// Rows summed by one block of the segmented sum: 1024 where that gives every SM a block, else 128, because a block's rows
+// are a chain of additions (95 us for 1024 rows, whatever the number of blocks; at n = 6000 a sum now takes 8 us).
+static int update_tile_rows(size_t n) { return n >= (size_t{148} << 10) ? kUpdateTile : kUpdateTileSmall; }
 
-__global__ void __launch_bounds__(256) sort_hist_kernel(const uint32_t* __restrict__ keys, size_t n, int shift, uint32_t* __restrict__ table, size_t n_units) {
+static size_t sort_units_of(size_t n) { return (n + sort_unit(n) - 1) / sort_unit(n); }
+static size_t tiles_of(size_t n) { return (n + update_tile_rows(n) - 1) / update_tile_rows(n); }
+
+// A workspace made for n points also serves fewer, and fewer points can need more units and tiles.
+size_t update_sort_units(size_t n) {
+    return std::max({sort_units_of(n), sort_units_of(std::min(n, (size_t{1} << 17) - 1)), sort_units_of(std::min(n, (size_t{1} << 20) - 1))});
+}
+size_t update_tiles(size_t n) { return std::max(tiles_of(n), tiles_of(std::min(n, (size_t{148} << 10) - 1))); }
+
+__global__ void __launch_bounds__(256) sort_hist_kernel(const uint32_t* __restrict__ keys, size_t n, int shift, uint32_t* __restrict__ table, size_t n_units, int unit_size) {
     __shared__ uint32_t h[8][256];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int i = lane; i < 256; i += 32) h[warp][i] = 0;
     __syncwarp();
     const size_t unit = static_cast<size_t>(blockIdx.x) * 8 + warp;
     if (unit < n_units) {
-        const size_t base = unit * kSortUnit;
-        for (int s = 0; s < kSortUnit / 32; ++s) {
-            const size_t idx = base + static_cast<size_t>(s) * 32 + lane;
-            if (idx < n) atomicAdd(&h[warp][(keys[idx] >> shift) & 255u], 1u);
+        const size_t base = unit * unit_size;
+        for (int s0 = 0; s0 < unit_size / 32; s0 += kSortAhead) {
+            uint32_t key[kSortAhead];
+#pragma unroll
+            for (int u = 0; u < kSortAhead; ++u) {
+                const size_t idx = base + static_cast<size_t>(s0 + u) * 32 + lane;
+                key[u] = idx < n ? keys[idx] : 0u;
+            }
+#pragma unroll
+            for (int u = 0; u < kSortAhead; ++u)
+                if (base + static_cast<size_t>(s0 + u) * 32 + lane < n) atomicAdd(&h[warp][(key[u] >> shift) & 255u], 1u);
         }
         __syncwarp();
         for (int i = lane; i < 256; i += 32) table[static_cast<size_t>(i) * n_units + unit] = h[warp][i];
@@ -619,7 +640,7 @@ void exclusive_scan_u32(uint32_t* data, size_t n, uint32_t* totals_tmp, cudaStre
 // Stable scatter: each warp re-reads its unit in order; lanes with equal digits are ranked by lane.
 __global__ void __launch_bounds__(256) sort_scatter_kernel(
     const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, size_t n, int shift,
-    const uint32_t* __restrict__ table, size_t n_units
+    const uint32_t* __restrict__ table, size_t n_units, int unit_size
 ) {
     __shared__ uint32_t base_s[8][256];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -627,25 +648,32 @@ __global__ void __launch_bounds__(256) sort_scatter_kernel(
     if (unit >= n_units) return;
     for (int i = lane; i < 256; i += 32) base_s[warp][i] = table[static_cast<size_t>(i) * n_units + unit];
     __syncwarp();
-    const size_t base = unit * kSortUnit;
+    const size_t base = unit * unit_size;
     const uint32_t lt_mask = (1u << lane) - 1u;
-    for (int s = 0; s < kSortUnit / 32; ++s) {
-        const size_t idx = base + static_cast<size_t>(s) * 32 + lane;
-        const bool valid = idx < n;
-        const uint32_t key = valid ? keys_in[idx] : 0u;
-        const uint32_t val = valid ? (vals_in ? vals_in[idx] : static_cast<uint32_t>(idx)) : 0u;
-        const uint32_t digit = valid ? ((key >> shift) & 255u) : 0xFFFFFFFFu;
-        const uint32_t peers = __match_any_sync(0xffffffffu, digit);
-        const uint32_t rank = __popc(peers & lt_mask);
-        uint32_t pos = 0;
-        if (valid) {
-            pos = base_s[warp][digit] + rank;
-            keys_out[pos] = key;
-            vals_out[pos] = val;
+    for (int s0 = 0; s0 < unit_size / 32; s0 += kSortAhead) {
+        uint32_t keys[kSortAhead], vals[kSortAhead];
+#pragma unroll
+        for (int u = 0; u < kSortAhead; ++u) {
+            const size_t idx = base + static_cast<size_t>(s0 + u) * 32 + lane;
+            const bool valid = idx < n;
+            keys[u] = valid ? keys_in[idx] : 0u;
+            vals[u] = valid ? (vals_in ? vals_in[idx] : static_cast<uint32_t>(idx)) : 0u;
         }
-        __syncwarp();
-        if (valid && rank == 0) base_s[warp][digit] += __popc(peers);
-        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < kSortAhead; ++u) {
+            const bool valid = base + static_cast<size_t>(s0 + u) * 32 + lane < n;
+            const uint32_t digit = valid ? ((keys[u] >> shift) & 255u) : 0xFFFFFFFFu;
+            const uint32_t peers = __match_any_sync(0xffffffffu, digit);
+            const uint32_t rank = __popc(peers & lt_mask);
+            if (valid) {
+                const uint32_t pos = base_s[warp][digit] + rank;
+                keys_out[pos] = keys[u];
+                vals_out[pos] = vals[u];
+            }
+            __syncwarp();
+            if (valid && rank == 0) base_s[warp][digit] += __popc(peers);
+            __syncwarp();
+        }
     }
 }
 
@@ -661,35 +689,30 @@ __global__ void segment_offsets_kernel(const uint32_t* __restrict__ sorted_keys,
     }
 }
 
-__global__ void counts_from_offsets_kernel(const uint32_t* __restrict__ off, size_t k, uint32_t* __restrict__ counts) {
-    const size_t c = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (c < k) counts[c] = off[c + 1] - off[c];
-}
-
-// One CTA sums the rows of kUpdateTile consecutive sorted points for a slab of 1024 columns.  The
+// One CTA sums the rows of TILE consecutive sorted points for a slab of 4 columns per thread.  The
 // first segment of the tile goes to partial slot 2t, the last one (if different) to slot 2t+1, and
 // segments that lie strictly inside the tile are final and go straight to `sums`.
-template <bool VEC>
+template <bool VEC, int TILE>
 __global__ void __launch_bounds__(256) segsum_tile_kernel(
     const float* __restrict__ x, const uint32_t* __restrict__ sorted_keys, const uint32_t* __restrict__ order, size_t n, size_t d, float* __restrict__ sums, float* __restrict__ partials
 ) {
-    __shared__ uint32_t skey[kUpdateTile];
-    __shared__ uint32_t sid[kUpdateTile];
+    __shared__ uint32_t skey[TILE];
+    __shared__ uint32_t sid[TILE];
     const size_t tile = blockIdx.x;
-    const size_t p0 = tile * kUpdateTile;
-    const int cnt = static_cast<int>(min(static_cast<size_t>(kUpdateTile), n - p0));
-    for (int i = threadIdx.x; i < cnt; i += 256) {
+    const size_t p0 = tile * TILE;
+    const int cnt = static_cast<int>(min(static_cast<size_t>(TILE), n - p0));
+    for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
         skey[i] = sorted_keys[p0 + i];
         sid[i] = order[p0 + i];
     }
     __syncthreads();
-    const size_t colbase = static_cast<size_t>(blockIdx.y) * 1024;
+    const size_t colbase = static_cast<size_t>(blockIdx.y) * 4 * blockDim.x;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     size_t col[4];
     bool cv[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-        col[e] = VEC ? (colbase + static_cast<size_t>(threadIdx.x) * 4 + e) : (colbase + threadIdx.x + 256 * e);
+        col[e] = VEC ? (colbase + static_cast<size_t>(threadIdx.x) * 4 + e) : (colbase + threadIdx.x + blockDim.x * e);
         cv[e] = col[e] < d;
     }
     auto flush = [&](uint32_t key, int kind) {
@@ -748,26 +771,27 @@ __global__ void __launch_bounds__(256) segsum_tile_kernel(
 
 // Combines the tile partials of every cluster whose points are not strictly inside one tile, in
 // tile order; empty clusters get zeros.
-template <bool VEC>
-__global__ void __launch_bounds__(256) segsum_fix_kernel(const uint32_t* __restrict__ off, size_t n, size_t d, const float* __restrict__ partials, float* __restrict__ sums) {
+template <bool VEC, int TILE>
+__global__ void __launch_bounds__(256) segsum_fix_kernel(const uint32_t* __restrict__ off, size_t n, size_t d, const float* __restrict__ partials, float* __restrict__ sums, uint32_t* __restrict__ counts) {
     const size_t c = blockIdx.x;
     const size_t s = off[c], e = off[c + 1];
-    const size_t colbase = static_cast<size_t>(blockIdx.y) * 1024;
+    if (blockIdx.y == 0 && threadIdx.x == 0) counts[c] = static_cast<uint32_t>(e - s);
+    const size_t colbase = static_cast<size_t>(blockIdx.y) * 4 * blockDim.x;
     size_t col[4];
     bool cv[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        col[q] = VEC ? (colbase + static_cast<size_t>(threadIdx.x) * 4 + q) : (colbase + threadIdx.x + 256 * q);
+        col[q] = VEC ? (colbase + static_cast<size_t>(threadIdx.x) * 4 + q) : (colbase + threadIdx.x + blockDim.x * q);
         cv[q] = col[q] < d;
     }
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     if (s < e) {
-        const size_t t0 = s / kUpdateTile, t1 = (e - 1) / kUpdateTile;
-        const size_t tile_end = min((t0 + 1) * kUpdateTile, n);
-        const bool direct = (t0 == t1) && (s > t0 * kUpdateTile) && (e < tile_end);
+        const size_t t0 = s / TILE, t1 = (e - 1) / TILE;
+        const size_t tile_end = min((t0 + 1) * TILE, n);
+        const bool direct = (t0 == t1) && (s > t0 * TILE) && (e < tile_end);
         if (direct) return;
         for (size_t t = t0; t <= t1; ++t) {
-            const size_t slot = (s <= t * kUpdateTile) ? (2 * t) : (2 * t + 1);
+            const size_t slot = (s <= t * TILE) ? (2 * t) : (2 * t + 1);
             const float* src = partials + slot * d;
             if (VEC) {
                 if (cv[0]) {
@@ -846,7 +870,7 @@ __global__ void __launch_bounds__(256) reduce_final_kernel(const double* __restr
 
 // Stable LSD radix sort of the indices 0 .. n-1 by key (keys < k): *sorted_keys and *order point into ws.keys_* / ws.vals_*.
 void launch_sort_by_key(const uint32_t* keys, size_t n, size_t k, UpdateWorkspace& ws, const uint32_t** sorted_keys_out, const uint32_t** order_out, cudaStream_t stream) {
-    const size_t n_units = update_sort_units(n);
+    const size_t n_units = sort_units_of(n);
     int bits = 1;
     while ((size_t{1} << bits) < k) ++bits;
     const int passes = (bits + 7) / 8;
@@ -859,10 +883,10 @@ void launch_sort_by_key(const uint32_t* keys, size_t n, size_t k, UpdateWorkspac
     uint32_t* scan_totals = ws.digit_table + 256 * n_units;
     for (int pass = 0; pass < passes; ++pass) {
         const int shift = pass * 8;
-        sort_hist_kernel<<<unit_blocks, 256, 0, stream>>>(kin, n, shift, ws.digit_table, n_units);
+        sort_hist_kernel<<<unit_blocks, 256, 0, stream>>>(kin, n, shift, ws.digit_table, n_units, sort_unit(n));
         SKM_LAUNCH_CHECK();
         exclusive_scan_u32(ws.digit_table, 256 * n_units, scan_totals, stream);
-        sort_scatter_kernel<<<unit_blocks, 256, 0, stream>>>(kin, vin, kout, vout, n, shift, ws.digit_table, n_units);
+        sort_scatter_kernel<<<unit_blocks, 256, 0, stream>>>(kin, vin, kout, vout, n, shift, ws.digit_table, n_units, sort_unit(n));
         SKM_LAUNCH_CHECK();
         kin = kout;
         vin = vout;
@@ -871,6 +895,18 @@ void launch_sort_by_key(const uint32_t* keys, size_t n, size_t k, UpdateWorkspac
     }
     *sorted_keys_out = kin;
     *order_out = vin;
+}
+
+template <bool VEC, int TILE>
+static void launch_segsum(const float* x, const uint32_t* sorted_keys, const uint32_t* order, size_t n, size_t k, size_t d, UpdateWorkspace& ws, float* sums, uint32_t* counts,
+                          cudaStream_t stream) {
+    // four columns per thread, no more warps than the columns need
+    const unsigned threads = static_cast<unsigned>(std::min<size_t>(256, ((d + 3) / 4 + 31) / 32 * 32));
+    const unsigned slabs = static_cast<unsigned>((d + 4 * threads - 1) / (4 * threads));
+    segsum_tile_kernel<VEC, TILE><<<dim3(static_cast<unsigned>(tiles_of(n)), slabs), threads, 0, stream>>>(x, sorted_keys, order, n, d, sums, ws.tile_partials);
+    SKM_LAUNCH_CHECK();
+    segsum_fix_kernel<VEC, TILE><<<dim3(static_cast<unsigned>(k), slabs), threads, 0, stream>>>(ws.seg_offsets, n, d, ws.tile_partials, sums, counts);
+    SKM_LAUNCH_CHECK();
 }
 
 void launch_update(
@@ -883,21 +919,12 @@ void launch_update(
     launch_sort_by_key(assign, n, k, ws, &sorted_keys, &order, stream);
     segment_offsets_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(sorted_keys, n, k, ws.seg_offsets);
     SKM_LAUNCH_CHECK();
-    counts_from_offsets_kernel<<<static_cast<unsigned>((k + 255) / 256), 256, 0, stream>>>(ws.seg_offsets, k, counts);
-    SKM_LAUNCH_CHECK();
-    const size_t n_tiles = update_tiles(n);
-    const unsigned slabs = static_cast<unsigned>((d + 1023) / 1024);
     const bool vec = (d % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
-    if (vec) {
-        segsum_tile_kernel<true><<<dim3(static_cast<unsigned>(n_tiles), slabs), 256, 0, stream>>>(x, sorted_keys, order, n, d, sums, ws.tile_partials);
-        SKM_LAUNCH_CHECK();
-        segsum_fix_kernel<true><<<dim3(static_cast<unsigned>(k), slabs), 256, 0, stream>>>(ws.seg_offsets, n, d, ws.tile_partials, sums);
-    } else {
-        segsum_tile_kernel<false><<<dim3(static_cast<unsigned>(n_tiles), slabs), 256, 0, stream>>>(x, sorted_keys, order, n, d, sums, ws.tile_partials);
-        SKM_LAUNCH_CHECK();
-        segsum_fix_kernel<false><<<dim3(static_cast<unsigned>(k), slabs), 256, 0, stream>>>(ws.seg_offsets, n, d, ws.tile_partials, sums);
-    }
-    SKM_LAUNCH_CHECK();
+    const bool big = update_tile_rows(n) == kUpdateTile;
+    if (vec && big) launch_segsum<true, kUpdateTile>(x, sorted_keys, order, n, k, d, ws, sums, counts, stream);
+    else if (vec) launch_segsum<true, kUpdateTileSmall>(x, sorted_keys, order, n, k, d, ws, sums, counts, stream);
+    else if (big) launch_segsum<false, kUpdateTile>(x, sorted_keys, order, n, k, d, ws, sums, counts, stream);
+    else launch_segsum<false, kUpdateTileSmall>(x, sorted_keys, order, n, k, d, ws, sums, counts, stream);
     if (wcss || not_pruned_total) {
         reduce_stats_kernel<<<kReduceBlocks, 256, 0, stream>>>(dist, not_pruned, n, ws.block_sums);
         SKM_LAUNCH_CHECK();
