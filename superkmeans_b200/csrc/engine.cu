@@ -169,7 +169,7 @@ Engine::Engine(const skm_config& cfg, size_t n_clusters, size_t d, bool hierarch
     copy_stream_ = acquire_stream();
     WorkStream work(stream_);
     ratios_host_ = make_ratios(d, epsilon0_);
-    SKM_CUDA(cudaMemcpy(ratios_dev_.ensure(d + 1), ratios_host_.data(), sizeof(float) * (d + 1), cudaMemcpyHostToDevice));
+    SKM_CUDA(cudaMemcpyAsync(ratios_dev_.ensure(d + 1), ratios_host_.data(), sizeof(float) * (d + 1), cudaMemcpyHostToDevice, stream_));
     scalars_dev_.ensure(8);
     np_total_dev_.ensure(1);
     scalars_host_.ensure(8);
@@ -182,6 +182,7 @@ Engine::Engine(const skm_config& cfg, size_t n_clusters, size_t d, bool hierarch
 
 Engine::~Engine() {
     if (draws_done_.valid()) draws_done_.wait();
+    if (default_stream_work_) cudaEventDestroy(default_stream_work_);
     // the streams are waited for: the buffers released after this are idle
     int prev = device_;
     cudaGetDevice(&prev);
@@ -198,6 +199,14 @@ const std::vector<skm_iter_stats>& Engine::stats(int phase) const {
         case SKM_STATS_REFINE: return stats_refine_;
         default: return stats_flat_;
     }
+}
+
+// Device arrays of a caller are usually written, and their memory was last used, by work on the default stream that nothing
+// waits for before the call; stream_ does not synchronise with that stream by itself.
+void Engine::wait_for_default_stream() {
+    if (!default_stream_work_) SKM_CUDA(cudaEventCreateWithFlags(&default_stream_work_, cudaEventDisableTiming));
+    SKM_CUDA(cudaEventRecord(default_stream_work_, cudaStreamLegacy));
+    SKM_CUDA(cudaStreamWaitEvent(stream_, default_stream_work_, 0));
 }
 
 // -------------------------------------------------------------------------------------------------
@@ -305,38 +314,58 @@ void Engine::allreduce_iteration(float* sums, size_t n_sums, uint32_t* counts, s
     allreduce(scalars, n_scalars, 1);
 }
 
-// dst[n x d] (device) = rotate(src).  Host sources are streamed through two staging buffers so
-// that the copy of chunk i+1 overlaps the rotation of chunk i.
-void Engine::rotate_to_device(const float* src, bool src_on_device, size_t n, float* dst, const std::function<void(size_t, size_t)>& after_rows, size_t piece) {
+// dst[n x d] (device) = the first n rows of src, or rows idx[0 .. n) of it, rotated or as they are.  Host sources are
+// streamed through two device chunks so that the copy of chunk i+1 overlaps the rotation of chunk i; the first chunk is on
+// its way before the rotation matrix is waited for.
+void Engine::load_rows(const float* src, bool src_on_device, const size_t* idx, size_t n, bool rotate, float* dst, const std::function<void(size_t, size_t)>& after_rows,
+                       size_t piece) {
     if (n == 0) return;
-    ensure_rotation();
-    if (src_on_device) {
-        PhaseScope ps(*this, PH_ROTATE);
-        launch_gemm_nt(src, d_, m_dev_.get(), d_, dst, d_, n, d_, d_, stream_);
+    PhaseScope ps(*this, PH_ROTATE);
+    const size_t row_bytes = sizeof(float) * d_;
+    if (src_on_device && !idx) {
+        if (rotate) {
+            ensure_rotation();
+            launch_gemm_nt(src, d_, m_dev_.get(), d_, dst, d_, n, d_, d_, stream_);
+        } else {
+            SKM_CUDA(cudaMemcpyAsync(dst, src, row_bytes * n, cudaMemcpyDeviceToDevice, stream_));
+        }
         return;
     }
-    PhaseScope ps_total(*this, PH_ROTATE);
-    const size_t rows = chunk_rows_for(d_, n);
+    if (src_on_device) {
+        static_assert(sizeof(size_t) == sizeof(uint64_t), "row indices are copied as they are");
+        DeviceBuffer<uint64_t> idx_dev;
+        DeviceBuffer<float> raw;
+        stage_.upload(idx_dev.ensure(n), idx, nullptr, n, sizeof(uint64_t), stream_);
+        if (rotate) ensure_rotation();
+        const size_t rows = chunk_rows_for(d_, n);
+        for (size_t r0 = 0; r0 < n; r0 += rows) {
+            const size_t cnt = std::min(rows, n - r0);
+            launch_gather_rows(src, idx_dev.get() + r0, rotate ? raw.ensure(rows * d_) : dst + r0 * d_, cnt, d_, stream_);
+            if (rotate) launch_gemm_nt(raw.get(), d_, m_dev_.get(), d_, dst + r0 * d_, d_, cnt, d_, d_, stream_);
+        }
+        return;
+    }
+    const size_t rows = streamed_rows(n);
     DeviceBuffer<float> raw[2];
-    raw[0].ensure(rows * d_);
-    if (n > rows) raw[1].ensure(rows * d_);
     cudaEvent_t copied[2], consumed[2];
     for (int i = 0; i < 2; ++i) {
+        if (rotate && (i == 0 || n > rows)) raw[i].ensure(rows * d_);
         SKM_CUDA(cudaEventCreateWithFlags(&copied[i], cudaEventDisableTiming));
         SKM_CUDA(cudaEventCreateWithFlags(&consumed[i], cudaEventDisableTiming));
     }
-    // the staging buffers may still be in use by earlier work that was enqueued on stream_
+    // what the copies write may still be in use by earlier work that was enqueued on stream_
     SKM_CUDA(cudaEventRecord(consumed[0], stream_));
     SKM_CUDA(cudaStreamWaitEvent(copy_stream_, consumed[0], 0));
     size_t ci = 0, handed = 0;
     for (size_t r0 = 0; r0 < n; r0 += rows, ++ci) {
         const int b = static_cast<int>(ci & 1);
         const size_t cnt = std::min(rows, n - r0);
-        if (ci >= 2) SKM_CUDA(cudaStreamWaitEvent(copy_stream_, consumed[b], 0));
-        SKM_CUDA(cudaMemcpyAsync(raw[b].get(), src + r0 * d_, sizeof(float) * cnt * d_, cudaMemcpyHostToDevice, copy_stream_));
+        if (ci >= 2 && rotate) SKM_CUDA(cudaStreamWaitEvent(copy_stream_, consumed[b], 0));
+        stage_.upload(rotate ? raw[b].get() : dst + r0 * d_, idx ? src : src + r0 * d_, idx ? idx + r0 : nullptr, cnt, row_bytes, copy_stream_);
         SKM_CUDA(cudaEventRecord(copied[b], copy_stream_));
+        if (rotate) ensure_rotation();
         SKM_CUDA(cudaStreamWaitEvent(stream_, copied[b], 0));
-        launch_gemm_nt(raw[b].get(), d_, m_dev_.get(), d_, dst + r0 * d_, d_, cnt, d_, d_, stream_);
+        if (rotate) launch_gemm_nt(raw[b].get(), d_, m_dev_.get(), d_, dst + r0 * d_, d_, cnt, d_, d_, stream_);
         SKM_CUDA(cudaEventRecord(consumed[b], stream_));
         const size_t done = r0 + cnt;
         if (after_rows && (done - handed >= piece || done == n)) {
@@ -344,17 +373,17 @@ void Engine::rotate_to_device(const float* src, bool src_on_device, size_t n, fl
             handed = done;
         }
     }
-    sync();
     for (int i = 0; i < 2; ++i) {
         cudaEventDestroy(copied[i]);
         cudaEventDestroy(consumed[i]);
     }
 }
 
-void Engine::upload_rows(const float* src, bool src_on_device, size_t n, float* dst) {
-    if (n == 0) return;
-    SKM_CUDA(cudaMemcpyAsync(dst, src, sizeof(float) * n * d_, src_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, stream_));
-    sync();
+// Rows per chunk of a host matrix of n rows: a quarter of it, so that the kernels run behind the copies, but no less than
+// 8 MB or a row tile per SM, and no more than chunk_rows_for.
+size_t Engine::streamed_rows(size_t n) const {
+    const size_t least = std::max<size_t>((size_t{8} << 20) / (sizeof(float) * d_), static_cast<size_t>(sm_count_of(device_)) * kTileM);
+    return std::min(chunk_rows_for(d_, n), std::max(least, (n + 3) / 4));
 }
 
 void Engine::prepare_update_workspace(size_t n, size_t k) {
@@ -395,13 +424,15 @@ void Engine::generate_centroids_from_host(const float* data, bool on_device, siz
         }
         SKM_CUDA(cudaMemcpyAsync(init_idx_dev_.ensure(k_cur), idx_host, sizeof(uint64_t) * k_cur, cudaMemcpyHostToDevice, stream_));
         launch_gather_rows(data, init_idx_dev_.get(), raw, k_cur, d_, stream_);
+    } else if (!sharded) {
+        stage_.upload(raw, data, idx.data(), k_cur, sizeof(float) * d_, stream_);
     } else {
         float* host = init_rows_host_.ensure(k_cur * d_);
 #pragma omp parallel for
         for (size_t i = 0; i < k_cur; ++i) {
             size_t g = idx[i];
-            const bool mine = !sharded || (g >= shard_row_offset_ && g < shard_row_offset_ + n_local);
-            if (sharded) g -= shard_row_offset_;
+            const bool mine = g >= shard_row_offset_ && g < shard_row_offset_ + n_local;
+            g -= shard_row_offset_;
             if (mine) std::memcpy(host + i * d_, data + g * d_, sizeof(float) * d_);
             else std::memset(host + i * d_, 0, sizeof(float) * d_);
         }
@@ -1189,6 +1220,7 @@ void Engine::train(const float* data, size_t n, bool on_device, const float* que
     if (sharded_() && hierarchical_) {
         throw std::runtime_error("sharded training is available for the flat algorithm only");
     }
+    if (on_device) wait_for_default_stream();
     const double alloc_ms0 = alloc_free_ms();
     timers_.begin(PH_TRAIN_TOTAL, stream_);
     try {
@@ -1201,13 +1233,6 @@ void Engine::train(const float* data, size_t n, bool on_device, const float* que
     timers_.end(stream_);
     sync();
     timers_.add_host(PH_ALLOC_FREE, alloc_free_ms() - alloc_ms0);
-}
-
-// Copies (and rotates unless the data is pre-rotated) the training rows into x_rot_; with sampling
-// the rows are the first n_samples entries of the shuffle (superkmeans.h:1385-1443).
-static void gather_host_rows(const float* data, const size_t* idx, size_t cnt, size_t d, float* out) {
-#pragma omp parallel for
-    for (size_t i = 0; i < cnt; ++i) std::memcpy(out + i * d, data + idx[i] * d, sizeof(float) * d);
 }
 
 void Engine::train_flat(const float* data, size_t n, bool on_device, const float* queries, size_t n_queries, float* centroids_out) {
@@ -1226,6 +1251,8 @@ void Engine::train_flat(const float* data, size_t n, bool on_device, const float
     // The Forgy shuffle runs over all n_samples indices with std::mt19937 (a tenth of a second at 1e7): on a thread of
     // its own, while this one allocates the buffers and starts the rotation.
     std::future<std::vector<size_t>> forgy = std::async(std::launch::async, [n_samples_global, k = k_, seed = cfg_.seed] { return forgy_indices(n_samples_global, k, seed); });
+    std::future<std::vector<size_t>> sampling;
+    if (n_samples_global < n_global) sampling = std::async(std::launch::async, [n, seed = cfg_.seed] { return sampling_permutation(n, seed); });
     bool centroids_ready = false;
     auto make_centroids = [&] {
         if (centroids_ready) return;
@@ -1251,41 +1278,16 @@ void Engine::train_flat(const float* data, size_t n, bool on_device, const float
 
     // GenerateCentroids picks among the first n_samples rows of the caller's data (:221-222).
     if (n_samples_global < n_global) {
-        make_centroids();
-        sampled_indices_ = sampling_permutation(n, cfg_.seed);
-        const size_t rows = chunk_rows_for(d_, n_samples_);
-        if (on_device) {
-            DeviceBuffer<uint64_t> idx_dev;
-            DeviceBuffer<float> raw;
-            idx_dev.ensure(rows);
-            raw.ensure(rows * d_);
-            std::vector<uint64_t> idx64(rows);
-            for (size_t r0 = 0; r0 < n_samples_; r0 += rows) {
-                const size_t cnt = std::min(rows, n_samples_ - r0);
-                for (size_t i = 0; i < cnt; ++i) idx64[i] = sampled_indices_[r0 + i];
-                SKM_CUDA(cudaMemcpyAsync(idx_dev.get(), idx64.data(), sizeof(uint64_t) * cnt, cudaMemcpyHostToDevice, stream_));
-                float* dst = rotate ? raw.get() : x_rot_.get() + r0 * d_;
-                launch_gather_rows(data, idx_dev.get(), dst, cnt, d_, stream_);
-                if (rotate) rotate_to_device(raw.get(), true, cnt, x_rot_.get() + r0 * d_);
-                sync();
-            }
-        } else {
-            std::vector<float> staged(rows * d_);
-            for (size_t r0 = 0; r0 < n_samples_; r0 += rows) {
-                const size_t cnt = std::min(rows, n_samples_ - r0);
-                gather_host_rows(data, sampled_indices_.data() + r0, cnt, d_, staged.data());
-                if (rotate) rotate_to_device(staged.data(), false, cnt, x_rot_.get() + r0 * d_);
-                else upload_rows(staged.data(), false, cnt, x_rot_.get() + r0 * d_);
-            }
-        }
+        sampled_indices_ = sampling.get();
+        load_rows(data, on_device, sampled_indices_.data(), n_samples_, rotate, x_rot_.get());
     } else {
         if (rotate && !on_device) {
             // Host input: the exact assignment of iteration 1 needs nothing but the rotated rows and the initial
             // centroids, so it runs piece by piece between the uploads instead of after the last one.
             uint2* top2 = top2_.ensure(n_samples_);
             float* y_split = y_split_.ensure(2 * k_ * d_);
-            rotate_to_device(
-                data, false, n_samples_, x_rot_.get(),
+            load_rows(
+                data, false, nullptr, n_samples_, true, x_rot_.get(),
                 [&](size_t r0, size_t cnt) {
                     if (!centroids_ready) {
                         make_centroids();
@@ -1297,10 +1299,8 @@ void Engine::train_flat(const float* data, size_t n, bool on_device, const float
                 },
                 static_cast<size_t>(sm_count_of(device_)) * kTileM * 14);   // ~14 waves of row tiles (one per SM) per piece
             first_assign_done_ = true;
-        } else if (rotate) {
-            rotate_to_device(data, on_device, n_samples_, x_rot_.get());
         } else {
-            upload_rows(data, on_device, n_samples_, x_rot_.get());
+            load_rows(data, on_device, nullptr, n_samples_, rotate, x_rot_.get());
         }
     }
     make_centroids();
@@ -1365,10 +1365,8 @@ void Engine::prepare_recall(const float* queries, size_t n_queries, bool rotate)
         SKM_CUDA(cudaMemcpyAsync(idx_dev.ensure(n_queries), idx.data(), sizeof(uint64_t) * n_queries, cudaMemcpyHostToDevice, stream_));
         launch_gather_rows(x_rot_.get(), idx_dev.get(), qr, n_queries, d_, stream_);
         sync();
-    } else if (rotate) {
-        rotate_to_device(queries, false, n_queries, qr);
     } else {
-        upload_rows(queries, false, n_queries, qr);
+        load_rows(queries, false, nullptr, n_queries, rotate, qr);
     }
     launch_row_sqnorms(qr, n_queries, d_, d_, query_norms_.ensure(n_queries), stream_);
     const size_t kmax = std::max(objective_k, centroids_to_explore_);
@@ -1398,17 +1396,15 @@ float Engine::compute_recall(size_t k_cur) {
 // GetOutputCentroids (superkmeans.h:1341-1351)
 void Engine::output_centroids(float* out_host) {
     PhaseScope ps(*this, PH_ROTATE);   // the reference's profiler books Unrotate under "rotator" too
+    const float* c = c_cur_.get();
+    DeviceBuffer<float> tmp;
     if (cfg_.unrotate_centroids) {
         ensure_rotation();
-        DeviceBuffer<float> tmp;
-        tmp.ensure(k_ * d_);
-        launch_gemm_nt(c_cur_.get(), d_, mt_dev_.get(), d_, tmp.get(), d_, k_, d_, d_, stream_);
-        SKM_CUDA(cudaMemcpyAsync(out_host, tmp.get(), sizeof(float) * k_ * d_, cudaMemcpyDeviceToHost, stream_));
-        sync();
-    } else {
-        SKM_CUDA(cudaMemcpyAsync(out_host, c_cur_.get(), sizeof(float) * k_ * d_, cudaMemcpyDeviceToHost, stream_));
-        sync();
+        launch_gemm_nt(c, d_, mt_dev_.get(), d_, tmp.ensure(k_ * d_), d_, k_, d_, d_, stream_);
+        c = tmp.get();
     }
+    stage_.download(out_host, c, sizeof(float) * k_ * d_, stream_);
+    timers_.flush();
 }
 
 // -------------------------------------------------------------------------------------------------
@@ -1452,40 +1448,8 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
 
     // ---- phase 1: mesoclustering (:161-257)
     generate_centroids_from_host(data, on_device, n_all, n_meso_, rotate);
-    if (n_all < n) {
-        sampled_indices_ = sampling_permutation(n, cfg_.seed);
-        const size_t rows = chunk_rows_for(d_, n_all);
-        std::vector<float> staged;
-        DeviceBuffer<uint64_t> idx_dev;
-        DeviceBuffer<float> raw;
-        std::vector<uint64_t> idx64;
-        if (on_device) {
-            idx_dev.ensure(rows);
-            raw.ensure(rows * d_);
-            idx64.resize(rows);
-        } else {
-            staged.resize(rows * d_);
-        }
-        for (size_t r0 = 0; r0 < n_all; r0 += rows) {
-            const size_t cnt = std::min(rows, n_all - r0);
-            if (on_device) {
-                for (size_t i = 0; i < cnt; ++i) idx64[i] = sampled_indices_[r0 + i];
-                SKM_CUDA(cudaMemcpyAsync(idx_dev.get(), idx64.data(), sizeof(uint64_t) * cnt, cudaMemcpyHostToDevice, stream_));
-                float* dst = rotate ? raw.get() : x_rot_.get() + r0 * d_;
-                launch_gather_rows(data, idx_dev.get(), dst, cnt, d_, stream_);
-                if (rotate) rotate_to_device(raw.get(), true, cnt, x_rot_.get() + r0 * d_);
-                sync();
-            } else {
-                gather_host_rows(data, sampled_indices_.data() + r0, cnt, d_, staged.data());
-                if (rotate) rotate_to_device(staged.data(), false, cnt, x_rot_.get() + r0 * d_);
-                else upload_rows(staged.data(), false, cnt, x_rot_.get() + r0 * d_);
-            }
-        }
-    } else {
-        if (rotate) rotate_to_device(data, on_device, n_all, x_rot_.get());
-        else upload_rows(data, on_device, n_all, x_rot_.get());
-    }
-    sync();
+    if (n_all < n) sampled_indices_ = sampling_permutation(n, cfg_.seed);
+    load_rows(data, on_device, n_all < n ? sampled_indices_.data() : nullptr, n_all, rotate, x_rot_.get());
     launch_row_sqnorms(x_rot_.get(), n_all, d_, d_, data_norms_.get(), stream_);
     SKM_CUDA(cudaMemcpyAsync(full_norms_.get(), data_norms_.get(), sizeof(float) * n_all, cudaMemcpyDeviceToDevice, stream_));
 
@@ -1629,10 +1593,11 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
     Entry entry(device_, stream_);
     if (n == 0) return;
     if (n_centroids == 0) throw std::invalid_argument("Value must be positive: n_centroids");
+    if (on_device) wait_for_default_stream();
     DeviceBuffer<float> c_dev_own, cn;
     const float* c_dev = centroids;
     if (!on_device) {
-        SKM_CUDA(cudaMemcpyAsync(c_dev_own.ensure(n_centroids * d_), centroids, sizeof(float) * n_centroids * d_, cudaMemcpyHostToDevice, stream_));
+        stage_.upload(c_dev_own.ensure(n_centroids * d_), centroids, nullptr, n_centroids, sizeof(float) * d_, stream_);
         c_dev = c_dev_own.get();
     }
     launch_row_sqnorms(c_dev, n_centroids, d_, d_, cn.ensure(n_centroids), stream_);
@@ -1651,19 +1616,19 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
         check_tc_error(stream_);
         return;
     }
-    const size_t rows = chunk_rows_for(d_, n);
-    DeviceBuffer<float> xb[2], xn[2], dist[2];
-    DeviceBuffer<uint32_t> knn[2];
+    const size_t rows = streamed_rows(n);
+    DeviceBuffer<float> xb[2], xn, dist;
+    DeviceBuffer<uint32_t> knn;
     cudaEvent_t copied[2], consumed[2];
     for (int i = 0; i < 2; ++i) {
-        xb[i].ensure(rows * d_);
-        xn[i].ensure(rows);
-        dist[i].ensure(rows);
-        knn[i].ensure(rows);
+        if (i == 0 || n > rows) xb[i].ensure(rows * d_);
         SKM_CUDA(cudaEventCreateWithFlags(&copied[i], cudaEventDisableTiming));
         SKM_CUDA(cudaEventCreateWithFlags(&consumed[i], cudaEventDisableTiming));
     }
-    // the staging buffers may still be in use by earlier work that was enqueued on stream_
+    xn.ensure(rows);
+    dist.ensure(rows);
+    knn.ensure(n);
+    // what the copies write may still be in use by earlier work that was enqueued on stream_
     SKM_CUDA(cudaEventRecord(consumed[0], stream_));
     SKM_CUDA(cudaStreamWaitEvent(copy_stream_, consumed[0], 0));
     size_t ci = 0;
@@ -1674,16 +1639,17 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
         const int b = static_cast<int>(ci & 1);
         const size_t cnt = std::min(rows, n - r0);
         if (ci >= 2) SKM_CUDA(cudaStreamWaitEvent(copy_stream_, consumed[b], 0));
-        SKM_CUDA(cudaMemcpyAsync(xb[b].get(), vectors + r0 * d_, sizeof(float) * cnt * d_, cudaMemcpyHostToDevice, copy_stream_));
+        stage_.upload(xb[b].get(), vectors + r0 * d_, nullptr, cnt, sizeof(float) * d_, copy_stream_);
         SKM_CUDA(cudaEventRecord(copied[b], copy_stream_));
         SKM_CUDA(cudaStreamWaitEvent(stream_, copied[b], 0));
-        launch_row_sqnorms(xb[b].get(), cnt, d_, d_, xn[b].get(), stream_);
-        launch_assign_full(xb[b].get(), c_dev, cnt, n_centroids, d_, xn[b].get(), cn.get(), knn[b].get(), dist[b].get(), top2_.ensure(rows), stream_, y_split_.ensure(2 * n_centroids * d_));
-        SKM_CUDA(cudaMemcpyAsync(out + r0, knn[b].get(), sizeof(uint32_t) * cnt, cudaMemcpyDeviceToHost, stream_));
+        launch_row_sqnorms(xb[b].get(), cnt, d_, d_, xn.get(), stream_);
+        launch_assign_full(xb[b].get(), c_dev, cnt, n_centroids, d_, xn.get(), cn.get(), knn.get() + r0, dist.get(), top2_.get(), stream_, y_split_.get());
         SKM_CUDA(cudaEventRecord(consumed[b], stream_));
     }
     timers_.end(stream_);
-    sync();
+    // the answers are a d-th of the rows: fetched once, so that no copy back holds up the next upload
+    stage_.download(out, knn.get(), sizeof(uint32_t) * n, stream_);
+    timers_.flush();
     for (int i = 0; i < 2; ++i) {
         cudaEventDestroy(copied[i]);
         cudaEventDestroy(consumed[i]);
@@ -1705,17 +1671,18 @@ void Engine::assign_training_points(const float* vectors, const float* centroids
         return;
     }
     if (n == 0) return;
+    if (on_device) wait_for_default_stream();
     partial_d_ = initial_partial_d(vertical_d_);
     launch_row_sqnorms(c_cur_.get(), k_, d_, partial_d_, centroid_norms_.get(), stream_);
 
-    // Seeds: one starting centroid per vector.
-    std::vector<uint32_t> seeds(n);
+    // Seeds: one starting centroid per vector.  With all rows trained they are the assignments of Train, which the
+    // search replaces in place; else they are put together on the host.
     const bool store_state = (cfg_.sampling_fraction == 1.0f);
-    if (cfg_.sampling_fraction == 1.0f) {
+    std::vector<uint32_t> seeds;
+    if (store_state) {
         if (n > assignments_.capacity()) throw std::runtime_error("AssignTrainingPoints needs the vectors used in Train()");
-        SKM_CUDA(cudaMemcpyAsync(seeds.data(), assignments_.get(), sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, stream_));
-        sync();
     } else {
+        seeds.resize(n);
         if (sampled_indices_.size() != n) throw std::runtime_error("AssignTrainingPoints needs the vectors used in Train()");
         std::vector<uint32_t> trained_assign(n_samples_);
         SKM_CUDA(cudaMemcpyAsync(trained_assign.data(), assignments_.get(), sizeof(uint32_t) * n_samples_, cudaMemcpyDeviceToHost, stream_));
@@ -1769,51 +1736,52 @@ void Engine::assign_training_points(const float* vectors, const float* centroids
         }
     }
 
+    DeviceBuffer<uint32_t> knn_own, np;
+    DeviceBuffer<float> xr, xn, dist_own;
+    uint32_t* knn = nullptr;
+    float* dist = nullptr;
+    // Device rows have a gigabyte of rotated copy at a time (every chunk costs a few host round trips and a last wave of
+    // row tiles), host rows a chunk of the upload.
+    const size_t rows = on_device ? std::min(n, std::max(chunk_rows_for(d_, n), (size_t{1} << 30) / (sizeof(float) * d_))) : streamed_rows(n);
     if (store_state) {
-        assignments_.ensure(n);
-        distances_.ensure(n);
+        knn = assignments_.get();
+        dist = distances_.ensure(n);
         n_state_rows_ = n;
+    } else {
+        knn = knn_own.ensure(n);
+        stage_.upload(knn, seeds.data(), nullptr, n, sizeof(uint32_t), stream_);
+        dist = dist_own.ensure(rows);
     }
-    const size_t rows = chunk_rows_for(d_, n);
-    DeviceBuffer<float> xr, xn, dist;
-    DeviceBuffer<uint32_t> knn, np;
     xr.ensure(rows * d_);
     xn.ensure(rows);
-    dist.ensure(rows);
-    knn.ensure(rows);
     np.ensure(rows);
     for (size_t r0 = 0; r0 < n; r0 += rows) {
         const size_t cnt = std::min(rows, n - r0);
-        if (cfg_.data_already_rotated) upload_rows(vectors + r0 * d_, on_device, cnt, xr.get());
-        else rotate_to_device(vectors + r0 * d_, on_device, cnt, xr.get());
+        load_rows(vectors + r0 * d_, on_device, nullptr, cnt, !cfg_.data_already_rotated, xr.get());
         launch_row_sqnorms(xr.get(), cnt, d_, partial_d_, xn.get(), stream_);
-        SKM_CUDA(cudaMemcpyAsync(knn.get(), seeds.data() + r0, sizeof(uint32_t) * cnt, cudaMemcpyHostToDevice, stream_));
-        run_pruned_pass(xr.get(), cnt, k_, c_cur_.get(), xn.get(), centroid_norms_.get(), knn.get(), dist.get(), np.get());
-        SKM_CUDA(cudaMemcpyAsync(out + r0, knn.get(), sizeof(uint32_t) * cnt, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, stream_));
-        if (store_state) {
-            SKM_CUDA(cudaMemcpyAsync(assignments_.get() + r0, knn.get(), sizeof(uint32_t) * cnt, cudaMemcpyDeviceToDevice, stream_));
-            SKM_CUDA(cudaMemcpyAsync(distances_.get() + r0, dist.get(), sizeof(float) * cnt, cudaMemcpyDeviceToDevice, stream_));
-        }
-        sync();
+        run_pruned_pass(xr.get(), cnt, k_, c_cur_.get(), xn.get(), centroid_norms_.get(), knn + r0, store_state ? dist + r0 : dist, np.get());
     }
+    if (on_device) SKM_CUDA(cudaMemcpyAsync(out, knn, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, stream_));
+    else stage_.download(out, knn, sizeof(uint32_t) * n, stream_);
+    sync();
 }
 
 void Engine::get_assignments(uint32_t* out, size_t n) {
     Entry entry(device_, stream_);
     if (n > n_state_rows_ || n > assignments_.capacity()) throw std::invalid_argument("more assignments requested than the engine holds");
-    SKM_CUDA(cudaMemcpy(out, assignments_.get(), sizeof(uint32_t) * n, cudaMemcpyDeviceToHost));
+    stage_.download(out, assignments_.get(), sizeof(uint32_t) * n, stream_);
 }
 
 void Engine::get_distances(float* out, size_t n) {
     Entry entry(device_, stream_);
     if (n > n_state_rows_ || n > distances_.capacity()) throw std::invalid_argument("more distances requested than the engine holds");
-    SKM_CUDA(cudaMemcpy(out, distances_.get(), sizeof(float) * n, cudaMemcpyDeviceToHost));
+    stage_.download(out, distances_.get(), sizeof(float) * n, stream_);
 }
 
 void Engine::get_rotated_centroids(float* out) {
     Entry entry(device_, stream_);
     if (!trained_) throw std::runtime_error("the model has not been trained");
-    SKM_CUDA(cudaMemcpy(out, c_cur_.get(), sizeof(float) * k_ * d_, cudaMemcpyDeviceToHost));
+    stage_.download(out, c_cur_.get(), sizeof(float) * k_ * d_, stream_);
 }
 
 // -------------------------------------------------------------------------------------------------

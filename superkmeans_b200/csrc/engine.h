@@ -14,47 +14,11 @@
 #include "../../include/skm_b200.h"
 #include "common.cuh"
 #include "comm_nccl.h"
+#include "engine_buffers.h"
+#include "host_copy.h"
 #include "host_logic.h"
 
 namespace skmb {
-
-// A typed array in memory that ALLOC / FREE hand out.
-template <class T, MemoryBlock (*ALLOC)(size_t), void (*FREE)(const MemoryBlock&)>
-class Buffer {
-  public:
-    Buffer() = default;
-    Buffer(const Buffer&) = delete;
-    Buffer& operator=(const Buffer&) = delete;
-    ~Buffer() { release(); }
-    void release() {
-        FREE(m_);
-        m_ = MemoryBlock{};
-        cap_ = 0;
-    }
-    // Grows (never shrinks) to at least `count` elements; contents are not preserved on growth.
-    T* ensure(size_t count) {
-        if (count > cap_ || !m_.p) {
-            release();
-            m_ = ALLOC(sizeof(T) * (count ? count : 1));
-            cap_ = count;
-        }
-        return get();
-    }
-    T* get() const { return static_cast<T*>(m_.p); }
-    size_t capacity() const { return cap_; }
-    void swap(Buffer& o) {
-        std::swap(m_, o.m_);
-        std::swap(cap_, o.cap_);
-    }
-
-  private:
-    MemoryBlock m_;
-    size_t cap_ = 0;
-};
-template <class T>
-using DeviceBuffer = Buffer<T, device_alloc, device_free>;
-template <class T>
-using PinnedBuffer = Buffer<T, pinned_alloc, pinned_free>;
 
 // Accumulating per-phase device timers (CUDA events on the engine's stream); names follow the
 // sections of the reference's profiler (profiler.h): rotator, norms_calc, search/1st_blas, search,
@@ -228,9 +192,10 @@ class Engine {
     // after_rows(r0, cnt), if given, is called (host side, work enqueued on stream_) whenever rows [r0, r0 + cnt) of dst
     // have been enqueued, in order, in pieces of at least `piece` rows: lets the caller's kernels run between the
     // copies of a host source instead of after them.
-    void rotate_to_device(const float* src, bool src_on_device, size_t n, float* dst, const std::function<void(size_t, size_t)>& after_rows = nullptr,
-                          size_t piece = 0);
-    void upload_rows(const float* src, bool src_on_device, size_t n, float* dst);
+    void load_rows(const float* src, bool src_on_device, const size_t* idx, size_t n, bool rotate, float* dst,
+                   const std::function<void(size_t, size_t)>& after_rows = nullptr, size_t piece = 0);
+    void wait_for_default_stream();
+    size_t streamed_rows(size_t n) const;
     void prepare_update_workspace(size_t n, size_t k);
     void run_iteration(bool gemm_only, const IterationInput& in, size_t iter_idx, bool is_first, std::vector<skm_iter_stats>& target);
     void run_pruned_pass(const float* x, size_t n, size_t k_cur, const float* y, const float* norms_x, const float* norms_y, uint32_t* knn, float* dist, uint32_t* not_pruned);
@@ -265,6 +230,8 @@ class Engine {
     int device_;
     cudaStream_t stream_ = nullptr;
     cudaStream_t copy_stream_ = nullptr;
+    HostStage stage_;
+    cudaEvent_t default_stream_work_ = nullptr;
 
     // sharding
     size_t shard_n_global_ = 0, shard_row_offset_ = 0;

@@ -1,0 +1,102 @@
+// See host_copy.h.
+#include "host_copy.h"
+
+#include <cstring>
+
+namespace skmb {
+
+namespace {
+
+bool is_pinned(const void* p) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeManaged;
+}
+
+// A thread per quarter of a megabyte, eight at most: more do not copy faster.
+int threads_for(size_t bytes) { return static_cast<int>(std::max<size_t>(1, std::min<size_t>(8, bytes >> 18))); }
+
+void copy_bytes(char* dst, const char* src, size_t bytes) {
+    const int threads = threads_for(bytes);
+    if (threads == 1) {
+        std::memcpy(dst, src, bytes);
+        return;
+    }
+#pragma omp parallel for num_threads(threads) schedule(static)
+    for (int t = 0; t < threads; ++t) {
+        const size_t b = bytes * t / threads, e = bytes * (t + 1) / threads;
+        std::memcpy(dst + b, src + b, e - b);
+    }
+}
+
+void gather_rows(char* dst, const char* src, const size_t* idx, size_t n, size_t row_bytes) {
+    const int threads = threads_for(n * row_bytes);
+#pragma omp parallel for num_threads(threads) schedule(static) if (threads > 1)
+    for (size_t i = 0; i < n; ++i) std::memcpy(dst + i * row_bytes, src + idx[i] * row_bytes, row_bytes);
+}
+
+} // namespace
+
+HostStage::~HostStage() {
+    for (cudaEvent_t e : copied_)
+        if (e) cudaEventDestroy(e);
+}
+
+// Piece i, free for the host, at least `bytes` long.
+char* HostStage::piece(int i, size_t bytes) {
+    if (!copied_[i]) SKM_CUDA(cudaEventCreateWithFlags(&copied_[i], cudaEventDisableTiming));
+    else SKM_CUDA(cudaEventSynchronize(copied_[i]));
+    return pieces_[i].ensure(bytes);
+}
+
+void HostStage::upload(void* dst, const void* src, const size_t* idx, size_t n, size_t row_bytes, cudaStream_t stream) {
+    if (n == 0 || row_bytes == 0) return;
+    if (!idx && is_pinned(src)) {
+        SKM_CUDA(cudaMemcpyAsync(dst, src, n * row_bytes, cudaMemcpyHostToDevice, stream));
+        return;
+    }
+    const size_t per_piece = std::max<size_t>(1, kPieceBytes / row_bytes);
+    for (size_t r0 = 0; r0 < n; r0 += per_piece) {
+        const size_t cnt = std::min(per_piece, n - r0);
+        const int i = next_;
+        next_ = (next_ + 1) % kPieces;
+        char* p = piece(i, cnt * row_bytes);
+        if (idx) gather_rows(p, static_cast<const char*>(src), idx + r0, cnt, row_bytes);
+        else copy_bytes(p, static_cast<const char*>(src) + r0 * row_bytes, cnt * row_bytes);
+        SKM_CUDA(cudaMemcpyAsync(static_cast<char*>(dst) + r0 * row_bytes, p, cnt * row_bytes, cudaMemcpyHostToDevice, stream));
+        SKM_CUDA(cudaEventRecord(copied_[i], stream));
+    }
+}
+
+void HostStage::download(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
+    if (bytes == 0) return;
+    if (is_pinned(dst)) {
+        SKM_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream));
+        SKM_CUDA(cudaStreamSynchronize(stream));
+        return;
+    }
+    const size_t n = (bytes + kPieceBytes - 1) / kPieceBytes;
+    int slot[kPieces];
+    auto enqueue = [&](size_t q) {
+        const size_t b = q * kPieceBytes, cnt = std::min(kPieceBytes, bytes - b);
+        const int i = next_;
+        next_ = (next_ + 1) % kPieces;
+        slot[q % kPieces] = i;
+        SKM_CUDA(cudaMemcpyAsync(piece(i, cnt), static_cast<const char*>(src) + b, cnt, cudaMemcpyDeviceToHost, stream));
+        SKM_CUDA(cudaEventRecord(copied_[i], stream));
+    };
+    // one piece less than the ring in flight: the one being emptied must not be reused
+    size_t sent = 0;
+    for (size_t q = 0; q < n; ++q) {
+        for (; sent < n && sent < q + kPieces - 1; ++sent) enqueue(sent);
+        const int i = slot[q % kPieces];
+        SKM_CUDA(cudaEventSynchronize(copied_[i]));
+        const size_t b = q * kPieceBytes;
+        copy_bytes(static_cast<char*>(dst) + b, pieces_[i].get(), std::min(kPieceBytes, bytes - b));
+    }
+}
+
+} // namespace skmb
