@@ -286,7 +286,7 @@ skm_status skm_op_pdxify(int device, const float* in, uint64_t n, uint64_t d, fl
  * the default stream).  The call returns after the outputs are written (it synchronises that stream).
  *
  * The intermediate data (norms, candidate pairs, a status word) live in one fixed array in the library's
- * device image, about 3.3 MiB, which every GPU that loads the library holds until the process exits.  Hence:
+ * device image, about 3.4 MiB, which every GPU that loads the library holds until the process exits.  Hence:
  *   - n <= SKM_NOALLOC_MAX_ROWS and k <= SKM_NOALLOC_MAX_CENTROIDS, else SKM_INVALID_ARGUMENT (split a
  *     larger batch of rows into several calls); d is not limited;
  *   - every call uses the same array: calls whose kernels can overlap on one GPU (two streams, two

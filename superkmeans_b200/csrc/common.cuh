@@ -102,6 +102,20 @@ void launch_transpose_square(const float* in, float* out, size_t n, cudaStream_t
 // y_split (2 * k * d floats, optional): scratch in which the tensor-core path keeps the centroids split into tf32 parts.
 void launch_assign_full(const float* x, const float* y, size_t n, size_t k, size_t d, const float* norms_x, const float* norms_y, uint32_t* out_knn, float* out_dist, uint2* top2_scratch, cudaStream_t stream, float* y_split = nullptr);
 
+// Exact assignment in fp32 without tensor cores, for few pairs (direct_assign.cu): knn and (if not null) dist; norms_x and
+// norms_y are filled unless n <= 8.  `arrived` must be zero before the first use and is zero after each.
+struct DirectScratch {
+    float* norms_x;             // n
+    float* norms_y;             // k
+    unsigned long long* keys;   // direct_key_count(n)
+    uint32_t* counters;         // direct_counter_count(n)
+    uint32_t* arrived;          // 1
+};
+size_t direct_key_count(size_t n);
+size_t direct_counter_count(size_t n);
+double direct_assign_seconds(size_t n, size_t k, size_t d);   // what it takes, roughly
+void launch_direct_assign(const float* x, const float* y, size_t n, size_t k, size_t d, const DirectScratch& s, uint32_t* knn, float* dist, cudaStream_t stream);
+
 struct PrunedParams {
     const float* x;             // n x d rotated points
     const float* y;             // k x d rotated centroids, row-major

@@ -386,6 +386,24 @@ size_t Engine::streamed_rows(size_t n) const {
     return std::min(chunk_rows_for(d_, n), std::max(least, (n + 3) / 4));
 }
 
+// Exact assignment of device rows: knn, dist, and the full norms of both sides.
+void Engine::exact_assignment(const float* x, size_t n, const float* c, size_t k, float* norms_x, bool norms_known, float* norms_c, uint32_t* knn, float* dist) {
+    const AssignRoute route = assign_route(n, k, d_);
+    if (route == AssignRoute::filter) {
+        exact_.begin(c, k, d_, n, norms_c, stream_);
+        exact_.rows(x, 0, n, norms_x, knn, dist, stream_);
+        exact_.settle_on_device(x, knn, dist, stream_);
+        return;
+    }
+    if (route == AssignRoute::direct) {
+        direct_.run(x, c, n, k, d_, norms_x, norms_c, knn, dist, stream_);
+        return;
+    }
+    launch_row_sqnorms(c, k, d_, d_, norms_c, stream_);
+    if (!norms_known) launch_row_sqnorms(x, n, d_, d_, norms_x, stream_);
+    launch_assign_full(x, c, n, k, d_, norms_x, norms_c, knn, dist, top2_.ensure(n), stream_, y_split_.ensure(2 * k * d_));
+}
+
 void Engine::prepare_update_workspace(size_t n, size_t k) {
     const size_t units = update_sort_units(n);
     const size_t tiles = update_tiles(n);
@@ -1096,13 +1114,13 @@ void Engine::run_iteration(bool gemm_only, const IterationInput& in, size_t iter
     const size_t n = in.n_samples, k_cur = in.n_clusters;
     float* norms = in.norms;
     if (gemm_only) {
-        launch_row_sqnorms(c_prev_.get(), k_cur, d_, d_, centroid_norms_.get(), stream_);
         PhaseScope ps(*this, PH_ASSIGN_FULL);
         if (is_first && first_assign_done_) {
             first_assign_done_ = false;   // done during the upload (train_flat)
+            if (exact_open_) exact_.settle_on_device(in.x, assignments_.get(), distances_.get(), stream_);
+            exact_open_ = false;
         } else {
-            launch_assign_full(in.x, c_prev_.get(), n, k_cur, d_, norms, centroid_norms_.get(), assignments_.get(), distances_.get(), top2_.ensure(n), stream_,
-                               y_split_.ensure(2 * k_cur * d_));
+            exact_assignment(in.x, n, c_prev_.get(), k_cur, norms, true, centroid_norms_.get(), assignments_.get(), distances_.get());
         }
     } else {
         launch_row_sqnorms(c_prev_.get(), k_cur, d_, partial_d_, centroid_norms_.get(), stream_);
@@ -1239,6 +1257,7 @@ void Engine::train_flat(const float* data, size_t n, bool on_device, const float
     stats_flat_.clear();
     n_queries_ = 0;
     first_assign_done_ = false;
+    exact_open_ = false;
     const size_t n_global = sharded_() ? shard_n_global_ : n;
     const size_t n_samples_global = n_vectors_to_sample(n_global, k_, cfg_.sampling_fraction, cfg_.max_points_per_cluster, false);
     if (n_samples_global < k_) {
@@ -1284,18 +1303,24 @@ void Engine::train_flat(const float* data, size_t n, bool on_device, const float
         if (rotate && !on_device) {
             // Host input: the exact assignment of iteration 1 needs nothing but the rotated rows and the initial
             // centroids, so it runs piece by piece between the uploads instead of after the last one.
-            uint2* top2 = top2_.ensure(n_samples_);
-            float* y_split = y_split_.ensure(2 * k_ * d_);
+            exact_open_ = assign_route(n_samples_, k_, d_) == AssignRoute::filter;
             load_rows(
                 data, false, nullptr, n_samples_, true, x_rot_.get(),
                 [&](size_t r0, size_t cnt) {
+                    const float* x = x_rot_.get() + r0 * d_;
+                    float* norms = data_norms_.get() + r0;
                     if (!centroids_ready) {
                         make_centroids();
-                        launch_row_sqnorms(c_prev_.get(), k_, d_, d_, centroid_norms_.get(), stream_);
+                        if (exact_open_) exact_.begin(c_prev_.get(), k_, d_, n_samples_, centroid_norms_.get(), stream_);
+                        else launch_row_sqnorms(c_prev_.get(), k_, d_, d_, centroid_norms_.get(), stream_);
                     }
-                    launch_row_sqnorms(x_rot_.get() + r0 * d_, cnt, d_, d_, data_norms_.get() + r0, stream_);
-                    launch_assign_full(x_rot_.get() + r0 * d_, c_prev_.get(), cnt, k_, d_, data_norms_.get() + r0, centroid_norms_.get(), assignments_.get() + r0,
-                                       distances_.get() + r0, top2 + r0, stream_, y_split);
+                    if (exact_open_) {
+                        exact_.rows(x, r0, cnt, norms, assignments_.get() + r0, distances_.get() + r0, stream_);
+                    } else {
+                        launch_row_sqnorms(x, cnt, d_, d_, norms, stream_);
+                        launch_assign_full(x, c_prev_.get(), cnt, k_, d_, norms, centroid_norms_.get(), assignments_.get() + r0, distances_.get() + r0, top2_.ensure(n_samples_) + r0,
+                                           stream_, y_split_.ensure(2 * k_ * d_));
+                    }
                 },
                 static_cast<size_t>(sm_count_of(device_)) * kTileM * 14);   // ~14 waves of row tiles (one per SM) per piece
             first_assign_done_ = true;
@@ -1600,22 +1625,21 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
         stage_.upload(c_dev_own.ensure(n_centroids * d_), centroids, nullptr, n_centroids, sizeof(float) * d_, stream_);
         c_dev = c_dev_own.get();
     }
-    launch_row_sqnorms(c_dev, n_centroids, d_, d_, cn.ensure(n_centroids), stream_);
+    cn.ensure(n_centroids);
     if (on_device) {
         DeviceBuffer<float> xn, dist;
-        xn.ensure(n);
-        dist.ensure(n);
-        top2_.ensure(n);
-        y_split_.ensure(2 * n_centroids * d_);
         {
             PhaseScope ps(*this, PH_ASSIGN_FULL);
-            launch_row_sqnorms(vectors, n, d_, d_, xn.get(), stream_);
-            launch_assign_full(vectors, c_dev, n, n_centroids, d_, xn.get(), cn.get(), out, dist.get(), top2_.get(), stream_, y_split_.get());
+            exact_assignment(vectors, n, c_dev, n_centroids, xn.ensure(n), false, cn.get(), out, dist.ensure(n));
         }
         sync();
-        check_tc_error(stream_);
+        if (assign_route(n, n_centroids, d_) != AssignRoute::direct) check_tc_error(stream_);   // (a direct call waits for nothing that can run out)
         return;
     }
+    const AssignRoute route = assign_route(n, n_centroids, d_);
+    const bool filtered = route == AssignRoute::filter, direct = route == AssignRoute::direct;
+    if (filtered) exact_.begin(c_dev, n_centroids, d_, n, cn.get(), stream_);
+    else if (!direct) launch_row_sqnorms(c_dev, n_centroids, d_, d_, cn.get(), stream_);
     const size_t rows = streamed_rows(n);
     DeviceBuffer<float> xb[2], xn, dist;
     DeviceBuffer<uint32_t> knn;
@@ -1632,8 +1656,6 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
     SKM_CUDA(cudaEventRecord(consumed[0], stream_));
     SKM_CUDA(cudaStreamWaitEvent(copy_stream_, consumed[0], 0));
     size_t ci = 0;
-    top2_.ensure(rows);
-    y_split_.ensure(2 * n_centroids * d_);
     timers_.begin(PH_ASSIGN_FULL, stream_);
     for (size_t r0 = 0; r0 < n; r0 += rows, ++ci) {
         const int b = static_cast<int>(ci & 1);
@@ -1642,9 +1664,28 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
         stage_.upload(xb[b].get(), vectors + r0 * d_, nullptr, cnt, sizeof(float) * d_, copy_stream_);
         SKM_CUDA(cudaEventRecord(copied[b], copy_stream_));
         SKM_CUDA(cudaStreamWaitEvent(stream_, copied[b], 0));
-        launch_row_sqnorms(xb[b].get(), cnt, d_, d_, xn.get(), stream_);
-        launch_assign_full(xb[b].get(), c_dev, cnt, n_centroids, d_, xn.get(), cn.get(), knn.get() + r0, dist.get(), top2_.get(), stream_, y_split_.get());
+        if (filtered) {
+            exact_.rows(xb[b].get(), r0, cnt, xn.get(), knn.get() + r0, dist.get(), stream_);
+        } else if (direct) {
+            direct_.run(xb[b].get(), c_dev, cnt, n_centroids, d_, xn.get(), cn.get(), knn.get() + r0, dist.get(), stream_);
+        } else {
+            launch_row_sqnorms(xb[b].get(), cnt, d_, d_, xn.get(), stream_);
+            launch_assign_full(xb[b].get(), c_dev, cnt, n_centroids, d_, xn.get(), cn.get(), knn.get() + r0, dist.get(), top2_.ensure(rows), stream_,
+                               y_split_.ensure(2 * n_centroids * d_));
+        }
         SKM_CUDA(cudaEventRecord(consumed[b], stream_));
+    }
+    if (filtered) {
+        // rows that the filter could not settle cross once more
+        const size_t listed = exact_.settle(stream_), per = exact_.slice_rows();
+        std::vector<uint32_t> idx32(listed);
+        stage_.download(idx32.data(), exact_.listed(), sizeof(uint32_t) * listed, stream_);
+        const std::vector<size_t> idx(idx32.begin(), idx32.end());
+        for (size_t at = 0; at < listed; at += per) {
+            const size_t cnt = std::min(per, listed - at);
+            stage_.upload(xb[0].ensure(cnt * d_), vectors, idx.data() + at, cnt, sizeof(float) * d_, stream_);
+            exact_.finish(xb[0].get(), at, cnt, knn.get(), nullptr, stream_);
+        }
     }
     timers_.end(stream_);
     // the answers are a d-th of the rows: fetched once, so that no copy back holds up the next upload
@@ -1654,7 +1695,7 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
         cudaEventDestroy(copied[i]);
         cudaEventDestroy(consumed[i]);
     }
-    check_tc_error(stream_);
+    if (!direct) check_tc_error(stream_);
 }
 
 // -------------------------------------------------------------------------------------------------
@@ -1831,11 +1872,22 @@ void Engine::op_find_nearest(int device, const float* x, const float* y, size_t 
     DeviceBuffer<uint32_t> knn;
     ctx.upload(xd, x, n * d);
     ctx.upload(yd, y, k * d);
-    launch_row_sqnorms(xd.get(), n, d, d, nx.ensure(n), ctx.stream);
-    launch_row_sqnorms(yd.get(), k, d, d, ny.ensure(k), ctx.stream);
     DeviceBuffer<uint2> top2;
     DeviceBuffer<float> ysplit;
-    launch_assign_full(xd.get(), yd.get(), n, k, d, nx.get(), ny.get(), knn.ensure(n), dist.ensure(n), top2.ensure(n), ctx.stream, ysplit.ensure(2 * k * d));
+    ExactAssign exact;
+    DirectAssign direct;
+    const AssignRoute route = assign_route(n, k, d);
+    if (route == AssignRoute::filter) {
+        exact.begin(yd.get(), k, d, n, ny.ensure(k), ctx.stream);
+        exact.rows(xd.get(), 0, n, nx.ensure(n), knn.ensure(n), dist.ensure(n), ctx.stream);
+        exact.settle_on_device(xd.get(), knn.get(), dist.get(), ctx.stream);
+    } else if (route == AssignRoute::direct) {
+        direct.run(xd.get(), yd.get(), n, k, d, nx.ensure(n), ny.ensure(k), knn.ensure(n), dist.ensure(n), ctx.stream);
+    } else {
+        launch_row_sqnorms(xd.get(), n, d, d, nx.ensure(n), ctx.stream);
+        launch_row_sqnorms(yd.get(), k, d, d, ny.ensure(k), ctx.stream);
+        launch_assign_full(xd.get(), yd.get(), n, k, d, nx.get(), ny.get(), knn.ensure(n), dist.ensure(n), top2.ensure(n), ctx.stream, ysplit.ensure(2 * k * d));
+    }
     ctx.download(out_knn, knn.get(), n);
     ctx.download(out_dist, dist.get(), n);
     ctx.sync();

@@ -15,6 +15,7 @@
 #include "common.cuh"
 #include "comm_nccl.h"
 #include "engine_buffers.h"
+#include "exact_assign.h"
 #include "host_copy.h"
 #include "host_logic.h"
 
@@ -195,6 +196,7 @@ class Engine {
     void load_rows(const float* src, bool src_on_device, const size_t* idx, size_t n, bool rotate, float* dst,
                    const std::function<void(size_t, size_t)>& after_rows = nullptr, size_t piece = 0);
     void wait_for_default_stream();
+    void exact_assignment(const float* x, size_t n, const float* c, size_t k, float* norms_x, bool norms_known, float* norms_c, uint32_t* knn, float* dist);
     size_t streamed_rows(size_t n) const;
     void prepare_update_workspace(size_t n, size_t k);
     void run_iteration(bool gemm_only, const IterationInput& in, size_t iter_idx, bool is_first, std::vector<skm_iter_stats>& target);
@@ -274,6 +276,9 @@ class Engine {
     DeviceBuffer<float> distances_;
     PrunePassBuffers prune_bufs_;
     std::vector<float> ratios_host_;
+    ExactAssign exact_;
+    DirectAssign direct_;
+    bool exact_open_ = false;            // rows of the first assignment wait to be settled (see train_flat)
     DeviceBuffer<uint2> top2_;           // candidate pairs of the tensor-core exact assignment
     DeviceBuffer<float> y_split_;        // centroids split into tf32 hi / lo parts for the tensor-core kernels
     // training with query vectors (recall after every iteration)

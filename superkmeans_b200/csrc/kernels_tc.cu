@@ -1117,16 +1117,21 @@ EncodeTiledFn encode_fn() {
 
 // Row-major fp32 matrix [rows][ld] of which the first `extent` columns are visible; boxes of 16
 // columns x box_rows rows, 64-byte swizzle, zero fill outside.
-CUtensorMap make_tmap(const float* base, size_t extent, size_t rows, size_t ld, uint32_t box_rows) {
+CUtensorMap make_tmap_of(CUtensorMapDataType type, size_t element, CUtensorMapSwizzle swizzle, const void* base, size_t extent, size_t rows, size_t ld, uint32_t box_cols,
+                         uint32_t box_rows) {
     CUtensorMap m;
     const cuuint64_t dims[2] = {extent, rows};
-    const cuuint64_t strides[1] = {ld * sizeof(float)};
-    const cuuint32_t box[2] = {static_cast<cuuint32_t>(BK), box_rows};
+    const cuuint64_t strides[1] = {ld * element};
+    const cuuint32_t box[2] = {box_cols, box_rows};
     const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                   CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const CUresult r = encode_fn()(&m, type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) throw CudaError("cuTensorMapEncodeTiled failed with code " + std::to_string(static_cast<int>(r)));
     return m;
+}
+
+CUtensorMap make_tmap(const float* base, size_t extent, size_t rows, size_t ld, uint32_t box_rows) {
+    return make_tmap_of(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, sizeof(float), CU_TENSOR_MAP_SWIZZLE_64B, base, extent, rows, ld, BK, box_rows);
 }
 
 // Splits y (rows x ld, 16-byte aligned, ld % 4 == 0) into y_split[0 .. rows*ld) = hi and y_split[rows*ld ..) = lo.
@@ -1182,7 +1187,13 @@ void set_debug_wait_injection(long long wait_limit_cycles, uint32_t producer_sto
     g_debug_producer_stop = producer_stops_after_kblocks;
 }
 
+bool wait_injected() { return g_debug_producer_stop != 0; }
+
 void launch_presplit(const float* y, size_t rows, size_t ld, float* y_split, cudaStream_t stream) { presplit(y, rows, ld, y_split, stream); }
+
+CUtensorMap make_half_tmap(const void* base, size_t cols, size_t rows, uint32_t box_rows) {
+    return make_tmap_of(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, CU_TENSOR_MAP_SWIZZLE_128B, base, cols, rows, cols, 64, box_rows);
+}
 
 CUtensorMap make_row_major_tmap(const float* base, size_t extent, size_t rows, size_t ld, uint32_t box_rows) { return make_tmap(base, extent, rows, ld, box_rows); }
 

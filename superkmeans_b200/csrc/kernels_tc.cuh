@@ -101,6 +101,7 @@ long long wait_limit();
 // assignment kernel stops after producer_stops_after_kblocks k-blocks (0 = never), so that the other roles wait
 // for tiles that never arrive.  The kernel then returns with an error code that fetch_error reports.
 void set_debug_wait_injection(long long wait_limit_cycles, uint32_t producer_stops_after_kblocks);
+bool wait_injected();   // a stop is set: only the kernels of launch_assign_full honour it
 
 // The per-device word (device memory) in which a tensor-core kernel records that one of its waits ran out; kernels that
 // consume such a kernel's output read it first and do nothing when it is set.

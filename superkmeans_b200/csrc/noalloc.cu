@@ -36,7 +36,9 @@ struct Scratch {
     uint2 pairs[kMaxRows];          // two best candidates per row (tensor-core pass -> fp32 refinement)
     float row_norms[kMaxRows];      // squared norms of the rows
     float centroid_norms[kMaxCentroids];
+    uint32_t counters[kMaxRows / 64];   // row tiles of the direct kernel
     int status;                     // set by a kernel whose bounded wait ran out; must be 0 on entry
+    uint32_t arrived;               // blocks of the direct kernel; must be 0 on entry
 };
 
 // In host code this name is only a handle for the runtime's symbol calls, never an address to hand to a kernel.
@@ -89,14 +91,25 @@ void find_nearest(int device, const float* x_dev, const float* y_dev, size_t n, 
 
     DeviceScope scope(device);
     Scratch* s = scratch_of_current_device(device);
-    SKM_CUDA(cudaMemsetAsync(&s->status, 0, sizeof(int), stream));
-    launch_row_sqnorms(x_dev, n, d, d, s->row_norms, stream);
-    launch_row_sqnorms(y_dev, k, d, d, s->centroid_norms, stream);
-    if (tc::eligible(x_dev, d, y_dev, d)) {
-        tc::launch_assign_full_flagged(x_dev, y_dev, n, k, d, s->row_norms, s->centroid_norms, out_knn_dev, out_dist_dev, s->pairs, &s->status, stream);
+    SKM_CUDA(cudaMemsetAsync(&s->status, 0, sizeof(s->status) + sizeof(s->arrived), stream));
+    // (the filter needs fp16 copies of both sides, which there is no room for here)
+    if (tc::enabled() && direct_assign_seconds(n, k, d) < 3e-4) {
+        DirectScratch scratch;
+        scratch.norms_x = s->row_norms;
+        scratch.norms_y = s->centroid_norms;
+        scratch.keys = reinterpret_cast<unsigned long long*>(s->pairs);
+        scratch.counters = s->counters;
+        scratch.arrived = &s->arrived;
+        launch_direct_assign(x_dev, y_dev, n, k, d, scratch, out_knn_dev, out_dist_dev, stream);
     } else {
-        // Rows that TMA cannot address (pitch or base not a multiple of 16 bytes): fp32 SIMT kernel, which needs the norms only.
-        launch_assign_full(x_dev, y_dev, n, k, d, s->row_norms, s->centroid_norms, out_knn_dev, out_dist_dev, nullptr, stream);
+        launch_row_sqnorms(x_dev, n, d, d, s->row_norms, stream);
+        launch_row_sqnorms(y_dev, k, d, d, s->centroid_norms, stream);
+        if (tc::eligible(x_dev, d, y_dev, d)) {
+            tc::launch_assign_full_flagged(x_dev, y_dev, n, k, d, s->row_norms, s->centroid_norms, out_knn_dev, out_dist_dev, s->pairs, &s->status, stream);
+        } else {
+            // Rows that TMA cannot address (pitch or base not a multiple of 16 bytes): fp32 SIMT kernel, which needs the norms only.
+            launch_assign_full(x_dev, y_dev, n, k, d, s->row_norms, s->centroid_norms, out_knn_dev, out_dist_dev, nullptr, stream);
+        }
     }
     int status = 0;
     SKM_CUDA(cudaMemcpyAsync(&status, &s->status, sizeof(int), cudaMemcpyDeviceToHost, stream));
