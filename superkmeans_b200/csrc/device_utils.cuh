@@ -24,4 +24,35 @@ __device__ __forceinline__ float ordered_to_float(uint32_t o) {
     return __uint_as_float(b);
 }
 
+// One row operation of a split (host_logic.h, SplitOp) for dimension j.
+template <class Op>
+__device__ __forceinline__ void apply_split_op(float* __restrict__ c, size_t d, size_t j, const Op op) {
+    const float up = 1.0f + (1.0f / 1024.0f), down = 1.0f - (1.0f / 1024.0f);
+    float* pd = c + static_cast<size_t>(op.dst) * d + j;
+    float* ps = c + static_cast<size_t>(op.src) * d + j;
+    if (op.kind == 0) {
+        const float v = *ps;
+        if ((j & 1) == 0) {
+            *pd = __fmul_rn(v, up);
+            *ps = __fmul_rn(v, down);
+        } else {
+            *pd = __fmul_rn(v, down);
+            *ps = __fmul_rn(v, up);
+        }
+    } else {
+        float val = __fmul_rn(op.wc, *pd);
+        val = __fadd_rn(val, *ps);
+        *pd = __fdiv_rn(val, __fadd_rn(op.wc, 1.0f));
+    }
+}
+
+// Unit length, by one warp.
+__device__ __forceinline__ void normalize_row(float* __restrict__ p, size_t d, int lane) {
+    float s = 0.f;
+    for (size_t j = lane; j < d; j += 32) s = fmaf(p[j], p[j], s);
+    s = warp_sum(s);
+    const float inv = 1.0f / sqrtf(s);
+    for (size_t j = lane; j < d; j += 32) p[j] *= inv;
+}
+
 } // namespace skmb

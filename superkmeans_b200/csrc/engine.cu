@@ -1204,13 +1204,17 @@ void Engine::run_iteration(bool gemm_only, const IterationInput& in, size_t iter
     s.not_pruned_pct = gemm_only ? -1.0f : avg_not_pruned;
     s.partial_d = gemm_only ? 0u : old_partial_d;
     target.push_back(s);
-    if (cfg_.verbose) {
-        std::cout << "Iteration " << iter_idx + 1 << " | Objective: " << cost_ << " | Shift: " << shift_ << " | Split: " << n_split_ << " | Recall: " << recall_;
-        if (gemm_only) std::cout << " [GEMM-only]";
-        else std::cout << " | Not Pruned %: " << avg_not_pruned * 100.0f << " | d': " << old_partial_d << " -> " << partial_d_;
-        std::cout << std::endl;
-    }
+    if (cfg_.verbose) print_iteration(s, partial_d_);
 }
+
+void Engine::print_iteration(const skm_iter_stats& s, uint32_t next_partial_d) const {
+    std::cout << "Iteration " << s.iteration << " | Objective: " << s.objective << " | Shift: " << s.shift << " | Split: " << s.split << " | Recall: " << s.recall;
+    if (s.is_gemm_only) std::cout << " [GEMM-only]";
+    else std::cout << " | Not Pruned %: " << s.not_pruned_pct * 100.0f << " | d': " << s.partial_d << " -> " << next_partial_d;
+    std::cout << std::endl;
+}
+
+void Engine::check_tensor_cores() { check_tc_error(stream_); }
 
 // -------------------------------------------------------------------------------------------------
 // Train
@@ -1525,16 +1529,18 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
 
     // ---- phase 2: fine clustering, one mesocluster after the other (:301-425)
     const std::vector<size_t> fine_nums = arrange_fine_clusters(k_, n_meso_, n_all, meso_sizes);
-    const size_t max_meso = *std::max_element(meso_sizes.begin(), meso_sizes.end());
-    meso_buffer_.ensure(std::max<size_t>(max_meso, 1) * d_);
-    meso_norms_.ensure(std::max<size_t>(max_meso, 1));
+    std::vector<size_t> rows_of(n_meso_);   // members whose index the partition holds
+    for (size_t m = 0; m < n_meso_; ++m) rows_of[m] = std::min<size_t>(meso_sizes[m], n_all - std::min(offsets[m], n_all));
+    auto gemm_only = [&](size_t n_fine) { return d_ < kDimensionThresholdForPruning || cfg_.use_blas_only || n_fine <= kNClustersThresholdForPruning; };
+    // Mesoclusters that never prune share their launches (train_fine_run); snapshots are per mesocluster and iteration.
+    auto shares = [&](size_t m) { return fine_nums[m] > 0 && rows_of[m] >= fine_nums[m] && gemm_only(fine_nums[m]) && !trace_on_ && tc::enabled() && d_ <= 16384; };
+    const size_t run_rows = (size_t{4} << 30) / (sizeof(float) * d_);   // of a run, unless one mesocluster has more
     // The Forgy rows of every mesocluster (a shuffle of its member positions each) are drawn ahead by a host thread.
-    auto meso_rows = [&](size_t m) { return std::min<size_t>(meso_sizes[m], n_all - std::min(offsets[m], n_all)); };
     std::vector<std::vector<size_t>> forgy(n_meso_);
     std::atomic<size_t> forgy_done{0};
     std::thread forgy_thread([&, seed = cfg_.seed] {
         for (size_t m = 0; m < n_meso_; ++m) {
-            if (fine_nums[m] != 0) forgy[m] = forgy_indices(meso_rows(m), fine_nums[m], seed);
+            if (fine_nums[m] != 0) forgy[m] = forgy_indices(rows_of[m], fine_nums[m], seed);
             forgy_done.store(m + 1, std::memory_order_release);
         }
     });
@@ -1548,9 +1554,25 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
     for (size_t m = 0; m < n_meso_; ++m) {
         const size_t n_fine = fine_nums[m];
         if (n_fine == 0) continue;
+        if (shares(m)) {
+            size_t last = m, run = 0, clusters = 0;
+            while (last < n_meso_ && shares(last) && (run == 0 || run + rows_of[last] <= run_rows)) {
+                run += rows_of[last];
+                clusters += fine_nums[last];
+                ++last;
+            }
+            while (forgy_done.load(std::memory_order_acquire) < last) std::this_thread::yield();
+            partial_d_ = initial_pd;
+            train_fine_run(m, last, offsets, rows_of, fine_nums, forgy, fine_offset);
+            fine_offset += clusters;
+            m = last - 1;
+            continue;
+        }
         partial_d_ = initial_pd;
-        const size_t msize = meso_rows(m);
+        const size_t msize = rows_of[m];
         n_samples_ = msize;
+        meso_buffer_.ensure(std::max<size_t>(msize, 1) * d_);
+        meso_norms_.ensure(std::max<size_t>(msize, 1));
         if (msize < n_fine) {
             throw std::runtime_error("a mesocluster holds fewer points than the fine clusters allotted to it");
         }
@@ -1560,7 +1582,7 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
         while (forgy_done.load(std::memory_order_acquire) <= m) std::this_thread::yield();
         generate_centroids_from_device_rows(meso_buffer_.get(), msize, n_fine, &forgy[m]);
 
-        const bool always_gemm_only = d_ < kDimensionThresholdForPruning || cfg_.use_blas_only || n_fine <= kNClustersThresholdForPruning;
+        const bool always_gemm_only = gemm_only(n_fine);
         bool partial_norms_computed = false;
         IterationInput in{meso_buffer_.get(), msize, msize, n_fine, meso_norms_.get()};
         for (size_t iter = 0; iter < cfg_.iters_fineclustering; ++iter) {

@@ -210,6 +210,10 @@ class Engine {
     void prepare_recall(const float* queries, size_t n_queries, bool rotate);
     float compute_recall(size_t k_cur);
     void train_hierarchical(const float* data, size_t n, bool on_device, float* centroids_out);
+    void train_fine_run(size_t first, size_t last, const std::vector<size_t>& offsets, const std::vector<size_t>& rows, const std::vector<size_t>& fine,
+                        const std::vector<std::vector<size_t>>& forgy, size_t fine_offset);
+    void print_iteration(const skm_iter_stats& s, uint32_t next_partial_d) const;
+    void check_tensor_cores();
     void output_centroids(float* out_host);
     void allreduce(void* buf, size_t count, int dtype);
     void allreduce_iteration(float* sums, size_t n_sums, uint32_t* counts, size_t n_counts, double* scalars, size_t n_scalars);

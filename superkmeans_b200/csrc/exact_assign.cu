@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(64) sample_mean_kernel(const float* __restrict
     if (blockIdx.x == 0 && threadIdx.x == 0) *n_listed = 0u;
     const size_t j = static_cast<size_t>(blockIdx.x) * 64 + threadIdx.x;
     if (j >= d) return;
-    float s = 0.f;
+    float s = 0.f;   // (d = 0: the mean stays what it is)
 #pragma unroll
     for (int q = 0; q < kMeanSamples; ++q) s += __ldg(y + (static_cast<size_t>(q) * k / kMeanSamples) * d + j);
     mean[j] = s * (1.0f / kMeanSamples);
@@ -133,11 +133,10 @@ __global__ void __launch_bounds__(256) centroid_fp16_kernel(const float* __restr
     if (lane == 0) stat_max(stats, kResidual, err);
 }
 
-// Per row: fp16 copy, norm, and for the filter {factor from accumulator to -2 x.c, width of the window above the smallest
-// filtered distance in which the true nearest centroid lies (infinite: the row is not filtered)}.
+// Per row: fp16 copy, norm, and {squared norm minus the mean, squared norm of the rounding error, squared norm, scale}.
 template <bool VEC>
-__global__ void __launch_bounds__(256) row_fp16_kernel(const float* __restrict__ x, size_t n, size_t d, size_t dp, const float* __restrict__ mean, const uint32_t* __restrict__ stats,
-                                                       float* __restrict__ norms, __half* __restrict__ out, float2* __restrict__ info) {
+__global__ void __launch_bounds__(256) row_fp16_kernel(const float* __restrict__ x, size_t n, size_t d, size_t dp, const float* __restrict__ mean, float* __restrict__ norms,
+                                                       __half* __restrict__ out, float4* __restrict__ info) {
     const size_t row = static_cast<size_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
     if (row >= n) return;
     const int lane = threadIdx.x & 31;
@@ -147,17 +146,23 @@ __global__ void __launch_bounds__(256) row_fp16_kernel(const float* __restrict__
     const float err = write_fp16_row<VEC>(xr, mean, d, dp, scale, out + row * dp, lane);
     if (lane != 0) return;
     norms[row] = nx.plain;
-    const float c2 = __uint_as_float(stats[kCentredNorm]), e2 = __uint_as_float(stats[kResidual]), p2 = __uint_as_float(stats[kPlainNorm]);
-    const bool usable = nx.plain < kLargest && p2 < kLargest && nx.centred < kLargest && c2 < kLargest && (nx.centred == 0.f || nx.centred > kSmallest) && (c2 == 0.f || c2 > kSmallest);
+    info[row] = make_float4(nx.centred, err, nx.plain, scale);
+}
+
+// For the filter: {factor from accumulator to -2 x.c, width of the window above the smallest filtered distance in which the
+// true nearest centroid lies (infinite: the row is not filtered)}.
+__device__ __forceinline__ float2 filter_terms(const float4 r, const uint32_t* __restrict__ stats, uint32_t k_blocks) {
+    const float c2 = __uint_as_float(__ldg(stats + kCentredNorm)), e2 = __uint_as_float(__ldg(stats + kResidual)), p2 = __uint_as_float(__ldg(stats + kPlainNorm));
+    const bool usable = r.z < kLargest && p2 < kLargest && r.x < kLargest && c2 < kLargest && (r.x == 0.f || r.x > kSmallest) && (c2 == 0.f || c2 > kSmallest);
     // |x.c - x^.c^| <= |x - x^| |c| + |x^| |c - c^|, plus a truncation of at most 2^-22 of the running sum for each 16-wide
     // product added (counted twice); the norms are rounded up
-    const float xn = sqrtf(nx.centred) * 1.0001f, xe = sqrtf(err) * 1.001f, cn = sqrtf(c2) * 1.0001f, ce = sqrtf(e2) * 1.001f;
-    const float trunc = (static_cast<float>(dp / 16) + 16.0f) * 4.8e-7f;
+    const float xn = sqrtf(r.x) * 1.0001f, xe = sqrtf(r.y) * 1.001f, cn = sqrtf(c2) * 1.0001f, ce = sqrtf(e2) * 1.001f;
+    const float trunc = (static_cast<float>(k_blocks * 4) + 16.0f) * 4.8e-7f;
     const float bound = xe * cn + (xn + xe) * ce + trunc * (xn + xe) * (cn + ce);
     // twice the distance's error on both sides; pairs that the decision treats as near-ties (1e-4 of the distance), and
     // the rounding of the fp32 distances it compares
-    const float window = 4.0f * bound + 2e-4f * (nx.centred + c2) + 4e-6f * (nx.plain + p2);
-    info[row] = make_float2(-2.0f / (scale * fp16_scale(c2)), usable ? window : INFINITY);
+    const float window = 4.0f * bound + 2e-4f * (r.x + c2) + 4e-6f * (r.z + p2);
+    return make_float2(-2.0f / (r.w * fp16_scale(c2)), usable ? window : INFINITY);
 }
 
 // -------------------------------------------------------------------------------------------------
@@ -196,9 +201,12 @@ static_assert(sizeof(FilterCtrl) <= F_CTRL_BYTES, "control block too large");
 struct FilterParams {
     size_t n;              // rows of this launch
     size_t first;          // index of its first row inside the batch
-    uint32_t col_tiles;    // of 256 centroids
+    uint32_t k;
     uint32_t k_blocks;     // of 64 columns
-    const float2* info;
+    const AssignTile* tiles;   // grouped: what every row tile is assigned to
+    size_t n_tiles;
+    const float4* info;
+    const uint32_t* stats;
     const float* norms_y;  // centred, padded to whole tiles
     uint4* cand;
     uint32_t* listed;
@@ -228,6 +236,7 @@ struct Best {
     }
 };
 
+template <bool GROUPED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(F_THREADS, 1)
     filter_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_y, const FilterParams p) {
     extern __shared__ uint8_t smem_raw[];
@@ -262,7 +271,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(F_THREADS, 1)
     tc_fence_after();
     const uint32_t tmem_base = ctrl->tmem_base;
 
-    const size_t n_row_tiles = (p.n + 255) / 256;
+    const size_t n_row_tiles = GROUPED ? p.n_tiles : (p.n + 255) / 256;
+    auto tile_at = [&](size_t rt) -> AssignTile {
+        if (GROUPED) return p.tiles[rt];
+        return {static_cast<uint32_t>(rt * 256), static_cast<uint32_t>(min(p.n - rt * 256, size_t{256})), 0u, p.k};
+    };
     const size_t pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
 
     if (warp == 0) {
@@ -270,9 +283,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(F_THREADS, 1)
             uint32_t kbt = 0;
             bool ok = true;
             for (size_t rt = pair; rt < n_row_tiles && ok; rt += n_pairs) {
-                const int x_row = static_cast<int>(rt * 256 + rank * 128);
-                for (uint32_t nt = 0; nt < p.col_tiles && ok; ++nt) {
-                    const int y_row = static_cast<int>(nt * 256 + rank * 128);
+                const AssignTile tile = tile_at(rt);
+                const uint32_t col_tiles = (tile.k + 255) / 256;
+                const int x_row = static_cast<int>(tile.row0 + rank * 128);
+                for (uint32_t nt = 0; nt < col_tiles && ok; ++nt) {
+                    const int y_row = static_cast<int>(tile.y0 + nt * 256 + rank * 128);
                     for (uint32_t kb = 0; kb < p.k_blocks; ++kb, ++kbt) {
                         const uint32_t s = kbt % F_STAGES, ph = (kbt / F_STAGES) & 1u;
                         if (!mbar_wait(&ctrl->empty[s], ph ^ 1u, wctx, 41)) {
@@ -300,7 +315,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(F_THREADS, 1)
             uint32_t kbt = 0, t = 0;
             bool ok = true;
             for (size_t rt = pair; rt < n_row_tiles && ok; rt += n_pairs) {
-                for (uint32_t nt = 0; nt < p.col_tiles && ok; ++nt, ++t) {
+                const uint32_t col_tiles = (tile_at(rt).k + 255) / 256;
+                for (uint32_t nt = 0; nt < col_tiles && ok; ++nt, ++t) {
                     const uint32_t b = t & 1u, tph = (t >> 1) & 1u;
                     if (!mbar_wait(&ctrl->acc_empty[b], tph ^ 1u, wctx, 42)) {
                         ok = false;
@@ -331,16 +347,27 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(F_THREADS, 1)
         uint32_t t = 0, row_tiles = 0;
         bool ok = true;
         for (size_t rt = pair; rt < n_row_tiles && ok; rt += n_pairs, ++row_tiles) {
-            const size_t row = rt * 256 + rank * 128 + lane_base + lane;
-            const bool valid = row < p.n;
-            const float2 info = valid ? p.info[row] : make_float2(0.f, 0.f);
+            const AssignTile tile = tile_at(rt);
+            const uint32_t col_tiles = (tile.k + 255) / 256;
+            const size_t row = static_cast<size_t>(tile.row0) + rank * 128 + lane_base + lane;
+            const bool valid = rank * 128 + lane_base + lane < tile.rows;
+            const float2 info = valid ? filter_terms(p.info[row], p.stats, p.k_blocks) : make_float2(0.f, 0.f);
             Best best;
             float limit = FLT_MAX;   // values from here on change nothing
-            for (uint32_t nt = 0; nt < p.col_tiles && ok; ++nt, ++t) {
+            for (uint32_t nt = 0; nt < col_tiles && ok; ++nt, ++t) {
                 const uint32_t b = t & 1u, tph = (t >> 1) & 1u;
                 float* ny = ctrl->ny[quarter][b];
                 // the two warps of a quarter fill (and read) their own halves
-                *reinterpret_cast<float4*>(ny + half * 128 + lane * 4) = __ldg(reinterpret_cast<const float4*>(p.norms_y + static_cast<size_t>(nt) * 256 + half * 128 + lane * 4));
+                if (GROUPED) {
+                    // (the columns behind the group's are another group's centroids)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const uint32_t c = nt * 256 + half * 128 + q * 32 + lane;
+                        ny[half * 128 + q * 32 + lane] = c < tile.k ? __ldg(p.norms_y + tile.y0 + c) : FLT_MAX;
+                    }
+                } else {
+                    *reinterpret_cast<float4*>(ny + half * 128 + lane * 4) = __ldg(reinterpret_cast<const float4*>(p.norms_y + static_cast<size_t>(nt) * 256 + half * 128 + lane * 4));
+                }
                 __syncwarp();
                 if (!__all_sync(0xffffffffu, mbar_wait(&ctrl->acc_full[b], tph, wctx, 44))) {
                     ok = false;
@@ -375,7 +402,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(F_THREADS, 1)
                         hits &= hits - 1;
                         const float v = ctrl->column[warp - 2][j][lane];
                         if (v < limit) {
-                            best.insert(v, nt * 256 + ch * 32 + j);
+                            best.insert(v, tile.y0 + nt * 256 + ch * 32 + j);
                             limit = fminf(best.v5, best.v1 + info.y);
                         }
                     }
@@ -527,6 +554,44 @@ __global__ void __launch_bounds__(256) gather_listed_rows_kernel(const float* __
     for (size_t j = threadIdx.x & 31; j < d; j += 32) out[i * d + j] = __ldg(src + j);
 }
 
+// The listed rows of a grouped pass: a warp computes the fp32 distances of a row to all centroids of its group.
+__global__ void __launch_bounds__(256) decide_listed_kernel(const float* __restrict__ x, const float* __restrict__ y, size_t d, const float* __restrict__ norms_x,
+                                                            const float* __restrict__ norms_y, const AssignTile* __restrict__ tiles, size_t n_tiles,
+                                                            const uint32_t* __restrict__ listed, const uint32_t* __restrict__ n_listed, uint32_t* __restrict__ out_knn,
+                                                            float* __restrict__ out_dist, const int* __restrict__ error) {
+    if (*reinterpret_cast<const volatile int*>(error) != 0) return;
+    const int lane = threadIdx.x & 31;
+    const uint32_t n = *n_listed;
+    for (uint32_t i = blockIdx.x * 8 + (threadIdx.x >> 5); i < n; i += gridDim.x * 8) {
+        const uint32_t row = listed[i];
+        size_t lo = 0, hi = n_tiles;   // the last tile that begins at or before the row
+        while (hi - lo > 1) {
+            const size_t mid = (lo + hi) / 2;
+            if (tiles[mid].row0 <= row) lo = mid;
+            else hi = mid;
+        }
+        const AssignTile tile = tiles[lo];
+        const float* xr = x + static_cast<size_t>(row) * d;
+        const float nx = norms_x[row];
+        float best = FLT_MAX;
+        uint32_t index = tile.y0;
+        for (uint32_t c = tile.y0; c < tile.y0 + tile.k; ++c) {
+            const float* yr = y + static_cast<size_t>(c) * d;
+            float s = 0.f;
+            for (size_t j = lane; j < d; j += 32) s = fmaf(__ldg(xr + j), __ldg(yr + j), s);
+            const float e = fmaf(-2.0f, warp_sum(s), nx) + norms_y[c];
+            if (e < best) {
+                best = e;
+                index = c;
+            }
+        }
+        if (lane == 0) {
+            out_knn[row] = index;
+            out_dist[row] = fmaxf(0.0f, best);
+        }
+    }
+}
+
 bool aligned16(const float* p, size_t d) { return d % 4 == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 unsigned warps_grid(size_t rows) { return static_cast<unsigned>((rows + 7) / 8); }
 
@@ -559,72 +624,107 @@ void DirectAssign::run(const float* x, const float* y, size_t n, size_t k, size_
     launch_direct_assign(x, y, n, k, d, s, knn, dist, stream);
 }
 
-void ExactAssign::begin(const float* y, size_t k, size_t d, size_t batch_rows, float* norms_y, cudaStream_t stream) {
-    listed_.ensure(batch_rows);
+void ExactAssign::centroids(const float* y, size_t k, float* norms_y, bool with_mean, cudaStream_t stream) {
     y_ = y;
     norms_y_ = norms_y;
     k_ = k;
-    d_ = d;
-    dp_ = (d + 7) / 8 * 8;
     kp_ = (k + 255) / 256 * 256;
     float* mean = mean_.ensure(dp_);
     float* centred = centred_norms_.ensure(kp_);
-    uint32_t* stats = reinterpret_cast<uint32_t*>(stats_.ensure(kStats));
+    uint32_t* stats = stats_.ensure(kStats);
     __half* yh = yh_.ensure(k * dp_);
-    sample_mean_kernel<<<static_cast<unsigned>((d + 63) / 64), 64, 0, stream>>>(y, k, d, mean, stats, n_listed_.ensure(1));
+    sample_mean_kernel<<<with_mean ? static_cast<unsigned>((d_ + 63) / 64) : 1u, 64, 0, stream>>>(y, k, with_mean ? d_ : 0, mean, stats, n_listed_.ensure(1));
     SKM_LAUNCH_CHECK();
-    if (aligned16(y, d)) {
-        centroid_norms_kernel<true><<<warps_grid(kp_), 256, 0, stream>>>(y, k, kp_, d, mean, norms_y, centred, stats);
+    if (aligned16(y, d_)) {
+        centroid_norms_kernel<true><<<warps_grid(kp_), 256, 0, stream>>>(y, k, kp_, d_, mean, norms_y, centred, stats);
         SKM_LAUNCH_CHECK();
-        centroid_fp16_kernel<true><<<warps_grid(k), 256, 0, stream>>>(y, k, d, dp_, mean, stats, yh);
+        centroid_fp16_kernel<true><<<warps_grid(k), 256, 0, stream>>>(y, k, d_, dp_, mean, stats, yh);
     } else {
-        centroid_norms_kernel<false><<<warps_grid(kp_), 256, 0, stream>>>(y, k, kp_, d, mean, norms_y, centred, stats);
+        centroid_norms_kernel<false><<<warps_grid(kp_), 256, 0, stream>>>(y, k, kp_, d_, mean, norms_y, centred, stats);
         SKM_LAUNCH_CHECK();
-        centroid_fp16_kernel<false><<<warps_grid(k), 256, 0, stream>>>(y, k, d, dp_, mean, stats, yh);
+        centroid_fp16_kernel<false><<<warps_grid(k), 256, 0, stream>>>(y, k, d_, dp_, mean, stats, yh);
     }
     SKM_LAUNCH_CHECK();
 }
 
-void ExactAssign::rows(const float* x, size_t first, size_t n, float* norms_x, uint32_t* out_knn, float* out_dist, cudaStream_t stream) {
-    if (n == 0) return;
+void ExactAssign::convert(const float* x, size_t n, float* norms_x, cudaStream_t stream) {
+    __half* xh = xh_.get();
+    if (aligned16(x, d_)) row_fp16_kernel<true><<<warps_grid(n), 256, 0, stream>>>(x, n, d_, dp_, mean_.get(), norms_x, xh, row_info_.get());
+    else row_fp16_kernel<false><<<warps_grid(n), 256, 0, stream>>>(x, n, d_, dp_, mean_.get(), norms_x, xh, row_info_.get());
+    SKM_LAUNCH_CHECK();
+}
+
+// Filter and decision of the n converted rows x.
+void ExactAssign::search(const float* x, size_t first, size_t n, const AssignTile* tiles, size_t n_tiles, const float* norms_x, uint32_t* out_knn, float* out_dist,
+                         cudaStream_t stream) {
     int device = 0, sms = 0;
     SKM_CUDA(cudaGetDevice(&device));
     SKM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    const size_t pairs = static_cast<size_t>(sms / 2);
-    // a gigabyte of fp16 rows at a time, in whole waves of row tiles
-    const size_t wave = pairs * 256;
-    const size_t per = std::min(n, std::max(wave, ((size_t{1} << 30) / (dp_ * sizeof(__half))) / wave * wave));
-    const CUtensorMap ty = make_half_tmap(yh_.get(), dp_, k_, 128);
-    const bool vec = aligned16(x, d_) && aligned16(y_, d_);
-    const uint32_t* stats = reinterpret_cast<const uint32_t*>(stats_.get());
-    SKM_CUDA(cudaFuncSetAttribute(filter_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(F_SMEM_BYTES)));
     FilterParams p{};
-    p.col_tiles = static_cast<uint32_t>(kp_ / 256);
+    p.n = n;
+    p.first = first;
+    p.k = static_cast<uint32_t>(k_);
     p.k_blocks = static_cast<uint32_t>((dp_ + FK - 1) / FK);
-    p.info = row_info_.ensure(per);
+    p.tiles = tiles;
+    p.n_tiles = tiles ? n_tiles : (n + 255) / 256;
+    p.info = row_info_.get();
+    p.stats = stats_.get();
     p.norms_y = centred_norms_.get();
-    p.cand = cand_.ensure(per);
+    p.cand = cand_.ensure(n);
     p.listed = listed_.get();
     p.n_listed = n_listed_.get();
     p.error = error_word();
     p.wait_limit = wait_limit();
-    __half* xh = xh_.ensure(per * dp_);
+    const CUtensorMap tx = make_half_tmap(xh_.get(), dp_, n, 128), ty = make_half_tmap(yh_.get(), dp_, k_, 128);
+    const unsigned grid = static_cast<unsigned>(2 * std::min<size_t>(static_cast<size_t>(sms / 2), p.n_tiles));
+    auto* kernel = tiles ? filter_tc_kernel<true> : filter_tc_kernel<false>;
+    SKM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(F_SMEM_BYTES)));
+    kernel<<<grid, F_THREADS, F_SMEM_BYTES, stream>>>(tx, ty, p);
+    SKM_LAUNCH_CHECK();
+    if (aligned16(x, d_) && aligned16(y_, d_)) decide_kernel<true><<<warps_grid(n), 256, 0, stream>>>(x, y_, n, k_, d_, norms_x, norms_y_, cand_.get(), out_knn, out_dist, p.error);
+    else decide_kernel<false><<<warps_grid(n), 256, 0, stream>>>(x, y_, n, k_, d_, norms_x, norms_y_, cand_.get(), out_knn, out_dist, p.error);
+    SKM_LAUNCH_CHECK();
+}
+
+void ExactAssign::begin(const float* y, size_t k, size_t d, size_t batch_rows, float* norms_y, cudaStream_t stream) {
+    listed_.ensure(batch_rows);
+    d_ = d;
+    dp_ = (d + 7) / 8 * 8;
+    centroids(y, k, norms_y, true, stream);
+}
+
+void ExactAssign::rows(const float* x, size_t first, size_t n, float* norms_x, uint32_t* out_knn, float* out_dist, cudaStream_t stream) {
+    // a gigabyte of fp16 rows at a time, in whole waves of row tiles
+    const size_t wave = 74 * 256;
+    const size_t per = std::min(n, std::max(wave, ((size_t{1} << 30) / (dp_ * sizeof(__half))) / wave * wave));
+    xh_.ensure(per * dp_);
+    row_info_.ensure(per);
     for (size_t r0 = 0; r0 < n; r0 += per) {
         const size_t cnt = std::min(per, n - r0);
-        const float* xr = x + r0 * d_;
-        if (vec) row_fp16_kernel<true><<<warps_grid(cnt), 256, 0, stream>>>(xr, cnt, d_, dp_, mean_.get(), stats, norms_x + r0, xh, row_info_.get());
-        else row_fp16_kernel<false><<<warps_grid(cnt), 256, 0, stream>>>(xr, cnt, d_, dp_, mean_.get(), stats, norms_x + r0, xh, row_info_.get());
-        SKM_LAUNCH_CHECK();
-        p.n = cnt;
-        p.first = first + r0;
-        const CUtensorMap tx = make_half_tmap(xh, dp_, cnt, 128);
-        const unsigned grid = static_cast<unsigned>(2 * std::min(pairs, (cnt + 255) / 256));
-        filter_tc_kernel<<<grid, F_THREADS, F_SMEM_BYTES, stream>>>(tx, ty, p);
-        SKM_LAUNCH_CHECK();
-        if (vec) decide_kernel<true><<<warps_grid(cnt), 256, 0, stream>>>(xr, y_, cnt, k_, d_, norms_x + r0, norms_y_, cand_.get(), out_knn + r0, out_dist + r0, p.error);
-        else decide_kernel<false><<<warps_grid(cnt), 256, 0, stream>>>(xr, y_, cnt, k_, d_, norms_x + r0, norms_y_, cand_.get(), out_knn + r0, out_dist + r0, p.error);
-        SKM_LAUNCH_CHECK();
+        convert(x + r0 * d_, cnt, norms_x + r0, stream);
+        search(x + r0 * d_, first + r0, cnt, nullptr, 0, norms_x + r0, out_knn + r0, out_dist + r0, stream);
     }
+}
+
+void ExactAssign::begin_groups(const float* x, size_t n, size_t d, const float* y, size_t k, float* norms_x, cudaStream_t stream) {
+    listed_.ensure(n);
+    d_ = d;
+    dp_ = (d + 7) / 8 * 8;
+    xh_.ensure(n * dp_);
+    row_info_.ensure(n);
+    sample_mean_kernel<<<static_cast<unsigned>((d + 63) / 64), 64, 0, stream>>>(y, k, d, mean_.ensure(dp_), stats_.ensure(kStats), n_listed_.ensure(1));
+    SKM_LAUNCH_CHECK();
+    convert(x, n, norms_x, stream);
+}
+
+void ExactAssign::assign_groups(const float* x, size_t n, const float* y, size_t k, const AssignTile* tiles, size_t n_tiles, const float* norms_x, float* norms_y, uint32_t* out_knn,
+                                float* out_dist, cudaStream_t stream) {
+    if (n_tiles == 0) return;
+    centroids(y, k, norms_y, false, stream);
+    SKM_CUDA(cudaMemsetAsync(cand_.ensure(n), 0xFF, sizeof(uint4) * n, stream));   // rows of no tile: nothing to decide
+    search(x, 0, n, tiles, n_tiles, norms_x, out_knn, out_dist, stream);
+    decide_listed_kernel<<<592, 256, 0, stream>>>(x, y, d_, norms_x, norms_y, tiles, n_tiles, listed_.get(), n_listed_.get(), out_knn, out_dist, error_word());
+    SKM_LAUNCH_CHECK();
 }
 
 size_t ExactAssign::settle(cudaStream_t stream) {

@@ -25,6 +25,11 @@ class DirectAssign {
     DeviceBuffer<uint32_t> counters_, arrived_;
 };
 
+// Up to 256 rows and the centroids they are assigned to: rows [row0, row0 + rows) of x, rows [y0, y0 + k) of y.
+struct AssignTile {
+    uint32_t row0, rows, y0, k;
+};
+
 // Nearest centroid of every row, in three steps:
 //   1. rows and centroids, centred on the mean of some centroids, are rounded to fp16 (scaled by powers of two) together
 //      with the norms of what the rounding took away;
@@ -50,13 +55,24 @@ class ExactAssign {
     // Both, for a batch that is still on the device.
     size_t settle_on_device(const float* x_batch, uint32_t* out_knn, float* out_dist, cudaStream_t stream);
 
+    // Many problems at once: every row tile has centroids of its own.  begin_groups converts the rows (which may then be
+    // assigned several times; y gives the mean), assign_groups assigns the rows of the tiles, which are sorted by row; the
+    // other rows' answers stay as they are.  Indices count from the beginning of y.
+    void begin_groups(const float* x, size_t n, size_t d, const float* y, size_t k, float* norms_x, cudaStream_t stream);
+    void assign_groups(const float* x, size_t n, const float* y, size_t k, const AssignTile* tiles, size_t n_tiles, const float* norms_x, float* norms_y, uint32_t* out_knn,
+                       float* out_dist, cudaStream_t stream);
+
   private:
+    void centroids(const float* y, size_t k, float* norms_y, bool with_mean, cudaStream_t stream);
+    void convert(const float* x, size_t n, float* norms_x, cudaStream_t stream);
+    void search(const float* x, size_t first, size_t n, const AssignTile* tiles, size_t n_tiles, const float* norms_x, uint32_t* out_knn, float* out_dist, cudaStream_t stream);
     const float* y_ = nullptr;
     const float* norms_y_ = nullptr;
     size_t k_ = 0, d_ = 0, dp_ = 0, kp_ = 0;
     DeviceBuffer<__half> xh_, yh_;
-    DeviceBuffer<float> mean_, centred_norms_, stats_;
-    DeviceBuffer<float2> row_info_;
+    DeviceBuffer<float> mean_, centred_norms_;
+    DeviceBuffer<uint32_t> stats_;
+    DeviceBuffer<float4> row_info_;
     DeviceBuffer<uint4> cand_;
     DeviceBuffer<uint32_t> listed_, n_listed_;
     PinnedBuffer<uint32_t> n_listed_host_;

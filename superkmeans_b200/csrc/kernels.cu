@@ -955,26 +955,7 @@ void launch_scale_by_counts(float* c, const uint32_t* counts, size_t k, size_t d
 __global__ void apply_split_ops_kernel(float* __restrict__ c, size_t d, const SplitOpDev* __restrict__ ops, size_t n_ops) {
     const size_t j = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (j >= d) return;
-    const float up = 1.0f + (1.0f / 1024.0f), down = 1.0f - (1.0f / 1024.0f);
-    for (size_t o = 0; o < n_ops; ++o) {
-        const SplitOpDev op = ops[o];
-        float* pd = c + static_cast<size_t>(op.dst) * d + j;
-        float* ps = c + static_cast<size_t>(op.src) * d + j;
-        if (op.kind == 0) {
-            const float v = *ps;
-            if ((j & 1) == 0) {
-                *pd = __fmul_rn(v, up);
-                *ps = __fmul_rn(v, down);
-            } else {
-                *pd = __fmul_rn(v, down);
-                *ps = __fmul_rn(v, up);
-            }
-        } else {
-            float val = __fmul_rn(op.wc, *pd);
-            val = __fadd_rn(val, *ps);
-            *pd = __fdiv_rn(val, __fadd_rn(op.wc, 1.0f));
-        }
-    }
+    for (size_t o = 0; o < n_ops; ++o) apply_split_op(c, d, j, ops[o]);
 }
 
 void launch_apply_split_ops(float* c, size_t d, const SplitOpDev* ops, size_t n_ops, cudaStream_t stream) {
@@ -987,13 +968,7 @@ void launch_apply_split_ops(float* c, size_t d, const SplitOpDev* ops, size_t n_
 __global__ void normalize_rows_kernel(float* __restrict__ c, size_t k, size_t d) {
     const size_t row = static_cast<size_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
     if (row >= k) return;
-    const int lane = threadIdx.x & 31;
-    float* p = c + row * d;
-    float s = 0.f;
-    for (size_t j = lane; j < d; j += 32) s = fmaf(p[j], p[j], s);
-    s = warp_sum(s);
-    const float inv = 1.0f / sqrtf(s);
-    for (size_t j = lane; j < d; j += 32) p[j] *= inv;
+    normalize_row(c + row * d, d, threadIdx.x & 31);
 }
 
 void launch_normalize_rows(float* c, size_t k, size_t d, cudaStream_t stream) {
