@@ -346,9 +346,6 @@ def run_reference_arm(args, spec, n):
 # kernel at n = 400 000 rows (same d and k), divided by the rows.  Traffic of these kernels grows with the rows (the
 # centroid side stays in L2), so a launch over r rows moves about r times this.
 TRAFFIC_PER_ROW = {
-    ("gemm_tc_kernel<ARGMIN>", 1024, 10_000): 3.59e9 / 4e5,
-    ("gemm_tc_kernel<PRUNE>", 1024, 10_000): 0.377e9 / 4e5,
-    ("walk_lists_kernel", 1024, 10_000): 5.86e9 / 4e5,
     # optimistic chain pass, captured at n = 1 000 000 in the first pruned iteration (the one with the longest centroid
     # lists: an upper figure for the later ones)
     ("sparse_chain_kernel", 1024, 10_000): 137.9e9 / 1e6,
@@ -492,12 +489,12 @@ def main():
     cands = []   # (kernel, phase ms over all timed steps, launches, bound, work per step)
     if kind == "assign":
         ms, calls = phase_acc["search/1st_blas"]
-        cands.append(("gemm_tc_kernel<ARGMIN>", ms, calls, "tensor", 2.0 * n_local * k * d))
+        cands.append(("filter_tc_kernel", ms, calls, "tensor", 2.0 * n_local * k * d))
     elif hier:
         n_meso = int(round(np.sqrt(k)))
         ms, calls = phase_acc["search/1st_blas"]
         # every phase sees ~k / n_meso centroids per point: 3 mesoclustering + 5 fine iterations, all exact
-        cands.append(("gemm_tc_kernel<ARGMIN>", ms, calls, "tensor", 2.0 * n_local * d * (3.0 * n_meso + 5.0 * k / n_meso)))
+        cands.append(("filter_tc_kernel", ms, calls, "tensor", 2.0 * n_local * d * (3.0 * n_meso + 5.0 * k / n_meso)))
         ms, calls = phase_acc["update_centroids"]
         cands.append(("segsum_tile_kernel", ms, calls, "hbm", 8.0 * n_local * d * 4.0))
         ms, calls = phase_acc["rotator"]
@@ -508,14 +505,14 @@ def main():
         d_partial = [s.partial_d for s in stats if not s.is_gemm_only]
         mean_pd = float(np.mean(d_partial)) if d_partial else 0.0
         ms, calls = phase_acc["search/1st_blas"]
-        cands.append(("gemm_tc_kernel<ARGMIN>", ms, calls, "tensor", sum(2.0 * n_local * k * d for s in stats if s.is_gemm_only)))
+        cands.append(("filter_tc_kernel", ms, calls, "tensor", sum(2.0 * n_local * k * d for s in stats if s.is_gemm_only)))
         ms, calls = phase_acc["search/first_test"]
         # a Train can mix routes (the automatic choice is taken per pass): rows that went through the ordered chain, rows
         # of the unordered dense chain, and rows that took first test + list walk
         chain_rows = chain["rows"]
         legacy_dense_rows = max(0, counters["dense_rows"] - chain_rows)
         listed_rows = max(0, n_local * len(d_partial) - chain_rows)
-        cands.append(("gemm_tc_kernel<PRUNE>", ms, calls, "tensor", 2.0 * listed_rows * k * mean_pd if ms > 0 else 0.0))
+        cands.append(("first_test_kernel", ms, calls, "tensor", 2.0 * listed_rows * k * mean_pd if ms > 0 else 0.0))
         ms, calls = phase_acc["search/dense"]
         if chain_rows >= legacy_dense_rows:
             # union pass over the first d' dimensions of every centroid + the chain over the gathered columns (128 rows per unit)

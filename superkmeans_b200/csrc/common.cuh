@@ -74,6 +74,7 @@ double alloc_free_ms();
 constexpr int kTileM = 128;        // points per CTA tile
 constexpr int kTileN = 128;        // centroids per GEMM sub-tile (SIMT path)
 constexpr int kChunk = 1024;       // centroids per pruning chunk (reference VECTOR_CHUNK_SIZE)
+constexpr int kListsPerTile = 16;  // candidate lists of a row tile: 4 groups of 32 rows x 4 groups of 64 of every 256 centroids
 constexpr int kHBlock = 64;        // dimensions per horizontal block (reference H_DIM_SIZE)
 constexpr int kUpdateTile = 1024;      // sorted points per segmented-sum tile
 constexpr int kUpdateTileSmall = 128;  // ... when there are few points
@@ -132,6 +133,7 @@ struct PrunedParams {
     uint32_t partial_d, vertical_d, horizontal_d;
     const float* best_in = nullptr;     // optional: exact distance to the previous centroid, per point
     const uint32_t* skip = nullptr;     // optional: 1 = leave this point to the dense kernel
+    bool same_points = false;           // x holds what it held in the pass before (its fp16 halves can be used again)
 };
 
 // Work split of one pruned pass.  Points whose ADSampling test would keep a large share of the
@@ -204,8 +206,8 @@ struct WalkParams {
     const float* y_pdx;
     const float* y_aux;
     const float* ratios;
-    const uint2* lists;          // n_tiles * 8 lists of cap_group entries (see tc::launch_first_test)
-    const uint32_t* list_offs;   // n_tiles * 8 * (n_chunks + 1)
+    const uint2* lists;          // n_tiles * kListsPerTile lists of cap_group entries (see tc::launch_first_test)
+    const uint32_t* list_offs;   // n_tiles * kListsPerTile * (n_chunks + 1)
     uint32_t cap_group;
     size_t n, k, d;
     uint32_t partial_d, vertical_d, horizontal_d;
@@ -219,7 +221,6 @@ struct WalkParams {
     uint32_t* redo;              // set to 1 for points whose group list overflowed
     uint32_t* redo_count;
     unsigned long long* pair_steps;            // += pairs advanced by one 64-dimension block
-    uint32_t rebalance_mask = 0x22;            // bit b: even the runs out after block b (here: after the 2nd and the 6th)
     const int* upstream_error = nullptr;       // set when the kernel that wrote the lists gave up on a wait: the lists are then not read
 };
 void launch_walk_lists(const WalkParams& w, int device, cudaStream_t stream);

@@ -602,9 +602,9 @@ void run_pruned_pass_sorted(const PrunedParams& p, PrunePassBuffers& b, float ra
     if (const char* v = std::getenv("SKM_DENSE_FLAG_MULT")) ws.flag_mult = static_cast<uint32_t>(std::max(1, std::atoi(v)));
     if (const char* v = std::getenv("SKM_DENSE_TILE_ROWS")) dense_tile_rows = static_cast<uint32_t>(std::max(1, std::atoi(v)));
 
-    // candidate lists: eight per tile, each with room for an eighth of its pairs (modes 5 / 8: a thirty-second)
-    const uint32_t cap_group = static_cast<uint32_t>(std::max<size_t>(128, mode == 8 ? p.k / 2 : p.k * 2));
-    const size_t list_tile_bytes = 8 * static_cast<size_t>(cap_group) * sizeof(uint2);
+    // candidate lists: sixteen per tile, each with room for an eighth of its pairs (modes 5 / 8: a thirty-second)
+    const uint32_t cap_group = static_cast<uint32_t>(std::max<size_t>(128, mode == 8 ? p.k / 4 : p.k));
+    const size_t list_tile_bytes = kListsPerTile * static_cast<size_t>(cap_group) * sizeof(uint2);
     const size_t lists_per_launch = std::max<size_t>(1, (static_cast<size_t>(6) << 30) / list_tile_bytes);
     // chain: at most ~1 GB of column lists per launch
     const size_t chain_per_launch = std::max<size_t>(1, (size_t{1} << 30) / (cols_stride * sizeof(uint16_t)));
@@ -799,14 +799,17 @@ void run_pruned_pass_sorted(const PrunedParams& p, PrunePassBuffers& b, float ra
             uint32_t* redo_count = redo_b + batch;
             SKM_CUDA(cudaMemsetAsync(redo_b, 0, sizeof(uint32_t) * (batch + 1), stream));
             const size_t per = std::min(n_lists, lists_per_launch);
-            uint2* lists = b.tc_lists.ensure(per * 8 * cap_group);
-            uint32_t* offs = b.tc_list_offs.ensure(per * 8 * (n_chunks + 1));
+            uint2* lists = b.tc_lists.ensure(per * kListsPerTile * cap_group);
+            uint32_t* offs = b.tc_list_offs.ensure(per * kListsPerTile * (n_chunks + 1));
+            const tc::SplitHalves xs = b.x_halves(cnt, p.partial_d), ys = b.y_halves(p.k, p.partial_d);
+            b.x_halves_valid = false;
+            tc::launch_split_points(xb, cnt, p.d, p.partial_d, xs, stream);
+            tc::launch_split_centroids(p.y, p.k, p.d, p.partial_d, p.norms_y, ys, stream);
             for (size_t t0 = 0; t0 < n_lists; t0 += per) {
                 const size_t nt = std::min(per, n_lists - t0);
                 {
                     SubPhase sub(timers, PH_PRUNE_FIRST_TEST, stream);
-                    tc::launch_first_test(xb, p.y, cnt, p.k, p.d, p.partial_d, nx_b, p.norms_y, best_b, nullptr, ratio_first, 0, nt, lists, offs, cap_group, stream, y_split,
-                                          map_lists + t0);
+                    tc::launch_first_test(xs, ys, cnt, p.k, p.partial_d, nx_b, p.norms_y, best_b, nullptr, ratio_first, 0, nt, lists, offs, cap_group, stream, map_lists + t0);
                 }
                 WalkParams w{};
                 w.x = xb;
@@ -889,6 +892,7 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
         }
     };
     if (p.n == 0) return;
+    if (!p.same_points) b.x_halves_valid = false;
     int mode = g_prune_split_mode;
     const bool auto_mode = mode == 0;
     if (((mode >= 6 && mode <= 8) || mode == 10 || mode == 11) && tc::eligible(p.x, p.d, p.y, p.d)) {
@@ -981,23 +985,31 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
         SKM_CUDA(cudaMemsetAsync(pair_steps, 0, sizeof(unsigned long long), stream));
         if (n_hard < p.n) {
             const size_t n_chunks = (p.k + kChunk - 1) / kChunk;
-            // eight lists per tile of 128 points, each with room for an eighth of its pairs (32 points x half the
-            // centroids); mode 5: a thirty-second, so that lists overflow
-            const uint32_t cap_group = static_cast<uint32_t>(std::max<size_t>(128, mode == 5 ? p.k / 2 : p.k * 2));
-            const size_t tile_bytes = 8 * static_cast<size_t>(cap_group) * sizeof(uint2);
+            // sixteen lists per tile of 128 points, each with room for an eighth of its pairs (32 points x a quarter of
+            // the centroids); mode 5: a thirty-second, so that lists overflow.  The automatic choice knows the share of pairs
+            // that will be listed and makes room for three times that, and for no less than 7 % (so that the buffer does not
+            // grow from pass to pass): at 1M x 4000 two gigabytes instead of four.
+            const size_t pairs_per_list = 8 * p.k;
+            double room = mode == 5 ? 1.0 / 32 : 1.0 / 8;
+            if (mode == 0) room = std::min(room, 0.012 + 3.0 * std::max(b.last_survival, 0.02));
+            const uint32_t cap_group = static_cast<uint32_t>(std::max<size_t>(128, static_cast<size_t>(static_cast<double>(pairs_per_list) * room)));
+            const size_t tile_bytes = kListsPerTile * static_cast<size_t>(cap_group) * sizeof(uint2);
             const size_t n_tiles = (p.n + kTileM - 1) / kTileM;
-            const size_t list_bytes_cap = static_cast<size_t>(6) << 30;
+            const size_t list_bytes_cap = static_cast<size_t>(3) << 30;
             // at least one tile per batch; when even one tile's lists exceed the cap (k in the millions) the batch is that one tile
             const size_t per_batch = std::min(n_tiles, std::max<size_t>(1, list_bytes_cap / tile_bytes));
-            uint2* lists = b.tc_lists.ensure(per_batch * 8 * cap_group);
-            uint32_t* offs = b.tc_list_offs.ensure(per_batch * 8 * (n_chunks + 1));
-            float* y_split = b.y_split.ensure(2 * p.k * p.d);
-            tc::launch_presplit(p.y, p.k, p.d, y_split, stream);
+            uint2* lists = b.tc_lists.ensure(per_batch * kListsPerTile * cap_group);
+            uint32_t* offs = b.tc_list_offs.ensure(per_batch * kListsPerTile * (n_chunks + 1));
+            // d' moves below vertical_d from pass to pass: the points are split that far, once
+            const tc::SplitHalves xs = b.x_halves(p.n, p.vertical_d), ys = b.y_halves(p.k, p.partial_d);
+            if (!(p.same_points && b.x_halves_valid)) tc::launch_split_points(p.x, p.n, p.d, p.vertical_d, xs, stream);
+            b.x_halves_valid = true;
+            tc::launch_split_centroids(p.y, p.k, p.d, p.partial_d, p.norms_y, ys, stream);
             for (size_t t0 = 0; t0 < n_tiles; t0 += per_batch) {
                 const size_t nt = std::min(per_batch, n_tiles - t0);
                 {
                     Sub sub(timers, PH_PRUNE_FIRST_TEST, stream);
-                    tc::launch_first_test(p.x, p.y, p.n, p.k, p.d, p.partial_d, p.norms_x, p.norms_y, ws.best, ws.flags, ratio_first, t0, nt, lists, offs, cap_group, stream, y_split);
+                    tc::launch_first_test(xs, ys, p.n, p.k, p.partial_d, p.norms_x, p.norms_y, ws.best, ws.flags, ratio_first, t0, nt, lists, offs, cap_group, stream);
                 }
                 WalkParams w{};
                 w.x = p.x;
@@ -1062,8 +1074,10 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
     launch_assign_pruned_dense(p, ws, n_hard, stream);
 }
 
-void Engine::run_pruned_pass(const float* x, size_t n, size_t k_cur, const float* y, const float* norms_x, const float* norms_y, uint32_t* knn, float* dist, uint32_t* not_pruned) {
+void Engine::run_pruned_pass(const float* x, size_t n, size_t k_cur, const float* y, const float* norms_x, const float* norms_y, uint32_t* knn, float* dist, uint32_t* not_pruned,
+                             bool same_points) {
     PrunedParams p{};
+    p.same_points = same_points;
     p.x = x;
     p.y = y;
     p.y_pdx = c_pdx_.get();
@@ -1125,7 +1139,8 @@ void Engine::run_iteration(bool gemm_only, const IterationInput& in, size_t iter
     } else {
         launch_row_sqnorms(c_prev_.get(), k_cur, d_, partial_d_, centroid_norms_.get(), stream_);
         PhaseScope ps(*this, PH_ASSIGN_PRUNED);
-        run_pruned_pass(in.x, n, k_cur, c_prev_.get(), norms, centroid_norms_.get(), assignments_.get(), distances_.get(), not_pruned_.get());
+        run_pruned_pass(in.x, n, k_cur, c_prev_.get(), norms, centroid_norms_.get(), assignments_.get(), distances_.get(), not_pruned_.get(), in.pruned_before);
+        in.pruned_before = true;
     }
     // UpdateCentroids + ComputeCost (superkmeans.h:729-765, :973-981)
     {

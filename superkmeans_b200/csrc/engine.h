@@ -18,6 +18,7 @@
 #include "exact_assign.h"
 #include "host_copy.h"
 #include "host_logic.h"
+#include "kernels_tc.cuh"
 
 namespace skmb {
 
@@ -95,6 +96,19 @@ struct PrunePassBuffers {
     unsigned long long total_fallback_rows = 0; // ... of which the candidate lists overflowed: redone by the exact chain pass
     DeviceBuffer<uint32_t> cand, cand_meta, replay_ovf, replay_np, positions2, hard_idx2, hard_idx3, n_hard_dev2;
     DeviceBuffer<float> replay_thr;
+    // fp16 halves of points and centroids for the first test with lists; those of the points serve all passes over the same rows
+    DeviceBuffer<__half> x_hi, x_lo, y_hi, y_lo;
+    DeviceBuffer<float> x_factor, y_factor;
+    bool x_halves_valid = false;
+    // `cols` columns of rows x d
+    tc::SplitHalves x_halves(size_t rows, uint32_t cols) {
+        const uint32_t pitch = (cols + 7) / 8 * 8;
+        return {x_hi.ensure(rows * pitch), x_lo.ensure(rows * pitch), x_factor.ensure(rows), pitch};
+    }
+    tc::SplitHalves y_halves(size_t rows, uint32_t cols) {
+        const uint32_t pitch = (cols + 7) / 8 * 8;
+        return {y_hi.ensure(rows * pitch), y_lo.ensure(rows * pitch), y_factor.ensure(1), pitch};
+    }
 };
 // mode: 0 = automatic: with rows that TMA can address, the points are taken in the order of their previous centroid and
 // every tile of 128 goes either through the first test + list walk or, when many of its points keep a large share of
@@ -185,6 +199,7 @@ class Engine {
         size_t n_samples_global;
         size_t n_clusters;
         float* norms;         // device, full or partial norms of x (rewritten when d' changes)
+        mutable bool pruned_before = false;   // a pruned pass over these rows has run
     };
 
     void start_rotation_draws();   // the Gaussian draws of a matrix that is still to be made, on a host thread
@@ -200,7 +215,8 @@ class Engine {
     size_t streamed_rows(size_t n) const;
     void prepare_update_workspace(size_t n, size_t k);
     void run_iteration(bool gemm_only, const IterationInput& in, size_t iter_idx, bool is_first, std::vector<skm_iter_stats>& target);
-    void run_pruned_pass(const float* x, size_t n, size_t k_cur, const float* y, const float* norms_x, const float* norms_y, uint32_t* knn, float* dist, uint32_t* not_pruned);
+    void run_pruned_pass(const float* x, size_t n, size_t k_cur, const float* y, const float* norms_x, const float* norms_y, uint32_t* knn, float* dist, uint32_t* not_pruned,
+                         bool same_points = false);
     void consolidate(size_t n_samples_global, size_t k_cur);
     // `precomputed`: the Forgy indices when the caller has already drawn them (on another thread, while buffers were allocated)
     void generate_centroids_from_host(const float* data, bool on_device, size_t n_points_global, size_t k_cur, bool rotate, const std::vector<size_t>* precomputed = nullptr);

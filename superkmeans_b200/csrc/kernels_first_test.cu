@@ -1,0 +1,400 @@
+// First ADSampling test on the tensor cores (batch_computers.h:297-409, pdxearch.h:118-143): the partial distances over the
+// first d' dimensions of every (point, centroid) pair against best * ratio[d'], survivors to candidate lists that
+// walk_lists_kernel takes up.
+//
+// Points and centroids come as fp16 pairs v * scale = hi + lo (scale a power of two, 22 bits: what two tf32 parts hold), and
+// a product is hi*hi + hi*lo + lo*hi with fp32 accumulation: fp32-level accuracy at twice the rate of tf32.  The points are
+// split once per training, over the dimensions d' can reach, not in every tile.
+//
+// Persistent pairs of CTAs (cta_group::2) on tiles of 256 rows x 256 centroids, as in exact_assign.cu:
+//   warp 0     TMA producer: 128 x 64 halves of each of the four parts per stage, three stages;
+//   warp 1     MMA issuer (leader only), two accumulators of 256 columns;
+//   warps 2-17 test, a warp per 32 rows and 64 columns: partial distance = ||x||^2 + ||c||^2 - 2 x.c, survivors appended to
+//              the warp's list.  The test is latency-bound (270 instructions per 32 columns, a scan and a walk over the
+//              survivors' bits among them), hence four warps per scheduler: with two it took 6500 cycles per tile.
+// Every wait is bounded (see kernels_tc.cu).
+#include <cfloat>
+#include <cmath>
+
+#include "common.cuh"
+#include "device_utils.cuh"
+#include "kernels_tc.cuh"
+#include "tc_ptx.cuh"
+
+namespace skmb {
+namespace tc {
+
+namespace {
+
+constexpr int TK = 64;
+constexpr int T_STAGES = 3;
+constexpr uint32_t T_PART_BYTES = 128 * TK * 2;
+constexpr uint32_t T_STAGE_BYTES = 4 * T_PART_BYTES;   // rows hi, rows lo, centroids hi, centroids lo
+constexpr int T_TEST_WARPS = 16;
+constexpr int T_THREADS = 64 + 32 * T_TEST_WARPS;
+constexpr uint32_t T_CTRL_BYTES = 8192 + T_TEST_WARPS * 8 * 32 * 4 + 256;
+constexpr uint32_t T_SMEM_BYTES = T_STAGES * T_STAGE_BYTES + T_CTRL_BYTES + 1024;
+
+struct TestCtrl {
+    alignas(16) float ny[4][2][256];   // per row quarter and accumulator
+    float column[T_TEST_WARPS][8 * 32];   // per test warp: 8 values of each of its lanes
+    uint64_t full[T_STAGES];           // (the leader's are used)
+    uint64_t empty[T_STAGES];
+    uint64_t acc_full[2];
+    uint64_t acc_empty[2];             // (the leader's are used)
+    uint32_t tmem_base;
+};
+static_assert(sizeof(TestCtrl) <= T_CTRL_BYTES, "control block too large");
+
+struct TestMaps {
+    CUtensorMap xhi, xlo, yhi, ylo;
+};
+
+struct TestParams {
+    size_t n, k;
+    uint32_t k_blocks;
+    size_t tile0, n_tiles;       // of 128 rows
+    const uint32_t* tile_map;    // null: tile0, tile0 + 1, ...
+    const float* factor_x;       // per row: -2 / scale
+    const float* factor_y;       // one: 1 / scale
+    const float* norms_x;
+    const float* norms_y;
+    const float* best_in;
+    const uint32_t* skip;
+    float ratio_first;
+    uint2* lists;
+    uint32_t* list_offs;
+    uint32_t cap_group;
+    int* error;
+    long long wait_limit;
+};
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T_THREADS, 1) first_test_kernel(const __grid_constant__ TestMaps maps, const TestParams p) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw_addr = smem_u32(smem_raw);
+    const uint32_t pad = (1024u - (raw_addr & 1023u)) & 1023u;
+    const uint32_t smem_base = raw_addr + pad;
+    TestCtrl* ctrl = reinterpret_cast<TestCtrl*>(smem_raw + pad + T_STAGES * T_STAGE_BYTES);
+    const WaitCtx wctx{p.error, p.wait_limit};
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank();
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < T_STAGES; ++s) {
+            mbar_init(&ctrl->full[s], 1);
+            mbar_init(&ctrl->empty[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&ctrl->acc_full[b], 1);
+            mbar_init(&ctrl->acc_empty[b], 2 * T_TEST_WARPS);   // a lane of each of the pair's test warps
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_proxy_async();
+    }
+    if (warp == 1) tmem_alloc_pair(&ctrl->tmem_base, TMEM_COLS);
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();   // the peer's barriers exist
+    tc_fence_after();
+    const uint32_t tmem_base = ctrl->tmem_base;
+
+    const size_t pair_tiles = (p.n_tiles + 1) / 2;
+    const uint32_t col_tiles = static_cast<uint32_t>((p.k + 255) / 256);
+    const size_t pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+    // this CTA's row tile of pair tile t (the second one of the last pair may not exist: a tile behind the last row)
+    auto tile_of = [&](size_t t) -> size_t {
+        const size_t q = 2 * t + rank;
+        if (q >= p.n_tiles) return (p.n + 127) / 128;
+        return p.tile_map ? static_cast<size_t>(__ldg(p.tile_map + q)) : p.tile0 + q;
+    };
+
+    if (warp == 0) {
+        if (lane == 0) {
+            uint32_t kbt = 0;
+            bool ok = true;
+            for (size_t t = pair; t < pair_tiles && ok; t += n_pairs) {
+                const int x_row = static_cast<int>(tile_of(t) * 128);
+                for (uint32_t nt = 0; nt < col_tiles && ok; ++nt) {
+                    const int y_row = static_cast<int>(nt * 256 + rank * 128);
+                    for (uint32_t kb = 0; kb < p.k_blocks; ++kb, ++kbt) {
+                        const uint32_t s = kbt % T_STAGES, ph = (kbt / T_STAGES) & 1u;
+                        if (!mbar_wait(&ctrl->empty[s], ph ^ 1u, wctx, 51)) {
+                            ok = false;
+                            break;
+                        }
+                        if (rank == 0) mbar_arrive_expect_tx(&ctrl->full[s], 2 * T_STAGE_BYTES);
+                        const uint32_t bar = cluster_address(&ctrl->full[s], 0);
+                        const uint32_t st = smem_base + s * T_STAGE_BYTES;
+                        const int col = static_cast<int>(kb * TK);
+                        tma_load_2d_pair(st, &maps.xhi, bar, col, x_row);
+                        tma_load_2d_pair(st + T_PART_BYTES, &maps.xlo, bar, col, x_row);
+                        tma_load_2d_pair(st + 2 * T_PART_BYTES, &maps.yhi, bar, col, y_row);
+                        tma_load_2d_pair(st + 3 * T_PART_BYTES, &maps.ylo, bar, col, y_row);
+                    }
+                }
+            }
+            if (!ok) {
+                // another role gave up: a millisecond for the copies that are in flight before the block's memory is let go
+                const long long t0 = clock64();
+                while (clock64() - t0 < 2000000) {
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t idesc = make_idesc_f16(256, 256);
+            uint32_t kbt = 0, u = 0;
+            bool ok = true;
+            for (size_t t = pair; t < pair_tiles && ok; t += n_pairs) {
+                for (uint32_t nt = 0; nt < col_tiles && ok; ++nt, ++u) {
+                    const uint32_t b = u & 1u, uph = (u >> 1) & 1u;
+                    if (!mbar_wait(&ctrl->acc_empty[b], uph ^ 1u, wctx, 52)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t acc = tmem_base + b * 256;
+                    for (uint32_t kb = 0; kb < p.k_blocks; ++kb, ++kbt) {
+                        const uint32_t s = kbt % T_STAGES, ph = (kbt / T_STAGES) & 1u;
+                        if (!mbar_wait(&ctrl->full[s], ph, wctx, 53)) {
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after();
+                        const uint32_t st = smem_base + s * T_STAGE_BYTES;
+#pragma unroll
+                        for (uint32_t kk = 0; kk < TK / 16; ++kk) {
+                            const uint64_t xh = make_desc_128(st + kk * 32), xl = make_desc_128(st + T_PART_BYTES + kk * 32);
+                            const uint64_t yh = make_desc_128(st + 2 * T_PART_BYTES + kk * 32), yl = make_desc_128(st + 3 * T_PART_BYTES + kk * 32);
+                            umma_f16_pair(acc, xh, yh, (kb | kk) != 0 ? 1u : 0u, idesc);
+                            umma_f16_pair(acc, xh, yl, 1u, idesc);
+                            umma_f16_pair(acc, xl, yh, 1u, idesc);
+                        }
+                        umma_commit_pair(&ctrl->empty[s]);
+                    }
+                    if (ok) umma_commit_pair(&ctrl->acc_full[b]);
+                }
+            }
+        }
+    } else {
+        const uint32_t quarter = warp & 3, part = static_cast<uint32_t>(warp - 2) >> 2;   // rows 32 quarter.., columns 64 part..
+        const uint32_t lane_base = 32u * quarter;
+        float* column = ctrl->column[warp - 2] + lane;
+        const float fy = *p.factor_y;
+        uint32_t u = 0;
+        bool ok = true;
+        for (size_t t = pair; t < pair_tiles && ok; t += n_pairs) {
+            const size_t q = 2 * t + rank;
+            const bool listed = q < p.n_tiles;
+            const size_t row = tile_of(t) * 128 + lane_base + lane;
+            const bool valid = listed && row < p.n;
+            const float nx = valid ? p.norms_x[row] : 0.f;
+            const float factor = valid ? p.factor_x[row] * fy : 0.f;
+            const float thr = valid && !(p.skip && p.skip[row]) ? p.best_in[row] * p.ratio_first : -FLT_MAX;
+            const size_t group = (listed ? q : 0) * kListsPerTile + part * 4 + quarter;
+            uint2* my_list = p.lists + group * p.cap_group;
+            uint32_t* my_offs = p.list_offs + group * ((p.k + 1023) / 1024 + 1);
+            uint32_t filled = 0;   // warp-uniform
+            for (uint32_t nt = 0; nt < col_tiles && ok; ++nt, ++u) {
+                const uint32_t b = u & 1u, uph = (u >> 1) & 1u;
+                const uint32_t col0 = nt * 256 + part * 64;
+                float* ny = ctrl->ny[quarter][b] + part * 64;   // the four warps of a quarter fill (and read) their own parts
+                if ((nt & 3u) == 0 && lane == 0 && listed) my_offs[nt >> 2] = filled;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) ny[i * 32 + lane] = col0 + i * 32 + lane < p.k ? __ldg(p.norms_y + col0 + i * 32 + lane) : INFINITY;   // never below a threshold
+                __syncwarp();
+                if (!__all_sync(0xffffffffu, mbar_wait(&ctrl->acc_full[b], uph, wctx, 54))) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t taddr = tmem_base + (lane_base << 16) + b * 256 + part * 64;
+                auto test = [&](uint32_t (&r)[32], int ch) {
+                    uint32_t mask = 0;
+#pragma unroll
+                    for (int j = 0; j < 32; j += 4) {
+                        const float4 nyv = *reinterpret_cast<const float4*>(ny + ch * 32 + j);
+                        const float p0 = fmaf(factor, __uint_as_float(r[j + 0]), nx) + nyv.x;
+                        const float p1 = fmaf(factor, __uint_as_float(r[j + 1]), nx) + nyv.y;
+                        const float p2 = fmaf(factor, __uint_as_float(r[j + 2]), nx) + nyv.z;
+                        const float p3 = fmaf(factor, __uint_as_float(r[j + 3]), nx) + nyv.w;
+                        r[j + 0] = __float_as_uint(p0);
+                        r[j + 1] = __float_as_uint(p1);
+                        r[j + 2] = __float_as_uint(p2);
+                        r[j + 3] = __float_as_uint(p3);
+                        mask |= (p0 < thr ? (1u << j) : 0u) | (p1 < thr ? (2u << j) : 0u) | (p2 < thr ? (4u << j) : 0u) | (p3 < thr ? (8u << j) : 0u);
+                    }
+                    if (!__any_sync(0xffffffffu, mask != 0)) return;
+                    // where a lane's survivors go: behind those of the lanes before it
+                    const uint32_t cnt = __popc(mask);
+                    uint32_t incl = cnt;
+#pragma unroll
+                    for (int off = 1; off < 32; off <<= 1) {
+                        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, off);
+                        if (lane >= off) incl += v;
+                    }
+                    uint32_t pos = filled + incl - cnt;
+                    filled += __shfl_sync(0xffffffffu, incl, 31);
+                    // They are few and found bit by bit, their values through a column of shared memory of the lane's own,
+                    // because registers cannot be indexed (unrolled over the columns, this outgrows the instruction cache).
+                    const uint32_t colbits = ((col0 + ch * 32) << 5) | static_cast<uint32_t>(lane);
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) {
+                        uint32_t sub = (mask >> (8 * h)) & 0xFFu;
+                        if (!__any_sync(0xffffffffu, sub != 0)) continue;
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) column[j * 32] = __uint_as_float(r[8 * h + j]);
+#pragma unroll 1
+                        while (sub) {
+                            const uint32_t j = __ffs(sub) - 1;
+                            sub &= sub - 1;
+                            if (pos < p.cap_group) my_list[pos] = make_uint2(colbits + ((8u * h + j) << 5), __float_as_uint(column[j * 32]));
+                            ++pos;
+                        }
+                        __syncwarp();
+                    }
+                };
+#pragma unroll 1
+                for (int ch = 0; ch < 2; ++ch) {
+                    uint32_t r[32];
+                    tmem_ld32(taddr + ch * 32, r);
+                    if (ch == 1) {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive_cluster(cluster_address(&ctrl->acc_empty[b], 0));
+                    }
+                    test(r, ch);
+                }
+            }
+            if (ok && lane == 0 && listed) my_offs[(p.k + 1023) / 1024] = filled;
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();   // nothing of the pair is in flight towards this CTA any more
+    if (warp == 1) tmem_dealloc_pair(tmem_base, TMEM_COLS);
+}
+
+// Power of two that maps a vector of this squared norm into [-2^14, 2^14]: hi and lo then hold 22 bits of every element down
+// to 2^-17 of the norm, and smaller ones to 2^-39 of it.
+__device__ __forceinline__ float split_scale(float sqnorm) {
+    if (!(sqnorm > 1e-36f) || !(sqnorm < 3e38f)) return 1.0f;
+    int e;
+    frexpf(sqrtf(sqnorm), &e);
+    return ldexpf(1.0f, 14 - e);
+}
+
+// (rows are 16-byte aligned and a multiple of 4 long, as everywhere on the tensor-core path)
+__device__ __forceinline__ float4 leading_columns(const float* __restrict__ row, uint32_t j, uint32_t cols) {
+    if (j >= cols) return make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v = __ldg(reinterpret_cast<const float4*>(row + j));
+    if (j + 1 >= cols) v.y = 0.f;
+    if (j + 2 >= cols) v.z = 0.f;
+    if (j + 3 >= cols) v.w = 0.f;
+    return v;
+}
+
+__device__ __forceinline__ void split_half_row(const float* __restrict__ row, uint32_t cols, uint32_t pitch, float scale, __half* __restrict__ hi, __half* __restrict__ lo, int lane) {
+    for (uint32_t j = 4 * lane; j < pitch; j += 128) {
+        const float4 v4 = leading_columns(row, j, cols);
+        const float v[4] = {v4.x * scale, v4.y * scale, v4.z * scale, v4.w * scale};
+        __align__(8) __half h[4], l[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            h[q] = __float2half_rn(v[q]);
+            l[q] = __float2half_rn(v[q] - __half2float(h[q]));
+        }
+        *reinterpret_cast<uint2*>(hi + j) = *reinterpret_cast<const uint2*>(h);
+        *reinterpret_cast<uint2*>(lo + j) = *reinterpret_cast<const uint2*>(l);
+    }
+}
+
+// The first `cols` columns of the points, a scale per row; one warp per row.
+__global__ void __launch_bounds__(256) split_points_kernel(const float* __restrict__ x, size_t n, size_t d, uint32_t cols, uint32_t pitch, __half* __restrict__ hi,
+                                                           __half* __restrict__ lo, float* __restrict__ factor) {
+    const size_t row = static_cast<size_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+    if (row >= n) return;
+    const int lane = threadIdx.x & 31;
+    const float* xr = x + row * d;
+    float s = 0.f;
+    for (uint32_t j = 4 * lane; j < cols; j += 128) {
+        const float4 v = leading_columns(xr, j, cols);
+        s = fmaf(v.x, v.x, s); s = fmaf(v.y, v.y, s); s = fmaf(v.z, v.z, s); s = fmaf(v.w, v.w, s);
+    }
+    const float scale = split_scale(warp_sum(s));
+    split_half_row(xr, cols, pitch, scale, hi + row * pitch, lo + row * pitch, lane);
+    if (lane == 0) factor[row] = -2.0f / scale;
+}
+
+// The centroids, one scale for all: every block finds the largest of the k squared norms over the columns in question.
+__global__ void __launch_bounds__(256) split_centroids_kernel(const float* __restrict__ y, size_t k, size_t d, uint32_t cols, uint32_t pitch, const float* __restrict__ norms,
+                                                              __half* __restrict__ hi, __half* __restrict__ lo, float* __restrict__ factor) {
+    __shared__ float part[8];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float m = 0.f;
+    for (size_t c = threadIdx.x; c < k; c += 256) m = fmaxf(m, __ldg(norms + c));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane == 0) part[warp] = m;
+    __syncthreads();
+    m = part[0];
+    for (int w = 1; w < 8; ++w) m = fmaxf(m, part[w]);
+    const float scale = split_scale(m);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *factor = 1.0f / scale;
+    for (size_t c = static_cast<size_t>(blockIdx.x) * 8 + warp; c < k; c += static_cast<size_t>(gridDim.x) * 8)
+        split_half_row(y + c * d, cols, pitch, scale, hi + c * pitch, lo + c * pitch, lane);
+}
+
+} // namespace
+
+void launch_split_points(const float* x, size_t n, size_t d, uint32_t cols, const SplitHalves& out, cudaStream_t stream) {
+    if (n == 0) return;
+    split_points_kernel<<<static_cast<unsigned>((n + 7) / 8), 256, 0, stream>>>(x, n, d, cols, out.pitch, out.hi, out.lo, out.factor);
+    SKM_LAUNCH_CHECK();
+}
+
+void launch_split_centroids(const float* y, size_t k, size_t d, uint32_t cols, const float* norms, const SplitHalves& out, cudaStream_t stream) {
+    if (k == 0) return;
+    split_centroids_kernel<<<static_cast<unsigned>(std::min<size_t>(296, (k + 7) / 8)), 256, 0, stream>>>(y, k, d, cols, out.pitch, norms, out.hi, out.lo, out.factor);
+    SKM_LAUNCH_CHECK();
+}
+
+void launch_first_test(const SplitHalves& x, const SplitHalves& y, size_t n, size_t k, uint32_t partial_d, const float* norms_x, const float* norms_y, const float* best_in,
+                       const uint32_t* skip, float ratio_first, size_t tile0, size_t n_tiles, uint2* lists, uint32_t* list_offs, uint32_t cap_group, cudaStream_t stream,
+                       const uint32_t* tile_map) {
+    if (n_tiles == 0 || k == 0) return;
+    int device = 0, sms = 0;
+    SKM_CUDA(cudaGetDevice(&device));
+    SKM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    TestMaps maps;
+    maps.xhi = make_half_tmap(x.hi, partial_d, n, 128, x.pitch);
+    maps.xlo = make_half_tmap(x.lo, partial_d, n, 128, x.pitch);
+    maps.yhi = make_half_tmap(y.hi, partial_d, k, 128, y.pitch);
+    maps.ylo = make_half_tmap(y.lo, partial_d, k, 128, y.pitch);
+    TestParams p{};
+    p.n = n;
+    p.k = k;
+    p.k_blocks = (partial_d + TK - 1) / TK;
+    p.tile0 = tile0;
+    p.n_tiles = n_tiles;
+    p.tile_map = tile_map;
+    p.factor_x = x.factor;
+    p.factor_y = y.factor;
+    p.norms_x = norms_x;
+    p.norms_y = norms_y;
+    p.best_in = best_in;
+    p.skip = skip;
+    p.ratio_first = ratio_first;
+    p.lists = lists;
+    p.list_offs = list_offs;
+    p.cap_group = cap_group;
+    p.error = error_word();
+    p.wait_limit = wait_limit();
+    SKM_CUDA(cudaFuncSetAttribute(first_test_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(T_SMEM_BYTES)));
+    const unsigned grid = static_cast<unsigned>(2 * std::min<size_t>(static_cast<size_t>(sms / 2), (n_tiles + 1) / 2));
+    first_test_kernel<<<grid, T_THREADS, T_SMEM_BYTES, stream>>>(maps, p);
+    SKM_LAUNCH_CHECK();
+}
+
+} // namespace tc
+} // namespace skmb

@@ -14,8 +14,8 @@
 //                beside it (element-wise, so the swizzle pattern never has to be decoded);
 //   warps 6-9    epilogue: tcgen05.ld, one thread per row.  Three epilogues: the two smallest
 //                ||x||^2 + ||y||^2 - 2 x.y per row (exact assignment), a plain store, and the first ADSampling
-//                test with survivor lists;
-//   warps 10-13  second half of the epilogue warps in the first-test mode (idle otherwise).
+//                test as union bits or counts (its lists: kernels_first_test.cu);
+//   warps 10-13  second half of the epilogue warps in the union and counting modes (idle otherwise).
 // chain_tc_kernel (320 threads, same roles) grows its accumulators segment by segment and tests after each.
 // Rows / columns / k beyond the matrix edges are zero-filled by TMA, so any n, k and K work as long as the row
 // pitch is a multiple of 16 bytes.
@@ -52,19 +52,14 @@ struct Params {
     size_t ldo;
     int* error;
     long long wait_limit;   // SM cycles after which a wait gives up
-    // first-test epilogue (MODE_PRUNE): rows [tile0 * 128, (tile0 + n_tiles) * 128) are processed; norms_x / norms_y
+    // union and counting epilogues: rows [tile0 * 128, (tile0 + n_tiles) * 128) are processed; norms_x / norms_y
     // hold the norms over the first kdim dimensions
     size_t tile0;
     size_t n_tiles;        // 0 = all row tiles (other modes)
     const float* best_in;  // n: exact distance to the previous centroid
     const uint32_t* skip;  // n or null: 1 = row handled elsewhere
     float ratio_first;     // ratios[kdim]
-    // eight lists per row tile: list (h * 4 + q) holds the pairs of rows 32q..32q+31 with the centroids of columns
-    // 128h..128h+127 of every 256-column tile; entries {centroid << 5 | row in the 32-row group, partial distance}
-    uint2* lists;
-    uint32_t* list_offs;   // per list: (n_chunks + 1) entry counts at the start of every 1024-centroid chunk
-    uint32_t cap_group;    // capacity of one list
-    // first-test and union modes: when set, entry t of the launch's tile range works on row tile tile_map[t]
+    // union mode: when set, entry t of the launch's tile range works on row tile tile_map[t]
     // (rows tile_map[t] * 128 ...) instead of row tile tile0 + t; lists and union words stay indexed by t
     const uint32_t* tile_map;
     // union epilogue (MODE_UNION): bit c of union_bits[t * union_words + c / 32] is set when at least one row of the
@@ -84,7 +79,7 @@ struct Params {
     uint32_t debug_producer_stop;
 };
 
-enum { MODE_ARGMIN = 0, MODE_STORE = 1, MODE_PRUNE = 2, MODE_UNION = 3, MODE_COUNT = 4 };
+enum { MODE_ARGMIN = 0, MODE_STORE = 1, MODE_UNION = 2, MODE_COUNT = 3 };
 constexpr float kUnionSlack = 1.0f / 512.0f;   // see the union epilogue
 
 template <int MODE>
@@ -107,7 +102,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_tc_kernel(const __grid_co
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&ctrl->tmem_full[b], 1);
-            mbar_init(&ctrl->tmem_empty[b], (MODE == MODE_PRUNE || MODE == MODE_UNION || MODE == MODE_COUNT) ? 256 : 128);
+            mbar_init(&ctrl->tmem_empty[b], (MODE == MODE_UNION || MODE == MODE_COUNT) ? 256 : 128);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_proxy_async();
@@ -118,7 +113,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_tc_kernel(const __grid_co
     tc_fence_after();
     const uint32_t tmem_base = ctrl->tmem_base;
 
-    constexpr bool kTiled = (MODE == MODE_PRUNE || MODE == MODE_UNION || MODE == MODE_COUNT);   // works on a given range / list of row tiles
+    constexpr bool kTiled = (MODE == MODE_UNION || MODE == MODE_COUNT);   // works on a given range / list of row tiles
     const size_t rt_begin = kTiled ? p.tile0 : 0;
     const size_t n_row_tiles = kTiled ? p.tile0 + p.n_tiles : (p.n + BM - 1) / BM;
     // row tile that entry rt of the loops below stands for
@@ -236,7 +231,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_tc_kernel(const __grid_co
         }
     } else if (warp < 10 || kTiled) {
         // ---------------------------------------------------------------- epilogue
-        // First-test mode: eight warps, two per quarter of the tile's rows; warps 6-9 take columns 0-127 of
+        // Union and counting modes: eight warps, two per quarter of the tile's rows; warps 6-9 take columns 0-127 of
         // every 256-column tile, warps 10-13 columns 128-255, each with a candidate list of its own.
         const uint32_t half = kTiled ? static_cast<uint32_t>(warp - 6) >> 2 : 0u;
         const uint32_t lane_base = 32u * (warp & 3);    // tensor-memory lanes this warp may read
@@ -252,17 +247,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_tc_kernel(const __grid_co
             float nx = 0.f, d1 = FLT_MAX, d2 = FLT_MAX;
             uint32_t i1 = 0, i2 = 0xFFFFFFFFu;
             if ((MODE == MODE_ARGMIN || kTiled) && row_valid) nx = p.norms_x[row];
-            // first-test epilogue: this warp's 32 rows share one candidate list; `filled` is warp-uniform
             float thr = -FLT_MAX;
-            uint32_t filled = 0;
-            uint2* my_list = nullptr;
-            uint32_t* my_offs = nullptr;
-            if (MODE == MODE_PRUNE) {
-                const size_t group = (rt - rt_begin) * 8 + half * 4 + (warp & 3);
-                my_list = p.lists + group * p.cap_group;
-                my_offs = p.list_offs + group * ((p.k + 1023) / 1024 + 1);
-                if (row_valid && !(p.skip && p.skip[row])) thr = p.best_in[row] * p.ratio_first;
-            }
             uint32_t* my_union = nullptr;
             if (MODE == MODE_UNION) {
                 my_union = p.union_bits + (rt - rt_begin) * static_cast<size_t>(p.union_words);
@@ -280,7 +265,6 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_tc_kernel(const __grid_co
                 const uint32_t b = t & 1u, tph = (t >> 1) & 1u;
                 const size_t col0 = static_cast<size_t>(nt) * BN;
                 float* ny = ctrl->ny[warp & 3][b];
-                if (MODE == MODE_PRUNE && (nt & 3u) == 0 && lane == 0) my_offs[nt >> 2] = filled;
                 if (MODE == MODE_COUNT && (nt & 3u) == 0) thr = row_valid ? __ldg(p.thr_rows + row * p.thr_chunks + (nt >> 2)) : -FLT_MAX;
                 if (MODE == MODE_ARGMIN) {
                     // each warp keeps its own copy, so no cross-warp barrier is needed
@@ -357,86 +341,6 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_tc_kernel(const __grid_co
                         const uint32_t n_valid = first >= p.k ? 0u : static_cast<uint32_t>(min(static_cast<size_t>(32), p.k - first));
                         mask &= n_valid >= 32u ? 0xFFFFFFFFu : ((1u << n_valid) - 1u);
                         counted += __popc(mask);
-                    } else if (MODE == MODE_PRUNE) {
-                        // test of the first checkpoint for 32 centroids, then a warp scan places every row's
-                        // survivors behind those of the lower lanes
-                        uint32_t mask = 0;
-#pragma unroll
-                        for (int j = 0; j < 32; j += 4) {
-                            const float4 nyv = *reinterpret_cast<const float4*>(ny + ch * 32 + j);
-                            const float p0 = fmaf(-2.0f, __uint_as_float(r[j + 0]), nx) + nyv.x;
-                            const float p1 = fmaf(-2.0f, __uint_as_float(r[j + 1]), nx) + nyv.y;
-                            const float p2 = fmaf(-2.0f, __uint_as_float(r[j + 2]), nx) + nyv.z;
-                            const float p3 = fmaf(-2.0f, __uint_as_float(r[j + 3]), nx) + nyv.w;
-                            r[j + 0] = __float_as_uint(p0);
-                            r[j + 1] = __float_as_uint(p1);
-                            r[j + 2] = __float_as_uint(p2);
-                            r[j + 3] = __float_as_uint(p3);
-                            mask |= (p0 < thr ? (1u << j) : 0u) | (p1 < thr ? (2u << j) : 0u) | (p2 < thr ? (4u << j) : 0u) | (p3 < thr ? (8u << j) : 0u);
-                        }
-                        {
-                            // columns past the last centroid (zero-filled by TMA) never count
-                            const size_t first = col0 + static_cast<size_t>(ch) * 32;
-                            const uint32_t n_valid = first >= p.k ? 0u : static_cast<uint32_t>(min(static_cast<size_t>(32), p.k - first));
-                            mask &= n_valid >= 32u ? 0xFFFFFFFFu : ((1u << n_valid) - 1u);
-                        }
-                        const uint32_t cnt = __popc(mask);
-                        uint32_t incl = cnt;
-#pragma unroll
-                        for (int off = 1; off < 32; off <<= 1) {
-                            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, off);
-                            if (lane >= off) incl += v;
-                        }
-                        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-                        if (total != 0) {
-                            const uint32_t colbits = static_cast<uint32_t>(col0 + ch * 32) << 5;
-                            if (total <= STAGE_ENTRIES) {
-                                // survivors are packed in shared memory first (predicated stores, no divergence) and
-                                // leave for global memory as contiguous runs
-                                uint2* stg = reinterpret_cast<uint2*>(smem + STAGES * STAGE_BYTES + SMEM_CTRL_BYTES) + (warp - 6) * STAGE_ENTRIES;
-                                // slot of column j = this lane's first slot + number of its survivors below j: no chain
-                                // of dependent additions through the 32 columns
-                                const uint32_t base = incl - cnt;
-#pragma unroll
-                                for (int j = 0; j < 32; ++j) {
-                                    if ((mask >> j) & 1u) stg[base + __popc(mask & ((1u << j) - 1u))] = make_uint2((colbits + (static_cast<uint32_t>(j) << 5)) | lane, r[j]);
-                                }
-                                __syncwarp();
-                                for (uint32_t i = lane; i < total; i += 32)
-                                    if (filled + i < p.cap_group) my_list[filled + i] = stg[i];
-                                __syncwarp();
-                            } else {
-                                // dense case (more than a quarter of the 32 x 32 block passes): eight columns at a time,
-                                // which always fit in the staging area
-                                uint2* stg = reinterpret_cast<uint2*>(smem + STAGES * STAGE_BYTES + SMEM_CTRL_BYTES) + (warp - 6) * STAGE_ENTRIES;
-                                uint32_t done = 0;
-#pragma unroll
-                                for (int sb = 0; sb < 4; ++sb) {
-                                    const uint32_t sub = (mask >> (8 * sb)) & 0xFFu;
-                                    const uint32_t c8 = __popc(sub);
-                                    uint32_t in8 = c8;
-#pragma unroll
-                                    for (int off = 1; off < 32; off <<= 1) {
-                                        const uint32_t v = __shfl_up_sync(0xffffffffu, in8, off);
-                                        if (lane >= off) in8 += v;
-                                    }
-                                    const uint32_t tot8 = __shfl_sync(0xffffffffu, in8, 31);
-                                    uint32_t pos = in8 - c8;
-#pragma unroll
-                                    for (int j = 8 * sb; j < 8 * sb + 8; ++j) {
-                                        const uint32_t bit = (mask >> j) & 1u;
-                                        if (bit) stg[pos] = make_uint2((colbits + (static_cast<uint32_t>(j) << 5)) | lane, r[j]);
-                                        pos += bit;
-                                    }
-                                    __syncwarp();
-                                    for (uint32_t i = lane; i < tot8; i += 32)
-                                        if (filled + done + i < p.cap_group) my_list[filled + done + i] = stg[i];
-                                    __syncwarp();
-                                    done += tot8;
-                                }
-                            }
-                            filled += total;
-                        }
                     } else if (row_valid) {
                         float* orow = p.out + row * p.ldo + col0 + ch * 32;
                         const size_t left = (col0 + ch * 32 < p.k) ? (p.k - (col0 + ch * 32)) : 0;
@@ -456,7 +360,6 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_tc_kernel(const __grid_co
                 mbar_arrive(&ctrl->tmem_empty[b]);
             }
             if (MODE == MODE_ARGMIN && ok && row_valid) p.out_top2[row] = make_uint2(i1, i2);
-            if (MODE == MODE_PRUNE && ok && lane == 0) my_offs[(n_col_tiles + 3) / 4] = filled;
             if (MODE == MODE_COUNT && ok && row_valid && counted != 0) atomicAdd(p.count_out + row, counted);   // the row's other half adds its own
         }
     }
@@ -1191,8 +1094,8 @@ bool wait_injected() { return g_debug_producer_stop != 0; }
 
 void launch_presplit(const float* y, size_t rows, size_t ld, float* y_split, cudaStream_t stream) { presplit(y, rows, ld, y_split, stream); }
 
-CUtensorMap make_half_tmap(const void* base, size_t cols, size_t rows, uint32_t box_rows) {
-    return make_tmap_of(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, CU_TENSOR_MAP_SWIZZLE_128B, base, cols, rows, cols, 64, box_rows);
+CUtensorMap make_half_tmap(const void* base, size_t cols, size_t rows, uint32_t box_rows, size_t pitch) {
+    return make_tmap_of(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, CU_TENSOR_MAP_SWIZZLE_128B, base, cols, rows, pitch ? pitch : cols, 64, box_rows);
 }
 
 CUtensorMap make_row_major_tmap(const float* base, size_t extent, size_t rows, size_t ld, uint32_t box_rows) { return make_tmap(base, extent, rows, ld, box_rows); }
@@ -1259,40 +1162,6 @@ void launch_assign_full_flagged(const float* x, const float* y, size_t n, size_t
     p.wait_limit = g_wait_limit;
     launch<MODE_ARGMIN>(tx, ty, ty, p, stream);
     refine_top2_kernel<<<static_cast<unsigned>((n + 7) / 8), 256, 0, stream>>>(x, y, n, k, d, norms_x, norms_y, top2_scratch, out_knn, out_dist, p.error);
-    note_kernel_launch();
-    SKM_CUDA(cudaGetLastError());
-}
-
-void launch_first_test(const float* x, const float* y, size_t n, size_t k, size_t d, uint32_t partial_d, const float* norms_x, const float* norms_y, const float* best_in,
-                       const uint32_t* skip, float ratio_first, size_t tile0, size_t n_tiles, uint2* lists, uint32_t* list_offs, uint32_t cap_group, cudaStream_t stream,
-                       const float* y_split, const uint32_t* tile_map) {
-    if (n_tiles == 0 || k == 0) return;
-    int device = 0;
-    SKM_CUDA(cudaGetDevice(&device));
-    const CUtensorMap tx = make_tmap(x, partial_d, n, d, BM);
-    const CUtensorMap ty = make_tmap(y_split ? y_split : y, partial_d, k, d, BN);
-    const CUtensorMap tylo = y_split ? make_tmap(y_split + k * d, partial_d, k, d, BN) : ty;
-    Params p{};
-    p.y_presplit = y_split != nullptr;
-    p.n = n;
-    p.k = k;
-    p.kdim = partial_d;
-    p.norms_x = norms_x;
-    p.norms_y = norms_y;
-    p.error = error_flag(device);
-    p.wait_limit = g_wait_limit;
-    p.tile0 = tile0;
-    p.n_tiles = n_tiles;
-    p.best_in = best_in;
-    p.skip = skip;
-    p.ratio_first = ratio_first;
-    p.lists = lists;
-    p.list_offs = list_offs;
-    p.cap_group = cap_group;
-    p.tile_map = tile_map;
-    SKM_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<MODE_PRUNE>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SMEM_BYTES)));
-    const int grid = static_cast<int>(std::min<size_t>(n_tiles, static_cast<size_t>(sm_count(device))));
-    gemm_tc_kernel<MODE_PRUNE><<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(tx, ty, tylo, p);
     note_kernel_launch();
     SKM_CUDA(cudaGetLastError());
 }

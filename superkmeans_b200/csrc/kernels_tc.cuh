@@ -1,6 +1,7 @@
 // Tensor-core (tcgen05 + TMA) variants of the dense kernels; see kernels_tc.cu.
 #pragma once
 
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <cstddef>
@@ -34,16 +35,28 @@ void launch_gemm_nt(const float* a, size_t lda, const float* b, size_t ldb, floa
 void launch_rotate(const float* a, size_t lda, const float* b, size_t ldb, float* out, size_t ldo, size_t n, size_t n_out, size_t k_dim, float* out_sqnorms,
                    cudaStream_t stream);
 
-// First ADSampling test on the tensor cores for the row tiles [tile0, tile0 + n_tiles) of 128 points: partial
-// distances over the first partial_d dimensions of every (point, centroid) pair, tested against
-// best_in * ratio_first.  Pairs that pass go to one of eight lists per row tile (list h * 4 + q: rows 32q..32q+31,
-// columns 128h..128h+127 of every 256-centroid tile) as {centroid << 5 | row in the 32-row group, partial
+// The leading columns of a row-major fp32 matrix as fp16 pairs: element * scale = hi + lo to 22 bits, scale a power of two.
+// For points a scale per row (factor[row] = -2 / scale), for centroids one for all (factor[0] = 1 / scale).
+struct SplitHalves {
+    __half* hi;       // rows x pitch
+    __half* lo;
+    float* factor;
+    uint32_t pitch;   // halves per row, a multiple of 8
+};
+void launch_split_points(const float* x, size_t n, size_t d, uint32_t cols, const SplitHalves& out, cudaStream_t stream);
+// norms: squared norms over at least the columns that will be used
+void launch_split_centroids(const float* y, size_t k, size_t d, uint32_t cols, const float* norms, const SplitHalves& out, cudaStream_t stream);
+
+// First ADSampling test on the tensor cores (kernels_first_test.cu) for the row tiles [tile0, tile0 + n_tiles) of 128
+// points: partial distances over the first partial_d dimensions of every (point, centroid) pair, tested against
+// best_in * ratio_first.  Pairs that pass go to one of sixteen lists per row tile (list c * 4 + q: rows 32q..32q+31,
+// columns 64c..64c+63 of every 256-centroid tile) as {centroid << 5 | row in the 32-row group, partial
 // distance}, at most cap_group entries per list, in centroid-tile order; list_offs receives, per list, the number
 // of entries before every 1024-centroid chunk and the total (which exceeds cap_group on overflow).
-void launch_first_test(const float* x, const float* y, size_t n, size_t k, size_t d, uint32_t partial_d, const float* norms_x, const float* norms_y, const float* best_in,
+// tile_map (optional): entry t of the range stands for row tile tile_map[t]; lists stay indexed by t.
+void launch_first_test(const SplitHalves& x, const SplitHalves& y, size_t n, size_t k, uint32_t partial_d, const float* norms_x, const float* norms_y, const float* best_in,
                        const uint32_t* skip, float ratio_first, size_t tile0, size_t n_tiles, uint2* lists, uint32_t* list_offs, uint32_t cap_group, cudaStream_t stream,
-                       const float* y_split = nullptr,   // y already split by launch_presplit, optional
-                       const uint32_t* tile_map = nullptr);   // optional: entry t of the range stands for row tile tile_map[t]; lists stay indexed by t
+                       const uint32_t* tile_map = nullptr);
 
 // The same first test (threshold widened by 1e-4 relative) for the row tiles tile_map[0 .. n_tiles), keeping only its
 // footprint: bit c of union_bits[t * union_words + c / 32] is set (atomic OR into zeroed memory) when some row of tile t

@@ -14,16 +14,14 @@ constexpr int BM = 128;
 constexpr int BN = 256;
 constexpr int BK = 16;
 constexpr int STAGES = 4;
-constexpr int NUM_THREADS = 448;   // warps 10-13 work only in the first-test epilogue and in no other mode
+constexpr int NUM_THREADS = 448;   // warps 10-13 work only in the union and counting epilogues
 constexpr uint32_t A_TILE_BYTES = BM * BK * 4;   // 8192
 constexpr uint32_t B_TILE_BYTES = BN * BK * 4;   // 16384
 constexpr uint32_t STAGE_BYTES = 2 * A_TILE_BYTES + 2 * B_TILE_BYTES;  // 49152
 constexpr uint32_t OFF_A_HI = 0, OFF_A_LO = A_TILE_BYTES, OFF_B_HI = 2 * A_TILE_BYTES, OFF_B_LO = 2 * A_TILE_BYTES + B_TILE_BYTES;
 constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t SMEM_CTRL_BYTES = 9216;
-constexpr uint32_t STAGE_ENTRIES = 256;   // per epilogue warp, first-test epilogue
-constexpr uint32_t SMEM_STAGE_BYTES = 8 * STAGE_ENTRIES * 8;
-constexpr uint32_t SMEM_BYTES = STAGES * STAGE_BYTES + SMEM_CTRL_BYTES + SMEM_STAGE_BYTES + 1024;  // + alignment slack
+constexpr uint32_t SMEM_BYTES = STAGES * STAGE_BYTES + SMEM_CTRL_BYTES + 1024;  // + alignment slack
 constexpr long long WAIT_LIMIT_CYCLES = 4000000000LL;
 // Where a kernel records that a wait ran out, and after how many SM clock cycles a wait gives up.  The limit travels
 // in the kernel parameters (host side: wait_limit()) so that a test can shorten it and watch a wait run out in
@@ -254,8 +252,9 @@ __device__ __forceinline__ void split4(float4 v, float4& hi, float4& lo) {
 
 // Row-major fp32 matrix [rows][ld] of which the first `extent` columns are visible; boxes of 16 columns x box_rows
 // rows, 64-byte swizzle, zero fill outside (defined in kernels_tc.cu).
-// Row-major fp16 matrix [rows][cols] (cols a multiple of 8); boxes of 64 columns x box_rows rows, 128-byte swizzle.
-CUtensorMap make_half_tmap(const void* base, size_t cols, size_t rows, uint32_t box_rows);
+// Row-major fp16 matrix [rows][pitch] (pitch a multiple of 8, 0: cols) of which the first cols columns are visible; boxes of
+// 64 columns x box_rows rows, 128-byte swizzle, zero fill outside.
+CUtensorMap make_half_tmap(const void* base, size_t cols, size_t rows, uint32_t box_rows, size_t pitch = 0);
 CUtensorMap make_row_major_tmap(const float* base, size_t extent, size_t rows, size_t ld, uint32_t box_rows);
 
 } // namespace tc
