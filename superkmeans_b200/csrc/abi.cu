@@ -148,8 +148,7 @@ int skm_last_prune_path(const skm_handle* h) { return (h && h->engine) ? h->engi
 skm_status skm_get_prune_counters(const skm_handle* h, uint64_t* out3) {
     SKM_NEED(h);
     if (!out3) return SKM_INVALID_ARGUMENT;
-    h->engine->prune_counters(out3);
-    return SKM_OK;
+    return guarded(g_op_error, [&] { h->engine->prune_counters(out3); });
 }
 skm_status skm_get_chain_counters(const skm_handle* h, uint64_t* out4) {
     SKM_NEED(h);

@@ -133,7 +133,8 @@ struct PrunedParams {
     uint32_t partial_d, vertical_d, horizontal_d;
     const float* best_in = nullptr;     // optional: exact distance to the previous centroid, per point
     const uint32_t* skip = nullptr;     // optional: 1 = leave this point to the dense kernel
-    bool same_points = false;           // x holds what it held in the pass before (its fp16 halves can be used again)
+    bool same_points = false;           // x holds what it held in the pass before (its fp16 halves can be used again), in which
+    double survival = 0.0;              // this share of the pairs passed the first test (says what a sample says otherwise)
 };
 
 // Work split of one pruned pass.  Points whose ADSampling test would keep a large share of the
@@ -152,10 +153,17 @@ struct PruneSplitWorkspace {
     float* sample_norms = nullptr;  // 128
     float* chain_norms_y = nullptr; // k x n_checkpoints
     uint32_t* n_hard_dev = nullptr; // 1
-    unsigned long long* alive_total = nullptr;  // 1: sampled pairs passing the first test
-    int n_sample = 128;
+    unsigned long long* alive_total = nullptr;  // 2: sampled pairs passing the first test, sampled points
     float ratio_first = 1.0f;       // ratios[partial_d], host copy
     uint32_t flag_mult = 16;        // a point is flagged when survivors * flag_mult >= n_sample
+};
+// What a pruned pass counts on the device.
+struct PrunePassCounters {
+    unsigned long long alive;       // pairs of the sampled points and centroids that passed the first test
+    unsigned long long sampled;     // points of that sample
+    uint32_t n_hard;                // points listed in hard_idx
+    uint32_t n_dropped;             // points that the first test dropped
+    uint32_t n_redo;                // points whose candidate list overflowed
 };
 size_t prune_split_positions_elems(size_t n);
 uint32_t prune_chain_checkpoints(uint32_t partial_d, uint32_t vertical_d, uint32_t horizontal_d);
@@ -165,7 +173,7 @@ void launch_exact_dist(const float* x, const float* y, const uint32_t* knn, size
 // out[j][row] when `transposed`.
 void launch_chain_norms(const float* m, size_t rows, size_t d, uint32_t partial_d, uint32_t vertical_d, uint32_t horizontal_d, bool transposed, float* out,
                         cudaStream_t stream);
-// Fills ws.best and ws.flags / ws.hard_idx / *ws.n_hard_dev.
+// Fills ws.best, ws.flags, ws.hard_idx (in any order), *ws.n_hard_dev and *ws.alive_total (both zero before).
 void launch_pruned_prepare(const PrunedParams& p, PruneSplitWorkspace& ws, cudaStream_t stream);
 // Runs the dense chain for the n_hard points listed in ws.hard_idx.
 void launch_assign_pruned_dense(const PrunedParams& p, PruneSplitWorkspace& ws, size_t n_hard, cudaStream_t stream);
@@ -243,7 +251,8 @@ void launch_scatter_sorted(const uint32_t* order, size_t cnt, const uint32_t* kn
 void launch_tile_flags(const uint32_t* row_flags, size_t n, uint32_t threshold, uint32_t* tile_flags, cudaStream_t stream);
 void launch_init_chain_rows(const uint32_t* tile_map, size_t n_tiles, size_t n, const uint32_t* prev, const float* best, uint32_t* knn, float* dist, uint32_t* not_pruned,
                             uint2* top2, cudaStream_t stream);
-void launch_classify(const PrunedParams& p, PruneSplitWorkspace& ws, cudaStream_t stream);
+// ... of every step-th tile of points, the only ones whose flags it then sets.
+void launch_classify(const PrunedParams& p, PruneSplitWorkspace& ws, cudaStream_t stream, size_t step = 1);
 void launch_iota_u32(uint32_t* out, size_t n, cudaStream_t stream);   // out[i] = i
 
 // k nearest rows of y for every row of q by ||q||^2 + ||y||^2 - 2 q.y (BatchComputer::FindKNearestNeighbors,
@@ -270,7 +279,7 @@ struct UpdateWorkspace {
     uint32_t* digit_table = nullptr;  // 256 * n_units
     uint32_t* seg_offsets = nullptr;  // k + 1
     float* tile_partials = nullptr;   // n_tiles * 2 * d
-    double* block_sums = nullptr;     // reduction partials (>= 1024)
+    double* reduce_scratch = nullptr; // kReduceScratchDoubles
     size_t n_cap = 0, k_cap = 0, d = 0;
 };
 // sizes of digit_table (256 per unit) and tile_partials (2 d per tile) for up to n points
@@ -281,25 +290,53 @@ size_t update_tiles(size_t n);
 // value buffers (keys_a/b, vals_a/b, digit_table must be allocated for n).
 void launch_sort_by_key(const uint32_t* keys, size_t n, size_t k, UpdateWorkspace& ws, const uint32_t** sorted_keys_out, const uint32_t** order_out, cudaStream_t stream);
 
-// counts[c] = |{i : assign[i] == c}|, sums[c] = sum of x rows assigned to c (deterministic order),
-// *wcss = sum_i dist[i] (double), *not_pruned_total = sum_i not_pruned[i] (may be null).
-void launch_update(const float* x, const uint32_t* assign, const float* dist, const uint32_t* not_pruned, size_t n, size_t k, size_t d, UpdateWorkspace& ws, float* sums, uint32_t* counts, double* wcss, unsigned long long* not_pruned_total, cudaStream_t stream);
+// What an iteration tells the host, in one copy.
+struct IterationReport {
+    double wcss;                    // this and the next are summed over the shards
+    double not_pruned;              // pairs that passed the first test
+    double shift;
+    int error;                      // of the tensor-core kernels (tc::error_word)
+};
+// Where the report's fields other than `shift` come from.
+struct UpdateStats {
+    const float* dist = nullptr;
+    const uint32_t* not_pruned = nullptr;      // null: an exact pass
+    const int* error = nullptr;                // may be null
+    IterationReport* report = nullptr;
+};
+// Partial sums of a reduction over the grid and the ticket of its last block (which leaves it at zero): all zero at first.
+constexpr size_t kReduceScratchDoubles = 2 * 512 + 1;
 
-// c[i][:] *= 1/counts[i] for non-empty clusters
-void launch_scale_by_counts(float* c, const uint32_t* counts, size_t k, size_t d, cudaStream_t stream);
+// counts[c] = |{i : assign[i] == c}|, sums[c] = sum of x rows assigned to c (deterministic order); `stats`, if given: the
+// report's fields other than `shift`.
+void launch_update(const float* x, const uint32_t* assign, size_t n, size_t k, size_t d, UpdateWorkspace& ws, float* sums, uint32_t* counts, const UpdateStats* stats, cudaStream_t stream);
 
 struct SplitOpDev {
     uint32_t dst, src, kind;
     float wc;
 };
 void launch_apply_split_ops(float* c, size_t d, const SplitOpDev* ops, size_t n_ops, cudaStream_t stream);
-void launch_normalize_rows(float* c, size_t k, size_t d, cudaStream_t stream);
 
 // PDX-blocked copy and first-vertical_d copy of a row-major k x d matrix
 void launch_pdxify(const float* c, float* pdx, float* aux, size_t k, size_t d, size_t vertical_d, cudaStream_t stream);
 
-// *out = sum_c ||a[c] - b[c]||^2
-void launch_shift(const float* a, const float* b, size_t k, size_t d, double* block_sums, double* out, cudaStream_t stream);
+// ConsolidateCentroids and ComputeShift (superkmeans.h:936-998) but for the splits, in one pass over c: rows times 1/counts
+// (counts null: done before), rows to unit length (normalize), the PDX copies, report->shift = sum of the
+// squared distances to prev.  With counts and normalize a matrix with an empty cluster (or splits to come) stops after the first
+// step: rows are normalized after the splits.
+struct ConsolidateParams {
+    float* c;
+    const float* prev;
+    const uint32_t* counts;
+    bool normalize;
+    bool splits_follow;   // with counts: clusters may be split that are not empty
+    float* pdx;
+    float* aux;
+    size_t k, d, vertical_d;
+    double* reduce_scratch;
+    IterationReport* report;
+};
+void launch_consolidate(const ConsolidateParams& p, cudaStream_t stream);
 
 // out[i][:] = in[idx[i]][:]; an index of all ones gives a row of zeros
 void launch_gather_rows(const float* in, const uint64_t* idx, float* out, size_t n_out, size_t d, cudaStream_t stream);

@@ -38,8 +38,6 @@ struct Entry {
     Entry(int device, cudaStream_t stream) : guard(device), work(stream) {}
 };
 
-__global__ void u64_to_f64_kernel(const unsigned long long* in, double* out) { *out = static_cast<double>(*in); }
-
 __global__ void widen_u32_kernel(const uint32_t* __restrict__ in, uint64_t* __restrict__ out, size_t n) {
     const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < n) out[i] = in[i];
@@ -170,9 +168,8 @@ Engine::Engine(const skm_config& cfg, size_t n_clusters, size_t d, bool hierarch
     WorkStream work(stream_);
     ratios_host_ = make_ratios(d, epsilon0_);
     SKM_CUDA(cudaMemcpyAsync(ratios_dev_.ensure(d + 1), ratios_host_.data(), sizeof(float) * (d + 1), cudaMemcpyHostToDevice, stream_));
-    scalars_dev_.ensure(8);
-    np_total_dev_.ensure(1);
-    scalars_host_.ensure(8);
+    report_dev_.ensure(1);
+    report_host_.ensure(1);
     if (hierarchical && n_clusters <= 128 && !cfg.suppress_warnings) {
         std::cout << "WARNING: n_clusters <= 128 is not recommended for HierarchicalSuperKMeans. "
                      "Consider using at least 128 clusters."
@@ -414,7 +411,8 @@ void Engine::prepare_update_workspace(size_t n, size_t k) {
     ws_.digit_table = ws_table_.ensure(256 * units + (256 * units) / 2048 + 64);
     ws_.seg_offsets = ws_offsets_.ensure(k + 1);
     ws_.tile_partials = ws_partials_.ensure(tiles * 2 * d_);
-    ws_.block_sums = ws_block_sums_.ensure(2048);
+    ws_.reduce_scratch = ws_reduce_.ensure(kReduceScratchDoubles);
+    SKM_CUDA(cudaMemsetAsync(ws_.reduce_scratch, 0, sizeof(double) * kReduceScratchDoubles, stream_));
     ws_.n_cap = n;
     ws_.k_cap = k;
     ws_.d = d_;
@@ -498,24 +496,30 @@ int prune_split_mode() { return g_prune_split_mode; }
 
 namespace {
 
-// The points listed in ws.hard_idx through the dense chain: on the tensor cores over a gathered copy of their
-// rows when `on_tensor_cores`, else with the SIMT kernel in place.
-void run_listed_dense(const PrunedParams& p, PruneSplitWorkspace& ws, PrunePassBuffers& b, size_t n_listed, bool on_tensor_cores, cudaStream_t stream) {
+// The points listed in ws.hard_idx through the dense chain on the tensor cores, over a gathered copy of their rows.  With a `side`
+// stream on that one, from where `stream` stands; the caller joins them (b.side_done).
+void run_listed_dense(const PrunedParams& p, PruneSplitWorkspace& ws, PrunePassBuffers& b, size_t n_listed, cudaStream_t stream, cudaStream_t side = nullptr) {
     if (n_listed == 0) return;
-    if (!on_tensor_cores) {
-        launch_assign_pruned_dense(p, ws, n_listed, stream);
-        return;
-    }
     const uint32_t n_ck = prune_chain_checkpoints(p.partial_d, p.vertical_d, p.horizontal_d);
     float* xl = b.listed_x.ensure(n_listed * p.d);
     float* bestl = b.listed_best.ensure(n_listed);
     uint32_t* knnl = b.listed_knn.ensure(n_listed);
-    launch_gather_listed(p.x, ws.best, p.knn, ws.hard_idx, n_listed, p.d, xl, bestl, knnl, stream);
-    launch_chain_norms(xl, n_listed, p.d, p.partial_d, p.vertical_d, p.horizontal_d, false, b.listed_norms.ensure(n_listed * n_ck), stream);
-    launch_chain_norms(p.y, p.k, p.d, p.partial_d, p.vertical_d, p.horizontal_d, true, ws.chain_norms_y, stream);
-    tc::launch_chain(xl, p.y, n_listed, p.k, p.d, p.partial_d, p.vertical_d, p.horizontal_d, b.listed_norms.get(), ws.chain_norms_y, p.ratios, bestl, knnl,
-                     b.listed_dist.ensure(n_listed), b.listed_np.ensure(n_listed), b.listed_top2.ensure(n_listed), b.y_split.ensure(2 * p.k * p.d), stream);
-    launch_scatter_listed(ws.hard_idx, n_listed, knnl, b.listed_dist.get(), b.listed_np.get(), p.knn, p.dist, p.not_pruned, stream);
+    float* normsl = b.listed_norms.ensure(n_listed * n_ck);
+    float* distl = b.listed_dist.ensure(n_listed);
+    uint32_t* npl = b.listed_np.ensure(n_listed);
+    uint2* top2l = b.listed_top2.ensure(n_listed);
+    float* y_split = b.y_split.ensure(2 * p.k * p.d);
+    const cudaStream_t s = side ? side : stream;
+    if (side) {
+        b.side_start.record(stream);
+        b.side_start.hold(side);
+    }
+    launch_gather_listed(p.x, ws.best, p.knn, ws.hard_idx, n_listed, p.d, xl, bestl, knnl, s);
+    launch_chain_norms(xl, n_listed, p.d, p.partial_d, p.vertical_d, p.horizontal_d, false, normsl, s);
+    launch_chain_norms(p.y, p.k, p.d, p.partial_d, p.vertical_d, p.horizontal_d, true, ws.chain_norms_y, s);
+    tc::launch_chain(xl, p.y, n_listed, p.k, p.d, p.partial_d, p.vertical_d, p.horizontal_d, normsl, ws.chain_norms_y, p.ratios, bestl, knnl, distl, npl, top2l, y_split, s);
+    launch_scatter_listed(ws.hard_idx, n_listed, knnl, distl, npl, p.knn, p.dist, p.not_pruned, s);
+    if (side) b.side_done.record(side);
 }
 
 } // namespace
@@ -587,14 +591,14 @@ void run_pruned_pass_sorted(const PrunedParams& p, PrunePassBuffers& b, float ra
     uint32_t* map_host = b.tile_map_host.ensure(2 * batch_tiles);
     unsigned long long* pair_steps = b.pair_steps_dev.ensure(1);
     unsigned long long* sparse_cols = b.sparse_cols_dev.ensure(1);
-    unsigned long long* counters_host = b.counters_host.ensure(2);
+    unsigned long long* counters_host = b.sorted_counters_host.ensure(2);
     SKM_CUDA(cudaMemsetAsync(pair_steps, 0, sizeof(unsigned long long), stream));
     SKM_CUDA(cudaMemsetAsync(sparse_cols, 0, sizeof(unsigned long long), stream));
 
     PruneSplitWorkspace ws;
     ws.sample = b.sample.ensure(128 * p.d);
     ws.sample_norms = b.sample_norms.ensure(128);
-    ws.alive_total = b.alive_total.ensure(1);
+    ws.alive_total = &b.counters.ensure(1)->alive;
     ws.ratio_first = ratio_first;
     ws.flag_mult = 22;   // a point is "expensive" from 6 of 128 sampled survivors up
     uint32_t dense_tile_rows = 16;   // a tile takes the chain when at least this many of its 128 points are expensive
@@ -809,7 +813,9 @@ void run_pruned_pass_sorted(const PrunedParams& p, PrunePassBuffers& b, float ra
                 const size_t nt = std::min(per, n_lists - t0);
                 {
                     SubPhase sub(timers, PH_PRUNE_FIRST_TEST, stream);
-                    tc::launch_first_test(xs, ys, cnt, p.k, p.partial_d, nx_b, p.norms_y, best_b, nullptr, ratio_first, 0, nt, lists, offs, cap_group, stream, map_lists + t0);
+                    tc::FirstTestRows rows;
+                    rows.tile_map = map_lists + t0;
+                    tc::launch_first_test(xs, ys, cnt, p.k, p.partial_d, nx_b, p.norms_y, best_b, ratio_first, 0, nt, lists, offs, cap_group, rows, stream);
                 }
                 WalkParams w{};
                 w.x = xb;
@@ -873,6 +879,11 @@ void run_pruned_pass_sorted(const PrunedParams& p, PrunePassBuffers& b, float ra
 
 } // namespace
 
+// A point that keeps one centroid in so many costs the walk more than a row of the dense chain.  One B200, ten iterations, with the
+// line at one in 44 / 22 / 16 / 12: first test + walk + chain of 1M x 1024, k = 4000: 73 / 63 / 59 / 57 ms; 250k x 1536, k = 2048:
+// 13.0 / 12.0 / 12.5 / 13.0; 30 000 x 768, k = 1000: 2.0 / 2.0 / 2.1 / 2.3, of which walk and chain overlap.
+constexpr size_t kHardShare = 12;
+
 // Share of (point, sampled centroid) pairs passing the first test from which the automatic choice takes the ordered chain
 // (a tuning aid: SKM_AUTO_CHAIN_SURVIVAL overrides it).
 static double auto_chain_survival() {
@@ -911,50 +922,63 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
     ws.sample = b.sample.ensure(128 * p.d);
     ws.sample_norms = b.sample_norms.ensure(128);
     ws.chain_norms_y = b.chain_norms_y.ensure(p.k * n_ck);
-    ws.n_hard_dev = b.n_hard_dev.ensure(1);
+    PrunePassCounters* counters = b.counters.ensure(1);
+    SKM_CUDA(cudaMemsetAsync(counters, 0, sizeof(PrunePassCounters), stream));
+    ws.n_hard_dev = &counters->n_hard;
+    ws.alive_total = &counters->alive;
     ws.ratio_first = ratio_first;
-    ws.alive_total = b.alive_total.ensure(1);
-    // with the tensor-core chain available, points from 6 of 128 sampled survivors up are cheaper there
-    if (tc::eligible(p.x, p.d, p.y, p.d) && (mode == 0)) ws.flag_mult = 22;
-    launch_pruned_prepare(p, ws, stream);
-    const int n_sample = static_cast<int>(std::min<size_t>(p.k, 128));
     const bool tc_ok = tc::eligible(p.x, p.d, p.y, p.d);
+    // Which family of routes: candidate lists cost one gathered 64-dimension block per surviving pair and step, so
+    // they win while few pairs survive the first test; past ~2.5 % of surviving pairs, and with at least 32 points
+    // per cluster (so that a tile of 128 ordered points spans few clusters), the points go, in the order of their
+    // previous centroid, through the chain over each tile's reachable centroids (whose cost follows the union of
+    // the tile's survivors, not their number).
+    // Measured on one B200, 10 iterations: 10M x 1024, k = 10 000 (survival 3.3 - 4.2 %): 5.0 s against 7.3 s;
+    // 1M x 1536, k = 4096 (2.2 %, then below 0.1 %): lists 0.22 s against 0.39 s; a shard of 1.25M x 1024 of the
+    // first workload (125 points per cluster): 0.58 s against 0.99 s.  Below 2^18 points the fixed costs of the
+    // ordered route (sort, batches, host round trips) outweigh it: 100k x 768, k = 1000: 23.5 ms against 16.9 ms.
+    auto ordered = [&](double survival) {
+        return auto_mode && tc_ok && p.k <= 65536 && survival >= auto_chain_survival() && p.n >= 32 * p.k && p.n >= (size_t{1} << 18);
+    };
+    if (mode == 0 && tc_ok && p.same_points && ordered(p.survival)) {
+        b.last_survival = p.survival;
+        run_pruned_pass_sorted(p, b, ratio_first, device, stream, timers, 10);
+        return;
+    }
     size_t n_hard = 0;
     bool use_chain = false, use_tc_lists = false;
     if (mode == 0) {
-        unsigned long long* host = b.counters_host.ensure(2);
-        host[0] = 0;
-        host[1] = 0;
-        SKM_CUDA(cudaMemcpyAsync(&host[0], ws.alive_total, sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
-        SKM_CUDA(cudaMemcpyAsync(&host[1], ws.n_hard_dev, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
-        SKM_CUDA(cudaStreamSynchronize(stream));
-        n_hard = static_cast<size_t>(host[1] & 0xFFFFFFFFull);
-        // Candidate lists cost one gathered block per surviving pair and step; the tensor-core chain costs a
-        // full product whatever survives.  Past roughly 0.8 % of surviving pairs the chain is cheaper.
-        const double survival = static_cast<double>(host[0]) / (static_cast<double>(p.n) * n_sample);
+        double survival = p.survival;
+        if (tc_ok) {
+            launch_exact_dist(p.x, p.y, p.knn, p.n, p.d, ws.best, stream);
+            // Which route is a question of the average only: points of about two tiles per SM answer it.
+            if (!p.same_points) launch_classify(p, ws, stream, ((p.n + kTileM - 1) / kTileM + 295) / 296);
+        } else {
+            launch_pruned_prepare(p, ws, stream);
+        }
+        if (!tc_ok || !p.same_points) {
+            PrunePassCounters* host = b.counters_host.ensure(1);
+            SKM_CUDA(cudaMemcpyAsync(host, counters, sizeof(PrunePassCounters), cudaMemcpyDeviceToHost, stream));
+            SKM_CUDA(cudaStreamSynchronize(stream));
+            n_hard = host->n_hard;
+            survival = static_cast<double>(host->alive) / (static_cast<double>(host->sampled) * std::min<size_t>(p.k, 128));
+        }
         b.last_survival = survival;
-        // Which family of routes: candidate lists cost one gathered 64-dimension block per surviving pair and step, so
-        // they win while few pairs survive the first test; past ~2.5 % of surviving pairs, and with at least 32 points
-        // per cluster (so that a tile of 128 ordered points spans few clusters), the points go, in the order of their
-        // previous centroid, through the chain over each tile's reachable centroids (whose cost follows the union of
-        // the tile's survivors, not their number).
-        // Measured on one B200, 10 iterations: 10M x 1024, k = 10 000 (survival 3.3 - 4.2 %): 5.0 s against 7.3 s;
-        // 1M x 1536, k = 4096 (2.2 %, then below 0.1 %): lists 0.22 s against 0.39 s; a shard of 1.25M x 1024 of the
-        // first workload (125 points per cluster): 0.58 s against 0.99 s.  Below 2^18 points the fixed costs of the
-        // ordered route (sort, batches, host round trips) outweigh it: 100k x 768, k = 1000: 23.5 ms against 16.9 ms.
-        if (auto_mode && tc_ok && p.k <= 65536 && survival >= auto_chain_survival() && p.n >= 32 * p.k && p.n >= (size_t{1} << 18)) {
+        if (!p.same_points && ordered(survival)) {
             run_pruned_pass_sorted(p, b, ratio_first, device, stream, timers, 10);
             return;
         }
         // The chain costs a full product whatever survives; lists cost a partial product plus one gathered
         // block per surviving pair and step, and their capacity is an eighth of all pairs.
-        use_chain = tc_ok && (survival > 0.08 || n_hard * 2 > p.n);
+        use_chain = tc_ok && survival > 0.08;
         use_tc_lists = tc_ok && !use_chain;
     } else if (mode == 3) {
+        launch_exact_dist(p.x, p.y, p.knn, p.n, p.d, ws.best, stream);
         if (!tc_ok) throw std::invalid_argument("the tensor-core chain needs 16-byte aligned rows (d % 4 == 0)");
         use_chain = true;
     } else {
         const bool dense = mode == 2;
+        launch_exact_dist(p.x, p.y, p.knn, p.n, p.d, ws.best, stream);
         use_tc_lists = mode == 4 || mode == 5;
         if (use_tc_lists && !tc_ok) throw std::invalid_argument("the tensor-core first test needs 16-byte aligned rows (d % 4 == 0)");
         fill_iota_kernel<<<static_cast<unsigned>((p.n + 255) / 256), 256, 0, stream>>>(ws.hard_idx, ws.flags, p.n, dense ? 1u : 0u);
@@ -977,25 +1001,31 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
     p.skip = ws.flags;
     if (use_tc_lists) {
         b.last_path = 4;
-        b.last_n_hard = n_hard;
-        uint32_t* redo = b.redo.ensure(p.n + 1);
-        uint32_t* redo_count = redo + p.n;
-        SKM_CUDA(cudaMemsetAsync(redo, 0, sizeof(uint32_t) * (p.n + 1), stream));
-        unsigned long long* pair_steps = b.pair_steps_dev.ensure(1);
-        SKM_CUDA(cudaMemsetAsync(pair_steps, 0, sizeof(unsigned long long), stream));
-        if (n_hard < p.n) {
+        uint32_t* redo = b.redo.ensure(p.n);
+        unsigned long long* pair_steps = b.walk_steps_dev.get();
+        if (!pair_steps) {
+            pair_steps = b.walk_steps_dev.ensure(1);
+            SKM_CUDA(cudaMemsetAsync(pair_steps, 0, sizeof(unsigned long long), stream));
+        }
+        if (mode != 0) SKM_CUDA(cudaMemsetAsync(redo, 0, sizeof(uint32_t) * p.n, stream));   // (no list of the automatic choice overflows)
+        {
             const size_t n_chunks = (p.k + kChunk - 1) / kChunk;
-            // sixteen lists per tile of 128 points, each with room for an eighth of its pairs (32 points x a quarter of
-            // the centroids); mode 5: a thirty-second, so that lists overflow.  The automatic choice knows the share of pairs
-            // that will be listed and makes room for three times that, and for no less than 7 % (so that the buffer does not
-            // grow from pass to pass): at 1M x 4000 two gigabytes instead of four.
-            const size_t pairs_per_list = 8 * p.k;
-            double room = mode == 5 ? 1.0 / 32 : 1.0 / 8;
-            if (mode == 0) room = std::min(room, 0.012 + 3.0 * std::max(b.last_survival, 0.02));
-            const uint32_t cap_group = static_cast<uint32_t>(std::max<size_t>(128, static_cast<size_t>(static_cast<double>(pairs_per_list) * room)));
+            // Sixteen lists per tile of 128 points (32 points x a quarter of the centroids).  The automatic choice lets the first
+            // test drop a point that keeps one centroid in kHardShare, and thereby knows how long a list can get; otherwise
+            // a list has room for an eighth of its pairs, in mode 5 a thirty-second, so that lists overflow.
+            tc::FirstTestRows rows;
+            rows.flags = ws.flags;
+            uint32_t cap_group = static_cast<uint32_t>(std::max<size_t>(128, p.k / (mode == 5 ? 4 : 1)));
+            if (mode == 0) {
+                SKM_CUDA(cudaMemsetAsync(ws.flags, 0, sizeof(uint32_t) * p.n, stream));
+                rows.limit = static_cast<uint32_t>(std::max<size_t>(tc::kFirstTestLimitStart, p.k / (4 * kHardShare)));
+                rows.dropped = ws.hard_idx;
+                rows.n_dropped = &counters->n_dropped;
+                cap_group = 32 * (rows.limit + 64);
+            }
             const size_t tile_bytes = kListsPerTile * static_cast<size_t>(cap_group) * sizeof(uint2);
             const size_t n_tiles = (p.n + kTileM - 1) / kTileM;
-            const size_t list_bytes_cap = static_cast<size_t>(3) << 30;
+            const size_t list_bytes_cap = static_cast<size_t>(6) << 30;
             // at least one tile per batch; when even one tile's lists exceed the cap (k in the millions) the batch is that one tile
             const size_t per_batch = std::min(n_tiles, std::max<size_t>(1, list_bytes_cap / tile_bytes));
             uint2* lists = b.tc_lists.ensure(per_batch * kListsPerTile * cap_group);
@@ -1009,7 +1039,20 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
                 const size_t nt = std::min(per_batch, n_tiles - t0);
                 {
                     Sub sub(timers, PH_PRUNE_FIRST_TEST, stream);
-                    tc::launch_first_test(xs, ys, p.n, p.k, p.partial_d, p.norms_x, p.norms_y, ws.best, ws.flags, ratio_first, t0, nt, lists, offs, cap_group, stream);
+                    tc::launch_first_test(xs, ys, p.n, p.k, p.partial_d, p.norms_x, p.norms_y, ws.best, ratio_first, t0, nt, lists, offs, cap_group, rows, stream);
+                }
+                if (mode == 0 && t0 + nt == n_tiles) {
+                    // The dropped points go through the chain beside the walk over the last lists: the two work on different
+                    // points, and one waits for the tensor cores or, with few points, for itself, the other for L2.
+                    const PrunePassCounters* host = b.counters_host.ensure(1);
+                    SKM_CUDA(cudaMemcpyAsync(b.counters_host.get(), counters, sizeof(PrunePassCounters), cudaMemcpyDeviceToHost, stream));
+                    SKM_CUDA(cudaStreamSynchronize(stream));
+                    n_hard = host->n_dropped;
+                    if (n_hard != 0) {
+                        const cudaStream_t side = b.side.get();
+                        Sub sub(timers, PH_PRUNE_DENSE, side);
+                        run_listed_dense(p, ws, b, n_hard, stream, side);
+                    }
                 }
                 WalkParams w{};
                 w.x = p.x;
@@ -1035,34 +1078,32 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
                 w.dist = p.dist;
                 w.not_pruned = p.not_pruned;
                 w.redo = redo;
-                w.redo_count = redo_count;
+                w.redo_count = &counters->n_redo;
                 w.pair_steps = pair_steps;
                 w.upstream_error = tc::error_word();
                 Sub sub(timers, PH_PRUNE_WALK, stream);
                 launch_walk_lists(w, device, stream);
             }
         }
-        {
-            Sub sub(timers, PH_PRUNE_DENSE, stream);
-            run_listed_dense(p, ws, b, n_hard, true, stream);
+        b.last_n_redo = 0;
+        if (mode == 0) {
+            if (n_hard != 0) b.side_done.hold(stream);
+        } else {
+            // points whose list overflowed
+            const PrunePassCounters* host = b.counters_host.ensure(1);
+            SKM_CUDA(cudaMemcpyAsync(b.counters_host.get(), counters, sizeof(PrunePassCounters), cudaMemcpyDeviceToHost, stream));
+            SKM_CUDA(cudaStreamSynchronize(stream));
+            n_hard = host->n_redo;
+            b.last_n_redo = n_hard;
+            b.total_redo_rows += n_hard;
+            if (n_hard != 0) {
+                Sub sub(timers, PH_PRUNE_DENSE, stream);
+                launch_compact_flags(redo, p.n, ws, stream);
+                run_listed_dense(p, ws, b, n_hard, stream);
+            }
         }
-        // points of groups whose list overflowed
-        unsigned long long* host = b.counters_host.ensure(2);
-        host[0] = 0;
-        host[1] = 0;
-        SKM_CUDA(cudaMemcpyAsync(&host[0], redo_count, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
-        SKM_CUDA(cudaMemcpyAsync(&host[1], pair_steps, sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
-        SKM_CUDA(cudaStreamSynchronize(stream));
-        const size_t n_redo = static_cast<size_t>(host[0] & 0xFFFFFFFFull);
-        b.last_n_redo = n_redo;
-        b.total_pair_steps += host[1];
-        b.total_dense_rows += n_hard + n_redo;
-        b.total_redo_rows += n_redo;
-        if (n_redo != 0) {
-            Sub sub(timers, PH_PRUNE_DENSE, stream);
-            launch_compact_flags(redo, p.n, ws, stream);
-            run_listed_dense(p, ws, b, n_redo, true, stream);
-        }
+        b.last_n_hard = n_hard;
+        b.total_dense_rows += n_hard;
         return;
     }
     b.last_path = 1;
@@ -1074,35 +1115,47 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
     launch_assign_pruned_dense(p, ws, n_hard, stream);
 }
 
-void Engine::run_pruned_pass(const float* x, size_t n, size_t k_cur, const float* y, const float* norms_x, const float* norms_y, uint32_t* knn, float* dist, uint32_t* not_pruned,
-                             bool same_points) {
+void Engine::prune_counters(uint64_t out[3]) {
+    const PrunePassBuffers& b = prune_bufs_;
+    unsigned long long walked = 0;
+    if (b.walk_steps_dev.get()) {
+        Entry entry(device_, stream_);
+        SKM_CUDA(cudaMemcpyAsync(&walked, b.walk_steps_dev.get(), sizeof(walked), cudaMemcpyDeviceToHost, stream_));
+        sync();
+    }
+    out[0] = b.total_dense_rows;
+    out[1] = b.total_pair_steps + walked;
+    out[2] = b.total_redo_rows;
+}
+
+PrunedParams Engine::pruned_params(const IterationInput& in) {
     PrunedParams p{};
-    p.same_points = same_points;
-    p.x = x;
-    p.y = y;
+    p.x = in.x;
+    p.y = c_prev_.get();
     p.y_pdx = c_pdx_.get();
     p.y_aux = c_aux_.get();
-    p.norms_x = norms_x;
-    p.norms_y = norms_y;
+    p.norms_x = in.norms;
+    p.norms_y = centroid_norms_.get();
     p.ratios = ratios_dev_.get();
-    p.knn = knn;
-    p.dist = dist;
-    p.not_pruned = not_pruned;
-    p.n = n;
-    p.k = k_cur;
+    p.knn = assignments_.get();
+    p.dist = distances_.get();
+    p.not_pruned = not_pruned_.get();
+    p.n = in.n_samples;
+    p.k = in.n_clusters;
     p.d = d_;
     p.partial_d = partial_d_;
     p.vertical_d = vertical_d_;
     p.horizontal_d = horizontal_d_;
-    run_pruned_pass_on(p, prune_bufs_, ratios_host_[partial_d_], device_, stream_, &timers_);
+    p.same_points = in.pruned_before;
+    p.survival = in.survival;
+    return p;
 }
 
 // -------------------------------------------------------------------------------------------------
-// ConsolidateCentroids (superkmeans.h:936-968): mean, split, optional normalisation, PDX copies.
-// counts_host_ holds this iteration's (globally reduced) cluster sizes.
+// SplitClusters (superkmeans.h:886-931, hierarchical_superkmeans.h:579-678) of the scaled centroids.
+// counts_host_ holds this iteration's (globally reduced) cluster sizes.  Returns whether there was anything to split.
 // -------------------------------------------------------------------------------------------------
-void Engine::consolidate(size_t n_samples_global, size_t k_cur) {
-    launch_scale_by_counts(c_cur_.get(), counts_.get(), k_cur, d_, stream_);
+bool Engine::split(size_t n_samples_global, size_t k_cur) {
     sizes_host_.assign(counts_host_.get(), counts_host_.get() + k_cur);
     if (!split_can_terminate(sizes_host_, n_samples_global, k_cur)) {
         throw std::runtime_error("cannot repopulate empty clusters: no cluster holds more than one point");
@@ -1110,18 +1163,46 @@ void Engine::consolidate(size_t n_samples_global, size_t k_cur) {
     std::vector<SplitOp> ops;
     n_split_ = hierarchical_ ? split_clusters_hierarchical(sizes_host_, n_samples_global, k_cur, cfg_.seed, ops)
                              : split_clusters_flat(sizes_host_, n_samples_global, k_cur, cfg_.seed, ops);
-    if (!ops.empty()) {
-        static_assert(sizeof(SplitOp) == sizeof(SplitOpDev), "layout");
-        SKM_CUDA(cudaMemcpyAsync(split_ops_dev_.ensure(ops.size()), ops.data(), sizeof(SplitOp) * ops.size(), cudaMemcpyHostToDevice, stream_));
-        launch_apply_split_ops(c_cur_.get(), d_, split_ops_dev_.get(), ops.size(), stream_);
-        sync();  // `ops` must outlive the asynchronous copy
-    }
-    if (cfg_.angular) launch_normalize_rows(c_cur_.get(), k_cur, d_, stream_);
-    launch_pdxify(c_cur_.get(), c_pdx_.get(), c_aux_.get(), k_cur, d_, vertical_d_, stream_);
+    if (ops.empty()) return false;
+    static_assert(sizeof(SplitOp) == sizeof(SplitOpDev), "layout");
+    SKM_CUDA(cudaMemcpyAsync(split_ops_dev_.ensure(ops.size()), ops.data(), sizeof(SplitOp) * ops.size(), cudaMemcpyHostToDevice, stream_));
+    launch_apply_split_ops(c_cur_.get(), d_, split_ops_dev_.get(), ops.size(), stream_);
+    sync();  // `ops` must outlive the asynchronous copy
+    return true;
+}
+
+// The report and the cluster sizes of what is enqueued, once it is done.
+void Engine::fetch_report(size_t k_cur) {
+    SKM_CUDA(cudaMemcpyAsync(counts_host_.ensure(k_), counts_.get(), sizeof(uint32_t) * k_cur, cudaMemcpyDeviceToHost, stream_));
+    SKM_CUDA(cudaMemcpyAsync(report_host_.get(), report_dev_.get(), sizeof(IterationReport), cudaMemcpyDeviceToHost, stream_));
+    sync();
+    if (report_host_.get()->error != 0) check_tc_error(stream_);
+}
+
+// ConsolidateCentroids without the splits, and ComputeShift.
+void Engine::consolidate(const IterationInput& in, bool scale) {
+    PhaseScope ps(*this, PH_CONSOLIDATE);
+    ConsolidateParams p{};
+    p.c = c_cur_.get();
+    p.prev = c_prev_.get();
+    p.counts = scale ? counts_.get() : nullptr;
+    p.normalize = cfg_.angular;
+    p.splits_follow = scale && hierarchical_;
+    p.pdx = c_pdx_.get();
+    p.aux = c_aux_.get();
+    p.k = in.n_clusters;
+    p.d = d_;
+    p.vertical_d = vertical_d_;
+    p.reduce_scratch = ws_.reduce_scratch;
+    p.report = report_dev_.get();
+    launch_consolidate(p, stream_);
 }
 
 // -------------------------------------------------------------------------------------------------
 // RunIteration<GEMM_ONLY> (superkmeans.h:786-879)
+//
+// Everything up to the shift is enqueued on the assumption that no cluster is split, which is rare, and the host waits once,
+// for the report; after a split the consolidation is finished again.
 // -------------------------------------------------------------------------------------------------
 void Engine::run_iteration(bool gemm_only, const IterationInput& in, size_t iter_idx, bool is_first, std::vector<skm_iter_stats>& target) {
     if (!is_first) c_cur_.swap(c_prev_);
@@ -1139,31 +1220,28 @@ void Engine::run_iteration(bool gemm_only, const IterationInput& in, size_t iter
     } else {
         launch_row_sqnorms(c_prev_.get(), k_cur, d_, partial_d_, centroid_norms_.get(), stream_);
         PhaseScope ps(*this, PH_ASSIGN_PRUNED);
-        run_pruned_pass(in.x, n, k_cur, c_prev_.get(), norms, centroid_norms_.get(), assignments_.get(), distances_.get(), not_pruned_.get(), in.pruned_before);
-        in.pruned_before = true;
+        run_pruned_pass_on(pruned_params(in), prune_bufs_, ratios_host_[partial_d_], device_, stream_, &timers_);
     }
     // UpdateCentroids + ComputeCost (superkmeans.h:729-765, :973-981)
     {
         PhaseScope ps(*this, PH_UPDATE);
-        launch_update(in.x, assignments_.get(), distances_.get(), gemm_only ? nullptr : not_pruned_.get(), n, k_cur, d_, ws_, c_cur_.get(), counts_.get(), scalars_dev_.get(),
-                      gemm_only ? nullptr : np_total_dev_.get(), stream_);
-        if (!gemm_only) {
-            u64_to_f64_kernel<<<1, 1, 0, stream_>>>(np_total_dev_.get(), scalars_dev_.get() + 1);
-            note_kernel_launch();
-            SKM_CUDA(cudaGetLastError());
-        }
+        UpdateStats stats;
+        stats.dist = distances_.get();
+        stats.not_pruned = gemm_only ? nullptr : not_pruned_.get();
+        stats.error = tc::error_word();
+        stats.report = report_dev_.get();
+        launch_update(in.x, assignments_.get(), n, k_cur, d_, ws_, c_cur_.get(), counts_.get(), &stats, stream_);
     }
-    allreduce_iteration(c_cur_.get(), k_cur * d_, counts_.get(), k_cur, scalars_dev_.get(), 2);
-    SKM_CUDA(cudaMemcpyAsync(counts_host_.ensure(k_), counts_.get(), sizeof(uint32_t) * k_cur, cudaMemcpyDeviceToHost, stream_));
-    SKM_CUDA(cudaMemcpyAsync(scalars_host_.get(), scalars_dev_.get(), sizeof(double) * 2, cudaMemcpyDeviceToHost, stream_));
-    sync();
-    check_tc_error(stream_);
-    const double wcss = scalars_host_.get()[0];
+    allreduce_iteration(c_cur_.get(), k_cur * d_, counts_.get(), k_cur, &report_dev_.get()->wcss, 2);
+    consolidate(in, true);
+    fetch_report(k_cur);
+    const IterationReport& report = *report_host_.get();
+    const double wcss = report.wcss;
 
     float avg_not_pruned = -1.0f;
     const uint32_t old_partial_d = partial_d_;
     if (!gemm_only) {
-        const TuneResult t = tune_partial_d(scalars_host_.get()[1], in.n_samples_global, k_cur, partial_d_, vertical_d_, cfg_.min_not_pruned_pct, cfg_.max_not_pruned_pct,
+        const TuneResult t = tune_partial_d(report.not_pruned, in.n_samples_global, k_cur, partial_d_, vertical_d_, cfg_.min_not_pruned_pct, cfg_.max_not_pruned_pct,
                                             cfg_.adjustment_factor_for_partial_d);
         avg_not_pruned = t.avg_not_pruned_pct;
         partial_d_ = t.new_partial_d;
@@ -1171,23 +1249,18 @@ void Engine::run_iteration(bool gemm_only, const IterationInput& in, size_t iter
             PhaseScope ps(*this, PH_NORMS);
             launch_row_sqnorms(in.x, n, d_, partial_d_, norms, stream_);
         }
+        in.pruned_before = true;
+        in.survival = report.not_pruned / (static_cast<double>(in.n_samples_global) * static_cast<double>(k_cur));
     }
-    {
-        PhaseScope ps(*this, PH_CONSOLIDATE);
-        consolidate(in.n_samples_global, k_cur);
+    if (split(in.n_samples_global, k_cur) || (hierarchical_ && cfg_.angular)) {
+        consolidate(in, false);
+        fetch_report(k_cur);
     }
 
     prev_cost_ = cost_;
     cost_ = static_cast<float>(wcss);
     last_cost_f64_ = wcss;
-    // ComputeShift (superkmeans.h:988-998)
-    {
-        PhaseScope ps(*this, PH_SHIFT);
-        launch_shift(c_cur_.get(), c_prev_.get(), k_cur, d_, ws_.block_sums, scalars_dev_.get() + 2, stream_);
-    }
-    SKM_CUDA(cudaMemcpyAsync(scalars_host_.get() + 2, scalars_dev_.get() + 2, sizeof(double), cudaMemcpyDeviceToHost, stream_));
-    sync();
-    shift_ = static_cast<float>(scalars_host_.get()[2]);
+    shift_ = static_cast<float>(report.shift);
 
     if (trace_on_) {
         Snapshot snap;
@@ -1837,7 +1910,12 @@ void Engine::assign_training_points(const float* vectors, const float* centroids
         const size_t cnt = std::min(rows, n - r0);
         load_rows(vectors + r0 * d_, on_device, nullptr, cnt, !cfg_.data_already_rotated, xr.get());
         launch_row_sqnorms(xr.get(), cnt, d_, partial_d_, xn.get(), stream_);
-        run_pruned_pass(xr.get(), cnt, k_, c_cur_.get(), xn.get(), centroid_norms_.get(), knn + r0, store_state ? dist + r0 : dist, np.get());
+        PrunedParams p = pruned_params(IterationInput{xr.get(), cnt, cnt, k_, xn.get()});
+        p.y = c_cur_.get();
+        p.knn = knn + r0;
+        p.dist = store_state ? dist + r0 : dist;
+        p.not_pruned = np.get();
+        run_pruned_pass_on(p, prune_bufs_, ratios_host_[partial_d_], device_, stream_, &timers_);
     }
     if (on_device) SKM_CUDA(cudaMemcpyAsync(out, knn, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, stream_));
     else stage_.download(out, knn, sizeof(uint32_t) * n, stream_);
@@ -1969,7 +2047,7 @@ void Engine::op_find_nearest_pruned(int device, const float* x, const float* y, 
     p.vertical_d = static_cast<uint32_t>(split.vertical_d);
     p.horizontal_d = static_cast<uint32_t>(split.horizontal_d);
     PrunePassBuffers bufs;
-    run_pruned_pass_on(p, bufs, ratios[partial_d], dev, ctx.stream);
+    run_pruned_pass_on(p, bufs, ratios[partial_d], dev, ctx.stream, nullptr);
     std::vector<uint32_t> np_host(n);
     ctx.download(knn_io, knn.get(), n);
     ctx.download(dist_out, dist.get(), n);
@@ -1984,7 +2062,8 @@ void Engine::op_update(int device, const float* x, const uint32_t* assign, const
     OpContext ctx(device);
     DeviceBuffer<float> xd, dd, sums, partials;
     DeviceBuffer<uint32_t> ad, counts, ka, kb, va, vb, table, offs;
-    DeviceBuffer<double> block_sums, wcss;
+    DeviceBuffer<double> reduce_scratch;
+    DeviceBuffer<IterationReport> report;
     ctx.upload(xd, x, n * d);
     ctx.upload(ad, assign, n);
     std::vector<float> zeros;
@@ -2002,14 +2081,18 @@ void Engine::op_update(int device, const float* x, const uint32_t* assign, const
     ws.digit_table = table.ensure(256 * units + (256 * units) / 2048 + 64);
     ws.seg_offsets = offs.ensure(k + 1);
     ws.tile_partials = partials.ensure(std::max<size_t>(tiles, 1) * 2 * d);
-    ws.block_sums = block_sums.ensure(2048);
-    launch_update(xd.get(), ad.get(), dd.get(), nullptr, n, k, d, ws, sums.ensure(k * d), counts.ensure(k), wcss.ensure(1), nullptr, ctx.stream);
+    ws.reduce_scratch = reduce_scratch.ensure(kReduceScratchDoubles);
+    SKM_CUDA(cudaMemsetAsync(ws.reduce_scratch, 0, sizeof(double) * kReduceScratchDoubles, ctx.stream));
+    UpdateStats stats;
+    stats.dist = dd.get();
+    stats.report = report.ensure(1);
+    launch_update(xd.get(), ad.get(), n, k, d, ws, sums.ensure(k * d), counts.ensure(k), &stats, ctx.stream);
     ctx.download(sums_out, sums.get(), k * d);
     ctx.download(counts_out, counts.get(), k);
-    double w = 0.0;
-    ctx.download(&w, wcss.get(), 1);
+    IterationReport r{};
+    ctx.download(&r, report.get(), 1);
     ctx.sync();
-    if (wcss_out) *wcss_out = w;
+    if (wcss_out) *wcss_out = r.wcss;
 }
 
 void Engine::op_pdxify(int device, const float* in, size_t n, size_t d, float* out) {

@@ -68,8 +68,9 @@ struct PrunePassBuffers {
     DeviceBuffer<uint2> tc_lists, listed_top2;
     DeviceBuffer<uint32_t> tc_list_offs, redo, listed_knn, listed_np;
     DeviceBuffer<float> listed_x, listed_best, listed_dist, listed_norms, y_split;
-    DeviceBuffer<unsigned long long> alive_total;
-    PinnedBuffer<unsigned long long> counters_host;
+    DeviceBuffer<PrunePassCounters> counters;
+    PinnedBuffer<PrunePassCounters> counters_host;
+    PinnedBuffer<unsigned long long> sorted_counters_host;
     double last_survival = 0;   // share of sampled (point, centroid) pairs that passed the first test in the last automatic choice
     int last_path = 0;   // 1 lists (+ dense for flagged points), 3 tensor-core chain, 4 tensor-core first test + list walk
     int grid = 0;
@@ -78,6 +79,7 @@ struct PrunePassBuffers {
     // running totals since the buffers were created: rows sent through a dense chain, (pair, 64-dimension block)
     // steps of the list walk, rows whose list overflowed
     unsigned long long total_dense_rows = 0, total_pair_steps = 0, total_redo_rows = 0;
+    DeviceBuffer<unsigned long long> walk_steps_dev;   // ... and on the device those that total_pair_steps lacks
     DeviceBuffer<unsigned long long> pair_steps_dev;
     // the pass over the points in the order of their previous centroid (paths 6-8)
     UpdateWorkspace sort_ws;
@@ -100,6 +102,38 @@ struct PrunePassBuffers {
     DeviceBuffer<__half> x_hi, x_lo, y_hi, y_lo;
     DeviceBuffer<float> x_factor, y_factor;
     bool x_halves_valid = false;
+    // a second stream, and the places where the two meet
+    struct Mark {
+        cudaEvent_t event = nullptr;
+        Mark() = default;
+        Mark(const Mark&) = delete;
+        Mark& operator=(const Mark&) = delete;
+        ~Mark() {
+            if (event) cudaEventDestroy(event);
+        }
+        void record(cudaStream_t s) {
+            if (!event) SKM_CUDA(cudaEventCreateWithFlags(&event, cudaEventDisableTiming));
+            SKM_CUDA(cudaEventRecord(event, s));
+        }
+        void hold(cudaStream_t s) const { SKM_CUDA(cudaStreamWaitEvent(s, event, 0)); }   // what follows on s waits for the mark
+    } side_start, side_done;
+    struct Side {
+        cudaStream_t stream = nullptr;
+        int device = 0;
+        Side() = default;
+        Side(const Side&) = delete;
+        Side& operator=(const Side&) = delete;
+        ~Side() {
+            if (stream) release_stream(stream, device);   // (waits)
+        }
+        cudaStream_t get() {
+            if (!stream) {
+                SKM_CUDA(cudaGetDevice(&device));
+                stream = acquire_stream();
+            }
+            return stream;
+        }
+    };
     // `cols` columns of rows x d
     tc::SplitHalves x_halves(size_t rows, uint32_t cols) {
         const uint32_t pitch = (cols + 7) / 8 * 8;
@@ -109,6 +143,7 @@ struct PrunePassBuffers {
         const uint32_t pitch = (cols + 7) / 8 * 8;
         return {y_hi.ensure(rows * pitch), y_lo.ensure(rows * pitch), y_factor.ensure(1), pitch};
     }
+    Side side;   // (last: its work ends before any buffer goes)
 };
 // mode: 0 = automatic: with rows that TMA can address, the points are taken in the order of their previous centroid and
 // every tile of 128 goes either through the first test + list walk or, when many of its points keep a large share of
@@ -118,7 +153,7 @@ struct PrunePassBuffers {
 // to a quarter so that the overflow route runs, 6 = ordered points, gathered chain for every tile, 7 = ordered points,
 // first test + list walk for every tile (overflowing tiles through the gathered chain), 8 = as 7 with the small lists
 // of mode 5, 9 = the automatic choice without ordering (dense chain for all points when the sampled survival rate is
-// high, else first test + list walk with flagged points on the dense chain), 10 = ordered points, every tile through
+// high, else first test + list walk with the points it drops on the dense chain), 10 = ordered points, every tile through
 // the optimistic chain pass with the exact gathered chain for the points it flags (mode 0 does the same for the tiles
 // it sends to the chain; mode 6 uses the exact gathered chain alone).
 void set_prune_split_mode(int mode);
@@ -157,11 +192,7 @@ class Engine {
     size_t n_state_rows() const { return n_state_rows_; }
     double last_objective_f64() const { return last_cost_f64_; }
     int last_prune_path() const { return prune_bufs_.last_path; }
-    void prune_counters(uint64_t out[3]) const {
-        out[0] = prune_bufs_.total_dense_rows;
-        out[1] = prune_bufs_.total_pair_steps;
-        out[2] = prune_bufs_.total_redo_rows;
-    }
+    void prune_counters(uint64_t out[3]);
     void chain_counters(uint64_t out[4]) const {
         out[0] = prune_bufs_.total_sparse_rows;
         out[1] = prune_bufs_.total_sparse_cols;
@@ -200,6 +231,7 @@ class Engine {
         size_t n_clusters;
         float* norms;         // device, full or partial norms of x (rewritten when d' changes)
         mutable bool pruned_before = false;   // a pruned pass over these rows has run
+        mutable double survival = 0.0;        // ... and what it said about the next one (PrunedParams)
     };
 
     void start_rotation_draws();   // the Gaussian draws of a matrix that is still to be made, on a host thread
@@ -215,9 +247,10 @@ class Engine {
     size_t streamed_rows(size_t n) const;
     void prepare_update_workspace(size_t n, size_t k);
     void run_iteration(bool gemm_only, const IterationInput& in, size_t iter_idx, bool is_first, std::vector<skm_iter_stats>& target);
-    void run_pruned_pass(const float* x, size_t n, size_t k_cur, const float* y, const float* norms_x, const float* norms_y, uint32_t* knn, float* dist, uint32_t* not_pruned,
-                         bool same_points = false);
-    void consolidate(size_t n_samples_global, size_t k_cur);
+    PrunedParams pruned_params(const IterationInput& in);
+    void consolidate(const IterationInput& in, bool scale);
+    void fetch_report(size_t k_cur);
+    bool split(size_t n_samples_global, size_t k_cur);
     // `precomputed`: the Forgy indices when the caller has already drawn them (on another thread, while buffers were allocated)
     void generate_centroids_from_host(const float* data, bool on_device, size_t n_points_global, size_t k_cur, bool rotate, const std::vector<size_t>* precomputed = nullptr);
     bool sharded_() const { return allreduce_fn_ != nullptr || comm_ != nullptr; }
@@ -309,9 +342,8 @@ class Engine {
     PinnedBuffer<uint32_t> recall_found_host_;
     float recall_ = 0.0f;
     DeviceBuffer<SplitOpDev> split_ops_dev_;
-    DeviceBuffer<double> scalars_dev_;   // [0] wcss, [1] not-pruned total (as double), [2] shift
-    DeviceBuffer<unsigned long long> np_total_dev_;
-    PinnedBuffer<double> scalars_host_;
+    DeviceBuffer<IterationReport> report_dev_;
+    PinnedBuffer<IterationReport> report_host_;
     PinnedBuffer<uint32_t> counts_host_;
     std::vector<uint32_t> sizes_host_;   // cluster_sizes after the last split
 
@@ -319,7 +351,7 @@ class Engine {
     UpdateWorkspace ws_;
     DeviceBuffer<uint32_t> ws_keys_a_, ws_keys_b_, ws_vals_a_, ws_vals_b_, ws_table_, ws_offsets_;
     DeviceBuffer<float> ws_partials_;
-    DeviceBuffer<double> ws_block_sums_;
+    DeviceBuffer<double> ws_reduce_;
 
     // hierarchical extras
     DeviceBuffer<float> full_norms_;      // immutable_data_norms

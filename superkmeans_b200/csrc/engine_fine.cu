@@ -163,7 +163,7 @@ void Engine::train_fine_run(size_t first, size_t last, const std::vector<size_t>
         }
         {
             PhaseScope ps(*this, PH_UPDATE);
-            launch_update(x, assignments_.get(), distances_.get(), nullptr, n, k, d_, ws_, c_cur_.get(), counts_.get(), nullptr, nullptr, stream_);
+            launch_update(x, assignments_.get(), n, k, d_, ws_, c_cur_.get(), counts_.get(), nullptr, stream_);
             group_cost_kernel<<<static_cast<unsigned>(n_groups), 256, 0, stream_>>>(distances_.get(), groups_dev.get(), sums_dev.get());
             SKM_LAUNCH_CHECK();
         }

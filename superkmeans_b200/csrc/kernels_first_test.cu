@@ -60,7 +60,10 @@ struct TestParams {
     const float* norms_x;
     const float* norms_y;
     const float* best_in;
-    const uint32_t* skip;
+    uint32_t* flags;             // may be null: per row, nonzero = leave this point out
+    uint32_t limit_slope;        // 2^-32: a row with kFirstTestLimitStart and this many survivors per column of a warp is left out from there on, and
+    uint32_t* dropped;           // appended here (its flag set)
+    uint32_t* n_dropped;
     float ratio_first;
     uint2* lists;
     uint32_t* list_offs;
@@ -190,7 +193,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T_THREADS, 1) first_
             const bool valid = listed && row < p.n;
             const float nx = valid ? p.norms_x[row] : 0.f;
             const float factor = valid ? p.factor_x[row] * fy : 0.f;
-            const float thr = valid && !(p.skip && p.skip[row]) ? p.best_in[row] * p.ratio_first : -FLT_MAX;
+            float thr = valid && !(p.flags && p.flags[row]) ? p.best_in[row] * p.ratio_first : -FLT_MAX;
+            uint32_t survivors = 0;
             const size_t group = (listed ? q : 0) * kListsPerTile + part * 4 + quarter;
             uint2* my_list = p.lists + group * p.cap_group;
             uint32_t* my_offs = p.list_offs + group * ((p.k + 1023) / 1024 + 1);
@@ -227,6 +231,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T_THREADS, 1) first_
                     if (!__any_sync(0xffffffffu, mask != 0)) return;
                     // where a lane's survivors go: behind those of the lanes before it
                     const uint32_t cnt = __popc(mask);
+                    survivors += cnt;
                     uint32_t incl = cnt;
 #pragma unroll
                     for (int off = 1; off < 32; off <<= 1) {
@@ -264,6 +269,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T_THREADS, 1) first_
                         if (lane == 0) mbar_arrive_cluster(cluster_address(&ctrl->acc_empty[b], 0));
                     }
                     test(r, ch);
+                }
+                // Too many survivors, or on the way there: from the start of a point that keeps 10 %, the sloped line saves three
+                // quarters of the pairs that would be listed in vain.
+                const bool drop = survivors >= kFirstTestLimitStart + __umulhi((nt + 1) * 64, p.limit_slope);
+                if (__any_sync(0xffffffffu, drop)) {
+                    if (drop) {
+                        survivors = 0;
+                        thr = -FLT_MAX;
+                        if (atomicExch(p.flags + row, 1u) == 0) p.dropped[atomicAdd(p.n_dropped, 1u)] = static_cast<uint32_t>(row);
+                    }
+                    __syncwarp();
                 }
             }
             if (ok && lane == 0 && listed) my_offs[(p.k + 1023) / 1024] = filled;
@@ -360,8 +376,7 @@ void launch_split_centroids(const float* y, size_t k, size_t d, uint32_t cols, c
 }
 
 void launch_first_test(const SplitHalves& x, const SplitHalves& y, size_t n, size_t k, uint32_t partial_d, const float* norms_x, const float* norms_y, const float* best_in,
-                       const uint32_t* skip, float ratio_first, size_t tile0, size_t n_tiles, uint2* lists, uint32_t* list_offs, uint32_t cap_group, cudaStream_t stream,
-                       const uint32_t* tile_map) {
+                       float ratio_first, size_t tile0, size_t n_tiles, uint2* lists, uint32_t* list_offs, uint32_t cap_group, const FirstTestRows& rows, cudaStream_t stream) {
     if (n_tiles == 0 || k == 0) return;
     int device = 0, sms = 0;
     SKM_CUDA(cudaGetDevice(&device));
@@ -377,13 +392,18 @@ void launch_first_test(const SplitHalves& x, const SplitHalves& y, size_t n, siz
     p.k_blocks = (partial_d + TK - 1) / TK;
     p.tile0 = tile0;
     p.n_tiles = n_tiles;
-    p.tile_map = tile_map;
+    p.tile_map = rows.tile_map;
     p.factor_x = x.factor;
     p.factor_y = y.factor;
     p.norms_x = norms_x;
     p.norms_y = norms_y;
     p.best_in = best_in;
-    p.skip = skip;
+    p.flags = rows.flags;
+    // a line from kFirstTestLimitStart at no column to the limit at all columns of a warp; without a limit one that no row reaches
+    p.limit_slope = 0xFFFFFFFFu;
+    if (rows.limit != 0xFFFFFFFFu) p.limit_slope = static_cast<uint32_t>(4294967296.0 * (rows.limit - std::min(rows.limit, kFirstTestLimitStart)) / (64.0 * ((k + 255) / 256)));
+    p.dropped = rows.dropped;
+    p.n_dropped = rows.n_dropped;
     p.ratio_first = ratio_first;
     p.lists = lists;
     p.list_offs = list_offs;

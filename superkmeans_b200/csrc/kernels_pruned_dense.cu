@@ -30,6 +30,21 @@ uint32_t prune_chain_checkpoints(uint32_t partial_d, uint32_t vertical_d, uint32
 size_t prune_split_positions_elems(size_t n) { return n + n / 2048 + 64; }
 
 // -------------------------------------------------------------------------------------------------
+// The rows of a block (`rows` of them from row0) whose flag is set, appended to a list in one step.
+__device__ __forceinline__ void append_flagged(const uint32_t* flags, int rows, size_t row0, uint32_t* __restrict__ list, uint32_t* __restrict__ n_list) {
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x;
+    for (int r0 = 0; r0 < rows; r0 += 32) {
+        const bool mine = r0 + lane < rows && flags[r0 + lane] != 0;
+        const uint32_t all = __ballot_sync(0xffffffffu, mine);
+        if (all == 0) continue;
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(n_list, static_cast<uint32_t>(__popc(all)));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (mine) list[at + __popc(all & ((1u << lane) - 1u))] = static_cast<uint32_t>(row0 + r0 + lane);
+    }
+}
+
 __global__ void __launch_bounds__(256) prev_dist_kernel(const float* __restrict__ x, const float* __restrict__ y, const uint32_t* __restrict__ knn, size_t n, size_t d,
                                                         float* __restrict__ best) {
     const size_t row = static_cast<size_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
@@ -70,11 +85,12 @@ __global__ void gather_sample_kernel(const float* __restrict__ y, size_t k, size
 // counted per point.
 __global__ void __launch_bounds__(256, 2) classify_kernel(
     const float* __restrict__ x, const float* __restrict__ sample, const float* __restrict__ sample_norms, const float* __restrict__ norms_x, const float* __restrict__ best,
-    size_t n, size_t d, uint32_t partial_d, int n_sample, float ratio_first, uint32_t flag_mult, uint32_t* __restrict__ flags, unsigned long long* __restrict__ alive_total
+    size_t n, size_t d, size_t tile_step, uint32_t partial_d, int n_sample, float ratio_first, uint32_t flag_mult, uint32_t* __restrict__ flags, unsigned long long* __restrict__ alive_total,
+    uint32_t* __restrict__ hard_idx, uint32_t* __restrict__ n_hard
 ) {
     __shared__ GemmSmem smem;
     __shared__ uint32_t cnt[kTileM];
-    const size_t row0 = static_cast<size_t>(blockIdx.x) * kTileM;
+    const size_t row0 = static_cast<size_t>(blockIdx.x) * tile_step * kTileM;
     const int m_valid = static_cast<int>(min(static_cast<size_t>(kTileM), n - row0));
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     if (threadIdx.x < kTileM) cnt[threadIdx.x] = 0;
@@ -98,14 +114,23 @@ __global__ void __launch_bounds__(256, 2) classify_kernel(
         if (c_alive) atomicAdd(&cnt[r], c_alive);
     }
     __syncthreads();
-    if (static_cast<int>(threadIdx.x) < m_valid) flags[row0 + threadIdx.x] = (cnt[threadIdx.x] * flag_mult >= static_cast<uint32_t>(n_sample)) ? 1u : 0u;
+    __shared__ uint32_t hard[kTileM];
+    if (static_cast<int>(threadIdx.x) < m_valid) {
+        hard[threadIdx.x] = (cnt[threadIdx.x] * flag_mult >= static_cast<uint32_t>(n_sample)) ? 1u : 0u;
+        flags[row0 + threadIdx.x] = hard[threadIdx.x];
+    }
+    __syncthreads();
+    if (hard_idx) append_flagged(hard, m_valid, row0, hard_idx, n_hard);
     // total number of sampled pairs that pass the first test (estimates the pass's survival rate)
     if (threadIdx.x < 32) {
         uint32_t s = 0;
         for (int r = threadIdx.x; r < m_valid; r += 32) s += cnt[r];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (threadIdx.x == 0 && s) atomicAdd(alive_total, static_cast<unsigned long long>(s));
+        if (threadIdx.x == 0) {
+            if (s) atomicAdd(alive_total, static_cast<unsigned long long>(s));
+            atomicAdd(alive_total + 1, static_cast<unsigned long long>(m_valid));
+        }
     }
 }
 
@@ -323,20 +348,7 @@ void launch_exact_dist(const float* x, const float* y, const uint32_t* knn, size
 void launch_pruned_prepare(const PrunedParams& p, PruneSplitWorkspace& ws, cudaStream_t stream) {
     if (p.n == 0) return;
     launch_exact_dist(p.x, p.y, p.knn, p.n, p.d, ws.best, stream);
-    const int n_sample = static_cast<int>(std::min<size_t>(p.k, kSample));
-    gather_sample_kernel<<<n_sample, 256, 0, stream>>>(p.y, p.k, p.d, n_sample, ws.sample);
-    SKM_LAUNCH_CHECK();
-    launch_row_sqnorms(ws.sample, n_sample, p.d, p.partial_d, ws.sample_norms, stream);
-    const float ratio_first = ws.ratio_first;
-    SKM_CUDA(cudaMemsetAsync(ws.alive_total, 0, sizeof(unsigned long long), stream));
-    classify_kernel<<<static_cast<unsigned>((p.n + kTileM - 1) / kTileM), 256, 0, stream>>>(p.x, ws.sample, ws.sample_norms, p.norms_x, ws.best, p.n, p.d, p.partial_d, n_sample,
-                                                                                             ratio_first, ws.flag_mult, ws.flags, ws.alive_total);
-    SKM_LAUNCH_CHECK();
-    copy_u32_kernel<<<static_cast<unsigned>((p.n + 255) / 256), 256, 0, stream>>>(ws.flags, ws.positions, p.n);
-    SKM_LAUNCH_CHECK();
-    exclusive_scan_u32(ws.positions, p.n, ws.positions + p.n, stream);
-    compact_flags_kernel<<<static_cast<unsigned>((p.n + 255) / 256), 256, 0, stream>>>(ws.flags, ws.positions, p.n, ws.hard_idx, ws.n_hard_dev);
-    SKM_LAUNCH_CHECK();
+    launch_classify(p, ws, stream);
 }
 
 // Rows listed in idx gathered into a compact matrix together with their threshold and previous assignment,
@@ -468,16 +480,17 @@ void launch_init_chain_rows(const uint32_t* tile_map, size_t n_tiles, size_t n, 
     SKM_LAUNCH_CHECK();
 }
 
-// flags / alive_total of launch_pruned_prepare without the exact distances and the compaction (the caller has the former and does not need the latter)
-void launch_classify(const PrunedParams& p, PruneSplitWorkspace& ws, cudaStream_t stream) {
+// What launch_pruned_prepare finds out from a sample, without the exact distances (ws.hard_idx null: no list)
+void launch_classify(const PrunedParams& p, PruneSplitWorkspace& ws, cudaStream_t stream, size_t step) {
     if (p.n == 0) return;
     const int n_sample = static_cast<int>(std::min<size_t>(p.k, kSample));
     gather_sample_kernel<<<n_sample, 256, 0, stream>>>(p.y, p.k, p.d, n_sample, ws.sample);
     SKM_LAUNCH_CHECK();
     launch_row_sqnorms(ws.sample, n_sample, p.d, p.partial_d, ws.sample_norms, stream);
-    SKM_CUDA(cudaMemsetAsync(ws.alive_total, 0, sizeof(unsigned long long), stream));
-    classify_kernel<<<static_cast<unsigned>((p.n + kTileM - 1) / kTileM), 256, 0, stream>>>(p.x, ws.sample, ws.sample_norms, p.norms_x, ws.best, p.n, p.d, p.partial_d, n_sample,
-                                                                                             ws.ratio_first, ws.flag_mult, ws.flags, ws.alive_total);
+    SKM_CUDA(cudaMemsetAsync(ws.alive_total, 0, 2 * sizeof(unsigned long long), stream));
+    const size_t tiles = (p.n + kTileM - 1) / kTileM;
+    classify_kernel<<<static_cast<unsigned>((tiles + step - 1) / step), 256, 0, stream>>>(p.x, ws.sample, ws.sample_norms, p.norms_x, ws.best, p.n, p.d, step, p.partial_d, n_sample,
+                                                                                             ws.ratio_first, ws.flag_mult, ws.flags, ws.alive_total, ws.hard_idx, ws.n_hard_dev);
     SKM_LAUNCH_CHECK();
 }
 

@@ -53,10 +53,16 @@ void launch_split_centroids(const float* y, size_t k, size_t d, uint32_t cols, c
 // columns 64c..64c+63 of every 256-centroid tile) as {centroid << 5 | row in the 32-row group, partial
 // distance}, at most cap_group entries per list, in centroid-tile order; list_offs receives, per list, the number
 // of entries before every 1024-centroid chunk and the total (which exceeds cap_group on overflow).
-// tile_map (optional): entry t of the range stands for row tile tile_map[t]; lists stay indexed by t.
+constexpr uint32_t kFirstTestLimitStart = 8;
+struct FirstTestRows {
+    const uint32_t* tile_map = nullptr;   // entry t of the range stands for row tile tile_map[t]; lists stay indexed by t
+    uint32_t* flags = nullptr;            // per row: nonzero = not tested, and set for
+    uint32_t limit = 0xFFFFFFFFu;         // a row with this many survivors (kFirstTestLimitStart at least) among a quarter of the columns,
+    uint32_t* dropped = nullptr;          // or clearly on the way there: it is left out from there on (no list then holds more than
+    uint32_t* n_dropped = nullptr;        // 32 * (limit + 64) pairs) and appended here, in any order (*n_dropped zero before)
+};
 void launch_first_test(const SplitHalves& x, const SplitHalves& y, size_t n, size_t k, uint32_t partial_d, const float* norms_x, const float* norms_y, const float* best_in,
-                       const uint32_t* skip, float ratio_first, size_t tile0, size_t n_tiles, uint2* lists, uint32_t* list_offs, uint32_t cap_group, cudaStream_t stream,
-                       const uint32_t* tile_map = nullptr);
+                       float ratio_first, size_t tile0, size_t n_tiles, uint2* lists, uint32_t* list_offs, uint32_t cap_group, const FirstTestRows& rows, cudaStream_t stream);
 
 // The same first test (threshold widened by 1e-4 relative) for the row tiles tile_map[0 .. n_tiles), keeping only its
 // footprint: bit c of union_bits[t * union_words + c / 32] is set (atomic OR into zeroed memory) when some row of tile t

@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,d,k", [(129, 132, 300), (1, 128, 1), (255, 256, 257), (4097, 200, 1025), (20_000, 1024, 2_100), (12_345, 384, 5_000)])
-@pytest.mark.parametrize("lists", [4, 5], ids=["roomy", "overflowing"])
+@pytest.mark.parametrize("lists", [4, 5, 9], ids=["roomy", "overflowing", "dropping"])
 def test_lists_agree_with_the_simt_search(n, d, k, lists):
     import superkmeans_b200 as skm
 
