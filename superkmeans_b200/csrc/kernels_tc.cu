@@ -1098,6 +1098,9 @@ CUtensorMap make_half_tmap(const void* base, size_t cols, size_t rows, uint32_t 
     return make_tmap_of(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, CU_TENSOR_MAP_SWIZZLE_128B, base, cols, rows, pitch ? pitch : cols, 64, box_rows);
 }
 
+CUtensorMap make_row_major_tmap_128(const float* base, size_t extent, size_t rows, size_t ld, uint32_t box_rows) {
+    return make_tmap_of(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, sizeof(float), CU_TENSOR_MAP_SWIZZLE_128B, base, extent, rows, ld, 32, box_rows);
+}
 CUtensorMap make_row_major_tmap(const float* base, size_t extent, size_t rows, size_t ld, uint32_t box_rows) { return make_tmap(base, extent, rows, ld, box_rows); }
 
 int* error_word() {

@@ -31,9 +31,8 @@ void launch_assign_full_flagged(const float* x, const float* y, size_t n, size_t
                                 uint2* top2_scratch, int* error_word, cudaStream_t stream);
 void launch_gemm_nt(const float* a, size_t lda, const float* b, size_t ldb, float* out, size_t ldo, size_t n, size_t n_out, size_t k_dim, cudaStream_t stream);
 // out[n][n_out] = a[n][k_dim] * b[n_out][k_dim]^T with the accumulation cut into four chains that are summed in fp32
-// registers (kernels_tc_rotate.cu): the rotation and un-rotation GEMM.  out_sqnorms (optional): squared norm of every output row.
-void launch_rotate(const float* a, size_t lda, const float* b, size_t ldb, float* out, size_t ldo, size_t n, size_t n_out, size_t k_dim, float* out_sqnorms,
-                   cudaStream_t stream);
+// registers (kernels_tc_rotate.cu): the rotation and un-rotation GEMM.  b is contiguous.
+void launch_rotate(const float* a, size_t lda, const float* b, float* out, size_t ldo, size_t n, size_t n_out, size_t k_dim, cudaStream_t stream);
 
 // The leading columns of a row-major fp32 matrix as fp16 pairs: element * scale = hi + lo to 22 bits, scale a power of two.
 // For points a scale per row (factor[row] = -2 / scale), for centroids one for all (factor[0] = 1 / scale).
