@@ -214,7 +214,8 @@ void Engine::start_rotation_draws() {
     draws_ = std::make_unique<NormalDraws>(d_ * d_, cfg_.seed);
     uint32_t* bits = draw_bits_.ensure(draws_->scratch());
     float* values = draw_values_.ensure(draws_->scratch());
-    draws_done_ = std::async(std::launch::async, [this, bits, values] { return draws_->make(bits, values); });
+    draws_->values_at(values);
+    draws_done_ = std::async(std::launch::async, [this, bits, values] { draws_->make(bits, values); });
 }
 
 void Engine::ensure_rotation() {
@@ -223,15 +224,15 @@ void Engine::ensure_rotation() {
     bool made = false;
     if (rotation_host_.empty()) {
         start_rotation_draws();
-        if (draws_done_.get()) {
-            float* dst = mt_dev_.ensure(d_ * d_);   // (not needed for the transpose yet)
-            const float* draws = dst;
-            for (const auto& piece : draws_->pieces()) {
-                SKM_CUDA(cudaMemcpyAsync(dst, piece.values, sizeof(float) * piece.count, cudaMemcpyHostToDevice, stream_));
-                dst += piece.count;
-            }
-            made = make_rotation_matrix_on_device(draws, d_, m, stream_);
+        float* draws = mt_dev_.ensure(d_ * d_);   // (not needed for the transpose yet)
+        size_t got = 0;
+        for (size_t t = 0; t < draws_->pieces() && got < d_ * d_; ++t) {
+            const auto piece = draws_->piece(t);
+            const size_t n = std::min(piece.count, d_ * d_ - got);
+            SKM_CUDA(cudaMemcpyAsync(draws + got, piece.values, sizeof(float) * n, cudaMemcpyHostToDevice, stream_));
+            got += n;
         }
+        made = got == d_ * d_ && make_rotation_matrix_on_device(draws, d_, m, stream_);
         if (!made) rotation_host_ = make_rotation_matrix(d_, cfg_.seed);
     }
     if (!made) SKM_CUDA(cudaMemcpyAsync(m, rotation_host_.data(), sizeof(float) * d_ * d_, cudaMemcpyHostToDevice, stream_));
@@ -1025,9 +1026,11 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
             }
             const size_t tile_bytes = kListsPerTile * static_cast<size_t>(cap_group) * sizeof(uint2);
             const size_t n_tiles = (p.n + kTileM - 1) / kTileM;
-            const size_t list_bytes_cap = static_cast<size_t>(6) << 30;
-            // at least one tile per batch; when even one tile's lists exceed the cap (k in the millions) the batch is that one tile
-            const size_t per_batch = std::min(n_tiles, std::max<size_t>(1, list_bytes_cap / tile_bytes));
+            // Equal batches of at most 2.5 GB of lists (of one tile, when even that has more): more would push blocks that a Train
+            // takes and gives back out of the parked pool, and cudaMalloc costs more than a second launch.
+            const size_t list_bytes_cap = static_cast<size_t>(5) << 29;
+            const size_t n_batches = std::min(n_tiles, (n_tiles * tile_bytes + list_bytes_cap - 1) / list_bytes_cap);
+            const size_t per_batch = (n_tiles + n_batches - 1) / n_batches;
             uint2* lists = b.tc_lists.ensure(per_batch * kListsPerTile * cap_group);
             uint32_t* offs = b.tc_list_offs.ensure(per_batch * kListsPerTile * (n_chunks + 1));
             // d' moves below vertical_d from pass to pass: the points are split that far, once
@@ -1541,6 +1544,10 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
     if (rotate || cfg_.unrotate_centroids) start_rotation_draws();
     partial_d_ = initial_partial_d(vertical_d_);
     const uint32_t initial_pd = partial_d_;
+    // The shuffles behind the first centroids and the sample run on threads of their own meanwhile.
+    std::future<std::vector<size_t>> meso_forgy = std::async(std::launch::async, [n_all, k = n_meso_, seed = cfg_.seed] { return forgy_indices(n_all, k, seed); });
+    std::future<std::vector<size_t>> sampling;
+    if (n_all < n) sampling = std::async(std::launch::async, [n, seed = cfg_.seed] { return sampling_permutation(n, seed); });
 
     c_cur_.ensure(k_ * d_);
     c_prev_.ensure(k_ * d_);
@@ -1564,9 +1571,11 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
     prepare_update_workspace(n_all, k_);
 
     // ---- phase 1: mesoclustering (:161-257)
-    generate_centroids_from_host(data, on_device, n_all, n_meso_, rotate);
-    if (n_all < n) sampled_indices_ = sampling_permutation(n, cfg_.seed);
-    load_rows(data, on_device, n_all < n ? sampled_indices_.data() : nullptr, n_all, rotate, x_rot_.get());
+    load_rows(data, on_device, n_all < n ? (sampled_indices_ = sampling.get()).data() : nullptr, n_all, rotate, x_rot_.get());
+    {
+        const std::vector<size_t> idx = meso_forgy.get();
+        generate_centroids_from_host(data, on_device, n_all, n_meso_, rotate, &idx);
+    }
     launch_row_sqnorms(x_rot_.get(), n_all, d_, d_, data_norms_.get(), stream_);
     SKM_CUDA(cudaMemcpyAsync(full_norms_.get(), data_norms_.get(), sizeof(float) * n_all, cudaMemcpyDeviceToDevice, stream_));
 
@@ -1623,21 +1632,29 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
     // Mesoclusters that never prune share their launches (train_fine_run); snapshots are per mesocluster and iteration.
     auto shares = [&](size_t m) { return fine_nums[m] > 0 && rows_of[m] >= fine_nums[m] && gemm_only(fine_nums[m]) && !trace_on_ && tc::enabled() && d_ <= 16384; };
     const size_t run_rows = (size_t{4} << 30) / (sizeof(float) * d_);   // of a run, unless one mesocluster has more
-    // The Forgy rows of every mesocluster (a shuffle of its member positions each) are drawn ahead by a host thread.
+    // The Forgy rows of every mesocluster (a shuffle of its member positions each) are drawn ahead by host threads.
     std::vector<std::vector<size_t>> forgy(n_meso_);
-    std::atomic<size_t> forgy_done{0};
-    std::thread forgy_thread([&, seed = cfg_.seed] {
-        for (size_t m = 0; m < n_meso_; ++m) {
-            if (fine_nums[m] != 0) forgy[m] = forgy_indices(rows_of[m], fine_nums[m], seed);
-            forgy_done.store(m + 1, std::memory_order_release);
-        }
-    });
+    std::vector<std::atomic<bool>> forgy_done(n_meso_);
+    std::atomic<size_t> forgy_next{0};
+    std::vector<std::thread> forgy_threads;
     struct Joiner {
-        std::thread& t;
+        std::vector<std::thread>& threads;
         ~Joiner() {
-            if (t.joinable()) t.join();
+            for (auto& t : threads) t.join();
         }
-    } joiner{forgy_thread};
+    } joiner{forgy_threads};
+    const size_t n_forgy_threads = n_all < 20'000 ? 1 : std::min<size_t>({6, n_meso_, std::max(1u, std::thread::hardware_concurrency())});   // (4 ns a row, 20 us a thread)
+    for (size_t t = 0; t < n_forgy_threads; ++t) {
+        forgy_threads.emplace_back([&, seed = cfg_.seed] {
+            for (size_t m; (m = forgy_next.fetch_add(1)) < n_meso_;) {
+                if (fine_nums[m] != 0) forgy[m] = forgy_indices(rows_of[m], fine_nums[m], seed);
+                forgy_done[m].store(true, std::memory_order_release);
+            }
+        });
+    }
+    auto wait_for_forgy = [&](size_t m) {
+        while (!forgy_done[m].load(std::memory_order_acquire)) std::this_thread::yield();
+    };
     size_t fine_offset = 0;
     for (size_t m = 0; m < n_meso_; ++m) {
         const size_t n_fine = fine_nums[m];
@@ -1649,7 +1666,7 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
                 clusters += fine_nums[last];
                 ++last;
             }
-            while (forgy_done.load(std::memory_order_acquire) < last) std::this_thread::yield();
+            for (size_t f = m; f < last; ++f) wait_for_forgy(f);
             partial_d_ = initial_pd;
             train_fine_run(m, last, offsets, rows_of, fine_nums, forgy, fine_offset);
             fine_offset += clusters;
@@ -1667,7 +1684,7 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
         const uint64_t* idx = meso_indices_dev_.get() + offsets[m];
         launch_gather_rows(x_rot_.get(), idx, meso_buffer_.get(), msize, d_, stream_);      // CompactMesoclusterToBuffer (:685-704)
         launch_gather_f32(full_norms_.get(), idx, meso_norms_.get(), msize, stream_);
-        while (forgy_done.load(std::memory_order_acquire) <= m) std::this_thread::yield();
+        wait_for_forgy(m);
         generate_centroids_from_device_rows(meso_buffer_.get(), msize, n_fine, &forgy[m]);
 
         const bool always_gemm_only = gemm_only(n_fine);

@@ -302,7 +302,7 @@ class Engine {
     float epsilon0_;
     std::vector<float> rotation_host_;  // d x d, empty until needed (a matrix made on the device is fetched on demand)
     std::unique_ptr<NormalDraws> draws_;   // of a matrix that is being made
-    std::future<bool> draws_done_;
+    std::future<void> draws_done_;
     PinnedBuffer<uint32_t> draw_bits_;
     PinnedBuffer<float> draw_values_;
     bool rotation_ready_ = false;

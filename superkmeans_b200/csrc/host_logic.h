@@ -6,6 +6,7 @@
 #pragma once
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstddef>
 #include <cstdint>
@@ -98,27 +99,97 @@ inline size_t n_vectors_to_sample(size_t n, size_t k, float sampling_fraction, u
     return std::min(by_n, by_clusters);
 }
 
-// Forgy initialisation (superkmeans.h:1110-1123): the first k entries of std::shuffle applied to
-// [0, n_points) with std::mt19937(seed).  std::shuffle is library-specific; this engine and the
-// oracle are both built with libstdc++.
-inline std::vector<size_t> forgy_indices(size_t n_points, size_t k, uint32_t seed) {
-    std::mt19937 rng(seed);
-    std::vector<size_t> indices(n_points);
-    std::iota(indices.begin(), indices.end(), size_t{0});
-    std::shuffle(indices.begin(), indices.end(), rng);
-    indices.resize(std::min(k, n_points));
-    return indices;
-}
+// The outputs of std::mt19937(seed) (Matsumoto and Nishimura's generator), a block of 624 at a time in loops without
+// dependencies from one element to the next, which the compiler vectorises: 0.55 us a block with the vectors every x86-64 has
+// (std::mt19937 takes 2.5), 0.3 us with AVX2.
+class Mt19937Blocks {
+  public:
+    static constexpr size_t N = 624;
+    explicit Mt19937Blocks(uint32_t seed) {
+        x_[0] = seed;
+        for (size_t i = 1; i < N; ++i) x_[i] = 1812433253u * (x_[i - 1] ^ (x_[i - 1] >> 30)) + static_cast<uint32_t>(i);
+    }
+    // the next N outputs
+    void next(uint32_t* out) {
+#if defined(__x86_64__)
+        static const bool avx2 = __builtin_cpu_supports("avx2");
+        if (avx2) return next_avx2(x_, out);
+#endif
+        step(x_, out);
+    }
 
-// Sampling permutation (superkmeans.h:1402-1407): a full shuffle of [0, n); the first n_samples
-// entries are the sample.
-inline std::vector<size_t> sampling_permutation(size_t n, uint32_t seed) {
-    std::mt19937 rng(seed);
+  private:
+    static inline __attribute__((always_inline)) uint32_t twist(uint32_t hi, uint32_t lo) {
+        const uint32_t v = (hi & 0x80000000u) | (lo & 0x7FFFFFFFu);
+        return (v >> 1) ^ ((0u - (v & 1u)) & 0x9908B0DFu);
+    }
+    static inline __attribute__((always_inline)) void step(uint32_t* x, uint32_t* out) {
+        constexpr size_t M = 397;
+        uint32_t y[N];
+        for (size_t i = 0; i < N - M; ++i) y[i] = x[i + M] ^ twist(x[i], x[i + 1]);
+        for (size_t i = N - M; i < 2 * (N - M); ++i) y[i] = y[i - (N - M)] ^ twist(x[i], x[i + 1]);
+        for (size_t i = 2 * (N - M); i < N - 1; ++i) y[i] = y[i - (N - M)] ^ twist(x[i], x[i + 1]);
+        y[N - 1] = y[M - 1] ^ twist(x[N - 1], y[0]);
+        for (size_t i = 0; i < N; ++i) {
+            uint32_t v = y[i];
+            x[i] = v;
+            v ^= v >> 11;
+            v ^= (v << 7) & 0x9D2C5680u;
+            v ^= (v << 15) & 0xEFC60000u;
+            out[i] = v ^ (v >> 18);
+        }
+    }
+#if defined(__x86_64__)
+    static __attribute__((target("avx2"))) void next_avx2(uint32_t* x, uint32_t* out) { step(x, out); }
+#endif
+    uint32_t x_[N];
+};
+
+// The same outputs one by one: a generator that std::shuffle takes in place of std::mt19937, with the same result.
+class Mt19937Stream {
+  public:
+    using result_type = uint32_t;
+    explicit Mt19937Stream(uint32_t seed) : blocks_(seed) {}
+    static constexpr result_type min() { return 0; }
+    static constexpr result_type max() { return 0xFFFFFFFFu; }
+    result_type operator()() {
+        if (at_ == Mt19937Blocks::N) {
+            blocks_.next(out_);
+            at_ = 0;
+        }
+        return out_[at_++];
+    }
+
+  private:
+    Mt19937Blocks blocks_;
+    uint32_t out_[Mt19937Blocks::N];
+    size_t at_ = Mt19937Blocks::N;
+};
+
+// The first k entries of std::shuffle applied to [0, n) with std::mt19937(seed); 32-bit entries while they suffice, because
+// the shuffle waits for memory.
+inline std::vector<size_t> shuffled_indices(size_t n, size_t k, uint32_t seed) {
+    Mt19937Stream rng(seed);
+    if (n <= 0xFFFFFFFFu) {
+        std::vector<uint32_t> idx(n);
+        std::iota(idx.begin(), idx.end(), 0u);
+        std::shuffle(idx.begin(), idx.end(), rng);
+        return std::vector<size_t>(idx.begin(), idx.begin() + static_cast<std::ptrdiff_t>(std::min(k, n)));
+    }
     std::vector<size_t> idx(n);
     std::iota(idx.begin(), idx.end(), size_t{0});
     std::shuffle(idx.begin(), idx.end(), rng);
+    idx.resize(std::min(k, n));
     return idx;
 }
+
+// Forgy initialisation (superkmeans.h:1110-1123).  std::shuffle is library-specific; this engine and the oracle are both
+// built with libstdc++.
+inline std::vector<size_t> forgy_indices(size_t n_points, size_t k, uint32_t seed) { return shuffled_indices(n_points, k, seed); }
+
+// Sampling permutation (superkmeans.h:1402-1407): a full shuffle of [0, n); the first n_samples
+// entries are the sample.
+inline std::vector<size_t> sampling_permutation(size_t n, uint32_t seed) { return shuffled_indices(n, n, seed); }
 
 // One row operation produced by the split logic, applied to the row-major centroid matrix in list
 // order by a device kernel (each dimension independently).
@@ -301,42 +372,6 @@ inline std::vector<size_t> arrange_fine_clusters(size_t n_clusters, size_t n_mes
     return out;
 }
 
-// The outputs of std::mt19937(seed) (Matsumoto and Nishimura's generator), a block of 624 at a time in loops without
-// dependencies from one element to the next, which the compiler vectorises: 3 million in 2 - 4 ms where std::mt19937
-// takes 12.
-class Mt19937Blocks {
-  public:
-    static constexpr size_t N = 624;
-    explicit Mt19937Blocks(uint32_t seed) {
-        x_[0] = seed;
-        for (size_t i = 1; i < N; ++i) x_[i] = 1812433253u * (x_[i - 1] ^ (x_[i - 1] >> 30)) + static_cast<uint32_t>(i);
-    }
-    // the next N outputs
-    void next(uint32_t* out) {
-        constexpr size_t M = 397;
-        uint32_t y[N];
-        for (size_t i = 0; i < N - M; ++i) y[i] = x_[i + M] ^ twist(x_[i], x_[i + 1]);
-        for (size_t i = N - M; i < 2 * (N - M); ++i) y[i] = y[i - (N - M)] ^ twist(x_[i], x_[i + 1]);
-        for (size_t i = 2 * (N - M); i < N - 1; ++i) y[i] = y[i - (N - M)] ^ twist(x_[i], x_[i + 1]);
-        y[N - 1] = y[M - 1] ^ twist(x_[N - 1], y[0]);
-        for (size_t i = 0; i < N; ++i) {
-            uint32_t v = y[i];
-            x_[i] = v;
-            v ^= v >> 11;
-            v ^= (v << 7) & 0x9D2C5680u;
-            v ^= (v << 15) & 0xEFC60000u;
-            out[i] = v ^ (v >> 18);
-        }
-    }
-
-  private:
-    static uint32_t twist(uint32_t hi, uint32_t lo) {
-        const uint32_t v = (hi & 0x80000000u) | (lo & 0x7FFFFFFFu);
-        return (v >> 1) ^ ((0u - (v & 1u)) & 0x9908B0DFu);
-    }
-    uint32_t x_[N];
-};
-
 // A source of random bits that reads prepared ones.
 struct BitsFromArray {
     using result_type = uint32_t;
@@ -347,68 +382,108 @@ struct BitsFromArray {
 };
 
 // The first `count` draws of std::normal_distribution<float>(0, 1) from std::mt19937(seed), made by several threads.
-// libstdc++ takes the bits two at a time until a pair is accepted and makes two draws of it, so a thread can start at any
-// even position of the bit sequence: thread t makes the draws of the pairs accepted in its stretch, while the next stretch
-// of bits is being generated.
+// libstdc++ uses Marsaglia's polar method: it takes the bits two at a time, accepts the pair if the point lies in the unit
+// disc, and makes two draws of it.  So any even position of the bits is a place to start: one thread generates them (the
+// only serial part, and the bound: 1.3 ms for the 3 million that d = 1536 needs), the others make the draws of one short stretch
+// after the other, and whoever uses them can begin before the last is made.  First which pairs are accepted, without
+// branches, then the logarithms: 3.5 ns a draw, against 10 in one loop that mispredicts every fifth pair.
 class NormalDraws {
   public:
     NormalDraws(size_t count, uint32_t seed) : count_(count), seed_(seed) {
-        threads_ = count < (size_t{1} << 15) ? 1u : std::min(16u, std::max(1u, std::thread::hardware_concurrency()));
+        threads_ = count < (size_t{1} << 15) ? 1u : std::min(8u, std::max(1u, std::thread::hardware_concurrency()));   // (more wait for the generator)
         // a pair is accepted with probability pi / 4; half a percent and 2000 pairs more than needed are a dozen standard deviations
         const double pairs = static_cast<double>((count + 1) / 2) / 0.7853 * 1.005 + 2000.0;
-        blocks_ = static_cast<size_t>(2.0 * pairs / Mt19937Blocks::N / threads_) + 1;
+        const size_t blocks = static_cast<size_t>(2.0 * pairs / Mt19937Blocks::N) + 1;
+        blocks_ = std::max<size_t>(16, (blocks + 47) / 48);
+        stretches_ = (blocks + blocks_ - 1) / blocks_;
+        made_.reset(new std::atomic<size_t>[stretches_]);
+        for (size_t t = 0; t < stretches_; ++t) made_[t].store(kNotYet);
     }
     // Words of scratch for make(), which writes draws into `values` (the same number of floats).
-    size_t scratch() const { return (blocks_ * threads_ + 1) * Mt19937Blocks::N; }
-    // False in the (practically impossible) case that the bits did not suffice.
-    bool make(uint32_t* bits, float* values) {
-        const size_t stretch = blocks_ * Mt19937Blocks::N;
-        std::vector<size_t> made(threads_, 0);
-        auto work = [&](unsigned t) {
-            const uint32_t* end = bits + (t + 1) * stretch;
-            float* out = values + t * stretch;
-            size_t n = 0;
-            BitsFromArray source{bits + t * stretch};
-            std::normal_distribution<float> draw(0.0f, 1.0f);
-            while (source.next < end) {
-                const float first = draw(source);   // (a pair is accepted long before the block behind the last stretch ends)
-                if (source.next > end) break;       // accepted in the next stretch
-                out[n++] = first;
-                out[n++] = draw(source);
+    size_t scratch() const { return stretches_ * blocks_ * Mt19937Blocks::N; }
+    // (before piece() is called)
+    void values_at(float* values) { values_ = values; }
+    void make(uint32_t* bits, float* values) {
+        std::atomic<size_t> generated{0}, taken{0};
+        auto work = [&] {
+            for (size_t t; (t = taken.fetch_add(1)) < stretches_;) {
+                while (generated.load(std::memory_order_acquire) <= t) std::this_thread::yield();
+                made_[t].store(draw_stretch(bits + t * stretch(), values + t * stretch()), std::memory_order_release);
             }
-            made[t] = n;
         };
-        Mt19937Blocks generator(seed_);
+        // (starting a thread takes longer than a stretch: the first starts the others)
         std::vector<std::thread> pool;
-        size_t generated = 0;
-        for (unsigned t = 0; t < threads_; ++t) {
-            for (; generated < (t + 1) * blocks_ + 1; ++generated) generator.next(bits + generated * Mt19937Blocks::N);
-            if (t + 1 < threads_) pool.emplace_back(work, t);
-            else work(t);
+        std::thread starter;
+        try {
+            if (threads_ > 1) {
+                starter = std::thread([&] {
+                    try {
+                        for (unsigned t = 2; t < threads_; ++t) pool.emplace_back(work);
+                    } catch (...) {
+                        // (fewer threads then)
+                    }
+                    work();
+                });
+            }
+        } catch (...) {
         }
+        Mt19937Blocks generator(seed_);
+        for (size_t t = 0; t < stretches_; ++t) {
+            for (size_t b = 0; b < blocks_; ++b) generator.next(bits + t * stretch() + b * Mt19937Blocks::N);
+            generated.store(t + 1, std::memory_order_release);
+        }
+        work();
+        if (starter.joinable()) starter.join();
         for (auto& th : pool) th.join();
-        pieces_.clear();
-        size_t total = 0;
-        for (unsigned t = 0; t < threads_ && total < count_; ++t) {
-            const size_t take = std::min(made[t], count_ - total);
-            pieces_.push_back({values + t * stretch, take});
-            total += take;
-        }
-        return total == count_;
     }
     struct Piece {
         const float* values;
         size_t count;
     };
-    // The draws in order, as pieces of `values`.
-    const std::vector<Piece>& pieces() const { return pieces_; }
+    // The draws in order, as up to pieces() pieces of `values`; piece(t) waits until make() has come to it.
+    size_t pieces() const { return stretches_; }
+    Piece piece(size_t t) const {
+        size_t n;
+        while ((n = made_[t].load(std::memory_order_acquire)) == kNotYet) std::this_thread::yield();
+        return {values_ + t * stretch(), n};
+    }
 
   private:
+    static constexpr size_t kNotYet = ~size_t{0};
+    size_t stretch() const { return blocks_ * Mt19937Blocks::N; }
+    size_t draw_stretch(const uint32_t* bits, float* out) const {
+        constexpr size_t kBatch = 512;
+        float x[kBatch], y[kBatch], r2[kBatch];
+        BitsFromArray source{bits};
+        size_t n = 0;
+        for (size_t left = stretch() / 2; left > 0;) {
+            const size_t pairs = std::min(left, kBatch);
+            left -= pairs;
+            size_t m = 0;
+            for (size_t i = 0; i < pairs; ++i) {
+                const float a = 2.0f * std::generate_canonical<float, 24>(source) - 1.0f;
+                const float b = 2.0f * std::generate_canonical<float, 24>(source) - 1.0f;
+                const float r = a * a + b * b;
+                x[m] = a;
+                y[m] = b;
+                r2[m] = r;
+                m += static_cast<size_t>((r <= 1.0f) & (r != 0.0f));
+            }
+            for (size_t i = 0; i < m; ++i) {
+                const float mult = std::sqrt(-2.0f * std::log(r2[i]) / r2[i]);
+                out[n++] = y[i] * mult;
+                out[n++] = x[i] * mult;
+            }
+        }
+        return n;
+    }
     size_t count_;
     uint32_t seed_;
     unsigned threads_;
-    size_t blocks_;   // generator blocks per stretch
-    std::vector<Piece> pieces_;
+    size_t blocks_;      // generator blocks per stretch
+    size_t stretches_;
+    std::unique_ptr<std::atomic<size_t>[]> made_;   // draws of a stretch
+    float* values_ = nullptr;
 };
 
 inline std::vector<float> normal_draws(size_t count, uint32_t seed) {
@@ -417,9 +492,14 @@ inline std::vector<float> normal_draws(size_t count, uint32_t seed) {
     std::unique_ptr<float[]> values(new float[draws.scratch()]);
     std::vector<float> out;
     out.reserve(count);
-    if (draws.make(bits.get(), values.get())) {
-        for (const auto& p : draws.pieces()) out.insert(out.end(), p.values, p.values + p.count);
-    } else {
+    draws.values_at(values.get());
+    draws.make(bits.get(), values.get());
+    for (size_t t = 0; t < draws.pieces() && out.size() < count; ++t) {
+        const auto p = draws.piece(t);
+        out.insert(out.end(), p.values, p.values + std::min(p.count, count - out.size()));
+    }
+    if (out.size() < count) {   // (practically impossible: too many pairs rejected)
+        out.clear();
         std::mt19937 gen(seed);
         std::normal_distribution<float> dist(0.0f, 1.0f);
         for (size_t i = 0; i < count; ++i) out.push_back(dist(gen));

@@ -15,9 +15,9 @@
 //
 // Steps 1 and 3 are right-looking over 32-wide panels with one launch per panel: every block of the trailing matrix
 // recomputes the 32 x 32 products it needs of the panel (three small products instead of one, against a launch and a
-// round trip saved), and the block that holds the next diagonal factorises it at once.  Measured (kernels, one B200): d = 768 1.9 ms,
-// d = 1536 6.2 ms; of those 0.7 and 2.5 ms are the solve of step 1 (latency of L2 loads and FMA chains), 0.75 and 1.9 ms
-// the two chains of d / 32 dependent launches.
+// round trip saved), and the block that holds the next diagonal factorises it at once.  Measured (kernels, one B200): d = 768
+// 1.3 ms, of which 0.25 ms are the solve of step 1 (0.88 with one batch of loads in flight instead of four; d = 1536: 2.5 - 3.0 ms
+// before) and 0.75 ms (d = 1536: 1.9) the two chains of d / 32 dependent launches.
 //
 // A matrix too close to singular for this (or too wide for step 1's row buffer) is declined: the caller takes the host's.
 #include <cmath>
@@ -307,26 +307,39 @@ __global__ void __launch_bounds__(kThreads) solve_rows_kernel(const double* __re
 #pragma unroll
         for (int u = 0; u < kRowsPerWarp; ++u) acc[u] = a[row[u] * dp + kb + lane];
         const double* __restrict__ rp = r + kb + lane;
-        for (size_t j0 = 0; j0 < kb; j0 += 16) {
-            double rv[16];
+        // four batches of loads in flight: the loop waits for L2, not for the FMAs
+        double rv[4][16];
+        auto load = [&](double (&v)[16], size_t j0) {
+            if (j0 >= kb) return;
 #pragma unroll
-            for (int q = 0; q < 16; ++q) rv[q] = __ldg(rp + (j0 + q) * dp);
+            for (int q = 0; q < 16; ++q) v[q] = __ldg(rp + (j0 + q) * dp);
+        };
 #pragma unroll
-            for (int q = 0; q < 16; ++q)
+        for (int b = 0; b < 4; ++b) load(rv[b], 16 * b);
+        for (size_t j0 = 0; j0 < kb; j0 += 64) {
 #pragma unroll
-                for (int u = 0; u < kRowsPerWarp; ++u) part[u][q & 3] = fma(mine[u][j0 + q], rv[q], part[u][q & 3]);
+            for (int b = 0; b < 4; ++b) {
+                const size_t j = j0 + 16 * b;
+                if (j >= kb) break;
+#pragma unroll
+                for (int q = 0; q < 16; ++q)
+#pragma unroll
+                    for (int u = 0; u < kRowsPerWarp; ++u) part[u][q & 3] = fma(mine[u][j + q], rv[b][q], part[u][q & 3]);
+                load(rv[b], j + 64);
+            }
         }
+        const double* __restrict__ inv = inverses + (kb / NB) * NB * NB + lane;
+        double iv[NB];
+#pragma unroll
+        for (int b = 0; b < NB; ++b) iv[b] = __ldg(inv + b * NB);
 #pragma unroll
         for (int u = 0; u < kRowsPerWarp; ++u) rest[warp][u][lane] = acc[u] - ((part[u][0] + part[u][1]) + (part[u][2] + part[u][3]));
         __syncwarp();
-        const double* __restrict__ inv = inverses + (kb / NB) * NB * NB + lane;
         double x[kRowsPerWarp] = {};
-#pragma unroll 8
-        for (int b = 0; b < NB; ++b) {
-            const double iv = __ldg(inv + b * NB);
 #pragma unroll
-            for (int u = 0; u < kRowsPerWarp; ++u) x[u] = fma(rest[warp][u][b], iv, x[u]);
-        }
+        for (int b = 0; b < NB; ++b)
+#pragma unroll
+            for (int u = 0; u < kRowsPerWarp; ++u) x[u] = fma(rest[warp][u][b], iv[b], x[u]);
 #pragma unroll
         for (int u = 0; u < kRowsPerWarp; ++u) {
             mine[u][kb + lane] = x[u];
