@@ -80,8 +80,9 @@ __global__ void __launch_bounds__(256) group_shift_kernel(const float* __restric
         const float* pa = a + static_cast<size_t>(g.y0 + c) * d;
         const float* pb = b + static_cast<size_t>(g.y0 + c) * d;
         float s = 0.f;
+#pragma unroll 8   // (bound by the latency of its loads)
         for (size_t j = lane; j < d; j += 32) {
-            const float t = pa[j] - pb[j];
+            const float t = __ldg(pa + j) - __ldg(pb + j);
             s = fmaf(t, t, s);
         }
         total += static_cast<double>(warp_sum(s));

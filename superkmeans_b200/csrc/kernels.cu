@@ -1010,14 +1010,26 @@ __global__ void __launch_bounds__(256) consolidate_kernel(const ConsolidateParam
         }
         const float scale = p.normalize ? 1.0f : mult;
         float s = 0.f;
-#pragma unroll 4
-        for (size_t j = lane; j < p.d; j += 32) {
-            const float val = __fmul_rn(c[j], scale);
-            c[j] = val;
-            pdx[pdx_offset(j, v, cs, p.vertical_d)] = val;
-            if (j < p.vertical_d) aux[j] = val;
-            const float t = val - prev[j];
-            s = fmaf(t, t, s);
+        constexpr int U = 8;   // loads in flight: the stores between them would hold them up
+        for (size_t j0 = lane; j0 < p.d; j0 += 32 * U) {
+            float cv[U], pv[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const size_t j = min(j0 + 32 * u, p.d - 1);
+                cv[u] = c[j];
+                pv[u] = prev[j];
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const size_t j = j0 + 32 * u;
+                if (j >= p.d) break;
+                const float val = __fmul_rn(cv[u], scale);
+                c[j] = val;
+                pdx[pdx_offset(j, v, cs, p.vertical_d)] = val;
+                if (j < p.vertical_d) aux[j] = val;
+                const float t = val - pv[u];
+                s = fmaf(t, t, s);
+            }
         }
         s = warp_sum(s);
         total += static_cast<double>(s);

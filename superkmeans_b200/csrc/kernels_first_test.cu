@@ -10,8 +10,10 @@
 //   warp 0     TMA producer: 128 x 64 halves of each of the four parts per stage, three stages;
 //   warp 1     MMA issuer (leader only), two accumulators of 256 columns;
 //   warps 2-17 test, a warp per 32 rows and 64 columns: partial distance = ||x||^2 + ||c||^2 - 2 x.c, survivors appended to
-//              the warp's list.  The test is latency-bound (270 instructions per 32 columns, a scan and a walk over the
-//              survivors' bits among them), hence four warps per scheduler: with two it took 6500 cycles per tile.
+//              the warp's list.  The test is what bounds the kernel, its latency more than its 200 instructions per 32
+//              columns: hence four warps per scheduler (with two it took 6500 cycles per tile), two columns per instruction
+//              and no scan for the places in the list.  1M x 1024, k = 4000, nine passes: 27.2 ms with one column per
+//              instruction and a scan by shuffles, 25.0 so.
 // Every wait is bounded (see kernels_tc.cu).
 #include <cfloat>
 #include <cmath>
@@ -38,6 +40,7 @@ constexpr uint32_t T_SMEM_BYTES = T_STAGES * T_STAGE_BYTES + T_CTRL_BYTES + 1024
 struct TestCtrl {
     alignas(16) float ny[4][2][256];   // per row quarter and accumulator
     float column[T_TEST_WARPS][8 * 32];   // per test warp: 8 values of each of its lanes
+    uint32_t filled[T_TEST_WARPS];
     uint64_t full[T_STAGES];           // (the leader's are used)
     uint64_t empty[T_STAGES];
     uint64_t acc_full[2];
@@ -46,13 +49,26 @@ struct TestCtrl {
 };
 static_assert(sizeof(TestCtrl) <= T_CTRL_BYTES, "control block too large");
 
+// pairs of floats
+__device__ __forceinline__ uint64_t pack2(float a, float b) { return static_cast<uint64_t>(__float_as_uint(a)) | static_cast<uint64_t>(__float_as_uint(b)) << 32; }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
 struct TestMaps {
     CUtensorMap xhi, xlo, yhi, ylo;
 };
 
 struct TestParams {
     size_t n, k;
-    uint32_t k_blocks;
+    uint32_t k_blocks, partial_d;
     size_t tile0, n_tiles;       // of 128 rows
     const uint32_t* tile_map;    // null: tile0, tile0 + 1, ...
     const float* factor_x;       // per row: -2 / scale
@@ -165,8 +181,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T_THREADS, 1) first_
                         }
                         tc_fence_after();
                         const uint32_t st = smem_base + s * T_STAGE_BYTES;
-#pragma unroll
-                        for (uint32_t kk = 0; kk < TK / 16; ++kk) {
+                        // (nothing but zeros behind partial_d)
+                        const uint32_t steps = min(static_cast<uint32_t>(TK / 16), (p.partial_d - kb * TK + 15) / 16);
+                        for (uint32_t kk = 0; kk < steps; ++kk) {
                             const uint64_t xh = make_desc_128(st + kk * 32), xl = make_desc_128(st + T_PART_BYTES + kk * 32);
                             const uint64_t yh = make_desc_128(st + 2 * T_PART_BYTES + kk * 32), yl = make_desc_128(st + 3 * T_PART_BYTES + kk * 32);
                             umma_f16_pair(acc, xh, yh, (kb | kk) != 0 ? 1u : 0u, idesc);
@@ -183,6 +200,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T_THREADS, 1) first_
         const uint32_t quarter = warp & 3, part = static_cast<uint32_t>(warp - 2) >> 2;   // rows 32 quarter.., columns 64 part..
         const uint32_t lane_base = 32u * quarter;
         float* column = ctrl->column[warp - 2] + lane;
+        uint32_t* filled = &ctrl->filled[warp - 2];   // pairs in the warp's list
         const float fy = *p.factor_y;
         uint32_t u = 0;
         bool ok = true;
@@ -193,17 +211,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T_THREADS, 1) first_
             const bool valid = listed && row < p.n;
             const float nx = valid ? p.norms_x[row] : 0.f;
             const float factor = valid ? p.factor_x[row] * fy : 0.f;
+            const uint64_t nx2 = pack2(nx, nx), factor2 = pack2(factor, factor);
             float thr = valid && !(p.flags && p.flags[row]) ? p.best_in[row] * p.ratio_first : -FLT_MAX;
             uint32_t survivors = 0;
             const size_t group = (listed ? q : 0) * kListsPerTile + part * 4 + quarter;
             uint2* my_list = p.lists + group * p.cap_group;
             uint32_t* my_offs = p.list_offs + group * ((p.k + 1023) / 1024 + 1);
-            uint32_t filled = 0;   // warp-uniform
+            if (lane == 0) *filled = 0;
+            __syncwarp();
             for (uint32_t nt = 0; nt < col_tiles && ok; ++nt, ++u) {
                 const uint32_t b = u & 1u, uph = (u >> 1) & 1u;
                 const uint32_t col0 = nt * 256 + part * 64;
                 float* ny = ctrl->ny[quarter][b] + part * 64;   // the four warps of a quarter fill (and read) their own parts
-                if ((nt & 3u) == 0 && lane == 0 && listed) my_offs[nt >> 2] = filled;
+                if ((nt & 3u) == 0 && lane == 0 && listed) my_offs[nt >> 2] = *filled;
 #pragma unroll
                 for (int i = 0; i < 2; ++i) ny[i * 32 + lane] = col0 + i * 32 + lane < p.k ? __ldg(p.norms_y + col0 + i * 32 + lane) : INFINITY;   // never below a threshold
                 __syncwarp();
@@ -213,39 +233,38 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T_THREADS, 1) first_
                 }
                 tc_fence_after();
                 const uint32_t taddr = tmem_base + (lane_base << 16) + b * 256 + part * 64;
+                const uint64_t minus_thr2 = pack2(-thr, -thr);
                 auto test = [&](uint32_t (&r)[32], int ch) {
-                    uint32_t mask = 0;
+                    // two columns per instruction; the sign of (distance - threshold) is the column's bit
+                    uint32_t bits[4] = {0, 0, 0, 0};
 #pragma unroll
-                    for (int j = 0; j < 32; j += 4) {
-                        const float4 nyv = *reinterpret_cast<const float4*>(ny + ch * 32 + j);
-                        const float p0 = fmaf(factor, __uint_as_float(r[j + 0]), nx) + nyv.x;
-                        const float p1 = fmaf(factor, __uint_as_float(r[j + 1]), nx) + nyv.y;
-                        const float p2 = fmaf(factor, __uint_as_float(r[j + 2]), nx) + nyv.z;
-                        const float p3 = fmaf(factor, __uint_as_float(r[j + 3]), nx) + nyv.w;
-                        r[j + 0] = __float_as_uint(p0);
-                        r[j + 1] = __float_as_uint(p1);
-                        r[j + 2] = __float_as_uint(p2);
-                        r[j + 3] = __float_as_uint(p3);
-                        mask |= (p0 < thr ? (1u << j) : 0u) | (p1 < thr ? (2u << j) : 0u) | (p2 < thr ? (4u << j) : 0u) | (p3 < thr ? (8u << j) : 0u);
+                    for (int h = 0; h < 4; ++h) {
+                        const float4 n0 = *reinterpret_cast<const float4*>(ny + ch * 32 + 8 * h), n1 = *reinterpret_cast<const float4*>(ny + ch * 32 + 8 * h + 4);
+                        const uint64_t nyv[4] = {pack2(n0.x, n0.y), pack2(n0.z, n0.w), pack2(n1.x, n1.y), pack2(n1.z, n1.w)};
+#pragma unroll
+                        for (int q = 3; q >= 0; --q) {
+                            uint32_t& lo = r[8 * h + 2 * q];
+                            uint32_t& hi = r[8 * h + 2 * q + 1];
+                            const uint64_t pd = add2(fma2(factor2, pack2(__uint_as_float(lo), __uint_as_float(hi)), nx2), nyv[q]);
+                            const uint64_t over = add2(pd, minus_thr2);
+                            lo = static_cast<uint32_t>(pd);
+                            hi = static_cast<uint32_t>(pd >> 32);
+                            bits[h] = __funnelshift_l(static_cast<uint32_t>(over >> 32), bits[h], 1);
+                            bits[h] = __funnelshift_l(static_cast<uint32_t>(over), bits[h], 1);
+                        }
                     }
+                    const uint32_t mask = bits[0] | bits[1] << 8 | bits[2] << 16 | bits[3] << 24;
                     if (!__any_sync(0xffffffffu, mask != 0)) return;
-                    // where a lane's survivors go: behind those of the lanes before it
+                    // where a lane's survivors go, in any order: a list is read chunk by chunk
                     const uint32_t cnt = __popc(mask);
                     survivors += cnt;
-                    uint32_t incl = cnt;
-#pragma unroll
-                    for (int off = 1; off < 32; off <<= 1) {
-                        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, off);
-                        if (lane >= off) incl += v;
-                    }
-                    uint32_t pos = filled + incl - cnt;
-                    filled += __shfl_sync(0xffffffffu, incl, 31);
+                    uint32_t pos = cnt != 0 ? atomicAdd(filled, cnt) : 0u;
                     // They are few and found bit by bit, their values through a column of shared memory of the lane's own,
                     // because registers cannot be indexed (unrolled over the columns, this outgrows the instruction cache).
                     const uint32_t colbits = ((col0 + ch * 32) << 5) | static_cast<uint32_t>(lane);
 #pragma unroll
                     for (int h = 0; h < 4; ++h) {
-                        uint32_t sub = (mask >> (8 * h)) & 0xFFu;
+                        uint32_t sub = bits[h];
                         if (!__any_sync(0xffffffffu, sub != 0)) continue;
 #pragma unroll
                         for (int j = 0; j < 8; ++j) column[j * 32] = __uint_as_float(r[8 * h + j]);
@@ -282,7 +301,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T_THREADS, 1) first_
                     __syncwarp();
                 }
             }
-            if (ok && lane == 0 && listed) my_offs[(p.k + 1023) / 1024] = filled;
+            if (ok && lane == 0 && listed) my_offs[(p.k + 1023) / 1024] = *filled;
         }
     }
     tc_fence_before();
@@ -390,6 +409,7 @@ void launch_first_test(const SplitHalves& x, const SplitHalves& y, size_t n, siz
     p.n = n;
     p.k = k;
     p.k_blocks = (partial_d + TK - 1) / TK;
+    p.partial_d = partial_d;
     p.tile0 = tile0;
     p.n_tiles = n_tiles;
     p.tile_map = rows.tile_map;

@@ -16,7 +16,7 @@
 // Steps 1 and 3 are right-looking over 32-wide panels with one launch per panel: every block of the trailing matrix
 // recomputes the 32 x 32 products it needs of the panel (three small products instead of one, against a launch and a
 // round trip saved), and the block that holds the next diagonal factorises it at once.  Measured (kernels, one B200): d = 768
-// 1.3 ms, of which 0.25 ms are the solve of step 1 (0.88 with one batch of loads in flight instead of four; d = 1536: 2.5 - 3.0 ms
+// 1.2 ms, of which 0.25 ms are the solve of step 1 (0.88 with one batch of loads in flight instead of four; d = 1536: 2.5 - 3.0 ms
 // before) and 0.75 ms (d = 1536: 1.9) the two chains of d / 32 dependent launches.
 //
 // A matrix too close to singular for this (or too wide for step 1's row buffer) is declined: the caller takes the host's.
@@ -31,7 +31,9 @@ namespace skmb {
 namespace {
 
 constexpr int NB = 32;    // panel width of the factorisations
-constexpr int GT = 64;    // tile of the products
+constexpr int GT = 64;    // tile of the products: GT x GN
+constexpr int GN = 32;
+constexpr int kProductThreads = GT / 4 * GN / 4;
 constexpr int GK = 16;
 constexpr int kThreads = 256;
 constexpr size_t kSolveSmem = 200 * 1024;
@@ -46,31 +48,50 @@ __global__ void widen_draws_kernel(const float* __restrict__ draws, size_t d, si
 
 // kGram: out = a^T a, blocks on and above the diagonal; with `minus_identity` I is subtracted and *largest becomes the
 // largest |entry| as an ordered integer (all ones for a NaN).   !kGram: out = a - a up(e).
-// 64 x 64 tiles, 4 x 4 per thread: 16 double FMAs per four 16-byte shared-memory loads, the FMA rate is the bound.
+// Tiles of 64 x 32, 4 x 4 per thread, the next 16 of K in registers meanwhile: twice the blocks of 64 x 64, so that most SMs have two that
+// wait for memory in turn (d = 768: 0.14 -> 0.085 ms a product, d = 1536: 0.6 -> 0.4).
 template <bool kGram>
-__global__ void __launch_bounds__(kThreads) product_kernel(const double* __restrict__ a, const double* __restrict__ e, size_t dp, double* __restrict__ out, bool minus_identity,
-                                                           unsigned long long* __restrict__ largest) {
+__global__ void __launch_bounds__(kProductThreads) product_kernel(const double* __restrict__ a, const double* __restrict__ e, size_t dp, double* __restrict__ out, bool minus_identity,
+                                                                  unsigned long long* __restrict__ largest) {
     __shared__ __align__(16) double sa[GK][GT + 2];
-    __shared__ __align__(16) double sb[GK][GT + 2];
-    const size_t i0 = static_cast<size_t>(blockIdx.y) * GT, j0 = static_cast<size_t>(blockIdx.x) * GT;
-    if (kGram && j0 < i0) return;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    __shared__ __align__(16) double sb[GK][GN + 2];
+    const size_t i0 = static_cast<size_t>(blockIdx.y) * GT, j0 = static_cast<size_t>(blockIdx.x) * GN;
+    if (kGram && j0 + GN <= i0) return;
+    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
     double acc[4][4] = {};
-    const size_t k_end = kGram ? dp : j0 + GT;   // up(e) is zero below the diagonal
+    const size_t k_end = kGram ? dp : j0 + GN;   // up(e) is zero below the diagonal
+    constexpr int NA = GK * GT / kProductThreads, NBV = GK * GN / kProductThreads;
+    double va[NA], vb[NBV];
+    auto fetch = [&](size_t k0) {
+#pragma unroll
+        for (int u = 0; u < NA; ++u) {
+            const int q = threadIdx.x + u * kProductThreads;
+            if (kGram) va[u] = a[(k0 + (q / GT)) * dp + i0 + q % GT];
+            else va[u] = a[(i0 + q / GK) * dp + k0 + q % GK];
+        }
+#pragma unroll
+        for (int u = 0; u < NBV; ++u) {
+            const int q = threadIdx.x + u * kProductThreads;
+            const size_t row = k0 + q / GN, col = j0 + q % GN;
+            if (kGram) vb[u] = a[row * dp + col];
+            else vb[u] = row < col ? e[row * dp + col] : (row == col ? 0.5 * e[row * dp + col] : 0.0);
+        }
+    };
+    fetch(0);
     for (size_t k0 = 0; k0 < k_end; k0 += GK) {
-        for (int q = threadIdx.x; q < GK * GT; q += kThreads) {
-            const int kk = q >> 6, c = q & 63;
-            if (kGram) {
-                sa[kk][c] = a[(k0 + kk) * dp + i0 + c];
-                sb[kk][c] = a[(k0 + kk) * dp + j0 + c];
-            } else {
-                const int r = q >> 4, k2 = q & 15;
-                sa[k2][r] = a[(i0 + r) * dp + k0 + k2];
-                const size_t row = k0 + kk, col = j0 + c;
-                sb[kk][c] = row < col ? e[row * dp + col] : (row == col ? 0.5 * e[row * dp + col] : 0.0);
-            }
+#pragma unroll
+        for (int u = 0; u < NA; ++u) {
+            const int q = threadIdx.x + u * kProductThreads;
+            if (kGram) sa[q / GT][q % GT] = va[u];
+            else sa[q % GK][q / GK] = va[u];
+        }
+#pragma unroll
+        for (int u = 0; u < NBV; ++u) {
+            const int q = threadIdx.x + u * kProductThreads;
+            sb[q / GN][q % GN] = vb[u];
         }
         __syncthreads();
+        if (k0 + GK < k_end) fetch(k0 + GK);
 #pragma unroll
         for (int kk = 0; kk < GK; ++kk) {
             double av[4], bv[4];
@@ -386,12 +407,12 @@ bool make_rotation_matrix_on_device(const float* draws, size_t d, float* out, cu
     float* signs = signs_buf.ensure(dp);
     unsigned long long* worst = worst_buf.ensure(1);
     const dim3 cells(static_cast<unsigned>((dp + 255) / 256), static_cast<unsigned>(dp));
-    const dim3 tiles(static_cast<unsigned>(dp / GT), static_cast<unsigned>(dp / GT));
+    const dim3 tiles(static_cast<unsigned>(dp / GN), static_cast<unsigned>(dp / GT));
 
     widen_draws_kernel<<<cells, 256, 0, stream>>>(draws, d, dp, a);
     SKM_LAUNCH_CHECK();
     SKM_CUDA(cudaMemsetAsync(worst, 0, sizeof(unsigned long long), stream));
-    product_kernel<true><<<tiles, kThreads, 0, stream>>>(a, nullptr, dp, g, false, nullptr);
+    product_kernel<true><<<tiles, kProductThreads, 0, stream>>>(a, nullptr, dp, g, false, nullptr);
     SKM_LAUNCH_CHECK();
     factorise<true>(g, dp, r, inverses, nullptr, d, worst, stream);
     const size_t smem = static_cast<size_t>(rows) * dp * sizeof(double);
@@ -409,9 +430,9 @@ bool make_rotation_matrix_on_device(const float* draws, size_t d, float* out, cu
     double* cur = q;
     double* next = a;
     for (int turn = 0;; ++turn) {
-        product_kernel<true><<<tiles, kThreads, 0, stream>>>(cur, nullptr, dp, g, true, worst);
+        product_kernel<true><<<tiles, kProductThreads, 0, stream>>>(cur, nullptr, dp, g, true, worst);
         SKM_LAUNCH_CHECK();
-        product_kernel<false><<<tiles, kThreads, 0, stream>>>(cur, g, dp, next, false, nullptr);
+        product_kernel<false><<<tiles, kProductThreads, 0, stream>>>(cur, g, dp, next, false, nullptr);
         SKM_LAUNCH_CHECK();
         std::swap(cur, next);
         unsigned long long bits = 0;
