@@ -168,8 +168,6 @@ Engine::Engine(const skm_config& cfg, size_t n_clusters, size_t d, bool hierarch
     WorkStream work(stream_);
     ratios_host_ = make_ratios(d, epsilon0_);
     SKM_CUDA(cudaMemcpyAsync(ratios_dev_.ensure(d + 1), ratios_host_.data(), sizeof(float) * (d + 1), cudaMemcpyHostToDevice, stream_));
-    report_dev_.ensure(1);
-    report_host_.ensure(1);
     if (hierarchical && n_clusters <= 128 && !cfg.suppress_warnings) {
         std::cout << "WARNING: n_clusters <= 128 is not recommended for HierarchicalSuperKMeans. "
                      "Consider using at least 128 clusters."
@@ -510,6 +508,9 @@ void run_listed_dense(const PrunedParams& p, PruneSplitWorkspace& ws, PrunePassB
     uint32_t* npl = b.listed_np.ensure(n_listed);
     uint2* top2l = b.listed_top2.ensure(n_listed);
     float* y_split = b.y_split.ensure(2 * p.k * p.d);
+    // Several blocks per tile shorten the chain but take SMs from the walk beside it: not when the walk over all points (about 0.55 ps
+    // per point and centroid) takes longer than one tile's chain (0.17 ns per centroid and dimension) anyway.
+    uint8_t* scratch = side && p.n > 300 * p.d ? nullptr : b.chain_scratch.ensure(tc::chain_scratch_bytes(n_listed));
     const cudaStream_t s = side ? side : stream;
     if (side) {
         b.side_start.record(stream);
@@ -518,7 +519,7 @@ void run_listed_dense(const PrunedParams& p, PruneSplitWorkspace& ws, PrunePassB
     launch_gather_listed(p.x, ws.best, p.knn, ws.hard_idx, n_listed, p.d, xl, bestl, knnl, s);
     launch_chain_norms(xl, n_listed, p.d, p.partial_d, p.vertical_d, p.horizontal_d, false, normsl, s);
     launch_chain_norms(p.y, p.k, p.d, p.partial_d, p.vertical_d, p.horizontal_d, true, ws.chain_norms_y, s);
-    tc::launch_chain(xl, p.y, n_listed, p.k, p.d, p.partial_d, p.vertical_d, p.horizontal_d, normsl, ws.chain_norms_y, p.ratios, bestl, knnl, distl, npl, top2l, y_split, s);
+    tc::launch_chain(xl, p.y, n_listed, p.k, p.d, p.partial_d, p.vertical_d, p.horizontal_d, normsl, ws.chain_norms_y, p.ratios, bestl, knnl, distl, npl, top2l, y_split, scratch, s);
     launch_scatter_listed(ws.hard_idx, n_listed, knnl, distl, npl, p.knn, p.dist, p.not_pruned, s);
     if (side) b.side_done.record(side);
 }
@@ -995,7 +996,7 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
         launch_chain_norms(p.x, p.n, p.d, p.partial_d, p.vertical_d, p.horizontal_d, false, b.chain_norms_x.ensure(p.n * n_ck), stream);
         launch_chain_norms(p.y, p.k, p.d, p.partial_d, p.vertical_d, p.horizontal_d, true, ws.chain_norms_y, stream);
         tc::launch_chain(p.x, p.y, p.n, p.k, p.d, p.partial_d, p.vertical_d, p.horizontal_d, b.chain_norms_x.get(), ws.chain_norms_y, p.ratios, ws.best, p.knn, p.dist,
-                         p.not_pruned, b.top2.ensure(p.n), b.y_split.ensure(2 * p.k * p.d), stream);
+                         p.not_pruned, b.top2.ensure(p.n), b.y_split.ensure(2 * p.k * p.d), b.chain_scratch.ensure(tc::chain_scratch_bytes(p.n)), stream);
         return;
     }
     p.best_in = ws.best;
@@ -1156,10 +1157,10 @@ PrunedParams Engine::pruned_params(const IterationInput& in) {
 
 // -------------------------------------------------------------------------------------------------
 // SplitClusters (superkmeans.h:886-931, hierarchical_superkmeans.h:579-678) of the scaled centroids.
-// counts_host_ holds this iteration's (globally reduced) cluster sizes.  Returns whether there was anything to split.
+// counts_host() holds this iteration's (globally reduced) cluster sizes.  Returns whether there was anything to split.
 // -------------------------------------------------------------------------------------------------
 bool Engine::split(size_t n_samples_global, size_t k_cur) {
-    sizes_host_.assign(counts_host_.get(), counts_host_.get() + k_cur);
+    sizes_host_.assign(counts_host(), counts_host() + k_cur);
     if (!split_can_terminate(sizes_host_, n_samples_global, k_cur)) {
         throw std::runtime_error("cannot repopulate empty clusters: no cluster holds more than one point");
     }
@@ -1176,10 +1177,9 @@ bool Engine::split(size_t n_samples_global, size_t k_cur) {
 
 // The report and the cluster sizes of what is enqueued, once it is done.
 void Engine::fetch_report(size_t k_cur) {
-    SKM_CUDA(cudaMemcpyAsync(counts_host_.ensure(k_), counts_.get(), sizeof(uint32_t) * k_cur, cudaMemcpyDeviceToHost, stream_));
-    SKM_CUDA(cudaMemcpyAsync(report_host_.get(), report_dev_.get(), sizeof(IterationReport), cudaMemcpyDeviceToHost, stream_));
+    SKM_CUDA(cudaMemcpyAsync(outcome_host_.get(), outcome_.get(), sizeof(uint32_t) * (kReportWords + k_cur), cudaMemcpyDeviceToHost, stream_));
     sync();
-    if (report_host_.get()->error != 0) check_tc_error(stream_);
+    if (report_host()->error != 0) check_tc_error(stream_);
 }
 
 // ConsolidateCentroids without the splits, and ComputeShift.
@@ -1188,7 +1188,7 @@ void Engine::consolidate(const IterationInput& in, bool scale) {
     ConsolidateParams p{};
     p.c = c_cur_.get();
     p.prev = c_prev_.get();
-    p.counts = scale ? counts_.get() : nullptr;
+    p.counts = scale ? counts() : nullptr;
     p.normalize = cfg_.angular;
     p.splits_follow = scale && hierarchical_;
     p.pdx = c_pdx_.get();
@@ -1197,7 +1197,7 @@ void Engine::consolidate(const IterationInput& in, bool scale) {
     p.d = d_;
     p.vertical_d = vertical_d_;
     p.reduce_scratch = ws_.reduce_scratch;
-    p.report = report_dev_.get();
+    p.report = report();
     launch_consolidate(p, stream_);
 }
 
@@ -1232,19 +1232,19 @@ void Engine::run_iteration(bool gemm_only, const IterationInput& in, size_t iter
         stats.dist = distances_.get();
         stats.not_pruned = gemm_only ? nullptr : not_pruned_.get();
         stats.error = tc::error_word();
-        stats.report = report_dev_.get();
-        launch_update(in.x, assignments_.get(), n, k_cur, d_, ws_, c_cur_.get(), counts_.get(), &stats, stream_);
+        stats.report = report();
+        launch_update(in.x, assignments_.get(), n, k_cur, d_, ws_, c_cur_.get(), counts(), &stats, stream_);
     }
-    allreduce_iteration(c_cur_.get(), k_cur * d_, counts_.get(), k_cur, &report_dev_.get()->wcss, 2);
+    allreduce_iteration(c_cur_.get(), k_cur * d_, counts(), k_cur, &report()->wcss, 2);
     consolidate(in, true);
     fetch_report(k_cur);
-    const IterationReport& report = *report_host_.get();
-    const double wcss = report.wcss;
+    const IterationReport& told = *report_host();
+    const double wcss = told.wcss;
 
     float avg_not_pruned = -1.0f;
     const uint32_t old_partial_d = partial_d_;
     if (!gemm_only) {
-        const TuneResult t = tune_partial_d(report.not_pruned, in.n_samples_global, k_cur, partial_d_, vertical_d_, cfg_.min_not_pruned_pct, cfg_.max_not_pruned_pct,
+        const TuneResult t = tune_partial_d(told.not_pruned, in.n_samples_global, k_cur, partial_d_, vertical_d_, cfg_.min_not_pruned_pct, cfg_.max_not_pruned_pct,
                                             cfg_.adjustment_factor_for_partial_d);
         avg_not_pruned = t.avg_not_pruned_pct;
         partial_d_ = t.new_partial_d;
@@ -1253,7 +1253,7 @@ void Engine::run_iteration(bool gemm_only, const IterationInput& in, size_t iter
             launch_row_sqnorms(in.x, n, d_, partial_d_, norms, stream_);
         }
         in.pruned_before = true;
-        in.survival = report.not_pruned / (static_cast<double>(in.n_samples_global) * static_cast<double>(k_cur));
+        in.survival = told.not_pruned / (static_cast<double>(in.n_samples_global) * static_cast<double>(k_cur));
     }
     if (split(in.n_samples_global, k_cur) || (hierarchical_ && cfg_.angular)) {
         consolidate(in, false);
@@ -1263,7 +1263,7 @@ void Engine::run_iteration(bool gemm_only, const IterationInput& in, size_t iter
     prev_cost_ = cost_;
     cost_ = static_cast<float>(wcss);
     last_cost_f64_ = wcss;
-    shift_ = static_cast<float>(report.shift);
+    shift_ = static_cast<float>(told.shift);
 
     if (trace_on_) {
         Snapshot snap;
@@ -1273,7 +1273,7 @@ void Engine::run_iteration(bool gemm_only, const IterationInput& in, size_t iter
         snap.centroids.resize(k_cur * d_);
         snap.assign.resize(n);
         snap.dist.resize(n);
-        snap.sizes_pre.assign(counts_host_.get(), counts_host_.get() + k_cur);
+        snap.sizes_pre.assign(counts_host(), counts_host() + k_cur);
         snap.sizes_post.assign(sizes_host_.begin(), sizes_host_.begin() + k_cur);
         SKM_CUDA(cudaMemcpyAsync(snap.centroids.data(), c_cur_.get(), sizeof(float) * k_cur * d_, cudaMemcpyDeviceToHost, stream_));
         SKM_CUDA(cudaMemcpyAsync(snap.assign.data(), assignments_.get(), sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, stream_));
@@ -1380,8 +1380,7 @@ void Engine::train_flat(const float* data, size_t n, bool on_device, const float
     c_pdx_.ensure(k_ * d_);
     c_aux_.ensure(k_ * static_cast<size_t>(vertical_d_) + 1);
     centroid_norms_.ensure(k_);
-    counts_.ensure(k_);
-    counts_host_.ensure(k_);
+    reserve_outcome(k_);
     assignments_.ensure(n_samples_);
     distances_.ensure(n_samples_);
     not_pruned_.ensure(n_samples_);
@@ -1554,8 +1553,7 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
     c_pdx_.ensure(k_ * d_);
     c_aux_.ensure(k_ * static_cast<size_t>(vertical_d_) + 1);
     centroid_norms_.ensure(k_);
-    counts_.ensure(k_);
-    counts_host_.ensure(k_);
+    reserve_outcome(k_);
     assignments_.ensure(n);
     distances_.ensure(n);
     not_pruned_.ensure(n_all);

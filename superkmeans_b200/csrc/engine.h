@@ -69,6 +69,7 @@ struct PrunePassBuffers {
     DeviceBuffer<uint32_t> tc_list_offs, redo, listed_knn, listed_np;
     DeviceBuffer<float> listed_x, listed_best, listed_dist, listed_norms, y_split;
     DeviceBuffer<PrunePassCounters> counters;
+    DeviceBuffer<uint8_t> chain_scratch;
     PinnedBuffer<PrunePassCounters> counters_host;
     PinnedBuffer<unsigned long long> sorted_counters_host;
     double last_survival = 0;   // share of sampled (point, centroid) pairs that passed the first test in the last automatic choice
@@ -324,7 +325,18 @@ class Engine {
     DeviceBuffer<float> c_cur_, c_prev_; // row-major centroids (horizontal_centroids / prev_centroids)
     DeviceBuffer<float> c_pdx_, c_aux_;  // PDX-blocked copy and first-vertical_d copy
     DeviceBuffer<float> centroid_norms_;
-    DeviceBuffer<uint32_t> counts_;
+    // an iteration's report and, behind it, its cluster sizes: one copy brings both to the host
+    DeviceBuffer<uint32_t> outcome_;
+    PinnedBuffer<uint32_t> outcome_host_;
+    static constexpr size_t kReportWords = (sizeof(IterationReport) + 15) / 16 * 4;
+    uint32_t* counts() const { return outcome_.get() + kReportWords; }
+    uint32_t* counts_host() const { return outcome_host_.get() + kReportWords; }
+    IterationReport* report() const { return reinterpret_cast<IterationReport*>(outcome_.get()); }
+    const IterationReport* report_host() const { return reinterpret_cast<const IterationReport*>(outcome_host_.get()); }
+    void reserve_outcome(size_t k) {
+        outcome_.ensure(kReportWords + k);
+        outcome_host_.ensure(kReportWords + k);
+    }
     DeviceBuffer<uint32_t> assignments_, not_pruned_;
     DeviceBuffer<float> distances_;
     PrunePassBuffers prune_bufs_;
@@ -342,9 +354,6 @@ class Engine {
     PinnedBuffer<uint32_t> recall_found_host_;
     float recall_ = 0.0f;
     DeviceBuffer<SplitOpDev> split_ops_dev_;
-    DeviceBuffer<IterationReport> report_dev_;
-    PinnedBuffer<IterationReport> report_host_;
-    PinnedBuffer<uint32_t> counts_host_;
     std::vector<uint32_t> sizes_host_;   // cluster_sizes after the last split
 
     // update workspace

@@ -164,15 +164,15 @@ void Engine::train_fine_run(size_t first, size_t last, const std::vector<size_t>
         }
         {
             PhaseScope ps(*this, PH_UPDATE);
-            launch_update(x, assignments_.get(), n, k, d_, ws_, c_cur_.get(), counts_.get(), nullptr, stream_);
+            launch_update(x, assignments_.get(), n, k, d_, ws_, c_cur_.get(), counts(), nullptr, stream_);
             group_cost_kernel<<<static_cast<unsigned>(n_groups), 256, 0, stream_>>>(distances_.get(), groups_dev.get(), sums_dev.get());
             SKM_LAUNCH_CHECK();
         }
-        SKM_CUDA(cudaMemcpyAsync(counts_host_.get(), counts_.get(), sizeof(uint32_t) * k, cudaMemcpyDeviceToHost, stream_));
+        SKM_CUDA(cudaMemcpyAsync(counts_host(), counts(), sizeof(uint32_t) * k, cudaMemcpyDeviceToHost, stream_));
         SKM_CUDA(cudaMemcpyAsync(sums.get(), sums_dev.get(), sizeof(double) * n_groups, cudaMemcpyDeviceToHost, stream_));
         {
             PhaseScope ps(*this, PH_CONSOLIDATE);
-            group_means_kernel<<<static_cast<unsigned>(k), 256, 0, stream_>>>(c_cur_.get(), c_prev_.get(), counts_.get(), group_of_dev.get(), groups_dev.get(), d_);
+            group_means_kernel<<<static_cast<unsigned>(k), 256, 0, stream_>>>(c_cur_.get(), c_prev_.get(), counts(), group_of_dev.get(), groups_dev.get(), d_);
             SKM_LAUNCH_CHECK();
         }
         sync();
@@ -184,7 +184,7 @@ void Engine::train_fine_run(size_t first, size_t last, const std::vector<size_t>
             ops_of[q].clear();
             Group& g = groups[q];
             if (!g.active) continue;
-            std::vector<uint32_t> s(counts_host_.get() + g.y0, counts_host_.get() + g.y0 + g.k);
+            std::vector<uint32_t> s(counts_host() + g.y0, counts_host() + g.y0 + g.k);
             if (!split_can_terminate(s, g.rows, g.k)) {
                 failure[q] = "cannot repopulate empty clusters: no cluster holds more than one point";
                 continue;

@@ -206,6 +206,7 @@ struct SplitOp {
 // SuperKMeans::SplitClusters (superkmeans.h:890-928).  `sizes` is updated in place exactly like
 // cluster_sizes.  Returns n_split.
 inline size_t split_clusters_flat(std::vector<uint32_t>& sizes, size_t n_samples, size_t n_clusters, uint32_t seed, std::vector<SplitOp>& ops) {
+    if (std::find(sizes.begin(), sizes.begin() + static_cast<std::ptrdiff_t>(n_clusters), 0u) == sizes.begin() + static_cast<std::ptrdiff_t>(n_clusters)) return 0;
     size_t n_split = 0;
     std::mt19937 rng(seed);
     // The walk below draws ~n_clusters numbers per empty cluster (tens of millions when a thousand clusters are empty), so

@@ -383,6 +383,17 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_tc_kernel(const __grid_co
 // precomputed cumulative norms, and updates a bit mask of surviving centroids.  Every quantity a row
 // needs (survivor masks, survivor count, chunk minimum) is private to its thread.
 // =================================================================================================
+// What the two threads of a row (one per half of the columns) tell each other at the end of a chunk, and a block that looks
+// at one unit of the chunk only tells merge_chain_kernel.
+struct ChainPartial {
+    uint32_t cnt;          // survivors of the first test in this chunk
+    uint32_t prev_first;   // the previous centroid is among them
+    float cb;              // best final distance of the chunk, FLT_MAX if none
+    uint32_t cbi;
+    float t1, t2;          // the two smallest final distances of the row so far (candidates for the refinement)
+    uint32_t i1, i2;
+};
+
 struct ChainParams {
     size_t n, k;
     uint32_t d, partial_d, vertical_d, horizontal_d;
@@ -395,6 +406,8 @@ struct ChainParams {
     float* dist;
     uint32_t* not_pruned;
     uint2* top2;                    // out: the two smallest final distances seen by the chain, per point
+    uint32_t chunk_begin, chunk_end;   // chunks of 1024 centroids
+    ChainPartial* partial;             // with SLICES
     int* error;
     long long wait_limit;
 };
@@ -442,16 +455,6 @@ struct ChainMaps {
 // hi/lo by the splitter warps, Y hi and lo straight from global memory), two accumulators of 256 columns.
 // The two accumulators belong to two neighbouring centroid units that advance through the segments in
 // turn, so the tensor pipe works on one unit while the rows' threads test the other.
-// What the two threads of a row (one per half of the columns) tell each other at the end of a chunk.
-struct ChainPartial {
-    uint32_t cnt;          // survivors of the first test in this chunk
-    uint32_t prev_first;   // the previous centroid is among them
-    float cb;              // best final distance of the chunk, FLT_MAX if none
-    uint32_t cbi;
-    float t1, t2;          // the two smallest final distances of the row so far (candidates for the refinement)
-    uint32_t i1, i2;
-};
-
 struct ChainCtrl {
     uint64_t full[STAGES];
     uint64_t conv[STAGES];
@@ -476,16 +479,19 @@ constexpr int CHAIN_THREADS = 448;
 // Order of work shared by all roles: row tile, chunk of 1024 centroids, pair of 256-centroid units, segment,
 // unit of the pair.  `a` (0 / 1) is the unit's accumulator.
 #define CHAIN_FOR_EACH_UNIT_SEGMENT(...)                                                                  \
-    for (size_t rt = blockIdx.x; rt < n_row_tiles && ok; rt += gridDim.x) {                               \
-        for (uint32_t chunk = 0; chunk < n_chunks && ok; ++chunk) {                                       \
+    for (size_t item = blockIdx.x; item < n_row_tiles * SLICES && ok; item += gridDim.x) {                \
+        const size_t rt = item / SLICES;                                                                \
+        for (uint32_t chunk = p.chunk_begin; chunk < p.chunk_end && ok; ++chunk) {                        \
             const size_t c0 = static_cast<size_t>(chunk) * kChunk;                                        \
             const uint32_t cs = static_cast<uint32_t>(min(static_cast<size_t>(kChunk), p.k - c0));        \
-            const uint32_t n_units = (cs + BN - 1) / BN;                                                  \
-            for (uint32_t pair = 0; pair * 2 < n_units && ok; ++pair) {                                   \
+            const uint32_t unit0 = static_cast<uint32_t>(item % SLICES);                                \
+            const uint32_t all_units = (cs + BN - 1) / BN;                                                \
+            const uint32_t n_units = SLICES > 1 ? min(unit0 + 1, all_units) : all_units;                \
+            for (uint32_t pair = 0; unit0 + pair * 2 < n_units && ok; ++pair) {                           \
                 for (uint32_t seg = 0; seg < p.n_seg && ok; ++seg) {                                      \
                     const SegInfo si = chain_segment(p, seg);                                             \
                     for (uint32_t a = 0; a < 2 && ok; ++a) {                                              \
-                        const uint32_t unit = pair * 2 + a;                                               \
+                        const uint32_t unit = unit0 + pair * 2 + a;                                       \
                         if (unit >= n_units) break;                                                       \
                         __VA_ARGS__                                                                       \
                     }                                                                                     \
@@ -494,6 +500,8 @@ constexpr int CHAIN_THREADS = 448;
         }                                                                                                 \
     }
 
+// SLICES: 1, or 4 for a block per unit of the only chunk, whose findings go to partial[slice][row].
+template <uint32_t SLICES>
 __global__ void __launch_bounds__(CHAIN_THREADS, 1) chain_tc_kernel(const __grid_constant__ ChainMaps maps, const ChainParams p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw_addr = smem_u32(smem_raw);
@@ -528,7 +536,6 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1) chain_tc_kernel(const __grid
     const uint32_t tmem_base = ctrl->tmem_base;
 
     const size_t n_row_tiles = (p.n + BM - 1) / BM;
-    const uint32_t n_chunks = static_cast<uint32_t>((p.k + kChunk - 1) / kChunk);
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
@@ -640,7 +647,7 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1) chain_tc_kernel(const __grid
         uint32_t uses[2] = {0, 0};
         uint32_t xchg_uses = 0;
         bool ok = true;
-        size_t cur_rt = ~size_t{0};
+        size_t cur_item = ~size_t{0};
         uint32_t cur_chunk = 0xFFFFFFFFu;
         size_t row = 0;
         bool row_valid = false;
@@ -689,13 +696,20 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1) chain_tc_kernel(const __grid
             }
             // the two smallest of both halves, for the end of the row (the halves' own pairs cover disjoint columns
             // and stay as they are)
+            float v1, v2;
             if (other.t1 < t1) {
                 o2 = (t1 < other.t2) ? i1 : other.i2;
                 o1 = other.i1;
+                v1 = other.t1;
+                v2 = fminf(t1, other.t2);
             } else {
                 o1 = i1;
                 o2 = (other.t1 < t2) ? other.i1 : i2;
+                v1 = t1;
+                v2 = fminf(other.t1, t2);
             }
+            if (SLICES > 1 && half == 0 && row_valid)
+                p.partial[cur_item % SLICES * p.n + row] = ChainPartial{cnt_all, prev_all ? 1u : 0u, mb, mbi, v1, v2, o1, o2};
             cnt = 0;
             prev_first = false;
             cb = FLT_MAX;
@@ -703,7 +717,7 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1) chain_tc_kernel(const __grid
             return true;
         };
         auto close_row = [&]() {
-            if (row_valid && half == 0) {
+            if (row_valid && half == 0 && SLICES == 1) {
                 p.knn[row] = bestidx;
                 p.dist[row] = best;
                 p.not_pruned[row] = npc;
@@ -711,15 +725,15 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1) chain_tc_kernel(const __grid
             }
         };
         CHAIN_FOR_EACH_UNIT_SEGMENT({
-            if (rt != cur_rt) {
-                if (cur_rt != ~size_t{0}) {
+            if (item != cur_item) {
+                if (cur_item != ~size_t{0}) {
                     if (!close_chunk()) {
                         ok = false;
                         break;
                     }
                     close_row();
                 }
-                cur_rt = rt;
+                cur_item = item;
                 cur_chunk = chunk;
                 row = rt * BM + row_in_tile;
                 row_valid = row < p.n;
@@ -861,7 +875,7 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1) chain_tc_kernel(const __grid
                 else alive0[q] = alive[q];
             }
         })
-        if (ok && cur_rt != ~size_t{0}) {
+        if (ok && cur_item != ~size_t{0}) {
             if (close_chunk()) close_row();
         }
     }
@@ -870,6 +884,70 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1) chain_tc_kernel(const __grid
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
+}
+
+// The end of a chunk (close_chunk above) for rows whose units were looked at by blocks of their own.  `state` carries a row from chunk
+// to chunk, `best` is the threshold that the next chunk's blocks read.
+struct ChainState {
+    uint32_t bestidx, npc;
+    float t1, t2;
+    uint32_t i1, i2;
+};
+
+__global__ void __launch_bounds__(128) merge_chain_kernel(const ChainPartial* __restrict__ partial, uint32_t n_units, size_t n, bool first, bool last, const float* __restrict__ best_in,
+                                                          float* __restrict__ best_state, ChainState* __restrict__ state, uint32_t* __restrict__ knn, float* __restrict__ dist,
+                                                          uint32_t* __restrict__ not_pruned, uint2* __restrict__ top2, const int* __restrict__ error) {
+    const size_t row = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    // (partials of a chain that gave up on a wait are not read)
+    if (row >= n || *reinterpret_cast<const volatile int*>(error) != 0) return;
+    ChainState st{};
+    float best;
+    if (first) {
+        st = {knn[row], 0u, FLT_MAX, FLT_MAX, 0xFFFFFFFFu, 0xFFFFFFFFu};
+        best = best_in[row];
+    } else {
+        st = state[row];
+        best = best_state[row];
+    }
+    uint32_t cnt = 0, prev_first = 0, mbi = 0;
+    float mb = FLT_MAX;
+    for (uint32_t u = 0; u < n_units; ++u) {
+        const ChainPartial q = partial[u * n + row];
+        cnt += q.cnt;
+        prev_first |= q.prev_first;
+        if (q.cb < mb || (q.cb == mb && q.cbi < mbi)) {
+            mb = q.cb;
+            mbi = q.cbi;
+        }
+        if (q.t1 < st.t1) {
+            if (st.t1 < q.t2) {
+                st.t2 = st.t1;
+                st.i2 = st.i1;
+            } else {
+                st.t2 = q.t2;
+                st.i2 = q.i2;
+            }
+            st.t1 = q.t1;
+            st.i1 = q.i1;
+        } else if (q.t1 < st.t2) {
+            st.t2 = q.t1;
+            st.i2 = q.i1;
+        }
+    }
+    st.npc += cnt;
+    if (mb < FLT_MAX && !(cnt == 1u && prev_first)) {
+        best = mb;
+        st.bestidx = mbi;
+    }
+    if (!last) {
+        state[row] = st;
+        best_state[row] = best;
+        return;
+    }
+    knn[row] = st.bestidx;
+    dist[row] = best;
+    not_pruned[row] = st.npc;
+    top2[row] = make_uint2(st.i1, st.i2);
 }
 
 // After the chain: the exact squared distance (direct differences, fp32) of a point to the chain's
@@ -1247,9 +1325,20 @@ void launch_gemm_nt(const float* a, size_t lda, const float* b, size_t ldb, floa
     launch<MODE_STORE>(tx, ty, ty, p, stream);
 }
 
+// Few rows: a block per row tile leaves most SMs idle, and one tile alone takes 0.13 ms at k = 1000, d = 768.  While every tile
+// can have four blocks, each takes one of the (at most four) units of a chunk, a launch per chunk, and merge_chain_kernel
+// does what the tile's rows do at the end of a chunk: 0.05 ms instead of those 0.13.
+constexpr uint32_t kChainSlices = kChunk / BN;
+size_t chain_scratch_bytes(size_t n) {
+    int device = 0;
+    SKM_CUDA(cudaGetDevice(&device));
+    if ((n + BM - 1) / BM * kChainSlices > static_cast<size_t>(sm_count(device))) return 0;
+    return n * (kChainSlices * sizeof(ChainPartial) + sizeof(ChainState) + sizeof(float));
+}
+
 void launch_chain(const float* x, const float* y, size_t n, size_t k, size_t d, uint32_t partial_d, uint32_t vertical_d, uint32_t horizontal_d, const float* chain_norms_x,
                   const float* chain_norms_y, const float* ratios, const float* best_in, uint32_t* knn, float* dist, uint32_t* not_pruned, uint2* top2_scratch,
-                  float* y_split, cudaStream_t stream) {
+                  float* y_split, void* scratch, cudaStream_t stream) {
     if (n == 0 || k == 0) return;
     int device = 0;
     SKM_CUDA(cudaGetDevice(&device));
@@ -1280,12 +1369,30 @@ void launch_chain(const float* x, const float* y, size_t n, size_t k, size_t d, 
     p.top2 = top2_scratch;
     p.error = error_flag(device);
     p.wait_limit = g_wait_limit;
-    SKM_CUDA(cudaFuncSetAttribute(chain_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(C_SMEM_BYTES)));
     const size_t row_tiles = (n + BM - 1) / BM;
-    const int grid = static_cast<int>(std::min<size_t>(row_tiles, static_cast<size_t>(sm_count(device))));
-    chain_tc_kernel<<<grid, CHAIN_THREADS, C_SMEM_BYTES, stream>>>(maps, p);
-    note_kernel_launch();
-    SKM_CUDA(cudaGetLastError());
+    const uint32_t n_chunks = static_cast<uint32_t>((k + kChunk - 1) / kChunk);
+    if (!scratch || chain_scratch_bytes(n) == 0) {
+        p.chunk_end = n_chunks;
+        SKM_CUDA(cudaFuncSetAttribute(chain_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(C_SMEM_BYTES)));
+        chain_tc_kernel<1><<<static_cast<unsigned>(std::min<size_t>(row_tiles, static_cast<size_t>(sm_count(device)))), CHAIN_THREADS, C_SMEM_BYTES, stream>>>(maps, p);
+        SKM_LAUNCH_CHECK();
+    } else {
+        SKM_CUDA(cudaFuncSetAttribute(chain_tc_kernel<kChainSlices>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(C_SMEM_BYTES)));
+        p.partial = static_cast<ChainPartial*>(scratch);
+        ChainState* state = reinterpret_cast<ChainState*>(p.partial + kChainSlices * n);
+        float* best = reinterpret_cast<float*>(state + n);
+        for (uint32_t c = 0; c < n_chunks; ++c) {
+            const size_t cs = std::min<size_t>(kChunk, k - static_cast<size_t>(c) * kChunk);
+            p.chunk_begin = c;
+            p.chunk_end = c + 1;
+            p.best_in = c == 0 ? best_in : best;
+            chain_tc_kernel<kChainSlices><<<static_cast<unsigned>(row_tiles * kChainSlices), CHAIN_THREADS, C_SMEM_BYTES, stream>>>(maps, p);
+            SKM_LAUNCH_CHECK();
+            merge_chain_kernel<<<static_cast<unsigned>((n + 127) / 128), 128, 0, stream>>>(p.partial, static_cast<uint32_t>((cs + BN - 1) / BN), n, c == 0, c + 1 == n_chunks, best_in, best,
+                                                                                          state, knn, dist, not_pruned, top2_scratch, p.error);
+            SKM_LAUNCH_CHECK();
+        }
+    }
     refine_chain_kernel<<<static_cast<unsigned>((n + 7) / 8), 256, 0, stream>>>(x, y, n, k, d, top2_scratch, knn, dist, p.error, nullptr);
     note_kernel_launch();
     SKM_CUDA(cudaGetLastError());

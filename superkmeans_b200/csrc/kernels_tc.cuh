@@ -107,9 +107,10 @@ void launch_refine_chain_tiles(const float* x, const float* y, size_t n, size_t 
 // (launch_chain_norms; point norms row-major, centroid norms checkpoint-major); best_in the exact distance to the previous centroid; knn the previous
 // assignment on entry and the new one on return.  The winner is settled, and its distance recomputed, in
 // fp32 among the chain's winner and its two runner-ups (top2_scratch: n entries).
+size_t chain_scratch_bytes(size_t n);   // of `scratch` below (optional: lets a few rows have several blocks per tile); may be none
 void launch_chain(const float* x, const float* y, size_t n, size_t k, size_t d, uint32_t partial_d, uint32_t vertical_d, uint32_t horizontal_d, const float* chain_norms_x,
                   const float* chain_norms_y, const float* ratios, const float* best_in, uint32_t* knn, float* dist, uint32_t* not_pruned, uint2* top2_scratch,
-                  float* y_split, cudaStream_t stream);   // y_split: 2 * k * d floats of scratch for the tf32 parts of the centroids
+                  float* y_split, void* scratch, cudaStream_t stream);   // y_split: 2 * k * d floats of scratch for the tf32 parts of the centroids
 
 // SM cycles after which a wait inside a tensor-core kernel gives up (about two seconds unless a test shortened it).
 long long wait_limit();

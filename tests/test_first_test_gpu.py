@@ -1,4 +1,4 @@
-"""First ADSampling test on the tensor cores and the walk over its lists, at the edges of their tiles."""
+"""First ADSampling test on the tensor cores, the walk over its lists and the dense chain, at the edges of their tiles."""
 import numpy as np
 import pytest
 
@@ -8,8 +8,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,d,k", [(129, 132, 300), (1, 128, 1), (255, 256, 257), (4097, 200, 1025), (20_000, 1024, 2_100), (12_345, 384, 5_000)])
-@pytest.mark.parametrize("lists", [4, 5, 9], ids=["roomy", "overflowing", "dropping"])
-def test_lists_agree_with_the_simt_search(n, d, k, lists):
+@pytest.mark.parametrize("lists", [3, 4, 5, 9], ids=["none", "roomy", "overflowing", "dropping"])
+def test_tensor_core_routes_agree_with_the_simt_search(n, d, k, lists):
     import superkmeans_b200 as skm
 
     eng = skm.engine
