@@ -115,6 +115,7 @@ struct DirectScratch {
 size_t direct_key_count(size_t n);
 size_t direct_counter_count(size_t n);
 double direct_assign_seconds(size_t n, size_t k, size_t d);   // what it takes, roughly
+bool direct_assign_counts_arrivals(size_t n, size_t d);       // whether a call of these sizes uses *arrived
 void launch_direct_assign(const float* x, const float* y, size_t n, size_t k, size_t d, const DirectScratch& s, uint32_t* knn, float* dist, cudaStream_t stream);
 
 struct PrunedParams {

@@ -270,10 +270,12 @@ size_t direct_counter_count(size_t n) { return (n + kCell - 1) / kCell; }
 
 double direct_assign_seconds(size_t n, size_t k, size_t d) { return 1.2e-5 + static_cast<double>(n) * static_cast<double>(k) * static_cast<double>(d) / 1.3e13; }
 
+bool direct_assign_counts_arrivals(size_t n, size_t d) { return n <= kQueryRows && n * d * sizeof(float) <= kQuerySmem - 4096; }
+
 void launch_direct_assign(const float* x, const float* y, size_t n, size_t k, size_t d, const DirectScratch& s, uint32_t* knn, float* dist, cudaStream_t stream) {
     if (n == 0 || k == 0) return;
     const bool vec = d % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
-    if (n <= kQueryRows && n * d * sizeof(float) <= kQuerySmem - 4096) {
+    if (direct_assign_counts_arrivals(n, d)) {
         if (vec) launch_query<true>(x, y, n, k, d, s, knn, dist, stream);
         else launch_query<false>(x, y, n, k, d, s, knn, dist, stream);
         return;

@@ -480,7 +480,7 @@ constexpr int CHAIN_THREADS = 448;
 // unit of the pair.  `a` (0 / 1) is the unit's accumulator.
 #define CHAIN_FOR_EACH_UNIT_SEGMENT(...)                                                                  \
     for (size_t item = blockIdx.x; item < n_row_tiles * SLICES && ok; item += gridDim.x) {                \
-        const size_t rt = item / SLICES;                                                                \
+        [[maybe_unused]] const size_t rt = item / SLICES;                                                                \
         for (uint32_t chunk = p.chunk_begin; chunk < p.chunk_end && ok; ++chunk) {                        \
             const size_t c0 = static_cast<size_t>(chunk) * kChunk;                                        \
             const uint32_t cs = static_cast<uint32_t>(min(static_cast<size_t>(kChunk), p.k - c0));        \

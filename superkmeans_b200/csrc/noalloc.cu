@@ -10,8 +10,8 @@
 //
 // Consequences of sharing one array:
 //   * sizes are bounded (kMaxRows, kMaxCentroids); larger requests are refused, not truncated;
-//   * the array keeps what the last call left in it: the status word is cleared at the start of every call,
-//     everything else is written before it is read;
+//   * the array keeps what the last call left in it: words that count or report are cleared at the start of a call that uses
+//     them, everything else is written before it is read;
 //   * two calls whose kernels overlap on the same GPU (different streams, different host threads) write the
 //     same scratch and race.  Callers serialise them.
 //
@@ -91,9 +91,11 @@ void find_nearest(int device, const float* x_dev, const float* y_dev, size_t n, 
 
     DeviceScope scope(device);
     Scratch* s = scratch_of_current_device(device);
-    SKM_CUDA(cudaMemsetAsync(&s->status, 0, sizeof(s->status) + sizeof(s->arrived), stream));
     // (the filter needs fp16 copies of both sides, which there is no room for here)
     if (tc::enabled() && direct_assign_seconds(n, k, d) < 3e-4) {
+        // nothing here waits for anything that can run out: no status to clear or to read, and one launch less of each is a
+        // quarter of a call of 5000 x 300 x 128 (56 us with both, 44 without)
+        if (direct_assign_counts_arrivals(n, d)) SKM_CUDA(cudaMemsetAsync(&s->arrived, 0, sizeof(s->arrived), stream));
         DirectScratch scratch;
         scratch.norms_x = s->row_norms;
         scratch.norms_y = s->centroid_norms;
@@ -101,7 +103,11 @@ void find_nearest(int device, const float* x_dev, const float* y_dev, size_t n, 
         scratch.counters = s->counters;
         scratch.arrived = &s->arrived;
         launch_direct_assign(x_dev, y_dev, n, k, d, scratch, out_knn_dev, out_dist_dev, stream);
-    } else {
+        SKM_CUDA(cudaStreamSynchronize(stream));
+        return;
+    }
+    SKM_CUDA(cudaMemsetAsync(&s->status, 0, sizeof(s->status), stream));
+    {
         launch_row_sqnorms(x_dev, n, d, d, s->row_norms, stream);
         launch_row_sqnorms(y_dev, k, d, d, s->centroid_norms, stream);
         if (tc::eligible(x_dev, d, y_dev, d)) {
