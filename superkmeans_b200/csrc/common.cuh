@@ -277,19 +277,21 @@ struct UpdateWorkspace {
     uint32_t* keys_b = nullptr;   // n
     uint32_t* vals_a = nullptr;   // n
     uint32_t* vals_b = nullptr;   // n
-    uint32_t* digit_table = nullptr;  // 256 * n_units
+    uint32_t* digit_table = nullptr;  // update_table_words(n, k)
     uint32_t* seg_offsets = nullptr;  // k + 1
     float* tile_partials = nullptr;   // n_tiles * 2 * d
     double* reduce_scratch = nullptr; // kReduceScratchDoubles
     size_t n_cap = 0, k_cap = 0, d = 0;
 };
-// sizes of digit_table (256 per unit) and tile_partials (2 d per tile) for up to n points
-size_t update_sort_units(size_t n);
+// sizes of digit_table and tile_partials (2 d per tile) for up to n points and k clusters
+size_t update_table_words(size_t n, size_t k);
 size_t update_tiles(size_t n);
 
 // Stable sort of the indices 0 .. n-1 by keys[i] (< k): *sorted_keys_out / *order_out point into the workspace's key and
-// value buffers (keys_a/b, vals_a/b, digit_table must be allocated for n).
-void launch_sort_by_key(const uint32_t* keys, size_t n, size_t k, UpdateWorkspace& ws, const uint32_t** sorted_keys_out, const uint32_t** order_out, cudaStream_t stream);
+// value buffers (keys_a/b, vals_a/b, digit_table must be allocated for n).  seg_offsets (k + 1, may be null): where every key
+// begins, if the function returns true.
+bool launch_sort_by_key(const uint32_t* keys, size_t n, size_t k, UpdateWorkspace& ws, const uint32_t** sorted_keys_out, const uint32_t** order_out, uint32_t* seg_offsets,
+                        cudaStream_t stream);
 
 // What an iteration tells the host, in one copy.
 struct IterationReport {

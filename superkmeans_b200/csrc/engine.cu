@@ -401,13 +401,12 @@ void Engine::exact_assignment(const float* x, size_t n, const float* c, size_t k
 }
 
 void Engine::prepare_update_workspace(size_t n, size_t k) {
-    const size_t units = update_sort_units(n);
     const size_t tiles = update_tiles(n);
     ws_.keys_a = ws_keys_a_.ensure(n);
     ws_.keys_b = ws_keys_b_.ensure(n);
     ws_.vals_a = ws_vals_a_.ensure(n);
     ws_.vals_b = ws_vals_b_.ensure(n);
-    ws_.digit_table = ws_table_.ensure(256 * units + (256 * units) / 2048 + 64);
+    ws_.digit_table = ws_table_.ensure(update_table_words(n, k));
     ws_.seg_offsets = ws_offsets_.ensure(k + 1);
     ws_.tile_partials = ws_partials_.ensure(tiles * 2 * d_);
     ws_.reduce_scratch = ws_reduce_.ensure(kReduceScratchDoubles);
@@ -558,15 +557,14 @@ void run_pruned_pass_sorted(const PrunedParams& p, PrunePassBuffers& b, float ra
     const size_t cols_stride = n_chunks * kChunk;
 
     // ---- order of the points by previous centroid
-    const size_t units = update_sort_units(p.n);
     b.sort_ws.keys_a = b.sort_keys_a.ensure(p.n);
     b.sort_ws.keys_b = b.sort_keys_b.ensure(p.n);
     b.sort_ws.vals_a = b.sort_vals_a.ensure(p.n);
     b.sort_ws.vals_b = b.sort_vals_b.ensure(p.n);
-    b.sort_ws.digit_table = b.sort_table.ensure(256 * units + (256 * units) / 2048 + 64);
+    b.sort_ws.digit_table = b.sort_table.ensure(update_table_words(p.n, p.k));
     const uint32_t* sorted_keys = nullptr;
     const uint32_t* order = nullptr;
-    launch_sort_by_key(p.knn, p.n, p.k, b.sort_ws, &sorted_keys, &order, stream);
+    launch_sort_by_key(p.knn, p.n, p.k, b.sort_ws, &sorted_keys, &order, nullptr, stream);
 
     // ---- centroid side, once per pass
     float* y_split = b.y_split.ensure(2 * p.k * p.d);
@@ -1604,7 +1602,7 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
         // sort of the point indices by mesocluster - on the device, with the update's radix sort.
         const uint32_t* sorted_keys = nullptr;
         const uint32_t* order = nullptr;
-        launch_sort_by_key(assignments_.get(), n_all, n_meso_, ws_, &sorted_keys, &order, stream_);
+        launch_sort_by_key(assignments_.get(), n_all, n_meso_, ws_, &sorted_keys, &order, nullptr, stream_);
         widen_u32_kernel<<<static_cast<unsigned>((n_all + 255) / 256), 256, 0, stream_>>>(order, meso_indices_dev_.get(), n_all);
         note_kernel_launch();
         SKM_CUDA(cudaGetLastError());
@@ -2088,12 +2086,12 @@ void Engine::op_update(int device, const float* x, const uint32_t* assign, const
         ctx.upload(dd, zeros.data(), n);
     }
     UpdateWorkspace ws;
-    const size_t units = update_sort_units(n), tiles = update_tiles(n);
+    const size_t tiles = update_tiles(n);
     ws.keys_a = ka.ensure(n);
     ws.keys_b = kb.ensure(n);
     ws.vals_a = va.ensure(n);
     ws.vals_b = vb.ensure(n);
-    ws.digit_table = table.ensure(256 * units + (256 * units) / 2048 + 64);
+    ws.digit_table = table.ensure(update_table_words(n, k));
     ws.seg_offsets = offs.ensure(k + 1);
     ws.tile_partials = partials.ensure(std::max<size_t>(tiles, 1) * 2 * d);
     ws.reduce_scratch = reduce_scratch.ensure(kReduceScratchDoubles);

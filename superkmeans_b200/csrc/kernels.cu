@@ -516,15 +516,25 @@ static size_t sort_units_of(size_t n) { return (n + sort_unit(n) - 1) / sort_uni
 static size_t tiles_of(size_t n) { return (n + update_tile_rows(n) - 1) / update_tile_rows(n); }
 
 // A workspace made for n points also serves fewer, and fewer points can need more units and tiles.
-size_t update_sort_units(size_t n) {
+static size_t update_sort_units(size_t n) {
     return std::max({sort_units_of(n), sort_units_of(std::min(n, (size_t{1} << 17) - 1)), sort_units_of(std::min(n, (size_t{1} << 20) - 1))});
+}
+// Up to 1024 clusters are sorted in one pass of ten bits: each of the five launches of a second pass takes 2 - 6 us however few the
+// points are (30 000 points, 1000 clusters: 31 -> 19 us), and at 1M points the larger table is less than a pass over them.
+// From there on eight bits at a time: the tables of a warp no longer fit a block of eight.
+static int sort_bits(size_t k) { return k > 256 && k <= 1024 ? 10 : 8; }
+size_t update_table_words(size_t n, size_t k) {
+    const size_t words = (size_t{1} << (k > 256 ? 10 : 8)) * update_sort_units(n);
+    return words + words / 2048 + 64;
 }
 size_t update_tiles(size_t n) { return std::max(tiles_of(n), tiles_of(std::min(n, (size_t{148} << 10) - 1))); }
 
+template <int BITS>
 __global__ void __launch_bounds__(256) sort_hist_kernel(const uint32_t* __restrict__ keys, size_t n, int shift, uint32_t* __restrict__ table, size_t n_units, int unit_size) {
-    __shared__ uint32_t h[8][256];
+    constexpr int DIGITS = 1 << BITS;
+    __shared__ uint32_t h[8][DIGITS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = lane; i < 256; i += 32) h[warp][i] = 0;
+    for (int i = lane; i < DIGITS; i += 32) h[warp][i] = 0;
     __syncwarp();
     const size_t unit = static_cast<size_t>(blockIdx.x) * 8 + warp;
     if (unit < n_units) {
@@ -538,10 +548,10 @@ __global__ void __launch_bounds__(256) sort_hist_kernel(const uint32_t* __restri
             }
 #pragma unroll
             for (int u = 0; u < kSortAhead; ++u)
-                if (base + static_cast<size_t>(s0 + u) * 32 + lane < n) atomicAdd(&h[warp][(key[u] >> shift) & 255u], 1u);
+                if (base + static_cast<size_t>(s0 + u) * 32 + lane < n) atomicAdd(&h[warp][(key[u] >> shift) & (DIGITS - 1u)], 1u);
         }
         __syncwarp();
-        for (int i = lane; i < 256; i += 32) table[static_cast<size_t>(i) * n_units + unit] = h[warp][i];
+        for (int i = lane; i < DIGITS; i += 32) table[static_cast<size_t>(i) * n_units + unit] = h[warp][i];
     }
 }
 
@@ -638,15 +648,20 @@ void exclusive_scan_u32(uint32_t* data, size_t n, uint32_t* totals_tmp, cudaStre
 }
 
 // Stable scatter: each warp re-reads its unit in order; lanes with equal digits are ranked by lane.
+template <int BITS>
 __global__ void __launch_bounds__(256) sort_scatter_kernel(
     const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, size_t n, int shift,
-    const uint32_t* __restrict__ table, size_t n_units, int unit_size
+    const uint32_t* __restrict__ table, size_t n_units, int unit_size, uint32_t* __restrict__ seg_offsets, size_t k
 ) {
-    __shared__ uint32_t base_s[8][256];
+    constexpr int DIGITS = 1 << BITS;
+    __shared__ uint32_t base_s[8][DIGITS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const size_t unit = static_cast<size_t>(blockIdx.x) * 8 + warp;
+    // the only pass knows where every key begins
+    if (seg_offsets && blockIdx.x == 0)
+        for (size_t c = threadIdx.x; c <= k; c += 256) seg_offsets[c] = c < DIGITS ? table[c * n_units] : static_cast<uint32_t>(n);
     if (unit >= n_units) return;
-    for (int i = lane; i < 256; i += 32) base_s[warp][i] = table[static_cast<size_t>(i) * n_units + unit];
+    for (int i = lane; i < DIGITS; i += 32) base_s[warp][i] = table[static_cast<size_t>(i) * n_units + unit];
     __syncwarp();
     const size_t base = unit * unit_size;
     const uint32_t lt_mask = (1u << lane) - 1u;
@@ -662,7 +677,7 @@ __global__ void __launch_bounds__(256) sort_scatter_kernel(
 #pragma unroll
         for (int u = 0; u < kSortAhead; ++u) {
             const bool valid = base + static_cast<size_t>(s0 + u) * 32 + lane < n;
-            const uint32_t digit = valid ? ((keys[u] >> shift) & 255u) : 0xFFFFFFFFu;
+            const uint32_t digit = valid ? ((keys[u] >> shift) & (DIGITS - 1u)) : 0xFFFFFFFFu;
             const uint32_t peers = __match_any_sync(0xffffffffu, digit);
             const uint32_t rank = __popc(peers & lt_mask);
             if (valid) {
@@ -880,25 +895,31 @@ __global__ void __launch_bounds__(256) reduce_stats_kernel(UpdateStats u, size_t
 }
 
 // Stable LSD radix sort of the indices 0 .. n-1 by key (keys < k): *sorted_keys and *order point into ws.keys_* / ws.vals_*.
-void launch_sort_by_key(const uint32_t* keys, size_t n, size_t k, UpdateWorkspace& ws, const uint32_t** sorted_keys_out, const uint32_t** order_out, cudaStream_t stream) {
-    const size_t n_units = sort_units_of(n);
+template <int BITS>
+static void launch_sort_pass(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout, size_t n, int shift, const UpdateWorkspace& ws, uint32_t* seg_offsets, size_t k,
+                             cudaStream_t stream) {
+    const size_t n_units = sort_units_of(n), words = n_units << BITS;
+    const unsigned blocks = static_cast<unsigned>((n_units + 7) / 8);
+    sort_hist_kernel<BITS><<<blocks, 256, 0, stream>>>(kin, n, shift, ws.digit_table, n_units, sort_unit(n));
+    SKM_LAUNCH_CHECK();
+    exclusive_scan_u32(ws.digit_table, words, ws.digit_table + words, stream);   // (block totals behind the table)
+    sort_scatter_kernel<BITS><<<blocks, 256, 0, stream>>>(kin, vin, kout, vout, n, shift, ws.digit_table, n_units, sort_unit(n), seg_offsets, k);
+    SKM_LAUNCH_CHECK();
+}
+
+bool launch_sort_by_key(const uint32_t* keys, size_t n, size_t k, UpdateWorkspace& ws, const uint32_t** sorted_keys_out, const uint32_t** order_out, uint32_t* seg_offsets,
+                        cudaStream_t stream) {
     int bits = 1;
     while ((size_t{1} << bits) < k) ++bits;
-    const int passes = (bits + 7) / 8;
+    const int per_pass = sort_bits(k), passes = (bits + per_pass - 1) / per_pass;
+    if (passes > 1) seg_offsets = nullptr;
     const uint32_t* kin = keys;
     const uint32_t* vin = nullptr;
     uint32_t* kout = ws.keys_a;
     uint32_t* vout = ws.vals_a;
-    const unsigned unit_blocks = static_cast<unsigned>((n_units + 7) / 8);
-    // The scan's block totals live in a dedicated region at the end of digit_table (allocated by the caller).
-    uint32_t* scan_totals = ws.digit_table + 256 * n_units;
     for (int pass = 0; pass < passes; ++pass) {
-        const int shift = pass * 8;
-        sort_hist_kernel<<<unit_blocks, 256, 0, stream>>>(kin, n, shift, ws.digit_table, n_units, sort_unit(n));
-        SKM_LAUNCH_CHECK();
-        exclusive_scan_u32(ws.digit_table, 256 * n_units, scan_totals, stream);
-        sort_scatter_kernel<<<unit_blocks, 256, 0, stream>>>(kin, vin, kout, vout, n, shift, ws.digit_table, n_units, sort_unit(n));
-        SKM_LAUNCH_CHECK();
+        if (per_pass == 10) launch_sort_pass<10>(kin, vin, kout, vout, n, pass * 10, ws, seg_offsets, k, stream);
+        else launch_sort_pass<8>(kin, vin, kout, vout, n, pass * 8, ws, seg_offsets, k, stream);
         kin = kout;
         vin = vout;
         kout = (kout == ws.keys_a) ? ws.keys_b : ws.keys_a;
@@ -906,6 +927,7 @@ void launch_sort_by_key(const uint32_t* keys, size_t n, size_t k, UpdateWorkspac
     }
     *sorted_keys_out = kin;
     *order_out = vin;
+    return seg_offsets != nullptr;
 }
 
 template <bool VEC, int TILE>
@@ -925,9 +947,10 @@ void launch_update(const float* x, const uint32_t* assign, size_t n, size_t k, s
     if (n == 0) return;
     const uint32_t* sorted_keys = nullptr;
     const uint32_t* order = nullptr;
-    launch_sort_by_key(assign, n, k, ws, &sorted_keys, &order, stream);
-    segment_offsets_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(sorted_keys, n, k, ws.seg_offsets);
-    SKM_LAUNCH_CHECK();
+    if (!launch_sort_by_key(assign, n, k, ws, &sorted_keys, &order, ws.seg_offsets, stream)) {
+        segment_offsets_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(sorted_keys, n, k, ws.seg_offsets);
+        SKM_LAUNCH_CHECK();
+    }
     const bool vec = (d % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
     const bool big = update_tile_rows(n) == kUpdateTile;
     if (vec && big) launch_segsum<true, kUpdateTile>(x, sorted_keys, order, n, k, d, ws, sums, counts, stream);

@@ -6,7 +6,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,k,d", [(1, 1, 1), (127, 5, 3), (128, 5, 4), (129, 40, 64), (2047, 256, 130), (6000, 91, 768), (131071, 300, 20), (131072, 300, 20),
-                                   (151551, 77, 12), (151552, 77, 12), (1048575, 5, 4), (1048576, 5, 4)])
+                                   (151551, 77, 12), (151552, 77, 12), (1048575, 5, 4), (1048576, 5, 4), (5000, 257, 8), (5000, 1024, 8), (5000, 1025, 8), (300_000, 1000, 8)])
 def test_update_centroids_at_the_edges(n, k, d):
     import superkmeans_b200 as skm
 
