@@ -46,6 +46,9 @@ void pinned_free(const MemoryBlock& m);
 // A non-blocking stream of the current device; release_stream waits for the work on it.
 cudaStream_t acquire_stream();
 void release_stream(cudaStream_t s, int device);
+// Events that measure time, from a bounded pool of the current device.
+cudaEvent_t acquire_timing_event();
+void release_timing_event(cudaEvent_t e, int device);
 // While one is alive, what its thread allocates and releases is used by work on `stream`.
 class WorkStream {
   public:

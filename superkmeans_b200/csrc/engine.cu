@@ -79,30 +79,17 @@ int resolve_device(int device) {
 // Phase timers
 // -------------------------------------------------------------------------------------------------
 PhaseTimers::~PhaseTimers() {
-    for (auto& p : pending_) {
-        cudaEventDestroy(p.a);
-        cudaEventDestroy(p.b);
+    for (auto* list : {&pending_, &open_}) {
+        for (auto& p : *list) {
+            release_timing_event(p.a, device_);
+            release_timing_event(p.b, device_);
+        }
     }
-    for (auto& p : open_) {
-        cudaEventDestroy(p.a);
-        cudaEventDestroy(p.b);
-    }
-    for (auto e : pool_) cudaEventDestroy(e);
-}
-
-cudaEvent_t PhaseTimers::get() {
-    if (!pool_.empty()) {
-        cudaEvent_t e = pool_.back();
-        pool_.pop_back();
-        return e;
-    }
-    cudaEvent_t e;
-    SKM_CUDA(cudaEventCreate(&e));
-    return e;
 }
 
 void PhaseTimers::begin(int phase, cudaStream_t s) {
-    Pending p{phase, get(), get()};
+    if (device_ < 0) SKM_CUDA(cudaGetDevice(&device_));   // (the owner's, always the same)
+    Pending p{phase, acquire_timing_event(), acquire_timing_event()};
     SKM_CUDA(cudaEventRecord(p.a, s));
     open_.push_back(p);
 }
@@ -122,8 +109,8 @@ void PhaseTimers::flush() {
             ms[p.phase] += t;
             calls[p.phase] += 1;
         }
-        pool_.push_back(p.a);
-        pool_.push_back(p.b);
+        release_timing_event(p.a, device_);
+        release_timing_event(p.b, device_);
     }
     pending_.clear();
 }
@@ -494,9 +481,17 @@ int prune_split_mode() { return g_prune_split_mode; }
 
 namespace {
 
-// The points listed in ws.hard_idx through the dense chain on the tensor cores, over a gathered copy of their rows.  With a `side`
-// stream on that one, from where `stream` stands; the caller joins them (b.side_done).
-void run_listed_dense(const PrunedParams& p, PruneSplitWorkspace& ws, PrunePassBuffers& b, size_t n_listed, cudaStream_t stream, cudaStream_t side = nullptr) {
+// The centroids' side of run_listed_dense.
+void prepare_listed_dense(const PrunedParams& p, PruneSplitWorkspace& ws, PrunePassBuffers& b, cudaStream_t stream) {
+    launch_chain_norms(p.y, p.k, p.d, p.partial_d, p.vertical_d, p.horizontal_d, true, ws.chain_norms_y, stream);
+    tc::launch_presplit(p.y, p.k, p.d, b.y_split.ensure(2 * p.k * p.d), stream);
+}
+
+// The points listed in ws.hard_idx through the dense chain on the tensor cores, over a gathered copy of their rows
+// (prepare_listed_dense has run).  With a `side` stream on that one, from where `stream` stands; the caller joins them
+// (b.side_done).  `beside` is called when the chain is on its way.
+void run_listed_dense(const PrunedParams& p, PruneSplitWorkspace& ws, PrunePassBuffers& b, size_t n_listed, cudaStream_t stream, cudaStream_t side = nullptr,
+                      const std::function<void()>& beside = nullptr) {
     if (n_listed == 0) return;
     const uint32_t n_ck = prune_chain_checkpoints(p.partial_d, p.vertical_d, p.horizontal_d);
     float* xl = b.listed_x.ensure(n_listed * p.d);
@@ -506,7 +501,6 @@ void run_listed_dense(const PrunedParams& p, PruneSplitWorkspace& ws, PrunePassB
     float* distl = b.listed_dist.ensure(n_listed);
     uint32_t* npl = b.listed_np.ensure(n_listed);
     uint2* top2l = b.listed_top2.ensure(n_listed);
-    float* y_split = b.y_split.ensure(2 * p.k * p.d);
     // Several blocks per tile shorten the chain but take SMs from the walk beside it: not when the walk over all points (about 0.55 ps
     // per point and centroid) takes longer than one tile's chain (0.17 ns per centroid and dimension) anyway.
     uint8_t* scratch = side && p.n > 300 * p.d ? nullptr : b.chain_scratch.ensure(tc::chain_scratch_bytes(n_listed));
@@ -517,8 +511,8 @@ void run_listed_dense(const PrunedParams& p, PruneSplitWorkspace& ws, PrunePassB
     }
     launch_gather_listed(p.x, ws.best, p.knn, ws.hard_idx, n_listed, p.d, xl, bestl, knnl, s);
     launch_chain_norms(xl, n_listed, p.d, p.partial_d, p.vertical_d, p.horizontal_d, false, normsl, s);
-    launch_chain_norms(p.y, p.k, p.d, p.partial_d, p.vertical_d, p.horizontal_d, true, ws.chain_norms_y, s);
-    tc::launch_chain(xl, p.y, n_listed, p.k, p.d, p.partial_d, p.vertical_d, p.horizontal_d, normsl, ws.chain_norms_y, p.ratios, bestl, knnl, distl, npl, top2l, y_split, scratch, s);
+    tc::launch_chain(xl, p.y, n_listed, p.k, p.d, p.partial_d, p.vertical_d, p.horizontal_d, normsl, ws.chain_norms_y, p.ratios, bestl, knnl, distl, npl, top2l, b.y_split.get(), scratch,
+                     s, beside);
     launch_scatter_listed(ws.hard_idx, n_listed, knnl, distl, npl, p.knn, p.dist, p.not_pruned, s);
     if (side) b.side_done.record(side);
 }
@@ -992,9 +986,9 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
         b.total_dense_rows += p.n;
         Sub sub(timers, PH_PRUNE_DENSE, stream);
         launch_chain_norms(p.x, p.n, p.d, p.partial_d, p.vertical_d, p.horizontal_d, false, b.chain_norms_x.ensure(p.n * n_ck), stream);
-        launch_chain_norms(p.y, p.k, p.d, p.partial_d, p.vertical_d, p.horizontal_d, true, ws.chain_norms_y, stream);
+        prepare_listed_dense(p, ws, b, stream);
         tc::launch_chain(p.x, p.y, p.n, p.k, p.d, p.partial_d, p.vertical_d, p.horizontal_d, b.chain_norms_x.get(), ws.chain_norms_y, p.ratios, ws.best, p.knn, p.dist,
-                         p.not_pruned, b.top2.ensure(p.n), b.y_split.ensure(2 * p.k * p.d), b.chain_scratch.ensure(tc::chain_scratch_bytes(p.n)), stream);
+                         p.not_pruned, b.top2.ensure(p.n), b.y_split.get(), b.chain_scratch.ensure(tc::chain_scratch_bytes(p.n)), stream);
         return;
     }
     p.best_in = ws.best;
@@ -1037,24 +1031,20 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
             if (!(p.same_points && b.x_halves_valid)) tc::launch_split_points(p.x, p.n, p.d, p.vertical_d, xs, stream);
             b.x_halves_valid = true;
             tc::launch_split_centroids(p.y, p.k, p.d, p.partial_d, p.norms_y, ys, stream);
+            cudaStream_t side = nullptr;
+            if (mode == 0) {
+                side = b.side.get();
+                b.y_split.ensure(2 * p.k * p.d);
+                b.side_start.record(stream);
+                b.side_start.hold(side);
+                prepare_listed_dense(p, ws, b, side);
+                b.side_done.record(side);
+            }
             for (size_t t0 = 0; t0 < n_tiles; t0 += per_batch) {
                 const size_t nt = std::min(per_batch, n_tiles - t0);
                 {
                     Sub sub(timers, PH_PRUNE_FIRST_TEST, stream);
                     tc::launch_first_test(xs, ys, p.n, p.k, p.partial_d, p.norms_x, p.norms_y, ws.best, ratio_first, t0, nt, lists, offs, cap_group, rows, stream);
-                }
-                if (mode == 0 && t0 + nt == n_tiles) {
-                    // The dropped points go through the chain beside the walk over the last lists: the two work on different
-                    // points, and one waits for the tensor cores or, with few points, for itself, the other for L2.
-                    const PrunePassCounters* host = b.counters_host.ensure(1);
-                    SKM_CUDA(cudaMemcpyAsync(b.counters_host.get(), counters, sizeof(PrunePassCounters), cudaMemcpyDeviceToHost, stream));
-                    SKM_CUDA(cudaStreamSynchronize(stream));
-                    n_hard = host->n_dropped;
-                    if (n_hard != 0) {
-                        const cudaStream_t side = b.side.get();
-                        Sub sub(timers, PH_PRUNE_DENSE, side);
-                        run_listed_dense(p, ws, b, n_hard, stream, side);
-                    }
                 }
                 WalkParams w{};
                 w.x = p.x;
@@ -1083,13 +1073,30 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
                 w.redo_count = &counters->n_redo;
                 w.pair_steps = pair_steps;
                 w.upstream_error = tc::error_word();
-                Sub sub(timers, PH_PRUNE_WALK, stream);
-                launch_walk_lists(w, device, stream);
+                const auto walk = [&] {
+                    Sub sub(timers, PH_PRUNE_WALK, stream);
+                    launch_walk_lists(w, device, stream);
+                };
+                if (mode == 0 && t0 + nt == n_tiles) {
+                    // The dropped points go through the chain beside the walk over the last lists: the two work on different
+                    // points, and one waits for the tensor cores or, with few points, for itself, the other for L2.  (The chain
+                    // first: its blocks need most of an SM's shared memory.)
+                    const PrunePassCounters* host = b.counters_host.ensure(1);
+                    SKM_CUDA(cudaMemcpyAsync(b.counters_host.get(), counters, sizeof(PrunePassCounters), cudaMemcpyDeviceToHost, stream));
+                    SKM_CUDA(cudaStreamSynchronize(stream));
+                    n_hard = host->n_dropped;
+                    if (n_hard != 0) {
+                        Sub sub(timers, PH_PRUNE_DENSE, side);
+                        run_listed_dense(p, ws, b, n_hard, stream, side, walk);
+                        continue;
+                    }
+                }
+                walk();
             }
         }
         b.last_n_redo = 0;
         if (mode == 0) {
-            if (n_hard != 0) b.side_done.hold(stream);
+            b.side_done.hold(stream);
         } else {
             // points whose list overflowed
             const PrunePassCounters* host = b.counters_host.ensure(1);
@@ -1101,6 +1108,7 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
             if (n_hard != 0) {
                 Sub sub(timers, PH_PRUNE_DENSE, stream);
                 launch_compact_flags(redo, p.n, ws, stream);
+                prepare_listed_dense(p, ws, b, stream);
                 run_listed_dense(p, ws, b, n_hard, stream);
             }
         }
@@ -1521,7 +1529,6 @@ void Engine::output_centroids(float* out_host) {
         c = tmp.get();
     }
     stage_.download(out_host, c, sizeof(float) * k_ * d_, stream_);
-    timers_.flush();
 }
 
 // -------------------------------------------------------------------------------------------------
@@ -1813,7 +1820,6 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
     timers_.end(stream_);
     // the answers are a d-th of the rows: fetched once, so that no copy back holds up the next upload
     stage_.download(out, knn.get(), sizeof(uint32_t) * n, stream_);
-    timers_.flush();
     for (int i = 0; i < 2; ++i) {
         cudaEventDestroy(copied[i]);
         cudaEventDestroy(consumed[i]);

@@ -33,12 +33,15 @@ namespace skmb {
 enum Phase { PH_ROTATE = 0, PH_NORMS, PH_ASSIGN_FULL, PH_ASSIGN_PRUNED, PH_UPDATE, PH_CONSOLIDATE, PH_SHIFT, PH_TRAIN_TOTAL, PH_PRUNE_FIRST_TEST, PH_PRUNE_WALK, PH_PRUNE_DENSE,
              PH_ALLOC_FREE, PH_INIT_CENTROIDS, PH_ALLREDUCE, PH_HOST_OTHER, PH_COUNT };
 
+// Device time per phase, from events.  Reading them is left to whoever asks for the times: 3 us each, seven of them between two
+// iterations, were a fifth of the time that the GPU stood still there.
 class PhaseTimers {
   public:
     ~PhaseTimers();
     void begin(int phase, cudaStream_t s);
     void end(cudaStream_t s);
     void flush();  // call only after the stream has been synchronised
+    size_t pending() const { return pending_.size(); }
     void reset();
     void add_host(int phase, double milliseconds) {
         ms[phase] += milliseconds;
@@ -52,10 +55,9 @@ class PhaseTimers {
         int phase;
         cudaEvent_t a, b;
     };
-    cudaEvent_t get();
+    int device_ = -1;
     std::vector<Pending> pending_;
     std::vector<Pending> open_;
-    std::vector<cudaEvent_t> pool_;
 };
 
 // Device buffers of one pruned assignment pass (candidate lists, work split) and the pass itself:
@@ -213,8 +215,15 @@ class Engine {
     };
     void set_trace(bool on) { trace_on_ = on; }
     const std::vector<Snapshot>& trace() const { return trace_; }
-    const PhaseTimers& timers() const { return timers_; }
-    void reset_timers() { timers_.reset(); }
+    // (every entry point returns with its work done)
+    const PhaseTimers& timers() {
+        timers_.flush();
+        return timers_;
+    }
+    void reset_timers() {
+        timers_.flush();
+        timers_.reset();
+    }
 
     // Stateless operators (used by the skm_op_* entry points).
     static void op_rotate(int device, const float* m, const float* x, size_t n, size_t d, float* out, bool inverse);
@@ -269,7 +278,7 @@ class Engine {
     void allreduce_iteration(float* sums, size_t n_sums, uint32_t* counts, size_t n_counts, double* scalars, size_t n_scalars);
     void sync() {
         SKM_CUDA(cudaStreamSynchronize(stream_));
-        timers_.flush();
+        if (timers_.pending() > 4096) timers_.flush();
     }
     struct PhaseScope {
         Engine& e;

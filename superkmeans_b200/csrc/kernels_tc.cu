@@ -1338,11 +1338,10 @@ size_t chain_scratch_bytes(size_t n) {
 
 void launch_chain(const float* x, const float* y, size_t n, size_t k, size_t d, uint32_t partial_d, uint32_t vertical_d, uint32_t horizontal_d, const float* chain_norms_x,
                   const float* chain_norms_y, const float* ratios, const float* best_in, uint32_t* knn, float* dist, uint32_t* not_pruned, uint2* top2_scratch,
-                  float* y_split, void* scratch, cudaStream_t stream) {
+                  const float* y_split, void* scratch, cudaStream_t stream, const std::function<void()>& beside) {
     if (n == 0 || k == 0) return;
     int device = 0;
     SKM_CUDA(cudaGetDevice(&device));
-    presplit(y, k, d, y_split, stream);
     ChainMaps maps;
     const size_t extents[3] = {partial_d, vertical_d, d};
     for (int i = 0; i < 3; ++i) {
@@ -1376,6 +1375,7 @@ void launch_chain(const float* x, const float* y, size_t n, size_t k, size_t d, 
         SKM_CUDA(cudaFuncSetAttribute(chain_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(C_SMEM_BYTES)));
         chain_tc_kernel<1><<<static_cast<unsigned>(std::min<size_t>(row_tiles, static_cast<size_t>(sm_count(device)))), CHAIN_THREADS, C_SMEM_BYTES, stream>>>(maps, p);
         SKM_LAUNCH_CHECK();
+        if (beside) beside();
     } else {
         SKM_CUDA(cudaFuncSetAttribute(chain_tc_kernel<kChainSlices>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(C_SMEM_BYTES)));
         p.partial = static_cast<ChainPartial*>(scratch);
@@ -1388,6 +1388,7 @@ void launch_chain(const float* x, const float* y, size_t n, size_t k, size_t d, 
             p.best_in = c == 0 ? best_in : best;
             chain_tc_kernel<kChainSlices><<<static_cast<unsigned>(row_tiles * kChainSlices), CHAIN_THREADS, C_SMEM_BYTES, stream>>>(maps, p);
             SKM_LAUNCH_CHECK();
+            if (c == 0 && beside) beside();
             merge_chain_kernel<<<static_cast<unsigned>((n + 127) / 128), 128, 0, stream>>>(p.partial, static_cast<uint32_t>((cs + BN - 1) / BN), n, c == 0, c + 1 == n_chunks, best_in, best,
                                                                                           state, knn, dist, not_pruned, top2_scratch, p.error);
             SKM_LAUNCH_CHECK();

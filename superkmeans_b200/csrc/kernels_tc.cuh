@@ -6,6 +6,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <functional>
 
 namespace skmb {
 namespace tc {
@@ -110,7 +111,7 @@ void launch_refine_chain_tiles(const float* x, const float* y, size_t n, size_t 
 size_t chain_scratch_bytes(size_t n);   // of `scratch` below (optional: lets a few rows have several blocks per tile); may be none
 void launch_chain(const float* x, const float* y, size_t n, size_t k, size_t d, uint32_t partial_d, uint32_t vertical_d, uint32_t horizontal_d, const float* chain_norms_x,
                   const float* chain_norms_y, const float* ratios, const float* best_in, uint32_t* knn, float* dist, uint32_t* not_pruned, uint2* top2_scratch,
-                  float* y_split, void* scratch, cudaStream_t stream);   // y_split: 2 * k * d floats of scratch for the tf32 parts of the centroids
+                  const float* y_split, void* scratch, cudaStream_t stream, const std::function<void()>& beside = nullptr);   // y_split: 2 * k * d floats of scratch for the tf32 parts of the centroids
 
 // SM cycles after which a wait inside a tensor-core kernel gives up (about two seconds unless a test shortened it).
 long long wait_limit();

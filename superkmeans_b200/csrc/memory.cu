@@ -42,6 +42,7 @@ constexpr int kMaxDevices = 64;
 constexpr int kHost = -1;                 // "device" of pinned host blocks
 constexpr size_t kPinnedBound = size_t{256} << 20;
 constexpr size_t kMaxIdleStreams = 16;    // per device
+constexpr size_t kMaxIdleEvents = 1024;   // that measure time, per device
 
 enum class CacheMode { bounded, everything, nothing };
 
@@ -49,6 +50,7 @@ std::mutex g_mu;
 std::vector<Parked> g_parked;   // oldest first
 CacheMode g_mode = CacheMode::bounded;
 std::vector<cudaEvent_t> g_events[kMaxDevices];
+std::vector<cudaEvent_t> g_timing_events[kMaxDevices];
 std::vector<cudaStream_t> g_streams[kMaxDevices];
 
 // Sizes are rounded up to one of eight steps per power of two, so that requests that differ a little from call to call
@@ -257,6 +259,34 @@ void release_stream(cudaStream_t s, int device) {
     cudaStreamDestroy(s);
 }
 
+cudaEvent_t acquire_timing_event() {
+    int device = 0;
+    SKM_CUDA(cudaGetDevice(&device));
+    {
+        std::lock_guard<std::mutex> lock(g_mu);
+        auto& pool = g_timing_events[device];
+        if (!pool.empty()) {
+            const cudaEvent_t e = pool.back();
+            pool.pop_back();
+            return e;
+        }
+    }
+    cudaEvent_t e = nullptr;
+    SKM_CUDA(cudaEventCreate(&e));
+    return e;
+}
+
+void release_timing_event(cudaEvent_t e, int device) {
+    {
+        std::lock_guard<std::mutex> lock(g_mu);
+        if (g_timing_events[device].size() < kMaxIdleEvents) {
+            g_timing_events[device].push_back(e);
+            return;
+        }
+    }
+    cudaEventDestroy(e);
+}
+
 void set_workspace_cache(bool on) {
     {
         std::lock_guard<std::mutex> lock(g_mu);
@@ -270,7 +300,14 @@ bool workspace_cache_enabled() {
     return g_mode == CacheMode::everything;
 }
 
-void release_cached_memory() { give_back_all(take_all_parked()); }
+void release_cached_memory() {
+    give_back_all(take_all_parked());
+    std::lock_guard<std::mutex> lock(g_mu);
+    for (auto& pool : g_timing_events) {
+        for (cudaEvent_t e : pool) cudaEventDestroy(e);
+        pool.clear();
+    }
+}
 
 size_t cached_memory_bytes() {
     std::lock_guard<std::mutex> lock(g_mu);
