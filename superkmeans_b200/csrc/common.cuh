@@ -341,7 +341,13 @@ struct ConsolidateParams {
     size_t k, d, vertical_d;
     double* reduce_scratch;
     IterationReport* report;
+    const uint4* tell;      // told_words 16-byte words, among them the report, that the last block
+    uint4* told;            // copies to pinned host memory (told_words may be zero)
+    size_t told_words;
 };
+// Pinned host memory (16-byte aligned) = device memory, by a kernel of one block: a copy starts 8 us after the kernel before it ends,
+// the next kernel after 1.
+void launch_tell_host(const void* from, void* to, size_t bytes, cudaStream_t stream);
 void launch_consolidate(const ConsolidateParams& p, cudaStream_t stream);
 
 // out[i][:] = in[idx[i]][:]; an index of all ones gives a row of zeros

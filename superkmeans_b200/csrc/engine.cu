@@ -1082,7 +1082,7 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
                     // points, and one waits for the tensor cores or, with few points, for itself, the other for L2.  (The chain
                     // first: its blocks need most of an SM's shared memory.)
                     const PrunePassCounters* host = b.counters_host.ensure(1);
-                    SKM_CUDA(cudaMemcpyAsync(b.counters_host.get(), counters, sizeof(PrunePassCounters), cudaMemcpyDeviceToHost, stream));
+                    launch_tell_host(counters, b.counters_host.get(), sizeof(PrunePassCounters), stream);
                     SKM_CUDA(cudaStreamSynchronize(stream));
                     n_hard = host->n_dropped;
                     if (n_hard != 0) {
@@ -1183,7 +1183,7 @@ bool Engine::split(size_t n_samples_global, size_t k_cur) {
 
 // The report and the cluster sizes of what is enqueued, once it is done.
 void Engine::fetch_report(size_t k_cur) {
-    SKM_CUDA(cudaMemcpyAsync(outcome_host_.get(), outcome_.get(), sizeof(uint32_t) * (kReportWords + k_cur), cudaMemcpyDeviceToHost, stream_));
+    if (!told_by_kernel(k_cur)) SKM_CUDA(cudaMemcpyAsync(outcome_host_.get(), outcome_.get(), sizeof(uint32_t) * (kReportWords + k_cur), cudaMemcpyDeviceToHost, stream_));
     sync();
     if (report_host()->error != 0) check_tc_error(stream_);
 }
@@ -1204,6 +1204,11 @@ void Engine::consolidate(const IterationInput& in, bool scale) {
     p.vertical_d = vertical_d_;
     p.reduce_scratch = ws_.reduce_scratch;
     p.report = report();
+    if (told_by_kernel(in.n_clusters)) {
+        p.tell = reinterpret_cast<const uint4*>(outcome_.get());
+        p.told = reinterpret_cast<uint4*>(outcome_host_.get());
+        p.told_words = (kReportWords + in.n_clusters + 3) / 4;
+    }
     launch_consolidate(p, stream_);
 }
 

@@ -342,10 +342,14 @@ class Engine {
     uint32_t* counts_host() const { return outcome_host_.get() + kReportWords; }
     IterationReport* report() const { return reinterpret_cast<IterationReport*>(outcome_.get()); }
     const IterationReport* report_host() const { return reinterpret_cast<const IterationReport*>(outcome_host_.get()); }
+    // (whole 16-byte words)
     void reserve_outcome(size_t k) {
-        outcome_.ensure(kReportWords + k);
-        outcome_host_.ensure(kReportWords + k);
+        outcome_.ensure(kReportWords + k + 3);
+        outcome_host_.ensure(kReportWords + k + 3);
     }
+    // The kernel that ends an iteration writes its outcome to the host itself (see launch_tell_host) while that is not more than
+    // one block writes over PCIe in the time saved.
+    static bool told_by_kernel(size_t k) { return k <= 8192; }
     DeviceBuffer<uint32_t> assignments_, not_pruned_;
     DeviceBuffer<float> distances_;
     PrunePassBuffers prune_bufs_;

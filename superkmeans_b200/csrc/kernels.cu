@@ -1074,6 +1074,17 @@ __global__ void __launch_bounds__(256) consolidate_kernel(const ConsolidateParam
         __syncthreads();
     }
     if (threadIdx.x == 0) p.report->shift = sd[0];
+    __syncthreads();
+    for (size_t i = threadIdx.x; i < p.told_words; i += 256) p.told[i] = __ldcg(p.tell + i);
+}
+
+__global__ void __launch_bounds__(256) tell_host_kernel(const uint4* __restrict__ from, uint4* __restrict__ to, size_t words) {
+    for (size_t i = threadIdx.x; i < words; i += 256) to[i] = from[i];
+}
+
+void launch_tell_host(const void* from, void* to, size_t bytes, cudaStream_t stream) {
+    tell_host_kernel<<<1, 256, 0, stream>>>(static_cast<const uint4*>(from), static_cast<uint4*>(to), bytes / 16);
+    SKM_LAUNCH_CHECK();
 }
 
 void launch_consolidate(const ConsolidateParams& p, cudaStream_t stream) {
