@@ -1096,21 +1096,38 @@ void launch_consolidate(const ConsolidateParams& p, cudaStream_t stream) {
 // =================================================================================================
 // Gather / scatter by index
 // =================================================================================================
-__global__ void gather_rows_kernel(const float* __restrict__ in, const uint64_t* __restrict__ idx, float* __restrict__ out, size_t n_out, size_t d) {
-    const size_t row = blockIdx.x;
-    float* dst = out + row * d;
-    if (idx[row] == ~uint64_t{0}) {
-        // "no row here" (held by another shard): zeros
-        for (size_t j = threadIdx.x; j < d; j += blockDim.x) dst[j] = 0.f;
-        return;
+// A warp per row, four 16-byte loads in flight per lane (VEC: 16-byte aligned rows).  300 000 x 768: 0.66 ms with a block per row and
+// 4-byte loads, 0.27 so.
+template <bool VEC>
+__global__ void __launch_bounds__(256) gather_rows_kernel(const float* __restrict__ in, const uint64_t* __restrict__ idx, float* __restrict__ out, size_t n_out, size_t d) {
+    const size_t row = static_cast<size_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+    if (row >= n_out) return;
+    const int lane = threadIdx.x & 31;
+    const uint64_t from = idx[row];
+    // "no row here" (held by another shard): zeros
+    const bool none = from == ~uint64_t{0};
+    const float* __restrict__ src = in + (none ? 0 : from) * d;
+    float* __restrict__ dst = out + row * d;
+    if (VEC) {
+        for (size_t j0 = static_cast<size_t>(lane) * 4; j0 < d; j0 += 512) {
+            float4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = !none && j0 + 128 * u < d ? __ldg(reinterpret_cast<const float4*>(src + j0 + 128 * u)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (j0 + 128 * u < d) *reinterpret_cast<float4*>(dst + j0 + 128 * u) = v[u];
+        }
+    } else {
+#pragma unroll 4
+        for (size_t j = lane; j < d; j += 32) dst[j] = none ? 0.f : __ldg(src + j);
     }
-    const float* src = in + idx[row] * d;
-    for (size_t j = threadIdx.x; j < d; j += blockDim.x) dst[j] = src[j];
 }
 
 void launch_gather_rows(const float* in, const uint64_t* idx, float* out, size_t n_out, size_t d, cudaStream_t stream) {
     if (n_out == 0) return;
-    gather_rows_kernel<<<static_cast<unsigned>(n_out), 256, 0, stream>>>(in, idx, out, n_out, d);
+    const unsigned grid = static_cast<unsigned>((n_out + 7) / 8);
+    if (d % 4 == 0 && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) gather_rows_kernel<true><<<grid, 256, 0, stream>>>(in, idx, out, n_out, d);
+    else gather_rows_kernel<false><<<grid, 256, 0, stream>>>(in, idx, out, n_out, d);
     SKM_LAUNCH_CHECK();
 }
 
