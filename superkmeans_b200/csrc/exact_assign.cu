@@ -422,7 +422,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(F_THREADS, 1)
                     } else {
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive_cluster(cluster_address(&ctrl->acc_empty[b], 0));
+                        if (lane == 0) mbar_arrive_cluster_read(cluster_address(&ctrl->acc_empty[b], 0));
                     }
                     look(rb, ch + 1);
                     if (ch == slice0) tmem_ld_wait(ra);

@@ -13,7 +13,8 @@
 //              the warp's list.  The test is what bounds the kernel, its latency more than its 200 instructions per 32
 //              columns: hence four warps per scheduler (with two it took 6500 cycles per tile), two columns per instruction
 //              and no scan for the places in the list.  1M x 1024, k = 4000, nine passes: 27.2 ms with one column per
-//              instruction and a scan by shuffles, 25.0 so.
+//              instruction and a scan by shuffles, 25.0 so, and 20.1 since the accumulators are given back without a release
+//              at cluster scope, which waited for the lists' stores (a third of all stalls).
 // Every wait is bounded (see kernels_tc.cu).
 #include <cfloat>
 #include <cmath>
@@ -285,7 +286,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T_THREADS, 1) first_
                     if (ch == 1) {
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive_cluster(cluster_address(&ctrl->acc_empty[b], 0));
+                        if (lane == 0) mbar_arrive_cluster_read(cluster_address(&ctrl->acc_empty[b], 0));
                     }
                     test(r, ch);
                 }

@@ -237,7 +237,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ROT_THREADS, 1)
                 }
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(cluster_address(&ctrl->acc_empty[b], 0));
+                if (lane == 0) mbar_arrive_cluster_read(cluster_address(&ctrl->acc_empty[b], 0));
             }
             if (!ok || row >= p.n) continue;
             float* orow = p.out + row * p.ldo + col0;

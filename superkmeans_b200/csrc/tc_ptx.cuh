@@ -181,6 +181,11 @@ __device__ __forceinline__ uint32_t cluster_address(const void* p, uint32_t rank
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
+// The same for a thread that has only read tensor memory (and fenced that, tc_fence_before): it passes no data of its own, and a
+// release at cluster scope would wait for every global store it has under way.
+__device__ __forceinline__ void mbar_arrive_cluster_read(uint32_t cluster_bar) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
 // into this CTA's shared memory, counted by a barrier of either CTA of the pair
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t smem_dst, const CUtensorMap* tmap, uint32_t cluster_bar, int x, int y) {
     asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_dst),
