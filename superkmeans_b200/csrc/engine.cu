@@ -163,7 +163,7 @@ Engine::Engine(const skm_config& cfg, size_t n_clusters, size_t d, bool hierarch
 }
 
 Engine::~Engine() {
-    if (draws_done_.valid()) draws_done_.wait();
+    if (rotation_made_.valid()) rotation_made_.wait();
     if (default_stream_work_) cudaEventDestroy(default_stream_work_);
     // the streams are waited for: the buffers released after this are idle
     int prev = device_;
@@ -194,40 +194,67 @@ void Engine::wait_for_default_stream() {
 // -------------------------------------------------------------------------------------------------
 // Rotation (adsampling.h:76-85, :191-215, :273-298)
 // -------------------------------------------------------------------------------------------------
-void Engine::start_rotation_draws() {
-    if (rotation_ready_ || !rotation_host_.empty() || draws_) return;
-    draws_ = std::make_unique<NormalDraws>(d_ * d_, cfg_.seed);
-    uint32_t* bits = draw_bits_.ensure(draws_->scratch());
-    float* values = draw_values_.ensure(draws_->scratch());
-    draws_->values_at(values);
-    draws_done_ = std::async(std::launch::async, [this, bits, values] { draws_->make(bits, values); });
+// The matrix that is still to be made, on a host thread and a stream of their own: its draws take a millisecond and its two
+// hundred dependent launches two more, while the caller's rows are on their way.
+void Engine::start_rotation() {
+    if (rotation_ready_ || rotation_made_.valid() || !rotation_host_.empty()) return;
+    rotation_made_ = std::async(std::launch::async, [this] {
+        DeviceGuard guard(device_);
+        const cudaStream_t s = acquire_stream();
+        try {
+            WorkStream work(s);
+            NormalDraws draws(d_ * d_, cfg_.seed);
+            PinnedBuffer<uint32_t> bits;
+            PinnedBuffer<float> values;
+            draws.values_at(values.ensure(draws.scratch()));
+            bits.ensure(draws.scratch());
+            std::future<void> drawn;
+            if (draws.threads() > 1) drawn = std::async(std::launch::async, [&] { draws.make(bits.get(), values.get()); });
+            else draws.make(bits.get(), values.get());
+            float* m = m_dev_.ensure(d_ * d_);
+            float* to = mt_dev_.ensure(d_ * d_);   // (not needed for the transpose yet)
+            // as they come, in a few groups, read from host memory by a kernel: copies would queue behind those of the rows
+            const size_t per_group = (draws.pieces() + 3) / 4;
+            size_t got = 0;
+            for (size_t t0 = 0; t0 < draws.pieces(); t0 += per_group) {
+                DrawPieces p{};
+                p.values = draws.piece(t0).values;
+                p.stretch = draws.stretch();
+                for (size_t t = t0; t < std::min(draws.pieces(), t0 + per_group); ++t) {
+                    p.start[p.n++] = got;
+                    got = std::min(got + draws.piece(t).count, d_ * d_);
+                }
+                p.start[p.n] = got;
+                launch_collect_draws(p, to, s);
+            }
+            const bool made = got == d_ * d_ && make_rotation_matrix_on_device(to, d_, m, s);
+            if (!made) {
+                SKM_CUDA(cudaStreamSynchronize(s));
+                rotation_host_ = make_rotation_matrix(d_, cfg_.seed);
+                SKM_CUDA(cudaMemcpyAsync(m, rotation_host_.data(), sizeof(float) * d_ * d_, cudaMemcpyHostToDevice, s));
+            }
+            launch_transpose_square(m, to, d_, s);
+            SKM_CUDA(cudaStreamSynchronize(s));
+        } catch (...) {
+            release_stream(s, device_);
+            throw;
+        }
+        release_stream(s, device_);
+    });
 }
 
 void Engine::ensure_rotation() {
     if (rotation_ready_) return;
-    float* m = m_dev_.ensure(d_ * d_);
-    bool made = false;
-    if (rotation_host_.empty()) {
-        start_rotation_draws();
-        float* draws = mt_dev_.ensure(d_ * d_);   // (not needed for the transpose yet)
-        size_t got = 0;
-        for (size_t t = 0; t < draws_->pieces() && got < d_ * d_; ++t) {
-            const auto piece = draws_->piece(t);
-            const size_t n = std::min(piece.count, d_ * d_ - got);
-            SKM_CUDA(cudaMemcpyAsync(draws + got, piece.values, sizeof(float) * n, cudaMemcpyHostToDevice, stream_));
-            got += n;
-        }
-        made = got == d_ * d_ && make_rotation_matrix_on_device(draws, d_, m, stream_);
-        if (!made) rotation_host_ = make_rotation_matrix(d_, cfg_.seed);
+    start_rotation();
+    if (rotation_made_.valid()) {
+        rotation_made_.get();
+    } else {
+        float* m = m_dev_.ensure(d_ * d_);
+        SKM_CUDA(cudaMemcpyAsync(m, rotation_host_.data(), sizeof(float) * d_ * d_, cudaMemcpyHostToDevice, stream_));
+        launch_transpose_square(m, mt_dev_.ensure(d_ * d_), d_, stream_);
+        sync();
     }
-    if (!made) SKM_CUDA(cudaMemcpyAsync(m, rotation_host_.data(), sizeof(float) * d_ * d_, cudaMemcpyHostToDevice, stream_));
-    launch_transpose_square(m, mt_dev_.ensure(d_ * d_), d_, stream_);
-    sync();
     rotation_ready_ = true;
-    if (draws_done_.valid()) draws_done_.wait();
-    draws_.reset();
-    draw_bits_.release();
-    draw_values_.release();
 }
 
 void Engine::ensure_rotation_host() {
@@ -240,6 +267,8 @@ void Engine::ensure_rotation_host() {
 
 void Engine::set_rotation(const float* m_host) {
     Entry entry(device_, stream_);
+    if (rotation_made_.valid()) rotation_made_.wait();   // (of a Train that failed)
+    rotation_made_ = {};
     rotation_host_.assign(m_host, m_host + d_ * d_);
     rotation_ready_ = false;
     ensure_rotation();
@@ -1371,7 +1400,7 @@ void Engine::train_flat(const float* data, size_t n, bool on_device, const float
     }
     n_samples_ = sharded_() ? n : n_samples_global;
     const bool rotate = !cfg_.data_already_rotated;
-    if (rotate || cfg_.unrotate_centroids) start_rotation_draws();
+    if (rotate || cfg_.unrotate_centroids) start_rotation();
     partial_d_ = initial_partial_d(vertical_d_);
     // The Forgy shuffle runs over all n_samples indices with std::mt19937 (a tenth of a second at 1e7): on a thread of
     // its own, while this one allocates the buffers and starts the rotation.
@@ -1550,7 +1579,7 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
     }
     const size_t n_all = n_samples_;
     const bool rotate = !cfg_.data_already_rotated;
-    if (rotate || cfg_.unrotate_centroids) start_rotation_draws();
+    if (rotate || cfg_.unrotate_centroids) start_rotation();
     partial_d_ = initial_partial_d(vertical_d_);
     const uint32_t initial_pd = partial_d_;
     // The shuffles behind the first centroids and the sample run on threads of their own meanwhile.

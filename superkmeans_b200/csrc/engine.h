@@ -163,6 +163,15 @@ void set_prune_split_mode(int mode);
 int prune_split_mode();
 void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, int device, cudaStream_t stream, PhaseTimers* timers = nullptr);
 
+// Pieces of the draws in pinned memory, piece t at values + t * stretch, entries [start[t], start[t + 1]) of the whole.
+struct DrawPieces {
+    const float* values;
+    size_t stretch;
+    uint32_t n;
+    size_t start[NormalDraws::kMaxPieces + 1];
+};
+void launch_collect_draws(const DrawPieces& p, float* out, cudaStream_t stream);
+
 // out (device, d x d) = the matrix make_rotation_matrix computes, from its draws normal_draws(d * d, seed) (device), on `stream`
 // (synchronised once or twice on the way).  False: declined, nothing usable in `out` (rotation_matrix.cu).
 bool make_rotation_matrix_on_device(const float* draws, size_t d, float* out, cudaStream_t stream);
@@ -244,7 +253,7 @@ class Engine {
         mutable double survival = 0.0;        // ... and what it said about the next one (PrunedParams)
     };
 
-    void start_rotation_draws();   // the Gaussian draws of a matrix that is still to be made, on a host thread
+    void start_rotation();
     void ensure_rotation();
     void ensure_rotation_host();
     // after_rows(r0, cnt), if given, is called (host side, work enqueued on stream_) whenever rows [r0, r0 + cnt) of dst
@@ -311,10 +320,7 @@ class Engine {
     // pruner state
     float epsilon0_;
     std::vector<float> rotation_host_;  // d x d, empty until needed (a matrix made on the device is fetched on demand)
-    std::unique_ptr<NormalDraws> draws_;   // of a matrix that is being made
-    std::future<void> draws_done_;
-    PinnedBuffer<uint32_t> draw_bits_;
-    PinnedBuffer<float> draw_values_;
+    std::future<void> rotation_made_;   // valid while a matrix is being made
     bool rotation_ready_ = false;
     DeviceBuffer<float> m_dev_, mt_dev_, ratios_dev_;
     uint32_t vertical_d_ = 0, horizontal_d_ = 0, partial_d_ = 0;

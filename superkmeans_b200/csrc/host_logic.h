@@ -395,8 +395,8 @@ class NormalDraws {
         // a pair is accepted with probability pi / 4; half a percent and 2000 pairs more than needed are a dozen standard deviations
         const double pairs = static_cast<double>((count + 1) / 2) / 0.7853 * 1.005 + 2000.0;
         const size_t blocks = static_cast<size_t>(2.0 * pairs / Mt19937Blocks::N) + 1;
-        blocks_ = std::max<size_t>(16, (blocks + 47) / 48);
-        stretches_ = (blocks + blocks_ - 1) / blocks_;
+        blocks_ = std::max<size_t>(16, (blocks + kMaxPieces - 1) / kMaxPieces);
+        stretches_ = (blocks + blocks_ - 1) / blocks_;   // (kMaxPieces at most)
         made_.reset(new std::atomic<size_t>[stretches_]);
         for (size_t t = 0; t < stretches_; ++t) made_[t].store(kNotYet);
     }
@@ -437,12 +437,15 @@ class NormalDraws {
         if (starter.joinable()) starter.join();
         for (auto& th : pool) th.join();
     }
+    unsigned threads() const { return threads_; }
+    static constexpr size_t kMaxPieces = 48;
     struct Piece {
         const float* values;
         size_t count;
     };
     // The draws in order, as up to pieces() pieces of `values`; piece(t) waits until make() has come to it.
     size_t pieces() const { return stretches_; }
+    size_t stretch() const { return blocks_ * Mt19937Blocks::N; }   // from one piece to the next
     Piece piece(size_t t) const {
         size_t n;
         while ((n = made_[t].load(std::memory_order_acquire)) == kNotYet) std::this_thread::yield();
@@ -451,7 +454,6 @@ class NormalDraws {
 
   private:
     static constexpr size_t kNotYet = ~size_t{0};
-    size_t stretch() const { return blocks_ * Mt19937Blocks::N; }
     size_t draw_stretch(const uint32_t* bits, float* out) const {
         constexpr size_t kBatch = 512;
         float x[kBatch], y[kBatch], r2[kBatch];

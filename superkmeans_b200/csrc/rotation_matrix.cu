@@ -39,6 +39,14 @@ constexpr int kThreads = 256;
 constexpr size_t kSolveSmem = 200 * 1024;
 constexpr int kSolveMaxRows = 16;
 
+// A column of blocks per piece; pinned memory is read in place.
+__global__ void __launch_bounds__(kThreads) collect_draws_kernel(const DrawPieces p, float* __restrict__ out) {
+    const uint32_t t = blockIdx.y;
+    const float* from = p.values + t * p.stretch;
+    const size_t at = p.start[t], n = p.start[t + 1] - at;
+    for (size_t i = static_cast<size_t>(blockIdx.x) * kThreads + threadIdx.x; i < n; i += static_cast<size_t>(gridDim.x) * kThreads) out[at + i] = from[i];
+}
+
 // Double copy of the draws, padded with the identity to a multiple of GT, so that nothing below has edges.
 __global__ void widen_draws_kernel(const float* __restrict__ draws, size_t d, size_t dp, double* __restrict__ a) {
     const size_t j = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x, i = blockIdx.y;
@@ -388,6 +396,12 @@ void factorise(double* m, size_t dp, double* r, double* inverses, float* signs, 
 }
 
 } // namespace
+
+void launch_collect_draws(const DrawPieces& p, float* out, cudaStream_t stream) {
+    if (p.n == 0) return;
+    collect_draws_kernel<<<dim3(16, p.n), kThreads, 0, stream>>>(p, out);
+    SKM_LAUNCH_CHECK();
+}
 
 bool make_rotation_matrix_on_device(const float* draws, size_t d, float* out, cudaStream_t stream) {
     const size_t dp = (d + GT - 1) / GT * GT;
