@@ -163,8 +163,9 @@ Engine::Engine(const skm_config& cfg, size_t n_clusters, size_t d, bool hierarch
 }
 
 Engine::~Engine() {
-    if (rotation_made_.valid()) rotation_made_.wait();
+    drop_rotation();
     if (default_stream_work_) cudaEventDestroy(default_stream_work_);
+    if (rotation_event_) cudaEventDestroy(rotation_event_);
     // the streams are waited for: the buffers released after this are idle
     int prev = device_;
     cudaGetDevice(&prev);
@@ -194,60 +195,92 @@ void Engine::wait_for_default_stream() {
 // -------------------------------------------------------------------------------------------------
 // Rotation (adsampling.h:76-85, :191-215, :273-298)
 // -------------------------------------------------------------------------------------------------
-// The matrix that is still to be made, on a host thread and a stream of their own: its draws take a millisecond and its two
-// hundred dependent launches two more, while the caller's rows are on their way.
-void Engine::start_rotation() {
-    if (rotation_ready_ || rotation_made_.valid() || !rotation_host_.empty()) return;
+// The draws of a matrix that is being made.
+struct Engine::Drawing {
+    NormalDraws draws;
+    PinnedBuffer<uint32_t> bits;
+    PinnedBuffer<float> values;
+    std::future<void> drawn;   // (the last member: waits for its thread before the others go)
+    Drawing(size_t count, uint32_t seed) : draws(count, seed) {
+        bits.ensure(draws.scratch());
+        draws.values_at(values.ensure(draws.scratch()));
+        if (draws.threads() > 1) drawn = std::async(std::launch::async, [this] { draws.make(bits.get(), values.get()); });
+        else draws.make(bits.get(), values.get());
+    }
+};
+
+// Begins the matrix that is still to be made: its draws, on host threads (a millisecond), and, if the caller's rows are yet to be
+// staged, its two hundred dependent launches too (two more), on a thread and a stream of their own beside that.
+void Engine::start_rotation(bool beside) {
+    if (rotation_ready_ || drawing_ || !rotation_host_.empty()) return;
+    drawing_ = std::make_unique<Drawing>(d_ * d_, cfg_.seed);
+    if (!beside) return;
+    if (!rotation_event_) SKM_CUDA(cudaEventCreateWithFlags(&rotation_event_, cudaEventDisableTiming));
+    rotation_state_.store(RotationState::none);
     rotation_made_ = std::async(std::launch::async, [this] {
-        DeviceGuard guard(device_);
-        const cudaStream_t s = acquire_stream();
         try {
-            WorkStream work(s);
-            NormalDraws draws(d_ * d_, cfg_.seed);
-            PinnedBuffer<uint32_t> bits;
-            PinnedBuffer<float> values;
-            draws.values_at(values.ensure(draws.scratch()));
-            bits.ensure(draws.scratch());
-            std::future<void> drawn;
-            if (draws.threads() > 1) drawn = std::async(std::launch::async, [&] { draws.make(bits.get(), values.get()); });
-            else draws.make(bits.get(), values.get());
-            float* m = m_dev_.ensure(d_ * d_);
-            float* to = mt_dev_.ensure(d_ * d_);   // (not needed for the transpose yet)
-            // as they come, in a few groups, read from host memory by a kernel: copies would queue behind those of the rows
-            const size_t per_group = (draws.pieces() + 3) / 4;
-            size_t got = 0;
-            for (size_t t0 = 0; t0 < draws.pieces(); t0 += per_group) {
-                DrawPieces p{};
-                p.values = draws.piece(t0).values;
-                p.stretch = draws.stretch();
-                for (size_t t = t0; t < std::min(draws.pieces(), t0 + per_group); ++t) {
-                    p.start[p.n++] = got;
-                    got = std::min(got + draws.piece(t).count, d_ * d_);
-                }
-                p.start[p.n] = got;
-                launch_collect_draws(p, to, s);
-            }
-            const bool made = got == d_ * d_ && make_rotation_matrix_on_device(to, d_, m, s);
-            if (!made) {
-                SKM_CUDA(cudaStreamSynchronize(s));
-                rotation_host_ = make_rotation_matrix(d_, cfg_.seed);
-                SKM_CUDA(cudaMemcpyAsync(m, rotation_host_.data(), sizeof(float) * d_ * d_, cudaMemcpyHostToDevice, s));
-            }
-            launch_transpose_square(m, to, d_, s);
-            SKM_CUDA(cudaStreamSynchronize(s));
+            DeviceGuard guard(device_);
+            struct Stream {
+                const int device;
+                const cudaStream_t s;
+                explicit Stream(int device_) : device(device_), s(acquire_stream()) {}
+                ~Stream() { release_stream(s, device); }   // (waits)
+            } own(device_);
+            WorkStream work(own.s);
+            make_rotation(own.s);
+            SKM_CUDA(cudaEventRecord(rotation_event_, own.s));
+            rotation_state_.store(RotationState::enqueued, std::memory_order_release);
         } catch (...) {
-            release_stream(s, device_);
+            rotation_state_.store(RotationState::failed, std::memory_order_release);
             throw;
         }
-        release_stream(s, device_);
     });
+}
+
+// Enqueues on `stream`; returns before the last kernels have run.
+void Engine::make_rotation(cudaStream_t stream) {
+    NormalDraws& draws = drawing_->draws;
+    float* m = m_dev_.ensure(d_ * d_);
+    float* to = mt_dev_.ensure(d_ * d_);   // (not needed for the transpose yet)
+    // as they come, in a few groups, read from host memory by a kernel: copies would queue behind those of the rows
+    const size_t per_group = (draws.pieces() + 7) / 8;
+    size_t got = 0;
+    for (size_t t0 = 0; t0 < draws.pieces(); t0 += per_group) {
+        DrawPieces p{};
+        p.values = draws.piece(t0).values;
+        p.stretch = draws.stretch();
+        for (size_t t = t0; t < std::min(draws.pieces(), t0 + per_group); ++t) {
+            p.start[p.n++] = got;
+            got = std::min(got + draws.piece(t).count, d_ * d_);
+        }
+        p.start[p.n] = got;
+        launch_collect_draws(p, to, stream);
+    }
+    if (got != d_ * d_ || !make_rotation_matrix_on_device(to, d_, m, stream)) {
+        SKM_CUDA(cudaStreamSynchronize(stream));
+        rotation_host_ = make_rotation_matrix(d_, cfg_.seed);
+        SKM_CUDA(cudaMemcpyAsync(m, rotation_host_.data(), sizeof(float) * d_ * d_, cudaMemcpyHostToDevice, stream));
+    }
+    launch_transpose_square(m, to, d_, stream);
 }
 
 void Engine::ensure_rotation() {
     if (rotation_ready_) return;
-    start_rotation();
+    start_rotation(false);
     if (rotation_made_.valid()) {
-        rotation_made_.get();
+        // what follows is enqueued behind the last kernels, which are still to run
+        while (rotation_state_.load(std::memory_order_acquire) == RotationState::none) std::this_thread::yield();
+        if (rotation_state_.load() == RotationState::failed) {
+            std::future<void> failed = std::move(rotation_made_);
+            failed.wait();
+            drawing_.reset();
+            failed.get();   // (throws)
+        }
+        SKM_CUDA(cudaStreamWaitEvent(stream_, rotation_event_, 0));
+    } else if (drawing_) {
+        make_rotation(stream_);
+        sync();
+        drawing_.reset();
     } else {
         float* m = m_dev_.ensure(d_ * d_);
         SKM_CUDA(cudaMemcpyAsync(m, rotation_host_.data(), sizeof(float) * d_ * d_, cudaMemcpyHostToDevice, stream_));
@@ -255,6 +288,13 @@ void Engine::ensure_rotation() {
         sync();
     }
     rotation_ready_ = true;
+}
+
+// Ends what start_rotation began.
+void Engine::drop_rotation() {
+    if (rotation_made_.valid()) rotation_made_.wait();
+    rotation_made_ = {};
+    drawing_.reset();
 }
 
 void Engine::ensure_rotation_host() {
@@ -267,8 +307,7 @@ void Engine::ensure_rotation_host() {
 
 void Engine::set_rotation(const float* m_host) {
     Entry entry(device_, stream_);
-    if (rotation_made_.valid()) rotation_made_.wait();   // (of a Train that failed)
-    rotation_made_ = {};
+    drop_rotation();   // (of a Train that failed)
     rotation_host_.assign(m_host, m_host + d_ * d_);
     rotation_ready_ = false;
     ensure_rotation();
@@ -1385,6 +1424,7 @@ void Engine::train(const float* data, size_t n, bool on_device, const float* que
     }
     timers_.end(stream_);
     sync();
+    drop_rotation();
     timers_.add_host(PH_ALLOC_FREE, alloc_free_ms() - alloc_ms0);
 }
 
@@ -1400,7 +1440,7 @@ void Engine::train_flat(const float* data, size_t n, bool on_device, const float
     }
     n_samples_ = sharded_() ? n : n_samples_global;
     const bool rotate = !cfg_.data_already_rotated;
-    if (rotate || cfg_.unrotate_centroids) start_rotation();
+    if (rotate || cfg_.unrotate_centroids) start_rotation(!on_device);
     partial_d_ = initial_partial_d(vertical_d_);
     // The Forgy shuffle runs over all n_samples indices with std::mt19937 (a tenth of a second at 1e7): on a thread of
     // its own, while this one allocates the buffers and starts the rotation.
@@ -1579,7 +1619,7 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
     }
     const size_t n_all = n_samples_;
     const bool rotate = !cfg_.data_already_rotated;
-    if (rotate || cfg_.unrotate_centroids) start_rotation();
+    if (rotate || cfg_.unrotate_centroids) start_rotation(!on_device);
     partial_d_ = initial_partial_d(vertical_d_);
     const uint32_t initial_pd = partial_d_;
     // The shuffles behind the first centroids and the sample run on threads of their own meanwhile.

@@ -7,6 +7,7 @@
 #include <stdexcept>
 #include <string>
 #include <functional>
+#include <atomic>
 #include <future>
 #include <memory>
 #include <vector>
@@ -253,7 +254,9 @@ class Engine {
         mutable double survival = 0.0;        // ... and what it said about the next one (PrunedParams)
     };
 
-    void start_rotation();
+    void start_rotation(bool beside);
+    void make_rotation(cudaStream_t stream);
+    void drop_rotation();
     void ensure_rotation();
     void ensure_rotation_host();
     // after_rows(r0, cnt), if given, is called (host side, work enqueued on stream_) whenever rows [r0, r0 + cnt) of dst
@@ -320,7 +323,12 @@ class Engine {
     // pruner state
     float epsilon0_;
     std::vector<float> rotation_host_;  // d x d, empty until needed (a matrix made on the device is fetched on demand)
-    std::future<void> rotation_made_;   // valid while a matrix is being made
+    struct Drawing;
+    std::unique_ptr<Drawing> drawing_;   // while a matrix is being made
+    std::future<void> rotation_made_;    // valid from when that is done on a thread of its own
+    enum class RotationState { none, enqueued, failed };
+    std::atomic<RotationState> rotation_state_{RotationState::none};
+    cudaEvent_t rotation_event_ = nullptr;   // behind its last kernel
     bool rotation_ready_ = false;
     DeviceBuffer<float> m_dev_, mt_dev_, ratios_dev_;
     uint32_t vertical_d_ = 0, horizontal_d_ = 0, partial_d_ = 0;
