@@ -348,6 +348,7 @@ struct ConsolidateParams {
 // Pinned host memory (16-byte aligned) = device memory, by a kernel of one block: a copy starts 8 us after the kernel before it ends,
 // the next kernel after 1.
 void launch_tell_host(const void* from, void* to, size_t bytes, cudaStream_t stream);
+void launch_tell_word(const void* from, void* to, cudaStream_t stream);   // four bytes
 void launch_consolidate(const ConsolidateParams& p, cudaStream_t stream);
 
 // out[i][:] = in[idx[i]][:]; an index of all ones gives a row of zeros

@@ -1536,7 +1536,6 @@ void Engine::train_flat(const float* data, size_t n, bool on_device, const float
     n_state_rows_ = n_samples_;
     trained_ = true;
     output_centroids(centroids_out);
-    check_tc_error(stream_);
     x_rot_.release();
     ws_partials_.release();
 }
@@ -1602,7 +1601,16 @@ void Engine::output_centroids(float* out_host) {
         launch_gemm_nt(c, d_, mt_dev_.get(), d_, tmp.ensure(k_ * d_), d_, k_, d_, d_, stream_);
         c = tmp.get();
     }
+    tell_error();
     stage_.download(out_host, c, sizeof(float) * k_ * d_, stream_);
+    check_told_error();
+}
+
+// The error word of the tensor-core kernels, on its way to the host ahead of a copy or a wait that the caller makes anyway, and
+// what it was once that is over.
+void Engine::tell_error() { launch_tell_word(tc::error_word(), error_host_.ensure(1), stream_); }
+void Engine::check_told_error() {
+    if (*error_host_.get() != 0) check_tc_error(stream_);
 }
 
 // -------------------------------------------------------------------------------------------------
@@ -1836,8 +1844,11 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
             PhaseScope ps(*this, PH_ASSIGN_FULL);
             exact_assignment(vectors, n, c_dev, n_centroids, xn.ensure(n), false, cn.get(), out, dist.ensure(n));
         }
+        // (a direct call waits for nothing that can run out)
+        const bool direct_call = assign_route(n, n_centroids, d_) == AssignRoute::direct;
+        if (!direct_call) tell_error();
         sync();
-        if (assign_route(n, n_centroids, d_) != AssignRoute::direct) check_tc_error(stream_);   // (a direct call waits for nothing that can run out)
+        if (!direct_call) check_told_error();
         return;
     }
     const AssignRoute route = assign_route(n, n_centroids, d_);
@@ -1892,13 +1903,14 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
         }
     }
     timers_.end(stream_);
+    if (!direct) tell_error();
     // the answers are a d-th of the rows: fetched once, so that no copy back holds up the next upload
     stage_.download(out, knn.get(), sizeof(uint32_t) * n, stream_);
     for (int i = 0; i < 2; ++i) {
         cudaEventDestroy(copied[i]);
         cudaEventDestroy(consumed[i]);
     }
-    if (!direct) check_tc_error(stream_);
+    if (!direct) check_told_error();
 }
 
 // -------------------------------------------------------------------------------------------------

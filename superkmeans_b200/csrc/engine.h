@@ -285,6 +285,9 @@ class Engine {
                         const std::vector<std::vector<size_t>>& forgy, size_t fine_offset);
     void print_iteration(const skm_iter_stats& s, uint32_t next_partial_d) const;
     void check_tensor_cores();
+    void tell_error();
+    void check_told_error();
+    PinnedBuffer<int> error_host_;
     void output_centroids(float* out_host);
     void allreduce(void* buf, size_t count, int dtype);
     void allreduce_iteration(float* sums, size_t n_sums, uint32_t* counts, size_t n_counts, double* scalars, size_t n_scalars);

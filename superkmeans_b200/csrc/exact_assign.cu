@@ -729,7 +729,7 @@ void ExactAssign::assign_groups(const float* x, size_t n, const float* y, size_t
 
 size_t ExactAssign::settle(cudaStream_t stream) {
     uint32_t* host = n_listed_host_.ensure(1);
-    SKM_CUDA(cudaMemcpyAsync(host, n_listed_.get(), sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
+    launch_tell_word(n_listed_.get(), host, stream);
     SKM_CUDA(cudaStreamSynchronize(stream));
     return *host;
 }

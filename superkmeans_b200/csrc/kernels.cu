@@ -1082,6 +1082,13 @@ __global__ void __launch_bounds__(256) tell_host_kernel(const uint4* __restrict_
     for (size_t i = threadIdx.x; i < words; i += 256) to[i] = from[i];
 }
 
+__global__ void tell_word_kernel(const uint32_t* __restrict__ from, uint32_t* __restrict__ to) { *to = *from; }
+
+void launch_tell_word(const void* from, void* to, cudaStream_t stream) {
+    tell_word_kernel<<<1, 1, 0, stream>>>(static_cast<const uint32_t*>(from), static_cast<uint32_t*>(to));
+    SKM_LAUNCH_CHECK();
+}
+
 void launch_tell_host(const void* from, void* to, size_t bytes, cudaStream_t stream) {
     tell_host_kernel<<<1, 256, 0, stream>>>(static_cast<const uint4*>(from), static_cast<uint4*>(to), bytes / 16);
     SKM_LAUNCH_CHECK();
