@@ -49,7 +49,7 @@ void release_stream(cudaStream_t s, int device);
 // Events that measure time, from a bounded pool of the current device.
 cudaEvent_t acquire_timing_event();
 void release_timing_event(cudaEvent_t e, int device);
-// While one is alive, what its thread allocates and releases is used by work on `stream`.
+// While one is alive, what its thread allocates and releases is used by work on `stream`, a stream of the current device.
 class WorkStream {
   public:
     explicit WorkStream(cudaStream_t stream);
@@ -60,6 +60,7 @@ class WorkStream {
   private:
     bool was_on_;
     cudaStream_t previous_;
+    int previous_device_;
 };
 void set_workspace_cache(bool on);
 bool workspace_cache_enabled();

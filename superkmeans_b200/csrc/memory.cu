@@ -25,6 +25,7 @@ std::atomic<unsigned long long> g_device_allocs{0};
 thread_local double g_alloc_ms = 0.0;
 thread_local bool t_on_stream = false;
 thread_local cudaStream_t t_stream = nullptr;
+thread_local int t_device = 0;   // of t_stream
 
 struct AllocClock {
     std::chrono::steady_clock::time_point t0 = std::chrono::steady_clock::now();
@@ -35,7 +36,8 @@ struct Parked {
     void* p;
     size_t bytes;
     int device;
-    cudaEvent_t last_use;   // null: idle
+    cudaEvent_t last_use = nullptr;   // null: idle
+    int event_device = 0;             // of last_use: the device of a pinned block's last user, which the next one need not share
 };
 
 constexpr int kMaxDevices = 64;
@@ -113,27 +115,49 @@ bool take_parked(size_t bytes, int device, Parked& out) {
     return true;
 }
 
-// Orders the new owner of a block after its last one.
-void settle(const Parked& b, int event_device) {
+// Orders the new owner of a block after its last one.  (An event goes back to the pool of its own device: only streams of that
+// one can record it.)
+void settle(const Parked& b) {
     if (!b.last_use) return;
-    if (b.device == kHost || !t_on_stream) cudaEventSynchronize(b.last_use);
-    else SKM_CUDA(cudaStreamWaitEvent(t_stream, b.last_use, 0));
+    const cudaError_t e = b.device == kHost || !t_on_stream ? cudaEventSynchronize(b.last_use) : cudaStreamWaitEvent(t_stream, b.last_use, 0);
+    if (e != cudaSuccess) {
+        give_back(b);
+        cuda_check(e, "wait for the last use of a parked block", __FILE__, __LINE__);
+    }
     std::lock_guard<std::mutex> lock(g_mu);
-    g_events[event_device].push_back(b.last_use);
+    g_events[b.event_device].push_back(b.last_use);
 }
 
-void park(Parked b, int event_device) {
-    if (t_on_stream) {
-        {
-            std::lock_guard<std::mutex> lock(g_mu);
-            auto& pool = g_events[event_device];
-            if (!pool.empty()) {
-                b.last_use = pool.back();
-                pool.pop_back();
-            }
+// An event recorded where t_stream stands, or null.
+cudaEvent_t mark_stream() {
+    cudaEvent_t event = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(g_mu);
+        auto& pool = g_events[t_device];
+        if (!pool.empty()) {
+            event = pool.back();
+            pool.pop_back();
         }
-        if (!b.last_use && cudaEventCreateWithFlags(&b.last_use, cudaEventDisableTiming) != cudaSuccess) b.last_use = nullptr;
-        if (!b.last_use || cudaEventRecord(b.last_use, t_stream) != cudaSuccess) {
+    }
+    int cur = t_device;
+    cudaGetDevice(&cur);
+    if (cur != t_device) cudaSetDevice(t_device);
+    if (!event && cudaEventCreateWithFlags(&event, cudaEventDisableTiming) != cudaSuccess) event = nullptr;
+    if (event && cudaEventRecord(event, t_stream) != cudaSuccess) {
+        cudaEventDestroy(event);
+        event = nullptr;
+    }
+    if (cur != t_device) cudaSetDevice(cur);
+    return event;
+}
+
+void park(Parked b) {
+    if (t_on_stream) {
+        b.last_use = mark_stream();
+        b.event_device = t_device;
+        if (!b.last_use) {
+            cudaStreamSynchronize(t_stream);
+            cudaGetLastError();   // (ours; the caller's next check is about its own work)
             give_back(b);
             return;
         }
@@ -169,13 +193,15 @@ unsigned long long device_alloc_count() { return g_device_allocs.load(std::memor
 void note_device_alloc() { g_device_allocs.fetch_add(1, std::memory_order_relaxed); }
 double alloc_free_ms() { return g_alloc_ms; }
 
-WorkStream::WorkStream(cudaStream_t stream) : was_on_(t_on_stream), previous_(t_stream) {
+WorkStream::WorkStream(cudaStream_t stream) : was_on_(t_on_stream), previous_(t_stream), previous_device_(t_device) {
+    SKM_CUDA(cudaGetDevice(&t_device));
     t_on_stream = true;
     t_stream = stream;
 }
 WorkStream::~WorkStream() {
     t_on_stream = was_on_;
     t_stream = previous_;
+    t_device = previous_device_;
 }
 
 MemoryBlock device_alloc(size_t bytes) {
@@ -185,7 +211,7 @@ MemoryBlock device_alloc(size_t bytes) {
     bytes = bucket(bytes);
     Parked b;
     if (take_parked(bytes, m.device, b)) {
-        settle(b, m.device);
+        settle(b);
         m.p = b.p;
         m.bytes = b.bytes;
         return m;
@@ -206,7 +232,7 @@ MemoryBlock device_alloc(size_t bytes) {
 void device_free(const MemoryBlock& m) {
     if (!m.p) return;
     AllocClock clock;
-    park(Parked{m.p, m.bytes, m.device, nullptr}, m.device);
+    park(Parked{m.p, m.bytes, m.device});
 }
 
 MemoryBlock pinned_alloc(size_t bytes) {
@@ -215,7 +241,7 @@ MemoryBlock pinned_alloc(size_t bytes) {
     bytes = bucket(bytes);
     Parked b;
     if (take_parked(bytes, kHost, b)) {
-        settle(b, m.device);
+        settle(b);
         m.p = b.p;
         m.bytes = b.bytes;
         return m;
@@ -227,7 +253,7 @@ MemoryBlock pinned_alloc(size_t bytes) {
 }
 
 void pinned_free(const MemoryBlock& m) {
-    if (m.p) park(Parked{m.p, m.bytes, kHost, nullptr}, m.device);
+    if (m.p) park(Parked{m.p, m.bytes, kHost});
 }
 
 cudaStream_t acquire_stream() {
