@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <future>
 #include <thread>
 #include <atomic>
@@ -31,11 +32,17 @@ struct DeviceGuard {
     }
 };
 
-// Every entry point: the engine's GPU is current, and memory it takes or gives up is used on its stream.
+// Every entry point: the engine's GPU is current, memory it takes or gives up is used on its stream, and a call that throws
+// too returns with its work done (the caller's arrays may be part of it).
 struct Entry {
     DeviceGuard guard;
     WorkStream work;
-    Entry(int device, cudaStream_t stream) : guard(device), work(stream) {}
+    cudaStream_t stream;
+    int unwinding = std::uncaught_exceptions();
+    Entry(int device, cudaStream_t stream_) : guard(device), work(stream_), stream(stream_) {}
+    ~Entry() {
+        if (std::uncaught_exceptions() > unwinding) cudaStreamSynchronize(stream);
+    }
 };
 
 __global__ void widen_u32_kernel(const uint32_t* __restrict__ in, uint64_t* __restrict__ out, size_t n) {
@@ -397,36 +404,21 @@ void Engine::load_rows(const float* src, bool src_on_device, const size_t* idx, 
         return;
     }
     const size_t rows = streamed_rows(n);
-    DeviceBuffer<float> raw[2];
-    cudaEvent_t copied[2], consumed[2];
-    for (int i = 0; i < 2; ++i) {
-        if (rotate && (i == 0 || n > rows)) raw[i].ensure(rows * d_);
-        SKM_CUDA(cudaEventCreateWithFlags(&copied[i], cudaEventDisableTiming));
-        SKM_CUDA(cudaEventCreateWithFlags(&consumed[i], cudaEventDisableTiming));
-    }
-    // what the copies write may still be in use by earlier work that was enqueued on stream_
-    SKM_CUDA(cudaEventRecord(consumed[0], stream_));
-    SKM_CUDA(cudaStreamWaitEvent(copy_stream_, consumed[0], 0));
-    size_t ci = 0, handed = 0;
-    for (size_t r0 = 0; r0 < n; r0 += rows, ++ci) {
-        const int b = static_cast<int>(ci & 1);
+    RowPipe pipe(stage_, copy_stream_, stream_);
+    if (rotate) pipe.reserve(rows * d_, n > rows ? 2 : 1);
+    size_t handed = 0;
+    for (size_t r0 = 0; r0 < n; r0 += rows) {
         const size_t cnt = std::min(rows, n - r0);
-        if (ci >= 2 && rotate) SKM_CUDA(cudaStreamWaitEvent(copy_stream_, consumed[b], 0));
-        stage_.upload(rotate ? raw[b].get() : dst + r0 * d_, idx ? src : src + r0 * d_, idx ? idx + r0 : nullptr, cnt, row_bytes, copy_stream_);
-        SKM_CUDA(cudaEventRecord(copied[b], copy_stream_));
+        const float* raw = pipe.upload(rotate ? nullptr : dst + r0 * d_, idx ? src : src + r0 * d_, idx ? idx + r0 : nullptr, cnt, row_bytes);
         if (rotate) ensure_rotation();
-        SKM_CUDA(cudaStreamWaitEvent(stream_, copied[b], 0));
-        if (rotate) launch_gemm_nt(raw[b].get(), d_, m_dev_.get(), d_, dst + r0 * d_, d_, cnt, d_, d_, stream_);
-        SKM_CUDA(cudaEventRecord(consumed[b], stream_));
+        pipe.arrive();
+        if (rotate) launch_gemm_nt(raw, d_, m_dev_.get(), d_, dst + r0 * d_, d_, cnt, d_, d_, stream_);
+        pipe.used();
         const size_t done = r0 + cnt;
         if (after_rows && (done - handed >= piece || done == n)) {
             after_rows(handed, done - handed);
             handed = done;
         }
-    }
-    for (int i = 0; i < 2; ++i) {
-        cudaEventDestroy(copied[i]);
-        cudaEventDestroy(consumed[i]);
     }
 }
 
@@ -1099,9 +1091,17 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
             if (!(p.same_points && b.x_halves_valid)) tc::launch_split_points(p.x, p.n, p.d, p.vertical_d, xs, stream);
             b.x_halves_valid = true;
             tc::launch_split_centroids(p.y, p.k, p.d, p.partial_d, p.norms_y, ys, stream);
+            // What the side stream uses is given back with events of `stream`, or is the caller's.
+            struct SideEnds {
+                cudaStream_t s = nullptr;
+                const int unwinding = std::uncaught_exceptions();
+                ~SideEnds() {
+                    if (s && std::uncaught_exceptions() > unwinding) cudaStreamSynchronize(s);
+                }
+            } side_ends;
             cudaStream_t side = nullptr;
             if (mode == 0) {
-                side = b.side.get();
+                side = side_ends.s = b.side.get();
                 b.y_split.ensure(2 * p.k * p.d);
                 b.side_start.record(stream);
                 b.side_start.hold(side);
@@ -1856,39 +1856,27 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
     if (filtered) exact_.begin(c_dev, n_centroids, d_, n, cn.get(), stream_);
     else if (!direct) launch_row_sqnorms(c_dev, n_centroids, d_, d_, cn.get(), stream_);
     const size_t rows = streamed_rows(n);
-    DeviceBuffer<float> xb[2], xn, dist;
+    DeviceBuffer<float> xn, dist;
     DeviceBuffer<uint32_t> knn;
-    cudaEvent_t copied[2], consumed[2];
-    for (int i = 0; i < 2; ++i) {
-        if (i == 0 || n > rows) xb[i].ensure(rows * d_);
-        SKM_CUDA(cudaEventCreateWithFlags(&copied[i], cudaEventDisableTiming));
-        SKM_CUDA(cudaEventCreateWithFlags(&consumed[i], cudaEventDisableTiming));
-    }
+    RowPipe pipe(stage_, copy_stream_, stream_);
+    pipe.reserve(rows * d_, n > rows ? 2 : 1);
     xn.ensure(rows);
     dist.ensure(rows);
     knn.ensure(n);
-    // what the copies write may still be in use by earlier work that was enqueued on stream_
-    SKM_CUDA(cudaEventRecord(consumed[0], stream_));
-    SKM_CUDA(cudaStreamWaitEvent(copy_stream_, consumed[0], 0));
-    size_t ci = 0;
     timers_.begin(PH_ASSIGN_FULL, stream_);
-    for (size_t r0 = 0; r0 < n; r0 += rows, ++ci) {
-        const int b = static_cast<int>(ci & 1);
+    for (size_t r0 = 0; r0 < n; r0 += rows) {
         const size_t cnt = std::min(rows, n - r0);
-        if (ci >= 2) SKM_CUDA(cudaStreamWaitEvent(copy_stream_, consumed[b], 0));
-        stage_.upload(xb[b].get(), vectors + r0 * d_, nullptr, cnt, sizeof(float) * d_, copy_stream_);
-        SKM_CUDA(cudaEventRecord(copied[b], copy_stream_));
-        SKM_CUDA(cudaStreamWaitEvent(stream_, copied[b], 0));
+        const float* xb = pipe.upload(nullptr, vectors + r0 * d_, nullptr, cnt, sizeof(float) * d_);
+        pipe.arrive();
         if (filtered) {
-            exact_.rows(xb[b].get(), r0, cnt, xn.get(), knn.get() + r0, dist.get(), stream_);
+            exact_.rows(xb, r0, cnt, xn.get(), knn.get() + r0, dist.get(), stream_);
         } else if (direct) {
-            direct_.run(xb[b].get(), c_dev, cnt, n_centroids, d_, xn.get(), cn.get(), knn.get() + r0, dist.get(), stream_);
+            direct_.run(xb, c_dev, cnt, n_centroids, d_, xn.get(), cn.get(), knn.get() + r0, dist.get(), stream_);
         } else {
-            launch_row_sqnorms(xb[b].get(), cnt, d_, d_, xn.get(), stream_);
-            launch_assign_full(xb[b].get(), c_dev, cnt, n_centroids, d_, xn.get(), cn.get(), knn.get() + r0, dist.get(), top2_.ensure(rows), stream_,
-                               y_split_.ensure(2 * n_centroids * d_));
+            launch_row_sqnorms(xb, cnt, d_, d_, xn.get(), stream_);
+            launch_assign_full(xb, c_dev, cnt, n_centroids, d_, xn.get(), cn.get(), knn.get() + r0, dist.get(), top2_.ensure(rows), stream_, y_split_.ensure(2 * n_centroids * d_));
         }
-        SKM_CUDA(cudaEventRecord(consumed[b], stream_));
+        pipe.used();
     }
     if (filtered) {
         // rows that the filter could not settle cross once more
@@ -1898,18 +1886,15 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
         const std::vector<size_t> idx(idx32.begin(), idx32.end());
         for (size_t at = 0; at < listed; at += per) {
             const size_t cnt = std::min(per, listed - at);
-            stage_.upload(xb[0].ensure(cnt * d_), vectors, idx.data() + at, cnt, sizeof(float) * d_, stream_);
-            exact_.finish(xb[0].get(), at, cnt, knn.get(), nullptr, stream_);
+            float* xl = pipe.buffer(0).ensure(cnt * d_);
+            stage_.upload(xl, vectors, idx.data() + at, cnt, sizeof(float) * d_, stream_);
+            exact_.finish(xl, at, cnt, knn.get(), nullptr, stream_);
         }
     }
     timers_.end(stream_);
     if (!direct) tell_error();
     // the answers are a d-th of the rows: fetched once, so that no copy back holds up the next upload
     stage_.download(out, knn.get(), sizeof(uint32_t) * n, stream_);
-    for (int i = 0; i < 2; ++i) {
-        cudaEventDestroy(copied[i]);
-        cudaEventDestroy(consumed[i]);
-    }
     if (!direct) check_told_error();
 }
 

@@ -2,6 +2,7 @@
 #include "host_copy.h"
 
 #include <cstring>
+#include <exception>
 
 namespace skmb {
 
@@ -97,6 +98,42 @@ void HostStage::download(void* dst, const void* src, size_t bytes, cudaStream_t 
         const size_t b = q * kPieceBytes;
         copy_bytes(static_cast<char*>(dst) + b, pieces_[i].get(), std::min(kPieceBytes, bytes - b));
     }
+}
+
+RowPipe::RowPipe(HostStage& stage, cudaStream_t copies, cudaStream_t work) : stage_(stage), copies_(copies), work_(work), unwinding_(std::uncaught_exceptions()) {}
+
+RowPipe::~RowPipe() {
+    if (std::uncaught_exceptions() > unwinding_) cudaStreamSynchronize(copies_);
+    for (cudaEvent_t e : {copied_[0], copied_[1], used_[0], used_[1]})
+        if (e) cudaEventDestroy(e);
+}
+
+void RowPipe::reserve(size_t floats, int buffers) {
+    for (int i = 0; i < buffers; ++i) buffers_[i].ensure(floats);
+}
+
+float* RowPipe::upload(float* to, const float* src, const size_t* idx, size_t n, size_t row_bytes) {
+    const int b = static_cast<int>(pieces_ & 1);
+    if (pieces_ == 0) {
+        for (cudaEvent_t* e : {&copied_[0], &copied_[1], &used_[0], &used_[1]}) SKM_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+        // what the copies write may still be in use by earlier work that was enqueued on the kernels' stream
+        SKM_CUDA(cudaEventRecord(used_[0], work_));
+        SKM_CUDA(cudaStreamWaitEvent(copies_, used_[0], 0));
+    }
+    if (!to) {
+        if (pieces_ >= 2) SKM_CUDA(cudaStreamWaitEvent(copies_, used_[b], 0));
+        to = buffers_[b].get();
+    }
+    stage_.upload(to, src, idx, n, row_bytes, copies_);
+    SKM_CUDA(cudaEventRecord(copied_[b], copies_));
+    return to;
+}
+
+void RowPipe::arrive() { SKM_CUDA(cudaStreamWaitEvent(work_, copied_[pieces_ & 1], 0)); }
+
+void RowPipe::used() {
+    SKM_CUDA(cudaEventRecord(used_[pieces_ & 1], work_));
+    ++pieces_;
 }
 
 } // namespace skmb

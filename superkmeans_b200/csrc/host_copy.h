@@ -35,4 +35,33 @@ class HostStage {
     int next_ = 0;
 };
 
+// Rows of a host matrix on their way through one or two device buffers, in turn: copies on one stream, the kernels that use the rows
+// on another.  Per piece: upload, arrive, the kernels, used.
+//
+// The buffers go back with an event of the kernels' stream, which says nothing about copies that it does not wait for yet, and a
+// pinned source is read until the last copy is done: when an exception ends the loop, the copies are waited for first.
+class RowPipe {
+  public:
+    RowPipe(HostStage& stage, cudaStream_t copies, cudaStream_t work);
+    ~RowPipe();
+    RowPipe(const RowPipe&) = delete;
+    RowPipe& operator=(const RowPipe&) = delete;
+
+    // Buffers of `floats` each, before the first upload.
+    void reserve(size_t floats, int buffers);
+    DeviceBuffer<float>& buffer(int i) { return buffers_[i]; }
+    // The next n rows (see HostStage::upload) to `to`, or to the next buffer if that is null; returns where they go.
+    float* upload(float* to, const float* src, const size_t* idx, size_t n, size_t row_bytes);
+    void arrive();   // what follows on the kernels' stream finds them there
+    void used();     // what uses them is enqueued
+
+  private:
+    HostStage& stage_;
+    cudaStream_t copies_, work_;
+    DeviceBuffer<float> buffers_[2];
+    cudaEvent_t copied_[2] = {}, used_[2] = {};
+    size_t pieces_ = 0;
+    int unwinding_;   // exceptions on their way when this was made
+};
+
 } // namespace skmb

@@ -1,0 +1,83 @@
+// Copies of host rows (host_copy.cu) when something goes wrong on the way (fake_cuda_runtime.h).
+#include <stdexcept>
+
+#include "../../superkmeans_b200/csrc/host_copy.h"
+#include "fake_cuda_runtime.h"
+
+using namespace skmb;
+
+namespace {
+
+constexpr size_t kRow = 64, kRows = 100;
+
+// An exception between a copy and the kernels that would have waited for it.
+void exception_behind_a_copy(bool pinned) {
+    const cudaStream_t copies = acquire_stream(), work = acquire_stream();
+    {
+        WorkStream on(work);
+        HostStage stage;
+        std::vector<float> rows(3 * kRows * kRow, 1.0f);
+        PinnedBuffer<float> pinned_rows;
+        const float* src = pinned ? pinned_rows.ensure(rows.size()) : rows.data();
+        const int events = fake::events_alive;
+        const float* raw = nullptr;
+        try {
+            RowPipe pipe(stage, copies, work);
+            pipe.reserve(kRows * kRow, 2);
+            for (int piece = 0; piece < 3; ++piece) {
+                raw = pipe.upload(nullptr, src + piece * kRows * kRow, nullptr, kRows, kRow * sizeof(float));
+                CHECK(fake::is_device_memory(raw) && fake::in_flight(raw, kRows * kRow * sizeof(float)));
+                if (piece == 2) throw std::runtime_error("no matrix");
+                pipe.arrive();
+                pipe.used();
+            }
+        } catch (const std::runtime_error&) {
+        }
+        // the buffers are parked now: their next owner waits for `work` only
+        CHECK(!fake::in_flight(raw, kRows * kRow * sizeof(float)));
+        CHECK(!fake::in_flight(src, rows.size() * sizeof(float)));
+        CHECK(fake::events_alive <= events + 2 + 4);   // of the two parked buffers and the stage's pieces
+    }
+    release_stream(copies, 0);
+    release_stream(work, 0);
+}
+
+// All pieces arrive in their place, from either kind of source, by index too.
+void rows_arrive() {
+    const cudaStream_t copies = acquire_stream(), work = acquire_stream();
+    {
+        WorkStream on(work);
+        HostStage stage;
+        std::vector<float> rows(7 * kRows * kRow), got(rows.size());
+        for (size_t i = 0; i < rows.size(); ++i) rows[i] = static_cast<float>(i);
+        std::vector<size_t> idx(7 * kRows);
+        for (size_t i = 0; i < idx.size(); ++i) idx[i] = idx.size() - 1 - i;
+        for (const size_t* by : {static_cast<const size_t*>(nullptr), static_cast<const size_t*>(idx.data())}) {
+            RowPipe pipe(stage, copies, work);
+            pipe.reserve(kRows * kRow, 2);
+            for (size_t r0 = 0; r0 < 7 * kRows; r0 += kRows) {
+                const float* at = pipe.upload(nullptr, by ? rows.data() : rows.data() + r0 * kRow, by ? by + r0 : nullptr, kRows, kRow * sizeof(float));
+                pipe.arrive();
+                SKM_CUDA(cudaMemcpyAsync(got.data() + r0 * kRow, at, kRows * kRow * sizeof(float), cudaMemcpyDeviceToHost, work));
+                pipe.used();
+            }
+            SKM_CUDA(cudaStreamSynchronize(work));
+            for (size_t r = 0; r < 7 * kRows; ++r)
+                for (size_t j = 0; j < kRow; ++j) CHECK(got[r * kRow + j] == rows[(by ? by[r] : r) * kRow + j]);
+        }
+    }
+    release_stream(copies, 0);
+    release_stream(work, 0);
+}
+
+} // namespace
+
+int main(int argc, char** argv) {
+    const std::string what = argc > 1 ? argv[1] : "";
+    if (what == "exception_behind_a_copy") exception_behind_a_copy(false);
+    else if (what == "exception_behind_a_pinned_copy") exception_behind_a_copy(true);
+    else if (what == "rows_arrive") rows_arrive();
+    else return 2;
+    std::puts("OK");
+    return 0;
+}
