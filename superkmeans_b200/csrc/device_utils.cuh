@@ -23,6 +23,14 @@ __device__ __forceinline__ float ordered_to_float(uint32_t o) {
     const uint32_t b = (o & 0x80000000u) ? (o & 0x7fffffffu) : ~o;
     return __uint_as_float(b);
 }
+// Ordered by distance, then by index; a NaN (of a kernel's own making, hence positive) comes last.
+__device__ __forceinline__ unsigned long long pair_key(float dist, uint32_t index) {
+    return (static_cast<unsigned long long>(float_to_ordered(dist)) << 32) | index;
+}
+__device__ __forceinline__ void store_answer(unsigned long long key, size_t row, uint32_t* __restrict__ knn, float* __restrict__ dist) {
+    knn[row] = static_cast<uint32_t>(key);
+    if (dist) dist[row] = fmaxf(0.0f, ordered_to_float(static_cast<uint32_t>(key >> 32)));
+}
 
 // One row operation of a split (host_logic.h, SplitOp) for dimension j.
 template <class Op>

@@ -21,14 +21,6 @@ constexpr size_t kQuerySmem = 48 * 1024;
 constexpr int kCell = 64;                        // rows and centroids of a tile
 constexpr int kDepth = 16;                       // columns per step
 
-__device__ __forceinline__ unsigned long long pair_key(float dist, uint32_t index) {
-    return (static_cast<unsigned long long>(float_to_ordered(dist)) << 32) | index;
-}
-__device__ __forceinline__ void store_answer(unsigned long long key, size_t row, uint32_t* __restrict__ knn, float* __restrict__ dist) {
-    knn[row] = static_cast<uint32_t>(key);
-    if (dist) dist[row] = fmaxf(0.0f, ordered_to_float(static_cast<uint32_t>(key >> 32)));
-}
-
 // Sum over the row in the order of row_sqnorms_kernel.
 template <bool VEC, class F>
 __device__ __forceinline__ void for_columns(size_t d, int lane, F f) {

@@ -554,7 +554,10 @@ __global__ void __launch_bounds__(256) gather_listed_rows_kernel(const float* __
     for (size_t j = threadIdx.x & 31; j < d; j += 32) out[i * d + j] = __ldg(src + j);
 }
 
-// The listed rows of a grouped pass: a warp computes the fp32 distances of a row to all centroids of its group.
+// The listed rows of a grouped pass, few of them: a warp computes the fp32 distances of a row to all centroids of its group.
+// With kDenseListed listed rows per tile and more this is the slower way (every row reads all centroids again), and
+// decide_listed_tiles_kernel does them.
+constexpr uint32_t kDenseListed = 32;
 __global__ void __launch_bounds__(256) decide_listed_kernel(const float* __restrict__ x, const float* __restrict__ y, size_t d, const float* __restrict__ norms_x,
                                                             const float* __restrict__ norms_y, const AssignTile* __restrict__ tiles, size_t n_tiles,
                                                             const uint32_t* __restrict__ listed, const uint32_t* __restrict__ n_listed, uint32_t* __restrict__ out_knn,
@@ -562,6 +565,7 @@ __global__ void __launch_bounds__(256) decide_listed_kernel(const float* __restr
     if (*reinterpret_cast<const volatile int*>(error) != 0) return;
     const int lane = threadIdx.x & 31;
     const uint32_t n = *n_listed;
+    if (n >= kDenseListed * n_tiles) return;
     for (uint32_t i = blockIdx.x * 8 + (threadIdx.x >> 5); i < n; i += gridDim.x * 8) {
         const uint32_t row = listed[i];
         size_t lo = 0, hi = n_tiles;   // the last tile that begins at or before the row
@@ -589,6 +593,106 @@ __global__ void __launch_bounds__(256) decide_listed_kernel(const float* __restr
             out_knn[row] = index;
             out_dist[row] = fmaxf(0.0f, best);
         }
+    }
+}
+
+// Many of them (clusters closer to each other than the rounding of the group's largest distances lets the filter see): 64 of a
+// tile's listed rows per block (blockIdx.y: which 64) against 64 centroids of the group at a time, 4 x 4 distances per
+// thread as in direct_assign.cu, bound by fp32 issue.  2.5M x 768 in 128 groups of 128 clusters, nearly all rows listed, eight
+// exact passes: 116 ms, 962 with a warp per row.
+constexpr int kListedRows = 64, kListedCols = 64, kListedDepth = 16;
+template <bool VEC>
+__global__ void __launch_bounds__(256) decide_listed_tiles_kernel(const float* __restrict__ x, const float* __restrict__ y, size_t d, const float* __restrict__ norms_x,
+                                                                  const float* __restrict__ norms_y, const AssignTile* __restrict__ tiles, size_t n_tiles,
+                                                                  const uint4* __restrict__ cand, const uint32_t* __restrict__ n_listed, uint32_t* __restrict__ out_knn,
+                                                                  float* __restrict__ out_dist, const int* __restrict__ error) {
+    __shared__ __align__(16) float sx[2][kListedDepth][kListedRows + 4], sy[2][kListedDepth][kListedCols + 4];
+    __shared__ uint32_t rows[kListedRows];
+    __shared__ uint32_t before[9];
+    if (*n_listed < kDenseListed * n_tiles || *reinterpret_cast<const volatile int*>(error) != 0) return;
+    const AssignTile tile = tiles[blockIdx.x];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // which rows: a thread per row of the tile
+    const bool mine = threadIdx.x < tile.rows && cand[tile.row0 + threadIdx.x].x == ~0u;
+    const uint32_t all = __ballot_sync(0xffffffffu, mine);
+    if (lane == 0) before[warp + 1] = __popc(all);
+    if (threadIdx.x == 0) before[0] = 0;
+    if (threadIdx.x < kListedRows) rows[threadIdx.x] = ~0u;
+    __syncthreads();
+    uint32_t rank = __popc(all & ((1u << lane) - 1u)), total = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+        if (w < warp) rank += before[w + 1];
+        total += before[w + 1];
+    }
+    const uint32_t first = blockIdx.y * kListedRows;
+    if (first >= total) return;
+    if (mine && rank >= first && rank < first + kListedRows) rows[rank - first] = tile.row0 + threadIdx.x;
+    __syncthreads();
+
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const int lr = threadIdx.x >> 2, lc = 4 * (threadIdx.x & 3);
+    const float* __restrict__ xr = rows[lr] != ~0u ? x + static_cast<size_t>(rows[lr]) * d : nullptr;
+    auto load = [&](const float* __restrict__ row, size_t j) {
+        if (!row || j >= d) return make_float4(0.f, 0.f, 0.f, 0.f);
+        if (VEC) return __ldg(reinterpret_cast<const float4*>(row + j));
+        float4 v = make_float4(__ldg(row + j), 0.f, 0.f, 0.f);
+        if (j + 1 < d) v.y = __ldg(row + j + 1);
+        if (j + 2 < d) v.z = __ldg(row + j + 2);
+        if (j + 3 < d) v.w = __ldg(row + j + 3);
+        return v;
+    };
+    float nx[4];
+    unsigned long long best[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        nx[r] = rows[ty * 4 + r] != ~0u ? norms_x[rows[ty * 4 + r]] : 0.f;
+        best[r] = ~0ull;
+    }
+    int buf = 0;
+    for (uint32_t col0 = 0; col0 < tile.k; col0 += kListedCols) {
+        const float* __restrict__ yr = col0 + lr < tile.k ? y + static_cast<size_t>(tile.y0 + col0 + lr) * d : nullptr;
+        float acc[4][4] = {};
+        float4 vx = load(xr, lc), vy = load(yr, lc);
+        for (size_t j0 = 0; j0 < d; j0 += kListedDepth, buf ^= 1) {
+            sx[buf][lc][lr] = vx.x; sx[buf][lc + 1][lr] = vx.y; sx[buf][lc + 2][lr] = vx.z; sx[buf][lc + 3][lr] = vx.w;
+            sy[buf][lc][lr] = vy.x; sy[buf][lc + 1][lr] = vy.y; sy[buf][lc + 2][lr] = vy.z; sy[buf][lc + 3][lr] = vy.w;
+            __syncthreads();
+            if (j0 + kListedDepth < d) {
+                vx = load(xr, j0 + kListedDepth + lc);
+                vy = load(yr, j0 + kListedDepth + lc);
+            }
+#pragma unroll
+            for (int q = 0; q < kListedDepth; ++q) {
+                const float4 a = *reinterpret_cast<const float4*>(&sx[buf][q][ty * 4]);
+                const float4 b = *reinterpret_cast<const float4*>(&sy[buf][q][tx * 4]);
+                const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(av[r], bv[c], acc[r][c]);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const uint32_t col = col0 + tx * 4 + c;
+            if (col >= tile.k) continue;
+            const float ny = __ldg(norms_y + tile.y0 + col);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const unsigned long long key = pair_key(fmaf(-2.0f, acc[r][c], nx[r]) + ny, tile.y0 + col);
+                best[r] = key < best[r] ? key : best[r];
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) {
+            const unsigned long long other = __shfl_xor_sync(0xffffffffu, best[r], o);
+            best[r] = other < best[r] ? other : best[r];
+        }
+        if (tx == 0 && rows[ty * 4 + r] != ~0u) store_answer(best[r], rows[ty * 4 + r], out_knn, out_dist);
     }
 }
 
@@ -724,6 +828,12 @@ void ExactAssign::assign_groups(const float* x, size_t n, const float* y, size_t
     SKM_CUDA(cudaMemsetAsync(cand_.ensure(n), 0xFF, sizeof(uint4) * n, stream));   // rows of no tile: nothing to decide
     search(x, 0, n, tiles, n_tiles, norms_x, out_knn, out_dist, stream);
     decide_listed_kernel<<<592, 256, 0, stream>>>(x, y, d_, norms_x, norms_y, tiles, n_tiles, listed_.get(), n_listed_.get(), out_knn, out_dist, error_word());
+    SKM_LAUNCH_CHECK();
+    const dim3 grid(static_cast<unsigned>(n_tiles), 256 / kListedRows);
+    if (aligned16(x, d_) && aligned16(y, d_))
+        decide_listed_tiles_kernel<true><<<grid, 256, 0, stream>>>(x, y, d_, norms_x, norms_y, tiles, n_tiles, cand_.get(), n_listed_.get(), out_knn, out_dist, error_word());
+    else
+        decide_listed_tiles_kernel<false><<<grid, 256, 0, stream>>>(x, y, d_, norms_x, norms_y, tiles, n_tiles, cand_.get(), n_listed_.get(), out_knn, out_dist, error_word());
     SKM_LAUNCH_CHECK();
 }
 

@@ -29,3 +29,51 @@ def test_shared_launches_decide_like_the_sequential_form(n, d, k, opts):
     assert np.abs(o0 - o1).max() <= 2e-2 * scale
     assert (a0 == a1).mean() >= 0.98
     assert a1.max() < k and np.isfinite(c1).all()
+
+
+def _two_levels(n, d, groups, each, spread, seed):
+    """Unit rows in `groups` groups of `each` clusters whose distances from each other are `spread` times those of the groups."""
+    rng = np.random.default_rng(seed)
+    c = np.repeat(rng.standard_normal((groups, d), dtype=np.float32), each, 0) + np.float32(spread) * rng.standard_normal((groups * each, d), dtype=np.float32)
+    x = c[rng.integers(0, groups * each, n)] + np.float32(spread / 2) * rng.standard_normal((n, d), dtype=np.float32)
+    return x / np.linalg.norm(x, axis=1, keepdims=True)
+
+
+@pytest.mark.parametrize("n,d,spread", [(20_000, 96, 0.1), (20_000, 96, 3e-2), (20_000, 96, 1e-3), (20_001, 33, 1e-3), (20_000, 260, 0.0)])
+def test_clusters_close_to_each_other(n, d, spread):
+    import superkmeans_b200 as skm
+
+    x = _two_levels(n, d, 14, 14, spread, n)
+    res = []
+    for trace in (True, False):
+        e = skm.Engine(196, d, skm.default_config(True, early_termination=0, suppress_warnings=1), hierarchical=True)
+        e.set_trace(trace)
+        c = e.train(x)
+        res.append([(s.iteration, s.objective) for s in e.stats(2)])
+        assert np.isfinite(c).all()
+    s0, s1 = res
+    assert [i for i, _ in s0] == [i for i, _ in s1]
+    # distances of unit rows by norms and products: a few roundings of 2 (|x|^2 + |c|^2) each
+    per_row = 4 * 2.0 ** -23
+    first = np.array([o for i, o in s0 if i == 1]), np.array([o for i, o in s1 if i == 1])
+    assert np.abs(first[0] - first[1]).sum() <= per_row * n + 1e-5 * first[0].sum()
+    # rows between coincident centroids fall either way, and splits follow from the sizes: alike, not equal
+    last = [sum(o for i, o in s if i == 5) for s in (s0, s1)]
+    assert abs(last[0] - last[1]) <= 0.1 * last[0] + per_row * n, last
+
+
+def test_clusters_close_to_each_other_take_no_cliff():
+    import superkmeans_b200 as skm
+
+    n, d, k = 200_000, 256, 1_600
+    times = []
+    for spread in (0.3, 1e-3):
+        x = _two_levels(n, d, 40, 40, spread, 1)
+        e = skm.Engine(k, d, skm.default_config(True, early_termination=0, suppress_warnings=1), hierarchical=True)
+        e.train(x)
+        e = skm.Engine(k, d, skm.default_config(True, early_termination=0, suppress_warnings=1), hierarchical=True)
+        e.train(x)
+        times.append(e.phase_times()["search/1st_blas"][0])
+    # every pair in fp32 on the second, one fp16 product per pair on the first; a row at a time it was 7.1 times as long
+    # here and 10 at 2.5M x 768
+    assert times[1] <= 4 * times[0], times
