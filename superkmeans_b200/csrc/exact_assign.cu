@@ -577,22 +577,15 @@ __global__ void __launch_bounds__(256) decide_listed_kernel(const float* __restr
         const AssignTile tile = tiles[lo];
         const float* xr = x + static_cast<size_t>(row) * d;
         const float nx = norms_x[row];
-        float best = FLT_MAX;
-        uint32_t index = tile.y0;
+        unsigned long long best = ~0ull;
         for (uint32_t c = tile.y0; c < tile.y0 + tile.k; ++c) {
             const float* yr = y + static_cast<size_t>(c) * d;
             float s = 0.f;
             for (size_t j = lane; j < d; j += 32) s = fmaf(__ldg(xr + j), __ldg(yr + j), s);
-            const float e = fmaf(-2.0f, warp_sum(s), nx) + norms_y[c];
-            if (e < best) {
-                best = e;
-                index = c;
-            }
+            const unsigned long long key = pair_key(fmaf(-2.0f, warp_sum(s), nx) + norms_y[c], c);
+            best = key < best ? key : best;
         }
-        if (lane == 0) {
-            out_knn[row] = index;
-            out_dist[row] = fmaxf(0.0f, best);
-        }
+        if (lane == 0) store_answer(best, row, out_knn, out_dist);
     }
 }
 

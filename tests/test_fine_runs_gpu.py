@@ -77,3 +77,23 @@ def test_clusters_close_to_each_other_take_no_cliff():
     # every pair in fp32 on the second, one fp16 product per pair on the first; a row at a time it was 7.1 times as long
     # here and 10 at 2.5M x 768
     assert times[1] <= 4 * times[0], times
+
+
+@pytest.mark.parametrize("spread", [0.3, 1e-3], ids=["few listed", "many listed"])
+@pytest.mark.parametrize("value", [np.nan, np.inf, 3e38])
+def test_a_row_without_a_distance(value, spread):
+    import superkmeans_b200 as skm
+
+    n, d, k = 20_000, 96, 196
+    x = _two_levels(n, d, 14, 14, spread, 2)
+    x[777, 5] = value
+    res = []
+    for trace in (True, False):
+        e = skm.Engine(k, d, skm.default_config(True, early_termination=0, suppress_warnings=1, seed=3), hierarchical=True)
+        e.set_trace(trace)
+        e.train(x)
+        res.append(np.array([s.objective for s in e.stats(2) if s.iteration == 1]))
+        assert e.assignments().max() < k
+    # the row counts for nothing in either form
+    assert np.isfinite(res[0]).all() == np.isfinite(res[1]).all()
+    assert (np.abs(res[0] - res[1]) <= 1e-5 * np.abs(res[0]) + 1e-3).all(), res
