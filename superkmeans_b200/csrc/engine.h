@@ -145,7 +145,7 @@ struct PrunePassBuffers {
     }
     tc::SplitHalves y_halves(size_t rows, uint32_t cols) {
         const uint32_t pitch = (cols + 7) / 8 * 8;
-        return {y_hi.ensure(rows * pitch), y_lo.ensure(rows * pitch), y_factor.ensure(1), pitch};
+        return {y_hi.ensure(rows * pitch), y_lo.ensure(rows * pitch), y_factor.ensure(rows + 1), pitch};
     }
     Side side;   // (last: its work ends before any buffer goes)
 };

@@ -4,7 +4,8 @@
 //
 // Points and centroids come as fp16 pairs v * scale = hi + lo (scale a power of two, 22 bits: what two tf32 parts hold), and
 // a product is hi*hi + hi*lo + lo*hi with fp32 accumulation: fp32-level accuracy at twice the rate of tf32.  The points are
-// split once per training, over the dimensions d' can reach, not in every tile.
+// split once per training, over the dimensions d' can reach, not in every tile, each with a scale of its own.  The centroids share
+// one while the smallest is no shorter than a thousandth of the longest, and have their own otherwise (kOneScaleSpread).
 //
 // Persistent pairs of CTAs (cta_group::2) on tiles of 256 rows x 256 centroids, as in exact_assign.cu:
 //   warp 0     TMA producer: 128 x 64 halves of each of the four parts per stage, three stages;
@@ -18,6 +19,7 @@
 // Every wait is bounded (see kernels_tc.cu).
 #include <cfloat>
 #include <cmath>
+#include <type_traits>
 
 #include "common.cuh"
 #include "device_utils.cuh"
@@ -35,11 +37,12 @@ constexpr uint32_t T_PART_BYTES = 128 * TK * 2;
 constexpr uint32_t T_STAGE_BYTES = 4 * T_PART_BYTES;   // rows hi, rows lo, centroids hi, centroids lo
 constexpr int T_TEST_WARPS = 16;
 constexpr int T_THREADS = 64 + 32 * T_TEST_WARPS;
-constexpr uint32_t T_CTRL_BYTES = 8192 + T_TEST_WARPS * 8 * 32 * 4 + 256;
+constexpr uint32_t T_CTRL_BYTES = 2 * 8192 + T_TEST_WARPS * 8 * 32 * 4 + 256;
 constexpr uint32_t T_SMEM_BYTES = T_STAGES * T_STAGE_BYTES + T_CTRL_BYTES + 1024;
 
 struct TestCtrl {
     alignas(16) float ny[4][2][256];   // per row quarter and accumulator
+    alignas(16) float fy[4][2][256];   // so the centroids' factors, where they differ
     float column[T_TEST_WARPS][8 * 32];   // per test warp: 8 values of each of its lanes
     uint32_t filled[T_TEST_WARPS];
     uint64_t full[T_STAGES];           // (the leader's are used)
@@ -55,6 +58,11 @@ __device__ __forceinline__ uint64_t pack2(float a, float b) { return static_cast
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
     uint64_t d;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
 __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
@@ -73,7 +81,7 @@ struct TestParams {
     size_t tile0, n_tiles;       // of 128 rows
     const uint32_t* tile_map;    // null: tile0, tile0 + 1, ...
     const float* factor_x;       // per row: -2 / scale
-    const float* factor_y;       // one: 1 / scale
+    const float* factor_y;       // per centroid: 1 / scale; behind them: not zero if they are all alike
     const float* norms_x;
     const float* norms_y;
     const float* best_in;
@@ -202,7 +210,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T_THREADS, 1) first_
         const uint32_t lane_base = 32u * quarter;
         float* column = ctrl->column[warp - 2] + lane;
         uint32_t* filled = &ctrl->filled[warp - 2];   // pairs in the warp's list
-        const float fy = *p.factor_y;
+        const bool one_scale = p.factor_y[p.k] != 0.f;
+        const float fy = one_scale ? p.factor_y[0] : 1.0f;
         uint32_t u = 0;
         bool ok = true;
         for (size_t t = pair; t < pair_tiles && ok; t += n_pairs) {
@@ -227,6 +236,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T_THREADS, 1) first_
                 if ((nt & 3u) == 0 && lane == 0 && listed) my_offs[nt >> 2] = *filled;
 #pragma unroll
                 for (int i = 0; i < 2; ++i) ny[i * 32 + lane] = col0 + i * 32 + lane < p.k ? __ldg(p.norms_y + col0 + i * 32 + lane) : INFINITY;   // never below a threshold
+                float* fys = ctrl->fy[quarter][b] + part * 64;
+                if (!one_scale) {
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) fys[i * 32 + lane] = col0 + i * 32 + lane < p.k ? __ldg(p.factor_y + col0 + i * 32 + lane) : 0.f;
+                }
                 __syncwarp();
                 if (!__all_sync(0xffffffffu, mbar_wait(&ctrl->acc_full[b], uph, wctx, 54))) {
                     ok = false;
@@ -235,18 +249,26 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T_THREADS, 1) first_
                 tc_fence_after();
                 const uint32_t taddr = tmem_base + (lane_base << 16) + b * 256 + part * 64;
                 const uint64_t minus_thr2 = pack2(-thr, -thr);
-                auto test = [&](uint32_t (&r)[32], int ch) {
+                auto test = [&](uint32_t (&r)[32], int ch, auto own_scales) {
                     // two columns per instruction; the sign of (distance - threshold) is the column's bit
                     uint32_t bits[4] = {0, 0, 0, 0};
 #pragma unroll
                     for (int h = 0; h < 4; ++h) {
                         const float4 n0 = *reinterpret_cast<const float4*>(ny + ch * 32 + 8 * h), n1 = *reinterpret_cast<const float4*>(ny + ch * 32 + 8 * h + 4);
                         const uint64_t nyv[4] = {pack2(n0.x, n0.y), pack2(n0.z, n0.w), pack2(n1.x, n1.y), pack2(n1.z, n1.w)};
+                        uint64_t factors[4] = {factor2, factor2, factor2, factor2};
+                        if constexpr (decltype(own_scales)::value) {
+                            const float4 f0 = *reinterpret_cast<const float4*>(fys + ch * 32 + 8 * h), f1 = *reinterpret_cast<const float4*>(fys + ch * 32 + 8 * h + 4);
+                            factors[0] = mul2(factor2, pack2(f0.x, f0.y));
+                            factors[1] = mul2(factor2, pack2(f0.z, f0.w));
+                            factors[2] = mul2(factor2, pack2(f1.x, f1.y));
+                            factors[3] = mul2(factor2, pack2(f1.z, f1.w));
+                        }
 #pragma unroll
                         for (int q = 3; q >= 0; --q) {
                             uint32_t& lo = r[8 * h + 2 * q];
                             uint32_t& hi = r[8 * h + 2 * q + 1];
-                            const uint64_t pd = add2(fma2(factor2, pack2(__uint_as_float(lo), __uint_as_float(hi)), nx2), nyv[q]);
+                            const uint64_t pd = add2(fma2(factors[q], pack2(__uint_as_float(lo), __uint_as_float(hi)), nx2), nyv[q]);
                             const uint64_t over = add2(pd, minus_thr2);
                             lo = static_cast<uint32_t>(pd);
                             hi = static_cast<uint32_t>(pd >> 32);
@@ -288,7 +310,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T_THREADS, 1) first_
                         __syncwarp();
                         if (lane == 0) mbar_arrive_cluster_read(cluster_address(&ctrl->acc_empty[b], 0));
                     }
-                    test(r, ch);
+                    if (one_scale) test(r, ch, std::false_type{});
+                    else test(r, ch, std::true_type{});
                 }
                 // Too many survivors, or on the way there: from the start of a point that keeps 10 %, the sloped line saves three
                 // quarters of the pairs that would be listed in vain.
@@ -312,13 +335,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T_THREADS, 1) first_
 }
 
 // Power of two that maps a vector of this squared norm into [-2^14, 2^14]: hi and lo then hold 22 bits of every element down
-// to 2^-17 of the norm, and smaller ones to 2^-39 of it.
+// to 2^-17 of the norm, and smaller ones to 2^-39 of it.  At most 2^74, so that the product of two factors is no less than the smallest
+// float.
 __device__ __forceinline__ float split_scale(float sqnorm) {
-    if (!(sqnorm > 1e-36f) || !(sqnorm < 3e38f)) return 1.0f;
+    if (!(sqnorm >= FLT_MIN) || !(sqnorm < 3e38f)) return 1.0f;
     int e;
     frexpf(sqrtf(sqnorm), &e);
-    return ldexpf(1.0f, 14 - e);
+    return ldexpf(1.0f, min(14 - e, 74));
 }
+
+// Largest ratio of two centroids' squared norms under one scale: a centroid 2^-10 as long as the longest still has its elements
+// to 2^-29 of its norm, all of d' <= 16 384 together to 2^-22.  (With one scale for all, a single centroid of norm 1e10 among
+// unit ones left nothing of these, and one of 1e7 a partial distance that was 1e-4 off.)  With a scale
+// per centroid nine passes over 600 000 x 1024, k = 4000, take 13.6 - 15.1 ms, with one for all 12.0.
+constexpr float kOneScaleSpread = 1048576.0f;
 
 // (rows are 16-byte aligned and a multiple of 4 long, as everywhere on the tensor-core path)
 __device__ __forceinline__ float4 leading_columns(const float* __restrict__ row, uint32_t j, uint32_t cols) {
@@ -362,23 +392,41 @@ __global__ void __launch_bounds__(256) split_points_kernel(const float* __restri
     if (lane == 0) factor[row] = -2.0f / scale;
 }
 
-// The centroids, one scale for all: every block finds the largest of the k squared norms over the columns in question.
+// The centroids: every block finds the largest and the smallest of the k squared norms over the columns in question (but for zeros and
+// what is no number, which no scale helps).
 __global__ void __launch_bounds__(256) split_centroids_kernel(const float* __restrict__ y, size_t k, size_t d, uint32_t cols, uint32_t pitch, const float* __restrict__ norms,
                                                               __half* __restrict__ hi, __half* __restrict__ lo, float* __restrict__ factor) {
-    __shared__ float part[8];
+    __shared__ float largest[8], smallest[8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float m = 0.f;
-    for (size_t c = threadIdx.x; c < k; c += 256) m = fmaxf(m, __ldg(norms + c));
+    float m = 0.f, s = FLT_MAX;
+    for (size_t c = threadIdx.x; c < k; c += 256) {
+        const float v = __ldg(norms + c);
+        m = fmaxf(m, v);
+        if (v > 0.f) s = fminf(s, v);
+    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (lane == 0) part[warp] = m;
+    for (int o = 16; o > 0; o >>= 1) {
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        s = fminf(s, __shfl_xor_sync(0xffffffffu, s, o));
+    }
+    if (lane == 0) {
+        largest[warp] = m;
+        smallest[warp] = s;
+    }
     __syncthreads();
-    m = part[0];
-    for (int w = 1; w < 8; ++w) m = fmaxf(m, part[w]);
-    const float scale = split_scale(m);
-    if (blockIdx.x == 0 && threadIdx.x == 0) *factor = 1.0f / scale;
-    for (size_t c = static_cast<size_t>(blockIdx.x) * 8 + warp; c < k; c += static_cast<size_t>(gridDim.x) * 8)
+    m = largest[0];
+    s = smallest[0];
+    for (int w = 1; w < 8; ++w) {
+        m = fmaxf(m, largest[w]);
+        s = fminf(s, smallest[w]);
+    }
+    const bool one_scale = m <= kOneScaleSpread * s || m == 0.f;
+    if (blockIdx.x == 0 && threadIdx.x == 0) factor[k] = one_scale ? 1.0f : 0.0f;
+    for (size_t c = static_cast<size_t>(blockIdx.x) * 8 + warp; c < k; c += static_cast<size_t>(gridDim.x) * 8) {
+        const float scale = split_scale(one_scale ? m : __ldg(norms + c));
         split_half_row(y + c * d, cols, pitch, scale, hi + c * pitch, lo + c * pitch, lane);
+        if (lane == 0) factor[c] = 1.0f / scale;
+    }
 }
 
 } // namespace

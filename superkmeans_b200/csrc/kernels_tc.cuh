@@ -36,7 +36,7 @@ void launch_gemm_nt(const float* a, size_t lda, const float* b, size_t ldb, floa
 void launch_rotate(const float* a, size_t lda, const float* b, float* out, size_t ldo, size_t n, size_t n_out, size_t k_dim, cudaStream_t stream);
 
 // The leading columns of a row-major fp32 matrix as fp16 pairs: element * scale = hi + lo to 22 bits, scale a power of two.
-// For points a scale per row (factor[row] = -2 / scale), for centroids one for all (factor[0] = 1 / scale).
+// For points factor[row] = -2 / scale, for centroids factor[row] = 1 / scale and, behind the last, whether they share one scale.
 struct SplitHalves {
     __half* hi;       // rows x pitch
     __half* lo;

@@ -34,3 +34,47 @@ def test_tensor_core_routes_agree_with_the_simt_search(n, d, k, lists):
         same = knn == want
         assert np.abs(dist - want_dist)[same].max() <= 1e-5 * max(1.0, float(want_dist.max()))
         assert np.abs(kept.astype(np.int64) - want_kept.astype(np.int64)).sum() <= 2 + 5e-3 * want_kept.sum()
+
+
+@pytest.mark.parametrize("lists", [4, 9], ids=["roomy", "dropping"])
+@pytest.mark.parametrize("kind", ["outlier 1e4", "outlier 1e7", "outlier 1e10", "outlier 1e18", "infinite outlier", "spread", "small", "zero"])
+def test_centroids_of_very_different_norms(kind, lists):
+    import superkmeans_b200 as skm
+
+    eng = skm.engine
+    if not eng.tensor_cores_enabled():
+        pytest.skip("tensor cores are switched off")
+    n, d, k = 6_000, 512, 700
+    rng = np.random.default_rng(len(kind))
+    x = datagen.gaussian_mixture(n, d, k // 2, 0.3, 9)
+    y = x[rng.choice(n, k, replace=False)] + np.float32(0.02) * rng.standard_normal((k, d), dtype=np.float32)
+    if kind.startswith("outlier"):
+        y[k // 3] *= np.float32(kind.split()[1])
+    elif kind == "infinite outlier":
+        y[k // 3, 7] = np.inf
+    elif kind == "spread":      # points and centroids of all sizes
+        s = (10.0 ** rng.uniform(-6, 6, (n, 1))).astype(np.float32)
+        x, y = x * s, y * (10.0 ** rng.uniform(-6, 6, (k, 1))).astype(np.float32)
+    elif kind == "small":       # squared norms at the lower end of fp32
+        x, y = x * np.float32(4e-19), y * np.float32(4e-19)
+    else:
+        y[k // 3] = 0
+    # the previous centroid: the nearest, or, for a third of the points, the one after it (further ones overflow the lists)
+    xd, yd = x.astype(np.float64), np.where(np.isfinite(y), y, np.float32(1e18)).astype(np.float64)
+    order = np.argpartition((yd ** 2).sum(1)[None, :] - 2 * xd @ yd.T, 1, axis=1)[:, :2].astype(np.uint32)
+    two = np.stack([((xd - yd[order[:, i]]) ** 2).sum(1) for i in range(2)], 1).argsort(1)
+    prev = order[np.arange(n), two[np.arange(n), (rng.random(n) < 0.33).astype(int)]]
+    for pd in (16, 100, eng.dimension_split(d)[1]):
+        try:
+            eng.set_prune_split(1)
+            want, want_dist, want_kept = eng.find_nearest_pruned(x, y, prev, pd)
+            eng.set_prune_split(lists)
+            knn, dist, kept = eng.find_nearest_pruned(x, y, prev, pd)
+        finally:
+            eng.set_prune_split(0)
+        assert (knn != want).sum() <= n // 1000, (pd, (knn != want).sum())
+        same = knn == want
+        scale = (x.astype(np.float64) ** 2).sum(1)[same] + want_dist[same]
+        # the fp32 search sums a distance by differences, the listed one recomputes it so: a rounding per sum of 64
+        assert (np.abs(dist.astype(np.float64) - want_dist)[same] <= 1e-5 * scale).all()
+        assert np.abs(kept.astype(np.int64) - want_kept.astype(np.int64)).sum() <= 2 + 5e-3 * want_kept.sum(), (pd, kept.sum(), want_kept.sum())
