@@ -205,8 +205,9 @@ int skm_get_prune_split(void);
  * bounded: when it runs out the kernel records a code, all of its roles leave their loops, tensor memory is released
  * and the kernel returns; the call that launched it then reports SKM_CUDA_ERROR and the context stays usable.  This
  * hook shortens the limit to wait_limit_cycles SM cycles (0 = back to the default of about two seconds) and makes the
- * TMA producer of the exact-assignment kernel stop after producer_stops_after_kblocks k-blocks (0 = never), so that
- * a test can watch that path without a fault or a hang.  No counterpart in the reference. */
+ * TMA producers of the exact-assignment kernels, the rotation, the first ADSampling test and the dense chain stop after
+ * producer_stops_after_kblocks stages (0 = never), so that a test can watch that path without a fault or a hang.  No
+ * counterpart in the reference. */
 skm_status skm_debug_wait_injection(uint64_t wait_limit_cycles, uint32_t producer_stops_after_kblocks);
 
 /* Profiling aid for the chain over gathered centroids (current device): SM cycles its roles spent waiting, summed over

@@ -213,6 +213,7 @@ struct FilterParams {
     uint32_t* n_listed;
     int* error;
     long long wait_limit;
+    uint32_t producer_stop;   // see set_debug_wait_injection
 };
 
 struct Best {
@@ -290,7 +291,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(F_THREADS, 1)
                     const int y_row = static_cast<int>(tile.y0 + nt * 256 + rank * 128);
                     for (uint32_t kb = 0; kb < p.k_blocks; ++kb, ++kbt) {
                         const uint32_t s = kbt % F_STAGES, ph = (kbt / F_STAGES) & 1u;
-                        if (!mbar_wait(&ctrl->empty[s], ph ^ 1u, wctx, 41)) {
+                        if ((p.producer_stop != 0 && kbt >= p.producer_stop) || !mbar_wait(&ctrl->empty[s], ph ^ 1u, wctx, 41)) {
                             ok = false;
                             break;
                         }
@@ -695,11 +696,11 @@ unsigned warps_grid(size_t rows) { return static_cast<unsigned>((rows + 7) / 8);
 } // namespace
 
 AssignRoute assign_route(size_t n, size_t k, size_t d) {
-    if (!tc::enabled() || tc::wait_injected()) return AssignRoute::blocks;
+    if (!tc::enabled()) return AssignRoute::blocks;
     const double elements = static_cast<double>(n) * static_cast<double>(d);
     const double columns = static_cast<double>((k + 255) / 256 * 256);
     auto rounds = [&](size_t rows, size_t workers) { return static_cast<double>((n + rows * workers - 1) / (rows * workers)); };
-    const double direct = direct_assign_seconds(n, k, d);
+    const double direct = tc::producer_stop() != 0 ? 1e9 : direct_assign_seconds(n, k, d);   // (a test of waits wants a kernel that waits)
     // the three-product kernel: five launches, two passes over the rows, 10 us per tile of 128 x 256 and 0.33 us per 16
     // dimensions of it
     const double blocks = d % 4 != 0 ? 1e9 : 4e-5 + elements * 8.0 / 5e12 + rounds(128, 148) * (columns / 256.0) * (1e-5 + static_cast<double>(d) / 16.0 * 3.3e-7);
@@ -772,6 +773,7 @@ void ExactAssign::search(const float* x, size_t first, size_t n, const AssignTil
     p.n_listed = n_listed_.get();
     p.error = error_word();
     p.wait_limit = wait_limit();
+    p.producer_stop = producer_stop();
     const CUtensorMap tx = make_half_tmap(xh_.get(), dp_, n, 128), ty = make_half_tmap(yh_.get(), dp_, k_, 128);
     const unsigned grid = static_cast<unsigned>(2 * std::min<size_t>(static_cast<size_t>(sms / 2), p.n_tiles));
     auto* kernel = tiles ? filter_tc_kernel<true> : filter_tc_kernel<false>;

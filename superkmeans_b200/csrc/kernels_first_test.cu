@@ -95,6 +95,7 @@ struct TestParams {
     uint32_t cap_group;
     int* error;
     long long wait_limit;
+    uint32_t producer_stop;      // see set_debug_wait_injection
 };
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T_THREADS, 1) first_test_kernel(const __grid_constant__ TestMaps maps, const TestParams p) {
@@ -146,7 +147,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T_THREADS, 1) first_
                     const int y_row = static_cast<int>(nt * 256 + rank * 128);
                     for (uint32_t kb = 0; kb < p.k_blocks; ++kb, ++kbt) {
                         const uint32_t s = kbt % T_STAGES, ph = (kbt / T_STAGES) & 1u;
-                        if (!mbar_wait(&ctrl->empty[s], ph ^ 1u, wctx, 51)) {
+                        if ((p.producer_stop != 0 && kbt >= p.producer_stop) || !mbar_wait(&ctrl->empty[s], ph ^ 1u, wctx, 51)) {
                             ok = false;
                             break;
                         }
@@ -479,6 +480,7 @@ void launch_first_test(const SplitHalves& x, const SplitHalves& y, size_t n, siz
     p.cap_group = cap_group;
     p.error = error_word();
     p.wait_limit = wait_limit();
+    p.producer_stop = producer_stop();
     SKM_CUDA(cudaFuncSetAttribute(first_test_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(T_SMEM_BYTES)));
     const unsigned grid = static_cast<unsigned>(2 * std::min<size_t>(static_cast<size_t>(sms / 2), (n_tiles + 1) / 2));
     first_test_kernel<<<grid, T_THREADS, T_SMEM_BYTES, stream>>>(maps, p);

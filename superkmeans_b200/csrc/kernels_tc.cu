@@ -410,6 +410,7 @@ struct ChainParams {
     ChainPartial* partial;             // with SLICES
     int* error;
     long long wait_limit;
+    uint32_t producer_stop;            // see set_debug_wait_injection
 };
 
 struct SegInfo {
@@ -549,7 +550,7 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1) chain_tc_kernel(const __grid
                 const int yrow = static_cast<int>(c0 + static_cast<size_t>(unit) * BN);
                 for (uint32_t kb = 0; kb < si.n_kb; ++kb, ++kbt) {
                     const uint32_t s = kbt % STAGES, ph = (kbt / STAGES) & 1u;
-                    if (!mbar_wait(&ctrl->empty[s], ph ^ 1u, wctx, 11)) {
+                    if ((p.producer_stop != 0 && kbt >= p.producer_stop) || !mbar_wait(&ctrl->empty[s], ph ^ 1u, wctx, 11)) {
                         ok = false;
                         break;
                     }
@@ -1168,7 +1169,7 @@ void set_debug_wait_injection(long long wait_limit_cycles, uint32_t producer_sto
     g_debug_producer_stop = producer_stops_after_kblocks;
 }
 
-bool wait_injected() { return g_debug_producer_stop != 0; }
+uint32_t producer_stop() { return g_debug_producer_stop; }
 
 void launch_presplit(const float* y, size_t rows, size_t ld, float* y_split, cudaStream_t stream) { presplit(y, rows, ld, y_split, stream); }
 
@@ -1368,6 +1369,7 @@ void launch_chain(const float* x, const float* y, size_t n, size_t k, size_t d, 
     p.top2 = top2_scratch;
     p.error = error_flag(device);
     p.wait_limit = g_wait_limit;
+    p.producer_stop = g_debug_producer_stop;
     const size_t row_tiles = (n + BM - 1) / BM;
     const uint32_t n_chunks = static_cast<uint32_t>((k + kChunk - 1) / kChunk);
     if (!scratch || chain_scratch_bytes(n) == 0) {

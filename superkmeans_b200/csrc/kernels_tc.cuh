@@ -117,11 +117,12 @@ void launch_chain(const float* x, const float* y, size_t n, size_t k, size_t d, 
 long long wait_limit();
 
 // Test hook for the bounded waits: every wait of the tensor-core kernels gives up after
-// wait_limit_cycles SM cycles (0 restores the default of about two seconds), and the TMA producer of the exact
-// assignment kernel stops after producer_stops_after_kblocks k-blocks (0 = never), so that the other roles wait
-// for tiles that never arrive.  The kernel then returns with an error code that fetch_error reports.
+// wait_limit_cycles SM cycles (0 restores the default of about two seconds), and the TMA producers of the exact
+// assignment kernels, the rotation, the first test with lists and the dense chain stop after producer_stops_after_kblocks stages
+// (0 = never), so that the other roles wait for tiles that never arrive.  The kernel then returns with an error code that
+// fetch_error reports.
 void set_debug_wait_injection(long long wait_limit_cycles, uint32_t producer_stops_after_kblocks);
-bool wait_injected();   // a stop is set: only the kernels of launch_assign_full honour it
+uint32_t producer_stop();   // what is set
 
 // The per-device word (device memory) in which a tensor-core kernel records that one of its waits ran out; kernels that
 // consume such a kernel's output read it first and do nothing when it is set.

@@ -56,6 +56,7 @@ struct RotParams {
     bool wide_stores;     // rows of out start on 32-byte boundaries
     int* error;
     long long wait_limit;
+    uint32_t producer_stop;   // see set_debug_wait_injection
 };
 
 struct RotCtrl {
@@ -119,7 +120,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ROT_THREADS, 1)
                 const int a_row = static_cast<int>(t / n_col_tiles * 256 + rank * 128), b_row = static_cast<int>(t % n_col_tiles * RN + rank * 128);
                 for (uint32_t k = 0; k < n_stages; ++k, ++it) {
                     const uint32_t s = it % ROT_STAGES, ph = (it / ROT_STAGES) & 1u;
-                    if (!mbar_wait(&ctrl->empty[s], ph ^ 1u, wctx, 31)) {
+                    if ((p.producer_stop != 0 && it >= p.producer_stop) || !mbar_wait(&ctrl->empty[s], ph ^ 1u, wctx, 31)) {
                         ok = false;
                         break;
                     }
@@ -278,6 +279,7 @@ void launch_rotate(const float* a, size_t lda, const float* b, float* out, size_
         p.wide_stores = ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 31) == 0;
         p.error = error_word();
         p.wait_limit = wait_limit();
+        p.producer_stop = producer_stop();
         SKM_CUDA(cudaFuncSetAttribute(rotate_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(ROT_SMEM_BYTES)));
         int sms = 0;
         SKM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
