@@ -2007,9 +2007,11 @@ void Engine::assign_training_points(const float* vectors, const float* centroids
         p.not_pruned = np.get();
         run_pruned_pass_on(p, prune_bufs_, ratios_host_[partial_d_], device_, stream_, &timers_);
     }
+    tell_error();
     if (on_device) SKM_CUDA(cudaMemcpyAsync(out, knn, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, stream_));
     else stage_.download(out, knn, sizeof(uint32_t) * n, stream_);
     sync();
+    check_told_error();
 }
 
 void Engine::get_assignments(uint32_t* out, size_t n) {
@@ -2143,6 +2145,7 @@ void Engine::op_find_nearest_pruned(int device, const float* x, const float* y, 
     ctx.download(dist_out, dist.get(), n);
     ctx.download(np_host.data(), np.get(), n);
     ctx.sync();
+    check_tc_error(ctx.stream);
     for (size_t i = 0; i < n; ++i) not_pruned_out[i] = np_host[i];
 }
 

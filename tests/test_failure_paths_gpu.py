@@ -77,6 +77,53 @@ def test_rotation(early_stop):
     np.testing.assert_array_equal(engine.rotate(m, x), want)
 
 
+@pytest.mark.parametrize("n,mode", [(4_096, 4), (4_096, 9), (2_000, 3), (30_000, 3)], ids=["first test", "first test that drops", "chain in slices", "chain"])
+def test_pruned_search(early_stop, n, mode):
+    from superkmeans_b200 import engine
+
+    d, k = 256, 1_500
+    x = datagen.gaussian_mixture(n, d, k, 0.3, 3)
+    y = x[:k].copy() if n >= k else np.concatenate([x, x])[:k].copy()
+    prev, _ = engine.find_nearest(x, y)
+    prev = np.where(np.arange(n) % 3 == 0, (prev + 1) % k, prev)
+    engine.set_prune_split(mode)
+    want = engine.find_nearest_pruned(x, y, prev, 48)
+    with early_stop, pytest.raises(RuntimeError, match="gave up waiting on a barrier"):
+        engine.find_nearest_pruned(x, y, prev, 48)
+    engine.set_prune_split(mode)
+    got = engine.find_nearest_pruned(x, y, prev, 48)
+    for a, b in zip(got, want):
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("where", ["host", "device"])
+@pytest.mark.parametrize("fraction", [1.0, 0.9])
+def test_assignment_of_training_points(early_stop, where, fraction):
+    import torch
+
+    import superkmeans_b200 as skm
+
+    n, d, k = 20_000, 256, 400
+    x = datagen.gaussian_mixture(n, d, k, 0.3, 3)
+    # rows that are rotated already: the first kernel with waits is the first test
+    e = skm.Engine(k, d, skm.default_config(False, iters=3, sampling_fraction=fraction, max_points_per_cluster=1000, early_termination=0, data_already_rotated=1))
+    c = e.train(x)
+
+    def call():
+        if where == "host":
+            return e.assign_training_points(x, c)
+        out = torch.empty(n, dtype=torch.int32, device="cuda")
+        e.assign_training_points(torch.from_numpy(x).cuda(), torch.from_numpy(c).cuda(), n=n, on_device=True, out=out)
+        return out.cpu().numpy().view(np.uint32)
+
+    with early_stop, pytest.raises(RuntimeError, match="gave up waiting on a barrier"):
+        call()
+    # the next call is about itself alone
+    a = e.assign(x, c)
+    got = call()
+    assert (got == a).mean() >= 0.995
+
+
 @pytest.mark.parametrize("hierarchical", [False, True])
 def test_training(early_stop, hierarchical):
     import superkmeans_b200 as skm
