@@ -14,6 +14,7 @@
 #include <atomic>
 #include <iostream>
 #include <numeric>
+#include <optional>
 #include <random>
 
 namespace skmb {
@@ -81,53 +82,6 @@ int resolve_device(int device) {
 }
 
 } // namespace
-
-// -------------------------------------------------------------------------------------------------
-// Phase timers
-// -------------------------------------------------------------------------------------------------
-PhaseTimers::~PhaseTimers() {
-    for (auto* list : {&pending_, &open_}) {
-        for (auto& p : *list) {
-            release_timing_event(p.a, device_);
-            release_timing_event(p.b, device_);
-        }
-    }
-}
-
-void PhaseTimers::begin(int phase, cudaStream_t s) {
-    if (device_ < 0) SKM_CUDA(cudaGetDevice(&device_));   // (the owner's, always the same)
-    Pending p{phase, acquire_timing_event(), acquire_timing_event()};
-    SKM_CUDA(cudaEventRecord(p.a, s));
-    open_.push_back(p);
-}
-
-void PhaseTimers::end(cudaStream_t s) {
-    if (open_.empty()) return;
-    Pending p = open_.back();
-    open_.pop_back();
-    cudaEventRecord(p.b, s);
-    pending_.push_back(p);
-}
-
-void PhaseTimers::flush() {
-    for (auto& p : pending_) {
-        float t = 0.f;
-        if (cudaEventElapsedTime(&t, p.a, p.b) == cudaSuccess) {
-            ms[p.phase] += t;
-            calls[p.phase] += 1;
-        }
-        release_timing_event(p.a, device_);
-        release_timing_event(p.b, device_);
-    }
-    pending_.clear();
-}
-
-void PhaseTimers::reset() {
-    for (int i = 0; i < PH_COUNT; ++i) {
-        ms[i] = 0.0;
-        calls[i] = 0;
-    }
-}
 
 // -------------------------------------------------------------------------------------------------
 // Construction (superkmeans.h:123-140, hierarchical_superkmeans.h:43-66)
@@ -1863,7 +1817,7 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
     xn.ensure(rows);
     dist.ensure(rows);
     knn.ensure(n);
-    timers_.begin(PH_ASSIGN_FULL, stream_);
+    std::optional<PhaseScope> phase(std::in_place, *this, PH_ASSIGN_FULL);
     for (size_t r0 = 0; r0 < n; r0 += rows) {
         const size_t cnt = std::min(rows, n - r0);
         const float* xb = pipe.upload(nullptr, vectors + r0 * d_, nullptr, cnt, sizeof(float) * d_);
@@ -1891,10 +1845,12 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
             exact_.finish(xl, at, cnt, knn.get(), nullptr, stream_);
         }
     }
-    timers_.end(stream_);
+    phase.reset();
     if (!direct) tell_error();
+    timers_.read_old();
     // the answers are a d-th of the rows: fetched once, so that no copy back holds up the next upload
     stage_.download(out, knn.get(), sizeof(uint32_t) * n, stream_);
+    timers_.finished();
     if (!direct) check_told_error();
 }
 

@@ -20,46 +20,9 @@
 #include "host_copy.h"
 #include "host_logic.h"
 #include "kernels_tc.cuh"
+#include "phase_timers.h"
 
 namespace skmb {
-
-// Accumulating per-phase device timers (CUDA events on the engine's stream); names follow the
-// sections of the reference's profiler (profiler.h): rotator, norms_calc, search/1st_blas, search,
-// update_centroids, consolidate, shift.
-// The last three are parts of the pruned assignment: first ADSampling test on the tensor cores, candidate-list walk, dense chain.
-// Then four spans that no kernel phase covers: device allocation and release (host wall clock), the initial centroids (Forgy
-// shuffle on the host, row gather, their rotation), the per-iteration sum across shards (device span of the collective,
-// which includes waiting for the slowest shard), and host-side work of an iteration between kernels (split decisions,
-// statistics, synchronisation).
-enum Phase { PH_ROTATE = 0, PH_NORMS, PH_ASSIGN_FULL, PH_ASSIGN_PRUNED, PH_UPDATE, PH_CONSOLIDATE, PH_SHIFT, PH_TRAIN_TOTAL, PH_PRUNE_FIRST_TEST, PH_PRUNE_WALK, PH_PRUNE_DENSE,
-             PH_ALLOC_FREE, PH_INIT_CENTROIDS, PH_ALLREDUCE, PH_HOST_OTHER, PH_COUNT };
-
-// Device time per phase, from events.  Reading them is left to whoever asks for the times: 3 us each, seven of them between two
-// iterations, were a fifth of the time that the GPU stood still there.
-class PhaseTimers {
-  public:
-    ~PhaseTimers();
-    void begin(int phase, cudaStream_t s);
-    void end(cudaStream_t s);
-    void flush();  // call only after the stream has been synchronised
-    size_t pending() const { return pending_.size(); }
-    void reset();
-    void add_host(int phase, double milliseconds) {
-        ms[phase] += milliseconds;
-        calls[phase] += 1;
-    }
-    double ms[PH_COUNT] = {};
-    uint64_t calls[PH_COUNT] = {};
-
-  private:
-    struct Pending {
-        int phase;
-        cudaEvent_t a, b;
-    };
-    int device_ = -1;
-    std::vector<Pending> pending_;
-    std::vector<Pending> open_;
-};
 
 // Device buffers of one pruned assignment pass (candidate lists, work split) and the pass itself:
 // preparation, candidate-list kernel for the cheap points, dense chain for the expensive ones.
@@ -292,8 +255,9 @@ class Engine {
     void allreduce(void* buf, size_t count, int dtype);
     void allreduce_iteration(float* sums, size_t n_sums, uint32_t* counts, size_t n_counts, double* scalars, size_t n_scalars);
     void sync() {
+        timers_.read_old();
         SKM_CUDA(cudaStreamSynchronize(stream_));
-        if (timers_.pending() > 4096) timers_.flush();
+        timers_.finished();
     }
     struct PhaseScope {
         Engine& e;

@@ -9,7 +9,7 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "superkmeans_b200", "csrc")
 CPP = os.path.join(ROOT, "tests", "cpp")
-SOURCES = {"memory_check": ["memory.cu"], "copies_check": ["memory.cu", "host_copy.cu"]}
+SOURCES = {"memory_check": ["memory.cu"], "copies_check": ["memory.cu", "host_copy.cu"], "timers_check": ["memory.cu", "phase_timers.cu"]}
 
 
 def _cuda_include():
@@ -35,7 +35,8 @@ def program(tmp_path_factory):
 
 
 @pytest.mark.parametrize("name,case", [("memory_check", "events_between_devices"), ("memory_check", "record_that_fails"),
-                                       ("copies_check", "exception_behind_a_copy"), ("copies_check", "exception_behind_a_pinned_copy"), ("copies_check", "rows_arrive")])
+                                       ("copies_check", "exception_behind_a_copy"), ("copies_check", "exception_behind_a_pinned_copy"), ("copies_check", "rows_arrive"),
+                                       ("timers_check", "many_calls"), ("timers_check", "nothing_unfinished_is_read")])
 def test_with_a_runtime_of_host_code(program, name, case):
     res = subprocess.run([program(name), case], capture_output=True, text=True, timeout=120)
     assert res.returncode == 0 and "OK" in res.stdout, res.stdout + res.stderr
