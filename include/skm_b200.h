@@ -210,6 +210,10 @@ int skm_get_prune_split(void);
  * counterpart in the reference. */
 skm_status skm_debug_wait_injection(uint64_t wait_limit_cycles, uint32_t producer_stops_after_kblocks);
 
+/* Test hook: device (or pinned host) allocations of between least_bytes and most_bytes fail as if there were no memory for
+ * them; most_bytes < least_bytes: none do.  No counterpart in the reference. */
+void skm_debug_alloc_failures(uint64_t least_bytes, uint64_t most_bytes, int pinned);
+
 /* Profiling aid for the chain over gathered centroids (current device): SM cycles its roles spent waiting, summed over
  * the CTAs of all launches since the last call, then cleared.  out16: [0] MMA thread waiting for the rows to hand an
  * accumulator back, [1] waiting for a stage, [2] its whole loop; [3] a row warp waiting for an accumulator, [4] fetching

@@ -17,6 +17,12 @@ struct CudaError : std::runtime_error {
     using std::runtime_error::runtime_error;
 };
 
+// Device or pinned memory that is not to be had, not even after everything parked has been given back: where there is a way that
+// needs less, it is taken.
+struct OutOfMemory : CudaError {
+    using CudaError::CudaError;
+};
+
 inline void cuda_check(cudaError_t e, const char* what, const char* file, int line) {
     if (e != cudaSuccess) {
         throw CudaError(std::string(what) + ": " + cudaGetErrorString(e) + " (" + file + ":" + std::to_string(line) + ")");
@@ -43,6 +49,8 @@ MemoryBlock device_alloc(size_t bytes);
 void device_free(const MemoryBlock& m);
 MemoryBlock pinned_alloc(size_t bytes);
 void pinned_free(const MemoryBlock& m);
+// Test hook: requests for between `least` and `most` bytes fail as if there were no memory for them (most < least: none).
+void set_debug_alloc_failures(size_t least, size_t most, bool pinned);
 // A non-blocking stream of the current device; release_stream waits for the work on it.
 cudaStream_t acquire_stream();
 void release_stream(cudaStream_t s, int device);

@@ -159,14 +159,24 @@ void Engine::wait_for_default_stream() {
 // The draws of a matrix that is being made.
 struct Engine::Drawing {
     NormalDraws draws;
-    PinnedBuffer<uint32_t> bits;
+    // Only the host reads the bits.  Pinned memory that is parked spares the few thousand page faults of a new array (0.2 ms of a Train of
+    // 100 000 x 768), but what is too large to be parked with the draws need not be pinned.
+    static constexpr size_t kPinnedBits = size_t{64} << 20;
+    PinnedBuffer<uint32_t> parked_bits;
+    std::unique_ptr<uint32_t[]> own_bits;
+    uint32_t* bits;
     PinnedBuffer<float> values;
     std::future<void> drawn;   // (the last member: waits for its thread before the others go)
     Drawing(size_t count, uint32_t seed) : draws(count, seed) {
-        bits.ensure(draws.scratch());
+        if (draws.scratch() * sizeof(uint32_t) <= kPinnedBits) {
+            bits = parked_bits.ensure(draws.scratch());
+        } else {
+            own_bits.reset(new uint32_t[draws.scratch()]);
+            bits = own_bits.get();
+        }
         draws.values_at(values.ensure(draws.scratch()));
-        if (draws.threads() > 1) drawn = std::async(std::launch::async, [this] { draws.make(bits.get(), values.get()); });
-        else draws.make(bits.get(), values.get());
+        if (draws.threads() > 1) drawn = std::async(std::launch::async, [this] { draws.make(bits, values.get()); });
+        else draws.make(bits, values.get());
     }
 };
 
@@ -174,7 +184,12 @@ struct Engine::Drawing {
 // staged, its two hundred dependent launches too (two more), on a thread and a stream of their own beside that.
 void Engine::start_rotation(bool beside) {
     if (rotation_ready_ || drawing_ || !rotation_host_.empty()) return;
-    drawing_ = std::make_unique<Drawing>(d_ * d_, cfg_.seed);
+    try {
+        drawing_ = std::make_unique<Drawing>(d_ * d_, cfg_.seed);
+    } catch (const OutOfMemory&) {
+        rotation_host_ = make_rotation_matrix(d_, cfg_.seed);   // (in ordinary memory; seconds from d = 2000 on)
+        return;
+    }
     if (!beside) return;
     if (!rotation_event_) SKM_CUDA(cudaEventCreateWithFlags(&rotation_event_, cudaEventDisableTiming));
     rotation_state_.store(RotationState::none);

@@ -48,6 +48,12 @@ constexpr size_t kMaxIdleEvents = 1024;   // that measure time, per device
 
 enum class CacheMode { bounded, everything, nothing };
 
+struct FailingSizes {
+    std::atomic<size_t> least{1}, most{0};
+    bool hit(size_t bytes) const { return bytes >= least.load(std::memory_order_relaxed) && bytes <= most.load(std::memory_order_relaxed); }
+};
+FailingSizes g_fail_device, g_fail_pinned;
+
 std::mutex g_mu;
 std::vector<Parked> g_parked;   // oldest first
 CacheMode g_mode = CacheMode::bounded;
@@ -204,29 +210,50 @@ WorkStream::~WorkStream() {
     t_device = previous_device_;
 }
 
-MemoryBlock device_alloc(size_t bytes) {
-    AllocClock clock;
+namespace {
+
+// A parked block, or a new one from ALLOC.
+template <class Alloc>
+MemoryBlock take_or_make(size_t bytes, bool pinned, const char* what, Alloc alloc) {
     MemoryBlock m;
     SKM_CUDA(cudaGetDevice(&m.device));
+    const bool fails = (pinned ? g_fail_pinned : g_fail_device).hit(bytes);
     bytes = bucket(bytes);
     Parked b;
-    if (take_parked(bytes, m.device, b)) {
+    if (!fails && take_parked(bytes, pinned ? kHost : m.device, b)) {
         settle(b);
         m.p = b.p;
         m.bytes = b.bytes;
         return m;
     }
     note_device_alloc();
-    cudaError_t e = cudaMalloc(&m.p, bytes);
-    if (e == cudaErrorMemoryAllocation) {
+    cudaError_t e = fails ? cudaErrorMemoryAllocation : alloc(&m.p, bytes);
+    if (e == cudaErrorMemoryAllocation && !fails) {
         // what is parked may be exactly what is missing
         cudaGetLastError();
         give_back_all(take_all_parked());
-        e = cudaMalloc(&m.p, bytes);
+        e = alloc(&m.p, bytes);
     }
-    cuda_check(e, "cudaMalloc", __FILE__, __LINE__);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();   // (the caller may know a way that needs less)
+        throw OutOfMemory(std::string(what) + ": " + cudaGetErrorString(e) + " (" + std::to_string(bytes) + " bytes)");
+    }
+    cuda_check(e, what, __FILE__, __LINE__);
     m.bytes = bytes;
     return m;
+}
+
+} // namespace
+
+void set_debug_alloc_failures(size_t least, size_t most, bool pinned) {
+    FailingSizes& f = pinned ? g_fail_pinned : g_fail_device;
+    f.least = least;
+    f.most = most;
+}
+
+MemoryBlock device_alloc(size_t bytes) {
+    AllocClock clock;
+    return take_or_make(bytes, false, "cudaMalloc", [](void** p, size_t n) { return cudaMalloc(p, n); });
 }
 
 void device_free(const MemoryBlock& m) {
@@ -236,20 +263,7 @@ void device_free(const MemoryBlock& m) {
 }
 
 MemoryBlock pinned_alloc(size_t bytes) {
-    MemoryBlock m;
-    SKM_CUDA(cudaGetDevice(&m.device));
-    bytes = bucket(bytes);
-    Parked b;
-    if (take_parked(bytes, kHost, b)) {
-        settle(b);
-        m.p = b.p;
-        m.bytes = b.bytes;
-        return m;
-    }
-    note_device_alloc();
-    SKM_CUDA(cudaHostAlloc(&m.p, bytes, cudaHostAllocPortable));
-    m.bytes = bytes;
-    return m;
+    return take_or_make(bytes, true, "cudaHostAlloc", [](void** p, size_t n) { return cudaHostAlloc(p, n, cudaHostAllocPortable); });
 }
 
 void pinned_free(const MemoryBlock& m) {

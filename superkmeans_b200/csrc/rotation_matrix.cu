@@ -19,7 +19,8 @@
 // 1.2 ms, of which 0.25 ms are the solve of step 1 (0.88 with one batch of loads in flight instead of four; d = 1536: 2.5 - 3.0 ms
 // before) and 0.75 ms (d = 1536: 1.9) the two chains of d / 32 dependent launches.
 //
-// A matrix too close to singular for this (or too wide for step 1's row buffer) is declined: the caller takes the host's.
+// A matrix too close to singular for this (or too wide for step 1's row buffer, or for the memory that is left: the scratch is 32 bytes
+// an element) is declined: the caller takes the host's.
 #include <cmath>
 #include <cstring>
 
@@ -403,7 +404,7 @@ void launch_collect_draws(const DrawPieces& p, float* out, cudaStream_t stream) 
     SKM_LAUNCH_CHECK();
 }
 
-bool make_rotation_matrix_on_device(const float* draws, size_t d, float* out, cudaStream_t stream) {
+static bool factorise_on_device(const float* draws, size_t d, float* out, cudaStream_t stream) {
     const size_t dp = (d + GT - 1) / GT * GT;
     // rows per block of the solve: as many as the row buffer holds, but no more than leave a block for most SMs
     int rows = kSolveMaxRows;
@@ -464,6 +465,14 @@ bool make_rotation_matrix_on_device(const float* draws, size_t d, float* out, cu
     signed_columns_kernel<<<dim3(static_cast<unsigned>((d + 255) / 256), static_cast<unsigned>(d)), 256, 0, stream>>>(cur, signs, d, dp, out);
     SKM_LAUNCH_CHECK();
     return true;
+}
+
+bool make_rotation_matrix_on_device(const float* draws, size_t d, float* out, cudaStream_t stream) {
+    try {
+        return factorise_on_device(draws, d, out, stream);
+    } catch (const OutOfMemory&) {
+        return false;
+    }
 }
 
 } // namespace skmb

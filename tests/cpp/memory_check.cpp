@@ -56,12 +56,43 @@ void record_that_fails() {
     CHECK(fake::device_in_use == 0 && fake::pinned_in_use == 0);
 }
 
+// What is parked is given back before an allocation counts as failed, of pinned memory too, and the failure leaves no error behind.
+template <class B>
+void memory_that_is_short(size_t& limit, size_t& in_use) {
+    limit = size_t{1} << 20;
+    cudaSetDevice(0);
+    const cudaStream_t s = acquire_stream();
+    {
+        WorkStream work(s);
+        {
+            B b;
+            b.ensure(900'000);
+        }
+        CHECK(in_use >= 900'000);
+        B b;
+        b.ensure(300'000);   // fits only once the other is gone
+        B more;
+        bool failed = false;
+        try {
+            more.ensure(900'000);
+        } catch (const OutOfMemory&) {
+            failed = true;
+        }
+        CHECK(failed && cudaGetLastError() == cudaSuccess);
+        more.ensure(100'000);
+        b.ensure(200'000);
+    }
+    release_stream(s, 0);
+}
+
 } // namespace
 
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "events_between_devices") events_between_devices();
     else if (what == "record_that_fails") record_that_fails();
+    else if (what == "device_memory_that_is_short") memory_that_is_short<DeviceBuffer<char>>(fake::device_limit, fake::device_in_use);
+    else if (what == "pinned_memory_that_is_short") memory_that_is_short<PinnedBuffer<char>>(fake::pinned_limit, fake::pinned_in_use);
     else return 2;
     std::puts("OK");
     return 0;

@@ -1,0 +1,35 @@
+"""Steps that need more memory than the way they replaced take that way when the memory is not there (a test hook makes the
+allocations of some sizes fail)."""
+import contextlib
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@contextlib.contextmanager
+def without(least, most=None, pinned=False):
+    from superkmeans_b200 import _lib
+
+    _lib.lib.skm_debug_alloc_failures(least, least if most is None else most, int(pinned))
+    try:
+        yield
+    finally:
+        _lib.lib.skm_debug_alloc_failures(1, 0, int(pinned))
+
+
+@pytest.mark.parametrize("beside", [False, True], ids=["asked for", "beside a training"])
+@pytest.mark.parametrize("pinned", [False, True])
+def test_rotation_matrix(pinned, beside):
+    import superkmeans_b200 as skm
+
+    d, n = 500, 400
+    # the scratch has four matrices of 512 x 512 doubles, the draws on the host at least d x d floats of pinned memory
+    with without(*((4 * d * d, 1 << 40, True) if pinned else (8 * 512 * 512, 8 * 512 * 512, False))):
+        e = skm.Engine(4, d, skm.default_config(False, sampling_fraction=1.0, iters=2))
+        if beside:
+            x = np.random.default_rng(0).standard_normal((n, d), dtype=np.float32)
+            assert np.isfinite(e.train(x)).all()
+        m = e.get_rotation()
+    np.testing.assert_array_equal(m, skm.engine.rotation_matrix(d, 42))
