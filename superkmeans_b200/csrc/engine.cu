@@ -1056,7 +1056,17 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
             uint2* lists = b.tc_lists.ensure(per_batch * kListsPerTile * cap_group);
             uint32_t* offs = b.tc_list_offs.ensure(per_batch * kListsPerTile * (n_chunks + 1));
             // d' moves below vertical_d from pass to pass: the points are split that far, once
-            const tc::SplitHalves xs = b.x_halves(p.n, p.vertical_d), ys = b.y_halves(p.k, p.partial_d);
+            tc::SplitHalves xs{};
+            try {
+                xs = b.x_halves(p.n, p.vertical_d);
+            } catch (const OutOfMemory&) {
+                // The ordered route splits a batch of rows at a time, in place of a quarter of all of them.
+                b.give_up_lists();
+                if (mode != 0) throw;
+                run_pruned_pass_sorted(p, b, ratio_first, device, stream, timers, 10);
+                return;
+            }
+            const tc::SplitHalves ys = b.y_halves(p.k, p.partial_d);
             if (!(p.same_points && b.x_halves_valid)) tc::launch_split_points(p.x, p.n, p.d, p.vertical_d, xs, stream);
             b.x_halves_valid = true;
             tc::launch_split_centroids(p.y, p.k, p.d, p.partial_d, p.norms_y, ys, stream);

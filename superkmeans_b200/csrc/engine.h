@@ -69,6 +69,14 @@ struct PrunePassBuffers {
     DeviceBuffer<__half> x_hi, x_lo, y_hi, y_lo;
     DeviceBuffer<float> x_factor, y_factor;
     bool x_halves_valid = false;
+    // The memory of the list route over all points, for the ordered one.
+    void give_up_lists() {
+        x_hi.release();
+        x_lo.release();
+        tc_lists.release();
+        tc_list_offs.release();
+        x_halves_valid = false;
+    }
     // a second stream, and the places where the two meet
     struct Mark {
         cudaEvent_t event = nullptr;

@@ -5,6 +5,8 @@ import contextlib
 import numpy as np
 import pytest
 
+from tests import datagen
+
 pytestmark = pytest.mark.gpu
 
 
@@ -33,3 +35,23 @@ def test_rotation_matrix(pinned, beside):
             assert np.isfinite(e.train(x)).all()
         m = e.get_rotation()
     np.testing.assert_array_equal(m, skm.engine.rotation_matrix(d, 42))
+
+
+def test_list_route():
+    import superkmeans_b200 as skm
+
+    n, d, k = 20_000, 256, 400
+    vertical = skm.engine.dimension_split(d)[1]
+    x = datagen.gaussian_mixture(n, d, k, 0.3, 4)
+
+    def train():
+        e = skm.Engine(k, d, skm.default_config(False, sampling_fraction=1.0, iters=5, early_termination=0))
+        e.train(x)
+        return e.assignments(), e.last_prune_path
+
+    want, path = train()
+    assert path == 4
+    with without(2 * n * vertical):   # a half of all points' leading columns
+        got, path = train()
+    assert path == 6
+    assert (got == want).mean() >= 0.999
