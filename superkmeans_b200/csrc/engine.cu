@@ -401,8 +401,7 @@ size_t Engine::streamed_rows(size_t n) const {
 // Exact assignment of device rows: knn, dist, and the full norms of both sides.
 void Engine::exact_assignment(const float* x, size_t n, const float* c, size_t k, float* norms_x, bool norms_known, float* norms_c, uint32_t* knn, float* dist) {
     const AssignRoute route = assign_route(n, k, d_);
-    if (route == AssignRoute::filter) {
-        exact_.begin(c, k, d_, n, norms_c, stream_);
+    if (route == AssignRoute::filter && exact_.begin(c, k, d_, n, n, norms_c, stream_)) {
         exact_.rows(x, 0, n, norms_x, knn, dist, stream_);
         exact_.settle_on_device(x, knn, dist, stream_);
         return;
@@ -1464,8 +1463,8 @@ void Engine::train_flat(const float* data, size_t n, bool on_device, const float
                     float* norms = data_norms_.get() + r0;
                     if (!centroids_ready) {
                         make_centroids();
-                        if (exact_open_) exact_.begin(c_prev_.get(), k_, d_, n_samples_, centroid_norms_.get(), stream_);
-                        else launch_row_sqnorms(c_prev_.get(), k_, d_, d_, centroid_norms_.get(), stream_);
+                        if (exact_open_) exact_open_ = exact_.begin(c_prev_.get(), k_, d_, n_samples_, n_samples_, centroid_norms_.get(), stream_);
+                        if (!exact_open_) launch_row_sqnorms(c_prev_.get(), k_, d_, d_, centroid_norms_.get(), stream_);
                     }
                     if (exact_open_) {
                         exact_.rows(x, r0, cnt, norms, assignments_.get() + r0, distances_.get() + r0, stream_);
@@ -1831,10 +1830,9 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
         return;
     }
     const AssignRoute route = assign_route(n, n_centroids, d_);
-    const bool filtered = route == AssignRoute::filter, direct = route == AssignRoute::direct;
-    if (filtered) exact_.begin(c_dev, n_centroids, d_, n, cn.get(), stream_);
-    else if (!direct) launch_row_sqnorms(c_dev, n_centroids, d_, d_, cn.get(), stream_);
     const size_t rows = streamed_rows(n);
+    const bool filtered = route == AssignRoute::filter && exact_.begin(c_dev, n_centroids, d_, n, rows, cn.get(), stream_), direct = route == AssignRoute::direct;
+    if (!filtered && !direct) launch_row_sqnorms(c_dev, n_centroids, d_, d_, cn.get(), stream_);
     DeviceBuffer<float> xn, dist;
     DeviceBuffer<uint32_t> knn;
     RowPipe pipe(stage_, copy_stream_, stream_);
@@ -1859,7 +1857,7 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
     }
     if (filtered) {
         // rows that the filter could not settle cross once more
-        const size_t listed = exact_.settle(stream_), per = exact_.slice_rows();
+        const size_t listed = exact_.settle(stream_), per = rows;
         std::vector<uint32_t> idx32(listed);
         stage_.download(idx32.data(), exact_.listed(), sizeof(uint32_t) * listed, stream_);
         const std::vector<size_t> idx(idx32.begin(), idx32.end());
@@ -2065,8 +2063,7 @@ void Engine::op_find_nearest(int device, const float* x, const float* y, size_t 
     ExactAssign exact;
     DirectAssign direct;
     const AssignRoute route = assign_route(n, k, d);
-    if (route == AssignRoute::filter) {
-        exact.begin(yd.get(), k, d, n, ny.ensure(k), ctx.stream);
+    if (route == AssignRoute::filter && exact.begin(yd.get(), k, d, n, n, ny.ensure(k), ctx.stream)) {
         exact.rows(xd.get(), 0, n, nx.ensure(n), knn.ensure(n), dist.ensure(n), ctx.stream);
         exact.settle_on_device(xd.get(), knn.get(), dist.get(), ctx.stream);
     } else if (route == AssignRoute::direct) {

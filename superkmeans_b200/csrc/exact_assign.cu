@@ -785,17 +785,40 @@ void ExactAssign::search(const float* x, size_t first, size_t n, const AssignTil
     SKM_LAUNCH_CHECK();
 }
 
-void ExactAssign::begin(const float* y, size_t k, size_t d, size_t batch_rows, float* norms_y, cudaStream_t stream) {
-    listed_.ensure(batch_rows);
+// A gigabyte of fp16 rows, in whole waves of row tiles.
+size_t ExactAssign::rows_at_once(size_t n) const {
+    const size_t wave = 74 * 256;
+    return std::min(n, std::max(wave, ((size_t{1} << 30) / (dp_ * sizeof(__half))) / wave * wave));
+}
+
+void ExactAssign::give_back() {
+    xh_.release();
+    yh_.release();
+    row_info_.release();
+    cand_.release();
+    listed_.release();
+}
+
+bool ExactAssign::begin(const float* y, size_t k, size_t d, size_t batch_rows, size_t piece_rows, float* norms_y, cudaStream_t stream) {
     d_ = d;
     dp_ = (d + 7) / 8 * 8;
+    try {
+        listed_.ensure(batch_rows);
+        const size_t per = rows_at_once(piece_rows);
+        xh_.ensure(per * dp_);
+        row_info_.ensure(per);
+        cand_.ensure(per);
+        yh_.ensure(k * dp_);
+    } catch (const OutOfMemory&) {
+        give_back();
+        return false;
+    }
     centroids(y, k, norms_y, true, stream);
+    return true;
 }
 
 void ExactAssign::rows(const float* x, size_t first, size_t n, float* norms_x, uint32_t* out_knn, float* out_dist, cudaStream_t stream) {
-    // a gigabyte of fp16 rows at a time, in whole waves of row tiles
-    const size_t wave = 74 * 256;
-    const size_t per = std::min(n, std::max(wave, ((size_t{1} << 30) / (dp_ * sizeof(__half))) / wave * wave));
+    const size_t per = rows_at_once(n);
     xh_.ensure(per * dp_);
     row_info_.ensure(per);
     for (size_t r0 = 0; r0 < n; r0 += per) {
@@ -857,10 +880,18 @@ void ExactAssign::finish(const float* x_listed, size_t at, size_t count, uint32_
 
 size_t ExactAssign::settle_on_device(const float* x_batch, uint32_t* out_knn, float* out_dist, cudaStream_t stream) {
     const size_t total = settle(stream);
-    const size_t per = slice_rows();
-    for (size_t at = 0; at < total; at += per) {
-        const size_t count = std::min(per, total - at);
-        float* xl = l_rows_.ensure(count * d_);
+    size_t per = std::max<size_t>(1, (size_t{1} << 30) / (sizeof(float) * d_)), count;   // (a gigabyte)
+    for (size_t at = 0; at < total; at += count) {
+        count = std::min(per, total - at);
+        float* xl = nullptr;
+        try {
+            xl = l_rows_.ensure(count * d_);
+        } catch (const OutOfMemory&) {
+            if (count <= 1024) throw;
+            per = count / 8;   // (smaller steps then)
+            count = 0;
+            continue;
+        }
         gather_listed_rows_kernel<<<warps_grid(count), 256, 0, stream>>>(x_batch, listed_.get() + at, count, d_, xl);
         SKM_LAUNCH_CHECK();
         finish(xl, at, count, out_knn, out_dist, stream);

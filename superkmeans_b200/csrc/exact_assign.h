@@ -42,16 +42,16 @@ struct AssignTile {
 class ExactAssign {
   public:
     // Once per set of centroids and batch of rows: fp16 centroids, their squared norms (also to norms_y, as
-    // launch_row_sqnorms gives them), an empty list.
-    void begin(const float* y, size_t k, size_t d, size_t batch_rows, float* norms_y, cudaStream_t stream);
+    // launch_row_sqnorms gives them), an empty list, and memory for up to piece_rows rows at a time.  False: there is not enough
+    // of it (the fp16 rows take a gigabyte at most), nothing has been done and none is held.
+    bool begin(const float* y, size_t k, size_t d, size_t batch_rows, size_t piece_rows, float* norms_y, cudaStream_t stream);
     // Rows [first, first + n) of the batch; their squared norms go to norms_x (as launch_row_sqnorms gives them).
     void rows(const float* x, size_t first, size_t n, float* norms_x, uint32_t* out_knn, float* out_dist, cudaStream_t stream);
     // Number of listed rows (waits for the stream); their indices inside the batch are in listed().
     size_t settle(cudaStream_t stream);
     const uint32_t* listed() const { return listed_.get(); }
-    // out_knn / out_dist (may be null) of the rows listed()[at .. at + count), given those rows; a gigabyte at most at a time.
+    // out_knn / out_dist (may be null) of the rows listed()[at .. at + count), given those rows.
     void finish(const float* x_listed, size_t at, size_t count, uint32_t* out_knn, float* out_dist, cudaStream_t stream);
-    size_t slice_rows() const { return std::max<size_t>(1, (size_t{1} << 30) / (sizeof(float) * d_)); }
     // Both, for a batch that is still on the device.
     size_t settle_on_device(const float* x_batch, uint32_t* out_knn, float* out_dist, cudaStream_t stream);
 
@@ -66,6 +66,8 @@ class ExactAssign {
     void centroids(const float* y, size_t k, float* norms_y, bool with_mean, cudaStream_t stream);
     void convert(const float* x, size_t n, float* norms_x, cudaStream_t stream);
     void search(const float* x, size_t first, size_t n, const AssignTile* tiles, size_t n_tiles, const float* norms_x, uint32_t* out_knn, float* out_dist, cudaStream_t stream);
+    size_t rows_at_once(size_t n) const;
+    void give_back();
     const float* y_ = nullptr;
     const float* norms_y_ = nullptr;
     size_t k_ = 0, d_ = 0, dp_ = 0, kp_ = 0;

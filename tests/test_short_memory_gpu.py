@@ -55,3 +55,34 @@ def test_list_route():
         got, path = train()
     assert path == 6
     assert (got == want).mean() >= 0.999
+
+
+def test_exact_assignment():
+    import torch
+
+    import superkmeans_b200 as skm
+
+    n, d, k = 20_000, 96, 2_000
+    x = datagen.gaussian_mixture(n, d, k, 0.3, 4)
+    c = x[:k].copy()
+    xd, cd, out = torch.from_numpy(x).cuda(), torch.from_numpy(c).cuda(), torch.empty(n, dtype=torch.int32, device="cuda")
+
+    def answers():
+        e = skm.Engine(k, d)
+        e.assign(xd, cd, n=n, on_device=True, out=out)
+        t = skm.Engine(k, d, skm.default_config(False, sampling_fraction=1.0, iters=1, early_termination=0))
+        t.train(x)
+        return [skm.engine.find_nearest(x, c)[0], e.assign(x, c), out.cpu().numpy().view(np.uint32), t.assignments()]
+
+    want = answers()
+    launches = skm.engine.kernel_launches()
+    with without(2 * n * d):   # the fp16 rows of the filter
+        got = answers()
+    assert skm.engine.kernel_launches() > launches
+    for a, b in zip(want, got):
+        assert (a != b).sum() <= 2   # rows at the same distance from two centroids
+    # a third of the rows has more equally near centroids than the filter keeps and is decided, slice after slice
+    x[::3], c[k // 2:] = x[0], x[0]
+    want = skm.engine.find_nearest(x, c)[0]
+    with without(12 * n * d // 10, 15 * n * d // 10):
+        np.testing.assert_array_equal(skm.engine.find_nearest(x, c)[0], want)
