@@ -1693,7 +1693,8 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
     for (size_t m = 0; m < n_meso_; ++m) rows_of[m] = std::min<size_t>(meso_sizes[m], n_all - std::min(offsets[m], n_all));
     auto gemm_only = [&](size_t n_fine) { return d_ < kDimensionThresholdForPruning || cfg_.use_blas_only || n_fine <= kNClustersThresholdForPruning; };
     // Mesoclusters that never prune share their launches (train_fine_run); snapshots are per mesocluster and iteration.
-    auto shares = [&](size_t m) { return fine_nums[m] > 0 && rows_of[m] >= fine_nums[m] && gemm_only(fine_nums[m]) && !trace_on_ && tc::enabled() && d_ <= 16384; };
+    bool room = true;   // for the rows of many
+    auto shares = [&](size_t m) { return room && fine_nums[m] > 0 && rows_of[m] >= fine_nums[m] && gemm_only(fine_nums[m]) && !trace_on_ && tc::enabled() && d_ <= 16384; };
     const size_t run_rows = (size_t{4} << 30) / (sizeof(float) * d_);   // of a run, unless one mesocluster has more
     // The Forgy rows of every mesocluster (a shuffle of its member positions each) are drawn ahead by host threads.
     std::vector<std::vector<size_t>> forgy(n_meso_);
@@ -1731,10 +1732,17 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
             }
             for (size_t f = m; f < last; ++f) wait_for_forgy(f);
             partial_d_ = initial_pd;
-            train_fine_run(m, last, offsets, rows_of, fine_nums, forgy, fine_offset);
-            fine_offset += clusters;
-            m = last - 1;
-            continue;
+            try {
+                train_fine_run(m, last, offsets, rows_of, fine_nums, forgy, fine_offset);
+                fine_offset += clusters;
+                m = last - 1;
+                continue;
+            } catch (const OutOfMemory&) {
+                // (nothing of the run has been kept: it starts over, one mesocluster after the other)
+                room = false;
+                meso_buffer_.release();
+                exact_.give_back();
+            }
         }
         partial_d_ = initial_pd;
         const size_t msize = rows_of[m];

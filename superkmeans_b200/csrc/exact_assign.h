@@ -61,13 +61,13 @@ class ExactAssign {
     void begin_groups(const float* x, size_t n, size_t d, const float* y, size_t k, float* norms_x, cudaStream_t stream);
     void assign_groups(const float* x, size_t n, const float* y, size_t k, const AssignTile* tiles, size_t n_tiles, const float* norms_x, float* norms_y, uint32_t* out_knn,
                        float* out_dist, cudaStream_t stream);
+    void give_back();   // the memory for rows and centroids
 
   private:
     void centroids(const float* y, size_t k, float* norms_y, bool with_mean, cudaStream_t stream);
     void convert(const float* x, size_t n, float* norms_x, cudaStream_t stream);
     void search(const float* x, size_t first, size_t n, const AssignTile* tiles, size_t n_tiles, const float* norms_x, uint32_t* out_knn, float* out_dist, cudaStream_t stream);
     size_t rows_at_once(size_t n) const;
-    void give_back();
     const float* y_ = nullptr;
     const float* norms_y_ = nullptr;
     size_t k_ = 0, d_ = 0, dp_ = 0, kp_ = 0;

@@ -86,3 +86,24 @@ def test_exact_assignment():
     want = skm.engine.find_nearest(x, c)[0]
     with without(12 * n * d // 10, 15 * n * d // 10):
         np.testing.assert_array_equal(skm.engine.find_nearest(x, c)[0], want)
+
+
+def test_fine_clusterings():
+    import superkmeans_b200 as skm
+
+    n, d, k = 20_000, 96, 200
+    x = datagen.gaussian_mixture(n, d, k // 3, 0.3, 4)
+
+    def train():
+        e = skm.Engine(k, d, skm.default_config(True, early_termination=0, suppress_warnings=1), hierarchical=True)
+        e.train(x)
+        return e.assignments(), [(s.iteration, s.objective) for s in e.stats(2)]
+
+    want, stats = train()
+    with without(2 * n * d):   # the fp16 rows of all mesoclusters
+        got, again = train()
+    assert [i for i, _ in stats] == [i for i, _ in again]
+    assert (got == want).mean() >= 0.98
+    # the first pass of every mesocluster starts from the same rows
+    a, b = (np.array([o for i, o in s if i == 1]) for s in (stats, again))
+    assert np.abs(a - b).max() <= 1e-5 * a.max()
