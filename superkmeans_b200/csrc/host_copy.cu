@@ -8,14 +8,16 @@ namespace skmb {
 
 namespace {
 
-bool is_pinned(const void* p) {
+cudaMemoryType type_of(const void* p) {
     cudaPointerAttributes a{};
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return cudaMemoryTypeUnregistered;
     }
-    return a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeManaged;
+    return a.type;
 }
+// Pinned or managed memory, and memory of a GPU that a caller gave in place of a host array: nothing to stage.
+bool copied_directly(const void* p) { return type_of(p) != cudaMemoryTypeUnregistered; }
 
 // A thread per quarter of a megabyte, eight at most: more do not copy faster.
 int threads_for(size_t bytes) { return static_cast<int>(std::max<size_t>(1, std::min<size_t>(8, bytes >> 18))); }
@@ -55,8 +57,13 @@ char* HostStage::piece(int i, size_t bytes) {
 
 void HostStage::upload(void* dst, const void* src, const size_t* idx, size_t n, size_t row_bytes, cudaStream_t stream) {
     if (n == 0 || row_bytes == 0) return;
-    if (!idx && is_pinned(src)) {
-        SKM_CUDA(cudaMemcpyAsync(dst, src, n * row_bytes, cudaMemcpyHostToDevice, stream));
+    if (!idx && copied_directly(src)) {
+        SKM_CUDA(cudaMemcpyAsync(dst, src, n * row_bytes, cudaMemcpyDefault, stream));
+        return;
+    }
+    if (idx && type_of(src) == cudaMemoryTypeDevice) {
+        for (size_t i = 0; i < n; ++i)
+            SKM_CUDA(cudaMemcpyAsync(static_cast<char*>(dst) + i * row_bytes, static_cast<const char*>(src) + idx[i] * row_bytes, row_bytes, cudaMemcpyDefault, stream));
         return;
     }
     const size_t per_piece = std::max<size_t>(1, kPieceBytes / row_bytes);
@@ -74,8 +81,8 @@ void HostStage::upload(void* dst, const void* src, const size_t* idx, size_t n, 
 
 void HostStage::download(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
     if (bytes == 0) return;
-    if (is_pinned(dst)) {
-        SKM_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream));
+    if (copied_directly(dst)) {
+        SKM_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, stream));
         SKM_CUDA(cudaStreamSynchronize(stream));
         return;
     }

@@ -70,6 +70,28 @@ void rows_arrive() {
     release_stream(work, 0);
 }
 
+// Device memory where host memory is expected.
+void device_memory() {
+    const cudaStream_t s = acquire_stream();
+    {
+        WorkStream on(s);
+        HostStage stage;
+        std::vector<float> rows(kRows * kRow, 3.0f);
+        for (size_t j = 0; j < kRow; ++j) rows[kRow + j] = 4.0f;
+        DeviceBuffer<float> src, dst, out;
+        SKM_CUDA(cudaMemcpyAsync(src.ensure(rows.size()), rows.data(), rows.size() * sizeof(float), cudaMemcpyHostToDevice, s));
+        stage.upload(dst.ensure(rows.size()), src.get(), nullptr, kRows, kRow * sizeof(float), s);
+        CHECK(fake::in_flight(src.get(), 1));   // (no host code has touched it)
+        stage.download(out.ensure(rows.size()), dst.get(), rows.size() * sizeof(float), s);
+        for (size_t i = 0; i < rows.size(); ++i) CHECK(out.get()[i] == rows[i]);
+        const std::vector<size_t> idx(kRows, 1);
+        stage.upload(dst.get(), src.get(), idx.data(), kRows, kRow * sizeof(float), s);
+        stage.download(out.get(), dst.get(), rows.size() * sizeof(float), s);
+        for (size_t i = 0; i < rows.size(); ++i) CHECK(out.get()[i] == 4.0f);
+    }
+    release_stream(s, 0);
+}
+
 } // namespace
 
 int main(int argc, char** argv) {
@@ -77,6 +99,7 @@ int main(int argc, char** argv) {
     if (what == "exception_behind_a_copy") exception_behind_a_copy(false);
     else if (what == "exception_behind_a_pinned_copy") exception_behind_a_copy(true);
     else if (what == "rows_arrive") rows_arrive();
+    else if (what == "device_memory") device_memory();
     else return 2;
     std::puts("OK");
     return 0;
