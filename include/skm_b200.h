@@ -252,10 +252,10 @@ skm_status skm_set_shard_comm(skm_handle* h, uint64_t n_global, uint64_t row_off
  * list workspaces) are kept by the library and reused by later calls that need about the same size on the same GPU, so
  * that repeated calls do not pay cudaMalloc / cudaFree (both synchronise the device) every time.  By default what is
  * kept stays within a sixteenth of the GPU's memory.  skm_set_workspace_cache(1) lifts that bound (repeated Train calls
- * over tens of gigabytes), skm_set_workspace_cache(0) keeps nothing from then on; skm_get_workspace_cache tells whether
- * the bound is lifted.  The memory goes back to the driver with skm_release_cached_memory, skm_set_workspace_cache(0)
+ * over tens of gigabytes), skm_set_workspace_cache(0) keeps nothing from then on, skm_set_workspace_cache(2) brings the
+ * bound back; skm_get_workspace_cache answers with the last of these numbers (2 at first).  The memory goes back to the driver with skm_release_cached_memory, skm_set_workspace_cache(0)
  * or the end of the process; an allocation that fails releases it and retries.  No counterpart in the reference. */
-void skm_set_workspace_cache(int enabled);
+void skm_set_workspace_cache(int mode);
 int skm_get_workspace_cache(void);
 void skm_release_cached_memory(void);
 uint64_t skm_cached_memory_bytes(void);

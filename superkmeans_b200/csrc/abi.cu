@@ -287,8 +287,10 @@ skm_status skm_set_shard_comm(skm_handle* h, uint64_t n_global, uint64_t row_off
     return guarded(h->err, [&] { h->engine->set_shard_nccl(n_global, row_offset, comm->comm.get()); });
 }
 
-void skm_set_workspace_cache(int enabled) { skmb::set_workspace_cache(enabled != 0); }
-int skm_get_workspace_cache(void) { return skmb::workspace_cache_enabled() ? 1 : 0; }
+void skm_set_workspace_cache(int mode) {
+    skmb::set_workspace_cache(mode == 0 ? skmb::CacheMode::nothing : (mode == 2 ? skmb::CacheMode::bounded : skmb::CacheMode::everything));
+}
+int skm_get_workspace_cache(void) { return static_cast<int>(skmb::workspace_cache()); }
 void skm_release_cached_memory(void) { skmb::release_cached_memory(); }
 uint64_t skm_cached_memory_bytes(void) { return skmb::cached_memory_bytes(); }
 

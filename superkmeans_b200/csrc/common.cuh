@@ -38,8 +38,8 @@ unsigned long long device_alloc_count();
 void note_device_alloc();
 
 // Device memory of DeviceBuffer, pinned host memory of PinnedBuffer, and the engines' streams.  What is released is parked
-// for the next request (memory.cu says within which bounds); set_workspace_cache(true) lifts the bound, so that repeated
-// Train calls over tens of gigabytes do not pay cudaMalloc / cudaFree either, and set_workspace_cache(false) parks nothing.
+// for the next request (memory.cu says within which bounds); CacheMode::everything lifts the bound, so that repeated
+// Train calls over tens of gigabytes do not pay cudaMalloc / cudaFree either, and CacheMode::nothing parks nothing.
 struct MemoryBlock {
     void* p = nullptr;
     size_t bytes = 0;   // true size: what was asked for, rounded up
@@ -70,8 +70,9 @@ class WorkStream {
     cudaStream_t previous_;
     int previous_device_;
 };
-void set_workspace_cache(bool on);
-bool workspace_cache_enabled();
+enum class CacheMode { nothing = 0, everything = 1, bounded = 2 };
+void set_workspace_cache(CacheMode mode);
+CacheMode workspace_cache();
 void release_cached_memory();
 size_t cached_memory_bytes();
 // wall-clock milliseconds this thread has spent inside device_alloc / device_free

@@ -5,8 +5,8 @@
 // a call or a handle gives up are parked here and handed to the next request of about their size.
 //
 //   * Bounded: by default the parked blocks of one GPU stay within a sixteenth of its memory and the pinned ones within
-//     256 MB; beyond that the blocks parked longest are returned to the driver.  set_workspace_cache(1) lifts the bound,
-//     set_workspace_cache(0) parks nothing, release_cached_memory() returns everything that is parked, and an
+//     256 MB; beyond that the blocks parked longest are returned to the driver.  CacheMode::everything lifts the bound,
+//     CacheMode::nothing parks nothing, release_cached_memory() returns everything that is parked, and an
 //     allocation that fails does so before it is tried again.
 //   * Safe between streams and threads: a block released while its thread works on a stream (WorkStream) carries an event
 //     recorded there, and whoever gets the block next makes its own stream wait for that event.  A block released
@@ -45,8 +45,6 @@ constexpr int kHost = -1;                 // "device" of pinned host blocks
 constexpr size_t kPinnedBound = size_t{256} << 20;
 constexpr size_t kMaxIdleStreams = 16;    // per device
 constexpr size_t kMaxIdleEvents = 1024;   // that measure time, per device
-
-enum class CacheMode { bounded, everything, nothing };
 
 struct FailingSizes {
     std::atomic<size_t> least{1}, most{0};
@@ -104,6 +102,25 @@ std::vector<Parked> take_all_parked() {
     std::lock_guard<std::mutex> lock(g_mu);
     std::vector<Parked> out;
     out.swap(g_parked);
+    return out;
+}
+
+// What is parked beyond the bounds, longest first (under g_mu).
+std::vector<Parked> over_the_bound() {
+    size_t total[kMaxDevices + 1] = {0};   // the host's last
+    auto slot = [](const Parked& q) { return q.device == kHost ? kMaxDevices : q.device; };
+    for (const Parked& q : g_parked) total[slot(q)] += q.bytes;
+    std::vector<Parked> out;
+    for (size_t i = 0; i < g_parked.size();) {
+        const Parked& q = g_parked[i];
+        if (total[slot(q)] <= bound_of(q.device)) {
+            ++i;
+            continue;
+        }
+        total[slot(q)] -= q.bytes;
+        out.push_back(q);
+        g_parked.erase(g_parked.begin() + static_cast<long>(i));
+    }
     return out;
 }
 
@@ -175,19 +192,7 @@ void park(Parked b) {
             surplus.push_back(b);
         } else {
             g_parked.push_back(b);
-            if (g_mode == CacheMode::bounded) {
-                size_t total = 0;
-                for (const Parked& q : g_parked) total += q.device == b.device ? q.bytes : 0;
-                for (size_t i = 0; i < g_parked.size() && total > bound_of(b.device);) {
-                    if (g_parked[i].device != b.device) {
-                        ++i;
-                        continue;
-                    }
-                    total -= g_parked[i].bytes;
-                    surplus.push_back(g_parked[i]);
-                    g_parked.erase(g_parked.begin() + static_cast<long>(i));
-                }
-            }
+            if (g_mode == CacheMode::bounded) surplus = over_the_bound();
         }
     }
     give_back_all(surplus);
@@ -327,17 +332,20 @@ void release_timing_event(cudaEvent_t e, int device) {
     cudaEventDestroy(e);
 }
 
-void set_workspace_cache(bool on) {
+void set_workspace_cache(CacheMode mode) {
+    std::vector<Parked> surplus;
     {
         std::lock_guard<std::mutex> lock(g_mu);
-        g_mode = on ? CacheMode::everything : CacheMode::nothing;
+        g_mode = mode;
+        if (mode == CacheMode::bounded) surplus = over_the_bound();
     }
-    if (!on) release_cached_memory();
+    if (mode == CacheMode::nothing) release_cached_memory();
+    give_back_all(surplus);
 }
 
-bool workspace_cache_enabled() {
+CacheMode workspace_cache() {
     std::lock_guard<std::mutex> lock(g_mu);
-    return g_mode == CacheMode::everything;
+    return g_mode;
 }
 
 void release_cached_memory() {

@@ -252,10 +252,15 @@ class Comm:
         self.close()
 
 
-def set_workspace_cache(enabled: bool) -> None:
-    """Keep device buffers between calls without a bound (True) or not at all (False); the default keeps a bounded amount
+def set_workspace_cache(mode: int) -> None:
+    """Keep device buffers between calls without a bound (True or 1), not at all (False or 0), or, the default, within a bound (2)
     (see skm_set_workspace_cache)."""
-    lib.skm_set_workspace_cache(int(enabled))
+    lib.skm_set_workspace_cache(int(mode))
+
+
+def workspace_cache() -> int:
+    """What set_workspace_cache was last given (2 at first)."""
+    return int(lib.skm_get_workspace_cache())
 
 
 def release_cached_memory() -> None:

@@ -85,6 +85,23 @@ void memory_that_is_short(size_t& limit, size_t& in_use) {
     release_stream(s, 0);
 }
 
+// The mode that was set is the one that is answered, and the bound holds again from when it is brought back.
+void modes() {
+    CHECK(workspace_cache() == CacheMode::bounded);
+    auto parked = [] {
+        use_and_park<DeviceBuffer<char>>(0, 30 << 20);   // (the fake device has 160 MB: ten of them may be parked)
+        use_and_park<PinnedBuffer<char>>(0, 30 << 20);
+        return std::pair<size_t, size_t>(fake::device_in_use, fake::pinned_in_use);
+    };
+    CHECK(parked().first == 0 && parked().second >= 30 << 20);
+    set_workspace_cache(CacheMode::everything);
+    CHECK(workspace_cache() == CacheMode::everything && parked().first >= 30 << 20);
+    set_workspace_cache(CacheMode::bounded);
+    CHECK(workspace_cache() == CacheMode::bounded && fake::device_in_use == 0 && fake::pinned_in_use >= 30 << 20);
+    set_workspace_cache(CacheMode::nothing);
+    CHECK(workspace_cache() == CacheMode::nothing && parked().first == 0 && parked().second == 0);
+}
+
 } // namespace
 
 int main(int argc, char** argv) {
@@ -93,6 +110,7 @@ int main(int argc, char** argv) {
     else if (what == "record_that_fails") record_that_fails();
     else if (what == "device_memory_that_is_short") memory_that_is_short<DeviceBuffer<char>>(fake::device_limit, fake::device_in_use);
     else if (what == "pinned_memory_that_is_short") memory_that_is_short<PinnedBuffer<char>>(fake::pinned_limit, fake::pinned_in_use);
+    else if (what == "modes") modes();
     else return 2;
     std::puts("OK");
     return 0;

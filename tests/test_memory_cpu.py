@@ -34,9 +34,22 @@ def program(tmp_path_factory):
     return make
 
 
-@pytest.mark.parametrize("name,case", [("memory_check", "events_between_devices"), ("memory_check", "record_that_fails"), ("memory_check", "device_memory_that_is_short"), ("memory_check", "pinned_memory_that_is_short"),
+@pytest.mark.parametrize("name,case", [("memory_check", "events_between_devices"), ("memory_check", "record_that_fails"), ("memory_check", "modes"), ("memory_check", "device_memory_that_is_short"), ("memory_check", "pinned_memory_that_is_short"),
                                        ("copies_check", "exception_behind_a_copy"), ("copies_check", "exception_behind_a_pinned_copy"), ("copies_check", "rows_arrive"), ("copies_check", "device_memory"),
                                        ("timers_check", "many_calls"), ("timers_check", "nothing_unfinished_is_read")])
 def test_with_a_runtime_of_host_code(program, name, case):
     res = subprocess.run([program(name), case], capture_output=True, text=True, timeout=120)
     assert res.returncode == 0 and "OK" in res.stdout, res.stdout + res.stderr
+
+
+def test_workspace_cache_answers_what_was_set():
+    from superkmeans_b200 import engine
+
+    before = engine.workspace_cache()
+    try:
+        for mode in (1, 0, 2):
+            engine.set_workspace_cache(mode)
+            assert engine.workspace_cache() == mode
+    finally:
+        engine.set_workspace_cache(before)
+    assert before == 2
