@@ -706,7 +706,8 @@ AssignRoute assign_route(size_t n, size_t k, size_t d) {
     const double blocks = d % 4 != 0 ? 1e9 : 4e-5 + elements * 8.0 / 5e12 + rounds(128, 148) * (columns / 256.0) * (1e-5 + static_cast<double>(d) / 16.0 * 3.3e-7);
     // the filter: six launches and a round trip, three passes (14 bytes an element), 2 n k d flop in tiles of 256 x 256
     const double filter = 8e-5 + elements * 14.0 / 5e12 + rounds(256, 74) * 74.0 * 256.0 * columns * std::max<double>(static_cast<double>(d), 128.0) / 5e14;
-    if (d <= 16384 && k < (size_t{1} << 31) && n >= 256 && filter < direct && filter < blocks) return AssignRoute::filter;
+    // (rows are listed by 32-bit indices)
+    if (d <= 16384 && k < (size_t{1} << 31) && n >= 256 && n < (size_t{1} << 32) && filter < direct && filter < blocks) return AssignRoute::filter;
     return direct < blocks ? AssignRoute::direct : AssignRoute::blocks;
 }
 
