@@ -14,8 +14,10 @@ __device__ __forceinline__ float warp_sum(float v) {
 }
 
 // Monotone map float -> uint32 (preserves <), so that (key << 32 | index) orders by distance then
-// by index under an unsigned 64-bit minimum.
+// by index under an unsigned 64-bit minimum.  A NaN comes last, and has to be asked for: the compiler may set the sign bit below with
+// a negation, which leaves a NaN's as it is.
 __device__ __forceinline__ uint32_t float_to_ordered(float f) {
+    if (f != f) return 0xFFFFFFFFu;
     const uint32_t b = __float_as_uint(f);
     return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
@@ -23,7 +25,7 @@ __device__ __forceinline__ float ordered_to_float(uint32_t o) {
     const uint32_t b = (o & 0x80000000u) ? (o & 0x7fffffffu) : ~o;
     return __uint_as_float(b);
 }
-// Ordered by distance, then by index; a NaN (of a kernel's own making, hence positive) comes last.
+// Ordered by distance, then by index.
 __device__ __forceinline__ unsigned long long pair_key(float dist, uint32_t index) {
     return (static_cast<unsigned long long>(float_to_ordered(dist)) << 32) | index;
 }
