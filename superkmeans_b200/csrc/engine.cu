@@ -59,6 +59,8 @@ size_t chunk_rows_for(size_t d, size_t n) {
     return std::max<size_t>(kTileM, std::min(rows, std::max<size_t>(n, 1)));
 }
 
+constexpr size_t kAskFrom = size_t{256} << 20;   // bytes of host rows, see Engine::assign
+
 void ensure_positive(bool ok, const char* name) {
     if (!ok) throw std::invalid_argument(std::string("Value must be positive: ") + name);
 }
@@ -1456,6 +1458,7 @@ void Engine::train_flat(const float* data, size_t n, bool on_device, const float
             // Host input: the exact assignment of iteration 1 needs nothing but the rotated rows and the initial
             // centroids, so it runs piece by piece between the uploads instead of after the last one.
             exact_open_ = assign_route(n_samples_, k_, d_) == AssignRoute::filter;
+            bool filtered = false, seen = false;   // (see Engine::assign)
             load_rows(
                 data, false, nullptr, n_samples_, true, x_rot_.get(),
                 [&](size_t r0, size_t cnt) {
@@ -1463,10 +1466,14 @@ void Engine::train_flat(const float* data, size_t n, bool on_device, const float
                     float* norms = data_norms_.get() + r0;
                     if (!centroids_ready) {
                         make_centroids();
-                        if (exact_open_) exact_open_ = exact_.begin(c_prev_.get(), k_, d_, n_samples_, n_samples_, centroid_norms_.get(), stream_);
+                        if (exact_open_) filtered = exact_open_ = exact_.begin(c_prev_.get(), k_, d_, n_samples_, n_samples_, centroid_norms_.get(), stream_);
                         if (!exact_open_) launch_row_sqnorms(c_prev_.get(), k_, d_, d_, centroid_norms_.get(), stream_);
                     }
-                    if (exact_open_) {
+                    if (filtered && r0 != 0 && !seen) {   // (from 265 000 rows on)
+                        seen = true;
+                        filtered = !exact_.in_vain(r0, stream_);
+                    }
+                    if (filtered) {
                         exact_.rows(x, r0, cnt, norms, assignments_.get() + r0, distances_.get() + r0, stream_);
                     } else {
                         launch_row_sqnorms(x, cnt, d_, d_, norms, stream_);
@@ -1839,7 +1846,8 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
     }
     const AssignRoute route = assign_route(n, n_centroids, d_);
     const size_t rows = streamed_rows(n);
-    const bool filtered = route == AssignRoute::filter && exact_.begin(c_dev, n_centroids, d_, n, rows, cn.get(), stream_), direct = route == AssignRoute::direct;
+    bool filtered = route == AssignRoute::filter && exact_.begin(c_dev, n_centroids, d_, n, rows, cn.get(), stream_);
+    const bool begun = filtered, direct = route == AssignRoute::direct;
     if (!filtered && !direct) launch_row_sqnorms(c_dev, n_centroids, d_, d_, cn.get(), stream_);
     DeviceBuffer<float> xn, dist;
     DeviceBuffer<uint32_t> knn;
@@ -1852,6 +1860,9 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
     for (size_t r0 = 0; r0 < n; r0 += rows) {
         const size_t cnt = std::min(rows, n - r0);
         const float* xb = pipe.upload(nullptr, vectors + r0 * d_, nullptr, cnt, sizeof(float) * d_);
+        // Listed rows have to cross once more.  (What the first piece came to is known by now; below a few milliseconds of copies the
+        // question costs more than it saves.)
+        if (filtered && r0 == rows && n * d_ * sizeof(float) >= kAskFrom && exact_.in_vain(r0, stream_)) filtered = false;
         pipe.arrive();
         if (filtered) {
             exact_.rows(xb, r0, cnt, xn.get(), knn.get() + r0, dist.get(), stream_);
@@ -1863,7 +1874,7 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
         }
         pipe.used();
     }
-    if (filtered) {
+    if (begun) {
         // rows that the filter could not settle cross once more
         const size_t listed = exact_.settle(stream_), per = rows;
         std::vector<uint32_t> idx32(listed);

@@ -133,15 +133,29 @@ __global__ void __launch_bounds__(256) centroid_fp16_kernel(const float* __restr
     if (lane == 0) stat_max(stats, kResidual, err);
 }
 
+// With centroids that the filter cannot tell apart (copies of one another, one of a norm far above the others', one that is no number)
+// every row ends in the list, and what the filter takes comes on top of the three-product kernel: 1M x 384 and 8192
+// centroids, one of them 1e6 long: 39.6 ms, where the three products alone take 33 - 36.  So a batch that has listed most of its
+// rows so far lists the others unseen (32.7).  Decided on the device, by the kernel before the filter, while nothing appends to the list.
+constexpr uint32_t kSeenRows = 4096;
+__device__ __forceinline__ bool hopeless(const uint32_t* n_listed, size_t rows_before) { return rows_before >= kSeenRows && 2 * static_cast<size_t>(*n_listed) > rows_before; }
+
 // Per row: fp16 copy, norm, and {squared norm minus the mean, squared norm of the rounding error, squared norm, scale}.
 template <bool VEC>
 __global__ void __launch_bounds__(256) row_fp16_kernel(const float* __restrict__ x, size_t n, size_t d, size_t dp, const float* __restrict__ mean, float* __restrict__ norms,
-                                                       __half* __restrict__ out, float4* __restrict__ info) {
+                                                       __half* __restrict__ out, float4* __restrict__ info, const uint32_t* __restrict__ n_listed, size_t rows_before,
+                                                       uint32_t* __restrict__ unseen) {
     const size_t row = static_cast<size_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+    const bool give_up = hopeless(n_listed, rows_before);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *unseen = give_up ? 1u : 0u;
     if (row >= n) return;
     const int lane = threadIdx.x & 31;
     const float* xr = x + row * d;
     const RowNorms nx = row_norms<VEC>(xr, mean, d, lane);
+    if (give_up) {
+        if (lane == 0) norms[row] = nx.plain;
+        return;
+    }
     const float scale = fp16_scale(nx.centred);
     const float err = write_fp16_row<VEC>(xr, mean, d, dp, scale, out + row * dp, lane);
     if (lane != 0) return;
@@ -211,6 +225,7 @@ struct FilterParams {
     uint4* cand;
     uint32_t* listed;
     uint32_t* n_listed;
+    const uint32_t* unseen;   // nonzero: list all rows
     int* error;
     long long wait_limit;
     uint32_t producer_stop;   // see set_debug_wait_injection
@@ -241,6 +256,20 @@ template <bool GROUPED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(F_THREADS, 1)
     filter_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_y, const FilterParams p) {
     extern __shared__ uint8_t smem_raw[];
+    if (!GROUPED && *p.unseen != 0) {   // (the same for all blocks)
+        for (size_t row0 = static_cast<size_t>(blockIdx.x) * F_THREADS; row0 < p.n; row0 += static_cast<size_t>(gridDim.x) * F_THREADS) {
+            const size_t row = row0 + threadIdx.x;
+            const uint32_t mine = __ballot_sync(0xffffffffu, row < p.n), lane_id = threadIdx.x & 31;
+            uint32_t at = 0;
+            if (lane_id == 0) at = atomicAdd(p.n_listed, static_cast<uint32_t>(__popc(mine)));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (row < p.n) {
+                p.listed[at + lane_id] = static_cast<uint32_t>(p.first + row);
+                p.cand[row].x = ~0u;
+            }
+        }
+        return;
+    }
     const uint32_t raw_addr = smem_u32(smem_raw);
     const uint32_t pad = (1024u - (raw_addr & 1023u)) & 1023u;
     const uint32_t smem_base = raw_addr + pad;
@@ -690,6 +719,8 @@ __global__ void __launch_bounds__(256) decide_listed_tiles_kernel(const float* _
     }
 }
 
+constexpr size_t kWaveRows = 74 * 256;   // a row tile for every pair of SMs
+
 bool aligned16(const float* p, size_t d) { return d % 4 == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 unsigned warps_grid(size_t rows) { return static_cast<unsigned>((rows + 7) / 8); }
 
@@ -732,7 +763,7 @@ void ExactAssign::centroids(const float* y, size_t k, float* norms_y, bool with_
     float* centred = centred_norms_.ensure(kp_);
     uint32_t* stats = stats_.ensure(kStats);
     __half* yh = yh_.ensure(k * dp_);
-    sample_mean_kernel<<<with_mean ? static_cast<unsigned>((d_ + 63) / 64) : 1u, 64, 0, stream>>>(y, k, with_mean ? d_ : 0, mean, stats, n_listed_.ensure(1));
+    sample_mean_kernel<<<with_mean ? static_cast<unsigned>((d_ + 63) / 64) : 1u, 64, 0, stream>>>(y, k, with_mean ? d_ : 0, mean, stats, n_listed_.ensure(2));
     SKM_LAUNCH_CHECK();
     if (aligned16(y, d_)) {
         centroid_norms_kernel<true><<<warps_grid(kp_), 256, 0, stream>>>(y, k, kp_, d_, mean, norms_y, centred, stats);
@@ -746,10 +777,10 @@ void ExactAssign::centroids(const float* y, size_t k, float* norms_y, bool with_
     SKM_LAUNCH_CHECK();
 }
 
-void ExactAssign::convert(const float* x, size_t n, float* norms_x, cudaStream_t stream) {
-    __half* xh = xh_.get();
-    if (aligned16(x, d_)) row_fp16_kernel<true><<<warps_grid(n), 256, 0, stream>>>(x, n, d_, dp_, mean_.get(), norms_x, xh, row_info_.get());
-    else row_fp16_kernel<false><<<warps_grid(n), 256, 0, stream>>>(x, n, d_, dp_, mean_.get(), norms_x, xh, row_info_.get());
+// (before: rows of the batch that have gone through the filter already)
+void ExactAssign::convert(const float* x, size_t n, size_t before, float* norms_x, cudaStream_t stream) {
+    auto* kernel = aligned16(x, d_) ? row_fp16_kernel<true> : row_fp16_kernel<false>;
+    kernel<<<warps_grid(n), 256, 0, stream>>>(x, n, d_, dp_, mean_.get(), norms_x, xh_.get(), row_info_.get(), n_listed_.get(), before, n_listed_.get() + 1);
     SKM_LAUNCH_CHECK();
 }
 
@@ -772,6 +803,7 @@ void ExactAssign::search(const float* x, size_t first, size_t n, const AssignTil
     p.cand = cand_.ensure(n);
     p.listed = listed_.get();
     p.n_listed = n_listed_.get();
+    p.unseen = n_listed_.get() + 1;
     p.error = error_word();
     p.wait_limit = wait_limit();
     p.producer_stop = producer_stop();
@@ -788,7 +820,7 @@ void ExactAssign::search(const float* x, size_t first, size_t n, const AssignTil
 
 // A gigabyte of fp16 rows, in whole waves of row tiles.
 size_t ExactAssign::rows_at_once(size_t n) const {
-    const size_t wave = 74 * 256;
+    const size_t wave = kWaveRows;
     return std::min(n, std::max(wave, ((size_t{1} << 30) / (dp_ * sizeof(__half))) / wave * wave));
 }
 
@@ -819,12 +851,17 @@ bool ExactAssign::begin(const float* y, size_t k, size_t d, size_t batch_rows, s
 }
 
 void ExactAssign::rows(const float* x, size_t first, size_t n, float* norms_x, uint32_t* out_knn, float* out_dist, cudaStream_t stream) {
-    const size_t per = rows_at_once(n);
+    const size_t per = rows_at_once(n), wave = kWaveRows;
     xh_.ensure(per * dp_);
     row_info_.ensure(per);
-    for (size_t r0 = 0; r0 < n; r0 += per) {
-        const size_t cnt = std::min(per, n - r0);
-        convert(x + r0 * d_, cnt, norms_x + r0, stream);
+    // the first launch of a batch of several waves is short, to see what the list comes to; it takes what is left of the last wave
+    // (from about a millisecond on, of which the launches are one or two percent)
+    const bool long_enough = static_cast<double>(n) * static_cast<double>(kp_) * std::max<double>(static_cast<double>(dp_), 128.0) > 5e11 && n > 2 * wave;
+    const size_t look = first == 0 && long_enough ? (n % wave >= kSeenRows ? n % wave : wave) : per;
+    size_t cnt;
+    for (size_t r0 = 0; r0 < n; r0 += cnt) {
+        cnt = std::min({per, n - r0, r0 == 0 ? look : per});
+        convert(x + r0 * d_, cnt, first + r0, norms_x + r0, stream);
         search(x + r0 * d_, first + r0, cnt, nullptr, 0, norms_x + r0, out_knn + r0, out_dist + r0, stream);
     }
 }
@@ -835,9 +872,9 @@ void ExactAssign::begin_groups(const float* x, size_t n, size_t d, const float* 
     dp_ = (d + 7) / 8 * 8;
     xh_.ensure(n * dp_);
     row_info_.ensure(n);
-    sample_mean_kernel<<<static_cast<unsigned>((d + 63) / 64), 64, 0, stream>>>(y, k, d, mean_.ensure(dp_), stats_.ensure(kStats), n_listed_.ensure(1));
+    sample_mean_kernel<<<static_cast<unsigned>((d + 63) / 64), 64, 0, stream>>>(y, k, d, mean_.ensure(dp_), stats_.ensure(kStats), n_listed_.ensure(2));
     SKM_LAUNCH_CHECK();
-    convert(x, n, norms_x, stream);
+    convert(x, n, 0, norms_x, stream);
 }
 
 void ExactAssign::assign_groups(const float* x, size_t n, const float* y, size_t k, const AssignTile* tiles, size_t n_tiles, const float* norms_x, float* norms_y, uint32_t* out_knn,

@@ -45,11 +45,13 @@ class ExactAssign {
     // launch_row_sqnorms gives them), an empty list, and memory for up to piece_rows rows at a time.  False: there is not enough
     // of it (the fp16 rows take a gigabyte at most), nothing has been done and none is held.
     bool begin(const float* y, size_t k, size_t d, size_t batch_rows, size_t piece_rows, float* norms_y, cudaStream_t stream);
-    // Rows [first, first + n) of the batch; their squared norms go to norms_x (as launch_row_sqnorms gives them).
+    // Rows [first, first + n) of the batch, one piece after the other; their squared norms go to norms_x (as launch_row_sqnorms gives them).
     void rows(const float* x, size_t first, size_t n, float* norms_x, uint32_t* out_knn, float* out_dist, cudaStream_t stream);
     // Number of listed rows (waits for the stream); their indices inside the batch are in listed().
     size_t settle(cudaStream_t stream);
     const uint32_t* listed() const { return listed_.get(); }
+    // Whether most of the first `done` rows are listed (waits for the stream): the rest had better not go through the filter.
+    bool in_vain(size_t done, cudaStream_t stream) { return 2 * settle(stream) > done; }
     // out_knn / out_dist (may be null) of the rows listed()[at .. at + count), given those rows.
     void finish(const float* x_listed, size_t at, size_t count, uint32_t* out_knn, float* out_dist, cudaStream_t stream);
     // Both, for a batch that is still on the device.
@@ -65,7 +67,7 @@ class ExactAssign {
 
   private:
     void centroids(const float* y, size_t k, float* norms_y, bool with_mean, cudaStream_t stream);
-    void convert(const float* x, size_t n, float* norms_x, cudaStream_t stream);
+    void convert(const float* x, size_t n, size_t before, float* norms_x, cudaStream_t stream);
     void search(const float* x, size_t first, size_t n, const AssignTile* tiles, size_t n_tiles, const float* norms_x, uint32_t* out_knn, float* out_dist, cudaStream_t stream);
     size_t rows_at_once(size_t n) const;
     const float* y_ = nullptr;
