@@ -14,12 +14,14 @@ __device__ __forceinline__ float warp_sum(float v) {
 }
 
 // Monotone map float -> uint32 (preserves <), so that (key << 32 | index) orders by distance then
-// by index under an unsigned 64-bit minimum.  A NaN comes last, and has to be asked for: the compiler may set the sign bit below with
-// a negation, which leaves a NaN's as it is.
+// by index under an unsigned 64-bit minimum.  A NaN that an operation made (0x7fffffff) comes last.  The last step is hidden from the
+// compiler, which would set the sign bit with a floating-point negation, and that leaves a NaN as it is: it then came first.
+// (Asking for it instead took 1 us of the 20 of a call of 5000 x 300 x 128.)
 __device__ __forceinline__ uint32_t float_to_ordered(float f) {
-    if (f != f) return 0xFFFFFFFFu;
-    const uint32_t b = __float_as_uint(f);
-    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+    const uint32_t b = __float_as_uint(f), flip = static_cast<uint32_t>(static_cast<int32_t>(b) >> 31) | 0x80000000u;
+    uint32_t key;
+    asm("xor.b32 %0, %1, %2;" : "=r"(key) : "r"(b), "r"(flip));
+    return key;
 }
 __device__ __forceinline__ float ordered_to_float(uint32_t o) {
     const uint32_t b = (o & 0x80000000u) ? (o & 0x7fffffffu) : ~o;
