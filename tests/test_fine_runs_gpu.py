@@ -94,6 +94,8 @@ def test_a_row_without_a_distance(value, spread):
         e.train(x)
         res.append(np.array([s.objective for s in e.stats(2) if s.iteration == 1]))
         assert e.assignments().max() < k
-    # the row counts for nothing in either form
-    assert np.isfinite(res[0]).all() == np.isfinite(res[1]).all()
-    assert (np.abs(res[0] - res[1]) <= 1e-5 * np.abs(res[0]) + 1e-3).all(), res
+    # the row counts for nothing, or (a finite one whose squared norm is not) for an infinity, in either form
+    finite = np.isfinite(res[0])
+    np.testing.assert_array_equal(res[0][~finite], res[1][~finite])
+    assert finite.sum() >= len(finite) - 1 and (finite.all() or value == 3e38)
+    assert (np.abs(res[0] - res[1])[finite] <= 1e-5 * np.abs(res[0][finite]) + 1e-3).all(), res
