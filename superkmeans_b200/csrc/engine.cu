@@ -957,10 +957,14 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
     // per cluster (so that a tile of 128 ordered points spans few clusters), the points go, in the order of their
     // previous centroid, through the chain over each tile's reachable centroids (whose cost follows the union of
     // the tile's survivors, not their number).
-    // Measured on one B200, 10 iterations: 10M x 1024, k = 10 000 (survival 3.3 - 4.2 %): 5.0 s against 7.3 s;
-    // 1M x 1536, k = 4096 (2.2 %, then below 0.1 %): lists 0.22 s against 0.39 s; a shard of 1.25M x 1024 of the
-    // first workload (125 points per cluster): 0.58 s against 0.99 s.  Below 2^18 points the fixed costs of the
-    // ordered route (sort, batches, host round trips) outweigh it: 100k x 768, k = 1000: 23.5 ms against 16.9 ms.
+    // Measured on one B200, a Train of ten iterations with every pass ordered against every pass by lists:
+    //   10M x 1024, k = 10 000 (survival 3.3 - 4.2 %)              3.39 s against 8.24
+    //   1.25M rows of it (125 points per cluster, 3.0 - 3.7 %)     0.50 s against 1.07
+    //   320 000 rows of it (32 points per cluster, 2.5 - 2.7 %)    0.22 s against 0.26
+    //   1M x 1536, k = 4096 (2.2 %, then below 0.1 %)              0.24 s against 0.11; 0.17 as chosen, because the sample puts the
+    //                                                              first pass just above the line
+    //   100k x 768, k = 1000 (7.7 %, then 0.2 %)                   12.9 ms against 6.5: below 2^18 points the fixed costs of the
+    //                                                              ordered route (sort, batches, host round trips) outweigh it
     auto ordered = [&](double survival) {
         return auto_mode && tc_ok && p.k <= 65536 && survival >= auto_chain_survival() && p.n >= 32 * p.k && p.n >= (size_t{1} << 18);
     };

@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_tc_kernel(const __grid_co
     } else if (warp < 10 || kTiled) {
         // ---------------------------------------------------------------- epilogue
         // Union and counting modes: eight warps, two per quarter of the tile's rows; warps 6-9 take columns 0-127 of
-        // every 256-column tile, warps 10-13 columns 128-255, each with a candidate list of its own.
+        // every 256-column tile, warps 10-13 columns 128-255.
         const uint32_t half = kTiled ? static_cast<uint32_t>(warp - 6) >> 2 : 0u;
         const uint32_t lane_base = 32u * (warp & 3);    // tensor-memory lanes this warp may read
         const uint32_t row_in_tile = lane_base + lane;

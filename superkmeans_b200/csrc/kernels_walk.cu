@@ -140,7 +140,8 @@ __device__ __forceinline__ bool walk_rest(bool alive, const float* __restrict__ 
 // Blocks of two warps, so that the few row groups of a small problem still reach every SM, and twelve of them to an SM: the
 // registers of four more are worth more as loads in flight.  One B200, nine passes of a Train each, against a block of 128
 // points before: 1M x 1024, k = 4000: 12.0 ms (21.0 before; 12.2 with sixteen blocks to an SM); 100k x 1536, k = 2000: 4.2 (6.1);
-// 30 000 x 768, k = 1000: 0.63 (0.59; 0.78 with sixteen).
+// 30 000 x 768, k = 1000: 0.63 (0.59; 0.78 with sixteen).  (With the share of the points that went to the dense chain then; the first
+// test now drops fewer of them, see kHardShare, and the first of the three takes 18.2 ms here.)
 constexpr int kWalkCtasPerSm = 12;
 
 __global__ void __launch_bounds__(kWalkThreads, kWalkCtasPerSm) walk_lists_kernel(const WalkParams w) {

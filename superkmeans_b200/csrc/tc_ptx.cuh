@@ -272,14 +272,15 @@ __device__ __forceinline__ void split4(float4 v, float4& hi, float4& lo) {
     lo.x = to_tf32(v.x - hi.x); lo.y = to_tf32(v.y - hi.y); lo.z = to_tf32(v.z - hi.z); lo.w = to_tf32(v.w - hi.w);
 }
 
+// Tensor maps (defined in kernels_tc.cu), zero fill outside the matrix.
 // Row-major fp32 matrix [rows][ld] of which the first `extent` columns are visible; boxes of 16 columns x box_rows
-// rows, 64-byte swizzle, zero fill outside (defined in kernels_tc.cu).
-// Row-major fp16 matrix [rows][pitch] (pitch a multiple of 8, 0: cols) of which the first cols columns are visible; boxes of
-// 64 columns x box_rows rows, 128-byte swizzle, zero fill outside.
-CUtensorMap make_half_tmap(const void* base, size_t cols, size_t rows, uint32_t box_rows, size_t pitch = 0);
+// rows, 64-byte swizzle.
+CUtensorMap make_row_major_tmap(const float* base, size_t extent, size_t rows, size_t ld, uint32_t box_rows);
 // ... in boxes of 32 columns, 128-byte swizzle
 CUtensorMap make_row_major_tmap_128(const float* base, size_t extent, size_t rows, size_t ld, uint32_t box_rows);
-CUtensorMap make_row_major_tmap(const float* base, size_t extent, size_t rows, size_t ld, uint32_t box_rows);
+// Row-major fp16 matrix [rows][pitch] (pitch a multiple of 8, 0: cols) of which the first cols columns are visible; boxes of
+// 64 columns x box_rows rows, 128-byte swizzle.
+CUtensorMap make_half_tmap(const void* base, size_t cols, size_t rows, uint32_t box_rows, size_t pitch = 0);
 
 } // namespace tc
 } // namespace skmb
