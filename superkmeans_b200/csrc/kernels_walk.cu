@@ -144,7 +144,7 @@ __device__ __forceinline__ bool walk_rest(bool alive, const float* __restrict__ 
 // test now drops fewer of them, see kHardShare, and the first of the three takes 18.2 ms here.)
 constexpr int kWalkCtasPerSm = 12;
 
-__global__ void __launch_bounds__(kWalkThreads, kWalkCtasPerSm) walk_lists_kernel(const WalkParams w) {
+__global__ void __launch_bounds__(kWalkThreads, kWalkCtasPerSm) walk_lists_kernel(const WalkParams w, const uint32_t share) {
     __shared__ WarpShared all[kWalkWarps];
     if (w.upstream_error && *reinterpret_cast<const volatile int*>(w.upstream_error) != 0) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -157,8 +157,8 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkCtasPerSm) walk_lists_kerne
     const float ratio_first = __ldg(w.ratios + w.partial_d);
     unsigned long long steps_done = 0;
 
-    for (size_t group = static_cast<size_t>(blockIdx.x) * kWalkWarps + warp; group < w.n_tiles * 4; group += static_cast<size_t>(gridDim.x) * kWalkWarps) {
-        const size_t tile = group >> 2;
+    for (size_t unit = static_cast<size_t>(blockIdx.x) * kWalkWarps + warp; unit < w.n_tiles * 4 * share; unit += static_cast<size_t>(gridDim.x) * kWalkWarps) {
+        const size_t group = unit / share, tile = group >> 2;
         const uint32_t quarter = static_cast<uint32_t>(group & 3);
         const size_t row0 = (w.tile_map ? static_cast<size_t>(w.tile_map[tile]) : w.tile0 + tile) * kTileM + quarter * kWalkRows;
         const size_t row = row0 + lane;
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkCtasPerSm) walk_lists_kerne
         const size_t list_id = tile * kListsPerTile + static_cast<size_t>(lane & (kWalkLists - 1)) * 4 + quarter;
         const uint32_t* offs = w.list_offs + list_id * (n_chunks + 1);
         const bool overflow = __any_sync(0xffffffffu, __ldg(offs + n_chunks) > w.cap_group);
-        bool active = row < w.n && !(w.skip && w.skip[row]);
+        bool active = row < w.n && !(w.skip && w.skip[row]) && lane * share / kWalkRows == unit % share;
         if (active && overflow) {
             // a list did not fit: its points go to the dense kernel
             w.redo[row] = 1u;
@@ -324,8 +324,14 @@ void launch_walk_lists(const WalkParams& w, int device, cudaStream_t stream) {
     if (w.n_tiles == 0) return;
     int sms = 0;
     SKM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    const unsigned grid = static_cast<unsigned>(std::min<size_t>((w.n_tiles * 4 + kWalkWarps - 1) / kWalkWarps, static_cast<size_t>(sms) * kWalkCtasPerSm));
-    walk_lists_kernel<<<grid, kWalkThreads, 0, stream>>>(w);
+    // Few points: their lists are shared by two or four warps (each reads them all and walks the pairs of its own points), while that
+    // makes no more than two warps for every place there is: a warp's pairs are a chain of gathers.  30 000 x 768, k = 1000, nine passes: 98
+    // us a pass with one warp, 81 with two, 77 with four, 94 with eight; 250 000 points: no difference up to four.
+    const size_t places = static_cast<size_t>(sms) * kWalkCtasPerSm * kWalkWarps;
+    uint32_t share = 1;
+    while (share < 4 && w.n_tiles * 4 * share * 2 <= 2 * places) share *= 2;
+    const unsigned grid = static_cast<unsigned>(std::min<size_t>((w.n_tiles * 4 * share + kWalkWarps - 1) / kWalkWarps, static_cast<size_t>(sms) * kWalkCtasPerSm));
+    walk_lists_kernel<<<grid, kWalkThreads, 0, stream>>>(w, share);
     SKM_LAUNCH_CHECK();
 }
 
