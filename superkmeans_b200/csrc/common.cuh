@@ -355,6 +355,10 @@ struct ConsolidateParams {
     uint4* told;            // copies to pinned host memory (told_words may be zero)
     size_t told_words;
 };
+// launch_update and launch_consolidate of means that need not have unit length (p.counts and p.normalize are not looked at), in one launch, for
+// the problems that small_update names.  x, p.c, p.prev: 16-byte aligned.
+bool small_update(size_t n, size_t k, size_t d);
+void launch_small_update(const float* x, const uint32_t* assign, size_t n, uint32_t* counts, const UpdateStats& stats, const ConsolidateParams& p, cudaStream_t stream);
 // Pinned host memory (16-byte aligned) = device memory, by a kernel of one block: a copy starts 8 us after the kernel before it ends,
 // the next kernel after 1.
 void launch_tell_host(const void* from, void* to, size_t bytes, cudaStream_t stream);

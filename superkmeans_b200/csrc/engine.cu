@@ -1243,6 +1243,10 @@ void Engine::fetch_report(size_t k_cur) {
 // ConsolidateCentroids without the splits, and ComputeShift.
 void Engine::consolidate(const IterationInput& in, bool scale) {
     PhaseScope ps(*this, PH_CONSOLIDATE);
+    launch_consolidate(consolidate_params(in, scale), stream_);
+}
+
+ConsolidateParams Engine::consolidate_params(const IterationInput& in, bool scale) {
     ConsolidateParams p{};
     p.c = c_cur_.get();
     p.prev = c_prev_.get();
@@ -1261,7 +1265,7 @@ void Engine::consolidate(const IterationInput& in, bool scale) {
         p.told = reinterpret_cast<uint4*>(outcome_host_.get());
         p.told_words = (kReportWords + in.n_clusters + 3) / 4;
     }
-    launch_consolidate(p, stream_);
+    return p;
 }
 
 // -------------------------------------------------------------------------------------------------
@@ -1289,17 +1293,22 @@ void Engine::run_iteration(bool gemm_only, const IterationInput& in, size_t iter
         run_pruned_pass_on(pruned_params(in), prune_bufs_, ratios_host_[partial_d_], device_, stream_, &timers_);
     }
     // UpdateCentroids + ComputeCost (superkmeans.h:729-765, :973-981)
-    {
+    UpdateStats stats;
+    stats.dist = distances_.get();
+    stats.not_pruned = gemm_only ? nullptr : not_pruned_.get();
+    stats.error = tc::error_word();
+    stats.report = report();
+    if (!sharded_() && !cfg_.angular && small_update(n, k_cur, d_)) {
         PhaseScope ps(*this, PH_UPDATE);
-        UpdateStats stats;
-        stats.dist = distances_.get();
-        stats.not_pruned = gemm_only ? nullptr : not_pruned_.get();
-        stats.error = tc::error_word();
-        stats.report = report();
-        launch_update(in.x, assignments_.get(), n, k_cur, d_, ws_, c_cur_.get(), counts(), &stats, stream_);
+        launch_small_update(in.x, assignments_.get(), n, counts(), stats, consolidate_params(in, true), stream_);
+    } else {
+        {
+            PhaseScope ps(*this, PH_UPDATE);
+            launch_update(in.x, assignments_.get(), n, k_cur, d_, ws_, c_cur_.get(), counts(), &stats, stream_);
+        }
+        allreduce_iteration(c_cur_.get(), k_cur * d_, counts(), k_cur, &report()->wcss, 2);
+        consolidate(in, true);
     }
-    allreduce_iteration(c_cur_.get(), k_cur * d_, counts(), k_cur, &report()->wcss, 2);
-    consolidate(in, true);
     fetch_report(k_cur);
     const IterationReport& told = *report_host();
     const double wcss = told.wcss;

@@ -241,6 +241,7 @@ class Engine {
     void prepare_update_workspace(size_t n, size_t k);
     void run_iteration(bool gemm_only, const IterationInput& in, size_t iter_idx, bool is_first, std::vector<skm_iter_stats>& target);
     PrunedParams pruned_params(const IterationInput& in);
+    ConsolidateParams consolidate_params(const IterationInput& in, bool scale);
     void consolidate(const IterationInput& in, bool scale);
     void fetch_report(size_t k_cur);
     bool split(size_t n_samples_global, size_t k_cur);

@@ -1078,6 +1078,144 @@ __global__ void __launch_bounds__(256) consolidate_kernel(const ConsolidateParam
     for (size_t i = threadIdx.x; i < p.told_words; i += 256) p.told[i] = __ldcg(p.tell + i);
 }
 
+// UpdateCentroids, ComputeCost, ConsolidateCentroids and ComputeShift of a small problem in one launch, a block per cluster: it looks for its
+// points among all of them (a piece at a time, their rows in a fixed order), adds their rows up, and has the cluster's centroid.
+constexpr int kSmallPiece = 4096;
+constexpr int kSmallLoads = 8;   // rows in flight per thread
+__global__ void __launch_bounds__(256) small_update_kernel(const float* __restrict__ x, const uint32_t* __restrict__ assign, size_t n, const UpdateStats u, uint32_t* __restrict__ counts,
+                                                           const ConsolidateParams p) {
+    __shared__ uint32_t ids[kSmallPiece];
+    __shared__ float4 parts[256];
+    __shared__ uint32_t found[8];
+    __shared__ double sd[3][8];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t cluster = blockIdx.x;
+    const uint32_t groups = static_cast<uint32_t>(p.d / 4), rows = 256 / groups;   // columns four at a time, rows beside each other
+    const uint32_t g = threadIdx.x % groups, r = threadIdx.x / groups;
+    double cost = 0.0;
+    unsigned long long not_pruned = 0;
+    uint32_t count = 0;
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (size_t base = 0; base < n; base += kSmallPiece) {
+        uint32_t mask = 0;
+#pragma unroll
+        for (int i = 0; i < kSmallPiece / 256; ++i) {
+            const size_t at = base + i * 256 + threadIdx.x;
+            if (at < n && __ldg(assign + at) == cluster) mask |= 1u << i;
+        }
+        const uint32_t mine = __popc(mask);
+        uint32_t before = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, before, o);
+            if (lane >= o) before += t;
+        }
+        if (lane == 31) found[warp] = before;
+        before -= mine;
+        __syncthreads();
+        uint32_t m = 0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+            if (w < warp) before += found[w];
+            m += found[w];
+        }
+        for (; mask; mask &= mask - 1) {
+            const uint32_t at = static_cast<uint32_t>(base) + (__ffs(mask) - 1) * 256 + threadIdx.x;
+            ids[before++] = at;
+            cost += static_cast<double>(u.dist[at]);
+            if (u.not_pruned) not_pruned += u.not_pruned[at];
+        }
+        __syncthreads();
+        count += m;
+        if (r < rows) {
+            for (uint32_t j = r; j < m; j += rows * kSmallLoads) {
+                float4 v[kSmallLoads];
+#pragma unroll
+                for (int q = 0; q < kSmallLoads; ++q)
+                    v[q] = j + q * rows < m ? __ldg(reinterpret_cast<const float4*>(x + static_cast<size_t>(ids[j + q * rows]) * p.d) + g) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int q = 0; q < kSmallLoads; ++q) {
+                    sum.x += v[q].x;
+                    sum.y += v[q].y;
+                    sum.z += v[q].z;
+                    sum.w += v[q].w;
+                }
+            }
+        }
+        __syncthreads();
+    }
+    parts[threadIdx.x] = sum;
+    __syncthreads();
+    float s = 0.f;
+    if (r == 0) {
+        for (uint32_t q = 1; q < rows; ++q) {
+            const float4 t = parts[q * groups + g];
+            sum.x += t.x;
+            sum.y += t.y;
+            sum.z += t.z;
+            sum.w += t.w;
+        }
+        const float mult = count ? static_cast<float>(1.0 / static_cast<double>(count)) : 1.0f;
+        const float val[4] = {__fmul_rn(sum.x, mult), __fmul_rn(sum.y, mult), __fmul_rn(sum.z, mult), __fmul_rn(sum.w, mult)};
+        const size_t chunk = cluster / kChunk, v = cluster % kChunk;
+        const size_t cs = min(static_cast<size_t>(kChunk), p.k - chunk * kChunk);
+        float* __restrict__ pdx = p.pdx + chunk * kChunk * p.d;
+        const float4 prev = *reinterpret_cast<const float4*>(p.prev + cluster * p.d + 4 * g);
+        const float pv[4] = {prev.x, prev.y, prev.z, prev.w};
+        *reinterpret_cast<float4*>(p.c + cluster * p.d + 4 * g) = make_float4(val[0], val[1], val[2], val[3]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const size_t j = 4 * g + q;
+            pdx[pdx_offset(j, v, cs, p.vertical_d)] = val[q];
+            if (j < p.vertical_d) p.aux[cluster * p.vertical_d + j] = val[q];
+            const float t = val[q] - pv[q];
+            s = fmaf(t, t, s);
+        }
+    }
+    // sums over the block, then over the blocks, always in the same order
+    double a[3] = {static_cast<double>(s), cost, static_cast<double>(not_pruned)};   // (counts below 2^53)
+    auto block_sums = [&](double (&v)[3]) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+            if (lane == 0) sd[i][warp] = v[i];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            v[i] = 0.0;
+            for (int w = 0; w < 8; ++w) v[i] += sd[i][w];
+        }
+        __syncthreads();
+    };
+    block_sums(a);
+    if (threadIdx.x == 0) {
+        counts[cluster] = count;
+        for (int i = 0; i < 3; ++i) p.reduce_scratch[3 * cluster + i] = a[i];
+    }
+    if (!last_block(p.reduce_scratch)) return;
+    a[0] = a[1] = a[2] = 0.0;
+    for (size_t c = threadIdx.x; c < p.k; c += 256)
+        for (int i = 0; i < 3; ++i) a[i] += __ldcg(p.reduce_scratch + 3 * c + i);
+    block_sums(a);
+    if (threadIdx.x == 0) {
+        p.report->shift = a[0];
+        p.report->wcss = a[1];
+        p.report->not_pruned = a[2];
+        p.report->error = u.error ? *u.error : 0;
+    }
+    __syncthreads();
+    for (size_t i = threadIdx.x; i < p.told_words; i += 256) p.told[i] = __ldcg(p.tell + i);
+}
+
+bool small_update(size_t n, size_t k, size_t d) { return d % 4 == 0 && d <= 1024 && 3 * k <= 2 * kReduceBlocks && n * d <= (size_t{1} << 19); }
+
+void launch_small_update(const float* x, const uint32_t* assign, size_t n, uint32_t* counts, const UpdateStats& stats, const ConsolidateParams& p, cudaStream_t stream) {
+    small_update_kernel<<<static_cast<unsigned>(p.k), 256, 0, stream>>>(x, assign, n, stats, counts, p);
+    SKM_LAUNCH_CHECK();
+}
+
 __global__ void __launch_bounds__(256) tell_host_kernel(const uint4* __restrict__ from, uint4* __restrict__ to, size_t words) {
     for (size_t i = threadIdx.x; i < words; i += 256) to[i] = from[i];
 }
