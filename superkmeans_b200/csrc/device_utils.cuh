@@ -67,4 +67,33 @@ __device__ __forceinline__ void normalize_row(float* __restrict__ p, size_t d, i
     for (size_t j = lane; j < d; j += 32) p[j] *= inv;
 }
 
+// Cumulative squared norm of `row` after each checkpoint of the chain: [0, d'), then each horizontal
+// block [vd + 64 b, vd + 64 (b+1)), then [d', vd) when d' < vd.  One warp per row; `out` has n_ck
+// entries and is written by lane 0; every lane returns the last of them.
+__device__ __forceinline__ float chain_norms_row(const float* __restrict__ row, uint32_t partial_d, uint32_t vertical_d, uint32_t horizontal_d, int lane, float* out,
+                                                size_t out_stride = 1) {
+    float cum = 0.f;
+    uint32_t ck = 0;
+    {
+        float s = 0.f;
+        for (uint32_t j = lane; j < partial_d; j += 32) s = fmaf(__ldg(row + j), __ldg(row + j), s);
+        cum += warp_sum(s);
+        if (lane == 0) out[ck * out_stride] = cum;
+        ++ck;
+    }
+    for (uint32_t h = 0; h < horizontal_d; h += kHBlock) {
+        const float a = __ldg(row + vertical_d + h + lane), b = __ldg(row + vertical_d + h + 32 + lane);
+        cum += warp_sum(fmaf(a, a, b * b));
+        if (lane == 0) out[ck * out_stride] = cum;
+        ++ck;
+    }
+    if (partial_d < vertical_d) {
+        float s = 0.f;
+        for (uint32_t j = partial_d + lane; j < vertical_d; j += 32) s = fmaf(__ldg(row + j), __ldg(row + j), s);
+        cum += warp_sum(s);
+        if (lane == 0) out[ck * out_stride] = cum;
+    }
+    return cum;
+}
+
 } // namespace skmb

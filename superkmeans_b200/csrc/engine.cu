@@ -511,39 +511,50 @@ int prune_split_mode() { return g_prune_split_mode; }
 
 namespace {
 
-// The centroids' side of run_listed_dense.
-void prepare_listed_dense(const PrunedParams& p, PruneSplitWorkspace& ws, PrunePassBuffers& b, cudaStream_t stream) {
-    launch_chain_norms(p.y, p.k, p.d, p.partial_d, p.vertical_d, p.horizontal_d, true, ws.chain_norms_y, stream);
-    tc::launch_presplit(p.y, p.k, p.d, b.y_split.ensure(2 * p.k * p.d), stream);
+tc::ChainShape chain_shape(const PrunedParams& p) { return {static_cast<uint32_t>(p.d), p.partial_d, p.vertical_d, p.horizontal_d}; }
+
+// Points whose halves the chain has at a time: about a gigabyte of them, a whole number of tiles of 256 for every pair of SMs.
+size_t chain_slice(const tc::ChainShape& shape, size_t n) {
+    constexpr size_t step = 74 * 256;
+    return std::min(n, std::max<size_t>(1, (size_t{1} << 30) / (2 * sizeof(__half) * shape.pitch()) / step) * step);
 }
 
-// The points listed in ws.hard_idx through the dense chain on the tensor cores, over a gathered copy of their rows
-// (prepare_listed_dense has run).  With a `side` stream on that one, from where `stream` stands; the caller joins them
-// (b.side_done).  `beside` is called when the chain is on its way.
-void run_listed_dense(const PrunedParams& p, PruneSplitWorkspace& ws, PrunePassBuffers& b, size_t n_listed, cudaStream_t stream, cudaStream_t side = nullptr,
-                      const std::function<void()>& beside = nullptr) {
-    if (n_listed == 0) return;
-    const uint32_t n_ck = prune_chain_checkpoints(p.partial_d, p.vertical_d, p.horizontal_d);
-    float* xl = b.listed_x.ensure(n_listed * p.d);
-    float* bestl = b.listed_best.ensure(n_listed);
-    uint32_t* knnl = b.listed_knn.ensure(n_listed);
-    float* normsl = b.listed_norms.ensure(n_listed * n_ck);
-    float* distl = b.listed_dist.ensure(n_listed);
-    uint32_t* npl = b.listed_np.ensure(n_listed);
-    uint2* top2l = b.listed_top2.ensure(n_listed);
+// The centroids' side of run_dense.
+void prepare_dense(const PrunedParams& p, PruneSplitWorkspace& ws, PrunePassBuffers& b, cudaStream_t stream) {
+    tc::launch_chain_centroids(p.y, p.k, chain_shape(p), b.chain_centroids(p.k, chain_shape(p), ws.chain_norms_y), stream);
+}
+
+// The points idx[0 .. n) (idx null: 0 .. n) through the dense chain on the tensor cores (prepare_dense has run).  With a `side` stream on that
+// one, from where `stream` stands; the caller joins them (b.side_done).  `beside` is called when the chain is on its way.
+void run_dense(const PrunedParams& p, PruneSplitWorkspace& ws, PrunePassBuffers& b, const uint32_t* idx, size_t n, cudaStream_t stream, cudaStream_t side = nullptr,
+               const std::function<void()>& beside = nullptr) {
+    if (n == 0) return;
+    const tc::ChainShape shape = chain_shape(p);
+    const size_t slice = chain_slice(shape, n);
+    const tc::ChainHalves xs = b.chain_points(slice, shape), ys = b.chain_centroids(p.k, shape, ws.chain_norms_y);
+    float* bestl = idx ? b.listed_best.ensure(slice) : nullptr;
+    uint32_t* knnl = idx ? b.listed_knn.ensure(slice) : nullptr;
+    float* distl = b.listed_dist.ensure(slice);
+    uint32_t* npl = idx ? b.listed_np.ensure(slice) : nullptr;
+    uint2* top2 = b.listed_top2.ensure(slice);
     // Several blocks per tile shorten the chain but take SMs from the walk beside it: not when the walk over all points (about 0.55 ps
     // per point and centroid) takes longer than one tile's chain (0.17 ns per centroid and dimension) anyway.
-    uint8_t* scratch = side && p.n > 300 * p.d ? nullptr : b.chain_scratch.ensure(tc::chain_scratch_bytes(n_listed));
+    uint8_t* scratch = side && p.n > 300 * p.d ? nullptr : b.chain_scratch.ensure(tc::chain_scratch_bytes(slice));
     const cudaStream_t s = side ? side : stream;
     if (side) {
         b.side_start.record(stream);
         b.side_start.hold(side);
     }
-    launch_gather_listed(p.x, ws.best, p.knn, ws.hard_idx, n_listed, p.d, xl, bestl, knnl, s);
-    launch_chain_norms(xl, n_listed, p.d, p.partial_d, p.vertical_d, p.horizontal_d, false, normsl, s);
-    tc::launch_chain(xl, p.y, n_listed, p.k, p.d, p.partial_d, p.vertical_d, p.horizontal_d, normsl, ws.chain_norms_y, p.ratios, bestl, knnl, distl, npl, top2l, b.y_split.get(), scratch,
-                     s, beside);
-    launch_scatter_listed(ws.hard_idx, n_listed, knnl, distl, npl, p.knn, p.dist, p.not_pruned, s);
+    for (size_t r0 = 0; r0 < n; r0 += slice) {
+        const size_t cnt = std::min(slice, n - r0);
+        const float* x = idx ? p.x : p.x + r0 * p.d;
+        const uint32_t* at = idx ? idx + r0 : nullptr;
+        uint32_t* knn = idx ? knnl : p.knn + r0;
+        uint32_t* not_pruned = idx ? npl : p.not_pruned + r0;
+        tc::launch_chain_points(x, at, ws.best, p.knn, cnt, shape, xs, bestl, knnl, s);
+        tc::launch_chain(cnt, p.k, shape, xs, ys, p.ratios, idx ? bestl : ws.best + r0, knn, distl, not_pruned, top2, scratch, s, r0 == 0 ? beside : nullptr);
+        tc::launch_refine_chain(x, p.y, cnt, p.k, p.d, top2, at, knn, not_pruned, idx ? p.knn : knn, idx ? p.dist : p.dist + r0, idx ? p.not_pruned : nullptr, s);
+    }
     if (side) b.side_done.record(side);
 }
 
@@ -1019,10 +1030,8 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
         b.last_n_hard = p.n;
         b.total_dense_rows += p.n;
         Sub sub(timers, PH_PRUNE_DENSE, stream);
-        launch_chain_norms(p.x, p.n, p.d, p.partial_d, p.vertical_d, p.horizontal_d, false, b.chain_norms_x.ensure(p.n * n_ck), stream);
-        prepare_listed_dense(p, ws, b, stream);
-        tc::launch_chain(p.x, p.y, p.n, p.k, p.d, p.partial_d, p.vertical_d, p.horizontal_d, b.chain_norms_x.get(), ws.chain_norms_y, p.ratios, ws.best, p.knn, p.dist,
-                         p.not_pruned, b.top2.ensure(p.n), b.y_split.get(), b.chain_scratch.ensure(tc::chain_scratch_bytes(p.n)), stream);
+        prepare_dense(p, ws, b, stream);
+        run_dense(p, ws, b, nullptr, p.n, stream);
         return;
     }
     p.best_in = ws.best;
@@ -1086,10 +1095,10 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
             cudaStream_t side = nullptr;
             if (mode == 0) {
                 side = side_ends.s = b.side.get();
-                b.y_split.ensure(2 * p.k * p.d);
+                b.chain_centroids(p.k, chain_shape(p), ws.chain_norms_y);
                 b.side_start.record(stream);
                 b.side_start.hold(side);
-                prepare_listed_dense(p, ws, b, side);
+                prepare_dense(p, ws, b, side);
                 b.side_done.record(side);
             }
             for (size_t t0 = 0; t0 < n_tiles; t0 += per_batch) {
@@ -1139,7 +1148,7 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
                     n_hard = host->n_dropped;
                     if (n_hard != 0) {
                         Sub sub(timers, PH_PRUNE_DENSE, side);
-                        run_listed_dense(p, ws, b, n_hard, stream, side, walk);
+                        run_dense(p, ws, b, ws.hard_idx, n_hard, stream, side, walk);
                         continue;
                     }
                 }
@@ -1160,8 +1169,8 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
             if (n_hard != 0) {
                 Sub sub(timers, PH_PRUNE_DENSE, stream);
                 launch_compact_flags(redo, p.n, ws, stream);
-                prepare_listed_dense(p, ws, b, stream);
-                run_listed_dense(p, ws, b, n_hard, stream);
+                prepare_dense(p, ws, b, stream);
+                run_dense(p, ws, b, ws.hard_idx, n_hard, stream);
             }
         }
         b.last_n_hard = n_hard;

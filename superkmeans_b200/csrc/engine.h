@@ -118,6 +118,19 @@ struct PrunePassBuffers {
         const uint32_t pitch = (cols + 7) / 8 * 8;
         return {y_hi.ensure(rows * pitch), y_lo.ensure(rows * pitch), y_factor.ensure(rows + 1), pitch};
     }
+    // the dense chain's (a slice of the) points and its centroids
+    DeviceBuffer<__half> chain_xh, chain_yh;
+    DeviceBuffer<float> chain_xf, chain_yf;
+    tc::ChainHalves chain_points(size_t rows, const tc::ChainShape& shape) {
+        const size_t halves = rows * shape.pitch();
+        __half* h = chain_xh.ensure(2 * halves);
+        return {h, h + halves, chain_xf.ensure(rows), chain_norms_x.ensure(rows * shape.n_seg())};
+    }
+    tc::ChainHalves chain_centroids(size_t k, const tc::ChainShape& shape, float* norms) {
+        const size_t halves = k * shape.pitch();
+        __half* h = chain_yh.ensure(2 * halves);
+        return {h, h + halves, chain_yf.ensure(k), norms};
+    }
     Side side;   // (last: its work ends before any buffer goes)
 };
 // mode: 0 = automatic: with rows that TMA can address, the points are taken in the order of their previous centroid and

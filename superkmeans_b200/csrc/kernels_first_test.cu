@@ -53,24 +53,6 @@ struct TestCtrl {
 };
 static_assert(sizeof(TestCtrl) <= T_CTRL_BYTES, "control block too large");
 
-// pairs of floats
-__device__ __forceinline__ uint64_t pack2(float a, float b) { return static_cast<uint64_t>(__float_as_uint(a)) | static_cast<uint64_t>(__float_as_uint(b)) << 32; }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-
 struct TestMaps {
     CUtensorMap xhi, xlo, yhi, ylo;
 };
@@ -333,16 +315,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T_THREADS, 1) first_
     __syncthreads();
     cluster_sync();   // nothing of the pair is in flight towards this CTA any more
     if (warp == 1) tmem_dealloc_pair(tmem_base, TMEM_COLS);
-}
-
-// Power of two that maps a vector of this squared norm into [-2^14, 2^14]: hi and lo then hold 22 bits of every element down
-// to 2^-17 of the norm, and smaller ones to 2^-39 of it.  At most 2^74, so that the product of two factors is no less than the smallest
-// float.
-__device__ __forceinline__ float split_scale(float sqnorm) {
-    if (!(sqnorm >= FLT_MIN) || !(sqnorm < 3e38f)) return 1.0f;
-    int e;
-    frexpf(sqrtf(sqnorm), &e);
-    return ldexpf(1.0f, min(14 - e, 74));
 }
 
 // Largest ratio of two centroids' squared norms under one scale: a centroid 2^-10 as long as the longest still has its elements

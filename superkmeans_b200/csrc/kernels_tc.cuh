@@ -99,19 +99,40 @@ void role_cycles(unsigned long long out[16]);
 // tensor cores process), for work accounting.
 void launch_build_cols(const uint32_t* union_bits, uint32_t union_words, size_t n_tiles, size_t k, uint16_t* cols, uint32_t* col_counts, size_t cols_stride,
                        unsigned long long* total_cols, cudaStream_t stream);
-// Exact fp32 refinement of the chain's winner and runner-ups (see launch_chain) for the rows of the listed tiles only.
+// Exact fp32 refinement of the chain's winner and runner-ups for the rows of the listed tiles only.
 void launch_refine_chain_tiles(const float* x, const float* y, size_t n, size_t k, size_t d, const uint2* top2, uint32_t* knn, float* dist, const uint32_t* tile_map,
                                size_t n_tiles, cudaStream_t stream);
 
-// Pruned assignment for all n points as a dense ADSampling chain on the tensor cores.  chain_norms_x /
-// chain_norms_y hold, per row, the cumulative squared norm after each of the chain's checkpoints
-// (launch_chain_norms; point norms row-major, centroid norms checkpoint-major); best_in the exact distance to the previous centroid; knn the previous
-// assignment on entry and the new one on return.  The winner is settled, and its distance recomputed, in
-// fp32 among the chain's winner and its two runner-ups (top2_scratch: n entries).
+// Order of the columns of a row in the dense ADSampling chain (kernels_chain.cu): the first d' dimensions, the horizontal ones in segments of
+// 64, the remaining vertical ones; every segment starts at a multiple of 64.
+struct ChainShape {
+    uint32_t d, partial_d, vertical_d, horizontal_d;
+    __host__ __device__ uint32_t n_seg() const { return 1u + horizontal_d / 64u + (partial_d < vertical_d ? 1u : 0u); }
+    __host__ __device__ uint32_t begin(uint32_t seg) const { return seg == 0 ? 0u : (partial_d + 63u) / 64u * 64u + (seg - 1u) * 64u; }   // (the tail behind the last of 64)
+    __host__ __device__ uint32_t length(uint32_t seg) const { return seg == 0 ? partial_d : (seg <= horizontal_d / 64u ? 64u : vertical_d - partial_d); }
+    __host__ __device__ uint32_t dims_after(uint32_t seg) const { return seg <= horizontal_d / 64u ? partial_d + seg * 64u : d; }
+    __host__ __device__ uint32_t pitch() const { return begin(1) + horizontal_d + (vertical_d - partial_d + 63u) / 64u * 64u; }
+};
+// Rows in that order as fp16 pairs (see SplitHalves), with factors and cumulative squared norms after every segment.
+struct ChainHalves {
+    __half* hi;      // rows x pitch
+    __half* lo;
+    float* factor;   // -2 / scale of a point, 1 / scale of a centroid
+    float* norms;    // points: rows x n_seg; centroids: n_seg x rows
+};
+// Points idx[i] of x, or with idx null the first n; with idx best_out[i] and knn_out[i] are theirs.  Rows are 16-byte aligned.
+void launch_chain_points(const float* x, const uint32_t* idx, const float* best, const uint32_t* knn, size_t n, const ChainShape& shape, const ChainHalves& out, float* best_out,
+                         uint32_t* knn_out, cudaStream_t stream);
+void launch_chain_centroids(const float* y, size_t k, const ChainShape& shape, const ChainHalves& out, cudaStream_t stream);
+
+// Pruned assignment of n points as a dense chain on the tensor cores.  best_in: exact distance to the previous centroid; knn: the previous
+// assignment on entry and the chain's winner on return, which launch_refine_chain settles among it and its two runner-ups (top2).
 size_t chain_scratch_bytes(size_t n);   // of `scratch` below (optional: lets a few rows have several blocks per tile); may be none
-void launch_chain(const float* x, const float* y, size_t n, size_t k, size_t d, uint32_t partial_d, uint32_t vertical_d, uint32_t horizontal_d, const float* chain_norms_x,
-                  const float* chain_norms_y, const float* ratios, const float* best_in, uint32_t* knn, float* dist, uint32_t* not_pruned, uint2* top2_scratch,
-                  const float* y_split, void* scratch, cudaStream_t stream, const std::function<void()>& beside = nullptr);   // y_split: 2 * k * d floats of scratch for the tf32 parts of the centroids
+void launch_chain(size_t n, size_t k, const ChainShape& shape, const ChainHalves& x, const ChainHalves& y, const float* ratios, const float* best_in, uint32_t* knn, float* dist,
+                  uint32_t* not_pruned, uint2* top2, void* scratch, cudaStream_t stream, const std::function<void()>& beside = nullptr);   // called behind the first launch
+// Exact fp32 distances decide among the chain's winner and runner-ups; row i of the chain is row idx[i] of x and of the results, or row i.
+void launch_refine_chain(const float* x, const float* y, size_t n, size_t k, size_t d, const uint2* top2, const uint32_t* idx, const uint32_t* knn, const uint32_t* not_pruned,
+                         uint32_t* knn_out, float* dist_out, uint32_t* not_pruned_out, cudaStream_t stream);
 
 // SM cycles after which a wait inside a tensor-core kernel gives up (about two seconds unless a test shortened it).
 long long wait_limit();

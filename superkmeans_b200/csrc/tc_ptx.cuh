@@ -5,6 +5,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <cfloat>
 #include <cstdint>
 
 namespace skmb {
@@ -270,6 +271,34 @@ __device__ __forceinline__ float to_tf32(float x) {
 __device__ __forceinline__ void split4(float4 v, float4& hi, float4& lo) {
     hi.x = to_tf32(v.x); hi.y = to_tf32(v.y); hi.z = to_tf32(v.z); hi.w = to_tf32(v.w);
     lo.x = to_tf32(v.x - hi.x); lo.y = to_tf32(v.y - hi.y); lo.z = to_tf32(v.z - hi.z); lo.w = to_tf32(v.w - hi.w);
+}
+
+// pairs of floats
+__device__ __forceinline__ uint64_t pack2(float a, float b) { return static_cast<uint64_t>(__float_as_uint(a)) | static_cast<uint64_t>(__float_as_uint(b)) << 32; }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+// Power of two that maps a vector of this squared norm into [-2^14, 2^14]: hi and lo then hold 22 bits of every element down
+// to 2^-17 of the norm, and smaller ones to 2^-39 of it.  At most 2^74, so that the product of two factors is no less than the smallest
+// float.
+__device__ __forceinline__ float split_scale(float sqnorm) {
+    if (!(sqnorm >= FLT_MIN) || !(sqnorm < 3e38f)) return 1.0f;
+    int e;
+    frexpf(sqrtf(sqnorm), &e);
+    return ldexpf(1.0f, min(14 - e, 74));
 }
 
 // Tensor maps (defined in kernels_tc.cu), zero fill outside the matrix.

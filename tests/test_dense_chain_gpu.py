@@ -1,0 +1,35 @@
+"""The dense chain on the tensor cores against the one in fp32, at the edges of its tiles (256 points, units of 256 centroids, chunks of
+1024) and of its segments."""
+import numpy as np
+import pytest
+
+from tests import datagen
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,k,d", [(1, 300, 132), (127, 257, 132), (129, 1_025, 200), (256, 1_024, 128), (257, 256, 260), (4_608, 1_300, 384), (4_609, 2_049, 256), (20_000, 513, 1_000),
+                                   (700, 5, 768), (700, 3_000, 1_540)])
+def test_chain_on_the_tensor_cores(n, k, d):
+    from superkmeans_b200 import engine
+
+    x = datagen.gaussian_mixture(n, d, max(k // 4, 1), 0.4, n + k)
+    y = datagen.gaussian_mixture(k, d, max(k // 4, 1), 0.4, k)
+    # rows of different magnitudes: every row has a scale of its own
+    x *= (10.0 ** np.random.default_rng(n).uniform(-3, 3, (n, 1))).astype(np.float32)
+    prev = np.random.default_rng(d).integers(0, k, n).astype(np.uint32)
+    vertical = engine.dimension_split(d)[1]
+    for partial in {16, vertical // 2, vertical - 3, vertical}:
+        out = {}
+        for mode in (2, 3):
+            engine.set_prune_split(mode)
+            try:
+                out[mode] = engine.find_nearest_pruned(x, y, prev, partial)
+            finally:
+                engine.set_prune_split(0)
+        knn, dist = out[3][0], out[3][1]
+        exact = ((x.astype(np.float64) - y[knn].astype(np.float64)) ** 2).sum(1)
+        assert (np.abs(dist - exact) <= 1e-5 * exact + 1e-12).all()
+        # pairs within rounding of a threshold of the search
+        assert (knn == out[2][0]).mean() >= 0.999 - 1.0 / n
+        assert abs(float(out[3][2].sum()) - float(out[2][2].sum())) <= 1e-3 * float(out[2][2].sum()) + 2
