@@ -400,7 +400,7 @@ size_t Engine::streamed_rows(size_t n) const {
     return std::min(chunk_rows_for(d_, n), std::max(least, (n + 3) / 4));
 }
 
-// Exact assignment of device rows: knn, dist, and the full norms of both sides.
+// Exact assignment of device rows: knn, dist (may be null: rows with one candidate are then not read again), and the full norms of both sides.
 void Engine::exact_assignment(const float* x, size_t n, const float* c, size_t k, float* norms_x, bool norms_known, float* norms_c, uint32_t* knn, float* dist) {
     const AssignRoute route = assign_route(n, k, d_);
     if (route == AssignRoute::filter && exact_.begin(c, k, d_, n, n, norms_c, stream_)) {
@@ -408,6 +408,8 @@ void Engine::exact_assignment(const float* x, size_t n, const float* c, size_t k
         exact_.settle_on_device(x, knn, dist, stream_);
         return;
     }
+    DeviceBuffer<float> own;
+    if (!dist) dist = own.ensure(n);
     if (route == AssignRoute::direct) {
         direct_.run(x, c, n, k, d_, norms_x, norms_c, knn, dist, stream_);
         return;
@@ -1854,10 +1856,10 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
     }
     cn.ensure(n_centroids);
     if (on_device) {
-        DeviceBuffer<float> xn, dist;
+        DeviceBuffer<float> xn;
         {
             PhaseScope ps(*this, PH_ASSIGN_FULL);
-            exact_assignment(vectors, n, c_dev, n_centroids, xn.ensure(n), false, cn.get(), out, dist.ensure(n));
+            exact_assignment(vectors, n, c_dev, n_centroids, xn.ensure(n), false, cn.get(), out, nullptr);
         }
         // (a direct call waits for nothing that can run out)
         const bool direct_call = assign_route(n, n_centroids, d_) == AssignRoute::direct;
@@ -1887,7 +1889,7 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
         if (filtered && r0 == rows && n * d_ * sizeof(float) >= kAskFrom && exact_.in_vain(r0, stream_)) filtered = false;
         pipe.arrive();
         if (filtered) {
-            exact_.rows(xb, r0, cnt, xn.get(), knn.get() + r0, dist.get(), stream_);
+            exact_.rows(xb, r0, cnt, xn.get(), knn.get() + r0, nullptr, stream_);
         } else if (direct) {
             direct_.run(xb, c_dev, cnt, n_centroids, d_, xn.get(), cn.get(), knn.get() + r0, dist.get(), stream_);
         } else {

@@ -141,7 +141,8 @@ constexpr uint32_t kSeenRows = 4096;
 __device__ __forceinline__ bool hopeless(const uint32_t* n_listed, size_t rows_before) { return rows_before >= kSeenRows && 2 * static_cast<size_t>(*n_listed) > rows_before; }
 
 // Per row: fp16 copy, norm, and {squared norm minus the mean, squared norm of the rounding error, squared norm, scale}.
-template <bool VEC>
+// With U the row is read once, all of it in flight (rows of at most 128 U columns, VEC); without, twice.
+template <bool VEC, int U>
 __global__ void __launch_bounds__(256) row_fp16_kernel(const float* __restrict__ x, size_t n, size_t d, size_t dp, const float* __restrict__ mean, float* __restrict__ norms,
                                                        __half* __restrict__ out, float4* __restrict__ info, const uint32_t* __restrict__ n_listed, size_t rows_before,
                                                        uint32_t* __restrict__ unseen) {
@@ -151,13 +152,52 @@ __global__ void __launch_bounds__(256) row_fp16_kernel(const float* __restrict__
     if (row >= n) return;
     const int lane = threadIdx.x & 31;
     const float* xr = x + row * d;
-    const RowNorms nx = row_norms<VEC>(xr, mean, d, lane);
+    RowNorms nx;
+    [[maybe_unused]] float4 v[U > 0 ? U : 1];
+    if constexpr (U > 0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] = 4 * lane + 128 * u < d ? __ldg(reinterpret_cast<const float4*>(xr + 4 * lane + 128 * u)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float a = 0.f, b = 0.f;   // (in the order of row_norms)
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (4 * lane + 128 * u < d) {
+                const float4 m = __ldg(reinterpret_cast<const float4*>(mean + 4 * lane + 128 * u));
+                a = fmaf(v[u].x, v[u].x, a); a = fmaf(v[u].y, v[u].y, a); a = fmaf(v[u].z, v[u].z, a); a = fmaf(v[u].w, v[u].w, a);
+                v[u] = make_float4(v[u].x - m.x, v[u].y - m.y, v[u].z - m.z, v[u].w - m.w);
+                b = fmaf(v[u].x, v[u].x, b); b = fmaf(v[u].y, v[u].y, b); b = fmaf(v[u].z, v[u].z, b); b = fmaf(v[u].w, v[u].w, b);
+            }
+        }
+        nx = {warp_sum(a), warp_sum(b)};
+    } else {
+        nx = row_norms<VEC>(xr, mean, d, lane);
+    }
     if (give_up) {
         if (lane == 0) norms[row] = nx.plain;
         return;
     }
     const float scale = fp16_scale(nx.centred);
-    const float err = write_fp16_row<VEC>(xr, mean, d, dp, scale, out + row * dp, lane);
+    float err;
+    if constexpr (U > 0) {
+        const float inv = 1.0f / scale;
+        err = 0.f;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (4 * lane + 128 * u < dp) {
+                const float t[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+                __align__(8) __half h[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    h[q] = __float2half_rn(t[q] * scale);
+                    const float r = fmaf(-__half2float(h[q]), inv, t[q]);
+                    err = fmaf(r, r, err);
+                }
+                *reinterpret_cast<uint2*>(out + row * dp + 4 * lane + 128 * u) = *reinterpret_cast<const uint2*>(h);
+            }
+        }
+        err = warp_sum(err);
+    } else {
+        err = write_fp16_row<VEC>(xr, mean, d, dp, scale, out + row * dp, lane);
+    }
     if (lane != 0) return;
     norms[row] = nx.plain;
     info[row] = make_float4(nx.centred, err, nx.plain, scale);
@@ -252,6 +292,13 @@ struct Best {
     }
 };
 
+// Columns of a column tile that are multiplied, half of them by the centroids of either CTA.  Groups of few centroids leave most of a tile
+// empty (300 000 x 768 rows, groups of 50: 110 us a pass with whole tiles, 90 so); without groups it is the last tile at most.
+template <bool GROUPED>
+__device__ __forceinline__ uint32_t filter_columns(uint32_t k, uint32_t nt) {
+    return GROUPED ? min(256u, (k - nt * 256 + 31) / 32 * 32) : 256u;
+}
+
 template <bool GROUPED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(F_THREADS, 1)
     filter_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_y, const FilterParams p) {
@@ -317,7 +364,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(F_THREADS, 1)
                 const uint32_t col_tiles = (tile.k + 255) / 256;
                 const int x_row = static_cast<int>(tile.row0 + rank * 128);
                 for (uint32_t nt = 0; nt < col_tiles && ok; ++nt) {
-                    const int y_row = static_cast<int>(tile.y0 + nt * 256 + rank * 128);
+                    const int y_row = static_cast<int>(tile.y0 + nt * 256 + rank * (filter_columns<GROUPED>(tile.k, nt) / 2));
                     for (uint32_t kb = 0; kb < p.k_blocks; ++kb, ++kbt) {
                         const uint32_t s = kbt % F_STAGES, ph = (kbt / F_STAGES) & 1u;
                         if ((p.producer_stop != 0 && kbt >= p.producer_stop) || !mbar_wait(&ctrl->empty[s], ph ^ 1u, wctx, 41)) {
@@ -341,13 +388,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(F_THREADS, 1)
         }
     } else if (warp == 1) {
         if (lane == 0 && rank == 0) {
-            constexpr uint32_t idesc = make_idesc_f16(256, 256);
             uint32_t kbt = 0, t = 0;
             bool ok = true;
             for (size_t rt = pair; rt < n_row_tiles && ok; rt += n_pairs) {
-                const uint32_t col_tiles = (tile_at(rt).k + 255) / 256;
+                const uint32_t k = tile_at(rt).k, col_tiles = (k + 255) / 256;
                 for (uint32_t nt = 0; nt < col_tiles && ok; ++nt, ++t) {
-                    const uint32_t b = t & 1u, tph = (t >> 1) & 1u;
+                    const uint32_t b = t & 1u, tph = (t >> 1) & 1u, idesc = make_idesc_f16(256, filter_columns<GROUPED>(k, nt));
                     if (!mbar_wait(&ctrl->acc_empty[b], tph ^ 1u, wctx, 42)) {
                         ok = false;
                         break;
@@ -440,6 +486,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(F_THREADS, 1)
                 };
                 uint32_t ra[32], rb[32];
                 const int slice0 = static_cast<int>(half) * 4;
+                auto give_back = [&] {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster_read(cluster_address(&ctrl->acc_empty[b], 0));
+                };
+                if (GROUPED && filter_columns<GROUPED>(tile.k, nt) != 256) {
+                    // only the columns that were multiplied: what stands in the others is older
+                    const int end = min(slice0 + 4, static_cast<int>(filter_columns<GROUPED>(tile.k, nt) / 32));
+#pragma unroll 1
+                    for (int ch = slice0; ch < end; ++ch) {
+                        tmem_ld32_issue(taddr + ch * 32, ra);
+                        tmem_ld_wait(ra);
+                        look(ra, ch);
+                    }
+                    give_back();
+                    continue;
+                }
                 tmem_ld32_issue(taddr + slice0 * 32, ra);
                 tmem_ld_wait(ra);
 #pragma unroll 1
@@ -447,13 +510,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(F_THREADS, 1)
                     tmem_ld32_issue(taddr + (ch + 1) * 32, rb);
                     look(ra, ch);
                     tmem_ld_wait(rb);
-                    if (ch == slice0) {
-                        tmem_ld32_issue(taddr + (ch + 2) * 32, ra);
-                    } else {
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive_cluster_read(cluster_address(&ctrl->acc_empty[b], 0));
-                    }
+                    if (ch == slice0) tmem_ld32_issue(taddr + (ch + 2) * 32, ra);
+                    else give_back();
                     look(rb, ch + 1);
                     if (ch == slice0) tmem_ld_wait(ra);
                 }
@@ -497,83 +555,117 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(F_THREADS, 1)
 
 // The decision: fp32 distances of a row's candidates, one warp per row (see refine_top2_kernel, whose sums, ties and
 // clamping these are).
+// What bounds it is the latency of its loads, one behind the other for a row (candidates, centroids), so a warp asks for the next row's
+// candidates and its first 512 columns before it decides the present one.
 template <bool VEC>
-__global__ void __launch_bounds__(256) decide_kernel(const float* __restrict__ x, const float* __restrict__ y, size_t n, size_t k, size_t d, const float* __restrict__ norms_x,
+__global__ void __launch_bounds__(256, 3) decide_kernel(const float* __restrict__ x, const float* __restrict__ y, size_t n, size_t k, size_t d, const float* __restrict__ norms_x,
                                                      const float* __restrict__ norms_y, const uint4* __restrict__ cand, uint32_t* __restrict__ out_knn, float* __restrict__ out_dist,
                                                      const int* __restrict__ error) {
-    const size_t row = static_cast<size_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
-    if (row >= n) return;
     if (*reinterpret_cast<const volatile int*>(error) != 0) return;   // the candidates were not written
     const int lane = threadIdx.x & 31;
-    const uint4 c4 = cand[row];
-    if (c4.x >= k) return;   // listed
-    const uint32_t c[4] = {c4.x, c4.y, c4.z, c4.w};
-    const int count = c4.y >= k ? 1 : (c4.z >= k ? 2 : (c4.w >= k ? 3 : 4));
-    const float* xr = x + row * d;
-    const float* yr[4];
+    constexpr int U = 4;
+    const size_t step = static_cast<size_t>(gridDim.x) * 8;
+    float4 v[U], v_next[U];
+    uint4 c_next = make_uint4(~0u, ~0u, ~0u, ~0u);
+    auto load_point = [&](float4 (&to)[U], size_t row, size_t j0) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) yr[q] = y + static_cast<size_t>(q < count ? c[q] : c[0]) * d;
-    float s[4] = {0.f, 0.f, 0.f, 0.f};
-    if (VEC) {
-        for (size_t j = static_cast<size_t>(lane) * 4; j < d; j += 128) {
-            const float4 v = __ldg(reinterpret_cast<const float4*>(xr + j));
+        for (int u = 0; u < U; ++u) to[u] = j0 + 128 * u < d ? __ldg(reinterpret_cast<const float4*>(x + row * d + j0 + 128 * u)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    auto ask = [&](size_t row) {
+        if (row >= n) return;
+        c_next = __ldg(cand + row);
+        if (VEC && out_dist) load_point(v_next, row, 4 * lane);
+    };
+    size_t row = static_cast<size_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+    ask(row);
+    for (; row < n; row += step) {
+        const uint4 c4 = c_next;
+        if (VEC && out_dist) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                if (q < count) {
-                    const float4 w = __ldg(reinterpret_cast<const float4*>(yr[q] + j));
-                    s[q] = fmaf(v.x, w.x, s[q]); s[q] = fmaf(v.y, w.y, s[q]); s[q] = fmaf(v.z, w.z, s[q]); s[q] = fmaf(v.w, w.w, s[q]);
+            for (int u = 0; u < U; ++u) v[u] = v_next[u];
+        }
+        ask(row + step);
+        if (c4.x >= k) continue;   // listed
+        const uint32_t c[4] = {c4.x, c4.y, c4.z, c4.w};
+        const int count = c4.y >= k ? 1 : (c4.z >= k ? 2 : (c4.w >= k ? 3 : 4));
+        if (count == 1 && !out_dist) {
+            if (lane == 0) out_knn[row] = c4.x;
+            continue;
+        }
+        const float* xr = x + row * d;
+        if (VEC && !out_dist) load_point(v, row, 4 * lane);
+        const float* yr[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) yr[q] = y + static_cast<size_t>(q < count ? c[q] : c[0]) * d;
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
+        if (VEC) {
+            for (size_t j0 = static_cast<size_t>(lane) * 4; j0 < d; j0 += 128 * U) {
+                if (j0 >= 128 * U) load_point(v, row, j0);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (q < count) {
+                        float4 w[U];
+#pragma unroll
+                        for (int u = 0; u < U; ++u) w[u] = j0 + 128 * u < d ? __ldg(reinterpret_cast<const float4*>(yr[q] + j0 + 128 * u)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            if (j0 + 128 * u < d) {
+                                s[q] = fmaf(v[u].x, w[u].x, s[q]); s[q] = fmaf(v[u].y, w[u].y, s[q]); s[q] = fmaf(v[u].z, w[u].z, s[q]); s[q] = fmaf(v[u].w, w[u].w, s[q]);
+                            }
+                        }
+                    }
                 }
             }
-        }
-    } else {
-        for (size_t j = lane; j < d; j += 32) {
-            const float v = __ldg(xr + j);
+        } else {
+            for (size_t j = lane; j < d; j += 32) {
+                const float xv = __ldg(xr + j);
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (q < count) s[q] = fmaf(v, __ldg(yr[q] + j), s[q]);
-        }
-    }
-    const float nx = norms_x[row];
-    float e[4];
-    float lowest = FLT_MAX;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        e[q] = FLT_MAX;
-        if (q < count) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
-            e[q] = fmaf(-2.0f, s[q], nx) + norms_y[c[q]];
-            lowest = fminf(lowest, e[q]);
-        }
-    }
-    // near-ties are settled with dot products accumulated in index order, a lane for each
-    int close = 0;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) close += (q < count && fabsf(e[q] - lowest) <= 1e-4f * fmaxf(fabsf(e[q]), fabsf(lowest))) ? 1 << q : 0;
-    if (__popc(close) > 1) {
-        float t = 0.f;
-        if (lane < 4 && ((close >> lane) & 1)) {
-            const float* yl = lane == 0 ? yr[0] : (lane == 1 ? yr[1] : (lane == 2 ? yr[2] : yr[3]));
-            for (size_t j = 0; j < d; ++j) t = fmaf(xr[j], yl[j], t);
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const float tq = __shfl_sync(0xffffffffu, t, q);
-            if ((close >> q) & 1) e[q] = fmaf(-2.0f, tq, nx) + norms_y[c[q]];
-        }
-    }
-    if (lane == 0) {
-        float be = e[0];
-        uint32_t bi = c[0];
-#pragma unroll
-        for (int q = 1; q < 4; ++q) {
-            if (q < count && (e[q] < be || (e[q] == be && c[q] < bi))) {
-                be = e[q];
-                bi = c[q];
+                for (int q = 0; q < 4; ++q)
+                    if (q < count) s[q] = fmaf(xv, __ldg(yr[q] + j), s[q]);
             }
         }
-        out_knn[row] = bi;
-        out_dist[row] = fmaxf(0.0f, be);
+        const float nx = norms_x[row];
+        float e[4];
+        float lowest = FLT_MAX;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            e[q] = FLT_MAX;
+            if (q < count) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
+                e[q] = fmaf(-2.0f, s[q], nx) + norms_y[c[q]];
+                lowest = fminf(lowest, e[q]);
+            }
+        }
+        // near-ties are settled with dot products accumulated in index order, a lane for each
+        int close = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) close += (q < count && fabsf(e[q] - lowest) <= 1e-4f * fmaxf(fabsf(e[q]), fabsf(lowest))) ? 1 << q : 0;
+        if (__popc(close) > 1) {
+            float t = 0.f;
+            if (lane < 4 && ((close >> lane) & 1)) {
+                const float* yl = lane == 0 ? yr[0] : (lane == 1 ? yr[1] : (lane == 2 ? yr[2] : yr[3]));
+                for (size_t j = 0; j < d; ++j) t = fmaf(xr[j], yl[j], t);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float tq = __shfl_sync(0xffffffffu, t, q);
+                if ((close >> q) & 1) e[q] = fmaf(-2.0f, tq, nx) + norms_y[c[q]];
+            }
+        }
+        if (lane == 0) {
+            float be = e[0];
+            uint32_t bi = c[0];
+#pragma unroll
+            for (int q = 1; q < 4; ++q) {
+                if (q < count && (e[q] < be || (e[q] == be && c[q] < bi))) {
+                    be = e[q];
+                    bi = c[q];
+                }
+            }
+            out_knn[row] = bi;
+            if (out_dist) out_dist[row] = fmaxf(0.0f, be);
+        }
     }
 }
 
@@ -779,7 +871,7 @@ void ExactAssign::centroids(const float* y, size_t k, float* norms_y, bool with_
 
 // (before: rows of the batch that have gone through the filter already)
 void ExactAssign::convert(const float* x, size_t n, size_t before, float* norms_x, cudaStream_t stream) {
-    auto* kernel = aligned16(x, d_) ? row_fp16_kernel<true> : row_fp16_kernel<false>;
+    auto* kernel = !aligned16(x, d_) ? row_fp16_kernel<false, 0> : d_ <= 512 ? row_fp16_kernel<true, 4> : d_ <= 1024 ? row_fp16_kernel<true, 8> : row_fp16_kernel<true, 0>;
     kernel<<<warps_grid(n), 256, 0, stream>>>(x, n, d_, dp_, mean_.get(), norms_x, xh_.get(), row_info_.get(), n_listed_.get(), before, n_listed_.get() + 1);
     SKM_LAUNCH_CHECK();
 }
@@ -813,8 +905,9 @@ void ExactAssign::search(const float* x, size_t first, size_t n, const AssignTil
     SKM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(F_SMEM_BYTES)));
     kernel<<<grid, F_THREADS, F_SMEM_BYTES, stream>>>(tx, ty, p);
     SKM_LAUNCH_CHECK();
-    if (aligned16(x, d_) && aligned16(y_, d_)) decide_kernel<true><<<warps_grid(n), 256, 0, stream>>>(x, y_, n, k_, d_, norms_x, norms_y_, cand_.get(), out_knn, out_dist, p.error);
-    else decide_kernel<false><<<warps_grid(n), 256, 0, stream>>>(x, y_, n, k_, d_, norms_x, norms_y_, cand_.get(), out_knn, out_dist, p.error);
+    const unsigned deciders = std::min<unsigned>(warps_grid(n), static_cast<unsigned>(sms) * 3);
+    auto* decide = aligned16(x, d_) && aligned16(y_, d_) ? decide_kernel<true> : decide_kernel<false>;
+    decide<<<deciders, 256, 0, stream>>>(x, y_, n, k_, d_, norms_x, norms_y_, cand_.get(), out_knn, out_dist, p.error);
     SKM_LAUNCH_CHECK();
 }
 
@@ -862,7 +955,7 @@ void ExactAssign::rows(const float* x, size_t first, size_t n, float* norms_x, u
     for (size_t r0 = 0; r0 < n; r0 += cnt) {
         cnt = std::min({per, n - r0, r0 == 0 ? look : per});
         convert(x + r0 * d_, cnt, first + r0, norms_x + r0, stream);
-        search(x + r0 * d_, first + r0, cnt, nullptr, 0, norms_x + r0, out_knn + r0, out_dist + r0, stream);
+        search(x + r0 * d_, first + r0, cnt, nullptr, 0, norms_x + r0, out_knn + r0, out_dist ? out_dist + r0 : nullptr, stream);
     }
 }
 
