@@ -149,6 +149,7 @@ struct PrunedParams {
     const uint32_t* skip = nullptr;     // optional: 1 = leave this point to the dense kernel
     bool same_points = false;           // x holds what it held in the pass before (its fp16 halves can be used again), in which
     double survival = 0.0;              // this share of the pairs passed the first test (says what a sample says otherwise)
+    float* norms_todo = nullptr;        // norms_x, if the pass has to make them
 };
 
 // Work split of one pruned pass.  Points whose ADSampling test would keep a large share of the
@@ -182,7 +183,8 @@ struct PrunePassCounters {
 size_t prune_split_positions_elems(size_t n);
 uint32_t prune_chain_checkpoints(uint32_t partial_d, uint32_t vertical_d, uint32_t horizontal_d);
 // out[i] = ||x_i - y_{knn[i]}||^2 accumulated directly in fp32 (no norm trick)
-void launch_exact_dist(const float* x, const float* y, const uint32_t* knn, size_t n, size_t d, float* out, cudaStream_t stream);
+// with norms, norms[i] = squared norm of the first `upto` values of row i (what launch_row_sqnorms computes, without reading the rows once more)
+void launch_exact_dist(const float* x, const float* y, const uint32_t* knn, size_t n, size_t d, float* out, cudaStream_t stream, size_t upto = 0, float* norms = nullptr);
 // Cumulative squared norm of every row of m after each checkpoint of the chain: out[row][j], or
 // out[j][row] when `transposed`.
 void launch_chain_norms(const float* m, size_t rows, size_t d, uint32_t partial_d, uint32_t vertical_d, uint32_t horizontal_d, bool transposed, float* out,

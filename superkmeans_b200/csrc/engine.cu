@@ -943,7 +943,13 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
     if (!p.same_points) b.x_halves_valid = false;
     int mode = g_prune_split_mode;
     const bool auto_mode = mode == 0;
+    // The norms, unless the pass that looks at every row anyway makes them on the way (1M x 1024: 0.2 ms a time).
+    auto norms_now = [&] {
+        if (p.norms_todo) launch_row_sqnorms(p.x, p.n, p.d, p.partial_d, p.norms_todo, stream);
+        p.norms_todo = nullptr;
+    };
     if (((mode >= 6 && mode <= 8) || mode == 10 || mode == 11) && tc::eligible(p.x, p.d, p.y, p.d)) {
+        norms_now();
         run_pruned_pass_sorted(p, b, ratio_first, device, stream, timers, mode);
         return;
     }
@@ -983,6 +989,7 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
     };
     if (mode == 0 && tc_ok && p.same_points && ordered(p.survival)) {
         b.last_survival = p.survival;
+        norms_now();
         run_pruned_pass_sorted(p, b, ratio_first, device, stream, timers, 10);
         return;
     }
@@ -991,10 +998,11 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
     if (mode == 0) {
         double survival = p.survival;
         if (tc_ok) {
-            launch_exact_dist(p.x, p.y, p.knn, p.n, p.d, ws.best, stream);
+            launch_exact_dist(p.x, p.y, p.knn, p.n, p.d, ws.best, stream, p.partial_d, p.norms_todo);
             // Which route is a question of the average only: points of about two tiles per SM answer it.
             if (!p.same_points) launch_classify(p, ws, stream, ((p.n + kTileM - 1) / kTileM + 295) / 296);
         } else {
+            norms_now();
             launch_pruned_prepare(p, ws, stream);
         }
         if (!tc_ok || !p.same_points) {
@@ -1014,11 +1022,13 @@ void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, 
         use_chain = tc_ok && survival > 0.08;
         use_tc_lists = tc_ok && !use_chain;
     } else if (mode == 3) {
+        norms_now();
         launch_exact_dist(p.x, p.y, p.knn, p.n, p.d, ws.best, stream);
         if (!tc_ok) throw std::invalid_argument("the tensor-core chain needs 16-byte aligned rows (d % 4 == 0)");
         use_chain = true;
     } else {
         const bool dense = mode == 2;
+        norms_now();
         launch_exact_dist(p.x, p.y, p.knn, p.n, p.d, ws.best, stream);
         use_tc_lists = mode == 4 || mode == 5;
         if (use_tc_lists && !tc_ok) throw std::invalid_argument("the tensor-core first test needs 16-byte aligned rows (d % 4 == 0)");
@@ -1221,6 +1231,8 @@ PrunedParams Engine::pruned_params(const IterationInput& in) {
     p.horizontal_d = horizontal_d_;
     p.same_points = in.pruned_before;
     p.survival = in.survival;
+    if (!in.partial_norms) p.norms_todo = in.norms;
+    in.partial_norms = true;
     return p;
 }
 
@@ -1296,7 +1308,7 @@ void Engine::run_iteration(bool gemm_only, const IterationInput& in, size_t iter
             if (exact_open_) exact_.settle_on_device(in.x, assignments_.get(), distances_.get(), stream_);
             exact_open_ = false;
         } else {
-            exact_assignment(in.x, n, c_prev_.get(), k_cur, norms, true, centroid_norms_.get(), assignments_.get(), distances_.get());
+            exact_assignment(in.x, n, c_prev_.get(), k_cur, norms, in.full_norms, centroid_norms_.get(), assignments_.get(), distances_.get());
         }
     } else {
         launch_row_sqnorms(c_prev_.get(), k_cur, d_, partial_d_, centroid_norms_.get(), stream_);
@@ -1331,10 +1343,7 @@ void Engine::run_iteration(bool gemm_only, const IterationInput& in, size_t iter
                                             cfg_.adjustment_factor_for_partial_d);
         avg_not_pruned = t.avg_not_pruned_pct;
         partial_d_ = t.new_partial_d;
-        if (t.changed) {
-            PhaseScope ps(*this, PH_NORMS);
-            launch_row_sqnorms(in.x, n, d_, partial_d_, norms, stream_);
-        }
+        if (t.changed) in.partial_norms = false;
         in.pruned_before = true;
         in.survival = told.not_pruned / (static_cast<double>(in.n_samples_global) * static_cast<double>(k_cur));
     }
@@ -1514,26 +1523,22 @@ void Engine::train_flat(const float* data, size_t n, bool on_device, const float
     make_centroids();
     sync();
 
-    {
+    IterationInput in{x_rot_.get(), n_samples_, n_samples_global, k_, data_norms_.get()};
+    // (the other ways to assign make the norms they need, and those of the upload are there)
+    in.full_norms = first_assign_done_ || n_queries > 0 || assign_route(n_samples_, k_, d_) == AssignRoute::blocks;
+    if (in.full_norms && !first_assign_done_) {
         PhaseScope ps(*this, PH_NORMS);
         launch_row_sqnorms(x_rot_.get(), n_samples_, d_, d_, data_norms_.get(), stream_);
     }
 
-    // Ground truth for the recall figure (superkmeans.h:243-274): needs the full norms computed just above.
+    // Ground truth for the recall figure (superkmeans.h:243-274): needs the full norms.
     if (n_queries > 0) prepare_recall(queries, n_queries, rotate);
 
     const bool always_gemm_only = d_ < kDimensionThresholdForPruning || cfg_.use_blas_only || k_ <= kNClustersThresholdForPruning;
-    bool partial_norms_computed = false;
     float best_recall = 0.0f;
     size_t iters_without_improvement = 0;
-    IterationInput in{x_rot_.get(), n_samples_, n_samples_global, k_, data_norms_.get()};
     for (size_t iter = 0; iter < cfg_.iters; ++iter) {
         const bool gemm_only = (iter == 0) || always_gemm_only;
-        if (!gemm_only && !partial_norms_computed) {
-            PhaseScope ps(*this, PH_NORMS);
-            launch_row_sqnorms(x_rot_.get(), n_samples_, d_, partial_d_, data_norms_.get(), stream_);
-            partial_norms_computed = true;
-        }
         run_iteration(gemm_only, in, iter, iter == 0, stats_flat_);
         if (cfg_.early_termination &&
             should_stop_early(shift_, cost_, prev_cost_, cfg_.tol, iter, n_queries_ > 0, recall_, cfg_.recall_tol, &best_recall, &iters_without_improvement)) {
@@ -1675,14 +1680,9 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
 
     {
         const bool always_gemm_only = d_ < kDimensionThresholdForPruning || cfg_.use_blas_only || n_meso_ <= kNClustersThresholdForPruning;
-        bool partial_norms_computed = false;
         IterationInput in{x_rot_.get(), n_all, n_all, n_meso_, data_norms_.get()};
         for (size_t iter = 0; iter < cfg_.iters_mesoclustering; ++iter) {
             const bool gemm_only = (iter == 0) || always_gemm_only;
-            if (!gemm_only && !partial_norms_computed) {
-                launch_row_sqnorms(x_rot_.get(), n_all, d_, partial_d_, data_norms_.get(), stream_);
-                partial_norms_computed = true;
-            }
             run_iteration(gemm_only, in, iter, iter == 0, stats_meso_);
             if (cfg_.early_termination && should_stop_early(shift_, cost_, prev_cost_, cfg_.tol, iter)) break;
         }
@@ -1790,14 +1790,9 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
         generate_centroids_from_device_rows(meso_buffer_.get(), msize, n_fine, &forgy[m]);
 
         const bool always_gemm_only = gemm_only(n_fine);
-        bool partial_norms_computed = false;
         IterationInput in{meso_buffer_.get(), msize, msize, n_fine, meso_norms_.get()};
         for (size_t iter = 0; iter < cfg_.iters_fineclustering; ++iter) {
             const bool gemm_only = (iter == 0) || always_gemm_only;
-            if (!gemm_only && !partial_norms_computed) {
-                launch_row_sqnorms(meso_buffer_.get(), msize, d_, partial_d_, meso_norms_.get(), stream_);
-                partial_norms_computed = true;
-            }
             run_iteration(gemm_only, in, iter, iter == 0, stats_fine_);
             if (cfg_.early_termination && should_stop_early(shift_, cost_, prev_cost_, cfg_.tol, iter)) break;
         }
@@ -1816,17 +1811,10 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
     SKM_CUDA(cudaMemcpyAsync(assignments_.get(), final_assignments_.get(), sizeof(uint32_t) * n_all, cudaMemcpyDeviceToDevice, stream_));
     {
         const bool always_gemm_only = d_ < kDimensionThresholdForPruning || k_ <= kNClustersThresholdForPruning;
-        bool partial_norms_computed = false;
         IterationInput in{x_rot_.get(), n_all, n_all, k_, data_norms_.get()};
         for (size_t iter = 0; iter < cfg_.iters_refinement; ++iter) {
-            if (!always_gemm_only && !partial_norms_computed) {
-                launch_row_sqnorms(x_rot_.get(), n_all, d_, partial_d_, data_norms_.get(), stream_);
-                partial_norms_computed = true;
-            } else if (always_gemm_only && !partial_norms_computed) {
-                // data_norms_ still holds whatever the mesoclustering left; GEMM-only needs full norms.
-                SKM_CUDA(cudaMemcpyAsync(data_norms_.get(), full_norms_.get(), sizeof(float) * n_all, cudaMemcpyDeviceToDevice, stream_));
-                partial_norms_computed = true;
-            }
+            // data_norms_ still holds whatever the mesoclustering left; GEMM-only needs full norms.
+            if (always_gemm_only && iter == 0) SKM_CUDA(cudaMemcpyAsync(data_norms_.get(), full_norms_.get(), sizeof(float) * n_all, cudaMemcpyDeviceToDevice, stream_));
             run_iteration(always_gemm_only, in, iter, false, stats_refine_);
         }
     }
@@ -2021,7 +2009,6 @@ void Engine::assign_training_points(const float* vectors, const float* centroids
     for (size_t r0 = 0; r0 < n; r0 += rows) {
         const size_t cnt = std::min(rows, n - r0);
         load_rows(vectors + r0 * d_, on_device, nullptr, cnt, !cfg_.data_already_rotated, xr.get());
-        launch_row_sqnorms(xr.get(), cnt, d_, partial_d_, xn.get(), stream_);
         PrunedParams p = pruned_params(IterationInput{xr.get(), cnt, cnt, k_, xn.get()});
         p.y = c_cur_.get();
         p.knn = knn + r0;

@@ -236,6 +236,8 @@ class Engine {
         float* norms;         // device, full or partial norms of x (rewritten when d' changes)
         mutable bool pruned_before = false;   // a pruned pass over these rows has run
         mutable double survival = 0.0;        // ... and what it said about the next one (PrunedParams)
+        mutable bool partial_norms = false;   // norms holds those over the first partial_d_ dimensions (a pruned pass makes them)
+        bool full_norms = true;               // before the first pruned pass: those over all dimensions
     };
 
     void start_rotation(bool beside);

@@ -46,18 +46,25 @@ __device__ __forceinline__ void append_flagged(const uint32_t* flags, int rows, 
 }
 
 __global__ void __launch_bounds__(256) prev_dist_kernel(const float* __restrict__ x, const float* __restrict__ y, const uint32_t* __restrict__ knn, size_t n, size_t d,
-                                                        float* __restrict__ best) {
+                                                        float* __restrict__ best, size_t upto, float* __restrict__ norms) {
     const size_t row = static_cast<size_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
     if (row >= n) return;
     const int lane = threadIdx.x & 31;
     const float* __restrict__ xr = x + row * d;
     const float* __restrict__ yr = y + static_cast<size_t>(knn[row]) * d;
-    float s = 0.f;
+    float s = 0.f, norm = 0.f;   // (the norm in the order of row_sqnorms_kernel)
     const bool vec = (d % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0) && ((reinterpret_cast<uintptr_t>(y) & 15) == 0);
+    const size_t upto4 = vec ? (upto & ~size_t{3}) : 0;
     if (vec) {
         for (size_t j = static_cast<size_t>(lane) * 4; j < d; j += 128) {
             const float4 a = __ldg(reinterpret_cast<const float4*>(xr + j));
             const float4 b = __ldg(reinterpret_cast<const float4*>(yr + j));
+            if (j < upto4) {
+                norm = fmaf(a.x, a.x, norm);
+                norm = fmaf(a.y, a.y, norm);
+                norm = fmaf(a.z, a.z, norm);
+                norm = fmaf(a.w, a.w, norm);
+            }
             float t;
             t = a.x - b.x; s = fmaf(t, t, s);
             t = a.y - b.y; s = fmaf(t, t, s);
@@ -71,7 +78,13 @@ __global__ void __launch_bounds__(256) prev_dist_kernel(const float* __restrict_
         }
     }
     s = warp_sum(s);
-    if (lane == 0) best[row] = s;
+    if (norms) {
+        for (size_t j = upto4 + lane; j < upto; j += 32) norm = fmaf(__ldg(xr + j), __ldg(xr + j), norm);
+        norm = warp_sum(norm);
+    }
+    if (lane != 0) return;
+    best[row] = s;
+    if (norms) norms[row] = norm;
 }
 
 // sample[s][:] = y[(s * k) / n_sample][:]
@@ -311,9 +324,9 @@ __global__ void __launch_bounds__(256, 2) assign_pruned_dense_kernel(const Prune
 }
 
 // -------------------------------------------------------------------------------------------------
-void launch_exact_dist(const float* x, const float* y, const uint32_t* knn, size_t n, size_t d, float* out, cudaStream_t stream) {
+void launch_exact_dist(const float* x, const float* y, const uint32_t* knn, size_t n, size_t d, float* out, cudaStream_t stream, size_t upto, float* norms) {
     if (n == 0) return;
-    prev_dist_kernel<<<static_cast<unsigned>((n + 7) / 8), 256, 0, stream>>>(x, y, knn, n, d, out);
+    prev_dist_kernel<<<static_cast<unsigned>((n + 7) / 8), 256, 0, stream>>>(x, y, knn, n, d, out, norms ? upto : 0, norms);
     SKM_LAUNCH_CHECK();
 }
 
