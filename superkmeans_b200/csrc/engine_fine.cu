@@ -70,13 +70,15 @@ __global__ void __launch_bounds__(256) group_cost_kernel(const float* __restrict
     }
 }
 
-// out[g] = sum of the squared differences of the group's centroids
+// out[g][slice] = sum of the squared differences of every kShiftSlices-th of the group's centroids (a block alone for all of them waits for
+// its loads: 50 groups of 50 x 768: 55 us)
+constexpr int kShiftSlices = 8;
 __global__ void __launch_bounds__(256) group_shift_kernel(const float* __restrict__ a, const float* __restrict__ b, size_t d, const Group* __restrict__ groups, double* __restrict__ out) {
     __shared__ double part[8];
     const Group g = groups[blockIdx.x];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double total = 0.0;
-    for (uint32_t c = warp; c < g.k; c += 8) {
+    for (uint32_t c = blockIdx.y * 8 + warp; c < g.k; c += 8 * kShiftSlices) {
         const float* pa = a + static_cast<size_t>(g.y0 + c) * d;
         const float* pb = b + static_cast<size_t>(g.y0 + c) * d;
         float s = 0.f;
@@ -92,7 +94,7 @@ __global__ void __launch_bounds__(256) group_shift_kernel(const float* __restric
     if (threadIdx.x == 0) {
         double t = 0.0;
         for (int w = 0; w < 8; ++w) t += part[w];
-        out[blockIdx.x] = t;
+        out[blockIdx.x * kShiftSlices + blockIdx.y] = t;
     }
 }
 
@@ -130,8 +132,20 @@ void Engine::train_fine_run(size_t first, size_t last, const std::vector<size_t>
     PinnedBuffer<double> sums;
     stage_.upload(group_of_dev.ensure(k), group_of.data(), nullptr, k, sizeof(uint32_t), stream_);
     groups_dev.ensure(n_groups);
-    sums_dev.ensure(2 * n_groups);
-    sums.ensure(2 * n_groups);
+    sums_dev.ensure(n_groups);
+    sums.ensure(n_groups);
+    // per iteration and group, in slices
+    const size_t shift_words = n_groups * kShiftSlices;
+    DeviceBuffer<double> all_shifts;
+    PinnedBuffer<double> shifts;
+    all_shifts.ensure(shift_words * cfg_.iters_fineclustering);
+    shifts.ensure(shift_words * cfg_.iters_fineclustering);
+    auto shifts_dev = [&](size_t iter) { return all_shifts.get() + shift_words * iter; };
+    auto shift_of = [&](size_t iter, size_t q) {
+        double t = 0.0;
+        for (int w = 0; w < kShiftSlices; ++w) t += shifts.get()[shift_words * iter + q * kShiftSlices + w];
+        return static_cast<float>(t);
+    };
     exact_.begin_groups(x, n, d_, c_prev_.get(), k, norms, stream_);
 
     struct State {
@@ -175,8 +189,9 @@ void Engine::train_fine_run(size_t first, size_t last, const std::vector<size_t>
             group_means_kernel<<<static_cast<unsigned>(k), 256, 0, stream_>>>(c_cur_.get(), c_prev_.get(), counts(), group_of_dev.get(), groups_dev.get(), d_);
             SKM_LAUNCH_CHECK();
         }
+        tell_error();
         sync();
-        check_tensor_cores();
+        check_told_error();
         // ConsolidateCentroids of every group (superkmeans.h:936-968)
         std::vector<const char*> failure(n_groups, nullptr);
 #pragma omp parallel for schedule(dynamic) if (n_groups > 8)
@@ -221,18 +236,21 @@ void Engine::train_fine_run(size_t first, size_t last, const std::vector<size_t>
         }
         {
             PhaseScope ps(*this, PH_SHIFT);
-            group_shift_kernel<<<static_cast<unsigned>(n_groups), 256, 0, stream_>>>(c_cur_.get(), c_prev_.get(), d_, groups_dev.get(), sums_dev.get() + n_groups);
+            group_shift_kernel<<<dim3(static_cast<unsigned>(n_groups), kShiftSlices), 256, 0, stream_>>>(c_cur_.get(), c_prev_.get(), d_, groups_dev.get(), shifts_dev(iter));
             SKM_LAUNCH_CHECK();
         }
-        SKM_CUDA(cudaMemcpyAsync(sums.get() + n_groups, sums_dev.get() + n_groups, sizeof(double) * n_groups, cudaMemcpyDeviceToHost, stream_));
-        sync();
+        // only early stopping asks for the shift before the end
+        if (cfg_.early_termination) {
+            SKM_CUDA(cudaMemcpyAsync(shifts.get() + shift_words * iter, shifts_dev(iter), sizeof(double) * shift_words, cudaMemcpyDeviceToHost, stream_));
+            sync();
+        }
         for (size_t q = 0; q < n_groups; ++q) {
             Group& g = groups[q];
             if (!g.active) continue;
             State& st = state[q];
             st.prev_cost = st.cost;
             st.cost = static_cast<float>(sums.get()[q]);
-            st.shift = static_cast<float>(sums.get()[n_groups + q]);
+            if (cfg_.early_termination) st.shift = shift_of(iter, q);
             st.cost_f64 = sums.get()[q];
             skm_iter_stats s{};
             s.iteration = iter + 1;
@@ -248,6 +266,13 @@ void Engine::train_fine_run(size_t first, size_t last, const std::vector<size_t>
                 g.active = 0;
                 tiles_current = false;
             }
+        }
+    }
+    if (!cfg_.early_termination) {
+        SKM_CUDA(cudaMemcpyAsync(shifts.get(), shifts_dev(0), sizeof(double) * shift_words * cfg_.iters_fineclustering, cudaMemcpyDeviceToHost, stream_));
+        sync();
+        for (size_t q = 0; q < n_groups; ++q) {
+            for (skm_iter_stats& s : state[q].stats) state[q].shift = s.shift = shift_of(s.iteration - 1, q);
         }
     }
     for (size_t q = 0; q < n_groups; ++q) {
