@@ -1,8 +1,14 @@
 // See host_copy.h.
 #include "host_copy.h"
 
+#include <algorithm>
+#include <cstdint>
 #include <cstring>
 #include <exception>
+
+#ifdef __SSE2__
+#include <emmintrin.h>
+#endif
 
 namespace skmb {
 
@@ -22,23 +28,49 @@ bool copied_directly(const void* p) { return type_of(p) != cudaMemoryTypeUnregis
 // A thread per quarter of a megabyte, eight at most: more do not copy faster.
 int threads_for(size_t bytes) { return static_cast<int>(std::max<size_t>(1, std::min<size_t>(8, bytes >> 18))); }
 
-void copy_bytes(char* dst, const char* src, size_t bytes) {
-    const int threads = threads_for(bytes);
-    if (threads == 1) {
-        std::memcpy(dst, src, bytes);
-        return;
+// Copies to memory that the GPU reads next, past the caches: what another core has just written to its cache the link fetches at
+// 30 GB/s (4 MB, eight threads: 138 us), what lies in memory at 50 (84 us).  Filling it takes 66 us in place of 44, beside the copy before.
+// publish() comes behind the last of a thread.
+void stream_bytes(char* dst, const char* src, size_t bytes) {
+#ifdef __SSE2__
+    const size_t head = std::min(bytes, static_cast<size_t>(-reinterpret_cast<uintptr_t>(dst) & 15));
+    std::memcpy(dst, src, head);
+    size_t i = head;
+    for (; i + 64 <= bytes; i += 64) {
+        __m128i v[4];
+        for (int q = 0; q < 4; ++q) v[q] = _mm_loadu_si128(reinterpret_cast<const __m128i*>(src + i) + q);
+        for (int q = 0; q < 4; ++q) _mm_stream_si128(reinterpret_cast<__m128i*>(dst + i) + q, v[q]);
     }
-#pragma omp parallel for num_threads(threads) schedule(static)
+    std::memcpy(dst + i, src + i, bytes - i);
+#else
+    std::memcpy(dst, src, bytes);
+#endif
+}
+void publish() {
+#ifdef __SSE2__
+    _mm_sfence();
+#endif
+}
+
+// `to_gpu`: the GPU reads dst, else the caller does.
+void copy_bytes(char* dst, const char* src, size_t bytes, bool to_gpu) {
+    const int threads = threads_for(bytes);
+#pragma omp parallel for num_threads(threads) schedule(static) if (threads > 1)
     for (int t = 0; t < threads; ++t) {
         const size_t b = bytes * t / threads, e = bytes * (t + 1) / threads;
-        std::memcpy(dst + b, src + b, e - b);
+        if (to_gpu) stream_bytes(dst + b, src + b, e - b);
+        else std::memcpy(dst + b, src + b, e - b);
+        publish();
     }
 }
 
 void gather_rows(char* dst, const char* src, const size_t* idx, size_t n, size_t row_bytes) {
     const int threads = threads_for(n * row_bytes);
 #pragma omp parallel for num_threads(threads) schedule(static) if (threads > 1)
-    for (size_t i = 0; i < n; ++i) std::memcpy(dst + i * row_bytes, src + idx[i] * row_bytes, row_bytes);
+    for (int t = 0; t < threads; ++t) {
+        for (size_t i = n * t / threads; i < n * (t + 1) / threads; ++i) stream_bytes(dst + i * row_bytes, src + idx[i] * row_bytes, row_bytes);
+        publish();
+    }
 }
 
 } // namespace
@@ -73,7 +105,7 @@ void HostStage::upload(void* dst, const void* src, const size_t* idx, size_t n, 
         next_ = (next_ + 1) % kPieces;
         char* p = piece(i, cnt * row_bytes);
         if (idx) gather_rows(p, static_cast<const char*>(src), idx + r0, cnt, row_bytes);
-        else copy_bytes(p, static_cast<const char*>(src) + r0 * row_bytes, cnt * row_bytes);
+        else copy_bytes(p, static_cast<const char*>(src) + r0 * row_bytes, cnt * row_bytes, true);
         SKM_CUDA(cudaMemcpyAsync(static_cast<char*>(dst) + r0 * row_bytes, p, cnt * row_bytes, cudaMemcpyHostToDevice, stream));
         SKM_CUDA(cudaEventRecord(copied_[i], stream));
     }
@@ -103,7 +135,7 @@ void HostStage::download(void* dst, const void* src, size_t bytes, cudaStream_t 
         const int i = slot[q % kPieces];
         SKM_CUDA(cudaEventSynchronize(copied_[i]));
         const size_t b = q * kPieceBytes;
-        copy_bytes(static_cast<char*>(dst) + b, pieces_[i].get(), std::min(kPieceBytes, bytes - b));
+        copy_bytes(static_cast<char*>(dst) + b, pieces_[i].get(), std::min(kPieceBytes, bytes - b), false);
     }
 }
 

@@ -9,7 +9,7 @@
 namespace skmb {
 
 // cudaMemcpy from or to pageable memory moves 11 GB/s (one thread fills the driver's staging buffer); eight threads fill
-// pinned memory at 70 GB/s (32 GB/s when they gather rows of 3 KB) and the link moves 55 GB/s from there, so the copies
+// pinned memory at 63 GB/s (32 GB/s when they gather rows of 3 KB) and the link moves 50 - 55 GB/s from there, so the copies
 // below run at 30 - 50 GB/s.  Memory that the GPU can read by itself is copied from directly.
 //
 // One per engine, used by one thread at a time; whoever owns it waits for both streams before it goes away.
