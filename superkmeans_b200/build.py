@@ -13,7 +13,7 @@ from concurrent.futures import ThreadPoolExecutor
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJDIR = os.path.join(HERE, "build")
-SOURCES = ["memory.cu", "host_copy.cu", "phase_timers.cu", "kernels.cu", "kernels_pruned_dense.cu", "kernels_tc.cu", "kernels_tc_sparse.cu", "kernels_tc_rotate.cu", "kernels_first_test.cu", "kernels_chain.cu", "kernels_walk.cu", "kernels_topk.cu", "kernels_replay.cu", "rotation_matrix.cu", "exact_assign.cu", "direct_assign.cu", "engine.cu", "engine_fine.cu",
+SOURCES = ["memory.cu", "host_copy.cu", "phase_timers.cu", "kernels.cu", "kernels_pruned_dense.cu", "kernels_tc.cu", "kernels_tc_sparse.cu", "kernels_tc_rotate.cu", "kernels_tc_rotate_half.cu", "kernels_first_test.cu", "kernels_chain.cu", "kernels_walk.cu", "kernels_topk.cu", "kernels_replay.cu", "rotation_matrix.cu", "exact_assign.cu", "direct_assign.cu", "engine.cu", "engine_fine.cu",
            "comm_nccl.cu", "noalloc.cu", "abi.cu"]
 HEADERS = ["common.cuh", "device_utils.cuh", "gemm_simt.cuh", "tc_ptx.cuh", "kernels_tc.cuh", "noalloc.h", "engine.h", "engine_buffers.h", "host_copy.h", "phase_timers.h", "exact_assign.h", "host_logic.h", "comm_nccl.h",
            os.path.join("..", "..", "include", "skm_b200.h")]

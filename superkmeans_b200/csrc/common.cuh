@@ -105,6 +105,8 @@ void launch_row_sqnorms(const float* x, size_t n, size_t ld, size_t upto, float*
 // out[n x n_out] = a[n x k_dim] * b[n_out x k_dim]^T, all row-major with leading dimensions lda,
 // ldb, ldo (NT GEMM).  Used for rotation (b = M) and un-rotation (b = M^T).
 void launch_gemm_nt(const float* a, size_t lda, const float* b, size_t ldb, float* out, size_t ldo, size_t n, size_t n_out, size_t k_dim, cudaStream_t stream);
+// The same for rows that a trained model is applied to; b is contiguous.
+void launch_rotate_to_assign(const float* a, size_t lda, const float* b, float* out, size_t ldo, size_t n, size_t n_out, size_t k_dim, cudaStream_t stream);
 
 // out[j*n + i] = in[i*n + j]
 void launch_transpose_square(const float* in, float* out, size_t n, cudaStream_t stream);

@@ -367,7 +367,8 @@ void Engine::load_rows(const float* src, bool src_on_device, const size_t* idx, 
     const size_t row_bytes = sizeof(float) * user_d_;
     const bool as_it_is = !rotate && d_ == user_d_;
     auto place = [&](const float* raw, float* to, size_t cnt) {
-        if (rotate) launch_gemm_nt(raw, user_d_, m_dev_.get(), user_d_, to, d_, cnt, d_, user_d_, stream_);
+        if (rotate && trained_) launch_rotate_to_assign(raw, user_d_, m_dev_.get(), to, d_, cnt, d_, user_d_, stream_);
+        else if (rotate) launch_gemm_nt(raw, user_d_, m_dev_.get(), user_d_, to, d_, cnt, d_, user_d_, stream_);
         else launch_move_gap(raw, cnt, user_d_, to, d_, vertical_dims_, stream_);
     };
     if (src_on_device && !idx) {
@@ -2109,7 +2110,8 @@ void Engine::op_rotate(int device, const float* m, const float* x, size_t n, siz
         b = mtd.get();
     }
     ctx.upload(xd, x, n * d);
-    launch_gemm_nt(xd.get(), d, b, d, od.ensure(n * d), d, n, d, d, ctx.stream);
+    if (inverse) launch_gemm_nt(xd.get(), d, b, d, od.ensure(n * d), d, n, d, d, ctx.stream);
+    else launch_rotate_to_assign(xd.get(), d, b, od.ensure(n * d), d, n, d, d, ctx.stream);
     ctx.download(out, od.get(), n * d);
     ctx.sync();
     check_tc_error(ctx.stream);

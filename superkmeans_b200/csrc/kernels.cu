@@ -102,6 +102,11 @@ void launch_gemm_nt(const float* a, size_t lda, const float* b, size_t ldb, floa
     SKM_LAUNCH_CHECK();
 }
 
+void launch_rotate_to_assign(const float* a, size_t lda, const float* b, float* out, size_t ldo, size_t n, size_t n_out, size_t k_dim, cudaStream_t stream) {
+    if (n != 0 && n_out != 0 && tc::enabled() && k_dim >= 32) tc::launch_rotate_halves(a, lda, b, out, ldo, n, n_out, k_dim, stream);
+    else launch_gemm_nt(a, lda, b, k_dim, out, ldo, n, n_out, k_dim, stream);
+}
+
 __global__ void transpose_square_kernel(const float* __restrict__ in, float* __restrict__ out, size_t n) {
     __shared__ float t[32][33];
     const size_t bx = static_cast<size_t>(blockIdx.x) * 32, by = static_cast<size_t>(blockIdx.y) * 32;

@@ -34,6 +34,8 @@ void launch_gemm_nt(const float* a, size_t lda, const float* b, size_t ldb, floa
 // out[n][n_out] = a[n][k_dim] * b[n_out][k_dim]^T with the accumulation cut into four chains that are summed in fp32
 // registers (kernels_tc_rotate.cu): the rotation and un-rotation GEMM.  b is contiguous.
 void launch_rotate(const float* a, size_t lda, const float* b, float* out, size_t ldo, size_t n, size_t n_out, size_t k_dim, cudaStream_t stream);
+// The same from fp16 halves (kernels_tc_rotate_half.cu), for any alignment of a and b.
+void launch_rotate_halves(const float* a, size_t lda, const float* b, float* out, size_t ldo, size_t n, size_t n_out, size_t k_dim, cudaStream_t stream);
 
 // The leading columns of a row-major fp32 matrix as fp16 pairs: element * scale = hi + lo to 22 bits, scale a power of two.
 // For points factor[row] = -2 / scale, for centroids factor[row] = 1 / scale and, behind the last, whether they share one scale.

@@ -1,0 +1,22 @@
+"""Rotation of rows of any width and magnitude: widths at the edges of what the conversion to fp16 halves holds in registers, rows that
+16-byte loads cannot address, row counts around a tile and around one tile per pair of SMs."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,d", [(1, 33), (130, 50), (255, 127), (257, 129), (300, 255), (140, 257), (600, 511), (300, 513), (300, 770), (256, 1_025), (130, 1_537), (70, 2_051),
+                                 (520, 132), (260, 516), (130, 1_028), (100, 1_540), (19_200, 128), (18_945, 260)])
+def test_rows_of_any_width_and_magnitude(n, d):
+    import superkmeans_b200 as skm
+
+    rng = np.random.default_rng(n + d)
+    x = rng.standard_normal((n, d), dtype=np.float32) * (10.0 ** rng.uniform(-25, 25, (n, 1))).astype(np.float32)
+    x[n // 2] = 0
+    m = rng.standard_normal((d, d), dtype=np.float32) * (10.0 ** rng.uniform(-3, 3, (d, 1))).astype(np.float32)
+    got = skm.engine.rotate(m, x)
+    want = x.astype(np.float64) @ m.T.astype(np.float64)
+    # 22 bits of either factor, and at most d / 4 terms one after the other in an accumulator that truncates
+    scale = np.linalg.norm(x.astype(np.float64), axis=1)[:, None] * np.linalg.norm(m.astype(np.float64), axis=1)
+    assert (np.abs(got - want) <= 3e-6 * scale).all()
