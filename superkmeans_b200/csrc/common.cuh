@@ -335,8 +335,7 @@ struct SplitOpDev {
     uint32_t dst, src, kind;
     float wc;
 };
-// columns from `shifted` on hold the dimension before theirs, or the third before (see Engine::d_): even ones are odd there
-void launch_apply_split_ops(float* c, size_t d, size_t shifted, const SplitOpDev* ops, size_t n_ops, cudaStream_t stream);
+void launch_apply_split_ops(float* c, size_t d, const SplitOpDev* ops, size_t n_ops, cudaStream_t stream);
 
 // PDX-blocked copy and first-vertical_d copy of a row-major k x d matrix
 void launch_pdxify(const float* c, float* pdx, float* aux, size_t k, size_t d, size_t vertical_d, cudaStream_t stream);
@@ -372,11 +371,6 @@ void launch_consolidate(const ConsolidateParams& p, cudaStream_t stream);
 
 // out[i][:] = in[idx[i]][:]; an index of all ones gives a row of zeros
 void launch_gather_rows(const float* in, const uint64_t* idx, float* out, size_t n_out, size_t d, cudaStream_t stream);
-
-// Rows of d_in values as rows of d_out with the difference as zeros in front of value `at`, or (d_out smaller) without the values there.
-void launch_move_gap(const float* in, size_t n, size_t d_in, float* out, size_t d_out, size_t at, cudaStream_t stream);
-// m (d x d) as the rotation of rows with a gap: m_gap (d_gap x d) = m with rows of zeros in front of row `at`, mt_gap (d x d_gap) its transpose.
-void launch_rotation_with_gap(const float* m, size_t d, size_t d_gap, size_t at, float* m_gap, float* mt_gap, cudaStream_t stream);
 void launch_gather_f32(const float* in, const uint64_t* idx, float* out, size_t n_out, cudaStream_t stream);
 // out[idx[i]] = in[i] + offset
 void launch_scatter_u32_offset(const uint32_t* in, const uint64_t* idx, uint32_t* out, size_t n, uint32_t offset, cudaStream_t stream);

@@ -36,15 +36,15 @@ __device__ __forceinline__ void store_answer(unsigned long long key, size_t row,
     if (dist) dist[row] = fmaxf(0.0f, ordered_to_float(static_cast<uint32_t>(key >> 32)));
 }
 
-// One row operation of a split (host_logic.h, SplitOp) for column j, an even dimension or an odd one.
+// One row operation of a split (host_logic.h, SplitOp) for dimension j.
 template <class Op>
-__device__ __forceinline__ void apply_split_op(float* __restrict__ c, size_t d, size_t j, bool even, const Op op) {
+__device__ __forceinline__ void apply_split_op(float* __restrict__ c, size_t d, size_t j, const Op op) {
     const float up = 1.0f + (1.0f / 1024.0f), down = 1.0f - (1.0f / 1024.0f);
     float* pd = c + static_cast<size_t>(op.dst) * d + j;
     float* ps = c + static_cast<size_t>(op.src) * d + j;
     if (op.kind == 0) {
         const float v = *ps;
-        if (even) {
+        if ((j & 1) == 0) {
             *pd = __fmul_rn(v, up);
             *ps = __fmul_rn(v, down);
         } else {

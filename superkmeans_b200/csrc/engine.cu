@@ -89,7 +89,7 @@ int resolve_device(int device) {
 // Construction (superkmeans.h:123-140, hierarchical_superkmeans.h:43-66)
 // -------------------------------------------------------------------------------------------------
 Engine::Engine(const skm_config& cfg, size_t n_clusters, size_t d, bool hierarchical, int device)
-    : cfg_(cfg), k_(n_clusters), user_d_(d), d_(d), hierarchical_(hierarchical), device_(0) {
+    : cfg_(cfg), k_(n_clusters), d_(d), hierarchical_(hierarchical), device_(0) {
     ensure_positive(n_clusters > 0, "n_clusters");
     ensure_positive(d > 0, "dimensionality");
     ensure_positive(cfg.iters > 0, "config.iters");
@@ -102,14 +102,7 @@ Engine::Engine(const skm_config& cfg, size_t n_clusters, size_t d, bool hierarch
     if (cfg_.data_already_rotated) cfg_.unrotate_centroids = 0;
     epsilon0_ = hierarchical ? kHierarchicalPrunerInitialThreshold : kPrunerInitialThreshold;
     const DimensionSplit split = dimension_split(d);
-    // (The horizontal dimensions are a multiple of 64.)  Not below 32 dimensions, where nothing runs on the tensor cores and the zeros would
-    // be a share of the rows, and not for the two-level algorithm, whose passes have the fp16 filter whatever the width: padded, 253 652 x 103
-    // took 10.1 ms in place of 10.7, and the first centroids of a mesocluster hang on every row's last digits.
-    const size_t gap = d < 32 || hierarchical ? 0 : (4 - d % 4) % 4;
-    d_ = d + gap;
-    vertical_dims_ = static_cast<uint32_t>(split.vertical_d);
-    vertical_d_ = static_cast<uint32_t>(split.vertical_d + gap);
-    shifted_ = gap % 2 == 0 ? d_ : vertical_d_;
+    vertical_d_ = static_cast<uint32_t>(split.vertical_d);
     horizontal_d_ = static_cast<uint32_t>(split.horizontal_d);
 
     int count = 0;
@@ -124,8 +117,7 @@ Engine::Engine(const skm_config& cfg, size_t n_clusters, size_t d, bool hierarch
     copy_stream_ = acquire_stream();
     WorkStream work(stream_);
     ratios_host_ = make_ratios(d, epsilon0_);
-    ratios_host_.resize(d_ + 1, 1.0f);   // (all dimensions, zeros or not)
-    SKM_CUDA(cudaMemcpyAsync(ratios_dev_.ensure(d_ + 1), ratios_host_.data(), sizeof(float) * (d_ + 1), cudaMemcpyHostToDevice, stream_));
+    SKM_CUDA(cudaMemcpyAsync(ratios_dev_.ensure(d + 1), ratios_host_.data(), sizeof(float) * (d + 1), cudaMemcpyHostToDevice, stream_));
     if (hierarchical && n_clusters <= 128 && !cfg.suppress_warnings) {
         std::cout << "WARNING: n_clusters <= 128 is not recommended for HierarchicalSuperKMeans. "
                      "Consider using at least 128 clusters."
@@ -195,9 +187,9 @@ struct Engine::Drawing {
 void Engine::start_rotation(bool beside) {
     if (rotation_ready_ || drawing_ || !rotation_host_.empty()) return;
     try {
-        drawing_ = std::make_unique<Drawing>(user_d_ * user_d_, cfg_.seed);
+        drawing_ = std::make_unique<Drawing>(d_ * d_, cfg_.seed);
     } catch (const OutOfMemory&) {
-        rotation_host_ = make_rotation_matrix(user_d_, cfg_.seed);   // (in ordinary memory; seconds from d = 2000 on)
+        rotation_host_ = make_rotation_matrix(d_, cfg_.seed);   // (in ordinary memory; seconds from d = 2000 on)
         return;
     }
     if (!beside) return;
@@ -226,8 +218,8 @@ void Engine::start_rotation(bool beside) {
 // Enqueues on `stream`; returns before the last kernels have run.
 void Engine::make_rotation(cudaStream_t stream) {
     NormalDraws& draws = drawing_->draws;
-    float* m = plain_rotation();
-    float* to = mt_dev_.ensure(user_d_ * d_);   // (not needed for the transpose yet)
+    float* m = m_dev_.ensure(d_ * d_);
+    float* to = mt_dev_.ensure(d_ * d_);   // (not needed for the transpose yet)
     // as they come, in a few groups, read from host memory by a kernel: copies would queue behind those of the rows
     const size_t per_group = (draws.pieces() + 7) / 8;
     size_t got = 0;
@@ -237,24 +229,17 @@ void Engine::make_rotation(cudaStream_t stream) {
         p.stretch = draws.stretch();
         for (size_t t = t0; t < std::min(draws.pieces(), t0 + per_group); ++t) {
             p.start[p.n++] = got;
-            got = std::min(got + draws.piece(t).count, user_d_ * user_d_);
+            got = std::min(got + draws.piece(t).count, d_ * d_);
         }
         p.start[p.n] = got;
         launch_collect_draws(p, to, stream);
     }
-    if (got != user_d_ * user_d_ || !make_rotation_matrix_on_device(to, user_d_, m, stream)) {
+    if (got != d_ * d_ || !make_rotation_matrix_on_device(to, d_, m, stream)) {
         SKM_CUDA(cudaStreamSynchronize(stream));
-        rotation_host_ = make_rotation_matrix(user_d_, cfg_.seed);
-        SKM_CUDA(cudaMemcpyAsync(m, rotation_host_.data(), sizeof(float) * user_d_ * user_d_, cudaMemcpyHostToDevice, stream));
+        rotation_host_ = make_rotation_matrix(d_, cfg_.seed);
+        SKM_CUDA(cudaMemcpyAsync(m, rotation_host_.data(), sizeof(float) * d_ * d_, cudaMemcpyHostToDevice, stream));
     }
-    place_rotation(stream);
-}
-
-// Both operands of the rotation and its inverse, from the plain matrix.
-void Engine::place_rotation(cudaStream_t stream) {
-    float* mt = mt_dev_.ensure(user_d_ * d_);
-    if (d_ == user_d_) launch_transpose_square(m_dev_.get(), mt, d_, stream);
-    else launch_rotation_with_gap(m_plain_.get(), user_d_, d_, vertical_dims_, m_dev_.ensure(d_ * user_d_), mt, stream);
+    launch_transpose_square(m, to, d_, stream);
 }
 
 void Engine::ensure_rotation() {
@@ -275,8 +260,9 @@ void Engine::ensure_rotation() {
         sync();
         drawing_.reset();
     } else {
-        SKM_CUDA(cudaMemcpyAsync(plain_rotation(), rotation_host_.data(), sizeof(float) * user_d_ * user_d_, cudaMemcpyHostToDevice, stream_));
-        place_rotation(stream_);
+        float* m = m_dev_.ensure(d_ * d_);
+        SKM_CUDA(cudaMemcpyAsync(m, rotation_host_.data(), sizeof(float) * d_ * d_, cudaMemcpyHostToDevice, stream_));
+        launch_transpose_square(m, mt_dev_.ensure(d_ * d_), d_, stream_);
         sync();
     }
     rotation_ready_ = true;
@@ -292,15 +278,15 @@ void Engine::drop_rotation() {
 void Engine::ensure_rotation_host() {
     ensure_rotation();
     if (!rotation_host_.empty()) return;
-    rotation_host_.resize(user_d_ * user_d_);
-    SKM_CUDA(cudaMemcpyAsync(rotation_host_.data(), plain_rotation(), sizeof(float) * user_d_ * user_d_, cudaMemcpyDeviceToHost, stream_));
+    rotation_host_.resize(d_ * d_);
+    SKM_CUDA(cudaMemcpyAsync(rotation_host_.data(), m_dev_.get(), sizeof(float) * d_ * d_, cudaMemcpyDeviceToHost, stream_));
     sync();
 }
 
 void Engine::set_rotation(const float* m_host) {
     Entry entry(device_, stream_);
     drop_rotation();   // (of a Train that failed)
-    rotation_host_.assign(m_host, m_host + user_d_ * user_d_);
+    rotation_host_.assign(m_host, m_host + d_ * d_);
     rotation_ready_ = false;
     ensure_rotation();
 }
@@ -308,7 +294,7 @@ void Engine::set_rotation(const float* m_host) {
 void Engine::get_rotation(float* m_out) {
     Entry entry(device_, stream_);
     ensure_rotation_host();
-    std::memcpy(m_out, rotation_host_.data(), sizeof(float) * user_d_ * user_d_);
+    std::memcpy(m_out, rotation_host_.data(), sizeof(float) * d_ * d_);
 }
 
 void Engine::set_shard(size_t n_global, size_t row_offset, skm_allreduce_fn fn, void* user) {
@@ -357,24 +343,25 @@ void Engine::allreduce_iteration(float* sums, size_t n_sums, uint32_t* counts, s
     allreduce(scalars, n_scalars, 1);
 }
 
-// dst[n x d_] (device) = the first n rows of src, or rows idx[0 .. n) of it, rotated or as they are.  Host sources are
+// dst[n x d] (device) = the first n rows of src, or rows idx[0 .. n) of it, rotated or as they are.  Host sources are
 // streamed through two device chunks so that the copy of chunk i+1 overlaps the rotation of chunk i; the first chunk is on
 // its way before the rotation matrix is waited for.
 void Engine::load_rows(const float* src, bool src_on_device, const size_t* idx, size_t n, bool rotate, float* dst, const std::function<void(size_t, size_t)>& after_rows,
                        size_t piece) {
     if (n == 0) return;
     PhaseScope ps(*this, PH_ROTATE);
-    const size_t row_bytes = sizeof(float) * user_d_;
-    const bool as_it_is = !rotate && d_ == user_d_;
-    auto place = [&](const float* raw, float* to, size_t cnt) {
-        if (rotate && trained_) launch_rotate_to_assign(raw, user_d_, m_dev_.get(), to, d_, cnt, d_, user_d_, stream_);
-        else if (rotate) launch_gemm_nt(raw, user_d_, m_dev_.get(), user_d_, to, d_, cnt, d_, user_d_, stream_);
-        else launch_move_gap(raw, cnt, user_d_, to, d_, vertical_dims_, stream_);
+    const size_t row_bytes = sizeof(float) * d_;
+    auto rotate_rows = [&](const float* raw, float* to, size_t cnt) {
+        if (trained_) launch_rotate_to_assign(raw, d_, m_dev_.get(), to, d_, cnt, d_, d_, stream_);
+        else launch_gemm_nt(raw, d_, m_dev_.get(), d_, to, d_, cnt, d_, d_, stream_);
     };
     if (src_on_device && !idx) {
-        if (rotate) ensure_rotation();
-        if (as_it_is) SKM_CUDA(cudaMemcpyAsync(dst, src, row_bytes * n, cudaMemcpyDeviceToDevice, stream_));
-        else place(src, dst, n);
+        if (rotate) {
+            ensure_rotation();
+            rotate_rows(src, dst, n);
+        } else {
+            SKM_CUDA(cudaMemcpyAsync(dst, src, row_bytes * n, cudaMemcpyDeviceToDevice, stream_));
+        }
         return;
     }
     if (src_on_device) {
@@ -386,21 +373,21 @@ void Engine::load_rows(const float* src, bool src_on_device, const size_t* idx, 
         const size_t rows = chunk_rows_for(d_, n);
         for (size_t r0 = 0; r0 < n; r0 += rows) {
             const size_t cnt = std::min(rows, n - r0);
-            launch_gather_rows(src, idx_dev.get() + r0, as_it_is ? dst + r0 * d_ : raw.ensure(rows * user_d_), cnt, user_d_, stream_);
-            if (!as_it_is) place(raw.get(), dst + r0 * d_, cnt);
+            launch_gather_rows(src, idx_dev.get() + r0, rotate ? raw.ensure(rows * d_) : dst + r0 * d_, cnt, d_, stream_);
+            if (rotate) rotate_rows(raw.get(), dst + r0 * d_, cnt);
         }
         return;
     }
     const size_t rows = streamed_rows(n);
     RowPipe pipe(stage_, copy_stream_, stream_);
-    if (!as_it_is) pipe.reserve(rows * user_d_, n > rows ? 2 : 1);
+    if (rotate) pipe.reserve(rows * d_, n > rows ? 2 : 1);
     size_t handed = 0;
     for (size_t r0 = 0; r0 < n; r0 += rows) {
         const size_t cnt = std::min(rows, n - r0);
-        const float* raw = pipe.upload(as_it_is ? dst + r0 * d_ : nullptr, idx ? src : src + r0 * user_d_, idx ? idx + r0 : nullptr, cnt, row_bytes);
+        const float* raw = pipe.upload(rotate ? nullptr : dst + r0 * d_, idx ? src : src + r0 * d_, idx ? idx + r0 : nullptr, cnt, row_bytes);
         if (rotate) ensure_rotation();
         pipe.arrive();
-        if (!as_it_is) place(raw, dst + r0 * d_, cnt);
+        if (rotate) rotate_rows(raw, dst + r0 * d_, cnt);
         pipe.used();
         const size_t done = r0 + cnt;
         if (after_rows && (done - handed >= piece || done == n)) {
@@ -418,9 +405,9 @@ size_t Engine::streamed_rows(size_t n) const {
 }
 
 // Exact assignment of device rows: knn, dist (may be null: rows with one candidate are then not read again), and the full norms of both sides.
-void Engine::exact_assignment(const float* x, size_t n, const float* c, size_t k, size_t d, float* norms_x, bool norms_known, float* norms_c, uint32_t* knn, float* dist) {
-    const AssignRoute route = assign_route(n, k, d);
-    if (route == AssignRoute::filter && exact_.begin(c, k, d, n, n, norms_c, stream_)) {
+void Engine::exact_assignment(const float* x, size_t n, const float* c, size_t k, float* norms_x, bool norms_known, float* norms_c, uint32_t* knn, float* dist) {
+    const AssignRoute route = assign_route(n, k, d_);
+    if (route == AssignRoute::filter && exact_.begin(c, k, d_, n, n, norms_c, stream_)) {
         exact_.rows(x, 0, n, norms_x, knn, dist, stream_);
         exact_.settle_on_device(x, knn, dist, stream_);
         return;
@@ -428,12 +415,12 @@ void Engine::exact_assignment(const float* x, size_t n, const float* c, size_t k
     DeviceBuffer<float> own;
     if (!dist) dist = own.ensure(n);
     if (route == AssignRoute::direct) {
-        direct_.run(x, c, n, k, d, norms_x, norms_c, knn, dist, stream_);
+        direct_.run(x, c, n, k, d_, norms_x, norms_c, knn, dist, stream_);
         return;
     }
-    launch_row_sqnorms(c, k, d, d, norms_c, stream_);
-    if (!norms_known) launch_row_sqnorms(x, n, d, d, norms_x, stream_);
-    launch_assign_full(x, c, n, k, d, norms_x, norms_c, knn, dist, top2_.ensure(n), stream_, y_split_.ensure(2 * k * d));
+    launch_row_sqnorms(c, k, d_, d_, norms_c, stream_);
+    if (!norms_known) launch_row_sqnorms(x, n, d_, d_, norms_x, stream_);
+    launch_assign_full(x, c, n, k, d_, norms_x, norms_c, knn, dist, top2_.ensure(n), stream_, y_split_.ensure(2 * k * d_));
 }
 
 void Engine::prepare_update_workspace(size_t n, size_t k) {
@@ -460,7 +447,7 @@ void Engine::generate_centroids_from_host(const float* data, bool on_device, siz
     std::vector<size_t> own;
     if (!precomputed) own = forgy_indices(n_points_global, k_cur, cfg_.seed);
     const std::vector<size_t>& idx = precomputed ? *precomputed : own;
-    float* raw = init_raw_.ensure(k_cur * user_d_);
+    float* raw = init_raw_.ensure(k_cur * d_);
     const bool sharded = sharded_();
     const size_t n_local = n_samples_;
     if (on_device) {
@@ -473,27 +460,25 @@ void Engine::generate_centroids_from_host(const float* data, bool on_device, siz
             idx_host[i] = g;
         }
         SKM_CUDA(cudaMemcpyAsync(init_idx_dev_.ensure(k_cur), idx_host, sizeof(uint64_t) * k_cur, cudaMemcpyHostToDevice, stream_));
-        launch_gather_rows(data, init_idx_dev_.get(), raw, k_cur, user_d_, stream_);
+        launch_gather_rows(data, init_idx_dev_.get(), raw, k_cur, d_, stream_);
     } else if (!sharded) {
-        stage_.upload(raw, data, idx.data(), k_cur, sizeof(float) * user_d_, stream_);
+        stage_.upload(raw, data, idx.data(), k_cur, sizeof(float) * d_, stream_);
     } else {
-        float* host = init_rows_host_.ensure(k_cur * user_d_);
+        float* host = init_rows_host_.ensure(k_cur * d_);
 #pragma omp parallel for
         for (size_t i = 0; i < k_cur; ++i) {
             size_t g = idx[i];
             const bool mine = g >= shard_row_offset_ && g < shard_row_offset_ + n_local;
             g -= shard_row_offset_;
-            if (mine) std::memcpy(host + i * user_d_, data + g * user_d_, sizeof(float) * user_d_);
-            else std::memset(host + i * user_d_, 0, sizeof(float) * user_d_);
+            if (mine) std::memcpy(host + i * d_, data + g * d_, sizeof(float) * d_);
+            else std::memset(host + i * d_, 0, sizeof(float) * d_);
         }
-        SKM_CUDA(cudaMemcpyAsync(raw, host, sizeof(float) * k_cur * user_d_, cudaMemcpyHostToDevice, stream_));
+        SKM_CUDA(cudaMemcpyAsync(raw, host, sizeof(float) * k_cur * d_, cudaMemcpyHostToDevice, stream_));
     }
-    if (sharded) allreduce(raw, k_cur * user_d_, 0);
+    if (sharded) allreduce(raw, k_cur * d_, 0);
     if (rotate) {
         ensure_rotation();
-        launch_gemm_nt(raw, user_d_, m_dev_.get(), user_d_, c_prev_.get(), d_, k_cur, d_, user_d_, stream_);
-    } else if (d_ != user_d_) {
-        launch_move_gap(raw, k_cur, user_d_, c_prev_.get(), d_, vertical_dims_, stream_);
+        launch_gemm_nt(raw, d_, m_dev_.get(), d_, c_prev_.get(), d_, k_cur, d_, d_, stream_);
     } else {
         SKM_CUDA(cudaMemcpyAsync(c_prev_.get(), raw, sizeof(float) * k_cur * d_, cudaMemcpyDeviceToDevice, stream_));
     }
@@ -937,9 +922,7 @@ void run_pruned_pass_sorted(const PrunedParams& p, PrunePassBuffers& b, float ra
 
 // A point that keeps one centroid in so many costs the walk more than a row of the dense chain.  One B200, ten iterations, with the
 // line at one in 44 / 22 / 16 / 12: first test + walk + chain of 1M x 1024, k = 4000: 73 / 63 / 59 / 57 ms; 250k x 1536, k = 2048:
-// 13.0 / 12.0 / 12.5 / 13.0; 30 000 x 768, k = 1000: 2.0 / 2.0 / 2.1 / 2.3, of which walk and chain overlap.  With the chain from fp16
-// halves a whole Train of the first with the line at one in 40 / 26 / 18 / 12 / 6: 98 / 90 / 88 / 82 / 88 ms; of the others no difference
-// but at 6 (29.9 ms against 28.7 - 29.1, and 7.5 against 6.9 - 7.0).
+// 13.0 / 12.0 / 12.5 / 13.0; 30 000 x 768, k = 1000: 2.0 / 2.0 / 2.1 / 2.3, of which walk and chain overlap.
 constexpr size_t kHardShare = 12;
 
 // Share of (point, sampled centroid) pairs passing the first test from which the automatic choice takes the ordered chain
@@ -1272,7 +1255,7 @@ bool Engine::split(size_t n_samples_global, size_t k_cur) {
     if (ops.empty()) return false;
     static_assert(sizeof(SplitOp) == sizeof(SplitOpDev), "layout");
     SKM_CUDA(cudaMemcpyAsync(split_ops_dev_.ensure(ops.size()), ops.data(), sizeof(SplitOp) * ops.size(), cudaMemcpyHostToDevice, stream_));
-    launch_apply_split_ops(c_cur_.get(), d_, shifted_, split_ops_dev_.get(), ops.size(), stream_);
+    launch_apply_split_ops(c_cur_.get(), d_, split_ops_dev_.get(), ops.size(), stream_);
     sync();  // `ops` must outlive the asynchronous copy
     return true;
 }
@@ -1329,7 +1312,7 @@ void Engine::run_iteration(bool gemm_only, const IterationInput& in, size_t iter
             if (exact_open_) exact_.settle_on_device(in.x, assignments_.get(), distances_.get(), stream_);
             exact_open_ = false;
         } else {
-            exact_assignment(in.x, n, c_prev_.get(), k_cur, d_, norms, in.full_norms, centroid_norms_.get(), assignments_.get(), distances_.get());
+            exact_assignment(in.x, n, c_prev_.get(), k_cur, norms, in.full_norms, centroid_norms_.get(), assignments_.get(), distances_.get());
         }
     } else {
         launch_row_sqnorms(c_prev_.get(), k_cur, d_, partial_d_, centroid_norms_.get(), stream_);
@@ -1360,7 +1343,7 @@ void Engine::run_iteration(bool gemm_only, const IterationInput& in, size_t iter
     float avg_not_pruned = -1.0f;
     const uint32_t old_partial_d = partial_d_;
     if (!gemm_only) {
-        const TuneResult t = tune_partial_d(told.not_pruned, in.n_samples_global, k_cur, partial_d_, vertical_dims_, cfg_.min_not_pruned_pct, cfg_.max_not_pruned_pct,
+        const TuneResult t = tune_partial_d(told.not_pruned, in.n_samples_global, k_cur, partial_d_, vertical_d_, cfg_.min_not_pruned_pct, cfg_.max_not_pruned_pct,
                                             cfg_.adjustment_factor_for_partial_d);
         avg_not_pruned = t.avg_not_pruned_pct;
         partial_d_ = t.new_partial_d;
@@ -1383,12 +1366,12 @@ void Engine::run_iteration(bool gemm_only, const IterationInput& in, size_t iter
         snap.n_samples = n;
         snap.n_clusters = k_cur;
         snap.partial_d_next = partial_d_;
-        snap.centroids.resize(k_cur * user_d_);
+        snap.centroids.resize(k_cur * d_);
         snap.assign.resize(n);
         snap.dist.resize(n);
         snap.sizes_pre.assign(counts_host(), counts_host() + k_cur);
         snap.sizes_post.assign(sizes_host_.begin(), sizes_host_.begin() + k_cur);
-        without_gap(c_cur_.get(), k_cur, snap.centroids.data());
+        SKM_CUDA(cudaMemcpyAsync(snap.centroids.data(), c_cur_.get(), sizeof(float) * k_cur * d_, cudaMemcpyDeviceToHost, stream_));
         SKM_CUDA(cudaMemcpyAsync(snap.assign.data(), assignments_.get(), sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, stream_));
         SKM_CUDA(cudaMemcpyAsync(snap.dist.data(), distances_.get(), sizeof(float) * n, cudaMemcpyDeviceToHost, stream_));
         sync();
@@ -1475,7 +1458,7 @@ void Engine::train_flat(const float* data, size_t n, bool on_device, const float
     n_samples_ = sharded_() ? n : n_samples_global;
     const bool rotate = !cfg_.data_already_rotated;
     if (rotate || cfg_.unrotate_centroids) start_rotation(!on_device);
-    partial_d_ = initial_partial_d(vertical_dims_);
+    partial_d_ = initial_partial_d(vertical_d_);
     // The Forgy shuffle runs over all n_samples indices with std::mt19937 (a tenth of a second at 1e7): on a thread of
     // its own, while this one allocates the buffers and starts the rotation.
     std::future<std::vector<size_t>> forgy = std::async(std::launch::async, [n_samples_global, k = k_, seed = cfg_.seed] { return forgy_indices(n_samples_global, k, seed); });
@@ -1555,7 +1538,7 @@ void Engine::train_flat(const float* data, size_t n, bool on_device, const float
     // Ground truth for the recall figure (superkmeans.h:243-274): needs the full norms.
     if (n_queries > 0) prepare_recall(queries, n_queries, rotate);
 
-    const bool always_gemm_only = user_d_ < kDimensionThresholdForPruning || cfg_.use_blas_only || k_ <= kNClustersThresholdForPruning;
+    const bool always_gemm_only = d_ < kDimensionThresholdForPruning || cfg_.use_blas_only || k_ <= kNClustersThresholdForPruning;
     float best_recall = 0.0f;
     size_t iters_without_improvement = 0;
     for (size_t iter = 0; iter < cfg_.iters; ++iter) {
@@ -1633,25 +1616,12 @@ void Engine::output_centroids(float* out_host) {
     DeviceBuffer<float> tmp;
     if (cfg_.unrotate_centroids) {
         ensure_rotation();
-        launch_gemm_nt(c, d_, mt_dev_.get(), d_, tmp.ensure(k_ * user_d_), user_d_, k_, user_d_, d_, stream_);
-        c = tmp.get();
-    } else if (d_ != user_d_) {
-        launch_move_gap(c, k_, d_, tmp.ensure(k_ * user_d_), user_d_, vertical_dims_, stream_);
+        launch_gemm_nt(c, d_, mt_dev_.get(), d_, tmp.ensure(k_ * d_), d_, k_, d_, d_, stream_);
         c = tmp.get();
     }
     tell_error();
-    stage_.download(out_host, c, sizeof(float) * k_ * user_d_, stream_);
+    stage_.download(out_host, c, sizeof(float) * k_ * d_, stream_);
     check_told_error();
-}
-
-// Rows of the engine's width as the caller knows them.
-void Engine::without_gap(const float* rows_dev, size_t n, float* out_host) {
-    DeviceBuffer<float> tmp;
-    if (d_ != user_d_) {
-        launch_move_gap(rows_dev, n, d_, tmp.ensure(n * user_d_), user_d_, vertical_dims_, stream_);
-        rows_dev = tmp.get();
-    }
-    stage_.download(out_host, rows_dev, sizeof(float) * n * user_d_, stream_);
 }
 
 // The error word of the tensor-core kernels, on its way to the host ahead of a copy or a wait that the caller makes anyway, and
@@ -1676,7 +1646,7 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
     const size_t n_all = n_samples_;
     const bool rotate = !cfg_.data_already_rotated;
     if (rotate || cfg_.unrotate_centroids) start_rotation(!on_device);
-    partial_d_ = initial_partial_d(vertical_dims_);
+    partial_d_ = initial_partial_d(vertical_d_);
     const uint32_t initial_pd = partial_d_;
     // The shuffles behind the first centroids and the sample run on threads of their own meanwhile.
     std::future<std::vector<size_t>> meso_forgy = std::async(std::launch::async, [n_all, k = n_meso_, seed = cfg_.seed] { return forgy_indices(n_all, k, seed); });
@@ -1713,7 +1683,7 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
     SKM_CUDA(cudaMemcpyAsync(full_norms_.get(), data_norms_.get(), sizeof(float) * n_all, cudaMemcpyDeviceToDevice, stream_));
 
     {
-        const bool always_gemm_only = user_d_ < kDimensionThresholdForPruning || cfg_.use_blas_only || n_meso_ <= kNClustersThresholdForPruning;
+        const bool always_gemm_only = d_ < kDimensionThresholdForPruning || cfg_.use_blas_only || n_meso_ <= kNClustersThresholdForPruning;
         IterationInput in{x_rot_.get(), n_all, n_all, n_meso_, data_norms_.get()};
         for (size_t iter = 0; iter < cfg_.iters_mesoclustering; ++iter) {
             const bool gemm_only = (iter == 0) || always_gemm_only;
@@ -1756,7 +1726,7 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
     const std::vector<size_t> fine_nums = arrange_fine_clusters(k_, n_meso_, n_all, meso_sizes);
     std::vector<size_t> rows_of(n_meso_);   // members whose index the partition holds
     for (size_t m = 0; m < n_meso_; ++m) rows_of[m] = std::min<size_t>(meso_sizes[m], n_all - std::min(offsets[m], n_all));
-    auto gemm_only = [&](size_t n_fine) { return user_d_ < kDimensionThresholdForPruning || cfg_.use_blas_only || n_fine <= kNClustersThresholdForPruning; };
+    auto gemm_only = [&](size_t n_fine) { return d_ < kDimensionThresholdForPruning || cfg_.use_blas_only || n_fine <= kNClustersThresholdForPruning; };
     // Mesoclusters that never prune share their launches (train_fine_run); snapshots are per mesocluster and iteration.
     bool room = true;   // for the rows of many
     auto shares = [&](size_t m) { return room && fine_nums[m] > 0 && rows_of[m] >= fine_nums[m] && gemm_only(fine_nums[m]) && !trace_on_ && tc::enabled() && d_ <= 16384; };
@@ -1838,13 +1808,13 @@ void Engine::train_hierarchical(const float* data, size_t n, bool on_device, flo
 
     // ---- phase 3: refinement over all clusters (:434-516)
     n_samples_ = n_all;
-    partial_d_ = std::max<uint32_t>(kMinPartialD, vertical_dims_ / 3);
+    partial_d_ = std::max<uint32_t>(kMinPartialD, vertical_d_ / 3);
     SKM_CUDA(cudaMemcpyAsync(c_cur_.get(), final_centroids_.get(), sizeof(float) * k_ * d_, cudaMemcpyDeviceToDevice, stream_));   // SetupCentroids (:788-815)
     launch_pdxify(c_cur_.get(), c_pdx_.get(), c_aux_.get(), k_, d_, vertical_d_, stream_);
     SKM_CUDA(cudaMemcpyAsync(c_prev_.get(), final_centroids_.get(), sizeof(float) * k_ * d_, cudaMemcpyDeviceToDevice, stream_));
     SKM_CUDA(cudaMemcpyAsync(assignments_.get(), final_assignments_.get(), sizeof(uint32_t) * n_all, cudaMemcpyDeviceToDevice, stream_));
     {
-        const bool always_gemm_only = user_d_ < kDimensionThresholdForPruning || k_ <= kNClustersThresholdForPruning;
+        const bool always_gemm_only = d_ < kDimensionThresholdForPruning || k_ <= kNClustersThresholdForPruning;
         IterationInput in{x_rot_.get(), n_all, n_all, k_, data_norms_.get()};
         for (size_t iter = 0; iter < cfg_.iters_refinement; ++iter) {
             // data_norms_ still holds whatever the mesoclustering left; GEMM-only needs full norms.
@@ -1873,7 +1843,7 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
     DeviceBuffer<float> c_dev_own, cn;
     const float* c_dev = centroids;
     if (!on_device) {
-        stage_.upload(c_dev_own.ensure(n_centroids * user_d_), centroids, nullptr, n_centroids, sizeof(float) * user_d_, stream_);
+        stage_.upload(c_dev_own.ensure(n_centroids * d_), centroids, nullptr, n_centroids, sizeof(float) * d_, stream_);
         c_dev = c_dev_own.get();
     }
     cn.ensure(n_centroids);
@@ -1881,42 +1851,42 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
         DeviceBuffer<float> xn;
         {
             PhaseScope ps(*this, PH_ASSIGN_FULL);
-            exact_assignment(vectors, n, c_dev, n_centroids, user_d_, xn.ensure(n), false, cn.get(), out, nullptr);
+            exact_assignment(vectors, n, c_dev, n_centroids, xn.ensure(n), false, cn.get(), out, nullptr);
         }
         // (a direct call waits for nothing that can run out)
-        const bool direct_call = assign_route(n, n_centroids, user_d_) == AssignRoute::direct;
+        const bool direct_call = assign_route(n, n_centroids, d_) == AssignRoute::direct;
         if (!direct_call) tell_error();
         sync();
         if (!direct_call) check_told_error();
         return;
     }
-    const AssignRoute route = assign_route(n, n_centroids, user_d_);
+    const AssignRoute route = assign_route(n, n_centroids, d_);
     const size_t rows = streamed_rows(n);
-    bool filtered = route == AssignRoute::filter && exact_.begin(c_dev, n_centroids, user_d_, n, rows, cn.get(), stream_);
+    bool filtered = route == AssignRoute::filter && exact_.begin(c_dev, n_centroids, d_, n, rows, cn.get(), stream_);
     const bool begun = filtered, direct = route == AssignRoute::direct;
-    if (!filtered && !direct) launch_row_sqnorms(c_dev, n_centroids, user_d_, user_d_, cn.get(), stream_);
+    if (!filtered && !direct) launch_row_sqnorms(c_dev, n_centroids, d_, d_, cn.get(), stream_);
     DeviceBuffer<float> xn, dist;
     DeviceBuffer<uint32_t> knn;
     RowPipe pipe(stage_, copy_stream_, stream_);
-    pipe.reserve(rows * user_d_, n > rows ? 2 : 1);
+    pipe.reserve(rows * d_, n > rows ? 2 : 1);
     xn.ensure(rows);
     dist.ensure(rows);
     knn.ensure(n);
     std::optional<PhaseScope> phase(std::in_place, *this, PH_ASSIGN_FULL);
     for (size_t r0 = 0; r0 < n; r0 += rows) {
         const size_t cnt = std::min(rows, n - r0);
-        const float* xb = pipe.upload(nullptr, vectors + r0 * user_d_, nullptr, cnt, sizeof(float) * user_d_);
+        const float* xb = pipe.upload(nullptr, vectors + r0 * d_, nullptr, cnt, sizeof(float) * d_);
         // Listed rows have to cross once more.  (What the first piece came to is known by now; below a few milliseconds of copies the
         // question costs more than it saves.)
-        if (filtered && r0 == rows && n * user_d_ * sizeof(float) >= kAskFrom && exact_.in_vain(r0, stream_)) filtered = false;
+        if (filtered && r0 == rows && n * d_ * sizeof(float) >= kAskFrom && exact_.in_vain(r0, stream_)) filtered = false;
         pipe.arrive();
         if (filtered) {
             exact_.rows(xb, r0, cnt, xn.get(), knn.get() + r0, nullptr, stream_);
         } else if (direct) {
-            direct_.run(xb, c_dev, cnt, n_centroids, user_d_, xn.get(), cn.get(), knn.get() + r0, dist.get(), stream_);
+            direct_.run(xb, c_dev, cnt, n_centroids, d_, xn.get(), cn.get(), knn.get() + r0, dist.get(), stream_);
         } else {
-            launch_row_sqnorms(xb, cnt, user_d_, user_d_, xn.get(), stream_);
-            launch_assign_full(xb, c_dev, cnt, n_centroids, user_d_, xn.get(), cn.get(), knn.get() + r0, dist.get(), top2_.ensure(rows), stream_, y_split_.ensure(2 * n_centroids * user_d_));
+            launch_row_sqnorms(xb, cnt, d_, d_, xn.get(), stream_);
+            launch_assign_full(xb, c_dev, cnt, n_centroids, d_, xn.get(), cn.get(), knn.get() + r0, dist.get(), top2_.ensure(rows), stream_, y_split_.ensure(2 * n_centroids * d_));
         }
         pipe.used();
     }
@@ -1928,8 +1898,8 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
         const std::vector<size_t> idx(idx32.begin(), idx32.end());
         for (size_t at = 0; at < listed; at += per) {
             const size_t cnt = std::min(per, listed - at);
-            float* xl = pipe.buffer(0).ensure(cnt * user_d_);
-            stage_.upload(xl, vectors, idx.data() + at, cnt, sizeof(float) * user_d_, stream_);
+            float* xl = pipe.buffer(0).ensure(cnt * d_);
+            stage_.upload(xl, vectors, idx.data() + at, cnt, sizeof(float) * d_, stream_);
             exact_.finish(xl, at, cnt, knn.get(), nullptr, stream_);
         }
     }
@@ -1948,7 +1918,7 @@ void Engine::assign(const float* vectors, const float* centroids, size_t n, size
 void Engine::assign_training_points(const float* vectors, const float* centroids, size_t n, size_t n_centroids, bool on_device, uint32_t* out) {
     Entry entry(device_, stream_);
     if (!trained_) throw std::runtime_error("AssignTrainingPoints requires SuperKMeans to be trained first");
-    if (cfg_.use_blas_only || user_d_ < kDimensionThresholdForPruning || k_ <= kNClustersThresholdForPruning) {
+    if (cfg_.use_blas_only || d_ < kDimensionThresholdForPruning || k_ <= kNClustersThresholdForPruning) {
         if (!cfg_.suppress_warnings) {
             std::cout << "WARNING: AssignTrainingPoints cannot use pruning, falling back to brute force Assign" << std::endl;
         }
@@ -1957,7 +1927,7 @@ void Engine::assign_training_points(const float* vectors, const float* centroids
     }
     if (n == 0) return;
     if (on_device) wait_for_default_stream();
-    partial_d_ = initial_partial_d(vertical_dims_);
+    partial_d_ = initial_partial_d(vertical_d_);
     launch_row_sqnorms(c_cur_.get(), k_, d_, partial_d_, centroid_norms_.get(), stream_);
 
     // Seeds: one starting centroid per vector.  With all rows trained they are the assignments of Train, which the
@@ -1985,11 +1955,11 @@ void Engine::assign_training_points(const float* vectors, const float* centroids
         } else {
             // Two-level seeds (:505-542): cluster the centroids into sqrt(k) groups and start every
             // unsampled vector at one representative centroid of its group.
-            std::vector<float> cent_host(n_centroids * user_d_), vec_host_own;
+            std::vector<float> cent_host(n_centroids * d_), vec_host_own;
             if (on_device) {
-                SKM_CUDA(cudaMemcpy(cent_host.data(), centroids, sizeof(float) * n_centroids * user_d_, cudaMemcpyDeviceToHost));
+                SKM_CUDA(cudaMemcpy(cent_host.data(), centroids, sizeof(float) * n_centroids * d_, cudaMemcpyDeviceToHost));
             } else {
-                std::memcpy(cent_host.data(), centroids, sizeof(float) * n_centroids * user_d_);
+                std::memcpy(cent_host.data(), centroids, sizeof(float) * n_centroids * d_);
             }
             skm_config tmp{};
             skm_default_config(&tmp, 0);
@@ -2002,12 +1972,12 @@ void Engine::assign_training_points(const float* vectors, const float* centroids
             tmp.angular = cfg_.angular;
             tmp.data_already_rotated = cfg_.data_already_rotated;
             const size_t n_meso = static_cast<size_t>(std::sqrt(n_centroids));
-            Engine nested(tmp, n_meso, user_d_, false, device_);
+            Engine nested(tmp, n_meso, d_, false, device_);
             if (rotation_ready_) {
                 ensure_rotation_host();
                 nested.set_rotation(rotation_host_.data());
             }
-            std::vector<float> meso_centroids(n_meso * user_d_);
+            std::vector<float> meso_centroids(n_meso * d_);
             nested.train(cent_host.data(), n_centroids, false, nullptr, 0, meso_centroids.data());
             std::vector<uint32_t> meso_assign(n), cent_to_meso(n_centroids);
             nested.assign(vectors, meso_centroids.data(), n, n_meso, false, meso_assign.data());
@@ -2042,7 +2012,7 @@ void Engine::assign_training_points(const float* vectors, const float* centroids
     np.ensure(rows);
     for (size_t r0 = 0; r0 < n; r0 += rows) {
         const size_t cnt = std::min(rows, n - r0);
-        load_rows(vectors + r0 * user_d_, on_device, nullptr, cnt, !cfg_.data_already_rotated, xr.get());
+        load_rows(vectors + r0 * d_, on_device, nullptr, cnt, !cfg_.data_already_rotated, xr.get());
         PrunedParams p = pruned_params(IterationInput{xr.get(), cnt, cnt, k_, xn.get()});
         p.y = c_cur_.get();
         p.knn = knn + r0;
@@ -2072,7 +2042,7 @@ void Engine::get_distances(float* out, size_t n) {
 void Engine::get_rotated_centroids(float* out) {
     Entry entry(device_, stream_);
     if (!trained_) throw std::runtime_error("the model has not been trained");
-    without_gap(c_cur_.get(), k_, out);
+    stage_.download(out, c_cur_.get(), sizeof(float) * k_ * d_, stream_);
 }
 
 // -------------------------------------------------------------------------------------------------

@@ -180,7 +180,7 @@ class Engine {
     void get_rotated_centroids(float* out);
 
     size_t n_clusters() const { return k_; }
-    size_t dimensionality() const { return user_d_; }
+    size_t dimensionality() const { return d_; }
     const skm_config& config() const { return cfg_; }
     bool trained() const { return trained_; }
     float sampling_fraction() const { return cfg_.sampling_fraction; }
@@ -243,9 +243,6 @@ class Engine {
     void start_rotation(bool beside);
     void make_rotation(cudaStream_t stream);
     void drop_rotation();
-    float* plain_rotation() { return d_ == user_d_ ? m_dev_.ensure(d_ * d_) : m_plain_.ensure(user_d_ * user_d_); }
-    void place_rotation(cudaStream_t stream);
-    void without_gap(const float* rows_dev, size_t n, float* out_host);
     void ensure_rotation();
     void ensure_rotation_host();
     // after_rows(r0, cnt), if given, is called (host side, work enqueued on stream_) whenever rows [r0, r0 + cnt) of dst
@@ -254,7 +251,7 @@ class Engine {
     void load_rows(const float* src, bool src_on_device, const size_t* idx, size_t n, bool rotate, float* dst,
                    const std::function<void(size_t, size_t)>& after_rows = nullptr, size_t piece = 0);
     void wait_for_default_stream();
-    void exact_assignment(const float* x, size_t n, const float* c, size_t k, size_t d, float* norms_x, bool norms_known, float* norms_c, uint32_t* knn, float* dist);
+    void exact_assignment(const float* x, size_t n, const float* c, size_t k, float* norms_x, bool norms_known, float* norms_c, uint32_t* knn, float* dist);
     size_t streamed_rows(size_t n) const;
     void prepare_update_workspace(size_t n, size_t k);
     void run_iteration(bool gemm_only, const IterationInput& in, size_t iter_idx, bool is_first, std::vector<skm_iter_stats>& target);
@@ -296,11 +293,7 @@ class Engine {
     std::vector<Snapshot> trace_;
 
     skm_config cfg_;
-    // The caller's rows have user_d_ values.  The engine's own (rotated rows, centroids) have d_, a multiple of four, so that TMA and 16-byte
-    // loads can address them: up to three zeros stand behind the leading dimensions (vertical_dims_ of them), which changes no
-    // distance and no norm.  vertical_d_ counts the zeros, dimensions d' and what decides about them do not.
-    size_t k_, user_d_, d_;
-    size_t shifted_;                // columns from here on hold a dimension of the other parity
+    size_t k_, d_;
     bool hierarchical_;
     int device_;
     cudaStream_t stream_ = nullptr;
@@ -320,7 +313,7 @@ class Engine {
 
     // pruner state
     float epsilon0_;
-    std::vector<float> rotation_host_;  // user_d_ x user_d_, empty until needed (a matrix made on the device is fetched on demand)
+    std::vector<float> rotation_host_;  // d x d, empty until needed (a matrix made on the device is fetched on demand)
     struct Drawing;
     std::unique_ptr<Drawing> drawing_;   // while a matrix is being made
     std::future<void> rotation_made_;    // valid from when that is done on a thread of its own
@@ -328,9 +321,8 @@ class Engine {
     std::atomic<RotationState> rotation_state_{RotationState::none};
     cudaEvent_t rotation_event_ = nullptr;   // behind its last kernel
     bool rotation_ready_ = false;
-    DeviceBuffer<float> m_dev_, mt_dev_, ratios_dev_;   // d_ x user_d_, user_d_ x d_, d_ + 1
-    DeviceBuffer<float> m_plain_;                       // user_d_ x user_d_, where that is not m_dev_
-    uint32_t vertical_d_ = 0, vertical_dims_ = 0, horizontal_d_ = 0, partial_d_ = 0;
+    DeviceBuffer<float> m_dev_, mt_dev_, ratios_dev_;
+    uint32_t vertical_d_ = 0, horizontal_d_ = 0, partial_d_ = 0;
 
     // iteration state
     bool trained_ = false;

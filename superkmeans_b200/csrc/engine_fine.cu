@@ -39,11 +39,11 @@ __global__ void __launch_bounds__(256) group_means_kernel(float* __restrict__ c,
 }
 
 // Split operations of a group in list order, a thread per dimension (see apply_split_ops_kernel).
-__global__ void group_split_kernel(float* __restrict__ c, size_t d, size_t shifted, const SplitOpDev* __restrict__ ops, const Group* __restrict__ groups) {
+__global__ void group_split_kernel(float* __restrict__ c, size_t d, const SplitOpDev* __restrict__ ops, const Group* __restrict__ groups) {
     const Group g = groups[blockIdx.y];
     const size_t j = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (j >= d) return;
-    for (uint32_t o = g.op0; o < g.op0 + g.ops; ++o) apply_split_op(c, d, j, (j & 1) == (j >= shifted ? 1 : 0), ops[o]);
+    for (uint32_t o = g.op0; o < g.op0 + g.ops; ++o) apply_split_op(c, d, j, ops[o]);
 }
 
 // normalize_rows_kernel for the active groups.
@@ -225,7 +225,7 @@ void Engine::train_fine_run(size_t first, size_t last, const std::vector<size_t>
                 static_assert(sizeof(SplitOp) == sizeof(SplitOpDev), "layout");
                 stage_.upload(split_ops_dev_.ensure(ops.size()), ops.data(), nullptr, ops.size(), sizeof(SplitOp), stream_);
                 stage_.upload(groups_dev.get(), groups.data(), nullptr, n_groups, sizeof(Group), stream_);
-                group_split_kernel<<<dim3(static_cast<unsigned>((d_ + 127) / 128), static_cast<unsigned>(n_groups)), 128, 0, stream_>>>(c_cur_.get(), d_, shifted_, split_ops_dev_.get(),
+                group_split_kernel<<<dim3(static_cast<unsigned>((d_ + 127) / 128), static_cast<unsigned>(n_groups)), 128, 0, stream_>>>(c_cur_.get(), d_, split_ops_dev_.get(),
                                                                                                                                         groups_dev.get());
                 SKM_LAUNCH_CHECK();
             }

@@ -972,15 +972,15 @@ void launch_update(const float* x, const uint32_t* assign, size_t n, size_t k, s
 // Consolidation
 // =================================================================================================
 // Every thread owns one dimension and replays the row operations in list order.
-__global__ void apply_split_ops_kernel(float* __restrict__ c, size_t d, size_t shifted, const SplitOpDev* __restrict__ ops, size_t n_ops) {
+__global__ void apply_split_ops_kernel(float* __restrict__ c, size_t d, const SplitOpDev* __restrict__ ops, size_t n_ops) {
     const size_t j = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (j >= d) return;
-    for (size_t o = 0; o < n_ops; ++o) apply_split_op(c, d, j, (j & 1) == (j >= shifted ? 1 : 0), ops[o]);
+    for (size_t o = 0; o < n_ops; ++o) apply_split_op(c, d, j, ops[o]);
 }
 
-void launch_apply_split_ops(float* c, size_t d, size_t shifted, const SplitOpDev* ops, size_t n_ops, cudaStream_t stream) {
+void launch_apply_split_ops(float* c, size_t d, const SplitOpDev* ops, size_t n_ops, cudaStream_t stream) {
     if (n_ops == 0) return;
-    apply_split_ops_kernel<<<static_cast<unsigned>((d + 127) / 128), 128, 0, stream>>>(c, d, shifted, ops, n_ops);
+    apply_split_ops_kernel<<<static_cast<unsigned>((d + 127) / 128), 128, 0, stream>>>(c, d, ops, n_ops);
     SKM_LAUNCH_CHECK();
 }
 
@@ -1278,36 +1278,6 @@ void launch_gather_rows(const float* in, const uint64_t* idx, float* out, size_t
     const unsigned grid = static_cast<unsigned>((n_out + 7) / 8);
     if (d % 4 == 0 && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) gather_rows_kernel<true><<<grid, 256, 0, stream>>>(in, idx, out, n_out, d);
     else gather_rows_kernel<false><<<grid, 256, 0, stream>>>(in, idx, out, n_out, d);
-    SKM_LAUNCH_CHECK();
-}
-
-__global__ void __launch_bounds__(256) move_gap_kernel(const float* __restrict__ in, size_t n, size_t d_in, float* __restrict__ out, size_t d_out, size_t at) {
-    const size_t row = static_cast<size_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
-    if (row >= n) return;
-    for (size_t j = threadIdx.x & 31; j < d_out; j += 32) {
-        // (unsigned wrap when the gap is taken out)
-        const size_t from = j < at ? j : j + d_in - d_out;
-        out[row * d_out + j] = d_out > d_in && j >= at && j < at + (d_out - d_in) ? 0.f : __ldg(in + row * d_in + from);
-    }
-}
-
-void launch_move_gap(const float* in, size_t n, size_t d_in, float* out, size_t d_out, size_t at, cudaStream_t stream) {
-    if (n == 0) return;
-    move_gap_kernel<<<static_cast<unsigned>((n + 7) / 8), 256, 0, stream>>>(in, n, d_in, out, d_out, at);
-    SKM_LAUNCH_CHECK();
-}
-
-__global__ void __launch_bounds__(256) rotation_with_gap_kernel(const float* __restrict__ m, size_t d, size_t d_gap, size_t at, float* __restrict__ m_gap, float* __restrict__ mt_gap) {
-    const size_t j = static_cast<size_t>(blockIdx.x) * 256 + threadIdx.x, i = blockIdx.y;
-    if (j >= d) return;
-    const size_t gap = d_gap - d;
-    const float v = i >= at && i < at + gap ? 0.f : __ldg(m + (i < at ? i : i - gap) * d + j);
-    m_gap[i * d + j] = v;
-    mt_gap[j * d_gap + i] = v;
-}
-
-void launch_rotation_with_gap(const float* m, size_t d, size_t d_gap, size_t at, float* m_gap, float* mt_gap, cudaStream_t stream) {
-    rotation_with_gap_kernel<<<dim3(static_cast<unsigned>((d + 255) / 256), static_cast<unsigned>(d_gap)), 256, 0, stream>>>(m, d, d_gap, at, m_gap, mt_gap);
     SKM_LAUNCH_CHECK();
 }
 

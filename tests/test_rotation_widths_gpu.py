@@ -17,6 +17,6 @@ def test_rows_of_any_width_and_magnitude(n, d):
     m = rng.standard_normal((d, d), dtype=np.float32) * (10.0 ** rng.uniform(-3, 3, (d, 1))).astype(np.float32)
     got = skm.engine.rotate(m, x)
     want = x.astype(np.float64) @ m.T.astype(np.float64)
-    # 22 bits of either factor, and at most d / 4 terms one after the other in an accumulator that truncates
+    # 22 bits of either factor; 64 terms one after the other in an accumulator that truncates, then fp32
     scale = np.linalg.norm(x.astype(np.float64), axis=1)[:, None] * np.linalg.norm(m.astype(np.float64), axis=1)
     assert (np.abs(got - want) <= 3e-6 * scale).all()
