@@ -102,6 +102,8 @@ void exclusive_scan_u32(uint32_t* data, size_t n, uint32_t* totals_tmp, cudaStre
 // out[i] = sum_{j < upto} x[i*ld + j]^2
 void launch_row_sqnorms(const float* x, size_t n, size_t ld, size_t upto, float* out, cudaStream_t stream);
 
+int sm_count();   // of the current device
+
 // out[n x n_out] = a[n x k_dim] * b[n_out x k_dim]^T, all row-major with leading dimensions lda,
 // ldb, ldo (NT GEMM).  Used for rotation (b = M) and un-rotation (b = M^T).
 void launch_gemm_nt(const float* a, size_t lda, const float* b, size_t ldb, float* out, size_t ldo, size_t n, size_t n_out, size_t k_dim, cudaStream_t stream);

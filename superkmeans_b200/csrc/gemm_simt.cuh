@@ -129,4 +129,68 @@ __device__ __forceinline__ void gemm_tile_nt(
     gemm_tile_nt_ex<true, false>(A, lda, m_valid, nullptr, B, ldb, n_valid, K, s, acc);
 }
 
+// The same for 32 x 128 tiles, for where tiles of 128 x 128 would leave most of the chip idle: 256 threads, thread (warp, lane) owns rows
+// 4 warp .. 4 warp + 3 and columns lane, lane + 32, lane + 64, lane + 96.  Every sum is made in the same order, so the two give the same
+// bits.  A step is 32 of the reduction's values, which a warp reads along the rows: coalesced whatever the alignment.
+struct GemmSmem32 {
+    float a[2][32][36];
+    float b[2][32][129];
+};
+
+template <bool ZERO_ACC, bool INDIRECT>
+__device__ __forceinline__ void gemm_tile32_nt(
+    const float* __restrict__ A, size_t lda, int m_valid, const uint32_t* row_idx, const float* __restrict__ B, size_t ldb, int n_valid, int K, GemmSmem32& s,
+    float (&acc)[4][4]
+) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (ZERO_ACC) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    }
+    float ra[4], rb[16];
+    auto load = [&](int k) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = warp + 8 * i;
+            ra[i] = r < m_valid && k < K ? __ldg(A + (INDIRECT ? row_idx[r] : static_cast<size_t>(r)) * lda + k) : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int r = warp + 8 * i;
+            rb[i] = r < n_valid && k < K ? __ldg(B + static_cast<size_t>(r) * ldb + k) : 0.f;
+        }
+    };
+    auto store = [&](int buffer) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s.a[buffer][lane][warp + 8 * i] = ra[i];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) s.b[buffer][lane][warp + 8 * i] = rb[i];
+    };
+    const int steps = (K + 31) / 32;
+    load(lane);
+    store(0);
+    __syncthreads();
+    for (int ks = 0; ks < steps; ++ks) {
+        const int cur = ks & 1;
+        const bool more = ks + 1 < steps;
+        if (more) load((ks + 1) * 32 + lane);
+#pragma unroll 8
+        for (int k = 0; k < 32; ++k) {
+            const float4 a = *reinterpret_cast<const float4*>(&s.a[cur][k][warp * 4]);
+            const float av[4] = {a.x, a.y, a.z, a.w};
+            float bv[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) bv[j] = s.b[cur][k][lane + 32 * j];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+        }
+        if (more) store(cur ^ 1);
+        __syncthreads();
+    }
+}
+
 } // namespace skmb

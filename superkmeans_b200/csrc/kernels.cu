@@ -87,6 +87,30 @@ __global__ void __launch_bounds__(256, 2) gemm_nt_kernel(
     }
 }
 
+__global__ void __launch_bounds__(256, 4) gemm_nt_small_kernel(
+    const float* __restrict__ a, size_t lda, const float* __restrict__ b, size_t ldb, float* __restrict__ out, size_t ldo, size_t n, size_t n_out, size_t k_dim
+) {
+    __shared__ GemmSmem32 smem;
+    const size_t row0 = static_cast<size_t>(blockIdx.x) * 32, col0 = static_cast<size_t>(blockIdx.y) * kTileN;
+    const int m_valid = static_cast<int>(min(size_t{32}, n - row0));
+    const int n_valid = static_cast<int>(min(static_cast<size_t>(kTileN), n_out - col0));
+    float acc[4][4];
+    gemm_tile32_nt<true, false>(a + row0 * lda, lda, m_valid, nullptr, b + col0 * ldb, ldb, n_valid, static_cast<int>(k_dim), smem, acc);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (warp * 4 + i < m_valid && lane + 32 * j < n_valid) out[(row0 + warp * 4 + i) * ldo + col0 + lane + 32 * j] = acc[i][j];
+}
+
+int sm_count() {
+    int device = 0, sms = 0;
+    SKM_CUDA(cudaGetDevice(&device));
+    SKM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    return std::max(sms, 1);
+}
+
 void launch_gemm_nt(const float* a, size_t lda, const float* b, size_t ldb, float* out, size_t ldo, size_t n, size_t n_out, size_t k_dim, cudaStream_t stream) {
     if (n == 0 || n_out == 0) return;
     // Tensor cores when TMA can address both operands: the rotation kernel cuts the accumulation into four chains summed
@@ -98,7 +122,14 @@ void launch_gemm_nt(const float* a, size_t lda, const float* b, size_t ldb, floa
     }
     // The point dimension is on grid.x (limit 2^31-1); output columns on grid.y.
     dim3 grid(static_cast<unsigned>((n + kTileM - 1) / kTileM), static_cast<unsigned>((n_out + kTileN - 1) / kTileN));
-    gemm_nt_kernel<<<grid, 256, 0, stream>>>(a, lda, b, ldb, out, ldo, n, n_out, k_dim);
+    // Few tiles take the time of one, which is shorter with 32 rows; from a tile for every second SM on they are no faster.  1000 x 355 by
+    // 355 x 355 (24 tiles): 49 us with 128 rows, 20 with 32; 3000 rows (72): 51 and 35; 6000 (141): 52 and 66.
+    if (2 * static_cast<size_t>(grid.x) * grid.y <= static_cast<size_t>(sm_count())) {
+        grid.x = static_cast<unsigned>((n + 31) / 32);
+        gemm_nt_small_kernel<<<grid, 256, 0, stream>>>(a, lda, b, ldb, out, ldo, n, n_out, k_dim);
+    } else {
+        gemm_nt_kernel<<<grid, 256, 0, stream>>>(a, lda, b, ldb, out, ldo, n, n_out, k_dim);
+    }
     SKM_LAUNCH_CHECK();
 }
 

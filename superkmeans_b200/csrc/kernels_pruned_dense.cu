@@ -171,31 +171,58 @@ __global__ void __launch_bounds__(256) chain_norms_kernel(const float* __restric
 // -------------------------------------------------------------------------------------------------
 // Dense chain
 // -------------------------------------------------------------------------------------------------
-struct DenseRowState {
-    uint32_t gidx[kTileM];
-    float best[kTileM];
-    uint32_t bestidx[kTileM];
-    uint32_t prev[kTileM];
-    uint32_t cnt[kTileM];
-    uint32_t npc[kTileM];
-    uint32_t prev_first[kTileM];
-    unsigned long long chunk_key[kTileM];
+// Tiles of 128 x 128 (8 x 8 values a thread) or of 32 x 128 (4 x 4), see gemm_simt.cuh.  Both make the same sums in the same order.
+template <int M>
+struct DenseTile {
+    using Smem = GemmSmem;
+    static constexpr int kPer = 8;
+    static __device__ __forceinline__ int row(int i) { return tile_row_of(threadIdx.x >> 4, i); }
+    static __device__ __forceinline__ int col(int j) { return tile_col_of(threadIdx.x & 15, j); }
+    template <bool ZERO_ACC>
+    static __device__ __forceinline__ void multiply(const float* a, size_t ld, int m_valid, const uint32_t* rows, const float* b, int n_valid, uint32_t K, Smem& s, float (&acc)[8][8]) {
+        gemm_tile_nt_ex<ZERO_ACC, true>(a, ld, m_valid, rows, b, ld, n_valid, static_cast<int>(K), s, acc);
+    }
+};
+template <>
+struct DenseTile<32> {
+    using Smem = GemmSmem32;
+    static constexpr int kPer = 4;
+    static __device__ __forceinline__ int row(int i) { return static_cast<int>(threadIdx.x >> 5) * 4 + i; }
+    static __device__ __forceinline__ int col(int j) { return static_cast<int>(threadIdx.x & 31) + 32 * j; }
+    template <bool ZERO_ACC>
+    static __device__ __forceinline__ void multiply(const float* a, size_t ld, int m_valid, const uint32_t* rows, const float* b, int n_valid, uint32_t K, Smem& s, float (&acc)[4][4]) {
+        gemm_tile32_nt<ZERO_ACC, true>(a, ld, m_valid, rows, b, ld, n_valid, static_cast<int>(K), s, acc);
+    }
 };
 
-__global__ void __launch_bounds__(256, 2) assign_pruned_dense_kernel(const PrunedParams p, const uint32_t* __restrict__ hard_idx, size_t n_hard, const float* __restrict__ best_in,
+template <int M>
+struct DenseRowState {
+    uint32_t gidx[M];
+    float best[M];
+    uint32_t bestidx[M];
+    uint32_t prev[M];
+    uint32_t cnt[M];
+    uint32_t npc[M];
+    uint32_t prev_first[M];
+    unsigned long long chunk_key[M];
+};
+
+template <int M>
+__global__ void __launch_bounds__(256, M == 32 ? 4 : 2) assign_pruned_dense_kernel(const PrunedParams p, const uint32_t* __restrict__ hard_idx, size_t n_hard, const float* __restrict__ best_in,
                                                                      const float* __restrict__ chain_norms_y, uint32_t n_ck) {
-    __shared__ GemmSmem smem;
-    __shared__ DenseRowState st;
-    extern __shared__ float nxc[];  // [kTileM][n_ck] cumulative norms of the tile's points
+    using Tile = DenseTile<M>;
+    constexpr int P = Tile::kPer;
+    __shared__ typename Tile::Smem smem;
+    __shared__ DenseRowState<M> st;
+    extern __shared__ float nxc[];  // [M][n_ck] cumulative norms of the tile's points
     const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;
     const int lane = tid & 31, warp = tid >> 5;
-    const size_t tile0 = static_cast<size_t>(blockIdx.x) * kTileM;
-    const int m_valid = static_cast<int>(min(static_cast<size_t>(kTileM), n_hard - tile0));
+    const size_t tile0 = static_cast<size_t>(blockIdx.x) * M;
+    const int m_valid = static_cast<int>(min(static_cast<size_t>(M), n_hard - tile0));
     const uint32_t n_hblocks = p.horizontal_d / kHBlock;
     const bool has_tail = p.partial_d < p.vertical_d;
 
-    if (tid < kTileM) {
+    if (tid < M) {
         const bool v = tid < m_valid;
         const uint32_t g = v ? hard_idx[tile0 + tid] : 0u;
         st.gidx[tid] = g;
@@ -212,7 +239,7 @@ __global__ void __launch_bounds__(256, 2) assign_pruned_dense_kernel(const Prune
     for (size_t chunk = 0; chunk < n_chunks; ++chunk) {
         const size_t c0 = chunk * kChunk;
         const size_t cs = min(static_cast<size_t>(kChunk), p.k - c0);
-        if (tid < kTileM) {
+        if (tid < M) {
             st.cnt[tid] = 0;
             st.prev_first[tid] = 0;
             st.chunk_key[tid] = ~0ull;
@@ -221,28 +248,28 @@ __global__ void __launch_bounds__(256, 2) assign_pruned_dense_kernel(const Prune
         for (size_t sub0 = 0; sub0 < cs; sub0 += kTileN) {
             const int n_valid = static_cast<int>(min(static_cast<size_t>(kTileN), cs - sub0));
             const float* __restrict__ yb = p.y + (c0 + sub0) * p.d;
-            float acc[8][8];
+            float acc[P][P];
             // ---- checkpoint 0: the first d' dimensions
-            gemm_tile_nt_ex<true, true>(p.x, p.d, m_valid, st.gidx, yb, p.d, n_valid, static_cast<int>(p.partial_d), smem, acc);
+            Tile::template multiply<true>(p.x, p.d, m_valid, st.gidx, yb, n_valid, p.partial_d, smem, acc);
             unsigned long long alive = 0ull;
             uint32_t dims = p.partial_d;
             {
                 const float ratio = __ldg(p.ratios + dims);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int r = tile_row_of(ty, i);
+                for (int i = 0; i < P; ++i) {
+                    const int r = Tile::row(i);
                     if (r >= m_valid) continue;
                     const float thr = st.best[r] * ratio;
                     const float nxv = nxc[r * n_ck];
                     uint32_t c_alive = 0;
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const int c = tile_col_of(tx, j);
+                    for (int j = 0; j < P; ++j) {
+                        const int c = Tile::col(j);
                         if (c < n_valid) {
                             const size_t gc = c0 + sub0 + c;
                             const float pd = fmaf(-2.0f, acc[i][j], nxv) + __ldg(chain_norms_y + gc);
                             if (pd < thr) {
-                                alive |= 1ull << (i * 8 + j);
+                                alive |= 1ull << (i * P + j);
                                 ++c_alive;
                                 if (static_cast<size_t>(st.prev[r]) == gc) st.prev_first[r] = 1;
                             }
@@ -256,22 +283,22 @@ __global__ void __launch_bounds__(256, 2) assign_pruned_dense_kernel(const Prune
             // ---- horizontal blocks, 64 dimensions at a time
             for (uint32_t hb = 0; hb < n_hblocks; ++hb) {
                 const size_t off = static_cast<size_t>(p.vertical_d) + static_cast<size_t>(hb) * kHBlock;
-                gemm_tile_nt_ex<false, true>(p.x + off, p.d, m_valid, st.gidx, yb + off, p.d, n_valid, kHBlock, smem, acc);
+                Tile::template multiply<false>(p.x + off, p.d, m_valid, st.gidx, yb + off, n_valid, kHBlock, smem, acc);
                 dims += kHBlock;
                 const float ratio = __ldg(p.ratios + dims);
                 const uint32_t ck = 1 + hb;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    if (((alive >> (i * 8)) & 0xFFull) == 0ull) continue;
-                    const int r = tile_row_of(ty, i);
+                for (int i = 0; i < P; ++i) {
+                    if (((alive >> (i * P)) & ((1ull << P) - 1)) == 0ull) continue;
+                    const int r = Tile::row(i);
                     const float thr = st.best[r] * ratio;
                     const float nxv = nxc[r * n_ck + ck];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        if (alive & (1ull << (i * 8 + j))) {
-                            const size_t gc = c0 + sub0 + tile_col_of(tx, j);
+                    for (int j = 0; j < P; ++j) {
+                        if (alive & (1ull << (i * P + j))) {
+                            const size_t gc = c0 + sub0 + Tile::col(j);
                             const float pd = fmaf(-2.0f, acc[i][j], nxv) + __ldg(chain_norms_y + static_cast<size_t>(ck) * p.k + gc);
-                            if (!(pd < thr)) alive &= ~(1ull << (i * 8 + j));
+                            if (!(pd < thr)) alive &= ~(1ull << (i * P + j));
                         }
                     }
                 }
@@ -279,19 +306,19 @@ __global__ void __launch_bounds__(256, 2) assign_pruned_dense_kernel(const Prune
             }
             // ---- the vertical dimensions not covered by the first checkpoint, then the final pick
             if (has_tail) {
-                gemm_tile_nt_ex<false, true>(p.x + p.partial_d, p.d, m_valid, st.gidx, yb + p.partial_d, p.d, n_valid, static_cast<int>(p.vertical_d - p.partial_d), smem, acc);
+                Tile::template multiply<false>(p.x + p.partial_d, p.d, m_valid, st.gidx, yb + p.partial_d, n_valid, p.vertical_d - p.partial_d, smem, acc);
             }
             const uint32_t ck_last = n_ck - 1;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                if (((alive >> (i * 8)) & 0xFFull) == 0ull) continue;
-                const int r = tile_row_of(ty, i);
+            for (int i = 0; i < P; ++i) {
+                if (((alive >> (i * P)) & ((1ull << P) - 1)) == 0ull) continue;
+                const int r = Tile::row(i);
                 const float b = st.best[r];
                 const float nxv = nxc[r * n_ck + ck_last];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    if (alive & (1ull << (i * 8 + j))) {
-                        const size_t gc = c0 + sub0 + tile_col_of(tx, j);
+                for (int j = 0; j < P; ++j) {
+                    if (alive & (1ull << (i * P + j))) {
+                        const size_t gc = c0 + sub0 + Tile::col(j);
                         const float pd = fmaf(-2.0f, acc[i][j], nxv) + __ldg(chain_norms_y + static_cast<size_t>(ck_last) * p.k + gc);
                         if (pd < b) {  // ratio[d] == 1
                             const unsigned long long key = (static_cast<unsigned long long>(float_to_ordered(pd)) << 32) | static_cast<unsigned long long>(gc);
@@ -302,7 +329,7 @@ __global__ void __launch_bounds__(256, 2) assign_pruned_dense_kernel(const Prune
             }
         }
         __syncthreads();
-        if (tid < kTileM) {
+        if (tid < M) {
             st.npc[tid] += st.cnt[tid];
             const unsigned long long key = st.chunk_key[tid];
             // pdxearch.h:140-143: when the previous centroid is the only survivor of the first test the
@@ -512,9 +539,16 @@ void launch_assign_pruned_dense(const PrunedParams& p, PruneSplitWorkspace& ws, 
     const uint32_t n_ck = prune_chain_checkpoints(p.partial_d, p.vertical_d, p.horizontal_d);
     if (n_ck > kMaxCheckpoints * 4) throw std::invalid_argument("dimensionality too large for the dense pruned kernel");
     launch_chain_norms(p.y, p.k, p.d, p.partial_d, p.vertical_d, p.horizontal_d, true, ws.chain_norms_y, stream);
-    const size_t dyn = sizeof(float) * kTileM * n_ck;
-    SKM_CUDA(cudaFuncSetAttribute(assign_pruned_dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dyn)));
-    assign_pruned_dense_kernel<<<static_cast<unsigned>((n_hard + kTileM - 1) / kTileM), 256, dyn, stream>>>(p, ws.hard_idx, n_hard, ws.best, ws.chain_norms_y, n_ck);
+    const auto launch = [&](auto kernel, int rows) {
+        const size_t dyn = sizeof(float) * rows * n_ck;
+        SKM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dyn)));
+        kernel<<<static_cast<unsigned>((n_hard + rows - 1) / rows), 256, dyn, stream>>>(p, ws.hard_idx, n_hard, ws.best, ws.chain_norms_y, n_ck);
+    };
+    // Up to a tile of 128 rows per SM the time is that of one block, and four times as many tiles of 32 rows are faster; from there on their
+    // smaller reuse of the operands costs as much.  5000 rows x 300 centroids x 130: 150 us with 128 rows, 79 with 32; 18 900: 152 and
+    // 138; 37 800: 202 and 267.  9000 x 1000 x 770: 1513 and 848; 37 800: 2235 and 2797.
+    if (n_hard <= static_cast<size_t>(sm_count()) * kTileM) launch(assign_pruned_dense_kernel<32>, 32);
+    else launch(assign_pruned_dense_kernel<kTileM>, kTileM);
     SKM_LAUNCH_CHECK();
 }
 
