@@ -4,7 +4,7 @@
 // of 768 dimensions kept one SM busy for 100 us and the others idle, and their passes around it (conversion, decision) cost
 // 60 us of launches and streams whatever the size.  Here the pairs themselves are divided:
 //   up to 8 rows   a warp per centroid, the rows in shared memory; bound by the centroids' bytes from L2 or HBM;
-//   more           64 x 64 tiles of rows x centroids, 4 x 4 per thread, bound by fp32 issue: 13 - 14 T multiply-adds per second.
+//   more           64 x 64 tiles of rows x centroids, 4 x 4 per thread, bound by fp32 issue: 14 - 18 T multiply-adds per second.
 // Distances are ||x||^2 + ||y||^2 - 2 x.y, the smallest wins, the lower index on a tie, clamped at zero when stored.
 #include <cfloat>
 
@@ -19,7 +19,7 @@ constexpr int kQueryRows = 8;
 constexpr int kQueryBlocks = 1184;               // at most: eight per SM
 constexpr size_t kQuerySmem = 48 * 1024;
 constexpr int kCell = 64;                        // rows and centroids of a tile
-constexpr int kDepth = 16;                       // columns per step
+constexpr int kDepth = 32;                       // columns per step
 
 // Sum over the row in the order of row_sqnorms_kernel.
 template <bool VEC, class F>
@@ -153,10 +153,10 @@ __global__ void __launch_bounds__(256) tile_prepare_kernel(const float* __restri
     }
 }
 
-// Loads a 64 x 16 piece of rows [row0, row0 + 64) into registers: thread t holds columns 4 (t & 3) .. + 3 of row t >> 2.
+// A thread's part of a 64 x 32 piece of rows [row0, row0 + 64): columns 4 (t & 7) .. + 3 of row t >> 3, or of row 32 + (t >> 3).
 template <bool VEC>
-__device__ __forceinline__ float4 load_cell(const float* __restrict__ m, size_t row0, size_t rows, size_t d, size_t j0) {
-    const size_t r = row0 + (threadIdx.x >> 2), j = j0 + 4 * (threadIdx.x & 3);
+__device__ __forceinline__ float4 load_cell(const float* __restrict__ m, size_t row0, size_t rows, size_t d, size_t j0, int half) {
+    const size_t r = row0 + (threadIdx.x >> 3) + 32 * half, j = j0 + 4 * (threadIdx.x & 7);
     if (r >= rows || j >= d) return make_float4(0.f, 0.f, 0.f, 0.f);
     const float* p = m + r * d + j;
     if (VEC) return __ldg(reinterpret_cast<const float4*>(p));
@@ -167,30 +167,48 @@ __device__ __forceinline__ float4 load_cell(const float* __restrict__ m, size_t 
     return v;
 }
 
+// In shared memory row r of column q lies at r ^ (q & 28): neither the transposing stores nor the reads have bank conflicts.
+__device__ __forceinline__ void store_cell(float (*cell)[kCell], int half, float4 v) {
+    const int q = 4 * (threadIdx.x & 7), r = ((threadIdx.x >> 3) + 32 * half) ^ q;
+    cell[q][r] = v.x; cell[q + 1][r] = v.y; cell[q + 2][r] = v.z; cell[q + 3][r] = v.w;
+}
+
+// A step costs at least the latency of a load from L2, which the step before covers: 32 columns take half as many as 16 (1000 x 1000 x 768:
+// 55 us, with 16 columns 64; 3000 x 3000 x 384: 189, 209; 20 x 1000 x 768: 30, 38; 5000 x 300 x 128: 18.5, 19.8).
 template <bool VEC>
 __global__ void __launch_bounds__(256) tile_kernel(const float* __restrict__ x, const float* __restrict__ y, size_t n, size_t k, size_t d, const float* __restrict__ norms_x,
                                                    const float* __restrict__ norms_y, unsigned long long* __restrict__ keys, uint32_t* __restrict__ counters,
                                                    uint32_t* __restrict__ knn, float* __restrict__ dist) {
-    __shared__ __align__(16) float sx[2][kDepth][kCell + 4], sy[2][kDepth][kCell + 4];
+    __shared__ __align__(16) float sx[2][kDepth][kCell], sy[2][kDepth][kCell];
     __shared__ bool last;
     const size_t row0 = static_cast<size_t>(blockIdx.y) * kCell, col0 = static_cast<size_t>(blockIdx.x) * kCell;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int lr = threadIdx.x >> 2, lc = 4 * (threadIdx.x & 3);
     float acc[4][4] = {};
-    float4 vx = load_cell<VEC>(x, row0, n, d, 0), vy = load_cell<VEC>(y, col0, k, d, 0);
+    float4 vx[2], vy[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        vx[h] = load_cell<VEC>(x, row0, n, d, 0, h);
+        vy[h] = load_cell<VEC>(y, col0, k, d, 0, h);
+    }
     int buf = 0;
     for (size_t j0 = 0; j0 < d; j0 += kDepth, buf ^= 1) {
-        sx[buf][lc][lr] = vx.x; sx[buf][lc + 1][lr] = vx.y; sx[buf][lc + 2][lr] = vx.z; sx[buf][lc + 3][lr] = vx.w;
-        sy[buf][lc][lr] = vy.x; sy[buf][lc + 1][lr] = vy.y; sy[buf][lc + 2][lr] = vy.z; sy[buf][lc + 3][lr] = vy.w;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            store_cell(sx[buf], h, vx[h]);
+            store_cell(sy[buf], h, vy[h]);
+        }
         __syncthreads();
         if (j0 + kDepth < d) {
-            vx = load_cell<VEC>(x, row0, n, d, j0 + kDepth);
-            vy = load_cell<VEC>(y, col0, k, d, j0 + kDepth);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                vx[h] = load_cell<VEC>(x, row0, n, d, j0 + kDepth, h);
+                vy[h] = load_cell<VEC>(y, col0, k, d, j0 + kDepth, h);
+            }
         }
 #pragma unroll
         for (int q = 0; q < kDepth; ++q) {
-            const float4 a = *reinterpret_cast<const float4*>(&sx[buf][q][ty * 4]);
-            const float4 b = *reinterpret_cast<const float4*>(&sy[buf][q][tx * 4]);
+            const float4 a = *reinterpret_cast<const float4*>(&sx[buf][q][(ty * 4) ^ (q & 28)]);
+            const float4 b = *reinterpret_cast<const float4*>(&sy[buf][q][(tx * 4) ^ (q & 28)]);
             const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
             for (int r = 0; r < 4; ++r)
