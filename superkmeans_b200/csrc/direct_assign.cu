@@ -4,7 +4,7 @@
 // of 768 dimensions kept one SM busy for 100 us and the others idle, and their passes around it (conversion, decision) cost
 // 60 us of launches and streams whatever the size.  Here the pairs themselves are divided:
 //   up to 8 rows   a warp per centroid, the rows in shared memory; bound by the centroids' bytes from L2 or HBM;
-//   more           64 x 64 tiles of rows x centroids, 4 x 4 per thread, bound by fp32 issue: 14 - 18 T multiply-adds per second.
+//   more           64 x 64 tiles of rows x centroids, 4 x 4 or 8 x 4 per thread, bound by reads of shared memory: 15 - 20 T multiply-adds per second.
 // Distances are ||x||^2 + ||y||^2 - 2 x.y, the smallest wins, the lower index on a tie, clamped at zero when stored.
 #include <cfloat>
 
@@ -153,10 +153,10 @@ __global__ void __launch_bounds__(256) tile_prepare_kernel(const float* __restri
     }
 }
 
-// A thread's part of a 64 x 32 piece of rows [row0, row0 + 64): columns 4 (t & 7) .. + 3 of row t >> 3, or of row 32 + (t >> 3).
+// A thread's part of a 64 x 32 piece of rows [row0, row0 + 64): columns 4 (t & 7) .. + 3 of row `at` + (t >> 3).
 template <bool VEC>
-__device__ __forceinline__ float4 load_cell(const float* __restrict__ m, size_t row0, size_t rows, size_t d, size_t j0, int half) {
-    const size_t r = row0 + (threadIdx.x >> 3) + 32 * half, j = j0 + 4 * (threadIdx.x & 7);
+__device__ __forceinline__ float4 load_cell(const float* __restrict__ m, size_t row0, size_t rows, size_t d, size_t j0, int at) {
+    const size_t r = row0 + at + (threadIdx.x >> 3), j = j0 + 4 * (threadIdx.x & 7);
     if (r >= rows || j >= d) return make_float4(0.f, 0.f, 0.f, 0.f);
     const float* p = m + r * d + j;
     if (VEC) return __ldg(reinterpret_cast<const float4*>(p));
@@ -168,57 +168,64 @@ __device__ __forceinline__ float4 load_cell(const float* __restrict__ m, size_t 
 }
 
 // In shared memory row r of column q lies at r ^ (q & 28): neither the transposing stores nor the reads have bank conflicts.
-__device__ __forceinline__ void store_cell(float (*cell)[kCell], int half, float4 v) {
-    const int q = 4 * (threadIdx.x & 7), r = ((threadIdx.x >> 3) + 32 * half) ^ q;
+__device__ __forceinline__ void store_cell(float (*cell)[kCell], int at, float4 v) {
+    const int q = 4 * (threadIdx.x & 7), r = (at + static_cast<int>(threadIdx.x >> 3)) ^ q;
     cell[q][r] = v.x; cell[q + 1][r] = v.y; cell[q + 2][r] = v.z; cell[q + 3][r] = v.w;
 }
 
 // A step costs at least the latency of a load from L2, which the step before covers: 32 columns take half as many as 16 (1000 x 1000 x 768:
 // 55 us, with 16 columns 64; 3000 x 3000 x 384: 189, 209; 20 x 1000 x 768: 30, 38; 5000 x 300 x 128: 18.5, 19.8).
-template <bool VEC>
-__global__ void __launch_bounds__(256) tile_kernel(const float* __restrict__ x, const float* __restrict__ y, size_t n, size_t k, size_t d, const float* __restrict__ norms_x,
+// R x 4 products a thread.
+template <bool VEC, int R>
+__global__ void __launch_bounds__(1024 / R) tile_kernel(const float* __restrict__ x, const float* __restrict__ y, size_t n, size_t k, size_t d, const float* __restrict__ norms_x,
                                                    const float* __restrict__ norms_y, unsigned long long* __restrict__ keys, uint32_t* __restrict__ counters,
                                                    uint32_t* __restrict__ knn, float* __restrict__ dist) {
+    constexpr int kAtOnce = 128 / R, kParts = kCell / kAtOnce;   // rows that a load takes, loads for a piece
     __shared__ __align__(16) float sx[2][kDepth][kCell], sy[2][kDepth][kCell];
     __shared__ bool last;
     const size_t row0 = static_cast<size_t>(blockIdx.y) * kCell, col0 = static_cast<size_t>(blockIdx.x) * kCell;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    float acc[4][4] = {};
-    float4 vx[2], vy[2];
+    float acc[R][4] = {};
+    float4 vx[kParts], vy[kParts];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        vx[h] = load_cell<VEC>(x, row0, n, d, 0, h);
-        vy[h] = load_cell<VEC>(y, col0, k, d, 0, h);
+    for (int h = 0; h < kParts; ++h) {
+        vx[h] = load_cell<VEC>(x, row0, n, d, 0, h * kAtOnce);
+        vy[h] = load_cell<VEC>(y, col0, k, d, 0, h * kAtOnce);
     }
     int buf = 0;
     for (size_t j0 = 0; j0 < d; j0 += kDepth, buf ^= 1) {
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            store_cell(sx[buf], h, vx[h]);
-            store_cell(sy[buf], h, vy[h]);
+        for (int h = 0; h < kParts; ++h) {
+            store_cell(sx[buf], h * kAtOnce, vx[h]);
+            store_cell(sy[buf], h * kAtOnce, vy[h]);
         }
         __syncthreads();
         if (j0 + kDepth < d) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                vx[h] = load_cell<VEC>(x, row0, n, d, j0 + kDepth, h);
-                vy[h] = load_cell<VEC>(y, col0, k, d, j0 + kDepth, h);
+            for (int h = 0; h < kParts; ++h) {
+                vx[h] = load_cell<VEC>(x, row0, n, d, j0 + kDepth, h * kAtOnce);
+                vy[h] = load_cell<VEC>(y, col0, k, d, j0 + kDepth, h * kAtOnce);
             }
         }
 #pragma unroll
         for (int q = 0; q < kDepth; ++q) {
-            const float4 a = *reinterpret_cast<const float4*>(&sx[buf][q][(ty * 4) ^ (q & 28)]);
-            const float4 b = *reinterpret_cast<const float4*>(&sy[buf][q][(tx * 4) ^ (q & 28)]);
-            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+            float av[R];
 #pragma unroll
-            for (int r = 0; r < 4; ++r)
+            for (int r = 0; r < R; r += 4) {
+                const float4 a = *reinterpret_cast<const float4*>(&sx[buf][q][(ty * R + r) ^ (q & 28)]);
+                av[r] = a.x; av[r + 1] = a.y; av[r + 2] = a.z; av[r + 3] = a.w;
+            }
+            const float4 b = *reinterpret_cast<const float4*>(&sy[buf][q][(tx * 4) ^ (q & 28)]);
+            const float bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int r = 0; r < R; ++r)
 #pragma unroll
                 for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(av[r], bv[c], acc[r][c]);
         }
     }
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const size_t row = row0 + ty * 4 + r;
+    for (int r = 0; r < R; ++r) {
+        const size_t row = row0 + ty * R + r;
         unsigned long long best = ~0ull;
         if (row < n) {
             const float nx = norms_x[row];
@@ -269,7 +276,12 @@ void launch_tiles(const float* x, const float* y, size_t n, size_t k, size_t d, 
     const size_t row_tiles = (n + kCell - 1) / kCell, col_tiles = (k + kCell - 1) / kCell;
     tile_prepare_kernel<VEC><<<static_cast<unsigned>((n + k + 7) / 8), 256, 0, stream>>>(x, y, n, k, d, s.norms_x, s.norms_y, s.keys, s.counters, row_tiles);
     SKM_LAUNCH_CHECK();
-    tile_kernel<VEC><<<dim3(static_cast<unsigned>(col_tiles), static_cast<unsigned>(row_tiles)), 256, 0, stream>>>(x, y, n, k, d, s.norms_x, s.norms_y, s.keys, s.counters, knn, dist);
+    // R + 4 reads of shared memory for 4 R products, which is what bounds the tiles: with 8 x 4 a thread they take 0.75 of the time, but
+    // a block of its own on an SM has too few warps then to cover their latency.  600 x 20 x 64 (10 tiles): 5.1 us with 4 x 4 a thread, 6.5 with 8 x 4;
+    // 5000 x 300 x 128 (395): 18.5 and 16.8; 1000 x 1000 x 768 (256): 55 and 51; 3000 x 3000 x 384: 189 and 172.
+    const dim3 grid(static_cast<unsigned>(col_tiles), static_cast<unsigned>(row_tiles));
+    if (row_tiles * col_tiles <= static_cast<size_t>(sm_count())) tile_kernel<VEC, 4><<<grid, 256, 0, stream>>>(x, y, n, k, d, s.norms_x, s.norms_y, s.keys, s.counters, knn, dist);
+    else tile_kernel<VEC, 8><<<grid, 128, 0, stream>>>(x, y, n, k, d, s.norms_x, s.norms_y, s.keys, s.counters, knn, dist);
     SKM_LAUNCH_CHECK();
 }
 

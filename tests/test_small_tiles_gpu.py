@@ -1,5 +1,5 @@
-"""Products of few rows on tiles of 32 rows: the same sums in the same order as tiles of 128 rows make, so a row's answer does not
-depend on how many others are with it."""
+"""Kernels that take other tiles, or other parts of a tile per thread, for few rows: the same sums in the same order, so a row's answer does
+not depend on how many others are with it."""
 import numpy as np
 import pytest
 
@@ -39,3 +39,20 @@ def test_product_of_few_rows(n, d):
     assert (np.abs(whole - want) <= d * 2.0 ** -24 * scale).all()   # a rounding per term
     for rows in (1, 31, 32, 33, 65, 900):
         assert (skm.engine.unrotate(m, x[:rows]) == whole[:rows]).all(), rows
+
+
+@pytest.mark.parametrize("n,k,d", [(2_000, 700, 33), (1_501, 701, 128), (1_300, 1_000, 101), (5_001, 193, 64), (10_000, 65, 100)])
+def test_direct_tiles_of_few_rows(n, k, d):
+    import superkmeans_b200 as skm
+
+    rng = np.random.default_rng(d)
+    x, y = rng.standard_normal((n, d), dtype=np.float32), rng.standard_normal((k, d), dtype=np.float32)
+    knn, dist = skm.engine.find_nearest(x, y)
+    x64, y64 = x.astype(np.float64), y.astype(np.float64)
+    true = (x64 ** 2).sum(1)[:, None] + (y64 ** 2).sum(1) - 2 * x64 @ y64.T
+    scale = (x64 ** 2).sum(1) + (y64 ** 2).sum(1).max()
+    assert (true[np.arange(n), knn] - true.min(1) <= 2 * d * 2.0 ** -24 * scale).all()   # a rounding per term, for either of two centroids
+    assert (np.abs(dist - true[np.arange(n), knn]) <= d * 2.0 ** -24 * scale).all()
+    for lo, hi in ((0, 9), (9, 73), (73, 137), (137, 400)):
+        a, b = skm.engine.find_nearest(x[lo:hi], y)
+        assert (a == knn[lo:hi]).all() and (b == dist[lo:hi]).all(), (lo, hi)
