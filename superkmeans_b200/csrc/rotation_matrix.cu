@@ -544,6 +544,8 @@ static bool factorise_on_device(const float* draws, size_t d, float* out, cudaSt
     DeviceBuffer<double> a_buf, w_buf, q_buf, g_buf, r_buf, inv_buf;
     DeviceBuffer<float> signs_buf;
     DeviceBuffer<unsigned long long> worst_buf;
+    PinnedBuffer<unsigned long long> bits;
+    bits.ensure(1);
     double* a = a_buf.ensure(dp * dp);
     double* w = w_buf.ensure(dp * dp);
     double* q = q_buf.ensure(dp * dp);
@@ -566,18 +568,18 @@ static bool factorise_on_device(const float* draws, size_t d, float* out, cudaSt
     double* cur = q;
     double* next = a;
     for (int turn = 0;; ++turn) {
+        if (turn > 0) SKM_CUDA(cudaMemsetAsync(worst, 0, sizeof(unsigned long long), stream));
         product_kernel<true><<<tiles, kProductThreads, 0, stream>>>(cur, nullptr, dp, g, true, worst);
         SKM_LAUNCH_CHECK();
         product_kernel<false><<<tiles, kProductThreads, 0, stream>>>(cur, g, dp, next, false, nullptr);
         SKM_LAUNCH_CHECK();
         std::swap(cur, next);
-        unsigned long long bits = 0;
-        SKM_CUDA(cudaMemcpyAsync(&bits, worst, sizeof(bits), cudaMemcpyDeviceToHost, stream));
-        SKM_CUDA(cudaMemsetAsync(worst, 0, sizeof(unsigned long long), stream));
+        // (a copy to pageable memory would keep other threads' calls waiting as long as the chain takes: 0.4 ms in which no rows are uploaded)
+        SKM_CUDA(cudaMemcpyAsync(bits.get(), worst, sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
         SKM_CUDA(cudaStreamSynchronize(stream));
         double e;
-        static_assert(sizeof(e) == sizeof(bits), "one word");
-        std::memcpy(&e, &bits, sizeof(e));   // a NaN when a pivot or a product was none
+        static_assert(sizeof(e) == sizeof(unsigned long long), "one word");
+        std::memcpy(&e, bits.get(), sizeof(e));   // a NaN when a pivot or a product was none
         if (!(e < 0.01) || turn == 4) return false;
         // What is left is at most d e^2: the result is rounded to 24 bits.
         if (e * e * static_cast<double>(d) < 1e-12) break;
