@@ -49,32 +49,57 @@ __device__ void bitonic_sort(unsigned long long* buf, int n) {
     __syncthreads();
 }
 
-// dots: n_q x slab_ld dot products of this slab (columns [0, slab_n) valid, global indices col0 + c).
-// state: n_q x k keys carried from slab to slab, ascending, ~0 = empty.
+// Where the lists of a pass go: the state that the next slab goes on with, or (out_idx given) the answers: indices and distances clamped at
+// zero as FindKNearestNeighbors stores them; empty slots: index 0xFFFFFFFF, distance FLT_MAX.
+struct TopkLists {
+    unsigned long long* state;   // n_q x k keys, ascending, ~0 = empty
+    uint32_t* out_idx;
+    float* out_dist;
+    __device__ __forceinline__ void put(size_t at, unsigned long long key) const {
+        if (!out_idx) {
+            state[at] = key;
+            return;
+        }
+        const bool empty = key == ~0ull;
+        out_idx[at] = empty ? 0xFFFFFFFFu : static_cast<uint32_t>(key & 0xFFFFFFFFull);
+        if (out_dist) out_dist[at] = empty ? FLT_MAX : fmaxf(0.0f, ordered_to_float(static_cast<uint32_t>(key >> 32)));
+    }
+};
+
+// dots: n_q x slab_ld dot products of this slab (columns [0, slab_n) valid, global indices col0 + c).  The first slab finds no state.
 __global__ void __launch_bounds__(kTopkThreads) topk_merge_kernel(const float* __restrict__ dots, size_t slab_ld, size_t slab_n, size_t col0, const float* __restrict__ norms_q,
-                                                                  const float* __restrict__ norms_y, uint32_t k, unsigned long long* __restrict__ state) {
+                                                                  const float* __restrict__ norms_y, uint32_t k, TopkLists lists) {
     __shared__ unsigned long long buf[kTopkBuf];
     __shared__ uint32_t count;
     __shared__ unsigned long long tau;
     const size_t q = blockIdx.x;
     const float nq = norms_q[q];
-    unsigned long long* st = state + q * k;
-    for (int i = threadIdx.x; i < kTopkBuf; i += kTopkThreads) buf[i] = (i < static_cast<int>(k)) ? st[i] : ~0ull;
+    const unsigned long long* st = lists.state + q * k;
+    const uint32_t carried = col0 == 0 ? 0u : k;
+    if (slab_n > 2 * kTopkThreads || carried) {
+        for (int i = threadIdx.x; i < kTopkBuf; i += kTopkThreads) buf[i] = i < static_cast<int>(carried) ? st[i] : ~0ull;
+    } else {
+        for (int i = threadIdx.x; i < 2 * kTopkThreads; i += kTopkThreads) buf[i] = ~0ull;
+    }
     if (threadIdx.x == 0) {
-        count = k;
-        tau = st[k - 1];
+        count = carried;
+        tau = carried ? st[k - 1] : ~0ull;
     }
     __syncthreads();
     const float* __restrict__ row = dots + q * slab_ld;
     for (size_t c0 = 0; c0 < slab_n; c0 += kTopkThreads) {
         const size_t c = c0 + threadIdx.x;
-        if (c < slab_n) {
-            const float dist = fmaf(-2.0f, row[c], nq) + norms_y[col0 + c];
-            const unsigned long long key = make_key(dist, static_cast<uint32_t>(col0 + c));
-            if (key < tau) {
-                const uint32_t pos = atomicAdd(&count, 1u);
-                buf[pos] = key;   // pos < k + kTopkThreads * rounds, bounded by the flush below
-            }
+        const float dist = c < slab_n ? fmaf(-2.0f, row[c], nq) + norms_y[col0 + c] : 0.f;
+        const unsigned long long key = make_key(dist, static_cast<uint32_t>(col0 + c));
+        // (a place per warp, then per key)
+        const bool kept = c < slab_n && key < tau;
+        const uint32_t all = __ballot_sync(0xffffffffu, kept);
+        if (all != 0) {
+            const int lane = threadIdx.x & 31;
+            uint32_t at = 0;
+            if (lane == 0) at = atomicAdd(&count, static_cast<uint32_t>(__popc(all)));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(all & ((1u << lane) - 1u));
+            if (kept) buf[at] = key;   // below k + kTopkThreads * rounds, bounded by the flush below
         }
         __syncthreads();
         // one more round adds at most kTopkThreads keys: flush while that still fits
@@ -88,31 +113,12 @@ __global__ void __launch_bounds__(kTopkThreads) topk_merge_kernel(const float* _
             __syncthreads();
         }
     }
-    // what lies behind the keys held is empty: among 300 centroids a sort of 512 takes half the time of one of the whole buffer
+    // what lies behind the keys held is empty: among 300 centroids a sort of 512 takes half the time of one of the whole buffer (9 us for 200
+    // lists; places counted key by key: 12)
     int held = 2;
     while (held < static_cast<int>(count)) held <<= 1;
     bitonic_sort(buf, held);
-    for (int i = threadIdx.x; i < static_cast<int>(k); i += kTopkThreads) st[i] = buf[i];
-}
-
-__global__ void topk_init_kernel(unsigned long long* state, size_t n) {
-    const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < n) state[i] = ~0ull;
-}
-
-// keys -> indices and distances (clamped at zero as FindKNearestNeighbors stores them; empty slots: index
-// 0xFFFFFFFF, distance FLT_MAX)
-__global__ void topk_finish_kernel(const unsigned long long* __restrict__ state, size_t n, uint32_t* __restrict__ idx, float* __restrict__ dist) {
-    const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const unsigned long long key = state[i];
-    if (key == ~0ull) {
-        idx[i] = 0xFFFFFFFFu;
-        if (dist) dist[i] = FLT_MAX;
-    } else {
-        idx[i] = static_cast<uint32_t>(key & 0xFFFFFFFFull);
-        if (dist) dist[i] = fmaxf(0.0f, ordered_to_float(static_cast<uint32_t>(key >> 32)));
-    }
+    for (int i = threadIdx.x; i < static_cast<int>(k); i += kTopkThreads) lists.put(q * k + i, i < held ? buf[i] : ~0ull);
 }
 
 // found[q] = number of the query's ground-truth points whose current cluster is among the clusters the query
@@ -146,17 +152,16 @@ void launch_topk_nn(const float* q, const float* y, size_t n_q, size_t n_y, size
                     float* out_dist, float* dots_scratch, unsigned long long* state, cudaStream_t stream) {
     if (n_q == 0 || k == 0) return;
     if (k > topk_max_k()) throw std::runtime_error("nearest-neighbour lists longer than " + std::to_string(topk_max_k()) + " entries are not supported");
-    const size_t n_state = n_q * k;
-    topk_init_kernel<<<static_cast<unsigned>((n_state + 255) / 256), 256, 0, stream>>>(state, n_state);
-    SKM_LAUNCH_CHECK();
-    for (size_t c0 = 0; c0 < n_y; c0 += kSlab) {
+    size_t c0 = 0;
+    do {
         const size_t cn = std::min(kSlab, n_y - c0);
         launch_gemm_nt(q, d, y + c0 * d, d, dots_scratch, kSlab, n_q, cn, d, stream);
-        topk_merge_kernel<<<static_cast<unsigned>(n_q), kTopkThreads, 0, stream>>>(dots_scratch, kSlab, cn, c0, norms_q, norms_y, k, state);
+        const bool last = cn == n_y - c0;
+        topk_merge_kernel<<<static_cast<unsigned>(n_q), kTopkThreads, 0, stream>>>(dots_scratch, kSlab, cn, c0, norms_q, norms_y, k,
+                                                                                  TopkLists{state, last ? out_idx : nullptr, last ? out_dist : nullptr});
         SKM_LAUNCH_CHECK();
-    }
-    topk_finish_kernel<<<static_cast<unsigned>((n_state + 255) / 256), 256, 0, stream>>>(state, n_state, out_idx, out_dist);
-    SKM_LAUNCH_CHECK();
+        c0 += kSlab;
+    } while (c0 < n_y);
 }
 
 void launch_recall_count(const uint32_t* gt, uint32_t objective_k, const uint32_t* promising, uint32_t n_explore, const uint32_t* assignments, size_t n_assignments,
