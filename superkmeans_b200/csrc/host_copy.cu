@@ -30,10 +30,11 @@ int threads_for(size_t bytes) { return static_cast<int>(std::max<size_t>(1, std:
 
 // Copies to memory that the GPU reads next, past the caches: what another core has just written to its cache the link fetches at
 // 30 GB/s (4 MB, eight threads: 138 us), what lies in memory at 50 (84 us).  Filling it takes 66 us in place of 44, beside the copy before.
+// A cache line must not be written both ways, so that only whole lines are streamed, the ends of a contiguous part are not.
 // publish() comes behind the last of a thread.
 void stream_bytes(char* dst, const char* src, size_t bytes) {
 #ifdef __SSE2__
-    const size_t head = std::min(bytes, static_cast<size_t>(-reinterpret_cast<uintptr_t>(dst) & 15));
+    const size_t head = std::min(bytes, static_cast<size_t>(-reinterpret_cast<uintptr_t>(dst) & 63));
     std::memcpy(dst, src, head);
     size_t i = head;
     for (; i + 64 <= bytes; i += 64) {
@@ -64,11 +65,17 @@ void copy_bytes(char* dst, const char* src, size_t bytes, bool to_gpu) {
     }
 }
 
+// Rows of whole cache lines are streamed.  Others share lines with their neighbours: a Train on 98 857 of 329 524 rows of 624 bytes took 13.3 ms
+// with streaming stores and 8.8 with plain ones.
 void gather_rows(char* dst, const char* src, const size_t* idx, size_t n, size_t row_bytes) {
     const int threads = threads_for(n * row_bytes);
+    const bool lines = row_bytes % 64 == 0 && reinterpret_cast<uintptr_t>(dst) % 64 == 0;
 #pragma omp parallel for num_threads(threads) schedule(static) if (threads > 1)
     for (int t = 0; t < threads; ++t) {
-        for (size_t i = n * t / threads; i < n * (t + 1) / threads; ++i) stream_bytes(dst + i * row_bytes, src + idx[i] * row_bytes, row_bytes);
+        for (size_t i = n * t / threads; i < n * (t + 1) / threads; ++i) {
+            if (lines) stream_bytes(dst + i * row_bytes, src + idx[i] * row_bytes, row_bytes);
+            else std::memcpy(dst + i * row_bytes, src + idx[i] * row_bytes, row_bytes);
+        }
         publish();
     }
 }
