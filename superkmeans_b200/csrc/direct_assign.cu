@@ -19,7 +19,6 @@ constexpr int kQueryRows = 8;
 constexpr int kQueryBlocks = 1184;               // at most: eight per SM
 constexpr size_t kQuerySmem = 48 * 1024;
 constexpr int kCell = 64;                        // rows and centroids of a tile
-constexpr int kDepth = 32;                       // columns per step
 
 // Sum over the row in the order of row_sqnorms_kernel.
 template <bool VEC, class F>
@@ -153,10 +152,10 @@ __global__ void __launch_bounds__(256) tile_prepare_kernel(const float* __restri
     }
 }
 
-// A thread's part of a 64 x 32 piece of rows [row0, row0 + 64): columns 4 (t & 7) .. + 3 of row `at` + (t >> 3).
-template <bool VEC>
+// A thread's part of a piece of D columns of rows [row0, row0 + 64): four columns of a row from `at` on.
+template <bool VEC, int D>
 __device__ __forceinline__ float4 load_cell(const float* __restrict__ m, size_t row0, size_t rows, size_t d, size_t j0, int at) {
-    const size_t r = row0 + at + (threadIdx.x >> 3), j = j0 + 4 * (threadIdx.x & 7);
+    const size_t r = row0 + at + threadIdx.x / (D / 4), j = j0 + 4 * (threadIdx.x % (D / 4));
     if (r >= rows || j >= d) return make_float4(0.f, 0.f, 0.f, 0.f);
     const float* p = m + r * d + j;
     if (VEC) return __ldg(reinterpret_cast<const float4*>(p));
@@ -167,21 +166,22 @@ __device__ __forceinline__ float4 load_cell(const float* __restrict__ m, size_t 
     return v;
 }
 
-// In shared memory row r of column q lies at r ^ (q & 28): neither the transposing stores nor the reads have bank conflicts.
+// In shared memory row r of column q lies at r ^ (q & 28): neither the reads nor, with 32 columns, the transposing stores have bank conflicts.
+template <int D>
 __device__ __forceinline__ void store_cell(float (*cell)[kCell], int at, float4 v) {
-    const int q = 4 * (threadIdx.x & 7), r = (at + static_cast<int>(threadIdx.x >> 3)) ^ q;
+    const int q = 4 * (threadIdx.x % (D / 4)), r = (at + static_cast<int>(threadIdx.x / (D / 4))) ^ q;
     cell[q][r] = v.x; cell[q + 1][r] = v.y; cell[q + 2][r] = v.z; cell[q + 3][r] = v.w;
 }
 
 // A step costs at least the latency of a load from L2, which the step before covers: 32 columns take half as many as 16 (1000 x 1000 x 768:
 // 55 us, with 16 columns 64; 3000 x 3000 x 384: 189, 209; 20 x 1000 x 768: 30, 38; 5000 x 300 x 128: 18.5, 19.8).
-// R x 4 products a thread.
-template <bool VEC, int R>
+// R x 4 products a thread, D columns a step.
+template <bool VEC, int R, int D>
 __global__ void __launch_bounds__(1024 / R) tile_kernel(const float* __restrict__ x, const float* __restrict__ y, size_t n, size_t k, size_t d, const float* __restrict__ norms_x,
                                                    const float* __restrict__ norms_y, unsigned long long* __restrict__ keys, uint32_t* __restrict__ counters,
                                                    uint32_t* __restrict__ knn, float* __restrict__ dist) {
-    constexpr int kAtOnce = 128 / R, kParts = kCell / kAtOnce;   // rows that a load takes, loads for a piece
-    __shared__ __align__(16) float sx[2][kDepth][kCell], sy[2][kDepth][kCell];
+    constexpr int kAtOnce = 4096 / (R * D), kParts = kCell / kAtOnce;   // rows that a load takes, loads for a piece
+    __shared__ __align__(16) float sx[2][D][kCell], sy[2][D][kCell];
     __shared__ bool last;
     const size_t row0 = static_cast<size_t>(blockIdx.y) * kCell, col0 = static_cast<size_t>(blockIdx.x) * kCell;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -189,38 +189,42 @@ __global__ void __launch_bounds__(1024 / R) tile_kernel(const float* __restrict_
     float4 vx[kParts], vy[kParts];
 #pragma unroll
     for (int h = 0; h < kParts; ++h) {
-        vx[h] = load_cell<VEC>(x, row0, n, d, 0, h * kAtOnce);
-        vy[h] = load_cell<VEC>(y, col0, k, d, 0, h * kAtOnce);
+        vx[h] = load_cell<VEC, D>(x, row0, n, d, 0, h * kAtOnce);
+        vy[h] = load_cell<VEC, D>(y, col0, k, d, 0, h * kAtOnce);
     }
     int buf = 0;
-    for (size_t j0 = 0; j0 < d; j0 += kDepth, buf ^= 1) {
+    for (size_t j0 = 0; j0 < d; j0 += D, buf ^= 1) {
 #pragma unroll
         for (int h = 0; h < kParts; ++h) {
-            store_cell(sx[buf], h * kAtOnce, vx[h]);
-            store_cell(sy[buf], h * kAtOnce, vy[h]);
+            store_cell<D>(sx[buf], h * kAtOnce, vx[h]);
+            store_cell<D>(sy[buf], h * kAtOnce, vy[h]);
         }
         __syncthreads();
-        if (j0 + kDepth < d) {
+        if (j0 + D < d) {
 #pragma unroll
             for (int h = 0; h < kParts; ++h) {
-                vx[h] = load_cell<VEC>(x, row0, n, d, j0 + kDepth, h * kAtOnce);
-                vy[h] = load_cell<VEC>(y, col0, k, d, j0 + kDepth, h * kAtOnce);
+                vx[h] = load_cell<VEC, D>(x, row0, n, d, j0 + D, h * kAtOnce);
+                vy[h] = load_cell<VEC, D>(y, col0, k, d, j0 + D, h * kAtOnce);
             }
         }
 #pragma unroll
-        for (int q = 0; q < kDepth; ++q) {
-            float av[R];
+        for (int half = 0; half < D; half += 16) {
+            if (half > 0 && j0 + half >= d) break;   // (zeros)
 #pragma unroll
-            for (int r = 0; r < R; r += 4) {
-                const float4 a = *reinterpret_cast<const float4*>(&sx[buf][q][(ty * R + r) ^ (q & 28)]);
-                av[r] = a.x; av[r + 1] = a.y; av[r + 2] = a.z; av[r + 3] = a.w;
+            for (int q = half; q < half + 16; ++q) {
+                float av[R];
+#pragma unroll
+                for (int r = 0; r < R; r += 4) {
+                    const float4 a = *reinterpret_cast<const float4*>(&sx[buf][q][(ty * R + r) ^ (q & 28)]);
+                    av[r] = a.x; av[r + 1] = a.y; av[r + 2] = a.z; av[r + 3] = a.w;
+                }
+                const float4 b = *reinterpret_cast<const float4*>(&sy[buf][q][(tx * 4) ^ (q & 28)]);
+                const float bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(av[r], bv[c], acc[r][c]);
             }
-            const float4 b = *reinterpret_cast<const float4*>(&sy[buf][q][(tx * 4) ^ (q & 28)]);
-            const float bv[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(av[r], bv[c], acc[r][c]);
         }
     }
 #pragma unroll
@@ -280,8 +284,11 @@ void launch_tiles(const float* x, const float* y, size_t n, size_t k, size_t d, 
     // a block of its own on an SM has too few warps then to cover their latency.  600 x 20 x 64 (10 tiles): 5.1 us with 4 x 4 a thread, 6.5 with 8 x 4;
     // 5000 x 300 x 128 (395): 18.5 and 16.8; 1000 x 1000 x 768 (256): 55 and 51; 3000 x 3000 x 384: 189 and 172.
     const dim3 grid(static_cast<unsigned>(col_tiles), static_cast<unsigned>(row_tiles));
-    if (row_tiles * col_tiles <= static_cast<size_t>(sm_count())) tile_kernel<VEC, 4><<<grid, 256, 0, stream>>>(x, y, n, k, d, s.norms_x, s.norms_y, s.keys, s.counters, knn, dist);
-    else tile_kernel<VEC, 8><<<grid, 128, 0, stream>>>(x, y, n, k, d, s.norms_x, s.norms_y, s.keys, s.counters, knn, dist);
+    // Up to 64 columns the tiles are mostly ends, which many blocks on an SM overlap: those of 16 columns a step take the least of it (5339 x 8002 x 32:
+    // 141 us, 154 with 32 columns, 179 with 8 x 4 as well).
+    if (row_tiles * col_tiles <= static_cast<size_t>(sm_count())) tile_kernel<VEC, 4, 32><<<grid, 256, 0, stream>>>(x, y, n, k, d, s.norms_x, s.norms_y, s.keys, s.counters, knn, dist);
+    else if (d <= 64) tile_kernel<VEC, 4, 16><<<grid, 256, 0, stream>>>(x, y, n, k, d, s.norms_x, s.norms_y, s.keys, s.counters, knn, dist);
+    else tile_kernel<VEC, 8, 32><<<grid, 128, 0, stream>>>(x, y, n, k, d, s.norms_x, s.norms_y, s.keys, s.counters, knn, dist);
     SKM_LAUNCH_CHECK();
 }
 
