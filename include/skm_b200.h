@@ -214,6 +214,10 @@ skm_status skm_debug_wait_injection(uint64_t wait_limit_cycles, uint32_t produce
  * them; most_bytes < least_bytes: none do.  No counterpart in the reference. */
 void skm_debug_alloc_failures(uint64_t least_bytes, uint64_t most_bytes, int pinned);
 
+/* Test hook: the dense chain takes this many points at a time (0 = as many as fit its gigabyte).  No counterpart in the
+ * reference. */
+void skm_debug_chain_slice(uint64_t rows);
+
 /* Profiling aid for the chain over gathered centroids (current device): SM cycles its roles spent waiting, summed over
  * the CTAs of all launches since the last call, then cleared.  out16: [0] MMA thread waiting for the rows to hand an
  * accumulator back, [1] waiting for a stage, [2] its whole loop; [3] a row warp waiting for an accumulator, [4] fetching

@@ -233,6 +233,8 @@ skm_status skm_debug_wait_injection(uint64_t wait_limit_cycles, uint32_t produce
 
 void skm_debug_alloc_failures(uint64_t least_bytes, uint64_t most_bytes, int pinned) { skmb::set_debug_alloc_failures(least_bytes, most_bytes, pinned != 0); }
 
+void skm_debug_chain_slice(uint64_t rows) { skmb::set_debug_chain_slice(rows); }
+
 skm_status skm_debug_role_cycles(uint64_t* out16) {
     g_create_error.clear();
     if (!out16) return SKM_INVALID_ARGUMENT;

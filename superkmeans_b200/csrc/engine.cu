@@ -519,11 +519,20 @@ namespace {
 
 tc::ChainShape chain_shape(const PrunedParams& p) { return {static_cast<uint32_t>(p.d), p.partial_d, p.vertical_d, p.horizontal_d}; }
 
-// Points whose halves the chain has at a time: about a gigabyte of them, a whole number of tiles of 256 for every pair of SMs.
+std::atomic<size_t> g_chain_slice{0};
+
+// Points whose halves the chain has at a time: about a gigabyte of them, a whole number of tiles for every pair of SMs.
 size_t chain_slice(const tc::ChainShape& shape, size_t n) {
-    constexpr size_t step = 74 * 256;
+    if (const size_t rows = g_chain_slice) return std::min(n, rows);
+    const size_t step = static_cast<size_t>(tc::sm_pairs()) * kChainTileRows;
     return std::min(n, std::max<size_t>(1, (size_t{1} << 30) / (2 * sizeof(__half) * shape.pitch()) / step) * step);
 }
+
+} // namespace
+
+void set_debug_chain_slice(size_t rows) { g_chain_slice = rows; }
+
+namespace {
 
 // The centroids' side of run_dense.
 void prepare_dense(const PrunedParams& p, PruneSplitWorkspace& ws, PrunePassBuffers& b, cudaStream_t stream) {
@@ -545,7 +554,9 @@ void run_dense(const PrunedParams& p, PruneSplitWorkspace& ws, PrunePassBuffers&
     uint2* top2 = b.listed_top2.ensure(slice);
     // Several blocks per tile shorten the chain but take SMs from the walk beside it: not when the walk over all points (about 0.55 ps
     // per point and centroid) takes longer than one tile's chain (0.17 ns per centroid and dimension) anyway.
-    uint8_t* scratch = side && p.n > 300 * p.d ? nullptr : b.chain_scratch.ensure(tc::chain_scratch_bytes(slice));
+    tc::ChainScratch scratch;
+    if (!(side && p.n > 300 * p.d)) scratch.rows = chain_scratch_rows(n, slice, static_cast<size_t>(tc::sm_pairs()));
+    if (scratch.rows != 0) scratch.p = b.chain_scratch.ensure(tc::chain_scratch_bytes(scratch.rows));
     const cudaStream_t s = side ? side : stream;
     if (side) {
         b.side_start.record(stream);

@@ -146,6 +146,8 @@ struct PrunePassBuffers {
 // it sends to the chain; mode 6 uses the exact gathered chain alone).
 void set_prune_split_mode(int mode);
 int prune_split_mode();
+// Points that the dense chain has at a time (0: as many as a gigabyte holds), for tests.
+void set_debug_chain_slice(size_t rows);
 void run_pruned_pass_on(PrunedParams p, PrunePassBuffers& b, float ratio_first, int device, cudaStream_t stream, PhaseTimers* timers = nullptr);
 
 // Pieces of the draws in pinned memory, piece t at values + t * stretch, entries [start[t], start[t + 1]) of the whole.

@@ -608,4 +608,18 @@ inline size_t pdx_offset(size_t row, size_t dim, size_t n, size_t d, size_t vert
     return base + vertical_d * cs + (h / kHDimSize) * cs * kHDimSize + v * kHDimSize + (h % kHDimSize);
 }
 
+// The dense chain (kernels_chain.cu) goes through its points in slices, on tiles of kChainTileRows points.  While every tile of a launch can have
+// a pair of SMs for each of the kChainUnits units of a chunk, the pairs of a tile tell each other what they found in scratch memory.
+constexpr size_t kChainTileRows = 256;
+constexpr size_t kChainUnits = 4;
+inline bool chain_shares_tiles(size_t n, size_t sm_pairs) { return (n + kChainTileRows - 1) / kChainTileRows * kChainUnits <= sm_pairs; }
+// Points that the scratch must have room for when n of them go through in slices of `slice`: the last slice, being shorter, may share its tiles
+// where the others do not.
+inline size_t chain_scratch_rows(size_t n, size_t slice, size_t sm_pairs) {
+    size_t rows = 0;
+    for (const size_t cnt : {std::min(n, slice), n % slice})
+        if (chain_shares_tiles(cnt, sm_pairs)) rows = std::max(rows, cnt);
+    return rows;
+}
+
 } // namespace skmb

@@ -27,6 +27,7 @@
 
 #include "common.cuh"
 #include "device_utils.cuh"
+#include "host_logic.h"
 #include "kernels_tc.cuh"
 #include "tc_ptx.cuh"
 
@@ -586,19 +587,17 @@ void launch_chain_centroids(const float* y, size_t k, const ChainShape& shape, c
 // Few rows: a pair of blocks per tile leaves most SMs idle.  While every tile can have four pairs, each takes one of the (at most four)
 // units of a chunk, a launch per chunk, and merge_chain_kernel does what the tile's rows do at the end of a chunk.
 constexpr uint32_t kChainSlices = kChunk / CN;
-static int sm_pairs() {
+static_assert(kChainSlices == kChainUnits && kChainTileRows == 256, "chain_shares_tiles counts them");
+int sm_pairs() {
     int device = 0, sms = 0;
     SKM_CUDA(cudaGetDevice(&device));
     SKM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     return sms / 2;
 }
-size_t chain_scratch_bytes(size_t n) {
-    if ((n + 255) / 256 * kChainSlices > static_cast<size_t>(sm_pairs())) return 0;
-    return n * (kChainSlices * sizeof(ChainPartial) + sizeof(ChainState) + sizeof(float));
-}
+size_t chain_scratch_bytes(size_t rows) { return rows * (kChainSlices * sizeof(ChainPartial) + sizeof(ChainState) + sizeof(float)); }
 
 void launch_chain(size_t n, size_t k, const ChainShape& shape, const ChainHalves& x, const ChainHalves& y, const float* ratios, const float* best_in, uint32_t* knn, float* dist,
-                  uint32_t* not_pruned, uint2* top2, void* scratch, cudaStream_t stream, const std::function<void()>& beside) {
+                  uint32_t* not_pruned, uint2* top2, const ChainScratch& scratch, cudaStream_t stream, const std::function<void()>& beside) {
     if (n == 0 || k == 0) return;
     const size_t pitch = shape.pitch();
     ChainMaps maps;
@@ -627,7 +626,7 @@ void launch_chain(size_t n, size_t k, const ChainShape& shape, const ChainHalves
     p.producer_stop = producer_stop();
     const size_t row_tiles = (n + 255) / 256;
     const uint32_t n_chunks = static_cast<uint32_t>((k + kChunk - 1) / kChunk);
-    if (!scratch || chain_scratch_bytes(n) == 0) {
+    if (n > scratch.rows || !chain_shares_tiles(n, static_cast<size_t>(sm_pairs()))) {
         p.chunk_end = n_chunks;
         SKM_CUDA(cudaFuncSetAttribute(chain_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(C_SMEM_BYTES)));
         chain_tc_kernel<1><<<static_cast<unsigned>(2 * std::min<size_t>(row_tiles, static_cast<size_t>(sm_pairs()))), C_THREADS, C_SMEM_BYTES, stream>>>(maps, p);
@@ -636,7 +635,7 @@ void launch_chain(size_t n, size_t k, const ChainShape& shape, const ChainHalves
         return;
     }
     SKM_CUDA(cudaFuncSetAttribute(chain_tc_kernel<kChainSlices>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(C_SMEM_BYTES)));
-    p.partial = static_cast<ChainPartial*>(scratch);
+    p.partial = static_cast<ChainPartial*>(scratch.p);
     ChainState* state = reinterpret_cast<ChainState*>(p.partial + kChainSlices * n);
     float* best = reinterpret_cast<float*>(state + n);
     for (uint32_t c = 0; c < n_chunks; ++c) {

@@ -129,9 +129,15 @@ void launch_chain_centroids(const float* y, size_t k, const ChainShape& shape, c
 
 // Pruned assignment of n points as a dense chain on the tensor cores.  best_in: exact distance to the previous centroid; knn: the previous
 // assignment on entry and the chain's winner on return, which launch_refine_chain settles among it and its two runner-ups (top2).
-size_t chain_scratch_bytes(size_t n);   // of `scratch` below (optional: lets a few rows have several blocks per tile); may be none
+int sm_pairs();   // of the current device
+// Memory (optional) that lets a few points have several blocks per tile, for launches of up to `rows` points.
+struct ChainScratch {
+    void* p = nullptr;
+    size_t rows = 0;
+};
+size_t chain_scratch_bytes(size_t rows);
 void launch_chain(size_t n, size_t k, const ChainShape& shape, const ChainHalves& x, const ChainHalves& y, const float* ratios, const float* best_in, uint32_t* knn, float* dist,
-                  uint32_t* not_pruned, uint2* top2, void* scratch, cudaStream_t stream, const std::function<void()>& beside = nullptr);   // called behind the first launch
+                  uint32_t* not_pruned, uint2* top2, const ChainScratch& scratch, cudaStream_t stream, const std::function<void()>& beside = nullptr);   // called behind the first launch
 // Exact fp32 distances decide among the chain's winner and runner-ups; row i of the chain is row idx[i] of x and of the results, or row i.
 void launch_refine_chain(const float* x, const float* y, size_t n, size_t k, size_t d, const uint2* top2, const uint32_t* idx, const uint32_t* knn, const uint32_t* not_pruned,
                          uint32_t* knn_out, float* dist_out, uint32_t* not_pruned_out, cudaStream_t stream);
