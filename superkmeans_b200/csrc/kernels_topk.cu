@@ -76,6 +76,7 @@ __global__ void __launch_bounds__(kTopkThreads) topk_merge_kernel(const float* _
     const float nq = norms_q[q];
     const unsigned long long* st = lists.state + q * k;
     const uint32_t carried = col0 == 0 ? 0u : k;
+    uint32_t held = carried;   // keys in the buffer, which every thread counts for itself: `count` may have moved on when it is read
     if (slab_n > 2 * kTopkThreads || carried) {
         for (int i = threadIdx.x; i < kTopkBuf; i += kTopkThreads) buf[i] = i < static_cast<int>(carried) ? st[i] : ~0ull;
     } else {
@@ -101,24 +102,25 @@ __global__ void __launch_bounds__(kTopkThreads) topk_merge_kernel(const float* _
             at = __shfl_sync(0xffffffffu, at, 0) + __popc(all & ((1u << lane) - 1u));
             if (kept) buf[at] = key;   // below k + kTopkThreads * rounds, bounded by the flush below
         }
-        __syncthreads();
+        held += static_cast<uint32_t>(__syncthreads_count(kept));
         // one more round adds at most kTopkThreads keys: flush while that still fits
-        if (count + kTopkThreads > kTopkBuf) {
+        if (held + kTopkThreads > kTopkBuf) {
             bitonic_sort(buf, kTopkBuf);
             for (int i = k + threadIdx.x; i < kTopkBuf; i += kTopkThreads) buf[i] = ~0ull;
             if (threadIdx.x == 0) {
                 count = k;
                 tau = buf[k - 1];
             }
+            held = k;
             __syncthreads();
         }
     }
     // what lies behind the keys held is empty: among 300 centroids a sort of 512 takes half the time of one of the whole buffer (9 us for 200
     // lists; places counted key by key: 12)
-    int held = 2;
-    while (held < static_cast<int>(count)) held <<= 1;
-    bitonic_sort(buf, held);
-    for (int i = threadIdx.x; i < static_cast<int>(k); i += kTopkThreads) lists.put(q * k + i, i < held ? buf[i] : ~0ull);
+    int sorted = 2;
+    while (sorted < static_cast<int>(held)) sorted <<= 1;
+    bitonic_sort(buf, sorted);
+    for (int i = threadIdx.x; i < static_cast<int>(k); i += kTopkThreads) lists.put(q * k + i, i < sorted ? buf[i] : ~0ull);
 }
 
 // found[q] = number of the query's ground-truth points whose current cluster is among the clusters the query

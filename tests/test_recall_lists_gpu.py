@@ -28,3 +28,29 @@ def test_recall_of_one_iteration(n, k, objective_k, explore):
     near, clusters = nearest(x64, objective_k), nearest(c64, visited)
     hits = sum(np.isin(assign[near[i]], clusters[i]).sum() for i in range(len(q)))
     assert abs(recall - hits / near.size) <= 2.0 / near.size + 1e-3, (recall, hits / near.size)   # a pair of equally near rows or centroids
+
+
+# after seven rounds of 256 rows the buffer of 2048 keys is one key short of a flush
+@pytest.mark.parametrize("n,objective_k", [(1_792, 5), (1_793, 5), (2_048, 5), (2_304, 256), (2_304, 300), (6_000, 1_536)])
+def test_lists_of_many_queries_repeat_themselves(n, objective_k):
+    """A list is full, or not, for all warps of its block at once: thousands of lists, several times over, give one recall."""
+    import superkmeans_b200 as skm
+
+    d, k = 32, 40
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((n, d), dtype=np.float32)
+    q = rng.standard_normal((3_000, d), dtype=np.float32)
+    recalls = set()
+    for _ in range(5):
+        e = skm.Engine(k, d, skm.default_config(False, iters=2, sampling_fraction=1.0, early_termination=0, objective_k=objective_k, ann_explore_fraction=0.1, suppress_warnings=1,
+                                                data_already_rotated=1, unrotate_centroids=0))
+        c = e.train(x, queries=q)
+        recalls.add(tuple(s.recall for s in e.stats(0)))
+    assert len(recalls) == 1
+    assign = e.assignments()
+    q64 = q.astype(np.float64)
+    # (the recall of an iteration looks at the centroids that it ends with)
+    rows = np.argpartition((x.astype(np.float64) ** 2).sum(1) - 2 * q64 @ x.astype(np.float64).T, objective_k - 1, axis=1)[:, :objective_k]
+    clusters = np.argpartition((c.astype(np.float64) ** 2).sum(1) - 2 * q64 @ c.astype(np.float64).T, 3, axis=1)[:, :4]
+    hits = sum(np.isin(assign[rows[i]], clusters[i]).sum() for i in range(len(q)))
+    assert abs(recalls.pop()[-1] - hits / rows.size) <= 1e-3   # pairs of equally near rows or centroids
