@@ -545,8 +545,20 @@ void run_dense(const PrunedParams& p, PruneSplitWorkspace& ws, PrunePassBuffers&
                const std::function<void()>& beside = nullptr) {
     if (n == 0) return;
     const tc::ChainShape shape = chain_shape(p);
-    const size_t slice = chain_slice(shape, n);
-    const tc::ChainHalves xs = b.chain_points(slice, shape), ys = b.chain_centroids(p.k, shape, ws.chain_norms_y);
+    size_t slice = chain_slice(shape, n);
+    tc::ChainHalves xs{};
+    for (;;) {
+        try {
+            xs = b.chain_points(slice, shape);
+            break;
+        } catch (const OutOfMemory&) {
+            // smaller slices, down to one tile
+            b.give_up_chain_points();
+            if (slice <= kChainTileRows) throw;
+            slice = std::max(kChainTileRows, slice / 2 / kChainTileRows * kChainTileRows);
+        }
+    }
+    const tc::ChainHalves ys = b.chain_centroids(p.k, shape, ws.chain_norms_y);
     float* bestl = idx ? b.listed_best.ensure(slice) : nullptr;
     uint32_t* knnl = idx ? b.listed_knn.ensure(slice) : nullptr;
     float* distl = b.listed_dist.ensure(slice);

@@ -126,6 +126,11 @@ struct PrunePassBuffers {
         __half* h = chain_xh.ensure(2 * halves);
         return {h, h + halves, chain_xf.ensure(rows), chain_norms_x.ensure(rows * shape.n_seg())};
     }
+    void give_up_chain_points() {
+        chain_xh.release();
+        chain_xf.release();
+        chain_norms_x.release();
+    }
     tc::ChainHalves chain_centroids(size_t k, const tc::ChainShape& shape, float* norms) {
         const size_t halves = k * shape.pitch();
         __half* h = chain_yh.ensure(2 * halves);

@@ -57,6 +57,48 @@ def test_list_route():
     assert (got == want).mean() >= 0.999
 
 
+def test_dense_chain_of_a_training():
+    """Unstructured rows go through the dense chain from the first pruned pass on."""
+    import superkmeans_b200 as skm
+
+    n, d, k = 20_000, 256, 400
+    x = np.random.default_rng(0).standard_normal((n, d), dtype=np.float32)
+
+    def train():
+        e = skm.Engine(k, d, skm.default_config(False, sampling_fraction=1.0, iters=3, early_termination=0, data_already_rotated=1))
+        c = e.train(x)
+        return c, e.assignments(), e.last_prune_path
+
+    want = train()
+    assert want[2] == 3
+    with without(4 * n * d + 1, 4 * n * (d + 128)):   # the halves of all points, whose segments are padded to 64 columns
+        got = train()
+    for a, b in zip(want, got):
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("least", [4_900, 2_500, 1_000])
+def test_dense_chain(least):
+    from superkmeans_b200 import _lib, engine
+
+    n, d, k = 20_000, 256, 400
+    x = datagen.gaussian_mixture(n, d, k, 0.3, 4)
+    y = datagen.gaussian_mixture(k, d, k, 0.3, 5)
+    prev = np.random.default_rng(0).integers(0, k, n).astype(np.uint32)
+    pitch = 320   # d' = 96: segments of 96, 64 and 96 columns
+    engine.set_prune_split(3)
+    try:
+        want = engine.find_nearest_pruned(x, y, prev, 96)
+        _lib.lib.skm_debug_chain_slice(9_728)
+        with without(4 * least * pitch, 4 * 9_728 * pitch):
+            got = engine.find_nearest_pruned(x, y, prev, 96)
+    finally:
+        _lib.lib.skm_debug_chain_slice(0)
+        engine.set_prune_split(0)
+    for a, b in zip(want, got):
+        np.testing.assert_array_equal(a, b)
+
+
 def test_exact_assignment():
     import torch
 
