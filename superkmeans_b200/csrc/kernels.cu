@@ -1118,6 +1118,7 @@ __global__ void __launch_bounds__(256) consolidate_kernel(const ConsolidateParam
 // points among all of them (a piece at a time, their rows in a fixed order), adds their rows up, and has the cluster's centroid.
 constexpr int kSmallPiece = 4096;
 constexpr int kSmallLoads = 8;   // rows in flight per thread
+constexpr uint32_t kSmallChain = 32;   // rows, or sums of rows, added one after the other: no more than in a tile of the large update
 __global__ void __launch_bounds__(256) small_update_kernel(const float* __restrict__ x, const uint32_t* __restrict__ assign, size_t n, const UpdateStats u, uint32_t* __restrict__ counts,
                                                            const ConsolidateParams p) {
     __shared__ uint32_t ids[kSmallPiece];
@@ -1130,8 +1131,8 @@ __global__ void __launch_bounds__(256) small_update_kernel(const float* __restri
     const uint32_t g = threadIdx.x % groups, r = threadIdx.x / groups;
     double cost = 0.0;
     unsigned long long not_pruned = 0;
-    uint32_t count = 0;
-    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    uint32_t count = 0, loads = 0;
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f), total = sum;
     for (size_t base = 0; base < n; base += kSmallPiece) {
         uint32_t mask = 0;
 #pragma unroll
@@ -1176,21 +1177,32 @@ __global__ void __launch_bounds__(256) small_update_kernel(const float* __restri
                     sum.z += v[q].z;
                     sum.w += v[q].w;
                 }
+                if (++loads % (kSmallChain / kSmallLoads) == 0) {
+                    total = make_float4(total.x + sum.x, total.y + sum.y, total.z + sum.z, total.w + sum.w);
+                    sum = make_float4(0.f, 0.f, 0.f, 0.f);
+                }
             }
         }
         __syncthreads();
     }
+    sum = make_float4(total.x + sum.x, total.y + sum.y, total.z + sum.z, total.w + sum.w);
     parts[threadIdx.x] = sum;
     __syncthreads();
     float s = 0.f;
     if (r == 0) {
+        total = make_float4(0.f, 0.f, 0.f, 0.f);
         for (uint32_t q = 1; q < rows; ++q) {
             const float4 t = parts[q * groups + g];
             sum.x += t.x;
             sum.y += t.y;
             sum.z += t.z;
             sum.w += t.w;
+            if (q % kSmallChain == 0) {
+                total = make_float4(total.x + sum.x, total.y + sum.y, total.z + sum.z, total.w + sum.w);
+                sum = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
         }
+        sum = make_float4(total.x + sum.x, total.y + sum.y, total.z + sum.z, total.w + sum.w);
         const float mult = count ? static_cast<float>(1.0 / static_cast<double>(count)) : 1.0f;
         const float val[4] = {__fmul_rn(sum.x, mult), __fmul_rn(sum.y, mult), __fmul_rn(sum.z, mult), __fmul_rn(sum.w, mult)};
         const size_t chunk = cluster / kChunk, v = cluster % kChunk;

@@ -34,3 +34,17 @@ def test_an_iteration_of_a_small_problem(n, k, d, skewed):
                 assert abs(st.shift - want) <= 1e-4 * want + 1e-9
         before = snap["centroids"].astype(np.float64)
     np.testing.assert_array_equal(c, e.trace()[-1]["centroids"])
+
+
+@pytest.mark.parametrize("n,d", [(512, 1_024), (2_048, 256), (8_192, 64)])
+def test_sums_of_many_equal_rows(n, d):
+    """512 rows a thread, of values that a sum of more than 256 of them rounds off all in one direction."""
+    import superkmeans_b200 as skm
+
+    v = (1.0 + np.linspace(0.5, 1.0, d) * 2.0 ** -16).astype(np.float32)
+    e = skm.Engine(1, d, skm.default_config(False, iters=1, sampling_fraction=1.0, early_termination=0, data_already_rotated=1))
+    e.set_trace(True)
+    e.train(np.tile(v, (n, 1)))
+    # half a unit of every partial sum: 2^-24 (1 + .. + 128) / 128 in a chain of 128 rows, and as in a chain of 32 for what adds such sums up
+    error = np.abs(e.trace()[-1]["centroids"][0].astype(np.float64) / v - 1)
+    assert error.max() <= 2.0 ** -24 * (129 / 2 + 33 / 2 + 1), error.max()
