@@ -267,8 +267,10 @@ uint64_t skm_cached_memory_bytes(void);
 /* ---- single operators of the path, for callers that hold their own state and for parity tests.
  * All arguments in host memory; each call uploads, runs the kernels and downloads. ------------- */
 
-/* ADSamplingPruner::Rotate, matrix branch (adsampling.h:191-215): out = x * m^T. */
+/* ADSamplingPruner::Rotate, matrix branch (adsampling.h:191-215): out = x * m^T, by the kernel that rotates the rows of a
+ * training, and by the one for rows that a trained model is applied to. */
 skm_status skm_op_rotate(int device, const float* m, const float* x, uint64_t n, uint64_t d, float* out);
+skm_status skm_op_rotate_to_assign(int device, const float* m, const float* x, uint64_t n, uint64_t d, float* out);
 /* ADSamplingPruner::Unrotate, matrix branch (adsampling.h:273-298): out = x * m. */
 skm_status skm_op_unrotate(int device, const float* m, const float* x, uint64_t n, uint64_t d, float* out);
 /* BatchComputer::FindNearestNeighbor (include/superkmeans/distance_computers/batch_computers.h:104-171)

@@ -299,12 +299,17 @@ uint64_t skm_cached_memory_bytes(void) { return skmb::cached_memory_bytes(); }
 // ---- operators ------------------------------------------------------------------------------
 skm_status skm_op_rotate(int device, const float* m, const float* x, uint64_t n, uint64_t d, float* out) {
     g_create_error.clear();
-    return guarded(g_op_error, [&] { Engine::op_rotate(device, m, x, n, d, out, false); });
+    return guarded(g_op_error, [&] { Engine::op_rotate(device, m, x, n, d, out, skmb::RotateOp::train); });
+}
+
+skm_status skm_op_rotate_to_assign(int device, const float* m, const float* x, uint64_t n, uint64_t d, float* out) {
+    g_create_error.clear();
+    return guarded(g_op_error, [&] { Engine::op_rotate(device, m, x, n, d, out, skmb::RotateOp::to_assign); });
 }
 
 skm_status skm_op_unrotate(int device, const float* m, const float* x, uint64_t n, uint64_t d, float* out) {
     g_create_error.clear();
-    return guarded(g_op_error, [&] { Engine::op_rotate(device, m, x, n, d, out, true); });
+    return guarded(g_op_error, [&] { Engine::op_rotate(device, m, x, n, d, out, skmb::RotateOp::back); });
 }
 
 skm_status skm_op_find_nearest(int device, const float* x, const float* y, uint64_t n, uint64_t k, uint64_t d, uint32_t* out_knn, float* out_dist) {

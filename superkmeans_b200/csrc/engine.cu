@@ -2093,18 +2093,18 @@ struct OpContext {
 };
 } // namespace
 
-void Engine::op_rotate(int device, const float* m, const float* x, size_t n, size_t d, float* out, bool inverse) {
+void Engine::op_rotate(int device, const float* m, const float* x, size_t n, size_t d, float* out, RotateOp op) {
     OpContext ctx(device);
     DeviceBuffer<float> md, mtd, xd, od;
     ctx.upload(md, m, d * d);
     const float* b = md.get();
-    if (inverse) {
+    if (op == RotateOp::back) {
         launch_transpose_square(md.get(), mtd.ensure(d * d), d, ctx.stream);
         b = mtd.get();
     }
     ctx.upload(xd, x, n * d);
-    if (inverse) launch_gemm_nt(xd.get(), d, b, d, od.ensure(n * d), d, n, d, d, ctx.stream);
-    else launch_rotate_to_assign(xd.get(), d, b, od.ensure(n * d), d, n, d, d, ctx.stream);
+    if (op == RotateOp::to_assign) launch_rotate_to_assign(xd.get(), d, b, od.ensure(n * d), d, n, d, d, ctx.stream);
+    else launch_gemm_nt(xd.get(), d, b, d, od.ensure(n * d), d, n, d, d, ctx.stream);
     ctx.download(out, od.get(), n * d);
     ctx.sync();
     check_tc_error(ctx.stream);

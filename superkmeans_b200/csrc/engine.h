@@ -168,6 +168,9 @@ void launch_collect_draws(const DrawPieces& p, float* out, cudaStream_t stream);
 // (synchronised once or twice on the way).  False: declined, nothing usable in `out` (rotation_matrix.cu).
 bool make_rotation_matrix_on_device(const float* draws, size_t d, float* out, cudaStream_t stream);
 
+// Rotation of the rows of a training, of rows that a trained model is applied to, and of centroids back.
+enum class RotateOp { train, to_assign, back };
+
 class Engine {
   public:
     Engine(const skm_config& cfg, size_t n_clusters, size_t d, bool hierarchical, int device);
@@ -227,7 +230,7 @@ class Engine {
     }
 
     // Stateless operators (used by the skm_op_* entry points).
-    static void op_rotate(int device, const float* m, const float* x, size_t n, size_t d, float* out, bool inverse);
+    static void op_rotate(int device, const float* m, const float* x, size_t n, size_t d, float* out, RotateOp op);
     static void op_find_nearest(int device, const float* x, const float* y, size_t n, size_t k, size_t d, uint32_t* out_knn, float* out_dist);
     static void op_find_nearest_pruned(int device, const float* x, const float* y, size_t n, size_t k, size_t d, float eps0, uint32_t partial_d, uint32_t* knn_io, float* dist_out,
                                        uint64_t* not_pruned_out);

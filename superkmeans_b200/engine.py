@@ -315,10 +315,11 @@ def device_allocations() -> int:
 
 # ---- stateless operators (host arrays in, host arrays out) ------------------------------------
 
-def rotate(m: np.ndarray, x: np.ndarray, device: int = -1) -> np.ndarray:
+def rotate(m: np.ndarray, x: np.ndarray, device: int = -1, to_assign: bool = False) -> np.ndarray:
+    """x m^T as a training rotates its rows, or as rows are rotated that a trained model is applied to."""
     m, x = _f32(m), _f32(x)
     out = np.empty_like(x)
-    check(lib.skm_op_rotate(device, m, x, x.shape[0], x.shape[1], out))
+    check((lib.skm_op_rotate_to_assign if to_assign else lib.skm_op_rotate)(device, m, x, x.shape[0], x.shape[1], out))
     return out
 
 

@@ -66,15 +66,20 @@ def test_exact_assignment(early_stop, n, k, d):
     np.testing.assert_array_equal(engine.find_nearest(x, y)[0], want)
 
 
-def test_rotation(early_stop):
+@pytest.mark.parametrize("which", ["of a training", "to assign", "back"])
+def test_rotation(early_stop, which):
     from superkmeans_b200 import engine
 
     rng = np.random.default_rng(1)
     x, m = rng.standard_normal((3_000, 256), dtype=np.float32), rng.standard_normal((256, 256), dtype=np.float32)
-    want = engine.rotate(m, x)
+
+    def rotate():
+        return engine.unrotate(m, x) if which == "back" else engine.rotate(m, x, to_assign=which == "to assign")
+
+    want = rotate()
     with early_stop, pytest.raises(RuntimeError, match="gave up waiting on a barrier"):
-        engine.rotate(m, x)
-    np.testing.assert_array_equal(engine.rotate(m, x), want)
+        rotate()
+    np.testing.assert_array_equal(rotate(), want)
 
 
 @pytest.mark.parametrize("n,mode", [(4_096, 4), (4_096, 9), (2_000, 3), (30_000, 3)], ids=["first test", "first test that drops", "chain in slices", "chain"])

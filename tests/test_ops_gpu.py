@@ -41,14 +41,14 @@ def test_rotate_and_unrotate(eng, ref, n, d):
     rng = np.random.default_rng(1)
     x = rng.standard_normal((n, d), dtype=np.float32)
     m = eng.rotation_matrix(d, 3)
-    r = eng.rotate(m, x)
     want = x.astype(np.float64) @ m.astype(np.float64).T
-    # fp32 accumulation level: rows have norm sqrt(d), outputs are O(1); a single long chain in tensor memory would be ~1e-5 * sqrt(d) off
-    assert np.abs(r - want).max() < 1e-6 * np.sqrt(d)
-    # tests/test_rotation.cpp: norms preserved, Unrotate(Rotate(x)) = x within 1e-4
-    assert np.abs(np.linalg.norm(r, axis=1) - np.linalg.norm(x, axis=1)).max() < 1e-4 * np.sqrt(d)
-    back = eng.unrotate(m, r)
-    assert np.abs(back - x).max() < 1e-4
+    for r in (eng.rotate(m, x), eng.rotate(m, x, to_assign=True)):
+        # fp32 accumulation level: rows have norm sqrt(d), outputs are O(1); a single long chain in tensor memory would be ~1e-5 * sqrt(d) off
+        assert np.abs(r - want).max() < 1e-6 * np.sqrt(d)
+        # tests/test_rotation.cpp: norms preserved, Unrotate(Rotate(x)) = x within 1e-4
+        assert np.abs(np.linalg.norm(r, axis=1) - np.linalg.norm(x, axis=1)).max() < 1e-4 * np.sqrt(d)
+        back = eng.unrotate(m, r)
+        assert np.abs(back - x).max() < 1e-4
 
 
 @pytest.mark.parametrize("n,k,d", [(5000, 1000, 64), (4097, 1025, 128), (333, 7, 33), (3000, 2500, 768), (1, 1, 4), (128, 128, 16)])

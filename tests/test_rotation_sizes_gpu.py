@@ -13,6 +13,6 @@ def test_rotation_and_back(n, d):
     x = rng.standard_normal((n, d), dtype=np.float32)
     m = rng.standard_normal((d, d), dtype=np.float32)
     scale = np.linalg.norm(x.astype(np.float64), axis=1)[:, None]
-    for got, mat in ((skm.engine.rotate(m, x), m.T), (skm.engine.unrotate(m, x), m)):
+    for got, mat in ((skm.engine.rotate(m, x), m.T), (skm.engine.rotate(m, x, to_assign=True), m.T), (skm.engine.unrotate(m, x), m)):
         want = x.astype(np.float64) @ mat.astype(np.float64)
         assert (np.abs(got - want) <= 3e-6 * scale * np.linalg.norm(mat.astype(np.float64), axis=0)).all()

@@ -1,4 +1,4 @@
-"""Rotation of rows of any width and magnitude: widths at the edges of what the conversion to fp16 halves holds in registers, rows that
+"""Rotation, of rows that a trained model is applied to, of rows of any width and magnitude: widths at the edges of what the conversion to fp16 halves holds in registers, rows that
 16-byte loads cannot address, row counts around a tile and around one tile per pair of SMs."""
 import numpy as np
 import pytest
@@ -15,7 +15,7 @@ def test_rows_of_any_width_and_magnitude(n, d):
     x = rng.standard_normal((n, d), dtype=np.float32) * (10.0 ** rng.uniform(-25, 25, (n, 1))).astype(np.float32)
     x[n // 2] = 0
     m = rng.standard_normal((d, d), dtype=np.float32) * (10.0 ** rng.uniform(-3, 3, (d, 1))).astype(np.float32)
-    got = skm.engine.rotate(m, x)
+    got = skm.engine.rotate(m, x, to_assign=True)
     want = x.astype(np.float64) @ m.T.astype(np.float64)
     # 22 bits of either factor; 64 terms one after the other in an accumulator that truncates, then fp32
     scale = np.linalg.norm(x.astype(np.float64), axis=1)[:, None] * np.linalg.norm(m.astype(np.float64), axis=1)
