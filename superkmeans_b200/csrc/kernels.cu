@@ -133,8 +133,12 @@ void launch_gemm_nt(const float* a, size_t lda, const float* b, size_t ldb, floa
     SKM_LAUNCH_CHECK();
 }
 
+// Rows that 16-byte loads cannot address have the fp32 tiles otherwise, whose sums of up to 64 products are closer to 64 bits than those of 22-bit
+// halves (rms error relative to a row's length: d = 33: 1.8e-8 against 2.0e-8, 50: 1.8e-8 and 1.9e-8, 57: 1.8e-8 both, 101: 1.8e-8 and 1.3e-8, 1023:
+// 1.8e-8 and 0.5e-8).  Aligned rows have the tf32 kernel otherwise: 3.4e-8 (d = 32) to 7.0e-8 (1536) against 1.9e-8 to 0.4e-8.
 void launch_rotate_to_assign(const float* a, size_t lda, const float* b, float* out, size_t ldo, size_t n, size_t n_out, size_t k_dim, cudaStream_t stream) {
-    if (n != 0 && n_out != 0 && tc::enabled() && k_dim >= 32) tc::launch_rotate_halves(a, lda, b, out, ldo, n, n_out, k_dim, stream);
+    const bool addressable = lda % 4 == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0;
+    if (n != 0 && n_out != 0 && tc::enabled() && k_dim >= (addressable ? 32 : 64)) tc::launch_rotate_halves(a, lda, b, out, ldo, n, n_out, k_dim, stream);
     else launch_gemm_nt(a, lda, b, k_dim, out, ldo, n, n_out, k_dim, stream);
 }
 
