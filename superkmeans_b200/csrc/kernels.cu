@@ -138,8 +138,14 @@ void launch_gemm_nt(const float* a, size_t lda, const float* b, size_t ldb, floa
 // 1.8e-8 and 0.5e-8).  Aligned rows have the tf32 kernel otherwise: 3.4e-8 (d = 32) to 7.0e-8 (1536) against 1.9e-8 to 0.4e-8.
 void launch_rotate_to_assign(const float* a, size_t lda, const float* b, float* out, size_t ldo, size_t n, size_t n_out, size_t k_dim, cudaStream_t stream) {
     const bool addressable = lda % 4 == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0;
-    if (n != 0 && n_out != 0 && tc::enabled() && k_dim >= (addressable ? 32 : 64)) tc::launch_rotate_halves(a, lda, b, out, ldo, n, n_out, k_dim, stream);
-    else launch_gemm_nt(a, lda, b, k_dim, out, ldo, n, n_out, k_dim, stream);
+    if (n != 0 && n_out != 0 && tc::enabled() && k_dim >= (addressable ? 32 : 64)) {
+        try {
+            tc::launch_rotate_halves(a, lda, b, out, ldo, n, n_out, k_dim, stream);
+            return;
+        } catch (const OutOfMemory&) {   // (of its scratch, before anything is launched; the fp32 tiles have none)
+        }
+    }
+    launch_gemm_nt(a, lda, b, k_dim, out, ldo, n, n_out, k_dim, stream);
 }
 
 __global__ void transpose_square_kernel(const float* __restrict__ in, float* __restrict__ out, size_t n) {

@@ -37,6 +37,17 @@ def test_rotation_matrix(pinned, beside):
     np.testing.assert_array_equal(m, skm.engine.rotation_matrix(d, 42))
 
 
+def test_rotation_of_odd_rows():
+    from superkmeans_b200 import engine
+
+    n, d = 20_000, 130
+    rng = np.random.default_rng(0)
+    x, m = rng.standard_normal((n, d), dtype=np.float32), rng.standard_normal((d, d), dtype=np.float32)
+    with without(4 * n * (d + 2), 4 * n * (d + 2) + 16 * d * (d + 6)):   # the padded rows and the halves of the matrix
+        got = engine.rotate(m, x, to_assign=True)
+    np.testing.assert_array_equal(got, engine.rotate(m, x))   # the fp32 tiles
+
+
 def test_list_route():
     import superkmeans_b200 as skm
 
