@@ -412,12 +412,12 @@ void Engine::exact_assignment(const float* x, size_t n, const float* c, size_t k
         exact_.settle_on_device(x, knn, dist, stream_);
         return;
     }
-    DeviceBuffer<float> own;
-    if (!dist) dist = own.ensure(n);
     if (route == AssignRoute::direct) {
         direct_.run(x, c, n, k, d_, norms_x, norms_c, knn, dist, stream_);
         return;
     }
+    DeviceBuffer<float> own;
+    if (!dist) dist = own.ensure(n);
     launch_row_sqnorms(c, k, d_, d_, norms_c, stream_);
     if (!norms_known) launch_row_sqnorms(x, n, d_, d_, norms_x, stream_);
     launch_assign_full(x, c, n, k, d_, norms_x, norms_c, knn, dist, top2_.ensure(n), stream_, y_split_.ensure(2 * k * d_));
