@@ -27,7 +27,7 @@ namespace skmb {
 // Device buffers of one pruned assignment pass (candidate lists, work split) and the pass itself:
 // preparation, candidate-list kernel for the cheap points, dense chain for the expensive ones.
 struct PrunePassBuffers {
-    DeviceBuffer<uint2> lists, top2;
+    DeviceBuffer<uint2> lists;
     DeviceBuffer<float> best, sample, sample_norms, chain_norms_y;
     DeviceBuffer<float> chain_norms_x;
     DeviceBuffer<uint32_t> flags, positions, hard_idx, n_hard_dev;
