@@ -392,24 +392,27 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(C_THREADS, 1) chain_
                     }
                 }
                 uint32_t al = bits[0] | bits[1] << 8 | bits[2] << 16 | bits[3] << 24;
+                uint32_t compete = 0;   // at the last checkpoint
                 if (first) {
                     const uint32_t lo = ch * 32;
                     al &= (cols_valid >= lo + 32) ? 0xFFFFFFFFu : (cols_valid > lo ? ((1u << (cols_valid - lo)) - 1u) : 0u);
                     cnt += __popc(al);
                     const size_t at = static_cast<size_t>(prev) - (col0 + lo);   // (wraps when the previous centroid is before these columns)
                     if (at < 32 && ((al >> at) & 1u)) prev_first = true;
+                    compete = al;
                 } else {
-                    al &= ch ? alive_hi : alive_lo;
+                    compete = ch ? alive_hi : alive_lo;
+                    al &= compete;
                 }
                 if (ch) alive_hi = al;
                 else alive_lo = al;
-                if (last && __any_sync(0xffffffffu, al != 0)) {
-                    // Last checkpoint: the pairs still alive compete.  thr == best here (ratio[d] == 1).
-                    // Runner-ups by the chain's own (slightly truncated) distances; the fp32 refinement afterwards decides among them and
-                    // the chain's winner.
+                if (last && __any_sync(0xffffffffu, compete != 0)) {
+                    // Last checkpoint: the pairs alive until here compete, those below the threshold (which is `best`: ratio[d] == 1) for the chain's
+                    // winner.  Its distances are truncated, by 3e-5 of the norms at d = 1536, so that a centroid a little nearer than the previous one may
+                    // end above it: the runner-ups are taken from all of them, and the fp32 refinement afterwards decides.
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
-                        if ((al >> j) & 1u) {
+                        if ((compete >> j) & 1u) {
                             const float pd = __uint_as_float(r[j]);
                             const uint32_t gc = static_cast<uint32_t>(col0 + ch * 32 + j);
                             if (pd < t2) {
@@ -419,7 +422,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(C_THREADS, 1) chain_
                                 t1 = nearer ? pd : t1;
                                 i1 = nearer ? gc : i1;
                             }
-                            if (pd < cb) {
+                            if (((al >> j) & 1u) && pd < cb) {
                                 cb = pd;
                                 cbi = gc;
                             }

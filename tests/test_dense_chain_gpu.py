@@ -33,3 +33,32 @@ def test_chain_on_the_tensor_cores(n, k, d):
         # pairs within rounding of a threshold of the search
         assert (knn == out[2][0]).mean() >= 0.999 - 1.0 / n
         assert abs(float(out[3][2].sum()) - float(out[2][2].sum())) <= 1e-3 * float(out[2][2].sum()) + 2
+
+
+@pytest.mark.parametrize("n,d", [(500, 132), (700, 256), (500, 768), (1_200, 1_024), (500, 1_536), (5_000, 384)])
+def test_a_centroid_a_little_nearer_than_the_previous_one(n, d):
+    """Every row has its previous centroid and one that is nearer by less than the rounding of the tensor cores' sums: the refinement sees it,
+    whatever those sums say."""
+    from superkmeans_b200 import engine
+
+    rng = np.random.default_rng(d)
+    x = rng.standard_normal((n, d))
+    x /= np.linalg.norm(x, axis=1, keepdims=True)
+
+    def away(r):
+        u = rng.standard_normal((n, d))
+        return x + r * u / np.linalg.norm(u, axis=1, keepdims=True)
+
+    y = np.empty((2 * n, d))
+    y[0::2], y[1::2] = away(0.3), away(0.3 * (1 - 5e-6))
+    x, y, prev = x.astype(np.float32), y.astype(np.float32), np.arange(0, 2 * n, 2, dtype=np.uint32)
+    found = {}
+    for mode in (2, 3):
+        engine.set_prune_split(mode)
+        try:
+            found[mode] = engine.find_nearest_pruned(x, y, prev, engine.dimension_split(d)[1] // 2)[0] == prev + 1
+        finally:
+            engine.set_prune_split(0)
+    # the search may drop it on the way, in either form; what the fp32 form finds is found, but for pairs within rounding of a threshold
+    assert found[2].mean() >= 0.5
+    assert (found[3] | ~found[2]).mean() >= 0.99, (found[2].mean(), found[3].mean())
