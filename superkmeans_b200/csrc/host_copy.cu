@@ -31,7 +31,10 @@ int threads_for(size_t bytes) { return static_cast<int>(std::max<size_t>(1, std:
 // Copies to memory that the GPU reads next, past the caches: what another core has just written to its cache the link fetches at
 // 30 GB/s (4 MB, eight threads: 138 us), what lies in memory at 50 (84 us).  Filling it takes 66 us in place of 44, beside the copy before.
 // A cache line must not be written both ways, so that only whole lines are streamed, the ends of a contiguous part are not.
-// publish() comes behind the last of a thread.
+// publish() comes behind the last of a thread.  A few rows are in one core's cache, and the link is not what they wait for: a call that assigns 32 KB of
+// rows takes 52.3 us with plain stores and 53.5 past the caches, 48 KB 53.2 and 54.6, 56 KB 57.2 and 54.6, 128 KB 62 and 58, 1 MB 101 and 83.  Beyond
+// the last level of the caches there is little in it either way: 350 MB: 7.4 - 8.0 ms and 7.8 - 8.3 when repeated, 8.8 and 8.4 the first time.
+constexpr size_t kStreamFrom = 56 << 10;
 void stream_bytes(char* dst, const char* src, size_t bytes) {
 #ifdef __SSE2__
     const size_t head = std::min(bytes, static_cast<size_t>(-reinterpret_cast<uintptr_t>(dst) & 63));
@@ -55,21 +58,29 @@ void publish() {
 
 // `to_gpu`: the GPU reads dst, else the caller does.
 void copy_bytes(char* dst, const char* src, size_t bytes, bool to_gpu) {
+    const bool past_caches = to_gpu && bytes >= kStreamFrom;
+    auto part = [&](size_t b, size_t e) {
+        if (past_caches) {
+            stream_bytes(dst + b, src + b, e - b);
+            publish();
+        } else {
+            std::memcpy(dst + b, src + b, e - b);
+        }
+    };
     const int threads = threads_for(bytes);
-#pragma omp parallel for num_threads(threads) schedule(static) if (threads > 1)
-    for (int t = 0; t < threads; ++t) {
-        const size_t b = bytes * t / threads, e = bytes * (t + 1) / threads;
-        if (to_gpu) stream_bytes(dst + b, src + b, e - b);
-        else std::memcpy(dst + b, src + b, e - b);
-        publish();
+    if (threads == 1) {   // (a team of one too costs a call with three copies most of a microsecond)
+        part(0, bytes);
+        return;
     }
+#pragma omp parallel for num_threads(threads) schedule(static)
+    for (int t = 0; t < threads; ++t) part(bytes * t / threads, bytes * (t + 1) / threads);
 }
 
 // Rows of whole cache lines are streamed.  Others share lines with their neighbours: a Train on 98 857 of 329 524 rows of 624 bytes took 13.3 ms
 // with streaming stores and 8.8 with plain ones.
 void gather_rows(char* dst, const char* src, const size_t* idx, size_t n, size_t row_bytes) {
     const int threads = threads_for(n * row_bytes);
-    const bool lines = row_bytes % 64 == 0 && reinterpret_cast<uintptr_t>(dst) % 64 == 0;
+    const bool lines = n * row_bytes >= kStreamFrom && row_bytes % 64 == 0 && reinterpret_cast<uintptr_t>(dst) % 64 == 0;
 #pragma omp parallel for num_threads(threads) schedule(static) if (threads > 1)
     for (int t = 0; t < threads; ++t) {
         for (size_t i = n * t / threads; i < n * (t + 1) / threads; ++i) {

@@ -1,4 +1,6 @@
 // Copies of host rows (host_copy.cu) when something goes wrong on the way (fake_cuda_runtime.h).
+#include <algorithm>
+#include <cstring>
 #include <stdexcept>
 
 #include "../../superkmeans_b200/csrc/host_copy.h"
@@ -70,6 +72,34 @@ void rows_arrive() {
     release_stream(work, 0);
 }
 
+// Pieces of all lengths around those from which the stores go past the caches, from rows that start anywhere.
+void pieces_of_any_length() {
+    const cudaStream_t s = acquire_stream();
+    {
+        WorkStream on(s);
+        HostStage stage;
+        std::vector<unsigned char> rows((3 << 20) + 128), got(rows.size());
+        for (size_t i = 0; i < rows.size(); ++i) rows[i] = static_cast<unsigned char>(i * 2654435761u >> 13);
+        for (const size_t row_bytes : {size_t{4}, size_t{60}, size_t{64}, size_t{256}}) {
+            for (const size_t bytes : {size_t{4}, size_t{60}, size_t{64}, size_t{4096}, size_t{57'340}, size_t{57'344}, size_t{57'348}, size_t{114'688}, size_t{600'000}, size_t{3} << 20}) {
+                const size_t n = bytes / row_bytes;
+                std::vector<size_t> idx(n);
+                for (size_t i = 0; i < n; ++i) idx[i] = n - 1 - i;
+                for (const size_t from : {size_t{0}, size_t{4}, size_t{68}}) {
+                    for (const bool gathered : {false, true}) {
+                        std::fill(got.begin(), got.end(), 0);
+                        stage.upload(got.data(), rows.data() + from, gathered ? idx.data() : nullptr, n, row_bytes, s);
+                        SKM_CUDA(cudaStreamSynchronize(s));
+                        for (size_t i = 0; i < n; ++i) CHECK(std::memcmp(got.data() + i * row_bytes, rows.data() + from + (gathered ? idx[i] : i) * row_bytes, row_bytes) == 0);
+                        CHECK(std::count(got.begin() + n * row_bytes, got.begin() + n * row_bytes + 64, 0) == 64);
+                    }
+                }
+            }
+        }
+    }
+    release_stream(s, 0);
+}
+
 // Device memory where host memory is expected.
 void device_memory() {
     const cudaStream_t s = acquire_stream();
@@ -99,6 +129,7 @@ int main(int argc, char** argv) {
     if (what == "exception_behind_a_copy") exception_behind_a_copy(false);
     else if (what == "exception_behind_a_pinned_copy") exception_behind_a_copy(true);
     else if (what == "rows_arrive") rows_arrive();
+    else if (what == "pieces_of_any_length") pieces_of_any_length();
     else if (what == "device_memory") device_memory();
     else return 2;
     std::puts("OK");

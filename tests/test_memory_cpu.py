@@ -35,7 +35,7 @@ def program(tmp_path_factory):
 
 
 @pytest.mark.parametrize("name,case", [("memory_check", "events_between_devices"), ("memory_check", "record_that_fails"), ("memory_check", "modes"), ("memory_check", "device_memory_that_is_short"), ("memory_check", "pinned_memory_that_is_short"),
-                                       ("copies_check", "exception_behind_a_copy"), ("copies_check", "exception_behind_a_pinned_copy"), ("copies_check", "rows_arrive"), ("copies_check", "device_memory"),
+                                       ("copies_check", "exception_behind_a_copy"), ("copies_check", "exception_behind_a_pinned_copy"), ("copies_check", "rows_arrive"), ("copies_check", "pieces_of_any_length"), ("copies_check", "device_memory"),
                                        ("timers_check", "many_calls"), ("timers_check", "nothing_unfinished_is_read")])
 def test_with_a_runtime_of_host_code(program, name, case):
     res = subprocess.run([program(name), case], capture_output=True, text=True, timeout=120)
