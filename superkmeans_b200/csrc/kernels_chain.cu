@@ -6,10 +6,15 @@
 // them (without clearing), turn them into ||x||^2 + ||c||^2 - 2 x.c over the dimensions seen so far with precomputed cumulative
 // norms, and update a bit mask of surviving centroids.
 //
-// Points and centroids come as fp16 pairs v * scale = hi + lo (a power of two per row, 22 bits: what two tf32 parts hold), products are
-// hi*hi + hi*lo + lo*hi with fp32 accumulation.  Their columns are laid out in the order of the chain, every segment from a
-// multiple of 64 on with zeros behind it, so that a segment is a run of whole stages whatever d' is.  A pass writes the halves of its
-// points (chain_points_kernel, which also gathers them and makes their cumulative norms) and of the centroids anyway.
+// Points and centroids come as fp16 pairs v * scale = hi + lo, products are hi*hi + hi*lo + lo*hi with fp32 accumulation.  The scale is a power of
+// two per row: values down to 2^-17 of the row's norm have 22 bits (as two tf32 parts have), smaller ones are off by 2^-39 of the norm at most, which is
+// far below what the accumulator's truncation and the norms' rounding leave (2^-24 of the norms).  Against 64 bits the chain is closer than
+// with tf32 parts, which take twice as many truncated additions: of 60 000 points these have another count of first-test survivors: 1024 columns,
+// k = 4000: 81 (tf32: 128) and, unstructured, 106 (229); 1536, k = 2048: 37 (67) and 67 (125); 768, k = 1000: 13 (15) and 3 (6); columns scaled from 1 to
+// 1e-6: 21 (28).
+// Their columns are laid out in the order of the chain, every segment from a multiple of 64 on with zeros behind it, so that a segment is a run
+// of whole stages whatever d' is.  A pass writes the halves of its points (chain_points_kernel, which also gathers them and makes their
+// cumulative norms) and of the centroids anyway.
 //
 // Persistent pairs of CTAs (cta_group::2) on tiles of 256 points x 256 centroids (a unit), 18 warps:
 //   warp 0      TMA producer: 128 x 64 halves of each of the four parts per stage and CTA, three stages;
@@ -19,8 +24,10 @@
 // The two accumulators belong to two neighbouring units that advance through the segments in turn, so the tensor pipe works on one
 // unit while the tests read the other.
 // What bounds it is the tests (their issue and latency, as in kernels_first_test.cu) and, beside the walk, the SMs shared with it.  One
-// B200, nine passes of a Train with the walk beside them, against three tf32 products on single CTAs whose points four warps split in
-// shared memory: 1M x 1024, k = 4000: 16.2 ms -> 10.5, 250 000 x 1536, k = 2048: 3.3 -> 2.5, 30 000 x 768, k = 1000: 0.45 -> 0.32.
+// B200, the phase of the chain against three tf32 products on single CTAs whose points four warps split in shared memory.  All points in the chain
+// (unstructured rows): 250 000 x 1024, k = 1000, two passes: 6.9 ms -> 4.5; 100 000 x 256, k = 2000, three: 3.7 -> 1.7; 60 000 x 512, k = 500, four: 1.65 -> 1.08.
+// Nine passes of a Train with the walk beside it: 1M x 1024, k = 4000: 23.3 -> 18.2 (the walk has fewer SMs meanwhile: 18.2 -> 20.5), 250 000 x 1536,
+// k = 2048: 5.8 - 6.4 -> 6.0, 30 000 x 768, k = 1000: 0.80 -> 0.71 - 0.76.
 // Every wait is bounded (see kernels_tc.cu).
 #include <cfloat>
 #include <cmath>

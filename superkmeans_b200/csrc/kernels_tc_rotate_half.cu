@@ -1,17 +1,19 @@
 // Rotation on the tensor cores as in kernels_tc_rotate.cu, out = A * B^T for row-major fp32 A [n][K] and B [n_out][K], from fp16 halves: for
-// rows that a trained model is applied to (AssignTrainingPoints).  The rows of a training itself stay with the tf32 kernel: it is
-// as accurate as it needs to be, and a training amplifies a difference in the last digits (a point that changes its mesocluster
-// shifts the first centroids of every point behind it), so that the same seed would no longer give the same model.
+// rows that a trained model is applied to (AssignTrainingPoints).  The rows of a training itself stay with the tf32 kernel: another last digit in
+// every row moves many points, and a training amplifies that (a point that changes its mesocluster shifts the first centroids of every
+// point behind it): with these rows the same seed gave centroids that were off by 0.01 to 0.2.  (The dense chain's fp16 halves are another matter: what it finds is
+// settled in fp32, so that they show only in a pair at a threshold: of nine trainings eight kept every bit, one was 3e-4 off.)
 //
-// Both operands are sums of two fp16 numbers, v * scale = hi + lo, to 22 bits and more (what two tf32 parts hold); a product is
+// Both operands are sums of two fp16 numbers, v * scale = hi + lo, to 22 bits of every value down to 2^-17 of the largest that shares its scale; a product is
 // hi*hi + hi*lo + lo*hi with fp32 accumulation, at twice the rate of tf32.  B arrives so, with a power of two per row as its scale.  A's
 // scale is one per row and 64 columns: that much is a stage, and the thread that has a row of it finds the largest element and writes the
 // halves over the row, in place.  The accumulator in tensor memory truncates on every addition, so that a long chain of products ends up
 // low (about 1e-8 a term, relative to |a| |b|): a chain here is those 64 columns, whose sum the epilogue multiplies by 1 / scale and adds
 // to its fp32 registers while the next ones go into the other accumulator.
 // One B200, products counted three times, against the tf32 kernel: 300 000 x 768: 1.75 ms -> 1.05 (608 -> 1007 TF/s),
-// 250 000 x 1536: 5.29 -> 3.10, 20 000 x 768: 0.16 -> 0.10, 100 000 x 770 (copied first): 3.23 -> 1.40.  Error against fp64, relative to a row's
-// length: 1.0e-7 (K = 32) to 1.7e-7 (2048); the tf32 kernel: 3e-7 (K = 128) to 3.7e-6 (2048).
+// 250 000 x 1536: 5.29 -> 3.10, 20 000 x 768: 0.16 -> 0.10, 100 000 x 770 (copied first): 3.23 -> 1.40.  Error against fp64 with an orthonormal B, relative to
+// a row's length, rms (largest of 2000 rows): 1.9e-8 (1.2e-7) at K = 32, 1.2e-8 (8e-8) at 132, 0.4e-8 (4e-8) at 1536; the tf32 kernel: 3.4e-8 (2.1e-7), 3.5e-8
+// (1.9e-7), 7.0e-8 (3.9e-7); the fp32 tiles: 1.8e-8 (2 - 3e-7) at any width.
 //
 // Persistent pairs of CTAs (cta_group::2) on tiles of 256 x 256 in turn, four groups of four warps that share the block's registers
 // unevenly (setmaxnreg): 64 a thread for the first, 112 for the second (a row of 64 values) and 168 for the others (128 sums):
