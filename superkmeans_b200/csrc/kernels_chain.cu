@@ -390,7 +390,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(C_THREADS, 1) chain_
                     for (int q = 3; q >= 0; --q) {
                         uint32_t& lo = r[8 * h + 2 * q];
                         uint32_t& hi = r[8 * h + 2 * q + 1];
-                        const uint64_t pd = add2(fma2(mul2(factor2, fv[q]), pack2(__uint_as_float(lo), __uint_as_float(hi)), nx2), nyv[q]);
+                        // (the sum takes one factor after the other: their product may be no float)
+                        const uint64_t pd = add2(fma2(mul2(factor2, pack2(__uint_as_float(lo), __uint_as_float(hi))), fv[q], nx2), nyv[q]);
                         const uint64_t over = add2(pd, minus_thr2);
                         lo = static_cast<uint32_t>(pd);
                         hi = static_cast<uint32_t>(pd >> 32);
@@ -521,11 +522,25 @@ __global__ void __launch_bounds__(128) merge_chain_kernel(const ChainPartial* __
     top2[row] = make_uint2(st.i1, st.i2);
 }
 
+// Power of two that maps the largest element of a row below 2^14, for rows whose squared norm is no normal number any more (shorter than 1e-19, longer
+// than 1.7e19): they are told apart in fp32 all the same.
+__device__ __forceinline__ float scale_of_largest(const float* __restrict__ row, uint32_t d, int lane) {
+    float m = 0.f;
+    for (uint32_t j = lane; j < d; j += 32) m = fmaxf(m, fabsf(__ldg(row + j)));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (!(m > 0.f) || m > FLT_MAX) return 1.0f;
+    int e;
+    frexpf(m, &e);
+    return ldexpf(1.0f, min(14 - e, 126));
+}
+
 // A row of points or centroids for the chain, by a warp: cumulative squared norms at the checkpoints, then the halves in the order of the
 // chain (ChainShape), zeros behind every segment.  Returns the scale.
 __device__ __forceinline__ float chain_row(const float* __restrict__ row, const ChainShape& s, float* norms, size_t norms_stride, __half* __restrict__ hi, __half* __restrict__ lo,
                                            int lane) {
-    const float scale = split_scale(chain_norms_row(row, s.partial_d, s.vertical_d, s.horizontal_d, lane, norms, norms_stride));
+    const float sqnorm = chain_norms_row(row, s.partial_d, s.vertical_d, s.horizontal_d, lane, norms, norms_stride);
+    const float scale = has_split_scale(sqnorm) ? split_scale(sqnorm) : scale_of_largest(row, s.d, lane);
     const uint32_t pitch = s.pitch(), h0 = s.begin(1), t0 = h0 + s.horizontal_d;
     for (uint32_t c = 4 * lane; c < pitch; c += 128) {
         float v[4] = {0.f, 0.f, 0.f, 0.f};

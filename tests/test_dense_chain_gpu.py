@@ -62,3 +62,25 @@ def test_a_centroid_a_little_nearer_than_the_previous_one(n, d):
     # the search may drop it on the way, in either form; what the fp32 form finds is found, but for pairs within rounding of a threshold
     assert found[2].mean() >= 0.5
     assert (found[3] | ~found[2]).mean() >= 0.99, (found[2].mean(), found[3].mean())
+
+
+# squared norms below the smallest normal float, and within a tenth of the largest
+@pytest.mark.parametrize("length", [1e-20, 3e-21, 1.75e19, 1.83e19])
+def test_rows_at_the_ends_of_what_floats_hold(length):
+    from superkmeans_b200 import engine
+
+    n, k, d = 700, 300, 256
+    rng = np.random.default_rng(7)
+    y = rng.standard_normal((k, d))
+    y /= np.linalg.norm(y, axis=1, keepdims=True)
+    at = rng.integers(0, k, n)
+    x = y[at] + 0.3 / np.sqrt(d) * rng.standard_normal((n, d))
+    x /= np.linalg.norm(x, axis=1, keepdims=True)
+    x, y, prev = (x * length).astype(np.float32), (y * length).astype(np.float32), rng.integers(0, k, n).astype(np.uint32)
+    for mode in (2, 3):
+        engine.set_prune_split(mode)
+        try:
+            knn = engine.find_nearest_pruned(x, y, prev, 96)[0]
+        finally:
+            engine.set_prune_split(0)
+        assert (knn == at).mean() >= 0.99, (mode, (knn == at).mean())   # the search may drop a centroid on the way
