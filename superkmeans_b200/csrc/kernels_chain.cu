@@ -522,8 +522,8 @@ __global__ void __launch_bounds__(128) merge_chain_kernel(const ChainPartial* __
     top2[row] = make_uint2(st.i1, st.i2);
 }
 
-// Power of two that maps the largest element of a row below 2^14, for rows whose squared norm is no normal number any more (shorter than 1e-19, longer
-// than 1.7e19): they are told apart in fp32 all the same.
+// Power of two that maps the largest element of a row below 2^14, for rows whose squared norm is no normal number any more: shorter than 1e-19, which fp32
+// tells apart all the same, or longer than 1.8e19, of which some checkpoints are still finite.
 __device__ __forceinline__ float scale_of_largest(const float* __restrict__ row, uint32_t d, int lane) {
     float m = 0.f;
     for (uint32_t j = lane; j < d; j += 32) m = fmaxf(m, fabsf(__ldg(row + j)));

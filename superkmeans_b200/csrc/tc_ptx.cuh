@@ -293,13 +293,15 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
 
 // Power of two that maps a vector of this squared norm into [-2^14, 2^14]: hi and lo then hold 22 bits of every element down
 // to 2^-17 of the norm, and smaller ones to 2^-39 of it.  At most 2^74, so that the product of two factors is no less than the smallest
-// float.
-__device__ __forceinline__ bool has_split_scale(float sqnorm) { return sqnorm >= FLT_MIN && sqnorm < 3e38f; }
+// float: vectors whose squared norm is less than a normal number get that (their elements still have 22 bits where their squares are floats at all).
+__device__ __forceinline__ bool has_split_scale(float sqnorm) { return sqnorm >= FLT_MIN && sqnorm <= FLT_MAX; }
 __device__ __forceinline__ float split_scale(float sqnorm) {
+    constexpr int kMost = 74;
+    if (sqnorm < FLT_MIN) return ldexpf(1.0f, kMost);
     if (!has_split_scale(sqnorm)) return 1.0f;
     int e;
     frexpf(sqrtf(sqnorm), &e);
-    return ldexpf(1.0f, min(14 - e, 74));
+    return ldexpf(1.0f, min(14 - e, kMost));
 }
 
 // Tensor maps (defined in kernels_tc.cu), zero fill outside the matrix.

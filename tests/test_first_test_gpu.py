@@ -78,3 +78,27 @@ def test_centroids_of_very_different_norms(kind, lists):
         # the fp32 search sums a distance by differences, the listed one recomputes it so: a rounding per sum of 64
         assert (np.abs(dist.astype(np.float64) - want_dist)[same] <= 1e-5 * scale).all()
         assert np.abs(kept.astype(np.int64) - want_kept.astype(np.int64)).sum() <= 2 + 5e-3 * want_kept.sum(), (pd, kept.sum(), want_kept.sum())
+
+
+# squared norms below the smallest normal float, and within a tenth of the largest
+@pytest.mark.parametrize("length", [1e-20, 3e-21, 1.75e19, 1.83e19])
+def test_rows_at_the_ends_of_what_floats_hold(length):
+    """Every row has a previous centroid near it, which leaves few to look at, and a nearer one."""
+    from superkmeans_b200 import engine
+
+    n, k, d = 900, 300, 256
+    rng = np.random.default_rng(3)
+    y = np.empty((2 * k, d))
+    y[0::2] = rng.standard_normal((k, d))
+    y[1::2] = y[0::2] + 0.5 * rng.standard_normal((k, d))
+    at = 2 * rng.integers(0, k, n)
+    x = y[at] + 0.1 * rng.standard_normal((n, d))
+    scale = length / np.linalg.norm(np.concatenate([x, y]), axis=1).max()
+    x, y, prev = (x * scale).astype(np.float32), (y * scale).astype(np.float32), (at + 1).astype(np.uint32)
+    for mode in (1, 4):
+        engine.set_prune_split(mode)
+        try:
+            knn = engine.find_nearest_pruned(x, y, prev, 96)[0]
+        finally:
+            engine.set_prune_split(0)
+        assert (knn == at).mean() >= 0.99, (mode, (knn == at).mean())   # the search may drop a centroid on the way
